@@ -479,6 +479,8 @@ int dpc_plan_create(dpc_ctx* ctx, const dpc_layer* layers, int n_layers, int bat
     return cuda_fail(err, "dpc_plan_create");
   }
   rc = tc_plan_init(p);
+  if (rc >= 0)
+    rc = res_plan_init(p);
   if (rc < 0)
   {
     dpc_plan_destroy(p);
@@ -501,7 +503,10 @@ int dpc_plan_update(dpc_plan* p, const dpc_layer* layers, int n_layers)
   p->h.assign(layers, layers + n_layers);
   DPC_CUDA(cudaMemcpy(p->d, layers, sizeof(dpc_layer) * n_layers, cudaMemcpyHostToDevice));
   tc_plan_free(p);
+  res_plan_free(p);
   rc = tc_plan_init(p);
+  if (rc >= 0)
+    rc = res_plan_init(p);
   return rc < 0 ? rc : DPC_OK;
 }
 
@@ -510,6 +515,7 @@ int dpc_plan_destroy(dpc_plan* p)
   if (!p)
     return DPC_OK;
   tc_plan_free(p);
+  res_plan_free(p);
   if (p->d)
     cudaFree(p->d);
   if (p->energy)

@@ -64,10 +64,14 @@ struct dpc_plan
   const float* e_terminal = nullptr; // terminal error the DFA / Psi kernels read
   dpc::TensorRun run;
   void* tc = nullptr; // tensor-core path state (tensor maps), owned by dpc_tc.cu
+  void* res = nullptr; // row-segment path state, owned by dpc_resident.cu
 };
 
 namespace dpc
 {
+// dpc_resident.cu — row segments of small networks.  DPC_OK: the plan has them, 1: it does not.
+int res_plan_init(dpc_plan* plan);
+void res_plan_free(dpc_plan* plan);
 // dpc_tc.cu — tensor-core (tcgen05/TMEM/TMA) path.  Each returns DPC_OK when it handled
 // layers [first, first+count) completely, 1 when the range is not eligible (the caller
 // then uses the CUDA-core kernels), or a negative status.

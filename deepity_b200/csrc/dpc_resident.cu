@@ -1,0 +1,1082 @@
+// Row-resident train step of small dense networks.
+//
+// Within a step the batch rows meet only in the weight updates: a forward sweep, any number of
+// settling steps, the refresh before learning and the closing energy are all row-local.  For a
+// network whose weights fit (or nearly fit) one SM's shared memory, a launch per phase is pure
+// latency -- a settling step of a 784-128-128-10 network at batch 64 is 2 MFLOP and took 44 us in
+// three launches.  Here one CTA owns R rows and walks all phases between two weight updates by
+// itself ("segment"): weights in shared memory (layer by layer, as many as fit, the others streamed
+// from L2), beliefs, errors and gated errors of its rows in shared memory, no launch and no global
+// traffic inside the settling loop, only barriers of the CTA.
+//
+// A pass is a list of warp tasks that leave partial sums in shared memory, a barrier, and an
+// elementwise pass that adds them in a fixed order and finishes (activation, error, gated error, or
+// the state update); all layers of a settling pass are independent (Jacobi) and share one list.
+//   forward, resident weights   lane = output, walking a slice of K: no reduction, no idle epilogue
+//                               lanes (lanes along K with a shuffle reduction spend 300 instructions
+//                               on 8 outputs of a 128-wide row, and a settling step is bound by issue
+//                               slots).  Row pitch 4 x odd floats, so the lanes' 16-byte reads of
+//                               neighbouring rows meet no bank conflict.
+//   forward, streamed weights   lanes along K (coalesced), G outputs x R rows, halving reduction
+//   state update                lane = 4 (or 1) input columns, walking a slice of the output rows
+//
+// The same tasks, i.e. the same order of additions, serve the sweep and every later pass: a belief
+// that the sweep produced has an error of exactly zero afterwards (Adam-type updates rely on it).
+#include <algorithm>
+#include <cstdlib>
+#include <cstring>
+
+#include "dpc_internal.h"
+#include "dpc_math.cuh"
+
+namespace dpc
+{
+namespace
+{
+constexpr int kThreads = 512, kWarps = kThreads / 32;
+constexpr int kMaxLayers = 96;
+constexpr size_t kSmemLimit = 227 * 1024, kStatic = 4 * 1024; // per block; of it static
+
+struct ResLayer // one per weight layer, built on the host
+{
+  int K, N;
+  int zoff, noff;    // offsets of layers l and l+1 in a row's state (multiples of 4)
+  int ldw, woff;     // row pitch and offset of W in shared memory; woff < 0: streamed
+  int vec;           // rows of W in global memory can be read 16 bytes at a time
+  int kw;            // columns per lane of a state task: 4 or 1
+  int fpart, fslice; // forward partial sums: offset, length of a slice of K
+  int bpart, bslice; // state partial sums: offset, length of a slice of the output rows
+};
+
+// Four neighbouring floats of a row's state (they belong to one layer).
+struct __align__(16) ResQuad
+{
+  int fpart, bpart;       // their partial sums of slice 0, row 0 (row pitch `pitch`)
+  short fslices, bslices; // slices of the prediction from below / of the feedback from above
+  short layer, valid;     // layer 1 .. n-1; columns that exist (the rest is padding)
+  int col, pitch;         // first column inside the layer, padded width of the layer
+  int pad[2];
+};
+
+struct ResParams
+{
+  const dpc_layer* layers;
+  // one table in global memory, copied to shared memory as it is:
+  //   ResLayer[nw] | ResQuad[S / 4] | forward tasks | state tasks, packed by pack()
+  const int4* table;
+  int table_vecs, a_quad, a_ft, a_bt; // its size in 16-byte units, byte offsets of the parts
+  int n, batch, S;                    // layers, rows, floats of one row's state (layers 1..n-1)
+  int nf, nb;                         // task counts
+  int N1p, K0p;                       // padded width of layer 1 and of the input
+  int ks0, kslice0;                   // input layer: slices of K and their length
+  int wfloats;                        // resident weights
+  int groups;                         // row groups
+  int ops, steps;
+  int simple, has_v, ce, top_clamped, top_down_off, top_n;
+  double* energy;
+};
+
+// layer (7 bits) | row block (2) | slice (5) | output or column block (11)
+__host__ __device__ __forceinline__ int pack(int l, int rb, int s, int blk)
+{
+  return l << 18 | rb << 16 | s << 11 | blk;
+}
+
+template <int R>
+constexpr int kRowsPerTask = R >= 4 ? 4 : R;
+
+template <int V>
+__device__ __forceinline__ float reduce_values(float (&a)[V], int lane)
+{
+  // the lanes exchange halves: after log2(V) steps lane i holds a partial sum of value
+  // i >> (5 - log2 V), the remaining steps add the lanes that hold the same one
+  int bit = 16;
+#pragma unroll
+  for (int w = V / 2; w >= 1; w >>= 1)
+  {
+    const bool upper = (lane & bit) != 0;
+#pragma unroll
+    for (int i = 0; i < w; ++i)
+    {
+      const float send = upper ? a[i] : a[i + w];
+      const float keep = upper ? a[i + w] : a[i];
+      a[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+    }
+    bit >>= 1;
+  }
+  float s = a[0];
+#pragma unroll
+  for (; bit >= 1; bit >>= 1)
+    s += __shfl_xor_sync(0xffffffffu, s, bit);
+  return s;
+}
+
+// Streamed weights: acc[r * G + g] += sum over this lane's k in [k0, k1) of x[r][k] * W[row g][k]
+template <int R, int G>
+__device__ __forceinline__ void dot_streamed(float (&acc)[R * G], const float* __restrict__ W, int ldw,
+                                             int rows_left, const float* x, int xs, int k0, int k1,
+                                             int lane, bool vec)
+{
+  const float* row[G];
+#pragma unroll
+  for (int g = 0; g < G; ++g)
+    row[g] = W + (size_t)min(g, rows_left - 1) * ldw;
+  if (vec)
+    for (int k = k0 + lane * 4; k < k1; k += 128)
+    {
+      float4 w[G];
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+        w[g] = *reinterpret_cast<const float4*>(row[g] + k);
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+      {
+        const float4 v = *reinterpret_cast<const float4*>(x + r * xs + k);
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+        {
+          float s = acc[r * G + g];
+          s = fmaf(v.x, w[g].x, s);
+          s = fmaf(v.y, w[g].y, s);
+          s = fmaf(v.z, w[g].z, s);
+          acc[r * G + g] = fmaf(v.w, w[g].w, s);
+        }
+      }
+    }
+  else
+#pragma unroll 2
+    for (int k = k0 + lane; k < k1; k += 32)
+    {
+      float w[G];
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+        w[g] = row[g][k];
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+      {
+        const float v = x[r * xs + k];
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+          acc[r * G + g] = fmaf(v, w[g], acc[r * G + g]);
+      }
+    }
+}
+
+// Resident weights: this lane's output over k in [k0, k1) (slices of multiples of 4, zero-padded).
+template <int RT>
+__device__ __forceinline__ void dot_resident(const float* w, const float* x, int S, int k0, int k1,
+                                             float* out, int pitch, bool valid)
+{
+  float acc[RT];
+#pragma unroll
+  for (int r = 0; r < RT; ++r)
+    acc[r] = 0.0f;
+#pragma unroll 4
+  for (int k = k0; k < k1; k += 4)
+  {
+    const float4 wv = *reinterpret_cast<const float4*>(w + k);
+#pragma unroll
+    for (int r = 0; r < RT; ++r)
+    {
+      const float4 v = *reinterpret_cast<const float4*>(x + r * S + k);
+      acc[r] = fmaf(v.x, wv.x, acc[r]);
+      acc[r] = fmaf(v.y, wv.y, acc[r]);
+      acc[r] = fmaf(v.z, wv.z, acc[r]);
+      acc[r] = fmaf(v.w, wv.w, acc[r]);
+    }
+  }
+  if (valid)
+#pragma unroll
+    for (int r = 0; r < RT; ++r)
+      out[r * pitch] = acc[r];
+}
+
+// One state task: sums over W rows [n0, n1) (n0 a multiple of 4) for this lane's KW columns.
+template <int RT, int KW>
+__device__ __forceinline__ void state_task(const float* W, int ldw, int n0, int n1, const float* g, int S,
+                                           float* out, int pitch)
+{
+  float acc[RT][KW];
+#pragma unroll
+  for (int r = 0; r < RT; ++r)
+#pragma unroll
+    for (int c = 0; c < KW; ++c)
+      acc[r][c] = 0.0f;
+  const float* w = W + (size_t)n0 * ldw;
+  int n = n0;
+  for (; n + 4 <= n1; n += 4, w += 4 * (size_t)ldw)
+  {
+    float wv[4][KW];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+    {
+      if constexpr (KW == 4)
+      {
+        const float4 v = *reinterpret_cast<const float4*>(w + j * (size_t)ldw);
+        wv[j][0] = v.x, wv[j][1] = v.y, wv[j][2] = v.z, wv[j][3] = v.w;
+      }
+      else
+        wv[j][0] = w[j * (size_t)ldw];
+    }
+#pragma unroll
+    for (int r = 0; r < RT; ++r)
+    {
+      const float4 v = *reinterpret_cast<const float4*>(g + r * S + n);
+#pragma unroll
+      for (int c = 0; c < KW; ++c)
+      {
+        acc[r][c] = fmaf(v.x, wv[0][c], acc[r][c]);
+        acc[r][c] = fmaf(v.y, wv[1][c], acc[r][c]);
+        acc[r][c] = fmaf(v.z, wv[2][c], acc[r][c]);
+        acc[r][c] = fmaf(v.w, wv[3][c], acc[r][c]);
+      }
+    }
+  }
+  for (; n < n1; ++n, w += ldw)
+#pragma unroll
+    for (int c = 0; c < KW; ++c)
+    {
+      const float wv = w[c];
+#pragma unroll
+      for (int r = 0; r < RT; ++r)
+        acc[r][c] = fmaf(g[r * S + n], wv, acc[r][c]);
+    }
+#pragma unroll
+  for (int r = 0; r < RT; ++r)
+#pragma unroll
+    for (int c = 0; c < KW; ++c)
+      out[r * pitch + c] = acc[r][c];
+}
+
+__device__ __forceinline__ void cp_async16(float* dst, const float* src)
+{
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+
+struct LayerConst // what a finished sum of layer l needs, one 16-byte read
+{
+  float a, ir;
+  int act, residual;
+};
+
+template <int R>
+__global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P)
+{
+  constexpr int RT = kRowsPerTask<R>;
+  constexpr int G = R == 8 ? 4 : 8, V = R * G, LPV = 32 / V; // outputs per group, lanes per value
+  extern __shared__ __align__(16) float sm[];
+  __shared__ __align__(16) LayerConst lc[kMaxLayers];
+  __shared__ const float* sW[kMaxLayers];
+  __shared__ float red[kWarps];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int S = P.S, nw = P.n - 1; // nw weight layers
+  const bool simple = P.simple != 0;
+
+  // ---- shared memory: weights | table | bias | Z E G(or f(z)) [V] | mu0 d0 | top mu, d | X / partials
+  float* Ws = sm;
+  unsigned char* tab = reinterpret_cast<unsigned char*>(Ws + P.wfloats);
+  const ResLayer* sl = reinterpret_cast<const ResLayer*>(tab);
+  const ResQuad* quad = reinterpret_cast<const ResQuad*>(tab + P.a_quad);
+  const int* ftab = reinterpret_cast<const int*>(tab + P.a_ft);
+  const int* btab = reinterpret_cast<const int*>(tab + P.a_bt);
+  float* bias = reinterpret_cast<float*>(tab + 16 * (size_t)P.table_vecs);
+  float* Z = bias + S;
+  float* E = Z + R * S;
+  float* Gb = E + R * S; // gated errors; SimplePC: f(z), the forward operand
+  float* Vb = Gb + R * S;
+  float* mu0 = Vb + (P.has_v ? R * S : 0);
+  float* d0 = mu0 + R * P.N1p;
+  float* topmu = d0 + R * P.N1p;
+  const int NT = P.top_n, NTp = (NT + 3) & ~3;
+  float* topd = topmu + R * NTp;
+  float* X = topd + R * NTp; // input rows; later the partial sums of the tasks
+
+  // elementwise passes over the R x S state: `ew` threads along a row, kThreads / ew rows at a time
+  const int ew = min(kThreads, (S + 31) & ~31), ex = tid % ew, ey = tid / ew, er = kThreads / ew;
+
+  for (int i = tid; i < P.table_vecs; i += kThreads)
+    reinterpret_cast<int4*>(tab)[i] = __ldg(P.table + i);
+  for (int l = tid; l <= nw; l += kThreads)
+  {
+    const dpc_layer& L = P.layers[l];
+    sW[l] = L.W;
+    lc[l] = LayerConst{L.a, L.ir, L.act, (L.flags & DPC_LAYER_RESIDUAL) ? 1 : 0};
+  }
+  __syncthreads();
+  for (int l = 1; l < nw; ++l)
+  {
+    const ResLayer L = sl[l];
+    if (L.woff < 0)
+      continue;
+    const float* src = sW[l];
+    float* dst = Ws + L.woff;
+    for (int r = warp; r < L.N; r += kWarps)
+      if (L.vec)
+        for (int c = lane * 4; c < L.K; c += 128)
+          cp_async16(dst + r * L.ldw + c, src + (size_t)r * L.K + c);
+      else
+        for (int c = lane; c < L.ldw; c += 32)
+          dst[r * L.ldw + c] = c < L.K ? src[(size_t)r * L.K + c] : 0.0f;
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int i = tid; i < S; i += kThreads)
+  {
+    const ResQuad q = quad[i >> 2];
+    bias[i] = (i & 3) < q.valid ? P.layers[q.layer - 1].b[q.col + (i & 3)] : 0.0f;
+  }
+
+  const bool first = P.ops & DPC_ROWS_FIRST;
+  double esum = 0.0;
+
+  for (int grp = blockIdx.x; grp < P.groups; grp += gridDim.x)
+  {
+    const int row0 = grp * R;
+    const int rows = min(R, P.batch - row0);
+    __syncthreads();
+
+    // ---------------------------------------------------------------- beliefs
+    if (ey < er)
+      for (int r = ey; r < R; r += er)
+        for (int i = ex; i < S; i += ew)
+        {
+          const ResQuad q = quad[i >> 2];
+          const int l = q.layer, w = sl[l - 1].N;
+          const bool in = r < rows && (i & 3) < q.valid;
+          const dpc_layer& L = P.layers[l];
+          const size_t o = (size_t)(row0 + r) * w + q.col + (i & 3);
+          float z = 0.0f, e = 0.0f, v = 0.0f;
+          if (in && ((P.top_clamped && l == nw) || !(P.ops & (DPC_ROWS_SWEEP | DPC_ROWS_ZERO_Z))))
+            z = L.z[o];
+          if (in && (P.ops & DPC_ROWS_LOAD_E))
+            e = L.e[o];
+          if (P.has_v)
+          {
+            if (in && !(P.ops & DPC_ROWS_ZERO_V) && L.v)
+              v = L.v[o];
+            Vb[r * S + i] = v;
+          }
+          Z[r * S + i] = z;
+          E[r * S + i] = e;
+          Gb[r * S + i] = simple && l < nw ? act_fwd(lc[l].act, z) : 0.0f;
+        }
+    // ---------------------------------------------------------------- the clamped input layer
+    {
+      const ResLayer L = sl[0];
+      const dpc_layer& D = P.layers[0];
+      if (first)
+      {
+        for (int r = 0; r < R; ++r)
+          for (int k = tid; k < P.K0p; k += kThreads)
+          {
+            float v = 0.0f;
+            if (r < rows && k < L.K)
+            {
+              const size_t o = (size_t)(row0 + r) * L.K + k;
+              v = D.z[o];
+              if (simple)
+              {
+                v = act_fwd(lc[0].act, v);
+                D.zF[o] = v;
+              }
+            }
+            X[r * P.K0p + k] = v;
+          }
+        __syncthreads();
+        float* part = X + R * P.K0p;
+        const int ng = (L.N + G - 1) / G, nt = ng * P.ks0;
+        for (int t = warp; t < nt; t += kWarps)
+        {
+          const int g0 = (t / P.ks0) * G, s = t % P.ks0;
+          const int k0 = s * P.kslice0, k1 = min(L.K, k0 + P.kslice0);
+          float acc[V];
+#pragma unroll
+          for (int i = 0; i < V; ++i)
+            acc[i] = 0.0f;
+          dot_streamed<R, G>(acc, sW[0] + (size_t)g0 * L.K, L.K, L.N - g0, X, P.K0p, k0, k1, lane,
+                             L.vec != 0);
+          const float v = reduce_values<V>(acc, lane);
+          if (lane % LPV == 0)
+            part[t * V + lane / LPV] = v;
+        }
+        __syncthreads();
+        for (int i = tid; i < R * L.N; i += kThreads)
+        {
+          const int r = i / L.N, c = i - r * L.N;
+          float v = 0.0f;
+          for (int s = 0; s < P.ks0; ++s)
+            v += part[((c / G) * P.ks0 + s) * V + r * G + c % G];
+          const float pre = lc[0].a * v + bias[L.noff + c];
+          float mu = pre, d = 1.0f;
+          if (!simple)
+            act_both(lc[0].act, pre, mu, d); // (a residual layer is never the first)
+          mu0[r * P.N1p + c] = mu;
+          d0[r * P.N1p + c] = d;
+          if (r < rows)
+          {
+            const size_t o = (size_t)(row0 + r) * L.N + c;
+            D.mu[o] = mu;
+            if (D.preact)
+              D.preact[o] = pre;
+          }
+        }
+      }
+      else
+        for (int i = tid; i < R * L.N; i += kThreads)
+        {
+          const int r = i / L.N, c = i - r * L.N;
+          const size_t o = (size_t)(row0 + r) * L.N + c;
+          mu0[r * P.N1p + c] = r < rows ? D.mu[o] : 0.0f;
+          d0[r * P.N1p + c] = (r < rows && !simple) ? act_deriv(lc[0].act, D.preact[o]) : 1.0f;
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+
+    // One forward task: partial sums of 32 outputs x RT rows (resident) or G outputs x R rows.
+    auto forward_task = [&](int entry)
+    {
+      const int l = entry >> 18, rb = (entry >> 16) & 3, s = (entry >> 11) & 31, blk = entry & 2047;
+      const ResLayer& L = sl[l];
+      const float* x = (simple ? Gb : Z) + L.zoff;
+      const int pitch = (L.N + 3) & ~3;
+      float* out = X + L.fpart + s * (R * pitch);
+      if (L.woff >= 0)
+      {
+        const int c = blk * 32 + lane, k0 = s * L.fslice;
+        dot_resident<RT>(Ws + L.woff + min(c, L.N - 1) * L.ldw, x + rb * RT * S, S, k0,
+                         min(L.K, k0 + L.fslice), out + rb * RT * pitch + c, pitch, c < L.N);
+        return;
+      }
+      float acc[V];
+#pragma unroll
+      for (int i = 0; i < V; ++i)
+        acc[i] = 0.0f;
+      const int g0 = blk * G;
+      dot_streamed<R, G>(acc, sW[l] + (size_t)g0 * L.K, L.K, L.N - g0, x, S, 0, L.K, lane, L.vec != 0);
+      const float v = reduce_values<V>(acc, lane);
+      const int idx = lane / LPV, r = idx / G, c = g0 + idx % G;
+      if (lane % LPV == 0 && c < L.N)
+        out[r * pitch + c] = v;
+    };
+    // The finished sum of state element i (of quad q) of row r: pre-activation of the layer below.
+    auto pre_of = [&](const ResQuad& q, int r, int i, int l)
+    {
+      const float* p = X + q.fpart + r * q.pitch + (i & 3);
+      float v = 0.0f;
+#pragma unroll 4
+      for (int s = 0; s < q.fslices; ++s)
+        v += p[s * (R * q.pitch)];
+      return lc[l].a * v + bias[i];
+    };
+    auto store_pred = [&](int l, int r, int c, float pre, float mu)
+    {
+      if (r < rows)
+      {
+        const dpc_layer& D = P.layers[l];
+        const size_t o = (size_t)(row0 + r) * sl[l].N + c;
+        D.mu[o] = mu;
+        if (D.preact)
+          D.preact[o] = pre;
+      }
+    };
+    auto predict = [&](int l, int r, int c, float pre, float& mu, float& d)
+    {
+      mu = pre, d = 1.0f;
+      if (!simple)
+      {
+        act_both(lc[l].act, pre, mu, d);
+        if (lc[l].residual)
+          mu += Z[r * S + sl[l].zoff + c];
+      }
+    };
+    // softmax cross-entropy error of the top layer from its logits (one warp per row)
+    auto ce_error = [&](bool energy)
+    {
+      for (int r = warp; r < R; r += kWarps)
+      {
+        const float* m = topmu + r * NTp;
+        const int to = sl[nw - 1].noff;
+        float mx = -INFINITY, s = 0.0f, en = 0.0f;
+        for (int j = lane; j < NT; j += 32)
+          mx = fmaxf(mx, m[j]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        for (int j = lane; j < NT; j += 32)
+          s += expf(m[j] - mx);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+          s += __shfl_xor_sync(0xffffffffu, s, o);
+        for (int j = lane; j < NT; j += 32)
+        {
+          const float p = expf(m[j] - mx) / s;
+          const float z = Z[r * S + to + j];
+          en -= z * logf(p + 1e-8f);
+          const float e = z - p;
+          E[r * S + to + j] = e;
+          if (!simple)
+            Gb[r * S + to + j] = e * topd[r * NTp + j];
+        }
+        if (energy && r < rows)
+          esum += 2.0 * (double)en; // (halved at the end; cross-entropy is not)
+      }
+      __syncthreads();
+    };
+
+    // ---------------------------------------------------------------- forward sweep
+    if (P.ops & DPC_ROWS_SWEEP)
+    {
+      int f = 0; // the task list is sorted by layer
+      for (int l = 0; l < nw; ++l)
+      {
+        const ResLayer& L = sl[l];
+        if (l > 0)
+        {
+          int t = f;
+          while (t < P.nf && (ftab[t] >> 18) == l)
+            ++t;
+          for (int q = f + warp; q < t; q += kWarps)
+            forward_task(ftab[q]);
+          f = t;
+          __syncthreads();
+        }
+        const bool copy = !(l + 1 == nw && P.top_clamped);
+        for (int i = tid; i < R * L.N; i += kThreads)
+        {
+          const int r = i / L.N, c = i - r * L.N, o = r * S + L.noff + c;
+          float mu, d;
+          if (l == 0)
+            mu = mu0[r * P.N1p + c], d = d0[r * P.N1p + c];
+          else
+          {
+            const float pre = pre_of(quad[(L.noff + c) >> 2], r, L.noff + c, l);
+            predict(l, r, c, pre, mu, d);
+            if (P.ops & DPC_ROWS_SWEEP_PRED)
+              store_pred(l, r, c, pre, mu);
+          }
+          if (copy)
+          {
+            Z[o] = mu;
+            if (simple && l + 1 < nw)
+              Gb[o] = act_fwd(lc[l + 1].act, mu);
+          }
+          if (l + 1 == nw) // the top prediction feeds the terminal error
+            topmu[r * NTp + c] = mu, topd[r * NTp + c] = d;
+        }
+        __syncthreads();
+      }
+      if (P.ops & DPC_ROWS_TERMINAL)
+      {
+        if (P.ce)
+          ce_error(false);
+        else
+        {
+          const int to = sl[nw - 1].noff;
+          for (int i = tid; i < R * NT; i += kThreads)
+          {
+            const int r = i / NT, c = i - r * NT;
+            E[r * S + to + c] = Z[r * S + to + c] - topmu[r * NTp + c];
+          }
+          __syncthreads();
+        }
+      }
+    }
+
+    // Forward pass of all layers.  err: errors (and gated errors) are recomputed; else the gated
+    // errors are refreshed from the errors that are there.
+    auto forward = [&](bool err, bool gate, bool energy, bool pred)
+    {
+      for (int t = warp; t < P.nf; t += kWarps)
+        forward_task(ftab[t]);
+      __syncthreads();
+      float local = 0.0f;
+      if (ey < er)
+        for (int r = ey; r < R; r += er)
+          for (int i = ex; i < S; i += ew)
+          {
+            const ResQuad q = quad[i >> 2];
+            if ((i & 3) >= q.valid)
+              continue;
+            const int l = q.layer - 1, c = q.col + (i & 3), o = r * S + i;
+            float mu, d;
+            if (l == 0)
+              mu = mu0[r * P.N1p + c], d = d0[r * P.N1p + c];
+            else
+            {
+              const float pre = pre_of(q, r, i, l);
+              predict(l, r, c, pre, mu, d);
+              if (pred)
+                store_pred(l, r, c, pre, mu);
+            }
+            const bool ce_top = P.ce && l == nw - 1;
+            if (ce_top)
+              topmu[r * NTp + c] = mu, topd[r * NTp + c] = d;
+            float e = E[o];
+            if (err && !ce_top)
+            {
+              e = Z[o] - mu;
+              E[o] = e;
+              if (r < rows)
+                local += e * e;
+            }
+            if (gate && !simple && !(err && ce_top))
+              Gb[o] = e * d;
+          }
+      if (energy)
+        esum += (double)local;
+      __syncthreads();
+      if (err && P.ce)
+        ce_error(energy);
+    };
+
+    // ---------------------------------------------------------------- settling
+    for (int t = 0; t < P.steps; ++t)
+    {
+      const bool last = t + 1 == P.steps;
+      forward(true, true, (P.ops & DPC_ROWS_ENERGY_EACH) != 0,
+              last && (P.ops & DPC_ROWS_PRED_LAST) != 0);
+      const float* gate = simple ? E : Gb;
+      for (int q = warp; q < P.nb; q += kWarps)
+      {
+        const int entry = btab[q];
+        const int l = entry >> 18, rb = (entry >> 16) & 3, s = (entry >> 11) & 31, blk = entry & 2047;
+        const ResLayer& L = sl[l];
+        const int n0 = s * L.bslice, n1 = min(L.N, n0 + L.bslice), pitch = (L.K + 3) & ~3;
+        const float* g = gate + L.noff + rb * RT * S;
+        const int k = (blk * 32 + lane) * L.kw;
+        float* out = X + L.bpart + (s * R + rb * RT) * pitch + k;
+        if (k < L.K)
+        {
+          if (L.kw == 4 && L.woff >= 0)
+            state_task<RT, 4>(Ws + L.woff + k, L.ldw, n0, n1, g, S, out, pitch);
+          else if (L.kw == 4)
+            state_task<RT, 4>(sW[l] + k, L.K, n0, n1, g, S, out, pitch);
+          else if (L.woff >= 0)
+            state_task<RT, 1>(Ws + L.woff + k, L.ldw, n0, n1, g, S, out, pitch);
+          else
+            state_task<RT, 1>(sW[l] + k, L.K, n0, n1, g, S, out, pitch);
+        }
+      }
+      __syncthreads();
+      const bool refresh_f = simple && !(last && !(P.ops & DPC_ROWS_ENERGY_LAST));
+      if (ey < er)
+        for (int r = ey; r < R; r += er)
+          for (int i = ex; i < S; i += ew)
+          {
+            const ResQuad q = quad[i >> 2];
+            const int l = q.layer, o = r * S + i;
+            if ((i & 3) >= q.valid || (l == nw && P.top_clamped))
+              continue;
+            const LayerConst C = lc[l];
+            float z = Z[o];
+            const float e = E[o];
+            if (l == nw || (P.top_down_off && l == nw - 1))
+            {
+              Z[o] = z - C.ir * e;
+              continue;
+            }
+            const float* pp = X + q.bpart + r * q.pitch + (i & 3);
+            float dz = 0.0f;
+#pragma unroll 4
+            for (int s = 0; s < q.bslices; ++s)
+              dz += pp[s * (R * q.pitch)];
+            if (simple)
+            {
+              z += C.ir * (dz * act_deriv(C.act, z) - e);
+              if (refresh_f)
+                Gb[o] = act_fwd(C.act, z);
+            }
+            else
+            {
+              const float fb = C.a * dz - e;
+              if (P.has_v)
+              {
+                const float beta = P.layers[l].momentum_beta;
+                const float v = beta * Vb[o] + (1.0f - beta) * fb;
+                Vb[o] = v;
+                z += C.ir * v;
+              }
+              else
+                z += C.ir * fb;
+              if (C.residual)
+                z += C.ir * E[r * S + sl[l].noff + q.col + (i & 3)];
+            }
+            Z[o] = z;
+          }
+      __syncthreads();
+    }
+    // ---------------------------------------------------------------- closing pass
+    if (P.ops & DPC_ROWS_REFRESH)
+      forward(false, true, false, (P.ops & DPC_ROWS_PRED_CLOSE) != 0);
+    if (P.ops & DPC_ROWS_PREACT)
+      forward(false, false, false, true);
+    if (P.ops & DPC_ROWS_ENERGY_LAST)
+      forward(true, (P.ops & DPC_ROWS_GATE_LAST) != 0, true, (P.ops & DPC_ROWS_PRED_CLOSE) != 0);
+    if (P.ops & DPC_ROWS_LOGITS)
+    {
+      // the top belief becomes the prediction below it
+      const int l = nw - 1;
+      if (l > 0)
+      {
+        for (int t = warp; t < P.nf; t += kWarps)
+          if ((ftab[t] >> 18) == l)
+            forward_task(ftab[t]);
+        __syncthreads();
+      }
+      for (int i = tid; i < R * NT; i += kThreads)
+      {
+        const int r = i / NT, c = i - r * NT, to = sl[l].noff;
+        float mu, d;
+        if (l == 0)
+          mu = mu0[r * P.N1p + c];
+        else
+        {
+          const float pre = pre_of(quad[(to + c) >> 2], r, to + c, l);
+          predict(l, r, c, pre, mu, d);
+          store_pred(l, r, c, pre, mu);
+        }
+        Z[r * S + to + c] = mu;
+      }
+      __syncthreads();
+    }
+
+    // ---------------------------------------------------------------- back to memory
+    if (ey < er)
+      for (int r = ey; r < rows; r += er)
+        for (int i = ex; i < S; i += ew)
+        {
+          const ResQuad q = quad[i >> 2];
+          if ((i & 3) >= q.valid)
+            continue;
+          const int l = q.layer, w = sl[l - 1].N, o = r * S + i;
+          const dpc_layer& L = P.layers[l];
+          const size_t m = (size_t)(row0 + r) * w + q.col + (i & 3);
+          if ((P.ops & DPC_ROWS_STORE_Z) && !(l == nw && P.top_clamped))
+            L.z[m] = Z[o];
+          if ((P.ops & DPC_ROWS_STORE_E) || ((P.ops & DPC_ROWS_TERMINAL) && l == nw))
+            L.e[m] = E[o];
+          if ((P.ops & DPC_ROWS_STORE_G) && !simple)
+            P.layers[l - 1].fe[m] = Gb[o];
+          if (simple && l < nw && (P.ops & DPC_ROWS_STORE_Z))
+            L.zF[m] = Gb[o];
+          if (P.has_v && (P.ops & DPC_ROWS_STORE_V) && L.v)
+            L.v[m] = Vb[o];
+        }
+    if (P.ops & DPC_ROWS_STORE_E)
+    {
+      float* e0 = P.layers[0].e + (size_t)row0 * sl[0].K;
+      for (int i = tid; i < rows * sl[0].K; i += kThreads)
+        e0[i] = 0.0f;
+    }
+  }
+  if (P.ops & (DPC_ROWS_ENERGY_EACH | DPC_ROWS_ENERGY_LAST))
+  {
+    float s = (float)esum;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0)
+      red[warp] = s;
+    __syncthreads();
+    if (tid == 0)
+    {
+      double t = 0.0;
+      for (int w = 0; w < kWarps; ++w)
+        t += (double)red[w];
+      atomicAdd(P.energy, 0.5 * t);
+    }
+  }
+}
+
+struct ResState
+{
+  ResParams P = {};
+  int R = 1;
+  size_t smem = 0;
+  void* dev = nullptr; // tables
+};
+
+inline int up4(int v)
+{
+  return (v + 3) & ~3;
+}
+
+// Tables for groups of R rows; 1 when they do not fit the shared memory.
+int build(dpc_plan* p, int R, int S, bool has_v)
+{
+  const int nw = p->n - 1, G = R == 8 ? 4 : 8, RT = std::min(R, 4), rbs = R / RT;
+  std::vector<ResLayer> rl(nw);
+  int off = 0;
+  for (int l = 0; l < nw; ++l)
+  {
+    const dpc_layer& L = p->h[l];
+    ResLayer& q = rl[l];
+    q = ResLayer{};
+    q.K = L.size, q.N = L.next_size;
+    q.noff = off;
+    q.zoff = l ? rl[l - 1].noff : 0;
+    off += up4(q.N);
+    q.vec = L.size % 4 == 0 && ((uintptr_t)L.W % 16) == 0;
+    q.ldw = up4(L.size) | 4; // 4 x odd: lanes that read 16 bytes of neighbouring rows share no bank
+    q.woff = -1;
+  }
+  const int N1p = up4(rl[0].N), K0p = up4(rl[0].K), NTp = up4(rl[nw - 1].N);
+  const int ng0 = (rl[0].N + G - 1) / G;
+  int ks0 = std::max(1, std::min(2 * kWarps / std::max(ng0, 1), (K0p + 127) / 128));
+  const int kslice0 = ((K0p + ks0 - 1) / ks0 + 3) & ~3;
+  ks0 = (K0p + kslice0 - 1) / kslice0;
+
+  std::vector<int> ft, bt;
+  size_t fparts = 0, bparts = 0;
+  // Slices: one layer's tasks alone should occupy the warps (the sweep runs layer by layer), a slice
+  // being worth its overhead from 32 inputs or 16 output rows on; halved while the partial sums of
+  // all layers take more than 32 KB.
+  auto tasks = [&](int shift)
+  {
+    ft.clear(), bt.clear();
+    fparts = bparts = 0;
+    for (int l = 1; l < nw; ++l)
+    {
+      ResLayer& q = rl[l];
+      const int np = up4(q.N), kp = up4(q.K);
+      q.fpart = (int)fparts;
+      if (q.woff >= 0)
+      {
+        const int blks = (q.N + 31) / 32;
+        int s = std::max(1, std::min({kWarps / (blks * rbs), q.K / 32, 16}) >> shift);
+        q.fslice = ((q.K + s - 1) / s + 3) & ~3;
+        s = (q.K + q.fslice - 1) / q.fslice;
+        for (int rb = 0; rb < rbs; ++rb)
+          for (int k = 0; k < s; ++k)
+            for (int b = 0; b < blks; ++b)
+              ft.push_back(pack(l, rb, k, b));
+        fparts += (size_t)s * R * np;
+      }
+      else
+      {
+        q.fslice = q.K;
+        for (int b = 0; b < (q.N + G - 1) / G; ++b)
+          ft.push_back(pack(l, 0, 0, b));
+        fparts += (size_t)R * np;
+      }
+      q.kw = q.K >= 96 && (q.woff >= 0 || q.vec) ? 4 : 1;
+      const int blks = (q.K + 32 * q.kw - 1) / (32 * q.kw);
+      int s = std::max(1, std::min({kWarps / (blks * rbs), q.N / 16, 16}) >> shift);
+      q.bslice = ((q.N + s - 1) / s + 3) & ~3;
+      s = (q.N + q.bslice - 1) / q.bslice;
+      q.bpart = (int)bparts;
+      for (int rb = 0; rb < rbs; ++rb)
+        for (int k = 0; k < s; ++k)
+          for (int b = 0; b < blks; ++b)
+            bt.push_back(pack(l, rb, k, b));
+      bparts += (size_t)s * R * kp;
+    }
+    return std::max(fparts, bparts) * sizeof(float) <= 32 * 1024;
+  };
+  auto fit_tasks = [&]()
+  {
+    for (int shift = 0; !tasks(shift) && shift < 4; ++shift)
+      ;
+  };
+  auto round16 = [](size_t b) { return (b + 15) & ~(size_t)15; };
+  auto table_bytes = [&]()
+  {
+    return round16(sizeof(ResLayer) * nw) + sizeof(ResQuad) * (S / 4) +
+           round16(sizeof(int) * ft.size()) + round16(sizeof(int) * bt.size());
+  };
+  auto others = [&]()
+  {
+    const size_t x = std::max({(size_t)R * K0p + (size_t)ng0 * ks0 * R * G, fparts, bparts});
+    const size_t f = table_bytes() / sizeof(float) + S + (size_t)R * S * (has_v ? 4 : 3) +
+                     2 * (size_t)R * N1p + 2 * (size_t)R * NTp + x;
+    return f * sizeof(float) + kStatic;
+  };
+  // residency: smallest layers first, against what is left beside everything else
+  for (int l = 1; l < nw; ++l)
+    rl[l].woff = 0;
+  fit_tasks();
+  size_t o = others();
+  for (int l = 1; l < nw; ++l)
+    rl[l].woff = -1;
+  fit_tasks();
+  o = std::max(o, others());
+  if (o > kSmemLimit)
+    return 1;
+  const size_t left = (kSmemLimit - o) / sizeof(float);
+  size_t used = 0;
+  std::vector<int> order;
+  for (int l = 1; l < nw; ++l)
+    order.push_back(l);
+  std::sort(order.begin(), order.end(), [&](int a, int b)
+            { return (size_t)rl[a].N * rl[a].ldw < (size_t)rl[b].N * rl[b].ldw; });
+  for (int l : order)
+  {
+    const size_t f = (size_t)rl[l].N * rl[l].ldw;
+    if (used + f <= left)
+      rl[l].woff = (int)used, used += f;
+  }
+  fit_tasks();
+  o = others() + used * sizeof(float);
+  if (o > kSmemLimit)
+    return 1;
+  std::vector<ResQuad> quads(S / 4);
+  for (int l = 0; l < nw; ++l)
+    for (int c = 0; c < rl[l].N; c += 4)
+    {
+      ResQuad& q = quads[(rl[l].noff + c) / 4];
+      q = ResQuad{};
+      q.layer = (short)(l + 1), q.col = c, q.valid = (short)std::min(4, rl[l].N - c);
+      q.pitch = up4(rl[l].N);
+      q.fpart = rl[l].fpart + c;
+      q.fslices = l > 0 ? (short)((rl[l].K + rl[l].fslice - 1) / rl[l].fslice) : 0;
+      if (l + 1 < nw)
+      {
+        const ResLayer& U = rl[l + 1];
+        q.bpart = U.bpart + c;
+        q.bslices = (short)((U.N + U.bslice - 1) / U.bslice);
+      }
+    }
+  std::vector<unsigned char> host(table_bytes(), 0);
+  size_t at = 0;
+  auto put = [&](const void* src, size_t len)
+  {
+    const size_t here = at;
+    if (len)
+      memcpy(host.data() + at, src, len);
+    at += round16(len);
+    return (int)here;
+  };
+  auto* st = new ResState();
+  ResParams& P = st->P;
+  put(rl.data(), sizeof(ResLayer) * nw);
+  P.a_quad = put(quads.data(), sizeof(ResQuad) * quads.size());
+  P.a_ft = put(ft.data(), sizeof(int) * ft.size());
+  P.a_bt = put(bt.data(), sizeof(int) * bt.size());
+  P.table_vecs = (int)(at / 16);
+  if (cudaMalloc(&st->dev, host.size()) != cudaSuccess ||
+      cudaMemcpy(st->dev, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+  {
+    cudaFree(st->dev);
+    delete st;
+    return cuda_fail(cudaGetLastError(), "row-resident plan tables");
+  }
+  P.table = static_cast<const int4*>(st->dev);
+  P.layers = p->d;
+  P.top_n = rl[nw - 1].N;
+  P.n = p->n, P.batch = p->batch, P.S = S;
+  P.nf = (int)ft.size(), P.nb = (int)bt.size();
+  P.N1p = N1p, P.K0p = K0p, P.ks0 = ks0, P.kslice0 = kslice0;
+  P.wfloats = (int)((used + 3) & ~(size_t)3);
+  P.groups = (p->batch + R - 1) / R;
+  P.simple = (p->h[0].flags & DPC_LAYER_INPUT_ACT) ? 1 : 0;
+  P.has_v = has_v ? 1 : 0;
+  P.energy = p->energy;
+  st->R = R;
+  st->smem = o;
+  p->res = st;
+  return DPC_OK;
+}
+} // namespace
+
+void res_plan_free(dpc_plan* p)
+{
+  auto* s = static_cast<ResState*>(p->res);
+  if (!s)
+    return;
+  cudaFree(s->dev);
+  delete s;
+  p->res = nullptr;
+}
+
+// Which plans run here: by shape only.  Plans with tensor-core layers do not; the others do while
+// re-reading the weights once per pass and row group from L2 costs less than the launches it saves.
+int res_plan_init(dpc_plan* p)
+{
+  p->res = nullptr;
+  if (getenv("DPC_DISABLE_RESIDENT"))
+    return 1;
+  const int n = p->n, nw = n - 1;
+  if (n > kMaxLayers || p->run.count > 0 || tc_extra_layer(p, 0))
+    return 1;
+  size_t wbytes = 0;
+  int S = 0;
+  bool has_v = false;
+  for (int l = 0; l < nw; ++l)
+  {
+    const dpc_layer& L = p->h[l];
+    if (L.next_size <= 0 || L.next_size > 8192 || (l > 0 && L.size > 16384) ||
+        ((L.flags ^ p->h[0].flags) & DPC_LAYER_INPUT_ACT) || (l == 0 && (L.flags & DPC_LAYER_RESIDUAL)))
+      return 1;
+    if (l > 0)
+      wbytes += sizeof(float) * (size_t)L.size * L.next_size;
+    has_v |= L.v != nullptr && l > 0;
+    S += up4(L.next_size);
+    if ((L.flags & DPC_LAYER_SOFTMAX_CE) || (l > 0 && tc_extra_layer(p, l)))
+      return 1;
+  }
+  static const size_t max_stream =
+      getenv("DPC_RESIDENT_MAX_BYTES") ? (size_t)atoll(getenv("DPC_RESIDENT_MAX_BYTES")) : 640 * 1024;
+  const size_t w0 = sizeof(float) * (size_t)p->h[0].size * p->h[0].next_size;
+  if (wbytes > max_stream || w0 > 4 * max_stream)
+    return 1;
+  int R = 1;
+  while (R < 8 && (p->batch + R - 1) / R > p->ctx->sm_count)
+    R *= 2;
+  for (; R >= 1; R /= 2)
+  {
+    const int rc = build(p, R, S, has_v);
+    if (rc <= 0)
+      return rc;
+  }
+  return 1;
+}
+
+template <int R>
+static int launch(dpc_plan* p, const ResState* st, const ResParams& P)
+{
+  static thread_local int configured = -1;
+  if (configured != p->ctx->device)
+  {
+    DPC_CUDA(cudaFuncSetAttribute(resident_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(kSmemLimit - kStatic)));
+    configured = p->ctx->device;
+  }
+  const int grid = std::min(P.groups, p->ctx->sm_count);
+  resident_kernel<R><<<grid, kThreads, st->smem - kStatic, p->ctx->stream>>>(P);
+  p->ctx->launches += 1;
+  const cudaError_t err = cudaPeekAtLastError();
+  return err == cudaSuccess ? DPC_OK : cuda_fail(cudaGetLastError(), "row-resident kernel");
+}
+} // namespace dpc
+
+using namespace dpc;
+
+int dpc_rows_available(dpc_plan* p)
+{
+  return p && p->res ? 1 : 0;
+}
+
+int dpc_rows_segment(dpc_plan* p, int ops, int steps, int top_clamped, int top_down_off)
+{
+  if (!p || !p->res || steps < 0)
+    return fail(DPC_ERR_INVALID, "dpc_rows_segment: not a row-resident plan, or a bad step count");
+  const auto* st = static_cast<const ResState*>(p->res);
+  ResParams P = st->P;
+  P.ops = ops, P.steps = steps;
+  P.top_clamped = top_clamped, P.top_down_off = top_down_off;
+  P.ce = (p->h[p->n - 1].flags & DPC_LAYER_SOFTMAX_CE) ? 1 : 0;
+  switch (st->R)
+  {
+  case 1:
+    return launch<1>(p, st, P);
+  case 2:
+    return launch<2>(p, st, P);
+  case 4:
+    return launch<4>(p, st, P);
+  default:
+    return launch<8>(p, st, P);
+  }
+}

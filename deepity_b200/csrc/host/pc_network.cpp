@@ -437,7 +437,7 @@ void PCNetwork::RandomizeWeights(std::mt19937& rng, const char* distribution)
 }
 
 // ------------------------------------------------------------------------------- state
-void PCNetwork::ResetState(bool beliefsOverwritten)
+void PCNetwork::ResetState(bool beliefsOverwritten, bool settleOverwritten)
 {
   RequireCompiled();
   const size_t B = (size_t)batchSize;
@@ -453,7 +453,7 @@ void PCNetwork::ResetState(bool beliefsOverwritten)
     Check(dpc_zero(ctx, z0, (size_t)(zend - z0) * sizeof(float)));
     Check(dpc_plan_invalidate(plan, 0, (int)layers.size(), DPC_WROTE_Z));
   }
-  if (kind == NetworkKind::FULL) // FullPCLayer::ResetState, src/layers/FullPCLayer.cpp:664-671
+  if (kind == NetworkKind::FULL && !settleOverwritten) // FullPCLayer::ResetState, src/layers/FullPCLayer.cpp:664-671
   {
     float* e0 = layers.front()->d.e;
     float* eend = layers.back()->d.e + Pad64(B * layers.back()->d.size);
@@ -751,9 +751,109 @@ void PCNetwork::RefreshPredictions()
   Check(dpc_sync(ctx));
 }
 
+// Whether the step's row-local stretches run as row segments (one launch each): a small network
+// without the features whose phases interleave rows (gradient staging, ePC sweeps, a ghost layer).
+bool PCNetwork::UseRowSegments()
+{
+  return !useEPC && !ghostTop && !gradSync && dpc_rows_available(plan);
+}
+
+// One row segment; what it stores follows from what it computes.
+void PCNetwork::RowSegment(int ops, int steps)
+{
+  const bool ce = layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE;
+  const bool clamped = layers.back()->clamped;
+  if ((ops & DPC_ROWS_REFRESH) && steps == 0)
+    ops |= DPC_ROWS_LOAD_E;
+  if (ops & DPC_ROWS_FIRST)
+    layers[0]->cacheValid = true;
+  if (steps > 0 || (ops & DPC_ROWS_ENERGY_LAST))
+    ops |= DPC_ROWS_STORE_E;
+  if (steps > 0 || (ops & (DPC_ROWS_SWEEP | DPC_ROWS_LOGITS | DPC_ROWS_ZERO_Z)))
+    ops |= DPC_ROWS_STORE_Z;
+  if (steps > 0 && useMomentum)
+    ops |= DPC_ROWS_STORE_V;
+  if (kind != NetworkKind::SIMPLE && (ops & (DPC_ROWS_REFRESH | DPC_ROWS_GATE_LAST)))
+    ops |= DPC_ROWS_STORE_G;
+  Check(dpc_rows_segment(plan, ops, steps, clamped ? 1 : 0,
+                         kind == NetworkKind::FULL && ce && !clamped ? 1 : 0));
+}
+
+void PCNetwork::RunTrainSegments(int mode, int steps)
+{
+  const bool ce = layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE;
+  const int n = (int)layers.size();
+  auto learn = [&] { Check(dpc_update_weights(plan, 0, n - 1, centerWeights ? 1 : 0)); };
+  if (kind == NetworkKind::DIRECT_KP)
+  {
+    bool fromOutput = true;
+    for (int i = 0; i + 1 < n && fromOutput; ++i)
+    {
+      const int a = layers[i]->d.act;
+      fromOutput = a == DPC_ACT_TANH || a == DPC_ACT_SIGMOID || a == DPC_ACT_RELU ||
+                   a == DPC_ACT_LINEAR || a == DPC_ACT_HARD_TANH;
+    }
+    RowSegment(DPC_ROWS_FIRST | DPC_ROWS_SWEEP | DPC_ROWS_TERMINAL |
+                   (fromOutput ? 0 : DPC_ROWS_SWEEP_PRED), 0);
+    Check(dpc_direct_feedback(plan, 0, n - 1, fromOutput ? DPC_DFA_FROM_OUTPUT : 0));
+    RowSegment(DPC_ROWS_REFRESH, steps);
+    learn();
+    Check(dpc_energy_reset(plan));
+    RowSegment(DPC_ROWS_ENERGY_LAST | (ce ? DPC_ROWS_GATE_LAST | DPC_ROWS_PRED_CLOSE : 0), 0);
+  }
+  else if (kind == NetworkKind::FULL)
+  {
+    const int open = DPC_ROWS_FIRST | DPC_ROWS_SWEEP | DPC_ROWS_TERMINAL | DPC_ROWS_ZERO_V;
+    if (useIPC)
+    {
+      // a weight update after every settling step; it also retires the input layer's prediction
+      for (int t = 0; t < steps; ++t)
+      {
+        RowSegment((t ? DPC_ROWS_FIRST : open) | DPC_ROWS_REFRESH, 1);
+        learn();
+      }
+      RowSegment((steps ? DPC_ROWS_FIRST : open) | DPC_ROWS_PREACT, 0);
+    }
+    else
+      RowSegment(open | DPC_ROWS_PREACT, steps);
+    Check(dpc_direct_feedback(plan, 0, n - 1, DPC_DFA_DECAY_W));
+    if (!useIPC)
+    {
+      RowSegment(DPC_ROWS_REFRESH, 0);
+      learn();
+    }
+    Check(dpc_energy_reset(plan));
+    RowSegment(DPC_ROWS_ENERGY_LAST | (ce ? DPC_ROWS_GATE_LAST | DPC_ROWS_PRED_CLOSE : 0), 0);
+  }
+  else if (mode == 0)
+  {
+    Check(dpc_energy_reset(plan));
+    RowSegment(DPC_ROWS_FIRST | DPC_ROWS_ZERO_Z | DPC_ROWS_ENERGY_LAST | DPC_ROWS_PRED_CLOSE, steps);
+    learn();
+  }
+  else if (mode == 1)
+  {
+    RowSegment(DPC_ROWS_FIRST | DPC_ROWS_SWEEP, steps);
+    learn();
+    Check(dpc_energy_reset(plan));
+    RowSegment(DPC_ROWS_ENERGY_LAST | DPC_ROWS_PRED_CLOSE, 0);
+  }
+  else
+  {
+    Check(dpc_energy_reset(plan));
+    RowSegment(DPC_ROWS_FIRST | DPC_ROWS_ZERO_Z | DPC_ROWS_ENERGY_EACH | DPC_ROWS_PRED_LAST, steps);
+    learn();
+  }
+}
+
 void PCNetwork::RunTrainPhases(int mode, int steps)
 {
   const int n = (int)layers.size();
+  if (UseRowSegments())
+  {
+    RunTrainSegments(mode, steps);
+    return;
+  }
   TransientScope scope(transientFlag, kind != NetworkKind::SIMPLE &&
                                           !(layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE));
   auto settle = [&](bool energy)
@@ -849,10 +949,12 @@ float PCNetwork::TrainStepRaw(int mode, const float* x, size_t nx, const float* 
   predictionsStale = false; // everything is recomputed from here on
   // DirectKP / Full steps open with the forward sweep over the whole stack; x and y must then
   // cover their layers completely (a short buffer leaves the rest at zero, as the memset would)
-  const bool sweepOverwrites = kind != NetworkKind::SIMPLE &&
+  // (a row segment starts from zero beliefs, errors and momentum by itself)
+  const bool segments = UseRowSegments();
+  const bool sweepOverwrites = (kind != NetworkKind::SIMPLE || segments) &&
                                nx >= (size_t)batchSize * layers.front()->d.size &&
                                ny >= (size_t)batchSize * layers.back()->d.size;
-  ResetState(sweepOverwrites);
+  ResetState(sweepOverwrites, segments && steps > 0);
   if (onDevice)
   {
     ClampDevice(0, x, nx);
@@ -920,6 +1022,15 @@ float PCNetwork::TrainStep(const std::vector<float>& x, const std::vector<float>
 void PCNetwork::RunPredictPhases(int steps, bool withProjection)
 {
   const int n = (int)layers.size();
+  if (UseRowSegments())
+  {
+    const bool logits =
+        kind == NetworkKind::FULL && (layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE);
+    RowSegment(DPC_ROWS_FIRST | (withProjection ? DPC_ROWS_SWEEP : DPC_ROWS_ZERO_Z) |
+                   DPC_ROWS_ZERO_V | (steps ? DPC_ROWS_PRED_LAST : DPC_ROWS_SWEEP_PRED) |
+                   (logits ? DPC_ROWS_LOGITS : 0), steps);
+    return;
+  }
   if (withProjection)
     ProjectForward();
   for (int t = 0; t < steps; ++t)
@@ -952,8 +1063,10 @@ void PCNetwork::PredictRaw(const float* x, size_t nx, int steps, bool withProjec
   if (kind != NetworkKind::SIMPLE)
     withProjection = true;
   predictionsStale = false;
-  ResetState(withProjection && kind != NetworkKind::SIMPLE &&
-             nx >= (size_t)batchSize * layers.front()->d.size);
+  const bool segments = UseRowSegments();
+  ResetState(((withProjection && kind != NetworkKind::SIMPLE) || segments) &&
+                 nx >= (size_t)batchSize * layers.front()->d.size,
+             segments && steps > 0);
   ClampHost(0, x, nx);
   for (int i = 1; i < n; ++i)
     layers[i]->clamped = false;

@@ -111,7 +111,9 @@ public:
   void Compile();
   void RandomizeWeights(std::mt19937& rng, const char* distribution = "normal");
 
-  void ResetState(bool beliefsOverwritten = false);
+  // beliefsOverwritten / settleOverwritten: the coming step overwrites all beliefs (errors and state
+  // momentum) before it reads one, so clearing them is skipped.
+  void ResetState(bool beliefsOverwritten = false, bool settleOverwritten = false);
   void Clamp(const std::vector<float>& input);
   void ClampHost(int layer, const float* data, size_t n);
   void ClampDevice(int layer, const float* data, size_t n);
@@ -211,6 +213,9 @@ private:
   void RefreshPredictions();
   void SyncGradients(size_t count);
   void ForwardRange(int first, int count, int flags);
+  bool UseRowSegments();
+  void RowSegment(int ops, int steps);
+  void RunTrainSegments(int mode, int steps);
   void RunTrainPhases(int mode, int steps);
   void RunPredictPhases(int steps, bool withProjection);
 

@@ -39,6 +39,7 @@
  *   DPC_DISABLE_LAYER_STREAMS  consecutive such layers of one phase are launched one after the other
  *                              on the context's stream instead of side by side on internal streams
  *                              that fork from it and join it again
+ *   DPC_DISABLE_RESIDENT       small networks run phase by phase instead of in row segments
  */
 #ifndef DEEPITY_B200_H
 #define DEEPITY_B200_H
@@ -349,6 +350,39 @@ DPC_API int dpc_apply_gradients(dpc_plan* plan, int first, int count, int which,
  * race, so order them on one stream or with events. */
 DPC_API int dpc_error_energy_static(void* stream, const float* z_dev, const float* mu_dev,
                                     float* e_dev, int64_t count, float* energy_dev);
+/* Row segments.  Between two weight updates a step is row-local: a plan whose weights are small
+ * enough (dpc_rows_available) runs everything from one update to the next -- sweep, settling steps,
+ * refresh, energy -- in ONE launch in which a thread block keeps a few batch rows' state on the chip.
+ * ops: bit set of DPC_ROWS_*, executed in this order; steps: settling steps (CalculateState +
+ * UpdateState, FullPCNetwork.cpp / DirectKPPCNetwork.cpp / SimplePCNetwork.cpp) between the sweep
+ * and the closing pass.  top_clamped: the last layer's belief is a clamped target; top_down_off:
+ * FullPC's rule under an unclamped cross-entropy head (FullPCLayer.cpp:318-324). */
+enum
+{
+  DPC_ROWS_FIRST = 1 << 0,       /* the clamped input layer's prediction is computed (and stored), not
+                                    taken from mu / preact of an earlier segment of the step        */
+  DPC_ROWS_SWEEP = 1 << 1,       /* forward sweep, z[l+1] = mu[l]                                    */
+  DPC_ROWS_SWEEP_PRED = 1 << 2,  /* the sweep stores mu and preact of every layer                    */
+  DPC_ROWS_TERMINAL = 1 << 3,    /* terminal error after the sweep                                   */
+  DPC_ROWS_ZERO_Z = 1 << 4,      /* beliefs start at zero instead of what memory holds               */
+  DPC_ROWS_ZERO_V = 1 << 5,      /* state momentum starts at zero                                    */
+  DPC_ROWS_LOAD_E = 1 << 6,      /* errors are read (a refresh without a settling step before it)    */
+  DPC_ROWS_ENERGY_EACH = 1 << 7, /* every settling step adds its energy                              */
+  DPC_ROWS_PRED_LAST = 1 << 8,   /* the last settling step stores mu and preact                      */
+  DPC_ROWS_REFRESH = 1 << 9,     /* gated errors from the settled beliefs and the stored errors      */
+  DPC_ROWS_PREACT = 1 << 10,     /* mu and preact from the settled beliefs                           */
+  DPC_ROWS_ENERGY_LAST = 1 << 11, /* closing pass: errors and energy                                 */
+  DPC_ROWS_GATE_LAST = 1 << 12,  /* ... and gated errors                                             */
+  DPC_ROWS_PRED_CLOSE = 1 << 13, /* the closing pass stores mu and preact                            */
+  DPC_ROWS_LOGITS = 1 << 14,     /* the last layer's belief becomes the prediction below it          */
+  DPC_ROWS_STORE_Z = 1 << 15,
+  DPC_ROWS_STORE_E = 1 << 16,
+  DPC_ROWS_STORE_G = 1 << 17,    /* fe */
+  DPC_ROWS_STORE_V = 1 << 18
+};
+DPC_API int dpc_rows_available(dpc_plan* plan);
+DPC_API int dpc_rows_segment(dpc_plan* plan, int ops, int steps, int top_clamped,
+                             int top_down_off);
 /* Energy accumulator of the plan (device-resident double). */
 DPC_API int dpc_energy_reset(dpc_plan* plan);
 DPC_API int dpc_energy_read(dpc_plan* plan, double* out); /* synchronous */
