@@ -55,14 +55,29 @@ struct __align__(16) ResQuad
   short fslices, bslices; // slices of the prediction from below / of the feedback from above
   short layer, valid;     // layer 1 .. n-1; columns that exist (the rest is padding)
   int col, pitch;         // first column inside the layer, padded width of the layer
-  int pad[2];
+  int down, up;           // state offsets of the same columns in the layer below / above (residuals)
+};
+
+// One warp task, everything its lanes need in two 16-byte reads.  Offsets in floats.
+struct __align__(16) ResTask
+{
+  int w, ldw;     // first weight and row pitch: in the resident weights, or in the layer's W
+  int x, len;     // first operand element of the first row; K (forward) or output rows (state) to walk
+  int out, pitch; // first partial sum of the first row, distance to the next row's
+  int lanes;      // lanes (resident forward: outputs, state: column groups) that exist
+  int kind;       // layer << 4 | T_*
+};
+enum
+{
+  T_STREAM = 1, // weights in global memory
+  T_VEC = 2     // forward: rows readable 16 bytes at a time; state: 4 columns per lane
 };
 
 struct ResParams
 {
   const dpc_layer* layers;
   // one table in global memory, copied to shared memory as it is:
-  //   ResLayer[nw] | ResQuad[S / 4] | forward tasks | state tasks, packed by pack()
+  //   ResLayer[nw] | ResQuad[S / 4] | forward tasks (sorted by layer) | state tasks
   const int4* table;
   int table_vecs, a_quad, a_ft, a_bt; // its size in 16-byte units, byte offsets of the parts
   int n, batch, S;                    // layers, rows, floats of one row's state (layers 1..n-1)
@@ -75,12 +90,6 @@ struct ResParams
   int simple, has_v, ce, top_clamped, top_down_off, top_n;
   double* energy;
 };
-
-// layer (7 bits) | row block (2) | slice (5) | output or column block (11)
-__host__ __device__ __forceinline__ int pack(int l, int rb, int s, int blk)
-{
-  return l << 18 | rb << 16 | s << 11 | blk;
-}
 
 template <int R>
 constexpr int kRowsPerTask = R >= 4 ? 4 : R;
@@ -162,17 +171,17 @@ __device__ __forceinline__ void dot_streamed(float (&acc)[R * G], const float* _
     }
 }
 
-// Resident weights: this lane's output over k in [k0, k1) (slices of multiples of 4, zero-padded).
+// Resident weights: this lane's output over `len` inputs (walked four at a time, zero-padded).
 template <int RT>
-__device__ __forceinline__ void dot_resident(const float* w, const float* x, int S, int k0, int k1,
-                                             float* out, int pitch, bool valid)
+__device__ __forceinline__ void dot_resident(const float* w, const float* x, int S, int len, float* out,
+                                             int pitch, bool valid)
 {
   float acc[RT];
 #pragma unroll
   for (int r = 0; r < RT; ++r)
     acc[r] = 0.0f;
 #pragma unroll 4
-  for (int k = k0; k < k1; k += 4)
+  for (int k = 0; k < len; k += 4)
   {
     const float4 wv = *reinterpret_cast<const float4*>(w + k);
 #pragma unroll
@@ -191,9 +200,9 @@ __device__ __forceinline__ void dot_resident(const float* w, const float* x, int
       out[r * pitch] = acc[r];
 }
 
-// One state task: sums over W rows [n0, n1) (n0 a multiple of 4) for this lane's KW columns.
+// One state task: sums over `len` rows of W for this lane's KW columns.
 template <int RT, int KW>
-__device__ __forceinline__ void state_task(const float* W, int ldw, int n0, int n1, const float* g, int S,
+__device__ __forceinline__ void state_task(const float* w, int ldw, int len, const float* g, int S,
                                            float* out, int pitch)
 {
   float acc[RT][KW];
@@ -202,9 +211,9 @@ __device__ __forceinline__ void state_task(const float* W, int ldw, int n0, int 
 #pragma unroll
     for (int c = 0; c < KW; ++c)
       acc[r][c] = 0.0f;
-  const float* w = W + (size_t)n0 * ldw;
-  int n = n0;
-  for (; n + 4 <= n1; n += 4, w += 4 * (size_t)ldw)
+  int n = 0;
+#pragma unroll 2
+  for (; n + 4 <= len; n += 4, w += 4 * (size_t)ldw)
   {
     float wv[4][KW];
 #pragma unroll
@@ -232,7 +241,7 @@ __device__ __forceinline__ void state_task(const float* W, int ldw, int n0, int 
       }
     }
   }
-  for (; n < n1; ++n, w += ldw)
+  for (; n < len; ++n, w += ldw)
 #pragma unroll
     for (int c = 0; c < KW; ++c)
     {
@@ -254,6 +263,68 @@ __device__ __forceinline__ void cp_async16(float* dst, const float* src)
                    (uint32_t)__cvta_generic_to_shared(dst)),
                "l"(src)
                : "memory");
+}
+
+__device__ __forceinline__ void get4(float (&v)[4], const float* p)
+{
+  const float4 t = *reinterpret_cast<const float4*>(p);
+  v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
+}
+__device__ __forceinline__ void put4(float* p, const float (&v)[4])
+{
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+// Sum of `slices` partial sums, four neighbours at once, in slice order.
+__device__ __forceinline__ void sum4(float (&v)[4], const float* p, int slices, int stride)
+{
+  get4(v, p);
+#pragma unroll 3
+  for (int s = 1; s < slices; ++s)
+  {
+    float t[4];
+    get4(t, p + s * stride);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      v[j] += t[j];
+  }
+}
+// Activation and derivative of four values with one dispatch.
+__device__ __forceinline__ void act4(int act, const float (&z)[4], float (&f)[4], float (&d)[4])
+{
+#define DPC_ACT4(A)                                                                               \
+  case A:                                                                                         \
+    _Pragma("unroll") for (int j = 0; j < 4; ++j) act_both(A, z[j], f[j], d[j]);                  \
+    break;
+  switch (act)
+  {
+    DPC_ACT4(DPC_ACT_RELU)
+    DPC_ACT4(DPC_ACT_GELU)
+    DPC_ACT4(DPC_ACT_SIGMOID)
+    DPC_ACT4(DPC_ACT_ESIGMOID)
+    DPC_ACT4(DPC_ACT_TANH)
+    DPC_ACT4(DPC_ACT_HARD_TANH)
+  default:
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      f[j] = z[j], d[j] = 1.0f;
+  }
+#undef DPC_ACT4
+}
+// f'(z) of four values whose f(z) is known.
+__device__ __forceinline__ void deriv4(int act, const float (&z)[4], const float (&f)[4], float (&d)[4])
+{
+  if (act_has_output_deriv(act))
+  {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      d[j] = act_deriv_from_output(act, f[j]);
+  }
+  else
+  {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      d[j] = act_deriv(act, z[j]);
+  }
 }
 
 struct LayerConst // what a finished sum of layer l needs, one 16-byte read
@@ -280,8 +351,8 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
   unsigned char* tab = reinterpret_cast<unsigned char*>(Ws + P.wfloats);
   const ResLayer* sl = reinterpret_cast<const ResLayer*>(tab);
   const ResQuad* quad = reinterpret_cast<const ResQuad*>(tab + P.a_quad);
-  const int* ftab = reinterpret_cast<const int*>(tab + P.a_ft);
-  const int* btab = reinterpret_cast<const int*>(tab + P.a_bt);
+  const ResTask* ftab = reinterpret_cast<const ResTask*>(tab + P.a_ft);
+  const ResTask* btab = reinterpret_cast<const ResTask*>(tab + P.a_bt);
   float* bias = reinterpret_cast<float*>(tab + 16 * (size_t)P.table_vecs);
   float* Z = bias + S;
   float* E = Z + R * S;
@@ -293,9 +364,6 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
   const int NT = P.top_n, NTp = (NT + 3) & ~3;
   float* topd = topmu + R * NTp;
   float* X = topd + R * NTp; // input rows; later the partial sums of the tasks
-
-  // elementwise passes over the R x S state: `ew` threads along a row, kThreads / ew rows at a time
-  const int ew = min(kThreads, (S + 31) & ~31), ex = tid % ew, ey = tid / ew, er = kThreads / ew;
 
   for (int i = tid; i < P.table_vecs; i += kThreads)
     reinterpret_cast<int4*>(tab)[i] = __ldg(P.table + i);
@@ -322,12 +390,34 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
           dst[r * L.ldw + c] = c < L.K ? src[(size_t)r * L.K + c] : 0.0f;
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
+  // Elementwise passes: a thread takes four neighbouring elements of a row at a time (most networks:
+  // one quad per thread, whose table entry then stays in registers).
+  const int S4 = S >> 2, nq = R * S4;
+  const int own_r = tid / S4, own_i = tid - own_r * S4;
+  const ResQuad own = quad[own_i];
+  auto for_quads = [&](auto&& f)
+  {
+    if (tid >= nq)
+      return;
+    int i = own_i, r = own_r;
+    ResQuad q = own;
+    for (int idx = tid;;)
+    {
+      f(q, i, r);
+      idx += kThreads;
+      if (idx >= nq)
+        break;
+      r = idx / S4, i = idx - r * S4;
+      q = quad[i];
+    }
+  };
   for (int i = tid; i < S; i += kThreads)
   {
     const ResQuad q = quad[i >> 2];
     bias[i] = (i & 3) < q.valid ? P.layers[q.layer - 1].b[q.col + (i & 3)] : 0.0f;
   }
 
+  const ResTask own_f = ftab[min(warp, max(P.nf - 1, 0))], own_b = btab[min(warp, max(P.nb - 1, 0))];
   const bool first = P.ops & DPC_ROWS_FIRST;
   double esum = 0.0;
 
@@ -338,30 +428,33 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
     __syncthreads();
 
     // ---------------------------------------------------------------- beliefs
-    if (ey < er)
-      for (int r = ey; r < R; r += er)
-        for (int i = ex; i < S; i += ew)
-        {
-          const ResQuad q = quad[i >> 2];
-          const int l = q.layer, w = sl[l - 1].N;
-          const bool in = r < rows && (i & 3) < q.valid;
-          const dpc_layer& L = P.layers[l];
-          const size_t o = (size_t)(row0 + r) * w + q.col + (i & 3);
-          float z = 0.0f, e = 0.0f, v = 0.0f;
-          if (in && ((P.top_clamped && l == nw) || !(P.ops & (DPC_ROWS_SWEEP | DPC_ROWS_ZERO_Z))))
-            z = L.z[o];
-          if (in && (P.ops & DPC_ROWS_LOAD_E))
-            e = L.e[o];
-          if (P.has_v)
-          {
-            if (in && !(P.ops & DPC_ROWS_ZERO_V) && L.v)
-              v = L.v[o];
-            Vb[r * S + i] = v;
-          }
-          Z[r * S + i] = z;
-          E[r * S + i] = e;
-          Gb[r * S + i] = simple && l < nw ? act_fwd(lc[l].act, z) : 0.0f;
-        }
+    for_quads([&](const ResQuad& q, int i, int r)
+              {
+                const int l = q.layer;
+                const dpc_layer& L = P.layers[l];
+                const size_t o = (size_t)(row0 + r) * sl[l - 1].N + q.col;
+                const bool load_z =
+                    (P.top_clamped && l == nw) || !(P.ops & (DPC_ROWS_SWEEP | DPC_ROWS_ZERO_Z));
+                const bool load_v = P.has_v && !(P.ops & DPC_ROWS_ZERO_V) && L.v;
+                float z[4], e[4], v[4], f[4], d[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                {
+                  const bool in = r < rows && j < q.valid;
+                  z[j] = in && load_z ? L.z[o + j] : 0.0f;
+                  e[j] = in && (P.ops & DPC_ROWS_LOAD_E) ? L.e[o + j] : 0.0f;
+                  v[j] = in && load_v ? L.v[o + j] : 0.0f;
+                  f[j] = 0.0f;
+                }
+                if (simple && l < nw)
+                  act4(lc[l].act, z, f, d);
+                const int t = r * S + 4 * i;
+                put4(Z + t, z);
+                put4(E + t, e);
+                put4(Gb + t, f);
+                if (P.has_v)
+                  put4(Vb + t, v);
+              });
     // ---------------------------------------------------------------- the clamped input layer
     {
       const ResLayer L = sl[0];
@@ -435,62 +528,100 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
 
-    // One forward task: partial sums of 32 outputs x RT rows (resident) or G outputs x R rows.
-    auto forward_task = [&](int entry)
+    // One forward task: partial sums of up to 32 outputs x RT rows (resident) or G x R (streamed).
+    auto forward_task = [&](const ResTask& t)
     {
-      const int l = entry >> 18, rb = (entry >> 16) & 3, s = (entry >> 11) & 31, blk = entry & 2047;
-      const ResLayer& L = sl[l];
-      const float* x = (simple ? Gb : Z) + L.zoff;
-      const int pitch = (L.N + 3) & ~3;
-      float* out = X + L.fpart + s * (R * pitch);
-      if (L.woff >= 0)
+      const float* x = (simple ? Gb : Z) + t.x;
+      float* out = X + t.out;
+      if (!(t.kind & T_STREAM))
       {
-        const int c = blk * 32 + lane, k0 = s * L.fslice;
-        dot_resident<RT>(Ws + L.woff + min(c, L.N - 1) * L.ldw, x + rb * RT * S, S, k0,
-                         min(L.K, k0 + L.fslice), out + rb * RT * pitch + c, pitch, c < L.N);
+        dot_resident<RT>(Ws + t.w + min(lane, t.lanes - 1) * t.ldw, x, S, t.len, out + lane, t.pitch,
+                         lane < t.lanes);
         return;
       }
       float acc[V];
 #pragma unroll
       for (int i = 0; i < V; ++i)
         acc[i] = 0.0f;
-      const int g0 = blk * G;
-      dot_streamed<R, G>(acc, sW[l] + (size_t)g0 * L.K, L.K, L.N - g0, x, S, 0, L.K, lane, L.vec != 0);
+      dot_streamed<R, G>(acc, sW[t.kind >> 4] + t.w, t.ldw, t.lanes, x, S, 0, t.len, lane,
+                         (t.kind & T_VEC) != 0);
       const float v = reduce_values<V>(acc, lane);
-      const int idx = lane / LPV, r = idx / G, c = g0 + idx % G;
-      if (lane % LPV == 0 && c < L.N)
-        out[r * pitch + c] = v;
+      const int idx = lane / LPV, r = idx / G, c = idx % G;
+      if (lane % LPV == 0 && c < t.lanes)
+        out[r * t.pitch + c] = v;
     };
-    // The finished sum of state element i (of quad q) of row r: pre-activation of the layer below.
-    auto pre_of = [&](const ResQuad& q, int r, int i, int l)
+    auto state_of = [&](const ResTask& t)
     {
-      const float* p = X + q.fpart + r * q.pitch + (i & 3);
-      float v = 0.0f;
-#pragma unroll 4
-      for (int s = 0; s < q.fslices; ++s)
-        v += p[s * (R * q.pitch)];
-      return lc[l].a * v + bias[i];
-    };
-    auto store_pred = [&](int l, int r, int c, float pre, float mu)
-    {
-      if (r < rows)
+      const float* g = (simple ? E : Gb) + t.x;
+      if (lane >= t.lanes)
+        return;
+      const int k = (t.kind & T_VEC) ? lane * 4 : lane;
+      float* out = X + t.out + k;
+      if (!(t.kind & T_STREAM))
       {
-        const dpc_layer& D = P.layers[l];
-        const size_t o = (size_t)(row0 + r) * sl[l].N + c;
-        D.mu[o] = mu;
-        if (D.preact)
-          D.preact[o] = pre;
+        if (t.kind & T_VEC)
+          state_task<RT, 4>(Ws + t.w + k, t.ldw, t.len, g, S, out, t.pitch);
+        else
+          state_task<RT, 1>(Ws + t.w + k, t.ldw, t.len, g, S, out, t.pitch);
       }
+      else if (t.kind & T_VEC)
+        state_task<RT, 4>(sW[t.kind >> 4] + t.w + k, t.ldw, t.len, g, S, out, t.pitch);
+      else
+        state_task<RT, 1>(sW[t.kind >> 4] + t.w + k, t.ldw, t.len, g, S, out, t.pitch);
     };
-    auto predict = [&](int l, int r, int c, float pre, float& mu, float& d)
+    // Prediction of the four elements of quad q (layer l + 1) in row r, from the partial sums or the
+    // clamped input layer's cache; padding comes out as zero.
+    auto predict = [&](const ResQuad& q, int i4, int r, bool pred, float (&mu)[4], float (&d)[4])
     {
-      mu = pre, d = 1.0f;
-      if (!simple)
+      const int l = q.layer - 1;
+      if (l == 0)
       {
-        act_both(lc[l].act, pre, mu, d);
-        if (lc[l].residual)
-          mu += Z[r * S + sl[l].zoff + c];
+        get4(mu, mu0 + r * P.N1p + q.col);
+        get4(d, d0 + r * P.N1p + q.col);
       }
+      else
+      {
+        float pre[4], b[4];
+        sum4(pre, X + q.fpart + r * q.pitch, q.fslices, R * q.pitch);
+        get4(b, bias + 4 * i4);
+        const LayerConst C = lc[l];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          pre[j] = C.a * pre[j] + b[j];
+        if (simple)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            mu[j] = pre[j], d[j] = 1.0f;
+        else
+        {
+          act4(C.act, pre, mu, d);
+          if (C.residual)
+          {
+            float z[4];
+            get4(z, Z + r * S + q.down);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              mu[j] += z[j];
+          }
+        }
+        if (pred && r < rows)
+        {
+          const dpc_layer& D = P.layers[l];
+          const size_t o = (size_t)(row0 + r) * sl[l].N + q.col;
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (j < q.valid)
+            {
+              D.mu[o + j] = mu[j];
+              if (D.preact)
+                D.preact[o + j] = pre[j];
+            }
+        }
+      }
+#pragma unroll
+      for (int j = 1; j < 4; ++j)
+        if (j >= q.valid)
+          mu[j] = d[j] = 0.0f;
     };
     // softmax cross-entropy error of the top layer from its logits (one warp per row)
     auto ce_error = [&](bool energy)
@@ -536,7 +667,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
         if (l > 0)
         {
           int t = f;
-          while (t < P.nf && (ftab[t] >> 18) == l)
+          while (t < P.nf && (ftab[t].kind >> 4) == l)
             ++t;
           for (int q = f + warp; q < t; q += kWarps)
             forward_task(ftab[q]);
@@ -544,27 +675,28 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
           __syncthreads();
         }
         const bool copy = !(l + 1 == nw && P.top_clamped);
-        for (int i = tid; i < R * L.N; i += kThreads)
+        const int n4 = (L.N + 3) >> 2;
+        for (int idx = tid; idx < R * n4; idx += kThreads)
         {
-          const int r = i / L.N, c = i - r * L.N, o = r * S + L.noff + c;
-          float mu, d;
-          if (l == 0)
-            mu = mu0[r * P.N1p + c], d = d0[r * P.N1p + c];
-          else
-          {
-            const float pre = pre_of(quad[(L.noff + c) >> 2], r, L.noff + c, l);
-            predict(l, r, c, pre, mu, d);
-            if (P.ops & DPC_ROWS_SWEEP_PRED)
-              store_pred(l, r, c, pre, mu);
-          }
+          const int r = idx / n4, i = (L.noff >> 2) + idx - r * n4, o = r * S + 4 * i;
+          const ResQuad q = quad[i];
+          float mu[4], d[4];
+          predict(q, i, r, (P.ops & DPC_ROWS_SWEEP_PRED) != 0, mu, d);
           if (copy)
           {
-            Z[o] = mu;
+            put4(Z + o, mu);
             if (simple && l + 1 < nw)
-              Gb[o] = act_fwd(lc[l + 1].act, mu);
+            {
+              float f4[4], d4[4];
+              act4(lc[l + 1].act, mu, f4, d4);
+              put4(Gb + o, f4);
+            }
           }
           if (l + 1 == nw) // the top prediction feeds the terminal error
-            topmu[r * NTp + c] = mu, topd[r * NTp + c] = d;
+          {
+            put4(topmu + r * NTp + q.col, mu);
+            put4(topd + r * NTp + q.col, d);
+          }
         }
         __syncthreads();
       }
@@ -589,42 +721,46 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
     // errors are refreshed from the errors that are there.
     auto forward = [&](bool err, bool gate, bool energy, bool pred)
     {
-      for (int t = warp; t < P.nf; t += kWarps)
+      if (warp < P.nf)
+        forward_task(own_f);
+      for (int t = warp + kWarps; t < P.nf; t += kWarps)
         forward_task(ftab[t]);
       __syncthreads();
       float local = 0.0f;
-      if (ey < er)
-        for (int r = ey; r < R; r += er)
-          for (int i = ex; i < S; i += ew)
-          {
-            const ResQuad q = quad[i >> 2];
-            if ((i & 3) >= q.valid)
-              continue;
-            const int l = q.layer - 1, c = q.col + (i & 3), o = r * S + i;
-            float mu, d;
-            if (l == 0)
-              mu = mu0[r * P.N1p + c], d = d0[r * P.N1p + c];
-            else
-            {
-              const float pre = pre_of(q, r, i, l);
-              predict(l, r, c, pre, mu, d);
-              if (pred)
-                store_pred(l, r, c, pre, mu);
-            }
-            const bool ce_top = P.ce && l == nw - 1;
-            if (ce_top)
-              topmu[r * NTp + c] = mu, topd[r * NTp + c] = d;
-            float e = E[o];
-            if (err && !ce_top)
-            {
-              e = Z[o] - mu;
-              E[o] = e;
-              if (r < rows)
-                local += e * e;
-            }
-            if (gate && !simple && !(err && ce_top))
-              Gb[o] = e * d;
-          }
+      for_quads([&](const ResQuad& q, int i, int r)
+                {
+                  const int o = r * S + 4 * i;
+                  float mu[4], d[4], e[4];
+                  predict(q, i, r, pred, mu, d);
+                  const bool ce_top = P.ce && q.layer == nw;
+                  if (ce_top)
+                  {
+                    put4(topmu + r * NTp + q.col, mu);
+                    put4(topd + r * NTp + q.col, d);
+                  }
+                  if (err && !ce_top)
+                  {
+                    float z[4];
+                    get4(z, Z + o);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                    {
+                      e[j] = z[j] - mu[j];
+                      if (r < rows)
+                        local += e[j] * e[j];
+                    }
+                    put4(E + o, e);
+                  }
+                  else
+                    get4(e, E + o);
+                  if (gate && !simple && !(err && ce_top))
+                  {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                      e[j] *= d[j];
+                    put4(Gb + o, e);
+                  }
+                });
       if (energy)
         esum += (double)local;
       __syncthreads();
@@ -638,74 +774,78 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
       const bool last = t + 1 == P.steps;
       forward(true, true, (P.ops & DPC_ROWS_ENERGY_EACH) != 0,
               last && (P.ops & DPC_ROWS_PRED_LAST) != 0);
-      const float* gate = simple ? E : Gb;
-      for (int q = warp; q < P.nb; q += kWarps)
-      {
-        const int entry = btab[q];
-        const int l = entry >> 18, rb = (entry >> 16) & 3, s = (entry >> 11) & 31, blk = entry & 2047;
-        const ResLayer& L = sl[l];
-        const int n0 = s * L.bslice, n1 = min(L.N, n0 + L.bslice), pitch = (L.K + 3) & ~3;
-        const float* g = gate + L.noff + rb * RT * S;
-        const int k = (blk * 32 + lane) * L.kw;
-        float* out = X + L.bpart + (s * R + rb * RT) * pitch + k;
-        if (k < L.K)
-        {
-          if (L.kw == 4 && L.woff >= 0)
-            state_task<RT, 4>(Ws + L.woff + k, L.ldw, n0, n1, g, S, out, pitch);
-          else if (L.kw == 4)
-            state_task<RT, 4>(sW[l] + k, L.K, n0, n1, g, S, out, pitch);
-          else if (L.woff >= 0)
-            state_task<RT, 1>(Ws + L.woff + k, L.ldw, n0, n1, g, S, out, pitch);
-          else
-            state_task<RT, 1>(sW[l] + k, L.K, n0, n1, g, S, out, pitch);
-        }
-      }
+      if (warp < P.nb)
+        state_of(own_b);
+      for (int t = warp + kWarps; t < P.nb; t += kWarps)
+        state_of(btab[t]);
       __syncthreads();
       const bool refresh_f = simple && !(last && !(P.ops & DPC_ROWS_ENERGY_LAST));
-      if (ey < er)
-        for (int r = ey; r < R; r += er)
-          for (int i = ex; i < S; i += ew)
-          {
-            const ResQuad q = quad[i >> 2];
-            const int l = q.layer, o = r * S + i;
-            if ((i & 3) >= q.valid || (l == nw && P.top_clamped))
-              continue;
-            const LayerConst C = lc[l];
-            float z = Z[o];
-            const float e = E[o];
-            if (l == nw || (P.top_down_off && l == nw - 1))
-            {
-              Z[o] = z - C.ir * e;
-              continue;
-            }
-            const float* pp = X + q.bpart + r * q.pitch + (i & 3);
-            float dz = 0.0f;
-#pragma unroll 4
-            for (int s = 0; s < q.bslices; ++s)
-              dz += pp[s * (R * q.pitch)];
-            if (simple)
-            {
-              z += C.ir * (dz * act_deriv(C.act, z) - e);
-              if (refresh_f)
-                Gb[o] = act_fwd(C.act, z);
-            }
-            else
-            {
-              const float fb = C.a * dz - e;
-              if (P.has_v)
-              {
-                const float beta = P.layers[l].momentum_beta;
-                const float v = beta * Vb[o] + (1.0f - beta) * fb;
-                Vb[o] = v;
-                z += C.ir * v;
-              }
-              else
-                z += C.ir * fb;
-              if (C.residual)
-                z += C.ir * E[r * S + sl[l].noff + q.col + (i & 3)];
-            }
-            Z[o] = z;
-          }
+      for_quads([&](const ResQuad& q, int i, int r)
+                {
+                  const int l = q.layer, o = r * S + 4 * i;
+                  if (l == nw && P.top_clamped)
+                    return;
+                  const LayerConst C = lc[l];
+                  float z[4], e[4];
+                  get4(z, Z + o);
+                  get4(e, E + o);
+                  if (l == nw || (P.top_down_off && l == nw - 1))
+                  {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                      z[j] -= C.ir * e[j];
+                    put4(Z + o, z);
+                    return;
+                  }
+                  float dz[4];
+                  sum4(dz, X + q.bpart + r * q.pitch, q.bslices, R * q.pitch);
+                  if (simple)
+                  {
+                    float f[4], d[4];
+                    get4(f, Gb + o);
+                    deriv4(C.act, z, f, d);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                      z[j] += C.ir * (dz[j] * d[j] - e[j]);
+                  }
+                  else
+                  {
+                    float fb[4], u[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                      fb[j] = C.a * dz[j] - e[j];
+                    if (P.has_v)
+                    {
+                      const float beta = P.layers[l].momentum_beta;
+                      float v[4];
+                      get4(v, Vb + o);
+#pragma unroll
+                      for (int j = 0; j < 4; ++j)
+                        fb[j] = beta * v[j] + (1.0f - beta) * fb[j];
+                      put4(Vb + o, fb);
+                    }
+                    if (C.residual)
+                      get4(u, E + r * S + q.up);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                    {
+                      z[j] += C.ir * fb[j];
+                      if (C.residual)
+                        z[j] += C.ir * u[j];
+                    }
+                  }
+#pragma unroll
+                  for (int j = 1; j < 4; ++j)
+                    if (j >= q.valid)
+                      z[j] = 0.0f;
+                  put4(Z + o, z);
+                  if (refresh_f)
+                  {
+                    float f[4], d[4];
+                    act4(C.act, z, f, d);
+                    put4(Gb + o, f);
+                  }
+                });
       __syncthreads();
     }
     // ---------------------------------------------------------------- closing pass
@@ -722,49 +862,49 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
       if (l > 0)
       {
         for (int t = warp; t < P.nf; t += kWarps)
-          if ((ftab[t] >> 18) == l)
+          if ((ftab[t].kind >> 4) == l)
             forward_task(ftab[t]);
         __syncthreads();
       }
-      for (int i = tid; i < R * NT; i += kThreads)
+      const int n4 = NTp >> 2;
+      for (int idx = tid; idx < R * n4; idx += kThreads)
       {
-        const int r = i / NT, c = i - r * NT, to = sl[l].noff;
-        float mu, d;
-        if (l == 0)
-          mu = mu0[r * P.N1p + c];
-        else
-        {
-          const float pre = pre_of(quad[(to + c) >> 2], r, to + c, l);
-          predict(l, r, c, pre, mu, d);
-          store_pred(l, r, c, pre, mu);
-        }
-        Z[r * S + to + c] = mu;
+        const int r = idx / n4, i = (sl[l].noff >> 2) + idx - r * n4;
+        float mu[4], d[4];
+        predict(quad[i], i, r, true, mu, d);
+        put4(Z + r * S + 4 * i, mu);
       }
       __syncthreads();
     }
 
     // ---------------------------------------------------------------- back to memory
-    if (ey < er)
-      for (int r = ey; r < rows; r += er)
-        for (int i = ex; i < S; i += ew)
-        {
-          const ResQuad q = quad[i >> 2];
-          if ((i & 3) >= q.valid)
-            continue;
-          const int l = q.layer, w = sl[l - 1].N, o = r * S + i;
-          const dpc_layer& L = P.layers[l];
-          const size_t m = (size_t)(row0 + r) * w + q.col + (i & 3);
-          if ((P.ops & DPC_ROWS_STORE_Z) && !(l == nw && P.top_clamped))
-            L.z[m] = Z[o];
-          if ((P.ops & DPC_ROWS_STORE_E) || ((P.ops & DPC_ROWS_TERMINAL) && l == nw))
-            L.e[m] = E[o];
-          if ((P.ops & DPC_ROWS_STORE_G) && !simple)
-            P.layers[l - 1].fe[m] = Gb[o];
-          if (simple && l < nw && (P.ops & DPC_ROWS_STORE_Z))
-            L.zF[m] = Gb[o];
-          if (P.has_v && (P.ops & DPC_ROWS_STORE_V) && L.v)
-            L.v[m] = Vb[o];
-        }
+    for_quads([&](const ResQuad& q, int i, int r)
+              {
+                if (r >= rows)
+                  return;
+                const int l = q.layer, o = r * S + 4 * i;
+                const dpc_layer& L = P.layers[l];
+                const size_t m = (size_t)(row0 + r) * sl[l - 1].N + q.col;
+                const bool st_z = (P.ops & DPC_ROWS_STORE_Z) && !(l == nw && P.top_clamped);
+                const bool st_e =
+                    (P.ops & DPC_ROWS_STORE_E) || ((P.ops & DPC_ROWS_TERMINAL) && l == nw);
+                float* fe = (P.ops & DPC_ROWS_STORE_G) && !simple ? P.layers[l - 1].fe : nullptr;
+                float* zf = simple && l < nw && (P.ops & DPC_ROWS_STORE_Z) ? L.zF : nullptr;
+                float* v = P.has_v && (P.ops & DPC_ROWS_STORE_V) ? L.v : nullptr;
+                for (int j = 0; j < q.valid; ++j)
+                {
+                  if (st_z)
+                    L.z[m + j] = Z[o + j];
+                  if (st_e)
+                    L.e[m + j] = E[o + j];
+                  if (fe)
+                    fe[m + j] = Gb[o + j];
+                  if (zf)
+                    zf[m + j] = Gb[o + j];
+                  if (v)
+                    v[m + j] = Vb[o + j];
+                }
+              });
     if (P.ops & DPC_ROWS_STORE_E)
     {
       float* e0 = P.layers[0].e + (size_t)row0 * sl[0].K;
@@ -829,49 +969,82 @@ int build(dpc_plan* p, int R, int S, bool has_v)
   const int kslice0 = ((K0p + ks0 - 1) / ks0 + 3) & ~3;
   ks0 = (K0p + kslice0 - 1) / kslice0;
 
-  std::vector<int> ft, bt;
+  std::vector<ResTask> ft, bt;
   size_t fparts = 0, bparts = 0;
-  // Slices: one layer's tasks alone should occupy the warps (the sweep runs layer by layer), a slice
-  // being worth its overhead from 32 inputs or 16 output rows on; halved while the partial sums of
-  // all layers take more than 32 KB.
+  // Slices: a settling pass has one list for all layers, so a layer's tasks get its share of the warps
+  // (rounded down: one round for all), a slice being worth its overhead from 16 inputs or output rows
+  // on; halved while the partial sums of all layers take more than 32 KB.
   auto tasks = [&](int shift)
   {
     ft.clear(), bt.clear();
     fparts = bparts = 0;
+    double fw = 0.0, bw = 0.0;
+    for (int l = 1; l < nw; ++l)
+    {
+      ResLayer& q = rl[l];
+      q.kw = q.K >= 96 && (q.woff >= 0 || q.vec) ? 4 : 1;
+      fw += (double)((q.N + 31) / 32) * q.K;
+      bw += (double)((q.K + 32 * q.kw - 1) / (32 * q.kw)) * q.kw * q.N;
+    }
     for (int l = 1; l < nw; ++l)
     {
       ResLayer& q = rl[l];
       const int np = up4(q.N), kp = up4(q.K);
+      const bool streamed = q.woff < 0;
+      ResTask t = {};
       q.fpart = (int)fparts;
-      if (q.woff >= 0)
+      if (!streamed)
       {
         const int blks = (q.N + 31) / 32;
-        int s = std::max(1, std::min({kWarps / (blks * rbs), q.K / 32, 16}) >> shift);
+        const double share = (double)blks * q.K / fw;
+        int s = std::max(1, std::min({(int)(kWarps * share / (blks * rbs) + 0.01), q.K / 16, 16}) >> shift);
         q.fslice = ((q.K + s - 1) / s + 3) & ~3;
         s = (q.K + q.fslice - 1) / q.fslice;
         for (int rb = 0; rb < rbs; ++rb)
           for (int k = 0; k < s; ++k)
             for (int b = 0; b < blks; ++b)
-              ft.push_back(pack(l, rb, k, b));
+            {
+              t.w = q.woff + b * 32 * q.ldw + k * q.fslice, t.ldw = q.ldw;
+              t.x = q.zoff + rb * RT * S + k * q.fslice;
+              t.len = std::min(q.K - k * q.fslice, q.fslice);
+              t.out = q.fpart + (k * R + rb * RT) * np + b * 32, t.pitch = np;
+              t.lanes = std::min(32, q.N - b * 32);
+              t.kind = l << 4;
+              ft.push_back(t);
+            }
         fparts += (size_t)s * R * np;
       }
       else
       {
         q.fslice = q.K;
-        for (int b = 0; b < (q.N + G - 1) / G; ++b)
-          ft.push_back(pack(l, 0, 0, b));
+        for (int b = 0; b < q.N; b += G)
+        {
+          t.w = b * q.K, t.ldw = q.K, t.x = q.zoff, t.len = q.K;
+          t.out = q.fpart + b, t.pitch = np, t.lanes = q.N - b;
+          t.kind = l << 4 | T_STREAM | (q.vec ? T_VEC : 0);
+          ft.push_back(t);
+        }
         fparts += (size_t)R * np;
       }
-      q.kw = q.K >= 96 && (q.woff >= 0 || q.vec) ? 4 : 1;
-      const int blks = (q.K + 32 * q.kw - 1) / (32 * q.kw);
-      int s = std::max(1, std::min({kWarps / (blks * rbs), q.N / 16, 16}) >> shift);
+      const int cols = 32 * q.kw, blks = (q.K + cols - 1) / cols;
+      const double share = (double)blks * q.kw * q.N / bw;
+      int s = std::max(1, std::min({(int)(kWarps * share / (blks * rbs) + 0.01), q.N / 8, 16}) >> shift);
       q.bslice = ((q.N + s - 1) / s + 3) & ~3;
       s = (q.N + q.bslice - 1) / q.bslice;
       q.bpart = (int)bparts;
       for (int rb = 0; rb < rbs; ++rb)
         for (int k = 0; k < s; ++k)
           for (int b = 0; b < blks; ++b)
-            bt.push_back(pack(l, rb, k, b));
+          {
+            t.ldw = streamed ? q.K : q.ldw;
+            t.w = (streamed ? 0 : q.woff) + k * q.bslice * t.ldw + b * cols;
+            t.x = q.noff + rb * RT * S + k * q.bslice;
+            t.len = std::min(q.N - k * q.bslice, q.bslice);
+            t.out = q.bpart + (k * R + rb * RT) * kp + b * cols, t.pitch = kp;
+            t.lanes = std::min(32, (q.K - b * cols + q.kw - 1) / q.kw);
+            t.kind = l << 4 | (streamed ? T_STREAM : 0) | (q.kw == 4 ? T_VEC : 0);
+            bt.push_back(t);
+          }
       bparts += (size_t)s * R * kp;
     }
     return std::max(fparts, bparts) * sizeof(float) <= 32 * 1024;
@@ -885,7 +1058,7 @@ int build(dpc_plan* p, int R, int S, bool has_v)
   auto table_bytes = [&]()
   {
     return round16(sizeof(ResLayer) * nw) + sizeof(ResQuad) * (S / 4) +
-           round16(sizeof(int) * ft.size()) + round16(sizeof(int) * bt.size());
+           sizeof(ResTask) * (std::max<size_t>(ft.size(), 1) + std::max<size_t>(bt.size(), 1));
   };
   auto others = [&]()
   {
@@ -930,6 +1103,8 @@ int build(dpc_plan* p, int R, int S, bool has_v)
       q = ResQuad{};
       q.layer = (short)(l + 1), q.col = c, q.valid = (short)std::min(4, rl[l].N - c);
       q.pitch = up4(rl[l].N);
+      q.down = rl[l].zoff + c; // residual layers are square
+      q.up = l + 1 < nw ? rl[l + 1].noff + c : 0;
       q.fpart = rl[l].fpart + c;
       q.fslices = l > 0 ? (short)((rl[l].K + rl[l].fslice - 1) / rl[l].fslice) : 0;
       if (l + 1 < nw)
@@ -953,8 +1128,11 @@ int build(dpc_plan* p, int R, int S, bool has_v)
   ResParams& P = st->P;
   put(rl.data(), sizeof(ResLayer) * nw);
   P.a_quad = put(quads.data(), sizeof(ResQuad) * quads.size());
-  P.a_ft = put(ft.data(), sizeof(int) * ft.size());
-  P.a_bt = put(bt.data(), sizeof(int) * bt.size());
+  P.nf = (int)ft.size(), P.nb = (int)bt.size();
+  ft.resize(std::max<size_t>(ft.size(), 1)); // (a network of one weight layer has no tasks)
+  bt.resize(std::max<size_t>(bt.size(), 1));
+  P.a_ft = put(ft.data(), sizeof(ResTask) * ft.size());
+  P.a_bt = put(bt.data(), sizeof(ResTask) * bt.size());
   P.table_vecs = (int)(at / 16);
   if (cudaMalloc(&st->dev, host.size()) != cudaSuccess ||
       cudaMemcpy(st->dev, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess)
@@ -967,7 +1145,6 @@ int build(dpc_plan* p, int R, int S, bool has_v)
   P.layers = p->d;
   P.top_n = rl[nw - 1].N;
   P.n = p->n, P.batch = p->batch, P.S = S;
-  P.nf = (int)ft.size(), P.nb = (int)bt.size();
   P.N1p = N1p, P.K0p = K0p, P.ks0 = ks0, P.kslice0 = kslice0;
   P.wfloats = (int)((used + 3) & ~(size_t)3);
   P.groups = (p->batch + R - 1) / R;
