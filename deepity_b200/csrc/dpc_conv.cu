@@ -8,7 +8,7 @@
 #include <algorithm>
 #include <cstring>
 
-#include "dpc_internal.h"
+#include "dpc_conv_internal.h"
 #include "dpc_math.cuh"
 
 namespace dpc
@@ -538,17 +538,6 @@ __global__ void conv_center_rows_kernel(const dpc_conv_layer L)
 using namespace dpc;
 using namespace dpc::conv;
 
-struct dpc_conv_plan
-{
-  dpc_ctx* ctx = nullptr;
-  int n = 0, batch = 0;
-  std::vector<dpc_conv_layer> h;
-  double* energy = nullptr;
-  double* energy_host = nullptr;
-  float* scratch = nullptr; // one state-sized buffer for split state updates (largest layer)
-  size_t scratch_floats = 0;
-};
-
 namespace
 {
 // How many ways to split a reduction of length K over CTAs when the tile grid alone does not
@@ -663,6 +652,11 @@ int dpc_conv_plan_create(dpc_ctx* ctx, const dpc_conv_layer* layers, int n_layer
     delete p;
     return cuda_fail(cudaGetLastError(), "conv plan scratch allocation");
   }
+  if ((rc = conv_res_init(p)) < 0)
+  {
+    dpc_conv_plan_destroy(p);
+    return rc;
+  }
   *out = p;
   return DPC_OK;
 }
@@ -674,8 +668,11 @@ int dpc_conv_plan_update(dpc_conv_plan* p, const dpc_conv_layer* layers, int n_l
   int rc = validate(layers, n_layers);
   if (rc != DPC_OK)
     return rc;
+  DPC_CUDA(cudaStreamSynchronize(p->ctx->stream));
   p->h.assign(layers, layers + n_layers);
-  return DPC_OK;
+  conv_res_free(p);
+  rc = conv_res_init(p);
+  return rc < 0 ? rc : DPC_OK;
 }
 
 int dpc_conv_plan_destroy(dpc_conv_plan* p)
@@ -684,6 +681,7 @@ int dpc_conv_plan_destroy(dpc_conv_plan* p)
     return DPC_OK;
   cudaSetDevice(p->ctx->device);
   cudaStreamSynchronize(p->ctx->stream);
+  conv_res_free(p);
   if (p->energy)
     cudaFree(p->energy);
   if (p->energy_host)

@@ -370,7 +370,12 @@ float SimpleConvPCNetwork::TrainStepRaw(const float* x, size_t nx, const float* 
     throw std::invalid_argument("deepity_b200: bad inference step count");
   SyncPlan();
   const int n = (int)layers.size();
-  ResetState();
+  // (an image segment starts from zero beliefs by itself; without a settling step the weight update
+  // reads the prediction instead of the derivative, which only the phases keep apart)
+  const bool images = steps > 0 && dpc_conv_images_available(plan);
+  if (!images || nx < (size_t)batchSize * layers.front()->GetInputSize() ||
+      ny < (size_t)batchSize * layers.back()->GetInputSize())
+    ResetState();
   ClampRaw(0, x, nx, onDevice);
   ClampRaw(n - 1, y, ny, onDevice);
   for (int i = 1; i + 1 < n; ++i)
@@ -380,6 +385,21 @@ float SimpleConvPCNetwork::TrainStepRaw(const float* x, size_t nx, const float* 
   const bool gate0 = layers[0]->gateIsPrediction;
   auto phases = [&]
   {
+    if (images)
+    {
+      Check(dpc_conv_images_segment(plan, DPC_ROWS_FIRST | DPC_ROWS_STORE_Z |
+                                              (withProjection ? DPC_ROWS_SWEEP : DPC_ROWS_ZERO_Z),
+                                    steps, 1));
+      for (auto& l : layers)
+        l->gateIsPrediction = false;
+      UpdateWeights();
+      Check(dpc_conv_energy_reset(plan));
+      Check(dpc_conv_images_segment(plan, DPC_ROWS_ENERGY_LAST | DPC_ROWS_PRED_CLOSE, 0, 1));
+      for (auto& l : layers)
+        l->gateIsPrediction = true;
+      layers.front()->cacheValid = true;
+      return;
+    }
     if (withProjection)
       ProjectForward();
     Settle(steps);
@@ -444,12 +464,25 @@ void SimpleConvPCNetwork::PredictRaw(const float* x, size_t nx, int steps, bool 
   const size_t count = (size_t)batchSize * layers.back()->GetInputSize();
   if (nout != count)
     throw std::invalid_argument("deepity_b200: Predict() output buffer has the wrong size");
-  ResetState();
+  const bool images = dpc_conv_images_available(plan);
+  if (!images || nx < (size_t)batchSize * layers.front()->GetInputSize())
+    ResetState();
   ClampRaw(0, x, nx, false);
   for (int i = 1; i < n; ++i)
     layers[i]->clamped = false;
   auto phases = [&]
   {
+    if (images)
+    {
+      Check(dpc_conv_images_segment(plan, DPC_ROWS_FIRST | DPC_ROWS_STORE_Z |
+                                              (withProjection ? DPC_ROWS_SWEEP : DPC_ROWS_ZERO_Z) |
+                                              (steps ? DPC_ROWS_PRED_LAST : DPC_ROWS_SWEEP_PRED),
+                                    steps, 0));
+      for (auto& l : layers)
+        l->gateIsPrediction = steps == 0;
+      layers.front()->cacheValid = true;
+      return;
+    }
     if (withProjection)
       ProjectForward();
     Settle(steps);
