@@ -20,8 +20,7 @@ constexpr int TM = 64, TN = 64, TK = 16, THREADS = 256, PADC = 4;
 enum ConvOp
 {
   C_FWD = 0, // preact[o, (b,p)] = sum_k W[o,k] * col(z)[k,(b,p)]       M=O    N=B*oH*oW K=C*kH*kW
-  C_BWD = 1, // dz[c, (b,y,x)]   = sum_k W^T[c,k=(o,ky,kx)] * g gathered  M=C    N=B*H*W   K=O*kH*kW
-  C_WG = 2   // dW[o, r]         = sum_(b,p) g[o,(b,p)] * col(z)[r,(b,p)] M=O    N=C*kH*kW K=B*oH*oW
+  C_BWD = 1  // dz[c, (b,y,x)]   = sum_k W^T[c,k=(o,ky,kx)] * g gathered  M=C    N=B*H*W   K=O*kH*kW
 };
 
 struct Tile
@@ -61,14 +60,12 @@ __global__ void __launch_bounds__(THREADS)
   int M, N, K;
   if (OP == C_FWD)
     M = O, N = batch * P, K = rows;
-  else if (OP == C_BWD)
-    M = C, N = batch * HW, K = O * KK;
   else
-    M = O, N = rows, K = batch * P;
+    M = C, N = batch * HW, K = O * KK;
   const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
   // k_chunk > 0: the reduction is split over blockIdx.z and the partial sums are added
-  // atomically into a zeroed buffer (g_W for the weight gradient, preact for the forward
-  // product, `split_out` for the state update); a second kernel applies the epilogue.
+  // atomically into a zeroed buffer (preact for the forward product, `split_out` for the state
+  // update); a second kernel applies the epilogue.
   int k_begin = 0, k_end = K;
   if (k_chunk > 0)
   {
@@ -82,7 +79,7 @@ __global__ void __launch_bounds__(THREADS)
 
   // ---- per-thread invariants of the B-operand gather: 4 consecutive n, one k per pass
   const int bn = n0 + ((t & 15) << 2);
-  int nb[4], ny[4], nx[4]; // FWD/BWD: image and (already offset) pixel origin; WG: (c, ky, kx)
+  int nb[4], ny[4], nx[4]; // image and (already offset) pixel origin
 #pragma unroll
   for (int j = 0; j < 4; ++j)
   {
@@ -98,16 +95,11 @@ __global__ void __launch_bounds__(THREADS)
       const int oy = p / oW, ox = p - oy * oW;
       nb[j] = b, ny[j] = oy * L.s_h - L.p_h, nx[j] = ox * L.s_w - L.p_w;
     }
-    else if (OP == C_BWD)
+    else
     {
       const int b = n / HW, q = n - b * HW;
       const int y = q / Wd, x = q - y * Wd;
       nb[j] = b, ny[j] = y + L.p_h, nx[j] = x + L.p_w;
-    }
-    else
-    {
-      const int c = n / KK, r = n - c * KK;
-      nb[j] = c, ny[j] = r / kW, nx[j] = r - (r / kW) * kW;
     }
   }
 
@@ -127,15 +119,10 @@ __global__ void __launch_bounds__(THREADS)
         {
           if (OP == C_FWD)
             v = L.W[(size_t)m * rows + k];
-          else if (OP == C_BWD)
+          else
           {
             const int o = k / KK, r = k - o * KK;
             v = L.W[(size_t)o * rows + m * KK + r];
-          }
-          else
-          {
-            const int b = k / P, p = k - b * P;
-            v = L.g[((size_t)b * O + m) * P + p];
           }
         }
         ra[j] = v;
@@ -144,23 +131,13 @@ __global__ void __launch_bounds__(THREADS)
     // B operand: k = t>>4, 4 consecutive n
     {
       const int k = k0 + (t >> 4);
-      int q0 = 0, q1 = 0, q2 = 0; // FWD: (c, ky, kx); BWD: (o, ky, kx); WG: (b, oy*s-p, ox*s-p)
+      int q0 = 0, q1 = 0, q2 = 0; // FWD: (c, ky, kx); BWD: (o, ky, kx)
       const bool kin = k < k_end;
       if (kin)
       {
-        if (OP == C_FWD || OP == C_BWD)
-        {
-          q0 = k / KK;
-          const int r = k - q0 * KK;
-          q1 = r / kW, q2 = r - q1 * kW;
-        }
-        else
-        {
-          q0 = k / P;
-          const int p = k - q0 * P;
-          const int oy = p / oW;
-          q1 = oy * L.s_h - L.p_h, q2 = (p - oy * oW) * L.s_w - L.p_w;
-        }
+        q0 = k / KK;
+        const int r = k - q0 * KK;
+        q1 = r / kW, q2 = r - q1 * kW;
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j)
@@ -174,7 +151,7 @@ __global__ void __launch_bounds__(THREADS)
             if (iy >= 0 && iy < H && ix >= 0 && ix < Wd)
               v = L.z[(((size_t)nb[j] * C + q0) * H + iy) * Wd + ix];
           }
-          else if (OP == C_BWD)
+          else
           {
             const int ty2 = ny[j] - q1, tx2 = nx[j] - q2;
             if (ty2 >= 0 && tx2 >= 0)
@@ -183,12 +160,6 @@ __global__ void __launch_bounds__(THREADS)
               if (oy * L.s_h == ty2 && ox * L.s_w == tx2 && oy < oH && ox < oW)
                 v = L.g[(((size_t)nb[j] * O + q0) * oH + oy) * oW + ox];
             }
-          }
-          else
-          {
-            const int iy = q1 + ny[j], ix = q2 + nx[j];
-            if (iy >= 0 && iy < H && ix >= 0 && ix < Wd)
-              v = L.z[(((size_t)q0 * C + nb[j]) * H + iy) * Wd + ix];
           }
         }
         rb[j] = v;
@@ -245,7 +216,7 @@ __global__ void __launch_bounds__(THREADS)
   }
 
   // ------------------------------------------------------------------ epilogues
-  if (OP != C_WG && k_chunk > 0)
+  if (k_chunk > 0)
   {
     float* dst = OP == C_FWD ? L.preact : split_out;
     const int PP = OP == C_FWD ? P : HW; // pixels per (image, channel) plane of the output
@@ -304,7 +275,7 @@ __global__ void __launch_bounds__(THREADS)
     if (flags & DPC_CONV_ENERGY)
       block_energy(esum, energy);
   }
-  else if (OP == C_BWD)
+  else
   {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -321,23 +292,6 @@ __global__ void __launch_bounds__(THREADS)
         const int b = n / HW, q = n - b * HW;
         const size_t o = ((size_t)b * C + m) * HW + q;
         L.z[o] += L.ir * (acc[i][j] - L.e[o]);
-      }
-    }
-  }
-  else
-  {
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-    {
-      const int m = m0 + ty * 4 + i;
-      if (m >= M)
-        continue;
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-      {
-        const int n = n0 + tx * 4 + j;
-        if (n < N)
-          atomicAdd(&L.g_W[(size_t)m * rows + n], acc[i][j]);
       }
     }
   }
@@ -431,37 +385,164 @@ __global__ void conv_relax_kernel(const dpc_conv_layer L, int batch)
     L.z[o] -= L.ir * L.e[o];
 }
 
-// g_b[o] = sum over (b, p) of g: one block per output channel, fixed summation order.
-__global__ void conv_bias_grad_kernel(const dpc_conv_layer L, int batch)
+// Weight and bias gradients of a range of layers in one launch: dW[o, r] = sum_(b,p) g[o,(b,p)]
+// col(z)[r,(b,p)] and db[o] = sum_(b,p) g[o,(b,p)], raw sums added atomically into zeroed g_W, g_b.
+// A block takes one 64 x 64 tile and one slice of the batch x pixel reduction of one layer; all layers
+// together fill the GPU, where one after the other each was a latency-bound launch (91 us for the four
+// layers of a 32x32x3 network at batch 128, 97 us more for bias sums of their own).  The
+// (image, pixel) of a k advances by additions, with a multiplication for the row instead of divisions.
+struct GradGroup
 {
-  const int o = blockIdx.x, P = L.out_h * L.out_w;
-  float s = 0.0f;
-  for (int idx = threadIdx.x; idx < batch * P; idx += blockDim.x)
-  {
-    const int b = idx / P, p = idx - b * P;
-    s += L.g[((size_t)b * L.out_c + o) * P + p];
-  }
-  __shared__ float red[32];
+  int layer, first, tiles_n, tiles, chunk; // first block, column tiles, tiles, k per slice
+};
+struct GradGroups
+{
+  GradGroup g[16];
+  int count;
+};
+__global__ void __launch_bounds__(THREADS)
+    conv_gradient_kernel(const dpc_conv_layer* __restrict__ layers, const GradGroups G, int batch)
+{
+  int gi = 0;
+  while (gi + 1 < G.count && (int)blockIdx.x >= G.g[gi + 1].first)
+    ++gi;
+  const GradGroup D = G.g[gi];
+  const dpc_conv_layer& L = layers[D.layer];
+  const int C = L.in_c, O = L.out_c, H = L.in_h, Wd = L.in_w, kW = L.k_w, oW = L.out_w;
+  const int P = L.out_h * oW, KK = L.k_h * kW, rows = C * KK;
+  const int local = blockIdx.x - D.first, tile_i = local % D.tiles, slice = local / D.tiles;
+  const int n0 = (tile_i % D.tiles_n) * TN, m0 = (tile_i / D.tiles_n) * TM;
+  const int k_begin = slice * D.chunk, k_end = min(batch * P, k_begin + D.chunk);
+  const float* __restrict__ g = L.g;
+  const float* __restrict__ z = L.z;
+  // p / oW as a multiplication, exact while p * oW < 2^32
+  const unsigned by_row = oW > 1 && (unsigned long long)P * oW < 0x100000000ull
+                              ? (unsigned)((0x100000000ull + oW - 1) / oW)
+                              : 0u;
+  __shared__ Tile tile;
+  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
+  // B operand: k = t>>4, four consecutive n = (c, ky, kx)
+  int zc[4], dy[4], dx[4];
 #pragma unroll
-  for (int w = 16; w > 0; w >>= 1)
-    s += __shfl_xor_sync(0xffffffffu, s, w);
-  if ((threadIdx.x & 31) == 0)
-    red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0)
+  for (int j = 0; j < 4; ++j)
   {
-    float tsum = 0.0f;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w)
-      tsum += red[w];
-    L.g_b[o] = tsum;
+    const int n = n0 + ((t & 15) << 2) + j;
+    const int c = n / KK, r = n - c * KK;
+    zc[j] = n < rows ? c * H * Wd : -1;
+    dy[j] = r / kW - L.p_h, dx[j] = r - (r / kW) * kW - L.p_w;
+  }
+  // A operand: row t>>2, four consecutive k
+  const int am = m0 + (t >> 2);
+  int ka = k_begin + ((t & 3) << 2), kb = k_begin + (t >> 4);
+  int ab = ka / P, ap = ka - ab * P, bb = kb / P, bp = kb - bb * P;
+  const bool vec = P % 4 == 0 && (reinterpret_cast<uintptr_t>(g) & 15) == 0;
+  float ra[4], rb[4], bsum = 0.0f;
+  auto fetch = [&]()
+  {
+    if (am < O && vec && ka + 3 < k_end)
+    {
+      const float4 v = *reinterpret_cast<const float4*>(g + ((size_t)ab * O + am) * P + ap);
+      ra[0] = v.x, ra[1] = v.y, ra[2] = v.z, ra[3] = v.w;
+    }
+    else
+    {
+      int b = ab, p = ap;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+      {
+        ra[j] = am < O && ka + j < k_end ? g[((size_t)b * O + am) * P + p] : 0.0f;
+        if (++p == P)
+          p = 0, ++b;
+      }
+    }
+    const int oy = by_row ? (int)__umulhi((unsigned)bp, by_row) : bp / oW, ox = bp - oy * oW;
+    const float* zi = z + (size_t)bb * C * H * Wd;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+    {
+      const int iy = oy * L.s_h + dy[j], ix = ox * L.s_w + dx[j];
+      rb[j] = kb < k_end && zc[j] >= 0 && (unsigned)iy < (unsigned)H && (unsigned)ix < (unsigned)Wd
+                  ? zi[zc[j] + iy * Wd + ix]
+                  : 0.0f;
+    }
+    ka += TK, kb += TK;
+    for (ap += TK; ap >= P; ap -= P)
+      ++ab;
+    for (bp += TK; bp >= P; bp -= P)
+      ++bb;
+  };
+  auto stash = [&]()
+  {
+    const int r = t >> 2, kq = (t & 3) << 2;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+    {
+      tile.a[kq + j][r] = ra[j];
+      bsum += ra[j];
+    }
+    *reinterpret_cast<float4*>(&tile.b[t >> 4][(t & 15) << 2]) = make_float4(rb[0], rb[1], rb[2], rb[3]);
+  };
+  float acc[4][4] = {};
+  fetch();
+  stash();
+  __syncthreads();
+  for (int k0 = k_begin; k0 < k_end; k0 += TK)
+  {
+    const bool more = k0 + TK < k_end;
+    if (more)
+      fetch();
+#pragma unroll
+    for (int k = 0; k < TK; ++k)
+    {
+      const float4 av = *reinterpret_cast<const float4*>(&tile.a[k][ty * 4]);
+      const float4 bv = *reinterpret_cast<const float4*>(&tile.b[k][tx * 4]);
+      const float a4[4] = {av.x, av.y, av.z, av.w};
+      const float b4[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          acc[i][j] = fmaf(a4[i], b4[j], acc[i][j]);
+    }
+    __syncthreads();
+    if (more)
+    {
+      stash();
+      __syncthreads();
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+  {
+    const int m = m0 + ty * 4 + i;
+    if (m >= O)
+      continue;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+    {
+      const int n = n0 + tx * 4 + j;
+      if (n < rows)
+        atomicAdd(&L.g_W[(size_t)m * rows + n], acc[i][j]);
+    }
+  }
+  if (n0 == 0)
+  {
+    bsum += __shfl_xor_sync(0xffffffffu, bsum, 1);
+    bsum += __shfl_xor_sync(0xffffffffu, bsum, 2);
+    if ((t & 3) == 0 && am < O)
+      atomicAdd(&L.g_b[am], bsum);
   }
 }
 
 // SGD / Adam / AdamW on W and b from the raw sums in g_W, g_b
 // (src/layers/SimpleConvPCLayer.cpp:424-556: SGD rate lr/B with decay (1-lambda) first;
 // Adam-type gradients are -(1/B) * sum).
-__global__ void conv_apply_kernel(const dpc_conv_layer L, int batch)
+// The sums are zeroed behind the update: the next gradient launch adds into them.  blockIdx.y = layer.
+__global__ void conv_apply_kernel(const dpc_conv_layer* __restrict__ layers, int first, int batch)
 {
+  const dpc_conv_layer L = layers[first + blockIdx.y];
+  if (L.out_c <= 0)
+    return;
   const size_t nW = (size_t)L.out_c * L.in_c * L.k_h * L.k_w;
   const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t nthr = (size_t)gridDim.x * blockDim.x;
@@ -476,18 +557,23 @@ __global__ void conv_apply_kernel(const dpc_conv_layer L, int batch)
       if (decay != 1.0f)
         w *= decay;
       L.W[o] = fmaf(alpha, L.g_W[o], w);
+      L.g_W[o] = 0.0f;
     }
     for (size_t j = tid; j < (size_t)L.out_c; j += nthr)
+    {
       L.b[j] = fmaf(alpha, L.g_b[j], L.b[j]);
+      L.g_b[j] = 0.0f;
+    }
     return;
   }
-  const float step = adam_step_size(L.lr, *L.t);
+  const float step = adam_step_size(L.lr, *L.t + 1); // (the counter itself moves on afterwards)
   const float lr_wd = L.opt == DPC_OPT_ADAMW ? L.lr * L.lmbda : -1.0f;
   const float gs = -1.0f / Bf;
   for (size_t o = tid; o < nW; o += nthr)
   {
     float m = L.m_W[o], v = L.v_W[o];
     L.W[o] = adam_update(L.W[o], gs * L.g_W[o], m, v, step, lr_wd);
+    L.g_W[o] = 0.0f;
     L.m_W[o] = m;
     L.v_W[o] = v;
   }
@@ -495,19 +581,25 @@ __global__ void conv_apply_kernel(const dpc_conv_layer L, int batch)
   {
     float m = L.m_b[j], v = L.v_b[j];
     L.b[j] = adam_update(L.b[j], gs * L.g_b[j], m, v, step, -1.0f);
+    L.g_b[j] = 0.0f;
     L.m_b[j] = m;
     L.v_b[j] = v;
   }
 }
 
-__global__ void conv_bump_counter_kernel(int32_t* t)
+__global__ void conv_bump_counter_kernel(const dpc_conv_layer* __restrict__ layers, int first)
 {
-  *t += 1;
+  const dpc_conv_layer& L = layers[first + threadIdx.x];
+  if (L.out_c > 0 && L.opt != DPC_OPT_SGD)
+    *L.t += 1;
 }
 
 // Row centring of W [O, C*kH*kW] (src/backend/CPUBackend.cpp:250-272): one block per row.
-__global__ void conv_center_rows_kernel(const dpc_conv_layer L)
+__global__ void conv_center_rows_kernel(const dpc_conv_layer* __restrict__ layers, int first)
 {
+  const dpc_conv_layer& L = layers[first + blockIdx.y];
+  if ((int)blockIdx.x >= L.out_c)
+    return;
   const int rows = L.in_c * L.k_h * L.k_w;
   float* row = L.W + (size_t)blockIdx.x * rows;
   float s = 0.0f;
@@ -613,6 +705,21 @@ int validate(const dpc_conv_layer* l, int n)
   return DPC_OK;
 }
 
+// The layer table on the device; the gradient sums start at zero (the update kernel leaves them so).
+int upload_layers(dpc_conv_plan* p)
+{
+  if (!p->d)
+    DPC_CUDA(cudaMalloc(&p->d, sizeof(dpc_conv_layer) * p->n));
+  DPC_CUDA(cudaMemcpy(p->d, p->h.data(), sizeof(dpc_conv_layer) * p->n, cudaMemcpyHostToDevice));
+  for (const auto& L : p->h)
+    if (L.out_c > 0)
+    {
+      DPC_CUDA(cudaMemset(L.g_W, 0, sizeof(float) * (size_t)L.out_c * L.in_c * L.k_h * L.k_w));
+      DPC_CUDA(cudaMemset(L.g_b, 0, sizeof(float) * L.out_c));
+    }
+  return DPC_OK;
+}
+
 int check_layer(dpc_conv_plan* p, int layer)
 {
   if (!p)
@@ -642,15 +749,19 @@ int dpc_conv_plan_create(dpc_ctx* ctx, const dpc_conv_layer* layers, int n_layer
     return cuda_fail(cudaGetLastError(), "conv plan allocation");
   }
   cudaMemset(p->energy, 0, sizeof(double));
+  if ((rc = upload_layers(p)) != DPC_OK)
+  {
+    dpc_conv_plan_destroy(p);
+    return rc;
+  }
   for (int i = 0; i < n_layers; ++i)
     p->scratch_floats = std::max(p->scratch_floats, (size_t)batch * layers[i].in_c *
                                                         layers[i].in_h * layers[i].in_w);
   if (cudaMalloc(&p->scratch, p->scratch_floats * sizeof(float)) != cudaSuccess)
   {
-    cudaFree(p->energy);
-    cudaFreeHost(p->energy_host);
-    delete p;
-    return cuda_fail(cudaGetLastError(), "conv plan scratch allocation");
+    const cudaError_t e = cudaGetLastError();
+    dpc_conv_plan_destroy(p);
+    return cuda_fail(e, "conv plan scratch allocation");
   }
   if ((rc = conv_res_init(p)) < 0)
   {
@@ -668,8 +779,26 @@ int dpc_conv_plan_update(dpc_conv_plan* p, const dpc_conv_layer* layers, int n_l
   int rc = validate(layers, n_layers);
   if (rc != DPC_OK)
     return rc;
+  // new rates only: see dpc_plan_update
+  bool structure = false;
+  for (int i = 0; i < n_layers && !structure; ++i)
+  {
+    dpc_conv_layer a = p->h[i], b = layers[i];
+    for (dpc_conv_layer* q : {&a, &b})
+      q->lr = q->ir = q->lmbda = 0.0f;
+    structure = memcmp(&a, &b, sizeof(dpc_conv_layer)) != 0;
+  }
+  if (!structure)
+  {
+    p->h.assign(layers, layers + n_layers);
+    DPC_CUDA(cudaMemcpyAsync(p->d, p->h.data(), sizeof(dpc_conv_layer) * n_layers,
+                             cudaMemcpyHostToDevice, p->ctx->stream));
+    return DPC_OK;
+  }
   DPC_CUDA(cudaStreamSynchronize(p->ctx->stream));
   p->h.assign(layers, layers + n_layers);
+  if ((rc = upload_layers(p)) != DPC_OK)
+    return rc;
   conv_res_free(p);
   rc = conv_res_init(p);
   return rc < 0 ? rc : DPC_OK;
@@ -682,6 +811,7 @@ int dpc_conv_plan_destroy(dpc_conv_plan* p)
   cudaSetDevice(p->ctx->device);
   cudaStreamSynchronize(p->ctx->stream);
   conv_res_free(p);
+  cudaFree(p->d);
   if (p->energy)
     cudaFree(p->energy);
   if (p->energy_host)
@@ -781,44 +911,70 @@ int dpc_conv_gate_with_prediction(dpc_conv_plan* p, int layer)
 
 int dpc_conv_update_weights(dpc_conv_plan* p, int layer, int center_rows)
 {
-  int rc = check_layer(p, layer);
-  if (rc != DPC_OK)
+  return dpc_conv_update_weights_range(p, layer, 1, center_rows);
+}
+
+int dpc_conv_update_weights_range(dpc_conv_plan* p, int first, int count, int center_rows)
+{
+  int rc = check_layer(p, first);
+  if (rc != DPC_OK || (rc = check_layer(p, first + count - 1)) != DPC_OK)
     return rc;
-  const dpc_conv_layer& L = p->h[layer];
-  if (L.out_c <= 0)
-    return DPC_OK;
   cudaStream_t st = p->ctx->stream;
-  const int rows = L.in_c * L.k_h * L.k_w;
-  const long long K = (long long)p->batch * L.out_h * L.out_w;
-  DPC_CUDA(cudaMemsetAsync(L.g_W, 0, sizeof(float) * (size_t)L.out_c * rows, st));
-  // Split the long reduction (batch x output pixels) over enough CTAs to fill the GPU.
-  const int tiles = cdiv_i(rows, TN) * cdiv_i(L.out_c, TM);
-  int splits = std::max(1, std::min<int>((int)(K / (4 * TK)) + 1, (2 * p->ctx->sm_count) / tiles));
-  int k_chunk = cdiv_i(K, splits);
-  k_chunk = cdiv_i(k_chunk, TK) * TK;
-  splits = cdiv_i(K, k_chunk);
-  dim3 grid(cdiv_i(rows, TN), cdiv_i(L.out_c, TM), splits);
-  conv_gemm_kernel<C_WG><<<grid, THREADS, 0, st>>>(L, nullptr, nullptr, p->batch, 0, p->energy,
-                                                  k_chunk);
-  if ((rc = conv_check_launch(p->ctx, "conv weight gradient kernel")) != DPC_OK)
-    return rc;
-  conv_bias_grad_kernel<<<L.out_c, 256, 0, st>>>(L, p->batch);
-  if ((rc = conv_check_launch(p->ctx, "conv bias gradient kernel")) != DPC_OK)
-    return rc;
-  if (L.opt != DPC_OPT_SGD)
+  while (count > 0)
   {
-    conv_bump_counter_kernel<<<1, 1, 0, st>>>(L.t);
-    if ((rc = conv_check_launch(p->ctx, "conv counter kernel")) != DPC_OK)
-      return rc;
-  }
-  conv_apply_kernel<<<elem_grid(p, (size_t)L.out_c * rows), THREADS, 0, st>>>(L, p->batch);
-  if ((rc = conv_check_launch(p->ctx, "conv apply kernel")) != DPC_OK)
-    return rc;
-  if (center_rows)
-  {
-    conv_center_rows_kernel<<<L.out_c, 128, 0, st>>>(L);
-    if ((rc = conv_check_launch(p->ctx, "conv center rows kernel")) != DPC_OK)
-      return rc;
+    const int c = std::min(count, 16);
+    GradGroups G = {};
+    int blocks = 0, adam = 0, max_o = 0;
+    size_t max_w = 0;
+    // every layer's reduction is split so that the layers together give about four blocks per SM
+    double total = 0.0;
+    for (int i = first; i < first + c; ++i)
+    {
+      const dpc_conv_layer& L = p->h[i];
+      if (L.out_c > 0)
+        total += (double)cdiv_i((long long)L.in_c * L.k_h * L.k_w, TN) * cdiv_i(L.out_c, TM) * p->batch *
+                 L.out_h * L.out_w;
+    }
+    for (int i = first; i < first + c; ++i)
+    {
+      const dpc_conv_layer& L = p->h[i];
+      if (L.out_c <= 0)
+        continue;
+      const int rows = L.in_c * L.k_h * L.k_w;
+      const long long K = (long long)p->batch * L.out_h * L.out_w;
+      GradGroup& g = G.g[G.count++];
+      g.layer = i, g.first = blocks;
+      g.tiles_n = cdiv_i(rows, TN), g.tiles = g.tiles_n * cdiv_i(L.out_c, TM);
+      long long chunk = (long long)(total / (4.0 * p->ctx->sm_count)) + 1;
+      chunk = std::min(std::max<long long>(chunk, 4 * TK), K);
+      g.chunk = cdiv_i(chunk, TK) * TK;
+      blocks += g.tiles * cdiv_i(K, g.chunk);
+      adam |= L.opt != DPC_OPT_SGD;
+      max_w = std::max(max_w, (size_t)L.out_c * rows);
+      max_o = std::max(max_o, L.out_c);
+    }
+    if (G.count > 0)
+    {
+      conv_gradient_kernel<<<blocks, THREADS, 0, st>>>(p->d, G, p->batch);
+      if ((rc = conv_check_launch(p->ctx, "conv gradient kernel")) != DPC_OK)
+        return rc;
+      conv_apply_kernel<<<dim3(elem_grid(p, max_w), c), THREADS, 0, st>>>(p->d, first, p->batch);
+      if ((rc = conv_check_launch(p->ctx, "conv apply kernel")) != DPC_OK)
+        return rc;
+      if (adam)
+      {
+        conv_bump_counter_kernel<<<1, c, 0, st>>>(p->d, first);
+        if ((rc = conv_check_launch(p->ctx, "conv counter kernel")) != DPC_OK)
+          return rc;
+      }
+      if (center_rows)
+      {
+        conv_center_rows_kernel<<<dim3(max_o, c), 128, 0, st>>>(p->d, first);
+        if ((rc = conv_check_launch(p->ctx, "conv center rows kernel")) != DPC_OK)
+          return rc;
+      }
+    }
+    first += c, count -= c;
   }
   return DPC_OK;
 }

@@ -9,6 +9,7 @@ struct dpc_conv_plan
   dpc_ctx* ctx = nullptr;
   int n = 0, batch = 0;
   std::vector<dpc_conv_layer> h;
+  dpc_conv_layer* d = nullptr; // device copy of the table
   double* energy = nullptr;
   double* energy_host = nullptr;
   float* scratch = nullptr; // one state-sized buffer for split state updates (largest layer)

@@ -12,10 +12,10 @@
 //   forward   out[o][p]  = sum_k W[o][k] z[koff[k] + base[p]]
 //   state     dz[c][q]   = sum_k W'[c][k] g[koff[k] + base[q]], one product per stride-parity class
 //             of input pixels: only the taps that hit an output pixel are in its k range
-// A warp owns 16 output channels x 8..32 pixels (mma.m16n8k8 on tf32, three passes hi*lo + lo*hi +
-// hi*hi with fp32 accumulation: the fp32 scheme of the tensor-core kernels of dpc_tc.cu).  The weights
-// come pre-arranged in fragment order (conv_pack_kernel, 700 KB, once per weight update), so a lane's
-// four elements are one 16-byte load, four of them in flight.  mma.sync and not tcgen05: the products
+// A warp owns 16 or 32 output channels x 8..32 pixels (mma.m16n8k8 on tf32, three passes hi*lo + lo*hi
+// + hi*hi with fp32 accumulation: the fp32 scheme of the tensor-core kernels of dpc_tc.cu).  The
+// weights come in fragment order (conv_pack_kernel, once per weight update), so a lane's four elements
+// are one 16-byte load, kDepth of them in flight.  mma.sync and not tcgen05: the products
 // of one image are 16..128 x 64..256 x 64..576, far below a 128-row tile.
 // Layers whose output is one pixel (dense heads) are dot products on the CUDA cores.
 // What bounds it: the tensor pipe and L2 bandwidth of the SM about equally.
@@ -34,6 +34,7 @@ namespace
 {
 constexpr int kThreads = 512, kWarps = kThreads / 32, kMaxLayers = 16;
 constexpr size_t kSmemLimit = 227 * 1024, kStatic = 4 * 1024;
+constexpr int kDepth = 4; // weight loads in flight; the packed steps and the koff table are padded to it
 
 struct RcLayer // per weight layer l; "up" is layer l + 1, the state it predicts
 {
@@ -53,7 +54,7 @@ struct __align__(16) RcTask
   int ktab;      // koff table
   int ntab;      // pixel table: base, pixel index pairs
   int m0, count; // first output row, pixels of the tile (dense: outputs or columns)
-  int ntl;       // 8-pixel tiles
+  int shape;     // 8 x (16-row tiles) + (8-pixel tiles)
   int what;      // layer << 2 | op
 };
 enum
@@ -75,82 +76,161 @@ struct RcParams
   const RcLayer* rl;
   const RcTask* tasks;          // forward (by layer), then state; copied to shared memory
   const unsigned short* order;  // both lists again, longest tasks first
-  const unsigned short* table;  // koff / pixel tables
+  const unsigned short* table;  // pixel tables
+  const uint2* koff;            // per step and lane % 4: byte offsets of its two k
   const float4* packed;
   int nw, batch;
-  int nf, nb, table_vecs;
+  int nf, nb, table_vecs, koff_vecs;
   int zfloats, mu0, efloat, gfloat, xoff, xfloats; // regions, in floats
-  int tab_at, task_at, order_at, bias_at, bias_n;  // further regions, float offsets
+  int tab_at, koff_at, task_at, order_at, bias_at, bias_n;  // further regions, float offsets
   int ops, steps, top_clamped;
   double* energy;
 };
 
-__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo)
+// The tensor core reads the leading 11 significant bits of a tf32 operand: x itself serves as its high
+// part, and the remainder is exact (its own trailing bits, 2^-21 of |x|, are not read).
+__device__ __forceinline__ uint32_t tf32_rest(float x)
 {
-  // round to 11 significant bits (ties away); the remainder is exact and the tensor core reads its
-  // leading 11 bits: 2^-22 of |x| is lost
-  hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-  lo = __float_as_uint(x - __uint_as_float(hi));
+  return __float_as_uint(x - __uint_as_float(__float_as_uint(x) & 0xffffe000u));
+}
+__device__ __forceinline__ float lds(uint32_t address)
+{
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(address));
+  return v;
 }
 
-__device__ __forceinline__ void mma8(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
+__device__ __forceinline__ void mma8(float (&c)[4], const float4& a, uint32_t b0, uint32_t b1)
 {
   asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
                "{%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+               : "r"(__float_as_uint(a.x)), "r"(__float_as_uint(a.y)), "r"(__float_as_uint(a.z)),
+                 "r"(__float_as_uint(a.w)), "r"(b0), "r"(b1));
 }
 
-// acc[j]: rows m0 + lane/4 (+8), pixels 8 j + 2 (lane % 4) (+1) of the task's tile
-template <int NTL>
-__device__ __forceinline__ void mma_tile(float (&acc)[NTL][4], const RcTask& t, const float4* packed,
-                                         const unsigned short* T, const float* sm, int lane)
+// acc[i][j]: rows m0 + 16 i + lane/4 (+8), pixels 8 j + 2 (lane % 4) (+1) of the task's tile
+template <int MT, int NTL>
+__device__ __forceinline__ void mma_tile(float (&acc)[MT][NTL][4], const RcTask& t, const float4* packed,
+                                         const unsigned short* T, const uint2* koff, const float* sm,
+                                         int lane)
 {
   const int g = lane >> 2, c = lane & 3;
-  const float* base[NTL];
+  uint32_t base[NTL];
+  float cor[MT][NTL][4]; // the two small products: chains of their own
 #pragma unroll
   for (int j = 0; j < NTL; ++j)
   {
     const int n = 8 * j + g;
-    base[j] = sm + T[t.ntab + 2 * (n < t.count ? n : 0)];
-    acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+    base[j] = (uint32_t)__cvta_generic_to_shared(sm + T[t.ntab + 2 * (n < t.count ? n : 0)]);
   }
+#pragma unroll
+  for (int i = 0; i < MT; ++i)
+#pragma unroll
+    for (int j = 0; j < NTL; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        acc[i][j][q] = cor[i][j][q] = 0.0f;
   if (t.ks == 0)
     return;
-  const float4* A = packed + t.w + lane;
-  const unsigned short* K = T + t.ktab + c;
-  float4 ring[4];
+  // (the loads of the last kDepth steps run past the task's weights, inside the buffer)
+  const float4* A[MT];
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
-    ring[u] = A[min(u, t.ks - 1) * 32];
-  for (int s0 = 0; s0 < t.ks; s0 += 4)
+  for (int i = 0; i < MT; ++i)
+    A[i] = packed + t.w + lane + i * t.ks * 32;
+  const uint2* K = koff + t.ktab + c;
+  float4 ring[kDepth][MT];
+#pragma unroll
+  for (int u = 0; u < kDepth; ++u)
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+      ring[u][i] = A[i][u * 32];
+  // operand values one step ahead, their offsets two (the table has two steps of zeros at its end)
+  float next[NTL][2];
+  uint2 k = K[0];
+#pragma unroll
+  for (int j = 0; j < NTL; ++j)
+    next[j][0] = lds(base[j] + k.x), next[j][1] = lds(base[j] + k.y);
+  k = K[4];
+  for (int s = 0; s < t.ks; s += kDepth)
   {
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int i = 0; i < MT; ++i)
+      A[i] += kDepth * 32;
+#pragma unroll
+    for (int u = 0; u < kDepth; ++u)
     {
-      const int s = s0 + u;
-      if (s >= t.ks)
-        break;
-      const float4 av = ring[u];
-      ring[u] = A[min(s + 4, t.ks - 1) * 32];
-      const int k0 = K[8 * s], k1 = K[8 * s + 4];
-      uint32_t ah[4], al[4];
-      split_tf32(av.x, ah[0], al[0]);
-      split_tf32(av.y, ah[1], al[1]);
-      split_tf32(av.z, ah[2], al[2]);
-      split_tf32(av.w, ah[3], al[3]);
+      uint32_t bh[NTL][2], bl[NTL][2];
 #pragma unroll
       for (int j = 0; j < NTL; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+        {
+          bh[j][h] = __float_as_uint(next[j][h]);
+          bl[j][h] = tf32_rest(next[j][h]);
+        }
+#pragma unroll
+      for (int j = 0; j < NTL; ++j)
+        next[j][0] = lds(base[j] + k.x), next[j][1] = lds(base[j] + k.y);
+      k = K[4 * u + 8];
+      float4 lo[MT];
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
       {
-        uint32_t bh0, bl0, bh1, bl1;
-        split_tf32(base[j][k0], bh0, bl0);
-        split_tf32(base[j][k1], bh1, bl1);
-        mma8(acc[j], ah, bl0, bl1);
-        mma8(acc[j], al, bh0, bh1);
-        mma8(acc[j], ah, bh0, bh1);
+        const float4 h = ring[u][i];
+        lo[i] = make_float4(__uint_as_float(tf32_rest(h.x)), __uint_as_float(tf32_rest(h.y)),
+                            __uint_as_float(tf32_rest(h.z)), __uint_as_float(tf32_rest(h.w)));
       }
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int j = 0; j < NTL; ++j)
+        {
+          mma8(cor[i][j], ring[u][i], bl[j][0], bl[j][1]);
+          mma8(acc[i][j], ring[u][i], bh[j][0], bh[j][1]);
+        }
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int j = 0; j < NTL; ++j)
+          mma8(cor[i][j], lo[i], bh[j][0], bh[j][1]);
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+        ring[u][i] = A[i][u * 32];
     }
+    K += 4 * kDepth;
   }
+#pragma unroll
+  for (int i = 0; i < MT; ++i)
+#pragma unroll
+    for (int j = 0; j < NTL; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        acc[i][j][q] += cor[i][j][q];
+}
+
+// Activation and derivative of N values with one dispatch.
+template <int N>
+__device__ __forceinline__ void act_rows(int act, const float (&z)[N], float (&f)[N], float (&d)[N])
+{
+#define DPC_ACT_ROWS(A)                                                                           \
+  case A:                                                                                         \
+    _Pragma("unroll") for (int j = 0; j < N; ++j) act_both(A, z[j], f[j], d[j]);                  \
+    break;
+  switch (act)
+  {
+    DPC_ACT_ROWS(DPC_ACT_RELU)
+    DPC_ACT_ROWS(DPC_ACT_GELU)
+    DPC_ACT_ROWS(DPC_ACT_SIGMOID)
+    DPC_ACT_ROWS(DPC_ACT_ESIGMOID)
+    DPC_ACT_ROWS(DPC_ACT_TANH)
+    DPC_ACT_ROWS(DPC_ACT_HARD_TANH)
+  default:
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      f[j] = z[j], d[j] = 1.0f;
+  }
+#undef DPC_ACT_ROWS
 }
 
 __global__ void __launch_bounds__(kThreads, 1) conv_resident_kernel(const RcParams P)
@@ -165,12 +245,15 @@ __global__ void __launch_bounds__(kThreads, 1) conv_resident_kernel(const RcPara
   const int nw = P.nw;
   float* mu0 = sm + P.mu0;
   const unsigned short* T = reinterpret_cast<const unsigned short*>(sm + P.tab_at);
+  const uint2* koff = reinterpret_cast<const uint2*>(sm + P.koff_at);
   const RcTask* tasks = reinterpret_cast<const RcTask*>(sm + P.task_at);
   const unsigned short* order = reinterpret_cast<const unsigned short*>(sm + P.order_at);
   float* bias = sm + P.bias_at;
 
   for (int i = tid; i < P.table_vecs; i += kThreads)
     reinterpret_cast<int4*>(sm + P.tab_at)[i] = __ldg(reinterpret_cast<const int4*>(P.table) + i);
+  for (int i = tid; i < P.koff_vecs; i += kThreads)
+    reinterpret_cast<int4*>(sm + P.koff_at)[i] = __ldg(reinterpret_cast<const int4*>(P.koff) + i);
   for (int i = tid; i < 2 * (P.nf + P.nb); i += kThreads)
     reinterpret_cast<int4*>(sm + P.task_at)[i] = __ldg(reinterpret_cast<const int4*>(P.tasks) + i);
   for (int i = tid; i < P.nf + P.nb; i += kThreads)
@@ -233,27 +316,81 @@ __global__ void __launch_bounds__(kThreads, 1) conv_resident_kernel(const RcPara
       const float e = l == 1 ? zv - mu0[m * L.HW + q] : sm[rl[l - 1].eoff + m * L.HW + q];
       *z = zv + s_ir[l] * (dz - e);
     };
-    auto run_tile = [&](const RcTask& t, auto ntl, float& local)
+    auto run_tile = [&](const RcTask& t, auto shape, float& local)
     {
-      constexpr int NTL = decltype(ntl)::value;
-      float acc[NTL][4];
-      mma_tile<NTL>(acc, t, P.packed, T, sm, lane);
+      constexpr int MT = decltype(shape)::value / 8, NTL = decltype(shape)::value % 8;
+      float acc[MT][NTL][4];
+      mma_tile<MT, NTL>(acc, t, P.packed, T, koff, sm, lane);
+      // Addresses are worked out once per pixel and shared by the rows of the lane; the activation is
+      // dispatched once per pixel.  (One call per element took half the kernel's instructions.)
       const int l = t.what >> 2, g = lane >> 2, c = lane & 3;
-      const bool state = (t.what & 3) == OP_STATE;
-      const int M = state ? rl[l].C : rl[l].O;
+      const RcLayer& L = rl[l];
+      constexpr int ROWS = 2 * MT; // rows m0 + g + 8 r
+      if ((t.what & 3) == OP_STATE)
+      {
+        const float* err = sm + (l == 1 ? P.mu0 : rl[l - 1].eoff);
+        const float ir = s_ir[l];
+#pragma unroll
+        for (int j = 0; j < NTL; ++j)
+#pragma unroll
+          for (int b = 0; b < 2; ++b)
+          {
+            const int n = 8 * j + 2 * c + b;
+            if (n >= t.count)
+              continue;
+            const int q = T[t.ntab + 2 * n + 1];
+            float* z = sm + L.zoff + T[L.zpix + q] + (t.m0 + g) * L.zplane;
+            const float* e = err + q + (t.m0 + g) * L.HW;
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r)
+              if (t.m0 + g + 8 * r < L.C)
+              {
+                const float zv = z[8 * r * L.zplane], ev = e[8 * r * L.HW];
+                z[8 * r * L.zplane] = zv + ir * (acc[r >> 1][j][2 * (r & 1) + b] - (l == 1 ? zv - ev : ev));
+              }
+          }
+        return;
+      }
 #pragma unroll
       for (int j = 0; j < NTL; ++j)
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int b = 0; b < 2; ++b)
         {
-          const int m = t.m0 + g + (q >> 1) * 8, n = 8 * j + 2 * c + (q & 1);
-          if (m >= M || n >= t.count)
+          const int n = 8 * j + 2 * c + b;
+          if (n >= t.count)
             continue;
           const int p = T[t.ntab + 2 * n + 1];
-          if (state)
-            finish_state(l, m, p, acc[j][q]);
-          else
-            finish_forward(l, m, p, acc[j][q], local);
+          float pre[ROWS], mu[ROWS], d[ROWS];
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r)
+            pre[r] = acc[r >> 1][j][2 * (r & 1) + b] + bias[L.boff + min(t.m0 + g + 8 * r, L.O - 1)];
+          act_rows<ROWS>(s_act[l], pre, mu, d);
+          float* zu = sm + L.uoff + T[L.upix + p];
+          float* gz = sm + L.goff + (l > 0 ? T[L.gpix + p] : 0);
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r)
+          {
+            const int m = t.m0 + g + 8 * r;
+            if (m >= L.O)
+              continue;
+            if (pred)
+            {
+              const size_t o = ((size_t)img * L.O + m) * L.P + p;
+              P.layers[l].preact[o] = pre[r];
+              P.layers[l].mu[o] = mu[r];
+            }
+            if (mode == 2)
+              mu0[m * L.P + p] = mu[r];
+            else if (mode == 1)
+              zu[m * L.uplane] = mu[r];
+            else
+            {
+              const float e = zu[m * L.uplane] - mu[r];
+              sm[L.eoff + m * L.P + p] = e;
+              gz[m * L.gplane] = e * d[r];
+              local += e * e;
+            }
+          }
         }
     };
     auto run_task = [&](const RcTask& t, float& local)
@@ -306,12 +443,23 @@ __global__ void __launch_bounds__(kThreads, 1) conv_resident_kernel(const RcPara
         break;
       }
       default:
-        if (t.ntl == 4)
-          run_tile(t, std::integral_constant<int, 4>(), local);
-        else if (t.ntl == 2)
-          run_tile(t, std::integral_constant<int, 2>(), local);
-        else
-          run_tile(t, std::integral_constant<int, 1>(), local);
+        switch (t.shape)
+        {
+        case 18:
+          run_tile(t, std::integral_constant<int, 18>(), local);
+          break;
+        case 17:
+          run_tile(t, std::integral_constant<int, 17>(), local);
+          break;
+        case 12:
+          run_tile(t, std::integral_constant<int, 12>(), local);
+          break;
+        case 10:
+          run_tile(t, std::integral_constant<int, 10>(), local);
+          break;
+        default:
+          run_tile(t, std::integral_constant<int, 9>(), local);
+        }
       }
     };
     // Tasks [first, first + count) of the cost-ordered list go to whichever warp is free.
@@ -510,12 +658,12 @@ __global__ void conv_pack_kernel(const dpc_conv_layer* __restrict__ layers, cons
   {
     const int s = i >> 5, lane = i & 31, m = blockIdx.x * 16 + (lane >> 2), k = 8 * s + (lane & 3);
     const int a0 = aoff[G.aoff + k], a1 = aoff[G.aoff + k + 4];
-    float4 v;
-    v.x = a0 >= 0 && m < G.M ? W[a0 + m * G.mstride] : 0.0f;
-    v.y = a0 >= 0 && m + 8 < G.M ? W[a0 + (m + 8) * G.mstride] : 0.0f;
-    v.z = a1 >= 0 && m < G.M ? W[a1 + m * G.mstride] : 0.0f;
-    v.w = a1 >= 0 && m + 8 < G.M ? W[a1 + (m + 8) * G.mstride] : 0.0f;
-    dst[i] = v;
+    float v[4];
+    v[0] = a0 >= 0 && m < G.M ? W[a0 + m * G.mstride] : 0.0f;
+    v[1] = a0 >= 0 && m + 8 < G.M ? W[a0 + (m + 8) * G.mstride] : 0.0f;
+    v[2] = a1 >= 0 && m < G.M ? W[a1 + m * G.mstride] : 0.0f;
+    v[3] = a1 >= 0 && m + 8 < G.M ? W[a1 + (m + 8) * G.mstride] : 0.0f;
+    dst[i] = make_float4(v[0], v[1], v[2], v[3]);
   }
 }
 
@@ -525,7 +673,6 @@ struct ResState
   size_t smem = 0;
   void* dev = nullptr;
   float4* packed = nullptr;
-  dpc_conv_layer* layers = nullptr;
   RcPack* packs = nullptr;
   int* aoff = nullptr;
   int n_packs = 0, max_mblocks = 0;
@@ -545,6 +692,7 @@ struct Builder
   std::vector<RcLayer> rl;
   std::vector<RcTask> ft, bt;
   std::vector<unsigned short> table;
+  std::vector<uint2> koffs;
   std::vector<RcPack> packs;
   std::vector<int> aoff;
   size_t packed = 0; // float4s
@@ -562,7 +710,7 @@ struct Builder
   {
     RcPack g = {};
     g.layer = layer, g.M = M, g.mstride = mstride;
-    g.ks = cdiv((int)src.size(), 8), g.mblocks = cdiv(M, 16);
+    g.ks = cdiv((int)src.size(), 8 * kDepth) * kDepth, g.mblocks = M > 16 ? 2 * cdiv(M, 32) : 1;
     g.w = (int)packed, g.aoff = (int)aoff.size();
     packed += (size_t)g.mblocks * g.ks * 32;
     aoff.insert(aoff.end(), src.begin(), src.end());
@@ -575,26 +723,37 @@ struct Builder
                  const std::vector<std::pair<long long, int>>& pixels, int want)
   {
     const RcPack g = packs[pack];
-    const int ktab = (int)table.size();
-    for (long long k : koff)
-      put(k);
-    for (int k = (int)koff.size(); k < 8 * g.ks; ++k)
-      put(0);
+    const int ktab = (int)koffs.size();
+    auto offset = [&](int k) { return k < (int)koff.size() ? (unsigned)(4 * koff[k]) : 0u; };
+    for (int s = 0; s < g.ks + 2; ++s)
+      for (int c = 0; c < 4; ++c)
+        koffs.push_back(make_uint2(offset(8 * s + c), offset(8 * s + c + 4)));
     const int ntab = (int)table.size();
     for (const auto& p : pixels)
       put(p.first), put(p.second);
-    // the widest tiles that still leave `want` tasks: a wider tile re-reads the weights less often
-    int ntl = 4;
-    while (ntl > 1 && g.mblocks * cdiv((int)pixels.size(), 8 * ntl) < want)
-      ntl /= 2;
-    for (int mb = 0; mb < g.mblocks; ++mb)
-      for (int n = 0; n < (int)pixels.size(); n += 8 * ntl)
+    // the widest tiles that still leave `want` tasks: per step a 32 x 16 tile reads and splits a third
+    // of what three 16 x 8 tiles do per product
+    const int count = (int)pixels.size();
+    const int shapes[5] = {18, 12, 17, 10, 9};
+    int shape = 9;
+    for (int q : shapes)
+      if ((q < 16 || g.M > 16) && 8 * (q % 8) < count + 8 &&
+          cdiv(g.M, 16 * (q / 8)) * cdiv(count, 8 * (q % 8)) >= want)
+      {
+        shape = q;
+        break;
+      }
+    if (g.M > 16 && shape < 16 && shape != 12)
+      shape = cdiv(g.M, 32) * cdiv(count, 8) * 2 >= want ? 17 : shape;
+    const int mt = shape / 8, ntl = shape % 8;
+    for (int m = 0; m < g.M; m += 16 * mt)
+      for (int n = 0; n < count; n += 8 * ntl)
       {
         RcTask t = {};
-        t.w = g.w + mb * g.ks * 32, t.ks = g.ks;
+        t.w = g.w + m / 16 * g.ks * 32, t.ks = g.ks;
         t.ktab = ktab, t.ntab = ntab + 2 * n;
-        t.m0 = 16 * mb, t.count = std::min(8 * ntl, (int)pixels.size() - n);
-        t.ntl = ntl, t.what = what;
+        t.m0 = m, t.count = std::min(8 * ntl, count - n);
+        t.shape = shape, t.what = what;
         list.push_back(t);
       }
   }
@@ -733,7 +892,7 @@ int conv_res_init(dpc_conv_plan* p)
       for (int o = 0; o < q.O; ++o)
       {
         RcTask t = {};
-        t.m0 = o, t.count = 1, t.ks = rows / 16, t.ntl = 1, t.what = l << 2 | OP_DENSE_FORWARD;
+        t.m0 = o, t.count = 1, t.ks = rows / 16, t.shape = 9, t.what = l << 2 | OP_DENSE_FORWARD;
         B.ft.push_back(t);
       }
     else
@@ -758,7 +917,7 @@ int conv_res_init(dpc_conv_plan* p)
       for (int r = 0; r < rows; r += 128)
       {
         RcTask t = {};
-        t.m0 = r, t.count = std::min(128, rows - r), t.ks = q.O / 2, t.ntl = 1;
+        t.m0 = r, t.count = std::min(128, rows - r), t.ks = q.O / 2, t.shape = 9;
         t.what = l << 2 | OP_DENSE_STATE;
         B.bt.push_back(t);
       }
@@ -805,7 +964,10 @@ int conv_res_init(dpc_conv_plan* p)
   for (size_t i = 0; i < order.size(); ++i)
     order[i] = (unsigned short)i;
   auto longer = [&](unsigned short a, unsigned short b)
-  { return tasks[a].ks * (tasks[a].ntl + 2) > tasks[b].ks * (tasks[b].ntl + 2); };
+  {
+    auto cost = [](const RcTask& t) { return t.ks * ((t.shape / 8) * (t.shape % 8) * 3 + 2); };
+    return cost(tasks[a]) > cost(tasks[b]);
+  };
   std::stable_sort(order.begin() + B.rl[0].fcount, order.begin() + B.ft.size(), longer);
   std::stable_sort(order.begin() + B.ft.size(), order.end(), longer);
   while (B.table.size() % 8)
@@ -813,6 +975,10 @@ int conv_res_init(dpc_conv_plan* p)
   order.resize((order.size() + 7) & ~(size_t)7);
   P.tab_at = (int)at;
   at += B.table.size() / 2;
+  while (B.koffs.size() % 2)
+    B.koffs.push_back(make_uint2(0, 0));
+  P.koff_at = (int)at;
+  at += 2 * B.koffs.size();
   P.task_at = (int)at;
   at += tasks.size() * (sizeof(RcTask) / 4);
   P.order_at = (int)at;
@@ -833,30 +999,31 @@ int conv_res_init(dpc_conv_plan* p)
   };
   const size_t o_rl = put(B.rl.data(), sizeof(RcLayer) * nw), o_t = put(tasks.data(), sizeof(RcTask) * tasks.size());
   const size_t o_o = put(order.data(), 2 * order.size()), o_tab = put(B.table.data(), 2 * B.table.size());
+  const size_t o_k = put(B.koffs.data(), sizeof(uint2) * B.koffs.size());
   const size_t o_p = put(B.packs.data(), sizeof(RcPack) * B.packs.size());
   const size_t o_a = put(B.aoff.data(), sizeof(int) * B.aoff.size());
-  const size_t o_l = put(p->h.data(), sizeof(dpc_conv_layer) * p->n);
   auto* st = new ResState();
   p->res = st;
   if (cudaMalloc(&st->dev, host.size()) != cudaSuccess ||
-      cudaMalloc(&st->packed, std::max<size_t>(B.packed, 1) * sizeof(float4)) != cudaSuccess ||
+      cudaMalloc(&st->packed, (B.packed + 32 * kDepth) * sizeof(float4)) != cudaSuccess ||
       cudaMemcpy(st->dev, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess)
   {
     conv_res_free(p);
     return cuda_fail(cudaGetLastError(), "image-resident plan tables");
   }
   auto* base = static_cast<unsigned char*>(st->dev);
-  st->layers = reinterpret_cast<dpc_conv_layer*>(base + o_l);
   st->packs = reinterpret_cast<RcPack*>(base + o_p);
   st->aoff = reinterpret_cast<int*>(base + o_a);
   st->n_packs = (int)B.packs.size();
   for (const auto& g : B.packs)
     st->max_mblocks = std::max(st->max_mblocks, g.mblocks);
-  P.layers = st->layers;
+  P.layers = p->d;
   P.rl = reinterpret_cast<RcLayer*>(base + o_rl);
   P.tasks = reinterpret_cast<RcTask*>(base + o_t);
   P.order = reinterpret_cast<unsigned short*>(base + o_o);
   P.table = reinterpret_cast<unsigned short*>(base + o_tab);
+  P.koff = reinterpret_cast<uint2*>(base + o_k);
+  P.koff_vecs = (int)(B.koffs.size() / 2);
   P.packed = st->packed;
   P.nw = nw, P.batch = p->batch;
   P.nf = (int)B.ft.size(), P.nb = (int)B.bt.size();
@@ -890,7 +1057,7 @@ int dpc_conv_images_segment(dpc_conv_plan* p, int ops, int steps, int top_clampe
   cudaStream_t s = p->ctx->stream;
   if (st->n_packs > 0)
   {
-    conv::conv_pack_kernel<<<dim3(st->max_mblocks, st->n_packs, 4), 256, 0, s>>>(st->layers, st->packs, st->aoff,
+    conv::conv_pack_kernel<<<dim3(st->max_mblocks, st->n_packs, 4), 256, 0, s>>>(p->d, st->packs, st->aoff,
                                                                              st->packed);
     p->ctx->launches += 1;
   }

@@ -464,6 +464,7 @@ int dpc_plan_create(dpc_ctx* ctx, const dpc_layer* layers, int n_layers, int bat
   p->batch = batch;
   p->h.assign(layers, layers + n_layers);
   p->e_terminal = layers[n_layers - 1].e;
+  p->init_precision = ctx->precision;
   cudaError_t err = cudaMalloc(&p->d, sizeof(dpc_layer) * n_layers);
   if (err == cudaSuccess)
     err = cudaMalloc(&p->energy, sizeof(double));
@@ -497,6 +498,23 @@ int dpc_plan_update(dpc_plan* p, const dpc_layer* layers, int n_layers)
   int rc = validate_layers(layers, n_layers, p->batch);
   if (rc != DPC_OK)
     return rc;
+  // New rates only (an epoch loop with a decaying learning rate): every kernel reads them from the
+  // table, so a stream-ordered copy is all there is to do.
+  bool structure = p->init_precision != p->ctx->precision;
+  for (int i = 0; i < n_layers && !structure; ++i)
+  {
+    dpc_layer a = p->h[i], b = layers[i];
+    for (dpc_layer* q : {&a, &b})
+      q->lr = q->ir = q->fl = q->lmbda = q->psi_decay = q->momentum_beta = 0.0f;
+    structure = memcmp(&a, &b, sizeof(dpc_layer)) != 0;
+  }
+  if (!structure)
+  {
+    p->h.assign(layers, layers + n_layers);
+    DPC_CUDA(cudaMemcpyAsync(p->d, p->h.data(), sizeof(dpc_layer) * n_layers, cudaMemcpyHostToDevice,
+                             p->ctx->stream));
+    return DPC_OK;
+  }
   DPC_CUDA(cudaStreamSynchronize(p->ctx->stream));
   if (p->e_terminal == p->h[p->n - 1].e)
     p->e_terminal = layers[n_layers - 1].e;
@@ -504,6 +522,7 @@ int dpc_plan_update(dpc_plan* p, const dpc_layer* layers, int n_layers)
   DPC_CUDA(cudaMemcpy(p->d, layers, sizeof(dpc_layer) * n_layers, cudaMemcpyHostToDevice));
   tc_plan_free(p);
   res_plan_free(p);
+  p->init_precision = p->ctx->precision;
   rc = tc_plan_init(p);
   if (rc >= 0)
     rc = res_plan_init(p);

@@ -57,6 +57,7 @@ struct dpc_plan
 {
   dpc_ctx* ctx = nullptr;
   int n = 0, batch = 0;
+  int init_precision = 0; // the context's when the tensor-core and row-segment state was built
   std::vector<dpc_layer> h; // host copy of the table
   dpc_layer* d = nullptr;   // device copy
   double* energy = nullptr; // device accumulator

@@ -96,7 +96,7 @@ void SimpleConvPCNetwork::SetOptimizer(OptimizerType o)
   opt = o;
   for (auto& l : layers)
     l->d.opt = (int)o;
-  dirty = true;
+  dirty = structureDirty = true;
 }
 
 void SimpleConvPCNetwork::Compile()
@@ -190,7 +190,11 @@ void SimpleConvPCNetwork::SyncPlan()
   for (auto& l : layers)
     table.push_back(l->d);
   Check(dpc_conv_plan_update(plan, table.data(), (int)table.size()));
-  DropGraphs();
+  // a step recorded as image segments reads its rates from the plan's table; the phase kernels take
+  // the layers by value
+  if (phasesRecorded || structureDirty)
+    DropGraphs();
+  phasesRecorded = structureDirty = false;
   dirty = false;
 }
 
@@ -340,8 +344,8 @@ void SimpleConvPCNetwork::UpdateWeights()
   {
     if (layers[i]->gateIsPrediction)
       Check(dpc_conv_gate_with_prediction(plan, i));
-    Check(dpc_conv_update_weights(plan, i, centerWeights ? 1 : 0));
   }
+  Check(dpc_conv_update_weights_range(plan, 0, n - 1, centerWeights ? 1 : 0));
 }
 
 void SimpleConvPCNetwork::ProjectForward()
@@ -426,6 +430,7 @@ float SimpleConvPCNetwork::TrainStepRaw(const float* x, size_t nx, const float* 
       }
       Check(dpc_graph_end(ctx, 0));
       graphKey[0] = key;
+      phasesRecorded |= !images;
     }
     Check(dpc_graph_launch(ctx, 0));
     for (auto& l : layers)
@@ -506,6 +511,7 @@ void SimpleConvPCNetwork::PredictRaw(const float* x, size_t nx, int steps, bool 
       }
       Check(dpc_graph_end(ctx, 1));
       graphKey[1] = key;
+      phasesRecorded |= !images;
     }
     Check(dpc_graph_launch(ctx, 1));
     for (auto& l : layers)

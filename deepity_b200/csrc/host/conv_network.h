@@ -107,7 +107,7 @@ private:
   std::vector<void*> allocations;
   float *pinnedX = nullptr, *pinnedY = nullptr, *pinnedOut = nullptr;
   OptimizerType opt = OptimizerType::SGD;
-  bool centerWeights = false, useGraph = true, dirty = false;
+  bool centerWeights = false, useGraph = true, dirty = false, structureDirty = false, phasesRecorded = false;
   long graphKey[4] = {-1, -1, -1, -1};
 };
 } // namespace Deep

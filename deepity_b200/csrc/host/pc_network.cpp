@@ -368,10 +368,25 @@ void PCNetwork::Dirty()
   dirty = true;
 }
 
+void PCNetwork::RatesChanged()
+{
+  ratesDirty = true;
+}
+
 void PCNetwork::SyncPlan()
 {
-  if (!dirty || !plan)
+  if (!plan || (!dirty && !ratesDirty))
     return;
+  if (!dirty)
+  {
+    // rates live in the plan's table, which recorded steps read too
+    std::vector<dpc_layer> table;
+    for (auto& l : layers)
+      table.push_back(l->d);
+    Check(dpc_plan_update(plan, table.data(), (int)table.size()));
+    ratesDirty = false;
+    return;
+  }
   EnsureOptimizerState();
   EnsureGradientStaging();
   std::vector<dpc_layer> table;
@@ -383,7 +398,7 @@ void PCNetwork::SyncPlan()
     Check(dpc_graph_drop(ctx, s));
     graphKey[s] = -1;
   }
-  dirty = false;
+  dirty = ratesDirty = false;
 }
 
 void PCNetwork::RandomizeWeights(std::mt19937& rng, const char* distribution)
@@ -1135,26 +1150,26 @@ void PCNetwork::SetLearningRate(float lr)
 {
   for (auto& l : layers)
     l->d.lr = lr;
-  Dirty();
+  RatesChanged();
 }
 void PCNetwork::SetFeedbackRate(float fl)
 {
   for (auto& l : layers)
     l->d.fl = fl;
-  Dirty();
+  RatesChanged();
 }
 void PCNetwork::SetInferenceRate(float ir)
 {
   for (auto& l : layers)
     l->d.ir = ir;
-  Dirty();
+  RatesChanged();
 }
 void PCNetwork::SetPsiDecay(float decay)
 {
   psiDecay = decay;
   for (auto& l : layers)
     l->d.psi_decay = decay;
-  Dirty();
+  RatesChanged();
 }
 void PCNetwork::SetUseCrossEntropy(bool enabled)
 {

@@ -207,6 +207,7 @@ private:
   void Check(int rc) const;
   void RequireCompiled() const;
   void Dirty(); // hyper-parameters changed: re-upload the plan, drop captured graphs
+  void RatesChanged(); // only learning / inference / feedback rates: re-upload the plan's table
   void SyncPlan();
   void EnsureOptimizerState();
   void EnsureGradientStaging();
@@ -231,7 +232,7 @@ private:
 
   OptimizerType opt = OptimizerType::SGD, optPsi = OptimizerType::SGD;
   bool centerWeights = false, crossEntropy = false, useMuPC = false, useResidual = false;
-  bool useEPC = false, useIPC = false, useMomentum = false, useGraph = true, dirty = false;
+  bool useEPC = false, useIPC = false, useMomentum = false, useGraph = true, dirty = false, ratesDirty = false;
   bool adamAllocated = false, psiAdamAllocated = false, pendingAsync = false;
   float momentumBeta = 0.9f, psiDecay = -1.0f;
   bool ghostTop = false;

@@ -525,6 +525,8 @@ DPC_API int dpc_conv_update_state(dpc_conv_plan* plan, int layer);
 DPC_API int dpc_conv_gate_with_prediction(dpc_conv_plan* plan, int layer);
 /* UpdateWeights (SimpleConvPCLayer.cpp:402-556) + optional CenterWeights. */
 DPC_API int dpc_conv_update_weights(dpc_conv_plan* plan, int layer, int center_rows);
+/* ... of layers [first, first+count), one gradient launch and one update launch for all of them. */
+DPC_API int dpc_conv_update_weights_range(dpc_conv_plan* plan, int first, int count, int center_rows);
 /* Image segments: like dpc_rows_segment, for networks whose state of one image fits a thread block
  * (dpc_conv_images_available).  ops: FIRST, SWEEP, SWEEP_PRED, ZERO_Z, PRED_LAST, ENERGY_LAST,
  * PRED_CLOSE and STORE_Z of the DPC_ROWS_* bits; errors and gated errors of the last pass are always
