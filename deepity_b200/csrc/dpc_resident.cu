@@ -22,6 +22,10 @@
 //
 // The same tasks, i.e. the same order of additions, serve the sweep and every later pass: a belief
 // that the sweep produced has an error of exactly zero afterwards (Adam-type updates rely on it).
+// Networks with an Adam-type optimizer ("exact") go further: an update m / (sqrt(v) + eps) turns a
+// rounding difference of a near-zero gradient into a step of full size, so every sum there has ONE
+// order -- ascending, one accumulator, as the phase kernels have it -- and no slices.  So do networks
+// whose activation has a kink, where such a difference flips a derivative between 0 and 1.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -41,11 +45,14 @@ struct ResLayer // one per weight layer, built on the host
 {
   int K, N;
   int zoff, noff;    // offsets of layers l and l+1 in a row's state (multiples of 4)
-  int ldw, woff;     // row pitch and offset of W in shared memory; woff < 0: streamed
+  int ldw, woff;     // row pitch and offset of W in shared memory
+  int rrows;         // rows of W that are resident (the first ones); the others are streamed
+  int lanes_k;       // exact networks: lanes along K, the narrow heads' order of additions
   int vec;           // rows of W in global memory can be read 16 bytes at a time
   int kw;            // columns per lane of a state task: 4 or 1
   int fpart, fslice; // forward partial sums: offset, length of a slice of K
-  int bpart, bslice; // state partial sums: offset, length of a slice of the output rows
+  int bpart, bslices; // state partial sums: offset, slices of the output rows
+  int pad[2];
 };
 
 // Four neighbouring floats of a row's state (they belong to one layer).
@@ -66,11 +73,14 @@ struct __align__(16) ResTask
   int out, pitch; // first partial sum of the first row, distance to the next row's
   int lanes;      // lanes (resident forward: outputs, state: column groups) that exist
   int kind;       // layer << 4 | T_*
+  int w2, len2;   // state: streamed rows that follow the resident ones in the same sum
+  int pad[2];
 };
 enum
 {
   T_STREAM = 1, // weights in global memory
-  T_VEC = 2     // forward: rows readable 16 bytes at a time; state: 4 columns per lane
+  T_VEC = 2,    // forward: rows readable 16 bytes at a time; state: 4 columns per lane
+  T_LANES = 4   // forward: lanes along K
 };
 
 struct ResParams
@@ -87,6 +97,7 @@ struct ResParams
   int wfloats;                        // resident weights
   int groups;                         // row groups
   int ops, steps;
+  int exact;                          // one order of additions everywhere
   int simple, has_v, ce, top_clamped, top_down_off, top_n;
   double* energy;
 };
@@ -200,17 +211,53 @@ __device__ __forceinline__ void dot_resident(const float* w, const float* x, int
       out[r * pitch] = acc[r];
 }
 
-// One state task: sums over `len` rows of W for this lane's KW columns.
-template <int RT, int KW>
-__device__ __forceinline__ void state_task(const float* w, int ldw, int len, const float* g, int S,
-                                           float* out, int pitch)
+// The same for rows of W in global memory.
+template <int RT>
+__device__ __forceinline__ void dot_rows(const float* __restrict__ w, const float* x, int S, int len,
+                                         float* out, int pitch, bool valid, bool vec)
 {
-  float acc[RT][KW];
+  float acc[RT];
 #pragma unroll
   for (int r = 0; r < RT; ++r)
+    acc[r] = 0.0f;
+  int k = 0;
+  if (vec)
+  {
+#pragma unroll 8
+    for (; k < len; k += 4)
+    {
+      const float4 wv = *reinterpret_cast<const float4*>(w + k);
 #pragma unroll
-    for (int c = 0; c < KW; ++c)
-      acc[r][c] = 0.0f;
+      for (int r = 0; r < RT; ++r)
+      {
+        const float4 v = *reinterpret_cast<const float4*>(x + r * S + k);
+        acc[r] = fmaf(v.x, wv.x, acc[r]);
+        acc[r] = fmaf(v.y, wv.y, acc[r]);
+        acc[r] = fmaf(v.z, wv.z, acc[r]);
+        acc[r] = fmaf(v.w, wv.w, acc[r]);
+      }
+    }
+  }
+  else
+#pragma unroll 8
+    for (; k < len; ++k)
+    {
+      const float wv = w[k];
+#pragma unroll
+      for (int r = 0; r < RT; ++r)
+        acc[r] = fmaf(x[r * S + k], wv, acc[r]);
+    }
+  if (valid)
+#pragma unroll
+    for (int r = 0; r < RT; ++r)
+      out[r * pitch] = acc[r];
+}
+
+// One state task: sums over `len` rows of W for this lane's KW columns.
+template <int RT, int KW>
+__device__ __forceinline__ void state_sum(float (&acc)[RT][KW], const float* w, int ldw, int len,
+                                          const float* g, int S)
+{
   int n = 0;
 #pragma unroll 2
   for (; n + 4 <= len; n += 4, w += 4 * (size_t)ldw)
@@ -250,11 +297,6 @@ __device__ __forceinline__ void state_task(const float* w, int ldw, int len, con
       for (int r = 0; r < RT; ++r)
         acc[r][c] = fmaf(g[r * S + n], wv, acc[r][c]);
     }
-#pragma unroll
-  for (int r = 0; r < RT; ++r)
-#pragma unroll
-    for (int c = 0; c < KW; ++c)
-      out[r * pitch + c] = acc[r][c];
 }
 
 __device__ __forceinline__ void cp_async16(float* dst, const float* src)
@@ -377,11 +419,11 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
   for (int l = 1; l < nw; ++l)
   {
     const ResLayer L = sl[l];
-    if (L.woff < 0)
+    if (L.rrows == 0)
       continue;
     const float* src = sW[l];
     float* dst = Ws + L.woff;
-    for (int r = warp; r < L.N; r += kWarps)
+    for (int r = warp; r < L.rrows; r += kWarps)
       if (L.vec)
         for (int c = lane * 4; c < L.K; c += 128)
           cp_async16(dst + r * L.ldw + c, src + (size_t)r * L.K + c);
@@ -480,6 +522,18 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
         __syncthreads();
         float* part = X + R * P.K0p;
         const int ng = (L.N + G - 1) / G, nt = ng * P.ks0;
+        if (P.exact && !L.lanes_k)
+        {
+          // one ascending sum per output: lane = output
+          constexpr int RBS = R / RT;
+          for (int t = warp; t < (L.N + 31) / 32 * RBS; t += kWarps)
+          {
+            const int c = t / RBS * 32 + lane, rb = t % RBS * RT;
+            dot_rows<RT>(sW[0] + (size_t)min(c, L.N - 1) * L.K, X + rb * P.K0p, P.K0p, L.K,
+                         part + (c / G) * V + rb * G + c % G, G, c < L.N, L.vec != 0);
+          }
+        }
+        else
         for (int t = warp; t < nt; t += kWarps)
         {
           const int g0 = (t / P.ks0) * G, s = t % P.ks0;
@@ -533,17 +587,22 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
     {
       const float* x = (simple ? Gb : Z) + t.x;
       float* out = X + t.out;
-      if (!(t.kind & T_STREAM))
+      const bool stream = t.kind & T_STREAM;
+      if (!(t.kind & T_LANES))
       {
-        dot_resident<RT>(Ws + t.w + min(lane, t.lanes - 1) * t.ldw, x, S, t.len, out + lane, t.pitch,
-                         lane < t.lanes);
+        const int row = min(lane, t.lanes - 1) * t.ldw;
+        if (!stream)
+          dot_resident<RT>(Ws + t.w + row, x, S, t.len, out + lane, t.pitch, lane < t.lanes);
+        else
+          dot_rows<RT>(sW[t.kind >> 4] + t.w + row, x, S, t.len, out + lane, t.pitch, lane < t.lanes,
+                       (t.kind & T_VEC) != 0);
         return;
       }
       float acc[V];
 #pragma unroll
       for (int i = 0; i < V; ++i)
         acc[i] = 0.0f;
-      dot_streamed<R, G>(acc, sW[t.kind >> 4] + t.w, t.ldw, t.lanes, x, S, 0, t.len, lane,
+      dot_streamed<R, G>(acc, (stream ? sW[t.kind >> 4] : Ws) + t.w, t.ldw, t.lanes, x, S, 0, t.len, lane,
                          (t.kind & T_VEC) != 0);
       const float v = reduce_values<V>(acc, lane);
       const int idx = lane / LPV, r = idx / G, c = idx % G;
@@ -557,17 +616,24 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
         return;
       const int k = (t.kind & T_VEC) ? lane * 4 : lane;
       float* out = X + t.out + k;
-      if (!(t.kind & T_STREAM))
+      auto run = [&](auto kw)
       {
-        if (t.kind & T_VEC)
-          state_task<RT, 4>(Ws + t.w + k, t.ldw, t.len, g, S, out, t.pitch);
-        else
-          state_task<RT, 1>(Ws + t.w + k, t.ldw, t.len, g, S, out, t.pitch);
-      }
-      else if (t.kind & T_VEC)
-        state_task<RT, 4>(sW[t.kind >> 4] + t.w + k, t.ldw, t.len, g, S, out, t.pitch);
+        constexpr int KW = decltype(kw)::value;
+        float acc[RT][KW] = {};
+        if (t.len > 0)
+          state_sum<RT, KW>(acc, Ws + t.w + k, t.ldw, t.len, g, S);
+        if (t.len2 > 0)
+          state_sum<RT, KW>(acc, sW[t.kind >> 4] + t.w2 + k, sl[t.kind >> 4].K, t.len2, g + t.len, S);
+#pragma unroll
+        for (int r = 0; r < RT; ++r)
+#pragma unroll
+          for (int c = 0; c < KW; ++c)
+            out[r * t.pitch + c] = acc[r][c];
+      };
+      if (t.kind & T_VEC)
+        run(std::integral_constant<int, 4>());
       else
-        state_task<RT, 1>(sW[t.kind >> 4] + t.w + k, t.ldw, t.len, g, S, out, t.pitch);
+        run(std::integral_constant<int, 1>());
     };
     // Prediction of the four elements of quad q (layer l + 1) in row r, from the partial sums or the
     // clamped input layer's cache; padding comes out as zero.
@@ -945,7 +1011,7 @@ inline int up4(int v)
 }
 
 // Tables for groups of R rows; 1 when they do not fit the shared memory.
-int build(dpc_plan* p, int R, int S, bool has_v)
+int build(dpc_plan* p, int R, int S, bool has_v, bool exact)
 {
   const int nw = p->n - 1, G = R == 8 ? 4 : 8, RT = std::min(R, 4), rbs = R / RT;
   std::vector<ResLayer> rl(nw);
@@ -961,11 +1027,14 @@ int build(dpc_plan* p, int R, int S, bool has_v)
     off += up4(q.N);
     q.vec = L.size % 4 == 0 && ((uintptr_t)L.W % 16) == 0;
     q.ldw = up4(L.size) | 4; // 4 x odd: lanes that read 16 bytes of neighbouring rows share no bank
-    q.woff = -1;
+    q.woff = q.rrows = 0;
+    // (the shapes of the narrow forward kernel)
+    q.lanes_k = exact && q.N <= 16 && q.K % 4 == 0 && q.K >= 128 && !(L.flags & DPC_LAYER_INPUT_ACT) &&
+                ((uintptr_t)L.z % 16) == 0 && q.vec;
   }
   const int N1p = up4(rl[0].N), K0p = up4(rl[0].K), NTp = up4(rl[nw - 1].N);
   const int ng0 = (rl[0].N + G - 1) / G;
-  int ks0 = std::max(1, std::min(2 * kWarps / std::max(ng0, 1), (K0p + 127) / 128));
+  int ks0 = exact ? 1 : std::max(1, std::min(2 * kWarps / std::max(ng0, 1), (K0p + 127) / 128));
   const int kslice0 = ((K0p + ks0 - 1) / ks0 + 3) & ~3;
   ks0 = (K0p + kslice0 - 1) / kslice0;
 
@@ -982,7 +1051,7 @@ int build(dpc_plan* p, int R, int S, bool has_v)
     for (int l = 1; l < nw; ++l)
     {
       ResLayer& q = rl[l];
-      q.kw = q.K >= 96 && (q.woff >= 0 || q.vec) ? 4 : 1;
+      q.kw = q.K >= 96 && (q.rrows == q.N || q.vec) ? 4 : 1;
       fw += (double)((q.N + 31) / 32) * q.K;
       bw += (double)((q.K + 32 * q.kw - 1) / (32 * q.kw)) * q.kw * q.N;
     }
@@ -990,62 +1059,81 @@ int build(dpc_plan* p, int R, int S, bool has_v)
     {
       ResLayer& q = rl[l];
       const int np = up4(q.N), kp = up4(q.K);
-      const bool streamed = q.woff < 0;
-      ResTask t = {};
       q.fpart = (int)fparts;
-      if (!streamed)
+      int s = 1;
+      if (!exact)
       {
         const int blks = (q.N + 31) / 32;
         const double share = (double)blks * q.K / fw;
-        int s = std::max(1, std::min({(int)(kWarps * share / (blks * rbs) + 0.01), q.K / 16, 16}) >> shift);
-        q.fslice = ((q.K + s - 1) / s + 3) & ~3;
-        s = (q.K + q.fslice - 1) / q.fslice;
-        for (int rb = 0; rb < rbs; ++rb)
-          for (int k = 0; k < s; ++k)
-            for (int b = 0; b < blks; ++b)
-            {
-              t.w = q.woff + b * 32 * q.ldw + k * q.fslice, t.ldw = q.ldw;
-              t.x = q.zoff + rb * RT * S + k * q.fslice;
-              t.len = std::min(q.K - k * q.fslice, q.fslice);
-              t.out = q.fpart + (k * R + rb * RT) * np + b * 32, t.pitch = np;
-              t.lanes = std::min(32, q.N - b * 32);
-              t.kind = l << 4;
-              ft.push_back(t);
-            }
-        fparts += (size_t)s * R * np;
+        s = std::max(1, std::min({(int)(kWarps * share / (blks * rbs) + 0.01), q.K / 16, 16}) >> shift);
       }
-      else
+      q.fslice = ((q.K + s - 1) / s + 3) & ~3;
+      s = q.rrows > 0 ? (q.K + q.fslice - 1) / q.fslice : 1;
+      // forward: resident rows, then streamed ones
+      for (int part = 0; part < 2; ++part)
       {
-        q.fslice = q.K;
-        for (int b = 0; b < q.N; b += G)
-        {
-          t.w = b * q.K, t.ldw = q.K, t.x = q.zoff, t.len = q.K;
-          t.out = q.fpart + b, t.pitch = np, t.lanes = q.N - b;
-          t.kind = l << 4 | T_STREAM | (q.vec ? T_VEC : 0);
-          ft.push_back(t);
-        }
-        fparts += (size_t)R * np;
+        const int n0 = part ? q.rrows : 0, n1 = part ? q.N : q.rrows;
+        const bool lanes = q.lanes_k || (part && !exact);
+        ResTask t = {};
+        t.ldw = part ? q.K : q.ldw, t.pitch = np;
+        t.kind = l << 4 | (part ? T_STREAM : 0) | (lanes ? T_LANES : 0) | (q.vec ? T_VEC : 0);
+        if (lanes)
+          for (int b = n0; b < n1; b += G)
+          {
+            t.w = (part ? 0 : q.woff) + b * t.ldw, t.x = q.zoff, t.len = q.K;
+            t.out = q.fpart + b, t.lanes = n1 - b;
+            ft.push_back(t);
+          }
+        else
+          for (int rb = 0; rb < rbs; ++rb)
+            for (int k = 0; k < (part ? 1 : s); ++k)
+              for (int b = n0; b < n1; b += 32)
+              {
+                t.w = (part ? 0 : q.woff) + b * t.ldw + k * q.fslice;
+                t.x = q.zoff + rb * RT * S + k * q.fslice;
+                t.len = std::min(q.K - k * q.fslice, part ? q.K : q.fslice);
+                t.out = q.fpart + (k * R + rb * RT) * np + b, t.lanes = std::min(32, n1 - b);
+                ft.push_back(t);
+              }
       }
+      fparts += (size_t)s * R * np;
+      // state: slices of the resident and of the streamed rows; exact: one sum over both
       const int cols = 32 * q.kw, blks = (q.K + cols - 1) / cols;
-      const double share = (double)blks * q.kw * q.N / bw;
-      int s = std::max(1, std::min({(int)(kWarps * share / (blks * rbs) + 0.01), q.N / 8, 16}) >> shift);
-      q.bslice = ((q.N + s - 1) / s + 3) & ~3;
-      s = (q.N + q.bslice - 1) / q.bslice;
       q.bpart = (int)bparts;
+      int slice = q.N;
+      if (!exact)
+      {
+        const double share = (double)blks * q.kw * q.N / bw;
+        const int want =
+            std::max(1, std::min({(int)(kWarps * share / (blks * rbs) + 0.01), q.N / 8, 16}) >> shift);
+        slice = ((q.N + want - 1) / want + 3) & ~3;
+      }
+      std::vector<std::pair<int, int>> cuts; // row ranges
+      if (exact)
+        cuts.push_back({0, q.N});
+      else
+        for (int part = 0; part < 2; ++part)
+          for (int n = part ? q.rrows : 0; n < (part ? q.N : q.rrows); n += slice)
+            cuts.push_back({n, std::min(n + slice, part ? q.N : q.rrows)});
+      q.bslices = (int)cuts.size();
       for (int rb = 0; rb < rbs; ++rb)
-        for (int k = 0; k < s; ++k)
+        for (int k = 0; k < q.bslices; ++k)
           for (int b = 0; b < blks; ++b)
           {
-            t.ldw = streamed ? q.K : q.ldw;
-            t.w = (streamed ? 0 : q.woff) + k * q.bslice * t.ldw + b * cols;
-            t.x = q.noff + rb * RT * S + k * q.bslice;
-            t.len = std::min(q.N - k * q.bslice, q.bslice);
+            const int n0 = cuts[k].first, n1 = cuts[k].second;
+            ResTask t = {};
+            t.ldw = q.ldw;
+            t.w = q.woff + n0 * q.ldw + b * cols;
+            t.len = std::max(0, std::min(n1, q.rrows) - n0);
+            t.w2 = (n0 + t.len) * q.K + b * cols;
+            t.len2 = n1 - n0 - t.len;
+            t.x = q.noff + rb * RT * S + n0;
             t.out = q.bpart + (k * R + rb * RT) * kp + b * cols, t.pitch = kp;
             t.lanes = std::min(32, (q.K - b * cols + q.kw - 1) / q.kw);
-            t.kind = l << 4 | (streamed ? T_STREAM : 0) | (q.kw == 4 ? T_VEC : 0);
+            t.kind = l << 4 | (q.kw == 4 ? T_VEC : 0);
             bt.push_back(t);
           }
-      bparts += (size_t)s * R * kp;
+      bparts += (size_t)q.bslices * R * kp;
     }
     return std::max(fparts, bparts) * sizeof(float) <= 32 * 1024;
   };
@@ -1067,15 +1155,16 @@ int build(dpc_plan* p, int R, int S, bool has_v)
                      2 * (size_t)R * N1p + 2 * (size_t)R * NTp + x;
     return f * sizeof(float) + kStatic;
   };
-  // residency: smallest layers first, against what is left beside everything else
+  // residency: smallest layers first, against what is left beside everything else; one that does not
+  // fit whole keeps as many blocks of 32 rows as do
   for (int l = 1; l < nw; ++l)
-    rl[l].woff = 0;
+    rl[l].rrows = rl[l].N;
   fit_tasks();
   size_t o = others();
   for (int l = 1; l < nw; ++l)
-    rl[l].woff = -1;
+    rl[l].rrows = 0;
   fit_tasks();
-  o = std::max(o, others());
+  o = std::max(o, others()) + 4096; // (a layer in two parts has a few tasks and sums more)
   if (o > kSmemLimit)
     return 1;
   const size_t left = (kSmemLimit - o) / sizeof(float);
@@ -1087,9 +1176,10 @@ int build(dpc_plan* p, int R, int S, bool has_v)
             { return (size_t)rl[a].N * rl[a].ldw < (size_t)rl[b].N * rl[b].ldw; });
   for (int l : order)
   {
-    const size_t f = (size_t)rl[l].N * rl[l].ldw;
-    if (used + f <= left)
-      rl[l].woff = (int)used, used += f;
+    const int fit = (int)std::min<size_t>((left - used) / rl[l].ldw, (size_t)rl[l].N);
+    rl[l].rrows = fit == rl[l].N ? fit : fit / 32 * 32;
+    rl[l].woff = (int)used;
+    used += (size_t)rl[l].rrows * rl[l].ldw;
   }
   fit_tasks();
   o = others() + used * sizeof(float);
@@ -1106,12 +1196,15 @@ int build(dpc_plan* p, int R, int S, bool has_v)
       q.down = rl[l].zoff + c; // residual layers are square
       q.up = l + 1 < nw ? rl[l + 1].noff + c : 0;
       q.fpart = rl[l].fpart + c;
-      q.fslices = l > 0 ? (short)((rl[l].K + rl[l].fslice - 1) / rl[l].fslice) : 0;
+      // (columns of streamed rows, and heads walked along K, have one sum)
+      q.fslices = l == 0 ? 0
+                  : c < rl[l].rrows && !rl[l].lanes_k ? (short)((rl[l].K + rl[l].fslice - 1) / rl[l].fslice)
+                                                      : 1;
       if (l + 1 < nw)
       {
         const ResLayer& U = rl[l + 1];
         q.bpart = U.bpart + c;
-        q.bslices = (short)((U.N + U.bslice - 1) / U.bslice);
+        q.bslices = (short)U.bslices;
       }
     }
   std::vector<unsigned char> host(table_bytes(), 0);
@@ -1150,6 +1243,7 @@ int build(dpc_plan* p, int R, int S, bool has_v)
   P.groups = (p->batch + R - 1) / R;
   P.simple = (p->h[0].flags & DPC_LAYER_INPUT_ACT) ? 1 : 0;
   P.has_v = has_v ? 1 : 0;
+  P.exact = exact ? 1 : 0;
   P.energy = p->energy;
   st->R = R;
   st->smem = o;
@@ -1180,10 +1274,12 @@ int res_plan_init(dpc_plan* p)
     return 1;
   size_t wbytes = 0;
   int S = 0;
-  bool has_v = false;
+  bool has_v = false, exact = false;
   for (int l = 0; l < nw; ++l)
   {
     const dpc_layer& L = p->h[l];
+    exact |= L.opt != DPC_OPT_SGD || (L.Psi && L.opt_psi != DPC_OPT_SGD) || L.act == DPC_ACT_RELU ||
+             L.act == DPC_ACT_HARD_TANH;
     if (L.next_size <= 0 || L.next_size > 8192 || (l > 0 && L.size > 16384) ||
         ((L.flags ^ p->h[0].flags) & DPC_LAYER_INPUT_ACT) || (l == 0 && (L.flags & DPC_LAYER_RESIDUAL)))
       return 1;
@@ -1204,7 +1300,7 @@ int res_plan_init(dpc_plan* p)
     R *= 2;
   for (; R >= 1; R /= 2)
   {
-    const int rc = build(p, R, S, has_v);
+    const int rc = build(p, R, S, has_v, exact);
     if (rc <= 0)
       return rc;
   }
