@@ -1,5 +1,6 @@
 // Context, memory, CUDA graphs, plans and the phase entry points of the dpc_* C ABI.
 #include <cstdio>
+#include <functional>
 #include <cstring>
 #include <string>
 
@@ -639,6 +640,17 @@ static FePlanes fe_planes(dpc_plan* p)
   return P;
 }
 
+// Whether the layer's forward pass runs on the narrow-head kernel: at most 16 output units and rows
+// that can be read 16 bytes at a time.
+static bool narrow_forward(const dpc_plan* p, int layer)
+{
+  const dpc_layer& L = p->h[layer];
+  return L.next_size > 0 && L.next_size <= 16 && L.size % 4 == 0 && L.size >= 128 && ((uintptr_t)L.z % 16) == 0 &&
+         ((uintptr_t)L.W % 16) == 0 &&
+         // SimplePC layers under an Adam-type optimizer keep the grouped kernel's order of additions
+         (!(L.flags & DPC_LAYER_INPUT_ACT) || (L.opt == DPC_OPT_SGD && ((uintptr_t)L.zF % 16) == 0));
+}
+
 static int forward_simt(dpc_plan* p, int first, int count, int flags)
 {
   cudaStream_t st = p->ctx->stream;
@@ -662,14 +674,7 @@ static int forward_simt(dpc_plan* p, int first, int count, int flags)
       // heads (at most 16 output units) with vector-loadable rows: one warp per batch row
       bool narrow = true;
       for (int i = f; i < f + c && narrow; ++i)
-      {
-        const dpc_layer& L = p->h[i];
-        if (L.next_size <= 0)
-          continue;
-        narrow = L.next_size <= 16 && L.size % 4 == 0 && L.size >= 128 &&
-                 !(L.flags & DPC_LAYER_INPUT_ACT) && ((uintptr_t)L.z % 16) == 0 &&
-                 ((uintptr_t)L.W % 16) == 0;
-      }
+        narrow = p->h[i].next_size <= 0 || narrow_forward(p, i);
       if (narrow)
       {
         if (p->batch >= 2048)
@@ -701,85 +706,98 @@ static int forward_simt(dpc_plan* p, int first, int count, int flags)
   return DPC_OK;
 }
 
+// Runs the jobs side by side: job 0 (the largest, by convention) on the context's stream, the others
+// on up to three streams that fork from it and join it (inside a graph capture: parallel branches).
+// The launches of one phase are independent of each other, and most of them leave SMs idle -- a head,
+// a cached input layer, a bias sum beside the tensor-core run -- so one after the other they would add
+// their latencies.
+using Job = std::function<int()>;
+static int run_side_by_side(dpc_ctx* ctx, const std::vector<Job>& jobs)
+{
+  int rc = DPC_OK;
+  if (jobs.size() < 2 || !ctx->fork_ev)
+  {
+    for (size_t q = 0; q < jobs.size() && rc == DPC_OK; ++q)
+      rc = jobs[q]();
+    return rc;
+  }
+  cudaStream_t main_stream = ctx->stream;
+  const int used = std::min((int)jobs.size() - 1, dpc_ctx::kSide);
+  bool forked = cudaEventRecord(ctx->fork_ev, main_stream) == cudaSuccess;
+  for (int s = 0; s < used && forked; ++s)
+    forked = cudaStreamWaitEvent(ctx->side[s], ctx->fork_ev, 0) == cudaSuccess;
+  if (!forked)
+    return cuda_fail(cudaGetLastError(), "fork of the per-layer streams");
+  for (size_t q = 0; q < jobs.size() && rc == DPC_OK; ++q)
+  {
+    const int lane = (int)q % (used + 1);
+    ctx->stream = lane == 0 ? main_stream : ctx->side[lane - 1];
+    rc = jobs[q]();
+  }
+  ctx->stream = main_stream;
+  // join whatever happened: a capture must not end with a stream still forked
+  bool joined = true;
+  for (int s = 0; s < used; ++s)
+    joined &= cudaEventRecord(ctx->join_ev[s], ctx->side[s]) == cudaSuccess &&
+              cudaStreamWaitEvent(main_stream, ctx->join_ev[s], 0) == cudaSuccess;
+  if (rc != DPC_OK)
+    return rc;
+  return joined ? DPC_OK : cuda_fail(cudaGetLastError(), "join of the per-layer streams");
+}
+
 // Splits [first, first+count) into what the tensor-core path takes (the part inside the run as
 // one piece, single layers outside it that fit the CTA-pair kernels one by one) and maximal
 // pieces for the CUDA-core kernels.  A piece the tensor-core entry point declines (returns 1)
-// goes to the CUDA-core kernels too.
-// `independent`: the layers of the range neither read what another layer of the range writes nor
-// write the same tensors (true of a settle pass, a state update and a weight update; not of a
-// sweep).  Consecutive single layers on the tensor cores then go to up to four streams that fork
-// from and join the context's stream (inside a graph capture: parallel branches), because one such
-// layer alone fills only a part of the GPU.
+// goes to the CUDA-core kernels too.  run_first: the run comes first in the list.
 template <typename TcFn, typename SimtFn>
-static int dispatch_range(dpc_plan* p, int first, int count, TcFn tc, SimtFn simt,
-                          bool independent = false)
+static std::vector<Job> pieces_of(dpc_plan* p, int first, int count, TcFn tc, SimtFn simt, bool run_first)
 {
   const int end = first + count;
   const int run0 = p->run.first, run1 = p->run.first + p->run.count;
-  dpc_ctx* ctx = p->ctx;
+  std::vector<Job> jobs;
   int i = first;
   while (i < end)
   {
-    int j, rc;
-    if (independent && ctx->fork_ev && tc_extra_layer(p, i) && i + 1 < end &&
-        tc_extra_layer(p, i + 1))
+    int j = i + 1;
+    const bool in_run = p->run.count > 0 && i >= run0 && i < run1;
+    if (in_run || tc_extra_layer(p, i))
     {
-      j = i + 2;
-      while (j < end && tc_extra_layer(p, j))
-        ++j;
-      cudaStream_t main_stream = ctx->stream;
-      const int used = std::min(j - i - 1, dpc_ctx::kSide);
-      bool forked = cudaEventRecord(ctx->fork_ev, main_stream) == cudaSuccess;
-      for (int s = 0; s < used && forked; ++s)
-        forked = cudaStreamWaitEvent(ctx->side[s], ctx->fork_ev, 0) == cudaSuccess;
-      if (!forked)
-        return cuda_fail(cudaGetLastError(), "fork of the per-layer streams");
-      rc = DPC_OK;
-      for (int q = i; q < j && rc == DPC_OK; ++q)
+      if (in_run)
+        j = std::min(end, run1);
+      Job job = [=]
       {
-        const int lane = (q - i) % (used + 1);
-        ctx->stream = lane == 0 ? main_stream : ctx->side[lane - 1];
-        rc = tc(q, 1);
-        if (rc > 0)
-          rc = simt(q, 1);
-      }
-      ctx->stream = main_stream;
-      // join whatever happened: a capture must not end with a stream still forked
-      bool joined = true;
-      for (int s = 0; s < used; ++s)
-        joined &= cudaEventRecord(ctx->join_ev[s], ctx->side[s]) == cudaSuccess &&
-                  cudaStreamWaitEvent(main_stream, ctx->join_ev[s], 0) == cudaSuccess;
-      if (rc != DPC_OK)
-        return rc;
-      if (!joined)
-        return cuda_fail(cudaGetLastError(), "join of the per-layer streams");
-      i = j;
-      continue;
-    }
-    if (p->run.count > 0 && i >= run0 && i < run1)
-    {
-      j = std::min(end, run1);
-      rc = tc(i, j - i);
-    }
-    else if (tc_extra_layer(p, i))
-    {
-      j = i + 1;
-      rc = tc(i, 1);
+        const int rc = tc(i, j - i);
+        return rc > 0 ? simt(i, j - i) : rc;
+      };
+      if (in_run && run_first)
+        jobs.insert(jobs.begin(), job);
+      else
+        jobs.push_back(job);
     }
     else
     {
-      j = i + 1;
       while (j < end && !(p->run.count > 0 && j >= run0 && j < run1) && !tc_extra_layer(p, j))
         ++j;
-      rc = 1;
+      jobs.push_back([=] { return simt(i, j - i); });
     }
-    if (rc < 0)
-      return rc;
-    if (rc != DPC_OK && (rc = simt(i, j - i)) != DPC_OK)
-      return rc;
     i = j;
   }
-  return DPC_OK;
+  return jobs;
+}
+
+// `independent`: the layers of the range neither read what another layer of the range writes nor
+// write the same tensors (true of a settle pass, a state update and a weight update; not of a
+// sweep): the pieces run side by side.
+template <typename TcFn, typename SimtFn>
+static int dispatch_range(dpc_plan* p, int first, int count, TcFn tc, SimtFn simt, bool independent = false)
+{
+  const std::vector<Job> jobs = pieces_of(p, first, count, tc, simt, independent);
+  if (independent)
+    return run_side_by_side(p->ctx, jobs);
+  int rc = DPC_OK;
+  for (size_t q = 0; q < jobs.size() && rc == DPC_OK; ++q)
+    rc = jobs[q]();
+  return rc;
 }
 
 int dpc_forward(dpc_plan* p, int first, int count, int flags)
@@ -789,10 +807,36 @@ int dpc_forward(dpc_plan* p, int first, int count, int flags)
     return rc;
   if (flags & DPC_FWD_CACHED)
     return forward_simt(p, first, count, flags);
-  return dispatch_range(
-      p, first, count, [&](int f, int c) { return tc_forward(p, f, c, flags); },
-      [&](int f, int c) { return forward_simt(p, f, c, flags); },
-      /*independent=*/!(flags & DPC_FWD_COPY_NEXT));
+  const bool cached_first = (flags & DPC_FWD_CACHED_FIRST) && count > 0;
+  flags &= ~DPC_FWD_CACHED_FIRST;
+  const bool independent = !(flags & DPC_FWD_COPY_NEXT);
+  const int skip = cached_first ? 1 : 0;
+  std::vector<Job> jobs = pieces_of(
+      p, first + skip, count - skip, [=](int f, int c) { return tc_forward(p, f, c, flags); },
+      [=](int f, int c) { return forward_simt(p, f, c, flags); }, independent);
+  if (cached_first)
+  {
+    const Job cached = [=] { return forward_simt(p, first, 1, flags | DPC_FWD_CACHED); };
+    // beside the others; in a sweep before them
+    jobs.insert(independent ? jobs.end() : jobs.begin(), cached);
+  }
+  if (independent)
+    return run_side_by_side(p->ctx, jobs);
+  for (size_t q = 0; q < jobs.size() && rc == DPC_OK; ++q)
+    rc = jobs[q]();
+  return rc;
+}
+
+int dpc_plan_fused_cross_entropy(dpc_plan* p)
+{
+  if (!p || p->n < 2 || !(p->h[p->n - 1].flags & DPC_LAYER_SOFTMAX_CE))
+    return 0;
+  const int head = p->n - 2;
+  auto tensor = [&](int l)
+  { return (p->run.count > 0 && l >= p->run.first && l < p->run.first + p->run.count) || tc_extra_layer(p, l); };
+  // the head must be a launch of its own: above the (clamped, separate) input layer or a tensor-core
+  // layer, else it shares the grouped launch of the layers below it
+  return head >= 1 && narrow_forward(p, head) && !tensor(head) && (head == 1 || tensor(head - 1)) ? 1 : 0;
 }
 
 int dpc_project_forward(dpc_plan* p, int first, int count, int skip_last_copy)
@@ -966,12 +1010,22 @@ static int update_state_simt(dpc_plan* p, int first, int count)
 
 int dpc_update_state(dpc_plan* p, int first, int count)
 {
+  return dpc_update_state_ex(p, first, count, first + count);
+}
+
+int dpc_update_state_ex(dpc_plan* p, int first, int count, int relax_from)
+{
   int rc = check_range(p, first, count);
   if (rc != DPC_OK)
     return rc;
-  return dispatch_range(
-      p, first, count, [&](int f, int c) { return tc_update_state(p, f, c); },
-      [&](int f, int c) { return update_state_simt(p, f, c); }, /*independent=*/true);
+  const int end = first + count;
+  relax_from = std::min(std::max(relax_from, first), end);
+  std::vector<Job> jobs = pieces_of(
+      p, first, relax_from - first, [=](int f, int c) { return tc_update_state(p, f, c); },
+      [=](int f, int c) { return update_state_simt(p, f, c); }, true);
+  for (int i = relax_from; i < end; ++i)
+    jobs.push_back([=] { return dpc_relax(p, i); });
+  return run_side_by_side(p->ctx, jobs);
 }
 
 int dpc_epc_reconstruct(dpc_plan* p, int layer)
@@ -1077,9 +1131,9 @@ static int weight_gemm_simt(dpc_plan* p, int first, int count, int mode, int fla
 
 // The DFA projection over layers [first, first+count): four-units-per-thread kernel where the
 // shapes allow it, the general kernel elsewhere.
+static int launch_dfa_group(dpc_plan* p, int i, int c, int from_output, bool v, const FePlanes& planes);
 static int launch_dfa_proj(dpc_plan* p, int first, int count, int from_output)
 {
-  cudaStream_t st = p->ctx->stream;
   wrote(p, K_FE, first, count);
   const FePlanes planes = fe_planes(p);
   auto vec_ok = [&](int i)
@@ -1089,6 +1143,7 @@ static int launch_dfa_proj(dpc_plan* p, int first, int count, int from_output)
            ((uintptr_t)L.fe % 16 == 0) && ((uintptr_t)L.preact % 16 == 0) &&
            (i + 1 >= p->n || (uintptr_t)p->h[i + 1].z % 16 == 0);
   };
+  std::vector<Job> jobs;
   int i = first;
   while (i < first + count)
   {
@@ -1098,52 +1153,65 @@ static int launch_dfa_proj(dpc_plan* p, int first, int count, int from_output)
            (!v || p->h[j].terminal_size == p->h[i].terminal_size))
       ++j;
     const int c = j - i;
-    int mxn = 1;
+    // (the layer under the terminal has no feedback weights above it: nothing to do)
+    bool any = false;
     for (int k = i; k < j; ++k)
-      mxn = std::max(mxn, p->h[k].next_size);
-    bool wide = v;
-    for (int k = i; k < j && wide; ++k)
-      wide = p->h[k].next_size <= 0 || p->h[k].next_size % 128 == 0;
-    const int ts4 = cdiv(std::max(p->h[i].terminal_size, 1), 4);
-    if (wide && ts4 <= 4 && cdiv(mxn, 128) * c >= 2 * p->ctx->sm_count)
-    {
-      // blocks of 128 columns x the whole batch
-      dim3 grid(cdiv(mxn, 128), c);
-      if (ts4 <= 1)
-        dfa_proj128_kernel<1><<<grid, 256, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, planes);
-      else if (ts4 == 2)
-        dfa_proj128_kernel<2><<<grid, 256, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, planes);
-      else if (ts4 == 3)
-        dfa_proj128_kernel<3><<<grid, 256, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, planes);
-      else
-        dfa_proj128_kernel<4><<<grid, 256, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, planes);
-    }
-    else if (v)
-    {
-      const int rpb =
-          cdiv(mxn, 256) * cdiv(p->batch, DFA4_ROWS) * c >= 4 * p->ctx->sm_count ? DFA4_ROWS : 32;
-      dim3 grid(cdiv(mxn, 256), cdiv(p->batch, rpb), c);
-      if (ts4 <= 1)
-        dfa_proj4_kernel<1><<<grid, 64, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, rpb, planes);
-      else if (ts4 == 2)
-        dfa_proj4_kernel<2><<<grid, 64, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, rpb, planes);
-      else if (ts4 == 3)
-        dfa_proj4_kernel<3><<<grid, 64, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, rpb, planes);
-      else
-        dfa_proj4_kernel<4><<<grid, 64, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, rpb, planes);
-    }
-    else
-    {
-      dim3 grid(cdiv(mxn, 128), cdiv(p->batch, DFA_ROWS), c);
-      dfa_proj_kernel<<<grid, 128, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output);
-    }
-    int rc = check_launch(p->ctx, "dfa_proj kernel");
-    if (rc != DPC_OK)
-      return rc;
-    if (v && planes.fe)
-      tc_fe_written(p, i, c); // this kernel wrote the operand copies itself
+      any |= p->h[k].next_size > 0 && k + 1 < p->n && p->h[k + 1].Psi != nullptr;
+    if (any)
+      jobs.push_back([=] { return launch_dfa_group(p, i, c, from_output, v, planes); });
     i = j;
   }
+  return run_side_by_side(p->ctx, jobs);
+}
+
+static int launch_dfa_group(dpc_plan* p, int i, int c, int from_output, bool v, const FePlanes& planes)
+{
+  cudaStream_t st = p->ctx->stream;
+  const int j = i + c;
+  int mxn = 1;
+  for (int k = i; k < j; ++k)
+    mxn = std::max(mxn, p->h[k].next_size);
+  bool wide = v;
+  for (int k = i; k < j && wide; ++k)
+    wide = p->h[k].next_size <= 0 || p->h[k].next_size % 128 == 0;
+  const int ts4 = cdiv(std::max(p->h[i].terminal_size, 1), 4);
+  if (wide && ts4 <= 4 && cdiv(mxn, 128) * c >= 2 * p->ctx->sm_count)
+  {
+    // blocks of 128 columns x the whole batch
+    dim3 grid(cdiv(mxn, 128), c);
+    if (ts4 <= 1)
+      dfa_proj128_kernel<1><<<grid, 256, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, planes);
+    else if (ts4 == 2)
+      dfa_proj128_kernel<2><<<grid, 256, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, planes);
+    else if (ts4 == 3)
+      dfa_proj128_kernel<3><<<grid, 256, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, planes);
+    else
+      dfa_proj128_kernel<4><<<grid, 256, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, planes);
+  }
+  else if (v)
+  {
+    const int rpb =
+        cdiv(mxn, 256) * cdiv(p->batch, DFA4_ROWS) * c >= 4 * p->ctx->sm_count ? DFA4_ROWS : 32;
+    dim3 grid(cdiv(mxn, 256), cdiv(p->batch, rpb), c);
+    if (ts4 <= 1)
+      dfa_proj4_kernel<1><<<grid, 64, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, rpb, planes);
+    else if (ts4 == 2)
+      dfa_proj4_kernel<2><<<grid, 64, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, rpb, planes);
+    else if (ts4 == 3)
+      dfa_proj4_kernel<3><<<grid, 64, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, rpb, planes);
+    else
+      dfa_proj4_kernel<4><<<grid, 64, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, rpb, planes);
+  }
+  else
+  {
+    dim3 grid(cdiv(mxn, 128), cdiv(p->batch, DFA_ROWS), c);
+    dfa_proj_kernel<<<grid, 128, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output);
+  }
+  int rc = check_launch(p->ctx, "dfa_proj kernel");
+  if (rc != DPC_OK)
+    return rc;
+  if (v && planes.fe)
+    tc_fe_written(p, i, c); // this kernel wrote the operand copies itself
   return DPC_OK;
 }
 
@@ -1202,6 +1270,23 @@ static int launch_psi_update(dpc_plan* p, int f, int c, int max_size, int grad_o
   return check_launch(p->ctx, grad_only ? "psi gradient kernel" : "psi_update kernel");
 }
 
+// Bias update (or its raw sums) of layers [f, f+c).
+static int launch_bias_update(dpc_plan* p, int f, int c, int max_next, int grad_only)
+{
+  const int rc = tc_fe_need(p, f, c);
+  if (rc != DPC_OK)
+    return rc;
+  const FePlanes fp = fe_planes(p);
+  // 256 threads: blocks of 64 columns where the feedback error is read from its planes,
+  // one column per thread (grid-stride) elsewhere
+  const bool by_blocks = fp.only || p->batch >= kBiasBlockRows;
+  dim3 gb(std::max(1, cdiv(max_next, by_blocks ? 64 : 256)), c);
+  launch_row_split(bias_update_kernel, gb, 256,
+                   by_blocks ? row_split(p->ctx, (long long)gb.x * c, p->batch, 256) : 1, p->ctx->stream, p->d,
+                   f, p->n, p->batch, grad_only, fp);
+  return check_launch(p->ctx, "bias_update kernel");
+}
+
 int dpc_update_weights(dpc_plan* p, int first, int count, int center_rows)
 {
   int rc = check_range(p, first, count);
@@ -1211,7 +1296,6 @@ int dpc_update_weights(dpc_plan* p, int first, int count, int center_rows)
     count -= 1;
   if (count <= 0)
     return DPC_OK;
-  cudaStream_t st = p->ctx->stream;
   bool any_adam = false, any_psi = false;
   int max_next = 0, max_size = 0;
   for (int i = first; i < first + count; ++i)
@@ -1224,13 +1308,16 @@ int dpc_update_weights(dpc_plan* p, int first, int count, int center_rows)
   }
   if (any_adam)
   {
-    bump_counters_kernel<<<cdiv(count, 256), 256, 0, st>>>(p->d, first, count, p->n);
+    bump_counters_kernel<<<cdiv(count, 256), 256, 0, p->ctx->stream>>>(p->d, first, count, p->n);
     if ((rc = check_launch(p->ctx, "bump_counters kernel")) != DPC_OK)
       return rc;
   }
-  rc = dispatch_range(
+  // the feedback-error planes are read by two of the jobs below: bring them up to date before the fork
+  if ((rc = tc_fe_need(p, first, count)) != DPC_OK)
+    return rc;
+  std::vector<Job> jobs = pieces_of(
       p, first, count,
-      [&](int f, int c) -> int
+      [=](int f, int c) -> int
       {
         bool all_sgd = true, all_staged = true;
         for (int i = f; i < f + c; ++i)
@@ -1261,37 +1348,24 @@ int dpc_update_weights(dpc_plan* p, int first, int count, int center_rows)
         }
         return DPC_OK;
       },
-      [&](int f, int c) { return weight_gemm_simt(p, f, c, WG_LEARN, 0); }, /*independent=*/true);
-  if (rc != DPC_OK)
-    return rc;
+      [=](int f, int c) { return weight_gemm_simt(p, f, c, WG_LEARN, 0); }, true);
   for (int f = first; f < first + count; f += kMaxZ)
   {
     const int c = std::min(kMaxZ, first + count - f);
-    if ((rc = tc_fe_need(p, f, c)) != DPC_OK)
-      return rc;
-    const FePlanes fp = fe_planes(p);
-    // 256 threads: blocks of 64 columns where the feedback error is read from its planes,
-    // one column per thread (grid-stride) elsewhere
-    const bool by_blocks = fp.only || p->batch >= kBiasBlockRows;
-    dim3 gb(std::max(1, cdiv(max_next, by_blocks ? 64 : 256)), c);
-    launch_row_split(bias_update_kernel, gb, 256,
-                     by_blocks ? row_split(p->ctx, (long long)gb.x * c, p->batch, 256) : 1, st, p->d,
-                     f, p->n, p->batch, 0, fp);
-    if ((rc = check_launch(p->ctx, "bias_update kernel")) != DPC_OK)
-      return rc;
+    jobs.push_back([=] { return launch_bias_update(p, f, c, max_next, 0); });
     if (any_psi)
-    {
-      if ((rc = launch_psi_update(p, f, c, max_size, 0)) != DPC_OK)
-        return rc;
-    }
-    if (center_rows)
-    {
-      dim3 gc(std::min(max_next, 1024), c);
-      wrote(p, K_W, f, c);
-      center_rows_kernel<<<gc, 256, 0, st>>>(p->d, f, p->n);
-      if ((rc = check_launch(p->ctx, "center_rows kernel")) != DPC_OK)
-        return rc;
-    }
+      jobs.push_back([=] { return launch_psi_update(p, f, c, max_size, 0); });
+  }
+  if ((rc = run_side_by_side(p->ctx, jobs)) != DPC_OK)
+    return rc;
+  for (int f = first; center_rows && f < first + count; f += kMaxZ)
+  {
+    const int c = std::min(kMaxZ, first + count - f);
+    dim3 gc(std::min(max_next, 1024), c);
+    wrote(p, K_W, f, c);
+    center_rows_kernel<<<gc, 256, 0, p->ctx->stream>>>(p->d, f, p->n);
+    if ((rc = check_launch(p->ctx, "center_rows kernel")) != DPC_OK)
+      return rc;
   }
   return DPC_OK;
 }
@@ -1352,15 +1426,7 @@ int dpc_weight_gradients(dpc_plan* p, int first, int count, int which)
   for (int f = first; f < first + count; f += kMaxZ)
   {
     const int c = std::min(kMaxZ, first + count - f);
-    if ((rc = tc_fe_need(p, f, c)) != DPC_OK)
-      return rc;
-    const FePlanes fp = fe_planes(p);
-    const bool by_blocks = fp.only || p->batch >= kBiasBlockRows;
-    dim3 gb(std::max(1, cdiv(max_next, by_blocks ? 64 : 256)), c);
-    launch_row_split(bias_update_kernel, gb, 256,
-                     by_blocks ? row_split(p->ctx, (long long)gb.x * c, p->batch, 256) : 1, st, p->d,
-                     f, p->n, p->batch, 1, fp);
-    if ((rc = check_launch(p->ctx, "bias gradient kernel")) != DPC_OK)
+    if ((rc = launch_bias_update(p, f, c, max_next, 1)) != DPC_OK)
       return rc;
     if (any_psi)
     {

@@ -204,6 +204,7 @@ __global__ void __launch_bounds__(NTHREADS)
   if (L.next_size <= 0)
     return;
   const int N = L.next_size, K = L.size;
+  const bool simple = (L.flags & DPC_LAYER_INPUT_ACT) != 0;
   const dpc_layer* Lup = (li + 1 < n_layers) ? &layers[li + 1] : nullptr;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = (blockIdx.x * (NTHREADS / 32) + warp) * RPW;
@@ -231,6 +232,30 @@ __global__ void __launch_bounds__(NTHREADS)
           zv[r][i] = (m0 + r < batch && k0 + i * 128 < K)
                          ? *reinterpret_cast<const float4*>(zrow + k0 + i * 128)
                          : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      }
+      if (simple)
+      {
+        // the operand is f(z), kept for the weight update (src/layers/SimplePCLayer.cpp:146-150)
+#pragma unroll
+        for (int r = 0; r < RPW; ++r)
+#pragma unroll
+          for (int i = 0; i < 8; i += 2)
+          {
+            const float in[8] = {zv[r][i].x,     zv[r][i].y,     zv[r][i].z,     zv[r][i].w,
+                                 zv[r][i + 1].x, zv[r][i + 1].y, zv[r][i + 1].z, zv[r][i + 1].w};
+            float f[8], d[8];
+            act_both8<false>(L.act, in, f, d);
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+            {
+              const int k = k0 + (i + q) * 128;
+              const bool in_range = m0 + r < batch && k < K;
+              zv[r][i + q] = in_range ? make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3])
+                                      : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+              if (in_range)
+                *reinterpret_cast<float4*>(L.zF + (size_t)(m0 + r) * K + k) = zv[r][i + q];
+            }
+          }
       }
 #pragma unroll
       for (int j = 0; j < 16; ++j)
@@ -261,25 +286,31 @@ __global__ void __launch_bounds__(NTHREADS)
   float esum = 0.0f;
   const bool next_ce = Lup && (Lup->flags & DPC_LAYER_SOFTMAX_CE);
   const bool do_err = (flags & DPC_FWD_ERR_NEXT) && Lup && !next_ce;
-  const bool do_fe = (flags & DPC_FWD_FE) && Lup && !(next_ce && (flags & DPC_FWD_ERR_NEXT));
+  const bool do_fe =
+      (flags & DPC_FWD_FE) && Lup && !simple && !(next_ce && (flags & DPC_FWD_ERR_NEXT));
   const bool do_copy = (flags & DPC_FWD_COPY_NEXT) && Lup;
+  const bool do_ce = next_ce && (flags & DPC_FWD_ERR_NEXT) && (flags & DPC_FWD_CE);
 #pragma unroll
   for (int r = 0; r < RPW; ++r)
   {
     // lanes 2n and 2n+1 end with the sum of output unit n; the even one finishes it
     const float mine = warp_reduce16(acc[r], lane);
     const int m = m0 + r, n = lane >> 1;
+    float out_pre = 0.0f, out_mu = 0.0f;
     if (m < batch && !(lane & 1) && n < N)
     {
       const size_t o = (size_t)m * N + n;
       const float pre = L.a * mine + L.b[n];
       float mu, d = 1.0f;
-      if (do_fe)
+      if (simple)
+        mu = pre;
+      else if (do_fe)
         act_both(L.act, pre, mu, d);
       else
         mu = act_fwd(L.act, pre);
-      if (L.flags & DPC_LAYER_RESIDUAL)
+      if (!simple && (L.flags & DPC_LAYER_RESIDUAL))
         mu += L.z[o];
+      out_pre = pre, out_mu = mu;
       if (!(flags & DPC_FWD_TRANSIENT))
       {
         const bool no_mu = do_copy && (flags & DPC_FWD_NO_MU);
@@ -302,9 +333,36 @@ __global__ void __launch_bounds__(NTHREADS)
       if (do_fe)
         L.fe[o] = e * d;
     }
+    if (do_ce)
+    {
+      // Softmax cross-entropy error of the layer above (softmax_ce_kernel and feedback_error_kernel in
+      // their order of operations): unit j moves to lane j.
+      const float logit = __shfl_sync(0xffffffffu, out_mu, 2 * lane & 31);
+      const float pre = __shfl_sync(0xffffffffu, out_pre, 2 * lane & 31);
+      const bool in = lane < N;
+      float mx = in ? logit : -INFINITY;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      float s = in ? expf(logit - mx) : 0.0f;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (in && m < batch)
+      {
+        const size_t o = (size_t)m * N + lane;
+        const float p = expf(logit - mx) / s;
+        const float z = do_copy ? logit : Lup->z[o];
+        esum -= 2.0f * z * logf(p + 1e-8f); // (halved with the Gaussian energies)
+        const float e = z - p;
+        Lup->e[o] = e;
+        if ((flags & DPC_FWD_FE) && !simple)
+          L.fe[o] = e * act_deriv(L.act, pre);
+      }
+    }
   }
   if (flags & DPC_FWD_ENERGY)
-    block_energy_add(do_err ? esum : 0.0f, energy);
+    block_energy_add(do_err || do_ce ? esum : 0.0f, energy);
 }
 
 // ---------------------------------------------------------------------------------------

@@ -532,6 +532,12 @@ void PCNetwork::ForwardRange(int first, int count, int flags)
 {
   int i = first;
   const int end = first + count;
+  auto run_end = [&](int j)
+  {
+    while (j < end && layers[j]->d.next_size > 0 && !layers[j]->clamped)
+      ++j;
+    return j;
+  };
   while (i < end)
   {
     PCLayer* l = layers[i].get();
@@ -542,10 +548,14 @@ void PCNetwork::ForwardRange(int first, int count, int flags)
     }
     if (l->clamped && l->cacheValid)
     {
-      // Nothing to do when neither the copy, the error nor fe is wanted.
+      // Nothing to do when neither the copy, the error nor fe is wanted; else one call with the
+      // layers above it.
+      const int j = run_end(i + 1);
       if (flags & (DPC_FWD_COPY_NEXT | DPC_FWD_ERR_NEXT | DPC_FWD_FE | DPC_FWD_ENERGY))
-        Check(dpc_forward(plan, i, 1, flags | DPC_FWD_CACHED));
-      ++i;
+        Check(dpc_forward(plan, i, j - i, flags | DPC_FWD_CACHED_FIRST));
+      else if (j > i + 1)
+        Check(dpc_forward(plan, i + 1, j - i - 1, flags));
+      i = j;
       continue;
     }
     if (l->clamped)
@@ -557,9 +567,7 @@ void PCNetwork::ForwardRange(int first, int count, int flags)
       ++i;
       continue;
     }
-    int j = i;
-    while (j < end && layers[j]->d.next_size > 0 && !layers[j]->clamped)
-      ++j;
+    const int j = run_end(i);
     Check(dpc_forward(plan, i, j - i, flags));
     i = j;
   }
@@ -646,8 +654,10 @@ float PCNetwork::CalculateState(bool needEnergy)
   // and its predictions are written only if somebody asks for them (RefreshPredictions).
   if (needEnergy && transientFlag)
     flags &= ~DPC_FWD_FE;
-  ForwardRange(0, n - 1, flags);
-  if (layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE)
+  const bool ce = (layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE) != 0;
+  const bool fused = ce && dpc_plan_fused_cross_entropy(plan);
+  ForwardRange(0, n - 1, flags | (fused ? DPC_FWD_CE : 0));
+  if (ce && !fused)
   {
     Check(dpc_error(plan, n - 1, needEnergy ? 1 : 0));
     if (kind != NetworkKind::SIMPLE)
@@ -673,16 +683,11 @@ void PCNetwork::UpdateState()
       ++i;
       continue;
     }
-    if (topDownMeaningless && i == n - 2)
-    {
-      Check(dpc_relax(plan, i));
-      ++i;
-      continue;
-    }
     int j = i;
-    while (j < n && !layers[j]->clamped && !(topDownMeaningless && j == n - 2))
+    while (j < n && !layers[j]->clamped)
       ++j;
-    Check(dpc_update_state(plan, i, j - i));
+    // an unclamped terminal layer relaxes, and so does the layer under a cross-entropy one
+    Check(dpc_update_state_ex(plan, i, j - i, topDownMeaningless ? n - 2 : n - 1));
     i = j;
   }
 }
@@ -746,13 +751,19 @@ void PCNetwork::UpdateWeights()
 // Inside a whole train step the predictions of the settling passes and of the pre-update
 // refresh are consumed only through the fused e / fe outputs (the final energy pass
 // recomputes and stores them), so those passes need not write preact/mu at all.  A softmax
-// head reads preact of the layer below through a separate kernel, so it keeps the stores.
+// error that follows the pass in kernels of its own reads them, so there the stores stay.
 struct TransientScope
 {
   int& flag;
   TransientScope(int& f, bool on) : flag(f) { flag = on ? DPC_FWD_TRANSIENT : 0; }
   ~TransientScope() { flag = 0; }
 };
+
+bool PCNetwork::PredictionsTransient()
+{
+  return kind != NetworkKind::SIMPLE && (!(layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE) ||
+                                         dpc_plan_fused_cross_entropy(plan));
+}
 
 // The last pass of a train step computes every layer's prediction for the energy but does not
 // store it; whoever wants to look at mu / preact afterwards gets them recomputed here from the
@@ -869,8 +880,7 @@ void PCNetwork::RunTrainPhases(int mode, int steps)
     RunTrainSegments(mode, steps);
     return;
   }
-  TransientScope scope(transientFlag, kind != NetworkKind::SIMPLE &&
-                                          !(layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE));
+  TransientScope scope(transientFlag, PredictionsTransient());
   auto settle = [&](bool energy)
   {
     CalculateState(energy);
@@ -1016,8 +1026,8 @@ float PCNetwork::TrainStepRaw(int mode, const float* x, size_t nx, const float* 
   else
     RunTrainPhases(mode, steps);
   // (same condition as the TransientScope of RunTrainPhases; a graph replay runs no host code)
-  predictionsStale =
-      kind != NetworkKind::SIMPLE && !(layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE);
+  predictionsStale = segments ? kind != NetworkKind::SIMPLE && !(layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE)
+                              : PredictionsTransient();
 
   double energy = 0.0;
   if (readEnergy)
@@ -1054,6 +1064,8 @@ void PCNetwork::RunPredictPhases(int steps, bool withProjection)
       EPCStep();
     else
     {
+      // (only the last pass's predictions can be looked at afterwards)
+      TransientScope scope(transientFlag, t + 1 < steps && PredictionsTransient());
       CalculateState(false);
       UpdateState();
     }

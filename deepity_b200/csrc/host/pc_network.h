@@ -215,6 +215,7 @@ private:
   void SyncGradients(size_t count);
   void ForwardRange(int first, int count, int flags);
   bool UseRowSegments();
+  bool PredictionsTransient(); // no pass but the last need store mu / preact
   void RowSegment(int ops, int steps);
   void RunTrainSegments(int mode, int steps);
   void RunTrainPhases(int mode, int steps);

@@ -261,6 +261,9 @@ enum
                                  computed with ERR_NEXT, else the one in memory            */
   DPC_FWD_CACHED = 1 << 4,    /* skip the GEMM, reuse preact/mu in memory (a clamped layer's
                                  cached prediction, DirectKPPCLayer.cpp:275-280)          */
+  DPC_FWD_CACHED_FIRST = 1 << 5, /* the first layer of the range is DPC_FWD_CACHED, the others not */
+  DPC_FWD_CE = 1 << 6,        /* with ERR_NEXT: the head's kernel computes the softmax cross-entropy
+                                 error of the last layer itself (see dpc_plan_fused_cross_entropy)  */
   DPC_FWD_NO_MU = 1 << 9,     /* with COPY_NEXT: mu[l] itself is not written (z[l+1] holds the
                                  same values and mu is recomputed before anyone reads it)  */
   DPC_FWD_NO_PREACT = 1 << 11, /* with COPY_NEXT and NO_MU: preact[l] is not written either (the
@@ -283,6 +286,10 @@ DPC_API int dpc_project_forward(dpc_plan* plan, int first, int count, int skip_l
  * first (a clamped input layer's prediction is cached and read again). */
 DPC_API int dpc_project_forward_ex(dpc_plan* plan, int first, int count, int skip_last_copy,
                                    int extra_flags);
+/* 1 when the last layer has a softmax cross-entropy error that the head's forward kernel can compute
+ * in its epilogue (DPC_FWD_CE; a head of at most 16 units launched on its own), else dpc_error and
+ * dpc_feedback_error follow the pass. */
+DPC_API int dpc_plan_fused_cross_entropy(dpc_plan* plan);
 /* Error of one layer against the prediction below: Gaussian e = z - mu, or softmax
  * cross-entropy when the layer has DPC_LAYER_SOFTMAX_CE.  with_energy accumulates into the
  * plan's energy accumulator (CPUBackend.cpp:602-629, 658-714). */
@@ -305,6 +312,8 @@ DPC_API int dpc_update_state(dpc_plan* plan, int first, int count);
 DPC_API int dpc_epc_reconstruct(dpc_plan* plan, int layer);
 DPC_API int dpc_epc_adjoint(dpc_plan* plan, int layer, int from_terminal, float scale,
                             int clamped);
+/* Same; layers [relax_from, first+count) relax, z -= ir*e, instead. */
+DPC_API int dpc_update_state_ex(dpc_plan* plan, int first, int count, int relax_from);
 /* z -= ir*e for one layer (the "output layer" branch of UpdateState). */
 DPC_API int dpc_relax(dpc_plan* plan, int layer);
 /* DirectFeedbackUpdate for every layer of the range whose upper neighbour has Psi:
