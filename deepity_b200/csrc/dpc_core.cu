@@ -699,7 +699,8 @@ static int forward_simt(dpc_plan* p, int first, int count, int flags)
     if (rc != DPC_OK)
       return rc;
   }
-  if (flags & DPC_FWD_FE)
+  const bool simple = (p->h[first].flags & DPC_LAYER_INPUT_ACT) != 0;
+  if ((flags & DPC_FWD_FE) || (simple && (flags & DPC_FWD_ERR_NEXT)))
     wrote(p, K_FE, first, count);
   if (flags & DPC_FWD_COPY_NEXT)
     wrote(p, K_Z, first + 1, count);
@@ -888,6 +889,8 @@ int dpc_error(dpc_plan* p, int layer, int with_energy)
     return fail(DPC_ERR_INVALID, "dpc_error: the input layer has no prediction below it");
   const dpc_layer& L = p->h[layer];
   cudaStream_t st = p->ctx->stream;
+  if (p->h[layer - 1].flags & DPC_LAYER_INPUT_ACT)
+    wrote(p, K_FE, layer - 1, 1);
   if (L.flags & DPC_LAYER_SOFTMAX_CE)
   {
     int blocks = std::min(cdiv(p->batch, NTHREADS / 32), p->ctx->sm_count * 8);
@@ -1010,10 +1013,10 @@ static int update_state_simt(dpc_plan* p, int first, int count)
 
 int dpc_update_state(dpc_plan* p, int first, int count)
 {
-  return dpc_update_state_ex(p, first, count, first + count);
+  return dpc_update_state_ex(p, first, count, first + count, 0);
 }
 
-int dpc_update_state_ex(dpc_plan* p, int first, int count, int relax_from)
+int dpc_update_state_ex(dpc_plan* p, int first, int count, int relax_from, int flags)
 {
   int rc = check_range(p, first, count);
   if (rc != DPC_OK)
@@ -1021,7 +1024,7 @@ int dpc_update_state_ex(dpc_plan* p, int first, int count, int relax_from)
   const int end = first + count;
   relax_from = std::min(std::max(relax_from, first), end);
   std::vector<Job> jobs = pieces_of(
-      p, first, relax_from - first, [=](int f, int c) { return tc_update_state(p, f, c); },
+      p, first, relax_from - first, [=](int f, int c) { return tc_update_state(p, f, c, (flags & DPC_STATE_FEED) != 0); },
       [=](int f, int c) { return update_state_simt(p, f, c); }, true);
   for (int i = relax_from; i < end; ++i)
     jobs.push_back([=] { return dpc_relax(p, i); });

@@ -19,6 +19,8 @@
 //     (same bytes as the fp32 tensor), so the grouped kernels load tensor-core-ready tiles by TMA
 //     (128-byte rows of 64 bf16, 128-byte swizzle) and run the one-ring pipeline of the TF32 mode
 //     with three MMAs per k-step: same arithmetic as scheme 2, no split warps, no second ring;
+//     (a run of SimplePC layers: the belief planes hold f(z), the operand, and the feedback-error
+//     planes the plain error of the layer above; the fp32 tensors of both operands are not kept);
 //   * the predictive-coding elementwise work runs in the epilogue straight out of tensor
 //     memory: bias + activation + error + energy + feedback error (forward), the state
 //     update (feedback), the SGD weight update (weight-shaped product).
@@ -63,6 +65,14 @@ enum
 };
 constexpr int WG_LEARN_MODE = 0, WG_DFA_MODE = 1, WG_GRAD_MODE = 2; // GRAD is or-ed in
 
+// what the state update writes into the belief planes
+enum
+{
+  FBP_BELIEF = 0, // z
+  FBP_NONE = 1,   // SimplePC: nothing, the weight update still needs f(z) as last fed to the products
+  FBP_FEED = 2    // SimplePC: f(z), the operand of the pass that follows
+};
+
 struct TcState
 {
   bool ok = false;
@@ -89,6 +99,7 @@ struct TcState
   bool store_maps = false;
   std::vector<uint8_t> dirty[3];
   bool planes = false;
+  bool simple = false; // the run's layers are SimplePC layers (planes only)
   // The run's feedback errors exist only as planes: every reader of them is a kernel that takes
   // the planes (feedback and weight-shaped products of this file, the bias column sums).
   bool fe_only = false;
@@ -120,7 +131,7 @@ struct TcParams
   int run_first;
   int M, N, K;
   int tiles_m, tiles_n;
-  int flags, mode;
+  int flags, mode; // feedback: mode = FBP_*
   double* energy;
   int* error_flag;
   // Chain mode (the sequential forward sweep): CTA b owns output tile b of EVERY layer and
@@ -310,7 +321,8 @@ __device__ __forceinline__ void load_fwd_meta(const TcParams& P, int li, FwdMeta
     M.up_z = M.up_e = nullptr, M.up_flags = 0;
   const long long r = li - P.run_first;
   M.fe_hi = P.fep ? P.fep + 2 * r * P.act_elems : nullptr;
-  M.upz_hi = P.zp ? P.zp + 2 * (r + 1) * P.act_elems : nullptr;
+  // (SimplePC planes hold f(z): the copied belief is split anew, with the activation)
+  M.upz_hi = P.zp && !(Lp->flags & DPC_LAYER_INPUT_ACT) ? P.zp + 2 * (r + 1) * P.act_elems : nullptr;
 }
 
 // Where the staged operand of the layer above sits (pair-mode forward only).
@@ -349,7 +361,9 @@ __device__ __forceinline__ void fwd_epilogue_tile(const TcParams& P, const FwdMe
   const bool Lup = L.up_z != nullptr;
   const bool next_ce = Lup && (L.up_flags & DPC_LAYER_SOFTMAX_CE);
   const bool do_err = (P.flags & DPC_FWD_ERR_NEXT) && Lup && !next_ce;
-  const bool do_fe = (P.flags & DPC_FWD_FE) && Lup && !(L.flags & DPC_LAYER_INPUT_ACT) &&
+  // (SimplePC: the "feedback error" is the error itself, kept as operand planes only)
+  const bool do_fe = (P.flags & DPC_FWD_FE) && Lup &&
+                     (!(L.flags & DPC_LAYER_INPUT_ACT) || L.fe_hi != nullptr) &&
                      !(next_ce && (P.flags & DPC_FWD_ERR_NEXT));
   const bool do_copy = (P.flags & DPC_FWD_COPY_NEXT) && Lup;
   const bool store = !(P.flags & DPC_FWD_TRANSIENT);
@@ -1175,13 +1189,47 @@ __global__ void __launch_bounds__(Cfg<OP, BN, THREE_X, BM, PAIR, KS>::THREADS, 1
               zz[4 * i] = y.x, zz[4 * i + 1] = y.y, zz[4 * i + 2] = y.z, zz[4 * i + 3] = y.w;
             }
             tc_ld16(taddr + c * 16, v);
+            if (P.mode != FBP_BELIEF)
+            {
+              // SimplePC (src/layers/SimplePCLayer.cpp:205-257): z += ir (f'(z) (e_above W) - e)
 #pragma unroll
-            for (int k = 0; k < 16; ++k)
-              zz[k] += L.ir * (L.a * v[k] - ee[k]);
+              for (int k = 0; k < 16; k += 8)
+              {
+                float z8[8], f8[8], d8[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                  z8[i] = zz[k + i];
+                act_both8<true>(L.act, z8, f8, d8);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                  zz[k + i] += L.ir * (v[k + i] * d8[i] - ee[k + i]);
+              }
+            }
+            else
+            {
+#pragma unroll
+              for (int k = 0; k < 16; ++k)
+                zz[k] += L.ir * (L.a * v[k] - ee[k]);
+            }
 #pragma unroll
             for (int i = 0; i < 4; ++i)
               *reinterpret_cast<float4*>(zbuf + row * 64 + ((i ^ sw) << 4)) =
                   make_float4(zz[4 * i], zz[4 * i + 1], zz[4 * i + 2], zz[4 * i + 3]);
+            if (P.mode == FBP_FEED)
+            {
+#pragma unroll
+              for (int k = 0; k < 16; k += 8)
+              {
+                float z8[8], f8[8], d8[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                  z8[i] = zz[k + i];
+                act_both8<false>(L.act, z8, f8, d8);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                  zz[k + i] = f8[i];
+              }
+            }
 #pragma unroll
             for (int k = 0; k < 16; k += 8)
             {
@@ -1199,7 +1247,8 @@ __global__ void __launch_bounds__(Cfg<OP, BN, THREE_X, BM, PAIR, KS>::THREADS, 1
             {
               const int col = n0 + c * 16, row0 = m - lane;
               tma_store_3d(&mapSE, zbuf + quarter * 2048, col, row0, lz);
-              tma_store_3d(&mapSF, obuf, col, row0, 2 * lz); // hi + mid
+              if (P.mode != FBP_NONE)
+                tma_store_3d(&mapSF, obuf, col, row0, 2 * lz); // hi + mid
               bulk_commit();
               // the stores have read their shared memory: the box may be refilled, the plane
               // buffer rewritten
@@ -1272,8 +1321,14 @@ __global__ void __launch_bounds__(Cfg<OP, BN, THREE_X, BM, PAIR, KS>::THREADS, 1
                 zz[k + q] += L.ir * uu[q];
             }
             st8(L.z + o + k, &zz[k]);
-            if (z_hi)
+            if (z_hi && P.mode != FBP_NONE)
+            {
+              if (P.mode == FBP_FEED)
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                  zz[k + q] = act_fwd(L.act, zz[k + q]);
               st_planes8(z_hi, P.act_elems, o + k, &zz[k]);
+            }
           }
         }
       }
@@ -1729,13 +1784,21 @@ __global__ void split_planes_kernel(const dpc_layer* __restrict__ layers, int fi
                                     int kind, __nv_bfloat16* base, long long elems)
 {
   const dpc_layer& L = layers[first + blockIdx.y];
-  const float* src = kind == PL_Z ? L.z : (kind == PL_FE ? L.fe : L.W);
+  const bool simple = (L.flags & DPC_LAYER_INPUT_ACT) != 0;
+  const float* src = kind == PL_Z ? L.z : kind == PL_W ? L.W : simple ? (&L)[1].e : L.fe;
   __nv_bfloat16* hi = base + 2 * (long long)(first + (int)blockIdx.y - run_first) * elems;
   for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8; i < elems;
        i += (long long)gridDim.x * blockDim.x * 8)
   {
-    const float4 a = *reinterpret_cast<const float4*>(src + i);
-    const float4 b = *reinterpret_cast<const float4*>(src + i + 4);
+    float4 a = *reinterpret_cast<const float4*>(src + i);
+    float4 b = *reinterpret_cast<const float4*>(src + i + 4);
+    if (simple && kind == PL_Z)
+    {
+      const float in[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+      float f[8], d[8];
+      act_both8<false>(L.act, in, f, d);
+      a = make_float4(f[0], f[1], f[2], f[3]), b = make_float4(f[4], f[5], f[6], f[7]);
+    }
     uint4 h, m;
     split8(a, b, h, m);
     *reinterpret_cast<uint4*>(hi + i) = h;
@@ -1839,6 +1902,13 @@ static bool planes_init(dpc_plan* plan, TcState* st, int first, int count, int H
   st->dirty[PL_FE].assign(count, 1);
   st->dirty[PL_W].assign(count, 1);
   st->planes = true;
+  if (st->simple)
+  {
+    // (a weight update before any forward pass multiplies f(z) = 0, as the zeroed fp32 tensor would)
+    cudaMemset(st->zp, 0, 2 * (size_t)(count + 1) * act * sizeof(__nv_bfloat16));
+    st->fe_only = true;
+    return true;
+  }
   // fp32 feedback errors can be dropped when nothing but the plane-reading kernels consumes
   // them: no ePC adjoint chain (it keeps its source in fe), feedback weights above every layer
   // of the run (else the direct-feedback product falls to the CUDA-core kernel, which reads fp32).
@@ -1882,15 +1952,22 @@ int tc_plan_init(dpc_plan* plan)
   if (B % TBM != 0)
     return DPC_OK;
   // Longest run of identical square DirectKP/Full layers at constant strides.
+  // A SimplePC run needs the operand planes (3xBF16, pair tiles), and its launches enough work: with
+  // few tiles the grouped CUDA-core kernels are as fast and need no split of f(z).
+  const bool simple_ok = pair_ok(B, 256) && split_scheme(plan) == 2 && !getenv("DPC_DISABLE_PLANES") &&
+                         !getenv("DPC_DISABLE_STAGED_OUTPUT") &&
+                         plan->ctx->precision != DPC_PRECISION_TF32;
   int best_first = 0, best_count = 0;
   int i = 0;
   while (i + 1 < n)
   {
     const dpc_layer& L0 = plan->h[i];
-    const bool ok0 = L0.next_size == L0.size && L0.size % 256 == 0 && L0.size >= 256 &&
-                     !(L0.flags & DPC_LAYER_INPUT_ACT) && L0.fe && L0.preact &&
+    const bool simple = (L0.flags & DPC_LAYER_INPUT_ACT) != 0;
+    const float* out0 = simple ? plan->h[i + 1].e : L0.fe;
+    const bool ok0 = L0.next_size == L0.size && L0.size % 256 == 0 && L0.size >= 256 && out0 &&
+                     (simple ? simple_ok : L0.preact != nullptr) &&
                      ((uintptr_t)L0.z % 128 == 0) && ((uintptr_t)L0.W % 128 == 0) &&
-                     ((uintptr_t)L0.fe % 128 == 0);
+                     ((uintptr_t)out0 % 128 == 0);
     if (!ok0)
     {
       ++i;
@@ -1902,16 +1979,18 @@ int tc_plan_init(dpc_plan* plan)
     {
       const dpc_layer& Lj = plan->h[j];
       const dpc_layer& Lp = plan->h[j - 1];
-      if (Lj.size != L0.size || Lj.next_size != L0.size || (Lj.flags & DPC_LAYER_INPUT_ACT))
+      if (Lj.size != L0.size || Lj.next_size != L0.size || ((Lj.flags ^ L0.flags) & DPC_LAYER_INPUT_ACT))
         break;
-      const int64_t dz = Lj.z - Lp.z, dw = Lj.W - Lp.W, df = Lj.fe - Lp.fe;
+      const int64_t dz = Lj.z - Lp.z, dw = Lj.W - Lp.W,
+                    df = simple ? plan->h[j + 1].e - Lj.e : Lj.fe - Lp.fe;
       if (j == i + 1)
         zs = dz, ws = dw, fs = df;
       if (dz != zs || dw != ws || df != fs || dz <= 0 || dw <= 0 || df <= 0)
         break;
       ++j;
     }
-    if (j - i > best_count)
+    const bool enough = !simple || (long long)(j - i) * B * L0.size * L0.size >= (1LL << 27);
+    if (enough && j - i > best_count)
     {
       best_first = i, best_count = j - i;
       plan->run.z_stride = zs, plan->run.w_stride = ws, plan->run.out_stride = fs;
@@ -1990,7 +2069,10 @@ static bool run_init(dpc_plan* plan, TcState* st, int best_first, int best_count
   }
   const dpc_layer& L0 = plan->h[best_first];
   const int H = L0.size;
+  st->simple = (L0.flags & DPC_LAYER_INPUT_ACT) != 0;
   bool ok = true;
+  if (!st->simple)
+  {
   ok &= make_map(&st->z_km, L0.z, H, B, best_count, plan->run.z_stride, TBM, false);
   ok &= make_map(&st->z_km64, L0.z, H, B, best_count, plan->run.z_stride, 64, false);
   ok &= make_map(&st->fe_km, L0.fe, H, B, best_count, plan->run.out_stride, TBM, false);
@@ -2001,6 +2083,7 @@ static bool run_init(dpc_plan* plan, TcState* st, int best_first, int best_count
   ok &= make_map(&st->z_mn, L0.z, H, B, best_count, plan->run.z_stride, 32, true);
   ok &= make_map(&st->fe_mn, L0.fe, H, B, best_count, plan->run.out_stride, 32, true);
   ok &= make_map(&st->w_mn, L0.W, H, H, best_count, plan->run.w_stride, 32, true);
+  }
   if (!ok)
   {
     // the driver refused a tensor map: stay on the CUDA-core path, audibly
@@ -2045,6 +2128,16 @@ static bool run_init(dpc_plan* plan, TcState* st, int best_first, int best_count
         make_store_map(&st->zp_st, st->zp, true, H, B, 2 * (best_count + 1), (int64_t)B * H) &&
         make_store_map(&st->w_st, L0.W, false, H, H, best_count, plan->run.w_stride) &&
         make_store_map(&st->wp_st, st->wp, true, H, H, 2 * best_count, (int64_t)H * H);
+  }
+  if (st->simple && !(st->planes && st->store_maps))
+  {
+    // nothing else multiplies f(z): the layers go back to the single-layer path
+    planes_free(st);
+    st->simple = false;
+    cudaFree(st->chain_counters);
+    st->chain_counters = nullptr;
+    plan->run = TensorRun();
+    return false;
   }
   if (!st->planes && !getenv("DPC_DISABLE_PLANES") && split_scheme(plan) == 2 && pair_ok(B, H))
   {
@@ -2249,6 +2342,8 @@ int tc_forward(dpc_plan* p, int first, int count, int flags)
   if (!st || !st->ok || !range_in_run(p, first, count))
     return 1;
   const int H = p->run.width, B = p->batch;
+  if (st->simple && (flags & DPC_FWD_ERR_NEXT))
+    flags |= DPC_FWD_FE; // the error of the layer above as operand planes
   // the pass after the last settling step: it only refreshes the errors the learning phase reads
   const bool refresh =
       (flags & DPC_FWD_FE) && !(flags & DPC_FWD_ERR_NEXT) && (flags & DPC_FWD_TRANSIENT);
@@ -2301,7 +2396,7 @@ int tc_forward(dpc_plan* p, int first, int count, int flags)
     if (flags & DPC_FWD_FE)
       planes_mark(st, PL_FE, r0, r0 + count, stale);
     if (flags & DPC_FWD_COPY_NEXT)
-      planes_mark(st, PL_Z, r0 + 1, r0 + count + 1, stale);
+      planes_mark(st, PL_Z, r0 + 1, r0 + count + 1, st->simple ? 1 : stale);
   }
   return rc;
 }
@@ -2314,7 +2409,7 @@ int tc_forward(dpc_plan* p, int first, int count, int flags)
 int tc_project_forward(dpc_plan* p, int first, int count, int flags)
 {
   auto* st = static_cast<TcState*>(p->tc);
-  if (!st || !st->ok || !range_in_run(p, first, count) || count < 2)
+  if (!st || !st->ok || !range_in_run(p, first, count) || count < 2 || st->simple)
     return 1;
   const int H = p->run.width, B = p->batch;
   // Narrow 128 x 32 tiles: B/128 * H/32 CTAs (128 for the 1024 x 512 layers of the deep-stack
@@ -2384,7 +2479,7 @@ int tc_project_forward(dpc_plan* p, int first, int count, int flags)
   return rc;
 }
 
-int tc_update_state(dpc_plan* p, int first, int count)
+int tc_update_state(dpc_plan* p, int first, int count, bool feed)
 {
   auto* st = static_cast<TcState*>(p->tc);
   if (st && st->ok && count == 1 && !range_in_run(p, first, 1))
@@ -2411,6 +2506,7 @@ int tc_update_state(dpc_plan* p, int first, int count)
       for (int i = first; i < first + count && plain; ++i)
         plain = !p->h[i].v && !(p->h[i].flags & DPC_LAYER_RESIDUAL);
       P.tstore = plain ? 1 : 0;
+      P.mode = !st->simple ? FBP_BELIEF : feed ? FBP_FEED : FBP_NONE;
       rc = launch<TC_FB, 256, 3, 128, true>(p, st, st->fep_km, st->wp_mn, P);
     }
     else
@@ -2428,7 +2524,7 @@ int tc_update_state(dpc_plan* p, int first, int count)
                      : launch<TC_FB, 128, 1>(p, st, st->fe_km, st->w_mn, P);
   }
   if (rc == DPC_OK)
-    planes_mark(st, PL_Z, r0, r0 + count, planes_kept(p, st) ? 0 : 1);
+    planes_mark(st, PL_Z, r0, r0 + count, planes_kept(p, st) && (!st->simple || feed) ? 0 : 1);
   return rc;
 }
 
@@ -2469,8 +2565,9 @@ int tc_weight_gemm(dpc_plan* p, int first, int count, int mode, int decay_w)
     TcParams P = base_params(p, st, first, count, H, H, B, 256, decay_w ? 1 : 0, mode, 256);
     if (!tf32 && planes_on(p, st))
     {
+      // (SimplePC: f(z) as last fed to the forward product, not of the beliefs as they are now)
       if ((rc = planes_need(p, st, PL_FE, r0, r0 + count)) != DPC_OK ||
-          (rc = planes_need(p, st, PL_Z, r0, r0 + count)) != DPC_OK)
+          (!st->simple && (rc = planes_need(p, st, PL_Z, r0, r0 + count)) != DPC_OK))
         return rc;
       // in-place SGD updates take the weight tile through shared memory and write it and its
       // planes back with bulk stores
@@ -2682,7 +2779,8 @@ std::string tc_describe(dpc_plan* p)
   const bool tf32 = p->ctx->precision == DPC_PRECISION_TF32;
   std::string out;
   int on_tc = 0;
-  if (p->run.count > 0)
+  const bool run_text = p->run.count > 0 && !st->simple;
+  if (run_text)
   {
     const bool pair = pair_ok(p->batch, p->run.width);
     std::string mode = tf32 ? "1xTF32"
@@ -2696,12 +2794,24 @@ std::string tc_describe(dpc_plan* p)
           (pair ? "CTA pairs 256x256" : "single-CTA tiles") + ", " + mode + "); ";
     on_tc += p->run.count;
   }
+  auto name = [&](int l)
+  {
+    return " " + std::to_string(l) + " (" + std::to_string(p->h[l].size) + "->" +
+           std::to_string(p->h[l].next_size) + ")";
+  };
+  if (p->run.count > 0 && st->simple)
+  {
+    out += "layer";
+    for (int l = p->run.first; l < p->run.first + p->run.count; ++l)
+      out += name(l);
+    out += " on tcgen05 (one launch per phase, CTA pairs 256x256, 3xBF16 from pre-split planes of f(z)); ";
+    on_tc += p->run.count;
+  }
   if (!st->extras.empty())
   {
     out += "layer";
     for (const auto& x : st->extras)
-      out += " " + std::to_string(x.layer) + " (" + std::to_string(p->h[x.layer].size) + "->" +
-             std::to_string(p->h[x.layer].next_size) + ")";
+      out += name(x.layer);
     out += std::string(" on tcgen05 (CTA pairs 256x256, ") +
            (tf32 ? "1xTF32" : split_scheme(p) == 2 ? "3xBF16 split in the kernel" : "3xTF32") + "); ";
     on_tc += (int)st->extras.size();

@@ -666,7 +666,7 @@ float PCNetwork::CalculateState(bool needEnergy)
   return 0.0f;
 }
 
-void PCNetwork::UpdateState()
+void PCNetwork::UpdateState(bool feedsForward)
 {
   RequireCompiled();
   const int n = (int)layers.size();
@@ -687,7 +687,8 @@ void PCNetwork::UpdateState()
     while (j < n && !layers[j]->clamped)
       ++j;
     // an unclamped terminal layer relaxes, and so does the layer under a cross-entropy one
-    Check(dpc_update_state_ex(plan, i, j - i, topDownMeaningless ? n - 2 : n - 1));
+    Check(dpc_update_state_ex(plan, i, j - i, topDownMeaningless ? n - 2 : n - 1,
+                              feedsForward ? DPC_STATE_FEED : 0));
     i = j;
   }
 }
@@ -755,14 +756,14 @@ void PCNetwork::UpdateWeights()
 struct TransientScope
 {
   int& flag;
-  TransientScope(int& f, bool on) : flag(f) { flag = on ? DPC_FWD_TRANSIENT : 0; }
-  ~TransientScope() { flag = 0; }
+  const int before;
+  TransientScope(int& f, bool on) : flag(f), before(f) { flag = on ? DPC_FWD_TRANSIENT : 0; }
+  ~TransientScope() { flag = before; }
 };
 
 bool PCNetwork::PredictionsTransient()
 {
-  return kind != NetworkKind::SIMPLE && (!(layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE) ||
-                                         dpc_plan_fused_cross_entropy(plan));
+  return !(layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE) || dpc_plan_fused_cross_entropy(plan);
 }
 
 // The last pass of a train step computes every layer's prediction for the energy but does not
@@ -880,11 +881,14 @@ void PCNetwork::RunTrainPhases(int mode, int steps)
     RunTrainSegments(mode, steps);
     return;
   }
-  TransientScope scope(transientFlag, PredictionsTransient());
-  auto settle = [&](bool energy)
+  TransientScope scope(transientFlag, kind != NetworkKind::SIMPLE && PredictionsTransient());
+  // last: nothing of this step's predictions is recomputed before somebody may look at them, or
+  // (SimplePC) before the weight update uses the operand f(z) they were made from
+  auto settle = [&](bool energy, bool last)
   {
+    TransientScope passes(transientFlag, transientFlag || (!last && PredictionsTransient()));
     CalculateState(energy);
-    UpdateState();
+    UpdateState(!last);
   };
   if (kind == NetworkKind::DIRECT_KP)
   {
@@ -906,7 +910,7 @@ void PCNetwork::RunTrainPhases(int mode, int steps)
     DirectFeedbackUpdate();
     sweepFeedsDfa = false;
     for (int t = 0; t < steps; ++t)
-      settle(false);
+      settle(false, false);
     UpdateWeights();
     Check(dpc_energy_reset(plan));
     CalculateState(true);
@@ -920,7 +924,7 @@ void PCNetwork::RunTrainPhases(int mode, int steps)
       if (useEPC)
         EPCStep();
       else
-        settle(false);
+        settle(false, false);
       if (useIPC)
       {
         UpdateWeights();
@@ -937,7 +941,7 @@ void PCNetwork::RunTrainPhases(int mode, int steps)
   else if (mode == 0)
   {
     for (int t = 0; t < steps; ++t)
-      settle(false);
+      settle(false, false);
     Check(dpc_energy_reset(plan));
     CalculateState(true);
     UpdateWeights();
@@ -946,7 +950,7 @@ void PCNetwork::RunTrainPhases(int mode, int steps)
   {
     ProjectForward();
     for (int t = 0; t < steps; ++t)
-      settle(false);
+      settle(false, t + 1 == steps);
     UpdateWeights();
     Check(dpc_energy_reset(plan));
     CalculateState(true);
@@ -955,7 +959,7 @@ void PCNetwork::RunTrainPhases(int mode, int steps)
   {
     Check(dpc_energy_reset(plan));
     for (int t = 0; t < steps; ++t)
-      settle(true);
+      settle(true, t + 1 == steps);
     UpdateWeights();
   }
   (void)n;
@@ -1027,7 +1031,10 @@ float PCNetwork::TrainStepRaw(int mode, const float* x, size_t nx, const float* 
     RunTrainPhases(mode, steps);
   // (same condition as the TransientScope of RunTrainPhases; a graph replay runs no host code)
   predictionsStale = segments ? kind != NetworkKind::SIMPLE && !(layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE)
-                              : PredictionsTransient();
+                              : kind != NetworkKind::SIMPLE && PredictionsTransient();
+  // (a replay runs no host code: the operand f(z) may be one state update behind the beliefs)
+  if (kind == NetworkKind::SIMPLE)
+    Check(dpc_plan_invalidate(plan, 0, n, DPC_WROTE_Z));
 
   double energy = 0.0;
   if (readEnergy)
@@ -1067,7 +1074,7 @@ void PCNetwork::RunPredictPhases(int steps, bool withProjection)
       // (only the last pass's predictions can be looked at afterwards)
       TransientScope scope(transientFlag, t + 1 < steps && PredictionsTransient());
       CalculateState(false);
-      UpdateState();
+      UpdateState(t + 1 < steps);
     }
   }
   if (kind == NetworkKind::FULL && (layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE))
@@ -1125,6 +1132,8 @@ void PCNetwork::PredictRaw(const float* x, size_t nx, int steps, bool withProjec
   }
   else
     RunPredictPhases(steps, withProjection);
+  if (kind == NetworkKind::SIMPLE)
+    Check(dpc_plan_invalidate(plan, 0, n, DPC_WROTE_Z));
   Check(dpc_copy_d2h_sync(ctx, pinnedOut, layers.back()->d.z, count * sizeof(float)));
   std::memcpy(out, pinnedOut, count * sizeof(float));
 }

@@ -123,7 +123,7 @@ public:
   float CalculateTerminalError();
   void DirectFeedbackUpdate();
   float CalculateState(bool needEnergy);
-  void UpdateState();
+  void UpdateState(bool feedsForward = false); // a forward pass follows before UpdateWeights()
   float Step(bool computeEnergy = true);
   void UpdateWeights();
 

@@ -312,8 +312,14 @@ DPC_API int dpc_update_state(dpc_plan* plan, int first, int count);
 DPC_API int dpc_epc_reconstruct(dpc_plan* plan, int layer);
 DPC_API int dpc_epc_adjoint(dpc_plan* plan, int layer, int from_terminal, float scale,
                             int clamped);
-/* Same; layers [relax_from, first+count) relax, z -= ir*e, instead. */
-DPC_API int dpc_update_state_ex(dpc_plan* plan, int first, int count, int relax_from);
+/* Same; layers [relax_from, first+count) relax, z -= ir*e, instead.  DPC_STATE_FEED: a forward pass
+ * over these layers follows before their next weight update, so the operand f(z) of SimplePC layers
+ * may move on with the beliefs (a weight update uses f(z) as last fed to the forward product). */
+enum
+{
+  DPC_STATE_FEED = 1
+};
+DPC_API int dpc_update_state_ex(dpc_plan* plan, int first, int count, int relax_from, int flags);
 /* z -= ir*e for one layer (the "output layer" branch of UpdateState). */
 DPC_API int dpc_relax(dpc_plan* plan, int layer);
 /* DirectFeedbackUpdate for every layer of the range whose upper neighbour has Psi:
