@@ -1952,8 +1952,11 @@ int tc_plan_init(dpc_plan* plan)
   if (B % TBM != 0)
     return DPC_OK;
   // Longest run of identical square DirectKP/Full layers at constant strides.
-  // A SimplePC run needs the operand planes (3xBF16, pair tiles), and its launches enough work: with
-  // few tiles the grouped CUDA-core kernels are as fast and need no split of f(z).
+  // A SimplePC run needs the operand planes (3xBF16, pair tiles) and, per layer, the work from which
+  // single layers leave the (more exact) CUDA-core kernels too.
+  long long min_work = 1LL << 29; // measured, see the single layers below
+  if (const char* e = getenv("DPC_RECTANGULAR_MIN_WORK"))
+    min_work = atoll(e);
   const bool simple_ok = pair_ok(B, 256) && split_scheme(plan) == 2 && !getenv("DPC_DISABLE_PLANES") &&
                          !getenv("DPC_DISABLE_STAGED_OUTPUT") &&
                          plan->ctx->precision != DPC_PRECISION_TF32;
@@ -1989,7 +1992,7 @@ int tc_plan_init(dpc_plan* plan)
         break;
       ++j;
     }
-    const bool enough = !simple || (long long)(j - i) * B * L0.size * L0.size >= (1LL << 27);
+    const bool enough = !simple || (long long)B * L0.size * L0.size >= min_work;
     if (enough && j - i > best_count)
     {
       best_first = i, best_count = j - i;
@@ -2012,9 +2015,6 @@ int tc_plan_init(dpc_plan* plan)
   // CUDA-core kernels by batch x inputs x outputs: 2^28 equal, 2^29 1.5x, 2^30 1.9x, 2^32 2.8x
   // faster; a lone first layer: 2^28.6 equal, 2^31.6 5 % of the step.  Hence 2^29;
   // DPC_RECTANGULAR_MIN_WORK overrides it.
-  long long min_work = 1LL << 29;
-  if (const char* e = getenv("DPC_RECTANGULAR_MIN_WORK"))
-    min_work = atoll(e);
   if (pair_ok(B, 256) && !getenv("DPC_DISABLE_RECTANGULAR"))
     for (int l = 0; l + 1 < n; ++l)
     {
