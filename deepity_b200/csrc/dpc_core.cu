@@ -674,18 +674,20 @@ static int forward_simt(dpc_plan* p, int first, int count, int flags)
       // heads (at most 16 output units) with vector-loadable rows: one warp per batch row
       bool narrow = true;
       for (int i = f; i < f + c && narrow; ++i)
-        narrow = p->h[i].next_size <= 0 || narrow_forward(p, i);
+        narrow = p->h[i].next_size <= 0 || (narrow_forward(p, i) && ((p->h[i].flags ^ p->h[f].flags) & DPC_LAYER_INPUT_ACT) == 0);
+      const bool simple = (p->h[f].flags & DPC_LAYER_INPUT_ACT) != 0;
       if (narrow)
       {
-        if (p->batch >= 2048)
+        if (p->batch >= 2048 && !simple) // (two rows of f(z) take too many registers)
         {
           dim3 grid(cdiv(p->batch, 2 * (NTHREADS / 32)), 1, c);
-          narrow_forward_kernel<2><<<grid, NTHREADS, 0, st>>>(p->d, f, p->n, p->batch, flags, p->energy);
+          narrow_forward_kernel<2, false><<<grid, NTHREADS, 0, st>>>(p->d, f, p->n, p->batch, flags, p->energy);
         }
         else
         {
           dim3 grid(cdiv(p->batch, NTHREADS / 32), 1, c);
-          narrow_forward_kernel<1><<<grid, NTHREADS, 0, st>>>(p->d, f, p->n, p->batch, flags, p->energy);
+          auto kern = simple ? narrow_forward_kernel<1, true> : narrow_forward_kernel<1, false>;
+          kern<<<grid, NTHREADS, 0, st>>>(p->d, f, p->n, p->batch, flags, p->energy);
         }
       }
       else
@@ -1178,18 +1180,23 @@ static int launch_dfa_group(dpc_plan* p, int i, int c, int from_output, bool v, 
   for (int k = i; k < j && wide; ++k)
     wide = p->h[k].next_size <= 0 || p->h[k].next_size % 128 == 0;
   const int ts4 = cdiv(std::max(p->h[i].terminal_size, 1), 4);
-  if (wide && ts4 <= 4 && cdiv(mxn, 128) * c >= 2 * p->ctx->sm_count)
+  const long long strips = (long long)cdiv(mxn, 128) * c;
+  if (wide && ts4 <= 4)
   {
-    // blocks of 128 columns x the whole batch
-    dim3 grid(cdiv(mxn, 128), c);
+    // blocks of 128 columns x the whole batch, or a share of it while there are fewer than four blocks
+    // per SM: FullPCN 3072-(1024x4)-10 at batch 4096 has 32 strips
+    int rpb = cdiv(p->batch, 32) * 32;
+    while (rpb > 32 && strips * cdiv(p->batch, rpb) < 4 * p->ctx->sm_count)
+      rpb = cdiv(rpb / 2, 32) * 32;
+    dim3 grid(cdiv(mxn, 128), c, cdiv(p->batch, rpb));
     if (ts4 <= 1)
-      dfa_proj128_kernel<1><<<grid, 256, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, planes);
+      dfa_proj128_kernel<1><<<grid, 256, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, rpb, planes);
     else if (ts4 == 2)
-      dfa_proj128_kernel<2><<<grid, 256, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, planes);
+      dfa_proj128_kernel<2><<<grid, 256, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, rpb, planes);
     else if (ts4 == 3)
-      dfa_proj128_kernel<3><<<grid, 256, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, planes);
+      dfa_proj128_kernel<3><<<grid, 256, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, rpb, planes);
     else
-      dfa_proj128_kernel<4><<<grid, 256, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, planes);
+      dfa_proj128_kernel<4><<<grid, 256, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, rpb, planes);
   }
   else if (v)
   {
@@ -1280,10 +1287,10 @@ static int launch_bias_update(dpc_plan* p, int f, int c, int max_next, int grad_
   if (rc != DPC_OK)
     return rc;
   const FePlanes fp = fe_planes(p);
-  // 256 threads: blocks of 64 columns where the feedback error is read from its planes,
-  // one column per thread (grid-stride) elsewhere
+  // 256 threads: blocks of 64 columns where the feedback error is read from its planes or the batch is
+  // large, of 32 columns elsewhere (a block takes several where the layer's own kind differs)
   const bool by_blocks = fp.only || p->batch >= kBiasBlockRows;
-  dim3 gb(std::max(1, cdiv(max_next, by_blocks ? 64 : 256)), c);
+  dim3 gb(std::max(1, cdiv(max_next, by_blocks ? 64 : 32)), c);
   launch_row_split(bias_update_kernel, gb, 256,
                    by_blocks ? row_split(p->ctx, (long long)gb.x * c, p->batch, 256) : 1, p->ctx->stream, p->d,
                    f, p->n, p->batch, grad_only, fp);

@@ -193,8 +193,8 @@ __device__ __forceinline__ float warp_reduce16(float (&a)[16], int lane)
 }
 
 // RPW batch rows per warp (2 on large batches: every weight vector fetched from L1 then serves two
-// rows).
-template <int RPW>
+// rows).  SIMPLE: SimplePC layers, whose operand is f(z).
+template <int RPW, bool SIMPLE>
 __global__ void __launch_bounds__(NTHREADS)
     narrow_forward_kernel(const dpc_layer* __restrict__ layers, int first, int n_layers, int batch,
                           int flags, double* energy)
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(NTHREADS)
   if (L.next_size <= 0)
     return;
   const int N = L.next_size, K = L.size;
-  const bool simple = (L.flags & DPC_LAYER_INPUT_ACT) != 0;
+  constexpr bool simple = SIMPLE;
   const dpc_layer* Lup = (li + 1 < n_layers) ? &layers[li + 1] : nullptr;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = (blockIdx.x * (NTHREADS / 32) + warp) * RPW;
@@ -1011,14 +1011,15 @@ __global__ void __launch_bounds__(64)
 }
 
 // The aligned projection for wide layers (next_size a multiple of 128) when there are enough
-// layers to fill the GPU with blocks of 128 columns x the whole batch: the 128 rows of Psi a
+// rows to fill the GPU with blocks of 128 columns x at least 128 rows: the 128 rows of Psi a
 // block needs come in through shared memory with coalesced loads ONCE per block (the kernel above
 // re-reads them with strided loads for every 128 batch rows), lane l of every warp owns columns
 // 4l..4l+3, warp w the batch rows w, w+8, ...: every access of a warp is one whole row segment.
 template <int TS4>
 __global__ void __launch_bounds__(256)
     dfa_proj128_kernel(const dpc_layer* __restrict__ layers, int first, int n_layers, int batch,
-                       const float* __restrict__ eT, int from_output, FePlanes planes)
+                       const float* __restrict__ eT, int from_output, int rows_per_block,
+                       FePlanes planes)
 {
   const int li = first + blockIdx.y;
   if (li + 1 >= n_layers)
@@ -1052,16 +1053,17 @@ __global__ void __launch_bounds__(256)
   __nv_bfloat16* hi = fe_plane_of(planes, li);
   const bool keep_fp32 = !(hi && planes.only);
   const int j = j0 + 4 * lane;
-  for (int b0 = 0; b0 < batch; b0 += ROWS)
+  const int b_begin = blockIdx.z * rows_per_block, b_end = min(batch, b_begin + rows_per_block);
+  for (int b0 = b_begin; b0 < b_end; b0 += ROWS)
   {
     __syncthreads();
     for (int idx = threadIdx.x; idx < ROWS * KC; idx += 256)
     {
       const int r = idx / KC, k = idx - r * KC;
-      es[r][k] = (b0 + r < batch && k < TS) ? eT[(size_t)(b0 + r) * TS + k] : 0.0f;
+      es[r][k] = (b0 + r < b_end && k < TS) ? eT[(size_t)(b0 + r) * TS + k] : 0.0f;
     }
     __syncthreads();
-    const int rows = min(ROWS, batch - b0);
+    const int rows = min(ROWS, b_end - b0);
 #pragma unroll 4
     for (int r = warp; r < rows; r += 8)
     {
@@ -1227,25 +1229,68 @@ __global__ void bias_update_kernel(const dpc_layer* __restrict__ layers, int fir
     return;
   }
   if (rank != 0)
-    return; // (a row-split launch over a layer that takes the column loop: one CTA does it all)
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
+    return; // (a row-split launch over a layer that takes the column sums: one CTA does them)
+  // Column sums in row order (the reference's): 32 columns at a time, the block copies groups of rows
+  // into shared memory, one buffer ahead, and one warp adds them up, a chain of dependent additions
+  // and nothing else.  (A thread that loads what it adds pays a memory latency every few rows: 145 us
+  // for a ten-column head at batch 4096.)
+  constexpr int CR = 64;
+  __shared__ float stage[2][CR][33];
+  const int cols = n < 32 ? n : 32, per = 256 / cols; // threads that copy one row, rows per round
+  const int cj = threadIdx.x % cols, cr = threadIdx.x / cols;
+  for (int j0 = blockIdx.x * 32; j0 < n; j0 += gridDim.x * 32)
   {
+    const int width = min(32, n - j0);
+    auto value = [&](int b)
+    {
+      const size_t o = (size_t)b * n + j0 + cj;
+      return hi ? __bfloat162float(hi[o]) + __bfloat162float(hi[planes.elems + o]) : g[o];
+    };
+    auto copy = [&](int b0, int buf)
+    {
+      if (cr < per && cj < width)
+#pragma unroll 8
+        for (int r = cr; r < CR; r += per)
+          if (b0 + r < batch)
+            stage[buf][r][cj] = value(b0 + r);
+    };
     float s = 0.0f;
-    if (hi)
-      for (int b = 0; b < batch; ++b)
-        s += __bfloat162float(hi[(size_t)b * n + j]) +
-             __bfloat162float(hi[planes.elems + (size_t)b * n + j]);
-    else
-      for (int b = 0; b < batch; ++b)
-        s += g[(size_t)b * n + j];
-    bias_apply(L, j, s, batch, grad_only);
+    copy(0, 0);
+    for (int b0 = 0, buf = 0; b0 < batch; b0 += CR, buf ^= 1)
+    {
+      __syncthreads();
+      copy(b0 + CR, buf ^ 1);
+      if (threadIdx.x < (unsigned)width)
+      {
+        const int rows = min(CR, batch - b0);
+        int r = 0;
+        for (; r + 16 <= rows; r += 16)
+        {
+          float v[16];
+#pragma unroll
+          for (int q = 0; q < 16; ++q)
+            v[q] = stage[buf][r + q][threadIdx.x];
+#pragma unroll
+          for (int q = 0; q < 16; ++q)
+            s += v[q];
+        }
+        for (; r < rows; ++r)
+          s += stage[buf][r][threadIdx.x];
+      }
+    }
+    if (threadIdx.x < (unsigned)width)
+      bias_apply(L, j0 + threadIdx.x, s, batch, grad_only);
+    __syncthreads();
   }
 }
 
-// One entry of the feedback-weight update: Psi[row][k] takes the raw sum over the batch of
-// z[b][row] * e_T[b][k] (SGD with optional decay, Adam, AdamW, or the sum itself into g_Psi).
+// `step`: adam_step_size of the layer (two powers and a root: once per thread, not per element)
+__device__ __forceinline__ float psi_step(const dpc_layer& L, float rate, int grad_only)
+{
+  return grad_only || L.opt_psi == DPC_OPT_SGD ? 0.0f : adam_step_size(rate, *L.t_Psi);
+}
 __device__ __forceinline__ void psi_apply(const dpc_layer& L, int row, int k, float sum, int batch,
-                                          int grad_only, bool full_kind, float rate)
+                                          int grad_only, bool full_kind, float rate, float step)
 {
   const size_t o = (size_t)row * L.psi_stride + k;
   if (grad_only)
@@ -1260,7 +1305,6 @@ __device__ __forceinline__ void psi_apply(const dpc_layer& L, int row, int k, fl
   }
   else
   {
-    const float step = adam_step_size(rate, *L.t_Psi);
     float lr_wd = -1.0f;
     if (L.opt_psi == DPC_OPT_ADAMW)
       lr_wd = rate * ((!full_kind && L.psi_decay >= 0.0f) ? L.psi_decay : L.lmbda);
@@ -1397,12 +1441,13 @@ __global__ void __launch_bounds__(256)
   float acc[4][KC];
   if (!batch_outer4<KC>(L.z, s, col, eT, TS, TS, batch, acc, es, part))
     return;
+  const float step = psi_step(L, rate, grad_only);
 #pragma unroll
   for (int c = 0; c < 4; ++c)
 #pragma unroll
     for (int k = 0; k < KC; ++k)
       if (k < TS)
-        psi_apply(L, col + c, k, acc[c][k], batch, grad_only, full_kind, rate);
+        psi_apply(L, col + c, k, acc[c][k], batch, grad_only, full_kind, rate, step);
 }
 
 // State update of a layer below a narrow one (at most KC <= 16 units above, own width a multiple of
@@ -1512,7 +1557,7 @@ __global__ void __launch_bounds__(256)
 // One entry of a weight update from the raw sum over the batch (the epilogue of
 // pc_gemm_kernel<OP_WG> for one element).
 __device__ __forceinline__ void weight_apply(const dpc_layer& L, size_t o, float sum, int batch,
-                                             int mode, int flags, bool simple)
+                                             int mode, int flags, bool simple, float step)
 {
   if (mode & WG_GRAD_ONLY)
   {
@@ -1527,7 +1572,7 @@ __device__ __forceinline__ void weight_apply(const dpc_layer& L, size_t o, float
     if (L.opt == DPC_OPT_ADAMW)
       lr_wd = L.lr * L.lmbda;
     float mm = L.m_W[o], vv = L.v_W[o];
-    w = adam_update(w, -1.0f * L.a * sum, mm, vv, adam_step_size(L.lr, *L.t), lr_wd);
+    w = adam_update(w, -1.0f * L.a * sum, mm, vv, step, lr_wd);
     L.m_W[o] = mm;
     L.v_W[o] = vv;
   }
@@ -1581,12 +1626,13 @@ __global__ void __launch_bounds__(256)
   float acc[4][KC];
   if (!batch_outer4<KC>(zin, s, col, g, M, M, batch, acc, es, part))
     return;
+  const float step = mode == WG_LEARN && L.opt != DPC_OPT_SGD ? adam_step_size(L.lr, *L.t) : 0.0f;
 #pragma unroll
   for (int c = 0; c < 4; ++c)
 #pragma unroll
     for (int k = 0; k < KC; ++k)
       if (k < M)
-        weight_apply(L, (size_t)k * s + col + c, acc[c][k], batch, mode, flags, simple);
+        weight_apply(L, (size_t)k * s + col + c, acc[c][k], batch, mode, flags, simple, step);
 }
 
 // Feedback-weight update Psi[l] (+)= (fl*a/B) z[l]^T e_T.  A block of 256 threads owns 64 rows of
@@ -1607,6 +1653,7 @@ __global__ void __launch_bounds__(256)
   const int TS = L.terminal_size, s = L.size;
   const bool full_kind = (L.flags & DPC_LAYER_FULLPC_PSI) != 0;
   const float rate = full_kind ? L.fl * L.a : L.fl;
+  const float step = psi_step(L, rate, grad_only);
   constexpr int PSI_ROWS = 64, GROUPS = 4, COLS = 64;
   __shared__ __align__(16) float es[PSI_ROWS][16];
   __shared__ float part[GROUPS][COLS][17];
@@ -1664,7 +1711,7 @@ __global__ void __launch_bounds__(256)
           if (k >= kn)
             continue;
           const float sum = ((part[0][rc][k] + part[1][rc][k]) + part[2][rc][k]) + part[3][rc][k];
-          psi_apply(L, row, kc + k, sum, batch, grad_only, full_kind, rate);
+          psi_apply(L, row, kc + k, sum, batch, grad_only, full_kind, rate, step);
         }
       }
       __syncthreads();

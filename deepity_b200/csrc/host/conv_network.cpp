@@ -32,12 +32,13 @@ void SimpleConvPCNetwork::RequireCompiled() const
     throw std::logic_error("deepity_b200: network used before Compile()");
 }
 
-SimpleConvPCNetwork::SimpleConvPCNetwork(int batchSize, DeviceType device, int deviceIndex)
+SimpleConvPCNetwork::SimpleConvPCNetwork(int batchSize, DeviceType deviceType, int deviceIndex)
     : batchSize(batchSize)
+    , device(deviceIndex)
 {
   if (batchSize <= 0)
     throw std::invalid_argument("deepity_b200: batch size must be positive");
-  if (device != DeviceType::DEVICE_GPU)
+  if (deviceType != DeviceType::DEVICE_GPU)
     throw std::invalid_argument("deepity_b200: this build has no CPU backend");
   Check(dpc_create(deviceIndex, &ctx));
 }
@@ -275,8 +276,17 @@ void SimpleConvPCNetwork::ClampRaw(int layer, const float* data, size_t n, bool 
   else
   {
     float* stage = layer == 0 ? pinnedX : pinnedY;
-    std::memcpy(stage, data, count * sizeof(float));
-    Check(dpc_copy_h2d(ctx, l->d.z, stage, count * sizeof(float)));
+    if (count >= HostCopier::kMinFloats)
+    {
+      if (!copier)
+        copier = HostCopier::Shared();
+      Check(copier->Upload(ctx, device, l->d.z, stage, data, count));
+    }
+    else
+    {
+      std::memcpy(stage, data, count * sizeof(float));
+      Check(dpc_copy_h2d(ctx, l->d.z, stage, count * sizeof(float)));
+    }
   }
   l->clamped = true;
   l->cacheValid = false;

@@ -100,7 +100,8 @@ private:
   void ForwardLayer(int i, int flags);
   void Settle(int steps);
 
-  int batchSize;
+  int batchSize, device;
+  std::shared_ptr<HostCopier> copier; // large inputs only
   dpc_ctx* ctx = nullptr;
   dpc_conv_plan* plan = nullptr;
   std::vector<std::unique_ptr<SimpleConvPCLayer>> layers;

@@ -36,6 +36,7 @@ void PCNetwork::RequireCompiled() const
 PCNetwork::PCNetwork(NetworkKind kind, int batchSize, int device)
     : kind(kind)
     , batchSize(batchSize)
+    , device(device)
 {
   if (batchSize <= 0)
     throw std::invalid_argument("deepity_b200: batch size must be positive");
@@ -501,8 +502,17 @@ void PCNetwork::ClampHost(int layer, const float* data, size_t n)
   }
   else
   {
-    std::memcpy(stage, data, count * sizeof(float));
-    Check(dpc_copy_h2d(ctx, l->d.z, stage, count * sizeof(float)));
+    if (count >= HostCopier::kMinFloats)
+    {
+      if (!copier)
+        copier = HostCopier::Shared();
+      Check(copier->Upload(ctx, device, l->d.z, stage, data, count));
+    }
+    else
+    {
+      std::memcpy(stage, data, count * sizeof(float));
+      Check(dpc_copy_h2d(ctx, l->d.z, stage, count * sizeof(float)));
+    }
   }
   Check(dpc_plan_invalidate(plan, layer, 1, DPC_WROTE_Z));
   l->clamped = true;

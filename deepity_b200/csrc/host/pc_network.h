@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "deepity_b200.h"
+#include "host_copy.h"
 
 namespace Deep
 {
@@ -222,7 +223,8 @@ private:
   void RunPredictPhases(int steps, bool withProjection);
 
   NetworkKind kind;
-  int batchSize;
+  int batchSize, device;
+  std::shared_ptr<HostCopier> copier; // large inputs only
   dpc_ctx* ctx = nullptr;
   dpc_plan* plan = nullptr;
   std::vector<std::unique_ptr<PCLayer>> layers;
