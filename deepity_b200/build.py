@@ -25,10 +25,9 @@ CSRC = os.path.join(PKG, "csrc")
 OUT = os.path.join(PKG, "libdeepity_b200.so")
 
 SOURCES = ["dpc_core.cu", "dpc_tc.cu", "dpc_static.cu", "dpc_conv.cu", "dpc_resident.cu", "dpc_conv_resident.cu",
-           os.path.join("host", "pc_network.cpp"), os.path.join("host", "conv_network.cpp"),
-           os.path.join("host", "host_copy.cpp")]
+           os.path.join("host", "pc_network.cpp"), os.path.join("host", "conv_network.cpp")]
 HEADERS = ["dpc_internal.h", "dpc_math.cuh", "dpc_simt.cuh", os.path.join("host", "pc_network.h"),
-           os.path.join("host", "conv_network.h"), os.path.join("host", "host_copy.h"),
+           os.path.join("host", "conv_network.h"),
            os.path.join(ROOT, "include", "deepity_b200.h")]
 
 

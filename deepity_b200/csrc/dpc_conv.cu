@@ -989,10 +989,23 @@ int dpc_conv_energy_reset(dpc_conv_plan* p)
 
 int dpc_conv_energy_read(dpc_conv_plan* p, double* out)
 {
-  if (!p || !out)
-    return fail(DPC_ERR_INVALID, "bad argument");
+  const int rc = dpc_conv_energy_fetch(p);
+  return rc == DPC_OK ? dpc_conv_energy_wait(p, out) : rc;
+}
+
+int dpc_conv_energy_fetch(dpc_conv_plan* p)
+{
+  if (!p)
+    return fail(DPC_ERR_INVALID, "null plan");
   DPC_CUDA(cudaMemcpyAsync(p->energy_host, p->energy, sizeof(double), cudaMemcpyDeviceToHost,
                            p->ctx->stream));
+  return DPC_OK;
+}
+
+int dpc_conv_energy_wait(dpc_conv_plan* p, double* out)
+{
+  if (!p || !out)
+    return fail(DPC_ERR_INVALID, "bad argument");
   DPC_CUDA(cudaStreamSynchronize(p->ctx->stream));
   *out = *p->energy_host;
   return DPC_OK;

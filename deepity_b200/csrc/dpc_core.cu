@@ -468,13 +468,13 @@ int dpc_plan_create(dpc_ctx* ctx, const dpc_layer* layers, int n_layers, int bat
   p->init_precision = ctx->precision;
   cudaError_t err = cudaMalloc(&p->d, sizeof(dpc_layer) * n_layers);
   if (err == cudaSuccess)
-    err = cudaMalloc(&p->energy, sizeof(double));
+    err = cudaMalloc(&p->energy, 2 * sizeof(double));
   if (err == cudaSuccess)
-    err = cudaMallocHost(&p->energy_host, sizeof(double));
+    err = cudaMallocHost(&p->energy_host, 2 * sizeof(double));
   if (err == cudaSuccess)
     err = cudaMemcpy(p->d, layers, sizeof(dpc_layer) * n_layers, cudaMemcpyHostToDevice);
   if (err == cudaSuccess)
-    err = cudaMemset(p->energy, 0, sizeof(double));
+    err = cudaMemset(p->energy, 0, 2 * sizeof(double));
   if (err != cudaSuccess)
   {
     dpc_plan_destroy(p);
@@ -1508,9 +1508,29 @@ int dpc_energy_read(dpc_plan* p, double* out)
 {
   if (!p || !out)
     return fail(DPC_ERR_INVALID, "null argument");
-  DPC_CUDA(cudaMemcpyAsync(p->energy_host, p->energy, sizeof(double), cudaMemcpyDeviceToHost,
+  const int rc = dpc_energy_fetch(p);
+  return rc == DPC_OK ? dpc_energy_wait(p, out) : rc;
+}
+
+int dpc_energy_fetch(dpc_plan* p)
+{
+  if (!p)
+    return fail(DPC_ERR_INVALID, "null plan");
+  DPC_CUDA(cudaMemcpyAsync(p->energy_host, p->energy, 2 * sizeof(double), cudaMemcpyDeviceToHost,
                            p->ctx->stream));
+  return DPC_OK;
+}
+
+int dpc_energy_wait(dpc_plan* p, double* out)
+{
+  if (!p || !out)
+    return fail(DPC_ERR_INVALID, "null argument");
   DPC_CUDA(cudaStreamSynchronize(p->ctx->stream));
   *out = *p->energy_host;
-  return tc_check_error(p);
+  if (*reinterpret_cast<int*>(p->energy_host + 1) != 0)
+  {
+    DPC_CUDA(cudaMemsetAsync(p->status(), 0, sizeof(int), p->ctx->stream));
+    return fail(DPC_ERR_TIMEOUT, "a tensor-core kernel gave up waiting on a pipeline barrier");
+  }
+  return DPC_OK;
 }

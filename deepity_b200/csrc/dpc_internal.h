@@ -60,8 +60,11 @@ struct dpc_plan
   int init_precision = 0; // the context's when the tensor-core and row-segment state was built
   std::vector<dpc_layer> h; // host copy of the table
   dpc_layer* d = nullptr;   // device copy
-  double* energy = nullptr; // device accumulator
-  double* energy_host = nullptr; // pinned
+  // device accumulator, followed by the status word that the tensor-core kernels raise when a bounded
+  // wait runs out: one copy brings both
+  double* energy = nullptr;
+  double* energy_host = nullptr; // pinned, same layout
+  int* status() const { return reinterpret_cast<int*>(energy + 1); }
   const float* e_terminal = nullptr; // terminal error the DFA / Psi kernels read
   dpc::TensorRun run;
   void* tc = nullptr; // tensor-core path state (tensor maps), owned by dpc_tc.cu
@@ -84,9 +87,6 @@ int tc_update_state(dpc_plan* plan, int first, int count, bool feed);
 int tc_project_forward(dpc_plan* plan, int first, int count, int flags);
 // mode: 0 learn, 1 direct feedback, +2: only store the raw sums in the layers' g_W.
 int tc_weight_gemm(dpc_plan* plan, int first, int count, int mode, int decay_w = 0);
-// Synchronous: reads the device-side status flag the kernels raise when a bounded wait runs
-// out; DPC_ERR_TIMEOUT if it was raised.
-int tc_check_error(dpc_plan* plan);
 void tc_set_chain_trace(dpc_plan* plan, unsigned long long* buf);
 // Operand planes (bf16 hi/mid copies of the run's beliefs, feedback errors and weights that the
 // 3xBF16 kernels read).  tc_touch: something outside dpc_tc.cu wrote the fp32 tensors `kind`

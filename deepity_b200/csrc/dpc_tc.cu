@@ -83,8 +83,6 @@ struct TcState
   bool up_maps = false;
   int* chain_counters = nullptr; // device: [layers of the run][row blocks]
   unsigned long long* trace = nullptr; // optional timing trace buffer of the chain kernel
-  int* error_flag = nullptr; // device
-  int* error_host = nullptr; // pinned
   int max_smem = 0;
   long long wait_cycles = kWaitCyclesDefault;
   int chain_target_bias = 0; // test hook: added to the sweep's publication target
@@ -2000,11 +1998,6 @@ int tc_plan_init(dpc_plan* plan)
     }
     i = j;
   }
-  if (cudaMalloc(&st->error_flag, sizeof(int)) != cudaSuccess ||
-      cudaMemset(st->error_flag, 0, sizeof(int)) != cudaSuccess ||
-      cudaMallocHost(&st->error_host, sizeof(int)) != cudaSuccess)
-    return DPC_OK;
-  *st->error_host = 0;
   if (best_count >= 1 && !run_init(plan, st, best_first, best_count))
     best_count = 0;
   // Layers outside the run whose three products fit the 256 x 256 CTA-pair tiles.
@@ -2154,12 +2147,8 @@ void tc_plan_free(dpc_plan* plan)
   auto* st = static_cast<TcState*>(plan->tc);
   if (!st)
     return;
-  if (st->error_flag)
-    cudaFree(st->error_flag);
   if (st->chain_counters)
     cudaFree(st->chain_counters);
-  if (st->error_host)
-    cudaFreeHost(st->error_host);
   planes_free(st);
   delete st;
   plan->tc = nullptr;
@@ -2171,23 +2160,6 @@ void tc_set_chain_trace(dpc_plan* plan, unsigned long long* buf)
   auto* st = static_cast<TcState*>(plan->tc);
   if (st)
     st->trace = buf;
-}
-
-int tc_check_error(dpc_plan* plan)
-{
-  auto* st = static_cast<TcState*>(plan->tc);
-  if (!st || !st->ok)
-    return DPC_OK;
-  if (cudaMemcpyAsync(st->error_host, st->error_flag, sizeof(int), cudaMemcpyDeviceToHost,
-                      plan->ctx->stream) != cudaSuccess ||
-      cudaStreamSynchronize(plan->ctx->stream) != cudaSuccess)
-    return fail(DPC_ERR_CUDA, "reading the tensor-core status flag failed");
-  if (*st->error_host)
-  {
-    cudaMemsetAsync(st->error_flag, 0, sizeof(int), plan->ctx->stream);
-    return fail(DPC_ERR_TIMEOUT, "a tensor-core kernel gave up waiting on a pipeline barrier");
-  }
-  return DPC_OK;
 }
 
 // CTA-pair kernels take 256 x 256 tiles; DPC_DISABLE_CTA_PAIRS keeps the single-CTA kernels
@@ -2325,7 +2297,7 @@ static TcParams base_params(dpc_plan* p, TcState* st, int first, int count, int 
   P.flags = flags;
   P.mode = mode;
   P.energy = p->energy;
-  P.error_flag = st->error_flag;
+  P.error_flag = p->status();
   P.chain = 0;
   P.chain_counters = nullptr;
   P.chain_target = 0;

@@ -32,13 +32,12 @@ void SimpleConvPCNetwork::RequireCompiled() const
     throw std::logic_error("deepity_b200: network used before Compile()");
 }
 
-SimpleConvPCNetwork::SimpleConvPCNetwork(int batchSize, DeviceType deviceType, int deviceIndex)
+SimpleConvPCNetwork::SimpleConvPCNetwork(int batchSize, DeviceType device, int deviceIndex)
     : batchSize(batchSize)
-    , device(deviceIndex)
 {
   if (batchSize <= 0)
     throw std::invalid_argument("deepity_b200: batch size must be positive");
-  if (deviceType != DeviceType::DEVICE_GPU)
+  if (device != DeviceType::DEVICE_GPU)
     throw std::invalid_argument("deepity_b200: this build has no CPU backend");
   Check(dpc_create(deviceIndex, &ctx));
 }
@@ -51,9 +50,8 @@ SimpleConvPCNetwork::~SimpleConvPCNetwork()
     dpc_conv_plan_destroy(plan);
   for (void* p : allocations)
     dpc_free(ctx, p);
-  for (float* p : {pinnedX, pinnedY, pinnedOut})
-    if (p)
-      dpc_free_host(ctx, p);
+  if (pinnedOut)
+    dpc_free_host(ctx, pinnedOut);
   if (ctx)
     dpc_destroy(ctx);
 }
@@ -157,11 +155,7 @@ void SimpleConvPCNetwork::Compile()
     }
   }
   void* p = nullptr;
-  const size_t inN = B * layers.front()->GetInputSize(), outN = B * layers.back()->GetInputSize();
-  Check(dpc_alloc_host(ctx, inN * sizeof(float), &p));
-  pinnedX = static_cast<float*>(p);
-  Check(dpc_alloc_host(ctx, outN * sizeof(float), &p));
-  pinnedY = static_cast<float*>(p);
+  const size_t outN = B * layers.back()->GetInputSize();
   Check(dpc_alloc_host(ctx, outN * sizeof(float), &p));
   pinnedOut = static_cast<float*>(p);
   std::vector<dpc_conv_layer> table;
@@ -275,18 +269,7 @@ void SimpleConvPCNetwork::ClampRaw(int layer, const float* data, size_t n, bool 
     Check(dpc_copy_d2d(ctx, l->d.z, data, count * sizeof(float)));
   else
   {
-    float* stage = layer == 0 ? pinnedX : pinnedY;
-    if (count >= HostCopier::kMinFloats)
-    {
-      if (!copier)
-        copier = HostCopier::Shared();
-      Check(copier->Upload(ctx, device, l->d.z, stage, data, count));
-    }
-    else
-    {
-      std::memcpy(stage, data, count * sizeof(float));
-      Check(dpc_copy_h2d(ctx, l->d.z, stage, count * sizeof(float)));
-    }
+    Check(dpc_copy_h2d(ctx, l->d.z, data, count * sizeof(float))); // (see PCNetwork::ClampHost)
   }
   l->clamped = true;
   l->cacheValid = false;
@@ -412,6 +395,7 @@ float SimpleConvPCNetwork::TrainStepRaw(const float* x, size_t nx, const float* 
       for (auto& l : layers)
         l->gateIsPrediction = true;
       layers.front()->cacheValid = true;
+      Check(dpc_conv_energy_fetch(plan));
       return;
     }
     if (withProjection)
@@ -420,6 +404,7 @@ float SimpleConvPCNetwork::TrainStepRaw(const float* x, size_t nx, const float* 
     UpdateWeights();
     Check(dpc_conv_energy_reset(plan));
     CalculateState(true);
+    Check(dpc_conv_energy_fetch(plan));
   };
   if (useGraph)
   {
@@ -453,7 +438,7 @@ float SimpleConvPCNetwork::TrainStepRaw(const float* x, size_t nx, const float* 
   else
     phases();
   double energy = 0.0;
-  Check(dpc_conv_energy_read(plan, &energy));
+  Check(dpc_conv_energy_wait(plan, &energy));
   layers.back()->clamped = false;
   return (float)energy;
 }

@@ -100,13 +100,12 @@ private:
   void ForwardLayer(int i, int flags);
   void Settle(int steps);
 
-  int batchSize, device;
-  std::shared_ptr<HostCopier> copier; // large inputs only
+  int batchSize;
   dpc_ctx* ctx = nullptr;
   dpc_conv_plan* plan = nullptr;
   std::vector<std::unique_ptr<SimpleConvPCLayer>> layers;
   std::vector<void*> allocations;
-  float *pinnedX = nullptr, *pinnedY = nullptr, *pinnedOut = nullptr;
+  float* pinnedOut = nullptr;
   OptimizerType opt = OptimizerType::SGD;
   bool centerWeights = false, useGraph = true, dirty = false, structureDirty = false, phasesRecorded = false;
   long graphKey[4] = {-1, -1, -1, -1};

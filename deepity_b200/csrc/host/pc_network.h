@@ -16,7 +16,6 @@
 #include <vector>
 
 #include "deepity_b200.h"
-#include "host_copy.h"
 
 namespace Deep
 {
@@ -220,23 +219,21 @@ private:
   void RowSegment(int ops, int steps);
   void RunTrainSegments(int mode, int steps);
   void RunTrainPhases(int mode, int steps);
+  void RunGroupedPhases(int mode, int steps);
   void RunPredictPhases(int steps, bool withProjection);
 
   NetworkKind kind;
-  int batchSize, device;
-  std::shared_ptr<HostCopier> copier; // large inputs only
+  int batchSize;
   dpc_ctx* ctx = nullptr;
   dpc_plan* plan = nullptr;
   std::vector<std::unique_ptr<PCLayer>> layers;
   std::vector<void*> allocations;
-  float* pinnedX = nullptr;
-  float* pinnedY = nullptr;
   float* pinnedOut = nullptr;
+  bool adamAllocated = false, psiAdamAllocated = false;
 
   OptimizerType opt = OptimizerType::SGD, optPsi = OptimizerType::SGD;
   bool centerWeights = false, crossEntropy = false, useMuPC = false, useResidual = false;
   bool useEPC = false, useIPC = false, useMomentum = false, useGraph = true, dirty = false, ratesDirty = false;
-  bool adamAllocated = false, psiAdamAllocated = false, pendingAsync = false;
   float momentumBeta = 0.9f, psiDecay = -1.0f;
   bool ghostTop = false;
   float* ghostET = nullptr;

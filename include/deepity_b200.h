@@ -400,7 +400,11 @@ DPC_API int dpc_rows_segment(dpc_plan* plan, int ops, int steps, int top_clamped
                              int top_down_off);
 /* Energy accumulator of the plan (device-resident double). */
 DPC_API int dpc_energy_reset(dpc_plan* plan);
-DPC_API int dpc_energy_read(dpc_plan* plan, double* out); /* synchronous */
+DPC_API int dpc_energy_read(dpc_plan* plan, double* out); /* synchronous: fetch + wait */
+/* The two halves: a stream-ordered copy of energy and status (part of a recorded step), and the wait
+ * for the stream. */
+DPC_API int dpc_energy_fetch(dpc_plan* plan);
+DPC_API int dpc_energy_wait(dpc_plan* plan, double* out); /* synchronous */
 
 /* ------------------------------------------------------------------------------------
  * Networks with host buffers: the binding surface.  kind: 0 SimplePCNetwork,
@@ -549,7 +553,9 @@ DPC_API int dpc_conv_update_weights_range(dpc_conv_plan* plan, int first, int co
 DPC_API int dpc_conv_images_available(dpc_conv_plan* plan);
 DPC_API int dpc_conv_images_segment(dpc_conv_plan* plan, int ops, int steps, int top_clamped);
 DPC_API int dpc_conv_energy_reset(dpc_conv_plan* plan);
-DPC_API int dpc_conv_energy_read(dpc_conv_plan* plan, double* out); /* synchronous */
+DPC_API int dpc_conv_energy_read(dpc_conv_plan* plan, double* out); /* synchronous: fetch + wait */
+DPC_API int dpc_conv_energy_fetch(dpc_conv_plan* plan);
+DPC_API int dpc_conv_energy_wait(dpc_conv_plan* plan, double* out); /* synchronous */
 
 /* The network with host buffers (include/deepity/networks/SimpleConvPCNetwork.h:30-131,
  * bindings/NetworkBindings.cpp:1850-2000). */
