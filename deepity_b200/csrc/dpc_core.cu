@@ -87,25 +87,29 @@ static inline int cdiv(int a, int b)
   return (a + b - 1) / b;
 }
 
-// Largest GEMM tile grid over a range for the given op.
-static void max_tiles(const dpc_plan* p, int first, int count, int op, int& tx, int& ty)
+// Launches the grouped GEMM over layers [first, first+count): 64 x 64 tiles, or 32 x 32 where the former
+// are fewer than the SMs (a CTA walks all of K by itself: smaller tiles are more and shorter walks).
+template <int OP>
+static int launch_gemm(dpc_plan* p, int first, int count, int flags, int mode, const float* epc_src = nullptr)
 {
-  tx = ty = 0;
+  int mx = 0, my = 0;
+  long long tiles = 0;
   for (int i = first; i < first + count; ++i)
   {
     const dpc_layer& L = p->h[i];
     if (L.next_size <= 0)
       continue;
-    int M, N;
-    if (op == OP_FWD)
-      M = p->batch, N = L.next_size;
-    else if (op == OP_FB)
-      M = p->batch, N = L.size;
-    else
-      M = L.next_size, N = L.size;
-    tx = std::max(tx, cdiv(N, BN));
-    ty = std::max(ty, cdiv(M, BM));
+    const int M = OP == OP_WG ? L.next_size : p->batch, N = OP == OP_FWD ? L.next_size : L.size;
+    mx = std::max(mx, N), my = std::max(my, M);
+    tiles += (long long)cdiv(M, 64) * cdiv(N, 64);
   }
+  if (tiles == 0)
+    return DPC_OK;
+  const int T = tiles < p->ctx->sm_count ? 32 : 64;
+  dim3 grid(cdiv(mx, T), cdiv(my, T), count);
+  auto kern = T == 32 ? pc_gemm_kernel<OP, 32> : pc_gemm_kernel<OP, 64>;
+  kern<<<grid, NTHREADS, 0, p->ctx->stream>>>(p->d, first, p->n, p->batch, flags, mode, p->energy, epc_src);
+  return check_launch(p->ctx, "grouped GEMM kernel");
 }
 
 static int elem_blocks(const dpc_plan* p, size_t max_elems)
@@ -667,10 +671,6 @@ static int forward_simt(dpc_plan* p, int first, int count, int flags)
     }
     else
     {
-      int tx, ty;
-      max_tiles(p, f, c, OP_FWD, tx, ty);
-      if (tx == 0)
-        continue;
       // heads (at most 16 output units) with vector-loadable rows: one warp per batch row
       bool narrow = true;
       for (int i = f; i < f + c && narrow; ++i)
@@ -692,9 +692,10 @@ static int forward_simt(dpc_plan* p, int first, int count, int flags)
       }
       else
       {
-        dim3 grid(tx, ty, c);
-        pc_gemm_kernel<OP_FWD><<<grid, NTHREADS, 0, st>>>(p->d, f, p->n, p->batch, flags, 0,
-                                                         p->energy);
+        const int rc = launch_gemm<OP_FWD>(p, f, c, flags, 0);
+        if (rc != DPC_OK)
+          return rc;
+        continue;
       }
     }
     int rc = check_launch(p->ctx, "forward kernel");
@@ -958,7 +959,6 @@ static int update_state_simt(dpc_plan* p, int first, int count)
   for (int f = first; f < first + count; f += kMaxZ)
   {
     const int c = std::min(kMaxZ, first + count - f);
-    int tx, ty;
     // Layers whose upper neighbour does not exist are handled by the relax kernel below.
     int cg = (f + c == p->n) ? c - 1 : c;
     int narrow_kc = cg > 0 ? narrow_above(p, f, cg) : 0;
@@ -983,15 +983,9 @@ static int update_state_simt(dpc_plan* p, int first, int count)
     }
     else if (cg > 0)
     {
-      max_tiles(p, f, cg, OP_FB, tx, ty);
-      if (tx > 0)
-      {
-        dim3 grid(tx, ty, cg);
-        pc_gemm_kernel<OP_FB><<<grid, NTHREADS, 0, st>>>(p->d, f, p->n, p->batch, 0, 0, p->energy);
-        int rc = check_launch(p->ctx, "update_state kernel");
-        if (rc != DPC_OK)
-          return rc;
-      }
+      const int rc = launch_gemm<OP_FB>(p, f, cg, 0, FB_STATE);
+      if (rc != DPC_OK)
+        return rc;
     }
     bool any_weightless = false;
     size_t mx = 0;
@@ -1073,10 +1067,7 @@ int dpc_epc_adjoint(dpc_plan* p, int layer, int from_terminal, float scale, int 
   } u;
   u.f = scale;
   const int packed = (u.i & ~1) | (clamped ? 1 : 0);
-  dim3 grid(cdiv(L.size, BN), cdiv(p->batch, BM), 1);
-  pc_gemm_kernel<OP_FB><<<grid, NTHREADS, 0, st>>>(p->d, layer, p->n, p->batch, packed, FB_ADJOINT,
-                                                  p->energy, src);
-  return check_launch(p->ctx, "epc_adjoint kernel");
+  return launch_gemm<OP_FB>(p, layer, 1, packed, FB_ADJOINT, src);
 }
 
 int dpc_relax(dpc_plan* p, int layer)
@@ -1097,7 +1088,6 @@ static int weight_gemm_simt(dpc_plan* p, int first, int count, int mode, int fla
   for (int f = first; f < first + count; f += kMaxZ)
   {
     const int c = std::min(kMaxZ, first + count - f);
-    int tx, ty;
     const int narrow_kc = narrow_above(p, f, c);
     bool staged_ok = true;
     for (int i = f; i < f + c; ++i)
@@ -1121,13 +1111,7 @@ static int weight_gemm_simt(dpc_plan* p, int first, int count, int mode, int fla
         return rc;
       continue;
     }
-    max_tiles(p, f, c, OP_WG, tx, ty);
-    if (tx == 0)
-      continue;
-    dim3 grid(tx, ty, c);
-    pc_gemm_kernel<OP_WG><<<grid, NTHREADS, 0, p->ctx->stream>>>(p->d, f, p->n, p->batch, flags,
-                                                                mode, p->energy);
-    int rc = check_launch(p->ctx, "weight kernel");
+    const int rc = launch_gemm<OP_WG>(p, f, c, flags, mode);
     if (rc != DPC_OK)
       return rc;
   }

@@ -9,7 +9,7 @@
 
 namespace dpc
 {
-constexpr int BM = 64, BN = 64, BK = 16, NTHREADS = 256, PAD = 4;
+constexpr int BK = 16, NTHREADS = 256;
 
 enum GemmOp
 {
@@ -34,75 +34,73 @@ enum
   FB_ADJOINT = 1 // ePC ComputeAdjoint + UpdateErrorEPC (fe holds src * f'(preact))
 };
 
-struct Tile
+// Operand tiles of the grouped GEMM below in shared memory, filled by cp.async several K steps ahead.
+//   K-major  (rows are the M/N index, k contiguous in memory): [T][BK + 4], element (row, k); threads
+//            read 16 bytes along k of the rows t, t + 16, ..: a pitch of 20 floats puts the 16-byte
+//            reads of eight neighbouring rows into distinct banks
+//   MN-major ([K, cols], cols contiguous): [BK][T], threads read T / 16 neighbouring columns
+template <int T, bool KMAJOR>
+constexpr int kTileFloats = KMAJOR ? T * (BK + 4) : BK * T;
+
+__device__ __forceinline__ void cp_async4(float* dst, const float* src, bool valid)
 {
-  float a[BK][BM + PAD];
-  float b[BK][BN + PAD];
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(valid ? 4 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, bool valid)
+{
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(valid ? 16 : 0)
+               : "memory");
+}
+
+// One 16-byte chunk of a tile (chunk index c < T * BK / 4); what lies outside the operand becomes zero.
+// vec: rows of the operand start on 16-byte boundaries and are multiples of four long.
+template <int J, typename F>
+__device__ __forceinline__ void tile_row(const float* p, F&& put)
+{
+  if (J == 4)
+  {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    put(0, v.x), put(1, v.y), put(J > 2 ? 2 : 0, v.z), put(J > 2 ? 3 : 0, v.w);
+  }
+  else
+  {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    put(0, v.x), put(1, v.y);
+  }
+}
+template <int T, bool KMAJOR>
+struct TileChunk
+{
+  int row, k;
+  __device__ __forceinline__ explicit TileChunk(int c)
+      : row(KMAJOR ? c / (BK / 4) : (c % (T / 4)) * 4), k(KMAJOR ? (c % (BK / 4)) * 4 : c / (T / 4))
+  {
+  }
+  __device__ __forceinline__ float* at(float* tile) const
+  {
+    return KMAJOR ? tile + row * (BK + 4) + k : tile + k * T + row;
+  }
+  __device__ __forceinline__ void load(float* tile, const float* __restrict__ G, int ld, int row0, int k0,
+                                       int nrows, int K, bool vec) const
+  {
+    float* dst = at(tile);
+    const int r = row0 + row, kk = k0 + k;
+    const bool in = r < nrows && kk < K;
+    const float* src = in ? (KMAJOR ? G + (size_t)r * ld + kk : G + (size_t)kk * ld + r) : G;
+    if (vec)
+    {
+      cp_async16(dst, src, in);
+      return;
+    }
+    const int left = KMAJOR ? K - kk : nrows - r;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      cp_async4(dst + j, in && j < left ? src + j : G, in && j < left);
+  }
 };
-
-// Operand whose rows are the M/N index with k contiguous: G[(row0+r)*ld + k0+k].
-template <bool kAct>
-__device__ __forceinline__ void fetch_kmajor(float (&reg)[4], const float* __restrict__ G, int ld,
-                                             int row0, int k0, int nrows, int K, bool vec,
-                                             int act)
-{
-  const int t = threadIdx.x;
-  const int r = row0 + (t >> 2), k = k0 + ((t & 3) << 2);
-  if (r < nrows && vec && k + 3 < K)
-  {
-    float4 v = *reinterpret_cast<const float4*>(G + (size_t)r * ld + k);
-    reg[0] = v.x, reg[1] = v.y, reg[2] = v.z, reg[3] = v.w;
-  }
-  else
-  {
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      reg[j] = (r < nrows && k + j < K) ? G[(size_t)r * ld + k + j] : 0.0f;
-  }
-  if (kAct)
-  {
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      reg[j] = (r < nrows && k + j < K) ? act_fwd(act, reg[j]) : 0.0f;
-  }
-}
-
-template <int COLS>
-__device__ __forceinline__ void stash_kmajor(float (*S)[COLS + PAD], const float (&reg)[4])
-{
-  const int t = threadIdx.x;
-  const int r = t >> 2, k = (t & 3) << 2;
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-    S[k + j][r] = reg[j];
-}
-
-// Operand stored [K, cols] with cols contiguous: G[(k0+k)*ld + col0+c].
-__device__ __forceinline__ void fetch_mnmajor(float (&reg)[4], const float* __restrict__ G, int ld,
-                                              int col0, int k0, int ncols, int K, bool vec)
-{
-  const int t = threadIdx.x;
-  const int k = k0 + (t >> 4), c = col0 + ((t & 15) << 2);
-  if (k < K && vec && c + 3 < ncols)
-  {
-    float4 v = *reinterpret_cast<const float4*>(G + (size_t)k * ld + c);
-    reg[0] = v.x, reg[1] = v.y, reg[2] = v.z, reg[3] = v.w;
-  }
-  else
-  {
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      reg[j] = (k < K && c + j < ncols) ? G[(size_t)k * ld + c + j] : 0.0f;
-  }
-}
-
-template <int COLS>
-__device__ __forceinline__ void stash_mnmajor(float (*S)[COLS + PAD], const float (&reg)[4])
-{
-  const int t = threadIdx.x;
-  const int k = t >> 4, c = (t & 15) << 2;
-  *reinterpret_cast<float4*>(&S[k][c]) = make_float4(reg[0], reg[1], reg[2], reg[3]);
-}
 
 __device__ __forceinline__ bool aligned16(const void* p)
 {
@@ -366,9 +364,13 @@ __global__ void __launch_bounds__(NTHREADS)
 }
 
 // ---------------------------------------------------------------------------------------
-// The grouped GEMM kernel.  OP selects operand layouts and the fused epilogue.
+// The grouped GEMM kernel.  OP selects operand layouts and the fused epilogue; T x T output tiles
+// (64: 4 x 4 outputs per thread, 32: 2 x 2 where 64 x 64 tiles would leave SMs idle), the operands
+// STAGES - 1 K steps ahead through cp.async.  Every output is one ascending sum over K whatever the
+// tile.  With one register-prefetched step the kernel waited for L2 in each of them: 784 -> 256 at
+// batch 256 took 67 us and takes 23 us now.
 // ---------------------------------------------------------------------------------------
-template <int OP>
+template <int OP, int T>
 __global__ void __launch_bounds__(NTHREADS)
     pc_gemm_kernel(const dpc_layer* __restrict__ layers, int first, int n_layers, int batch,
                    int flags, int mode, double* energy, const float* __restrict__ epc_src = nullptr)
@@ -386,7 +388,7 @@ __global__ void __launch_bounds__(NTHREADS)
     M = batch, N = L.size, K = L.next_size;
   else
     M = L.next_size, N = L.size, K = batch;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  const int m0 = blockIdx.y * T, n0 = blockIdx.x * T;
   if (m0 >= M || n0 >= N)
     return;
   const bool wg_stage = OP == OP_WG && (mode & WG_GRAD_ONLY);
@@ -411,91 +413,119 @@ __global__ void __launch_bounds__(NTHREADS)
     A = (simple && mode == WG_LEARN) ? Lup->e : L.fe, lda = L.next_size,
     Bm = simple ? L.zF : L.z, ldb = L.size;
 
-  __shared__ Tile tile;
+  constexpr bool A_K = OP != OP_WG, B_K = OP == OP_FWD; // K-major operands
+  constexpr int J = T / 16, STAGES = T == 64 ? 4 : 8;
+  constexpr int CHUNKS = T * BK / 4, PER = CHUNKS / NTHREADS; // 16-byte chunks per operand, per thread
+  __shared__ __align__(16) float tile_a[STAGES][kTileFloats<T, A_K>];
+  __shared__ __align__(16) float tile_b[STAGES][kTileFloats<T, B_K>];
   const bool vecA = aligned16(A) && (lda % 4 == 0);
   const bool vecB = aligned16(Bm) && (ldb % 4 == 0);
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
+  // T = 64: a chunk of both operands per thread; T = 32: half of the threads load each operand
+  const bool loads_a = PER > 0 || t < CHUNKS, loads_b = PER > 0 || t >= NTHREADS - CHUNKS;
+  const TileChunk<T, A_K> chunk_a(t % CHUNKS);
+  const TileChunk<T, B_K> chunk_b(t % CHUNKS);
+  auto load = [&](int k0, int slot)
+  {
+    if (k0 < K)
+    {
+      if (loads_a)
+        chunk_a.load(tile_a[slot], A, lda, m0, k0, M, K, vecA);
+      if (loads_b)
+        chunk_b.load(tile_b[slot], Bm, ldb, n0, k0, N, K, vecB);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
 
-  float acc[4][4];
+  float acc[J][J];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < J; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < J; ++j)
       acc[i][j] = 0.0f;
 
-  float ra[4], rb[4];
-  auto fetch = [&](int k0)
-  {
-    if (OP == OP_FWD)
-    {
-      if (simple)
-        fetch_kmajor<true>(ra, A, lda, m0, k0, M, K, vecA, L.act);
-      else
-        fetch_kmajor<false>(ra, A, lda, m0, k0, M, K, vecA, 0);
-      fetch_kmajor<false>(rb, Bm, ldb, n0, k0, N, K, vecB, 0);
-    }
-    else if (OP == OP_FB)
-    {
-      fetch_kmajor<false>(ra, A, lda, m0, k0, M, K, vecA, 0);
-      fetch_mnmajor(rb, Bm, ldb, n0, k0, N, K, vecB);
-    }
-    else
-    {
-      fetch_mnmajor(ra, A, lda, m0, k0, M, K, vecA);
-      fetch_mnmajor(rb, Bm, ldb, n0, k0, N, K, vecB);
-    }
-  };
-  auto stash = [&](int k0)
-  {
-    if (OP == OP_WG)
-      stash_mnmajor<BM>(tile.a, ra);
-    else
-      stash_kmajor<BM>(tile.a, ra);
-    if (OP == OP_FWD)
-      stash_kmajor<BN>(tile.b, rb);
-    else
-      stash_mnmajor<BN>(tile.b, rb);
-    if (OP == OP_FWD && simple && blockIdx.x == 0 && L.zF != nullptr)
-    {
-      // SimplePC keeps f(z) as last fed to the GEMM for its weight update
-      // (src/layers/SimplePCLayer.cpp:146-150).
-      const int t = threadIdx.x;
-      const int r = m0 + (t >> 2), k = k0 + ((t & 3) << 2);
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (r < M && k + j < K)
-          L.zF[(size_t)r * L.size + k + j] = ra[j];
-    }
-  };
-
-  fetch(0);
-  stash(0);
-  __syncthreads();
+  for (int q = 0; q < STAGES - 1; ++q)
+    load(q * BK, q);
+  int slot = 0;
   for (int k0 = 0; k0 < K; k0 += BK)
   {
-    const bool more = k0 + BK < K;
-    if (more)
-      fetch(k0 + BK);
-#pragma unroll
-    for (int k = 0; k < BK; ++k)
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    if (OP == OP_FWD && simple && loads_a)
     {
-      const float4 av = *reinterpret_cast<const float4*>(&tile.a[k][ty * 4]);
-      const float4 bv = *reinterpret_cast<const float4*>(&tile.b[k][tx * 4]);
-      const float a4[4] = {av.x, av.y, av.z, av.w};
-      const float b4[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          acc[i][j] = fmaf(a4[i], b4[j], acc[i][j]);
+      // SimplePC: the operand is f(z), kept as last fed to the GEMM for the weight update
+      // (src/layers/SimplePCLayer.cpp:146-150); each thread transforms what it copied
+      float* a = chunk_a.at(tile_a[slot]);
+      const int r = m0 + chunk_a.row, k = k0 + chunk_a.k;
+      if (r < M && k < K)
+      {
+        float4 v = *reinterpret_cast<const float4*>(a);
+        v.x = act_fwd(L.act, v.x);
+        v.y = k + 1 < K ? act_fwd(L.act, v.y) : 0.0f;
+        v.z = k + 2 < K ? act_fwd(L.act, v.z) : 0.0f;
+        v.w = k + 3 < K ? act_fwd(L.act, v.w) : 0.0f;
+        *reinterpret_cast<float4*>(a) = v;
+        if (blockIdx.x == 0 && L.zF != nullptr)
+        {
+          float* zf = L.zF + (size_t)r * L.size + k;
+          if (vecA && aligned16(L.zF))
+            *reinterpret_cast<float4*>(zf) = v;
+          else
+          {
+            zf[0] = v.x;
+            if (k + 1 < K)
+              zf[1] = v.y;
+            if (k + 2 < K)
+              zf[2] = v.z;
+            if (k + 3 < K)
+              zf[3] = v.w;
+          }
+        }
+      }
     }
-    __syncthreads();
-    if (more)
+    __syncthreads(); // the step has landed, and everybody is done with the slot that is refilled now
+    load(k0 + (STAGES - 1) * BK, slot == 0 ? STAGES - 1 : slot - 1);
+    const float* ta = tile_a[slot];
+    const float* tb = tile_b[slot];
+#pragma unroll
+    for (int k = 0; k < BK; k += 4)
     {
-      stash(k0 + BK);
-      __syncthreads();
+      float a[J][4], b[4][J];
+#pragma unroll
+      for (int i = 0; i < J; ++i)
+        if (A_K)
+        {
+          const float4 v = *reinterpret_cast<const float4*>(ta + (ty + 16 * i) * (BK + 4) + k);
+          a[i][0] = v.x, a[i][1] = v.y, a[i][2] = v.z, a[i][3] = v.w;
+        }
+#pragma unroll
+      for (int j = 0; j < J; ++j)
+        if (B_K)
+        {
+          const float4 v = *reinterpret_cast<const float4*>(tb + (tx + 16 * j) * (BK + 4) + k);
+          b[0][j] = v.x, b[1][j] = v.y, b[2][j] = v.z, b[3][j] = v.w;
+        }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+      {
+        if (!A_K)
+          tile_row<J>(ta + (k + q) * T + ty * J, [&](int i, float v) { a[i][q] = v; });
+        if (!B_K)
+          tile_row<J>(tb + (k + q) * T + tx * J, [&](int j, float v) { b[q][j] = v; });
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int i = 0; i < J; ++i)
+#pragma unroll
+          for (int j = 0; j < J; ++j)
+            acc[i][j] = fmaf(a[i][q], b[q][j], acc[i][j]);
     }
+    slot = slot + 1 == STAGES ? 0 : slot + 1;
   }
+  // output (i, j) of this thread
+  auto out_m = [&](int i) { return m0 + (A_K ? ty + 16 * i : ty * J + i); };
+  auto out_n = [&](int j) { return n0 + (B_K ? tx + 16 * j : tx * J + j); };
 
   // ------------------------------------------------------------------ epilogues
   float esum = 0.0f;
@@ -506,15 +536,15 @@ __global__ void __launch_bounds__(NTHREADS)
     const bool do_fe = (flags & DPC_FWD_FE) && Lup && !simple && !(next_ce && (flags & DPC_FWD_ERR_NEXT));
     const bool do_copy = (flags & DPC_FWD_COPY_NEXT) && Lup;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < J; ++i)
     {
-      const int m = m0 + ty * 4 + i;
+      const int m = out_m(i);
       if (m >= M)
         continue;
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
+      for (int j = 0; j < J; ++j)
       {
-        const int n = n0 + tx * 4 + j;
+        const int n = out_n(j);
         if (n >= N)
           continue;
         const size_t o = (size_t)m * N + n;
@@ -560,15 +590,15 @@ __global__ void __launch_bounds__(NTHREADS)
   else if (OP == OP_FB)
   {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < J; ++i)
     {
-      const int m = m0 + ty * 4 + i;
+      const int m = out_m(i);
       if (m >= M)
         continue;
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
+      for (int j = 0; j < J; ++j)
       {
-        const int n = n0 + tx * 4 + j;
+        const int n = out_n(j);
         if (n >= N)
           continue;
         const size_t o = (size_t)m * N + n;
@@ -614,13 +644,13 @@ __global__ void __launch_bounds__(NTHREADS)
     if (wg_stage)
     {
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < J; ++i)
       {
-        const int m = m0 + ty * 4 + i;
+        const int m = out_m(i);
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < J; ++j)
         {
-          const int n = n0 + tx * 4 + j;
+          const int n = out_n(j);
           if (m < M && n < N)
             L.g_W[(size_t)m * N + n] = acc[i][j];
         }
@@ -650,15 +680,15 @@ __global__ void __launch_bounds__(NTHREADS)
         lr_wd = L.lr * L.lmbda;
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < J; ++i)
     {
-      const int m = m0 + ty * 4 + i;
+      const int m = out_m(i);
       if (m >= M)
         continue;
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
+      for (int j = 0; j < J; ++j)
       {
-        const int n = n0 + tx * 4 + j;
+        const int n = out_n(j);
         if (n >= N)
           continue;
         const size_t o = (size_t)m * N + n;
