@@ -254,12 +254,13 @@ __device__ __forceinline__ void dot_rows(const float* __restrict__ w, const floa
 }
 
 // One state task: sums over `len` rows of W for this lane's KW columns.
-template <int RT, int KW>
+template <int RT, int KW, int UNROLL>
 __device__ __forceinline__ void state_sum(float (&acc)[RT][KW], const float* w, int ldw, int len,
                                           const float* g, int S)
 {
   int n = 0;
-#pragma unroll 2
+  // (streamed rows: the loads of 4 UNROLL rows are in flight together)
+#pragma unroll UNROLL
   for (; n + 4 <= len; n += 4, w += 4 * (size_t)ldw)
   {
     float wv[4][KW];
@@ -459,7 +460,6 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
     bias[i] = (i & 3) < q.valid ? P.layers[q.layer - 1].b[q.col + (i & 3)] : 0.0f;
   }
 
-  const ResTask own_f = ftab[min(warp, max(P.nf - 1, 0))], own_b = btab[min(warp, max(P.nb - 1, 0))];
   const bool first = P.ops & DPC_ROWS_FIRST;
   double esum = 0.0;
 
@@ -621,9 +621,9 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
         constexpr int KW = decltype(kw)::value;
         float acc[RT][KW] = {};
         if (t.len > 0)
-          state_sum<RT, KW>(acc, Ws + t.w + k, t.ldw, t.len, g, S);
+          state_sum<RT, KW, 2>(acc, Ws + t.w + k, t.ldw, t.len, g, S);
         if (t.len2 > 0)
-          state_sum<RT, KW>(acc, sW[t.kind >> 4] + t.w2 + k, sl[t.kind >> 4].K, t.len2, g + t.len, S);
+          state_sum<RT, KW, RT == 1 ? 6 : RT == 2 ? 4 : 2>(acc, sW[t.kind >> 4] + t.w2 + k, sl[t.kind >> 4].K, t.len2, g + t.len, S);
 #pragma unroll
         for (int r = 0; r < RT; ++r)
 #pragma unroll
@@ -783,14 +783,26 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
       }
     }
 
-    // Forward pass of all layers.  err: errors (and gated errors) are recomputed; else the gated
-    // errors are refreshed from the errors that are there.
-    auto forward = [&](bool err, bool gate, bool energy, bool pred)
+    // Settling steps, then the closing passes.  One loop, so that the code of a pass -- activations of
+    // four values in every kind -- exists once: with a copy per use the passes waited for instructions.
+    // err: errors (and gated errors) are recomputed; else the gated errors are refreshed from the
+    // errors that are there.
+    const int refresh_at = (P.ops & DPC_ROWS_REFRESH) ? P.steps : -1;
+    const int preact_at = (P.ops & DPC_ROWS_PREACT) ? P.steps + (refresh_at >= 0) : -1;
+    const int energy_at =
+        (P.ops & DPC_ROWS_ENERGY_LAST) ? P.steps + (refresh_at >= 0) + (preact_at >= 0) : -1;
+    const int passes = P.steps + (refresh_at >= 0) + (preact_at >= 0) + (energy_at >= 0);
+#pragma unroll 1
+    for (int t = 0; t < passes; ++t)
     {
-      if (warp < P.nf)
-        forward_task(own_f);
-      for (int t = warp + kWarps; t < P.nf; t += kWarps)
-        forward_task(ftab[t]);
+      const bool settles = t < P.steps, last = t + 1 == P.steps;
+      const bool err = settles || t == energy_at;
+      const bool gate = settles || t == refresh_at || (t == energy_at && (P.ops & DPC_ROWS_GATE_LAST));
+      const bool energy = settles ? (P.ops & DPC_ROWS_ENERGY_EACH) != 0 : t == energy_at;
+      const bool pred = settles ? last && (P.ops & DPC_ROWS_PRED_LAST)
+                                : t == preact_at || (P.ops & DPC_ROWS_PRED_CLOSE) != 0;
+      for (int q = warp; q < P.nf; q += kWarps)
+        forward_task(ftab[q]);
       __syncthreads();
       float local = 0.0f;
       for_quads([&](const ResQuad& q, int i, int r)
@@ -832,18 +844,10 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
       __syncthreads();
       if (err && P.ce)
         ce_error(energy);
-    };
-
-    // ---------------------------------------------------------------- settling
-    for (int t = 0; t < P.steps; ++t)
-    {
-      const bool last = t + 1 == P.steps;
-      forward(true, true, (P.ops & DPC_ROWS_ENERGY_EACH) != 0,
-              last && (P.ops & DPC_ROWS_PRED_LAST) != 0);
-      if (warp < P.nb)
-        state_of(own_b);
-      for (int t = warp + kWarps; t < P.nb; t += kWarps)
-        state_of(btab[t]);
+      if (!settles)
+        continue;
+      for (int q = warp; q < P.nb; q += kWarps)
+        state_of(btab[q]);
       __syncthreads();
       const bool refresh_f = simple && !(last && !(P.ops & DPC_ROWS_ENERGY_LAST));
       for_quads([&](const ResQuad& q, int i, int r)
@@ -914,13 +918,6 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
                 });
       __syncthreads();
     }
-    // ---------------------------------------------------------------- closing pass
-    if (P.ops & DPC_ROWS_REFRESH)
-      forward(false, true, false, (P.ops & DPC_ROWS_PRED_CLOSE) != 0);
-    if (P.ops & DPC_ROWS_PREACT)
-      forward(false, false, false, true);
-    if (P.ops & DPC_ROWS_ENERGY_LAST)
-      forward(true, (P.ops & DPC_ROWS_GATE_LAST) != 0, true, (P.ops & DPC_ROWS_PRED_CLOSE) != 0);
     if (P.ops & DPC_ROWS_LOGITS)
     {
       // the top belief becomes the prediction below it
