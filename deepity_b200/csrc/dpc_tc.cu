@@ -90,7 +90,7 @@ struct TcState
   // errors and weights, their tensor maps (layer coordinate 2l + plane) and, per layer, whether
   // the planes lag behind the fp32 tensor (1 = must be re-split before a kernel reads them).
   __nv_bfloat16 *zp = nullptr, *fep = nullptr, *wp = nullptr;
-  CUtensorMap zp_km, zp_km64, zp_mn, fep_km, fep_mn, wp_km128, wp_km64, wp_mn;
+  CUtensorMap zp_km, zp_km64, zp_mn, fep_km, fep_mn, wp_km128, wp_km64, wp_km32, wp_mn;
   CUtensorMap e_st, fep_st; // bulk-store maps: errors (fp32) and feedback-error planes (bf16)
   CUtensorMap z_st, zp_st;  // beliefs (fp32) and their planes, for the feedback kernel
   CUtensorMap w_st, wp_st;  // weights (fp32) and their planes, for the weight kernel
@@ -644,7 +644,10 @@ struct Cfg
   // updated in place and leaves with its planes through bulk tensor stores.
   static constexpr bool WGIO = PRE && PAIR && OP == TC_WG;
   static constexpr int STAGES = B16 ? NR
-                                : (TSTORE || FBIO || WGIO) ? 2
+                                // (three where a narrower tile leaves room: its few k-blocks are
+                                // mostly latency)
+                                : TSTORE ? (BN == 64 ? 3 : 2)
+                                : (FBIO || WGIO) ? (BN == 128 ? 3 : 2)
                                 : (PRE && KS == 2) ? 4
                                 : (STAGES_RAW < 2 ? 2 : (STAGES_RAW > 8 ? 8 : STAGES_RAW));
   static constexpr int RING_BYTES = B16 ? (NR + NB) * RAWB : STAGES * STAGE_BYTES;
@@ -1893,6 +1896,7 @@ static bool planes_init(dpc_plan* plan, TcState* st, int first, int count, int H
   ok &= make_map_bf16(&st->fep_mn, st->fep, H, B, 2 * count, (int64_t)act, 64);
   ok &= make_map_bf16(&st->wp_km128, st->wp, H, H, 2 * count, (int64_t)w, 128);
   ok &= make_map_bf16(&st->wp_km64, st->wp, H, H, 2 * count, (int64_t)w, 64);
+  ok &= make_map_bf16(&st->wp_km32, st->wp, H, H, 2 * count, (int64_t)w, 32);
   ok &= make_map_bf16(&st->wp_mn, st->wp, H, H, 2 * count, (int64_t)w, 64);
   if (!ok)
     return false;
@@ -2272,6 +2276,29 @@ static bool fe_only_now(const dpc_plan* p, const TcState* st)
   return planes_kept(p, st) && st->fe_only && p->ctx->precision != DPC_PRECISION_TF32;
 }
 
+// Width of the pair tiles (256 x BN) of a launch over `tiles256` tiles of 256 columns.  A launch takes
+// whole waves of one tile per SM pair, and a tile costs its width plus a fixed part (launch, pipeline
+// fill, last stores: about an eighth of a 256-wide tile): 7 tiles of a 256-wide stack at batch 256 are
+// one wave whatever their width, 88 tiles of a 512-wide one two waves or, halved, three half ones.  Wide
+// tiles re-read less of A and win where there are many waves.
+static int pair_tile_width(const dpc_plan* p, int tiles256, int narrowest)
+{
+  static const char* env = getenv("DPC_PAIR_TILE_WIDTH"); // (for comparing the variants)
+  if (env)
+    return std::max(atoi(env), narrowest);
+  const int pairs = p->ctx->sm_count / 2;
+  int best = 256;
+  double best_cost = 1e30;
+  for (int bn = 256; bn >= narrowest; bn /= 2)
+  {
+    const int tiles = tiles256 * (256 / bn);
+    const double cost = (double)((tiles + pairs - 1) / pairs) * (bn / 256.0 + 0.125);
+    if (cost < 0.97 * best_cost)
+      best = bn, best_cost = cost;
+  }
+  return best;
+}
+
 static TcParams base_params(dpc_plan* p, TcState* st, int first, int count, int M, int N, int K,
                             int BN, int flags, int mode, int BM = TBM)
 {
@@ -2325,7 +2352,9 @@ int tc_forward(dpc_plan* p, int first, int count, int flags)
   int rc;
   if (pair_ok(B, H))
   {
-    TcParams P = base_params(p, st, first, count, B, H, H, 256, flags, 0, 256);
+    const bool planes = !tf32 && planes_on(p, st);
+    const int bn = planes || tf32 ? pair_tile_width(p, count * (B / 256) * (H / 256), 64) : 256;
+    TcParams P = base_params(p, st, first, count, B, H, H, bn, flags, 0, 256);
     // What the epilogue reads from the layer above is the same for every layer of the launch
     // unless a softmax head sits right above the range: stage it through shared memory.
     const CUtensorMap* up = nullptr;
@@ -2339,17 +2368,22 @@ int tc_forward(dpc_plan* p, int first, int count, int flags)
       else if ((flags & DPC_FWD_FE) && !(flags & DPC_FWD_ERR_NEXT))
         P.stage_in = 2, up = &st->eup_km;
     }
-    if (!tf32 && planes_on(p, st))
+    if (planes)
     {
       if ((rc = planes_need(p, st, PL_Z, r0, r0 + count)) != DPC_OK ||
           (rc = planes_need(p, st, PL_W, r0, r0 + count)) != DPC_OK)
         return rc;
       P.tstore = (st->store_maps && P.stage_in != 0) ? 1 : 0;
-      rc = launch<TC_FWD, 256, 3, 128, true>(p, st, st->zp_km, st->wp_km128, P, up);
+      rc = bn == 64    ? launch<TC_FWD, 64, 3, 128, true>(p, st, st->zp_km, st->wp_km32, P, up)
+           : bn == 128 ? launch<TC_FWD, 128, 3, 128, true>(p, st, st->zp_km, st->wp_km64, P, up)
+                       : launch<TC_FWD, 256, 3, 128, true>(p, st, st->zp_km, st->wp_km128, P, up);
     }
+    else if (tf32)
+      rc = bn == 64    ? launch<TC_FWD, 64, 0, 128, true>(p, st, st->z_km, st->w_km32, P, up)
+           : bn == 128 ? launch<TC_FWD, 128, 0, 128, true>(p, st, st->z_km, st->w_km64, P, up)
+                       : launch<TC_FWD, 256, 0, 128, true>(p, st, st->z_km, st->w_km128, P, up);
     else
-      rc = tf32 ? launch<TC_FWD, 256, 0, 128, true>(p, st, st->z_km, st->w_km128, P, up)
-         : scheme == 2 ? launch<TC_FWD, 256, 2, 128, true>(p, st, st->z_km, st->w_km128, P, up)
+      rc = scheme == 2 ? launch<TC_FWD, 256, 2, 128, true>(p, st, st->z_km, st->w_km128, P, up)
                        : launch<TC_FWD, 256, 1, 128, true>(p, st, st->z_km, st->w_km128, P, up);
   }
   else if (tf32)
@@ -2465,8 +2499,10 @@ int tc_update_state(dpc_plan* p, int first, int count, bool feed)
   int rc;
   if (pair_ok(B, H))
   {
-    TcParams P = base_params(p, st, first, count, B, H, H, 256, 0, 0, 256);
-    if (!tf32 && planes_on(p, st))
+    const bool planes = !tf32 && planes_on(p, st);
+    const int bn = planes || tf32 ? pair_tile_width(p, count * (B / 256) * (H / 256), 128) : 256;
+    TcParams P = base_params(p, st, first, count, B, H, H, bn, 0, 0, 256);
+    if (planes)
     {
       if ((rc = planes_need(p, st, PL_FE, r0, r0 + count)) != DPC_OK ||
           (rc = planes_need(p, st, PL_W, r0, r0 + count)) != DPC_OK)
@@ -2479,11 +2515,14 @@ int tc_update_state(dpc_plan* p, int first, int count, bool feed)
         plain = !p->h[i].v && !(p->h[i].flags & DPC_LAYER_RESIDUAL);
       P.tstore = plain ? 1 : 0;
       P.mode = !st->simple ? FBP_BELIEF : feed ? FBP_FEED : FBP_NONE;
-      rc = launch<TC_FB, 256, 3, 128, true>(p, st, st->fep_km, st->wp_mn, P);
+      rc = bn == 128 ? launch<TC_FB, 128, 3, 128, true>(p, st, st->fep_km, st->wp_mn, P)
+                     : launch<TC_FB, 256, 3, 128, true>(p, st, st->fep_km, st->wp_mn, P);
     }
+    else if (tf32)
+      rc = bn == 128 ? launch<TC_FB, 128, 0, 128, true>(p, st, st->fe_km, st->w_mn, P)
+                     : launch<TC_FB, 256, 0, 128, true>(p, st, st->fe_km, st->w_mn, P);
     else
-      rc = tf32 ? launch<TC_FB, 256, 0, 128, true>(p, st, st->fe_km, st->w_mn, P)
-         : scheme == 2 ? launch<TC_FB, 256, 2, 128, true>(p, st, st->fe_km, st->w_mn, P)
+      rc = scheme == 2 ? launch<TC_FB, 256, 2, 128, true>(p, st, st->fe_km, st->w_mn, P)
                        : launch<TC_FB, 256, 1, 128, true>(p, st, st->fe_km, st->w_mn, P);
   }
   else if (tf32)
@@ -2534,8 +2573,10 @@ int tc_weight_gemm(dpc_plan* p, int first, int count, int mode, int decay_w)
   int rc;
   if (pair_ok(H, H))
   {
-    TcParams P = base_params(p, st, first, count, H, H, B, 256, decay_w ? 1 : 0, mode, 256);
-    if (!tf32 && planes_on(p, st))
+    const bool planes = !tf32 && planes_on(p, st);
+    const int bn = planes || tf32 ? pair_tile_width(p, count * (H / 256) * (H / 256), 128) : 256;
+    TcParams P = base_params(p, st, first, count, H, H, B, bn, decay_w ? 1 : 0, mode, 256);
+    if (planes)
     {
       // (SimplePC: f(z) as last fed to the forward product, not of the beliefs as they are now)
       if ((rc = planes_need(p, st, PL_FE, r0, r0 + count)) != DPC_OK ||
@@ -2547,11 +2588,14 @@ int tc_weight_gemm(dpc_plan* p, int first, int count, int mode, int decay_w)
                   !getenv("DPC_DISABLE_STAGED_INPUT"))
                      ? 1
                      : 0;
-      rc = launch<TC_WG, 256, 3, 128, true>(p, st, st->fep_mn, st->zp_mn, P);
+      rc = bn == 128 ? launch<TC_WG, 128, 3, 128, true>(p, st, st->fep_mn, st->zp_mn, P)
+                     : launch<TC_WG, 256, 3, 128, true>(p, st, st->fep_mn, st->zp_mn, P);
     }
+    else if (tf32)
+      rc = bn == 128 ? launch<TC_WG, 128, 0, 128, true>(p, st, st->fe_mn, st->z_mn, P)
+                     : launch<TC_WG, 256, 0, 128, true>(p, st, st->fe_mn, st->z_mn, P);
     else
-      rc = tf32 ? launch<TC_WG, 256, 0, 128, true>(p, st, st->fe_mn, st->z_mn, P)
-         : scheme == 2 ? launch<TC_WG, 256, 2, 128, true>(p, st, st->fe_mn, st->z_mn, P)
+      rc = scheme == 2 ? launch<TC_WG, 256, 2, 128, true>(p, st, st->fe_mn, st->z_mn, P)
                        : launch<TC_WG, 256, 1, 128, true>(p, st, st->fe_mn, st->z_mn, P);
   }
   else if (tf32)
