@@ -820,7 +820,10 @@ int dpc_forward(dpc_plan* p, int first, int count, int flags)
       [=](int f, int c) { return forward_simt(p, f, c, flags); }, independent);
   if (cached_first)
   {
-    const Job cached = [=] { return forward_simt(p, first, 1, flags | DPC_FWD_CACHED); };
+    // (transient passes: a refresh recomputes the feedback error of this clamped layer before anyone
+    // reads it, so a settling step computes the error alone)
+    const int keep = (flags & DPC_FWD_TRANSIENT) && (flags & DPC_FWD_ERR_NEXT) ? ~DPC_FWD_FE : ~0;
+    const Job cached = [=] { return forward_simt(p, first, 1, (flags & keep) | DPC_FWD_CACHED); };
     // beside the others; in a sweep before them
     jobs.insert(independent ? jobs.end() : jobs.begin(), cached);
   }
@@ -969,9 +972,9 @@ static int update_state_simt(dpc_plan* p, int first, int count)
       for (int i = f; i < f + cg; ++i)
         mxs = std::max(mxs, p->h[i].size);
       const int gx = cdiv(mxs, 128);
-      int rpb = p->batch;
-      while (rpb > 128 && (long long)gx * cg * cdiv(p->batch, rpb) < 2 * p->ctx->sm_count)
-        rpb = cdiv(rpb / 2, 128) * 128;
+      int rpb = cdiv(p->batch, 32) * 32;
+      while (rpb > 32 && (long long)gx * cg * cdiv(p->batch, rpb) < 4 * p->ctx->sm_count)
+        rpb = cdiv(rpb / 2, 32) * 32;
       dim3 grid(gx, cdiv(p->batch, rpb), cg);
       if (narrow_kc <= 12)
         narrow_state_kernel<12><<<grid, 256, 0, st>>>(p->d, f, p->n, p->batch, rpb);
@@ -1231,20 +1234,13 @@ int dpc_direct_feedback(dpc_plan* p, int first, int count, int decay_w)
 // Psi update (or its raw sums) of layers [f, f+c): the 128-columns-per-block kernel when every
 // layer of the launch that has feedback weights is a multiple of 128 wide with at most 16
 // terminal units, the general kernel otherwise.
-static int launch_psi_update(dpc_plan* p, int f, int c, int max_size, int grad_only)
+static int launch_psi_range(dpc_plan* p, int f, int c, int max_size, int grad_only, bool fast)
 {
   cudaStream_t st = p->ctx->stream;
-  bool fast = true;
   int ts = 0;
   for (int i = f; i < f + c && i < p->n; ++i)
-  {
-    const dpc_layer& L = p->h[i];
-    if (L.next_size <= 0 || L.Psi == nullptr || (L.flags & DPC_LAYER_INPUT_ACT))
-      continue;
-    if (L.size % 128 != 0 || L.terminal_size > 16)
-      fast = false;
-    ts = std::max(ts, L.terminal_size);
-  }
+    if (p->h[i].next_size > 0 && p->h[i].Psi != nullptr)
+      ts = std::max(ts, p->h[i].terminal_size);
   if (fast && ts > 0)
   {
     dim3 g(std::max(1, cdiv(max_size, 128)), c);
@@ -1262,6 +1258,28 @@ static int launch_psi_update(dpc_plan* p, int f, int c, int max_size, int grad_o
     psi_update_kernel<<<g, 256, 0, st>>>(p->d, f, p->n, p->batch, p->e_terminal, grad_only);
   }
   return check_launch(p->ctx, grad_only ? "psi gradient kernel" : "psi_update kernel");
+}
+
+static void psi_jobs(dpc_plan* p, int f, int c, int grad_only, std::vector<Job>& jobs)
+{
+  auto has_psi = [&](int i)
+  { return p->h[i].next_size > 0 && p->h[i].Psi != nullptr && !(p->h[i].flags & DPC_LAYER_INPUT_ACT); };
+  auto fits = [&](int i) { return !has_psi(i) || (p->h[i].size % 128 == 0 && p->h[i].terminal_size <= 16); };
+  bool all = true, adam = false;
+  for (int i = f; i < f + c && i < p->n; ++i)
+    all &= fits(i), adam |= has_psi(i) && p->h[i].opt_psi != DPC_OPT_SGD;
+  // Layers of both kinds: each run with its kernel (Adam-type updates keep one order of additions for
+  // all, that of the general kernel).
+  int i = f;
+  while (i < f + c)
+  {
+    const bool fast = all || (!adam && fits(i));
+    int j = i, mx = 0;
+    while (j < f + c && (all || adam || fits(j) == fits(i)))
+      mx = std::max(mx, p->h[j].size), ++j;
+    jobs.push_back([=] { return launch_psi_range(p, i, j - i, mx, grad_only, fast); });
+    i = j;
+  }
 }
 
 // Bias update (or its raw sums) of layers [f, f+c).
@@ -1291,14 +1309,13 @@ int dpc_update_weights(dpc_plan* p, int first, int count, int center_rows)
   if (count <= 0)
     return DPC_OK;
   bool any_adam = false, any_psi = false;
-  int max_next = 0, max_size = 0;
+  int max_next = 0;
   for (int i = first; i < first + count; ++i)
   {
     const dpc_layer& L = p->h[i];
     any_adam |= L.opt != DPC_OPT_SGD || (L.Psi && L.opt_psi != DPC_OPT_SGD);
     any_psi |= L.Psi != nullptr && !(L.flags & DPC_LAYER_INPUT_ACT);
     max_next = std::max(max_next, L.next_size);
-    max_size = std::max(max_size, L.size);
   }
   if (any_adam)
   {
@@ -1348,7 +1365,7 @@ int dpc_update_weights(dpc_plan* p, int first, int count, int center_rows)
     const int c = std::min(kMaxZ, first + count - f);
     jobs.push_back([=] { return launch_bias_update(p, f, c, max_next, 0); });
     if (any_psi)
-      jobs.push_back([=] { return launch_psi_update(p, f, c, max_size, 0); });
+      psi_jobs(p, f, c, 0, jobs);
   }
   if ((rc = run_side_by_side(p->ctx, jobs)) != DPC_OK)
     return rc;
@@ -1409,13 +1426,12 @@ int dpc_weight_gradients(dpc_plan* p, int first, int count, int which)
   if (rc != DPC_OK)
     return rc;
   bool any_psi = false;
-  int max_next = 0, max_size = 0;
+  int max_next = 0;
   for (int i = first; i < first + count; ++i)
   {
     const dpc_layer& L = p->h[i];
     any_psi |= L.Psi != nullptr && !(L.flags & DPC_LAYER_INPUT_ACT);
     max_next = std::max(max_next, L.next_size);
-    max_size = std::max(max_size, L.size);
   }
   for (int f = first; f < first + count; f += kMaxZ)
   {
@@ -1424,7 +1440,9 @@ int dpc_weight_gradients(dpc_plan* p, int first, int count, int which)
       return rc;
     if (any_psi)
     {
-      if ((rc = launch_psi_update(p, f, c, max_size, 1)) != DPC_OK)
+      std::vector<Job> jobs;
+      psi_jobs(p, f, c, 1, jobs);
+      if ((rc = run_side_by_side(p->ctx, jobs)) != DPC_OK)
         return rc;
     }
   }

@@ -733,6 +733,29 @@ __global__ void cached_forward_kernel(const dpc_layer* __restrict__ layers, int 
     const bool do_fe = (flags & DPC_FWD_FE) && !simple && !(next_ce && (flags & DPC_FWD_ERR_NEXT));
     const bool do_copy = (flags & DPC_FWD_COPY_NEXT) != 0;
     const size_t total = (size_t)batch * L.next_size;
+    // the pass of a settling step: errors (and feedback errors), 16 bytes at a time
+    if (do_err && !do_copy && total % 4 == 0 && aligned16(L.mu) && aligned16(Lup->z) && aligned16(Lup->e) &&
+        (!do_fe || (aligned16(L.fe) && aligned16(L.preact))))
+    {
+      const size_t n4 = total / 4;
+      for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4;
+           i += (size_t)gridDim.x * blockDim.x)
+      {
+        const float4 mu = reinterpret_cast<const float4*>(L.mu)[i];
+        const float4 z = reinterpret_cast<const float4*>(Lup->z)[i];
+        const float4 e = make_float4(z.x - mu.x, z.y - mu.y, z.z - mu.z, z.w - mu.w);
+        reinterpret_cast<float4*>(Lup->e)[i] = e;
+        esum += e.x * e.x, esum += e.y * e.y, esum += e.z * e.z, esum += e.w * e.w;
+        if (do_fe)
+        {
+          const float4 p = reinterpret_cast<const float4*>(L.preact)[i];
+          reinterpret_cast<float4*>(L.fe)[i] =
+              make_float4(e.x * act_deriv(L.act, p.x), e.y * act_deriv(L.act, p.y), e.z * act_deriv(L.act, p.z),
+                          e.w * act_deriv(L.act, p.w));
+        }
+      }
+    }
+    else
     for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < total;
          o += (size_t)gridDim.x * blockDim.x)
     {
@@ -1529,7 +1552,7 @@ __global__ void __launch_bounds__(256)
     }
     __syncthreads();
     const int rows = min(ROWS, b_end - b0);
-#pragma unroll 2
+#pragma unroll 4
     for (int r = warp; r < rows; r += 8)
     {
       const size_t o = (size_t)(b0 + r) * s + col;

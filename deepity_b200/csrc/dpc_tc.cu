@@ -111,7 +111,7 @@ struct TcState
   {
     int layer;
     bool simple;
-    CUtensorMap z_km, w_km128, fe_km, w_mn, fe_mn, z_mn;
+    CUtensorMap z_km, w_km128, w_km64, fe_km, w_mn, fe_mn, z_mn;
   };
   std::vector<Extra> extras;
 };
@@ -2042,6 +2042,7 @@ int tc_plan_init(dpc_plan* plan)
       ok &= make_map(&x.fe_km, a_out, s_out, B, 1, (int64_t)B * s_out, TBM, false);
       ok &= make_map(&x.fe_mn, a_out, s_out, B, 1, (int64_t)B * s_out, 32, true);
       ok &= make_map(&x.w_km128, L.W, s_in, s_out, 1, (int64_t)s_in * s_out, 128, false);
+      ok &= make_map(&x.w_km64, L.W, s_in, s_out, 1, (int64_t)s_in * s_out, 64, false);
       ok &= make_map(&x.w_mn, L.W, s_in, s_out, 1, (int64_t)s_in * s_out, 32, true);
       if (ok)
         st->extras.push_back(x);
@@ -2683,10 +2684,17 @@ bool tc_extra_layer(dpc_plan* p, int layer)
   return st && st->ok && find_extra(st, layer) != nullptr;
 }
 
-static TcParams extra_params(dpc_plan* p, TcState* st, int layer, int M, int N, int K, int flags,
-                             int mode)
+// A product of few 256 x 256 tiles on single-CTA tiles instead (forward 128 x 64, weights 128 x 128):
+// 3072 -> 1024 at batch 1024 is 16 tiles, 32 of 148 SMs for 150 us.
+static bool extra_narrow(const dpc_plan* p, int M, int N)
 {
-  TcParams P = base_params(p, st, layer, 1, M, N, K, 256, flags, mode, 256);
+  return (M / 256) * ((N + 255) / 256) * 4 <= p->ctx->sm_count;
+}
+
+static TcParams extra_params(dpc_plan* p, TcState* st, int layer, int M, int N, int K, int flags,
+                             int mode, int BN = 256, int BM = 256)
+{
+  TcParams P = base_params(p, st, layer, 1, M, N, K, BN, flags, mode, BM);
   P.run_first = layer; // the maps hold this layer only
   P.zp = P.fep = P.wp = nullptr;
   P.fe_only = 0;
@@ -2729,9 +2737,12 @@ int tc_extra_forward(dpc_plan* p, int layer, int flags)
     if (cudaPeekAtLastError() != cudaSuccess)
       return cuda_fail(cudaGetLastError(), "input_activation kernel launch");
   }
-  TcParams P = extra_params(p, st, layer, p->batch, L.next_size, L.size, flags, 0);
+  const bool narrow = !tf32 && scheme == 2 && extra_narrow(p, p->batch, L.next_size);
+  TcParams P = narrow ? extra_params(p, st, layer, p->batch, L.next_size, L.size, flags, 0, 64, TBM)
+                      : extra_params(p, st, layer, p->batch, L.next_size, L.size, flags, 0);
   const int rc =
-      tf32 ? launch<TC_FWD, 256, 0, 128, true>(p, st, x->z_km, x->w_km128, P)
+      narrow ? launch<TC_FWD, 64, 2>(p, st, x->z_km, x->w_km64, P)
+      : tf32 ? launch<TC_FWD, 256, 0, 128, true>(p, st, x->z_km, x->w_km128, P)
       : scheme == 2 ? launch<TC_FWD, 256, 2, 128, true>(p, st, x->z_km, x->w_km128, P)
                     : launch<TC_FWD, 256, 1, 128, true>(p, st, x->z_km, x->w_km128, P);
   // the belief it may have written can be the first layer of the run: its planes are stale
@@ -2770,8 +2781,11 @@ int tc_extra_weight_gemm(dpc_plan* p, int layer, int mode, int decay_w)
     return 1;
   const bool tf32 = p->ctx->precision == DPC_PRECISION_TF32 || fast_grad(p);
   const int scheme = split_scheme(p);
-  TcParams P = extra_params(p, st, layer, L.next_size, L.size, p->batch, decay_w ? 1 : 0, mode);
-  return tf32 ? launch<TC_WG, 256, 0, 128, true>(p, st, x->fe_mn, x->z_mn, P)
+  const bool narrow = !tf32 && scheme == 2 && extra_narrow(p, L.next_size, L.size);
+  TcParams P = narrow ? extra_params(p, st, layer, L.next_size, L.size, p->batch, decay_w ? 1 : 0, mode, 128, TBM)
+                      : extra_params(p, st, layer, L.next_size, L.size, p->batch, decay_w ? 1 : 0, mode);
+  return narrow ? launch<TC_WG, 128, 2>(p, st, x->fe_mn, x->z_mn, P)
+       : tf32 ? launch<TC_WG, 256, 0, 128, true>(p, st, x->fe_mn, x->z_mn, P)
        : scheme == 2 ? launch<TC_WG, 256, 2, 128, true>(p, st, x->fe_mn, x->z_mn, P)
                      : launch<TC_WG, 256, 1, 128, true>(p, st, x->fe_mn, x->z_mn, P);
 }
