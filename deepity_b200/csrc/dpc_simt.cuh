@@ -1283,29 +1283,31 @@ __global__ void bias_update_kernel(const dpc_layer* __restrict__ layers, int fir
   }
   if (rank != 0)
     return; // (a row-split launch over a layer that takes the column sums: one CTA does them)
-  // Column sums in row order (the reference's): 32 columns at a time, the block copies groups of rows
-  // into shared memory, one buffer ahead, and one warp adds them up, a chain of dependent additions
-  // and nothing else.  (A thread that loads what it adds pays a memory latency every few rows: 145 us
-  // for a ten-column head at batch 4096.)
-  constexpr int CR = 64;
-  __shared__ float stage[2][CR][33];
-  const int cols = n < 32 ? n : 32, per = 256 / cols; // threads that copy one row, rows per round
-  const int cj = threadIdx.x % cols, cr = threadIdx.x / cols;
+  // Column sums in row order (the reference's): up to 32 columns at a time, the block copies groups of
+  // rows into shared memory, one buffer ahead, and one warp adds them up, a chain of dependent
+  // additions and nothing else.  (A thread that loads what it adds pays a memory latency every few
+  // rows: five 2048-wide layers and a ten-column head at batch 4096 took 145 us so, 113 with sixteen
+  // loads in flight and a barrier per group, 71 this way.)
+  constexpr int STAGE = 4096; // floats per buffer
+  __shared__ float stage[2][STAGE];
+  const int cols = n < 32 ? n : 32;
+  const int CR = STAGE / cols; // rows per buffer
   for (int j0 = blockIdx.x * 32; j0 < n; j0 += gridDim.x * 32)
   {
-    const int width = min(32, n - j0);
-    auto value = [&](int b)
-    {
-      const size_t o = (size_t)b * n + j0 + cj;
-      return hi ? __bfloat162float(hi[o]) + __bfloat162float(hi[planes.elems + o]) : g[o];
-    };
+    const int width = min(cols, n - j0);
     auto copy = [&](int b0, int buf)
     {
-      if (cr < per && cj < width)
-#pragma unroll 8
-        for (int r = cr; r < CR; r += per)
-          if (b0 + r < batch)
-            stage[buf][r][cj] = value(b0 + r);
+      const int total = max(0, min(CR, batch - b0)) * cols;
+#pragma unroll
+      for (int q = 0; q < STAGE / 256; ++q)
+      {
+        const int i = q * 256 + threadIdx.x, r = i / cols, c = i - r * cols;
+        if (i < total && c < width)
+        {
+          const size_t o = (size_t)(b0 + r) * n + j0 + c;
+          stage[buf][i] = hi ? __bfloat162float(hi[o]) + __bfloat162float(hi[planes.elems + o]) : g[o];
+        }
+      }
     };
     float s = 0.0f;
     copy(0, 0);
@@ -1316,19 +1318,20 @@ __global__ void bias_update_kernel(const dpc_layer* __restrict__ layers, int fir
       if (threadIdx.x < (unsigned)width)
       {
         const int rows = min(CR, batch - b0);
+        const float* p = stage[buf] + threadIdx.x;
         int r = 0;
         for (; r + 16 <= rows; r += 16)
         {
           float v[16];
 #pragma unroll
           for (int q = 0; q < 16; ++q)
-            v[q] = stage[buf][r + q][threadIdx.x];
+            v[q] = p[(r + q) * cols];
 #pragma unroll
           for (int q = 0; q < 16; ++q)
             s += v[q];
         }
         for (; r < rows; ++r)
-          s += stage[buf][r][threadIdx.x];
+          s += p[r * cols];
       }
     }
     if (threadIdx.x < (unsigned)width)
@@ -1581,11 +1584,14 @@ __global__ void __launch_bounds__(256)
       const float ee[4] = {e4.x, e4.y, e4.z, e4.w};
       float vv[4] = {v4.x, v4.y, v4.z, v4.w};
       const float uu[4] = {u4.x, u4.y, u4.z, u4.w};
+      float dd[4];
+      if (simple)
+        act_deriv4(L.act, zz, dd);
 #pragma unroll
       for (int c = 0; c < 4; ++c)
       {
         if (simple)
-          zz[c] += L.ir * (acc[c] * act_deriv(L.act, zz[c]) - ee[c]);
+          zz[c] += L.ir * (acc[c] * dd[c] - ee[c]);
         else
         {
           const float fb = L.a * acc[c] - ee[c];
