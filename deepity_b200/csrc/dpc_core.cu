@@ -846,6 +846,14 @@ int dpc_plan_fused_cross_entropy(dpc_plan* p)
   return head >= 1 && narrow_forward(p, head) && !tensor(head) && (head == 1 || tensor(head - 1)) ? 1 : 0;
 }
 
+int dpc_plan_state_from_prediction(dpc_plan* p)
+{
+  return p && p->run.count > 0 && p->run.first <= 1 && p->run.first + p->run.count > 1 && p->h[0].mu &&
+                 (uintptr_t)p->h[0].mu % 32 == 0 && !(p->h[1].flags & DPC_LAYER_SOFTMAX_CE)
+             ? 1
+             : 0;
+}
+
 int dpc_project_forward(dpc_plan* p, int first, int count, int skip_last_copy)
 {
   return dpc_project_forward_ex(p, first, count, skip_last_copy, 0);
@@ -1022,8 +1030,12 @@ int dpc_update_state_ex(dpc_plan* p, int first, int count, int relax_from, int f
     return rc;
   const int end = first + count;
   relax_from = std::min(std::max(relax_from, first), end);
+  const bool from_mu = (flags & DPC_STATE_FIRST_MU) != 0;
+  if (from_mu && (first != 1 || relax_from == first || !dpc_plan_state_from_prediction(p)))
+    return fail(DPC_ERR_INVALID, "DPC_STATE_FIRST_MU: the range does not start at a tensor-core layer 1");
   std::vector<Job> jobs = pieces_of(
-      p, first, relax_from - first, [=](int f, int c) { return tc_update_state(p, f, c, (flags & DPC_STATE_FEED) != 0); },
+      p, first, relax_from - first,
+      [=](int f, int c) { return tc_update_state(p, f, c, (flags & DPC_STATE_FEED) != 0, from_mu && f == first); },
       [=](int f, int c) { return update_state_simt(p, f, c); }, true);
   for (int i = relax_from; i < end; ++i)
     jobs.push_back([=] { return dpc_relax(p, i); });

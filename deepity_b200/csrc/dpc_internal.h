@@ -83,7 +83,7 @@ int tc_plan_init(dpc_plan* plan);
 void tc_plan_free(dpc_plan* plan);
 int tc_forward(dpc_plan* plan, int first, int count, int flags);
 // feed (SimplePC run): a forward pass follows before the next weight update
-int tc_update_state(dpc_plan* plan, int first, int count, bool feed);
+int tc_update_state(dpc_plan* plan, int first, int count, bool feed, bool first_from_mu);
 int tc_project_forward(dpc_plan* plan, int first, int count, int flags);
 // mode: 0 learn, 1 direct feedback, +2: only store the raw sums in the layers' g_W.
 int tc_weight_gemm(dpc_plan* plan, int first, int count, int mode, int decay_w = 0);

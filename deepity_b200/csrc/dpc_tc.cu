@@ -81,6 +81,8 @@ struct TcState
   // l+1 = the layer above l): what the forward epilogue reads, staged through shared memory
   CUtensorMap zup_km, eup_km;
   bool up_maps = false;
+  CUtensorMap mu_st; // prediction of layer 0, for layers of the run above it (see first_from_mu)
+  bool mu_map = false;
   int* chain_counters = nullptr; // device: [layers of the run][row blocks]
   unsigned long long* trace = nullptr; // optional timing trace buffer of the chain kernel
   int max_smem = 0;
@@ -154,6 +156,9 @@ struct TcParams
   long long wait_cycles;        // limit of every bounded wait of this launch
   int fe_only;                  // the fp32 feedback error of the run's layers is not written
   int tstore;                   // the store maps of the launch are valid (staged epilogue outputs)
+  // Feedback: the error of the launch's first layer has not been computed; the epilogue takes
+  // z - mu of the layer below (a cached prediction) instead of reading it.
+  int first_from_mu;
 };
 
 // Chain mode: wait (bounded) until `target` epilogue warps have published one row block of the
@@ -694,7 +699,8 @@ template <int OP, int BN, int THREE_X, int BM = 128, bool PAIR = false, int KS =
 __global__ void __launch_bounds__(Cfg<OP, BN, THREE_X, BM, PAIR, KS>::THREADS, 1)
     pc_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                  const __grid_constant__ CUtensorMap mapU, const __grid_constant__ CUtensorMap mapSE,
-                 const __grid_constant__ CUtensorMap mapSF, const TcParams P)
+                 const __grid_constant__ CUtensorMap mapSF, const __grid_constant__ CUtensorMap mapM,
+                 const TcParams P)
 {
   using C = Cfg<OP, BN, THREE_X, BM, PAIR, KS>;
   extern __shared__ uint8_t smem_raw[];
@@ -1189,6 +1195,10 @@ __global__ void __launch_bounds__(Cfg<OP, BN, THREE_X, BM, PAIR, KS>::THREADS, 1
               ee[4 * i] = x.x, ee[4 * i + 1] = x.y, ee[4 * i + 2] = x.z, ee[4 * i + 3] = x.w;
               zz[4 * i] = y.x, zz[4 * i + 1] = y.y, zz[4 * i + 2] = y.z, zz[4 * i + 3] = y.w;
             }
+            if (P.first_from_mu && lrel == 0)
+#pragma unroll
+              for (int k = 0; k < 16; ++k)
+                ee[k] = zz[k] - ee[k];
             tc_ld16(taddr + c * 16, v);
             if (P.mode != FBP_BELIEF)
             {
@@ -1269,14 +1279,20 @@ __global__ void __launch_bounds__(Cfg<OP, BN, THREE_X, BM, PAIR, KS>::THREADS, 1
           if (nv <= 0)
             break;
           const size_t o = (size_t)m * P.N + n0 + c * 32;
+          const bool from_mu = P.first_from_mu && lrel == 0;
+          const float* e_src = from_mu ? P.layers[li - 1].mu : L.e;
           float ee[32], zz[32], v[32];
 #pragma unroll
           for (int k = 0; k < 32; k += 8)
           {
             if (k >= nv)
               continue;
-            ld8(L.e + o + k, &ee[k]);
+            ld8(e_src + o + k, &ee[k]);
             ld8(L.z + o + k, &zz[k]);
+            if (from_mu)
+#pragma unroll
+              for (int q = 0; q < 8; ++q)
+                ee[k + q] = zz[k + q] - ee[k + q];
           }
           tc_ld32(taddr + c * 32, v);
 #pragma unroll
@@ -1567,6 +1583,9 @@ __global__ void __launch_bounds__(Cfg<OP, BN, THREE_X, BM, PAIR, KS>::THREADS, 1
         const int m0 = (rem / P.tiles_n) * C::TILE_M + (int)rank * BM;
         const int n0 = (rem % P.tiles_n) * BN;
         const int lcoord = P.first + lrel - P.run_first;
+        const bool from_mu = P.first_from_mu && lrel == 0;
+        const CUtensorMap* emap = from_mu ? &mapM : &mapU;
+        const int ecoord = from_mu ? 0 : lcoord;
         for (int c = 0; c < BN / 16; ++c, ++q)
         {
           constexpr uint32_t NBUF = C::IN_BUFS > 0 ? C::IN_BUFS : 1;
@@ -1586,7 +1605,7 @@ __global__ void __launch_bounds__(Cfg<OP, BN, THREE_X, BM, PAIR, KS>::THREADS, 1
               tma_load_3d(ebuf + s4 * 2048, &mapSE, &in_full[b], n0 + 16 * c, m0 + 32 * s4, lcoord);
             else
             {
-              tma_load_3d(ebuf + s4 * 2048, &mapU, &in_full[b], n0 + 16 * c, m0 + 32 * s4, lcoord);
+              tma_load_3d(ebuf + s4 * 2048, emap, &in_full[b], n0 + 16 * c, m0 + 32 * s4, ecoord);
               tma_load_3d(zbuf + s4 * 2048, &mapSE, &in_full[b], n0 + 16 * c, m0 + 32 * s4, lcoord);
             }
           }
@@ -1812,11 +1831,13 @@ int launch(dpc_plan* p, TcState* st, const CUtensorMap& a, const CUtensorMap& b,
            const CUtensorMap* up = nullptr)
 {
   // forward: up = staged operand of the layer above, stores of errors and fe planes; feedback:
-  // loads of the layer's error, loads and stores of its belief, stores of the belief's planes
+  // loads of the layer's error (of the first layer: of the prediction below it), loads and stores
+  // of its belief, stores of the belief's planes
   const CUtensorMap& u = (OP == TC_FB && P.tstore) ? st->e_st : (up ? *up : a);
   const CUtensorMap& se = P.tstore ? (OP == TC_FB ? st->z_st : OP == TC_WG ? st->w_st : st->e_st) : a;
   const CUtensorMap& sf =
       P.tstore ? (OP == TC_FB ? st->zp_st : OP == TC_WG ? st->wp_st : st->fep_st) : a;
+  const CUtensorMap& mu = P.tstore && P.first_from_mu ? st->mu_st : a;
   using C = Cfg<OP, BN, THREE_X, BM, PAIR, KS>;
   static bool configured = false;
   auto kern = pc_tc_kernel<OP, BN, THREE_X, BM, PAIR, KS>;
@@ -1848,14 +1869,14 @@ int launch(dpc_plan* p, TcState* st, const CUtensorMap& a, const CUtensorMap& b,
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a, b, u, se, sf, P);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a, b, u, se, sf, mu, P);
     p->ctx->launches += 1;
     if (e != cudaSuccess)
       return cuda_fail(e, "tensor-core pair kernel launch");
     return DPC_OK;
   }
   const int grid = P.chain ? P.tiles_m * P.tiles_n : std::min(total, p->ctx->sm_count);
-  kern<<<grid, C::THREADS, C::SMEM_BYTES, p->ctx->stream>>>(a, b, u, se, sf, P);
+  kern<<<grid, C::THREADS, C::SMEM_BYTES, p->ctx->stream>>>(a, b, u, se, sf, mu, P);
   p->ctx->launches += 1;
   cudaError_t e = cudaPeekAtLastError();
   if (e != cudaSuccess)
@@ -2126,6 +2147,9 @@ static bool run_init(dpc_plan* plan, TcState* st, int best_first, int best_count
         make_store_map(&st->zp_st, st->zp, true, H, B, 2 * (best_count + 1), (int64_t)B * H) &&
         make_store_map(&st->w_st, L0.W, false, H, H, best_count, plan->run.w_stride) &&
         make_store_map(&st->wp_st, st->wp, true, H, H, 2 * best_count, (int64_t)H * H);
+    const dpc_layer& L1 = plan->h[0];
+    st->mu_map = L1.mu && L1.next_size == H && ((uintptr_t)L1.mu % 128) == 0 &&
+                 make_store_map(&st->mu_st, L1.mu, false, H, B, 1, (int64_t)B * H);
   }
   if (st->simple && !(st->planes && st->store_maps))
   {
@@ -2313,6 +2337,7 @@ static TcParams base_params(dpc_plan* p, TcState* st, int first, int count, int 
   P.wait_cycles = st->wait_cycles;
   P.fe_only = fe_only_now(p, st) ? 1 : 0;
   P.tstore = 0;
+  P.first_from_mu = 0;
   P.layers = p->d;
   P.first = first;
   P.count = count;
@@ -2486,7 +2511,7 @@ int tc_project_forward(dpc_plan* p, int first, int count, int flags)
   return rc;
 }
 
-int tc_update_state(dpc_plan* p, int first, int count, bool feed)
+int tc_update_state(dpc_plan* p, int first, int count, bool feed, bool first_from_mu)
 {
   auto* st = static_cast<TcState*>(p->tc);
   if (st && st->ok && count == 1 && !range_in_run(p, first, 1))
@@ -2503,6 +2528,7 @@ int tc_update_state(dpc_plan* p, int first, int count, bool feed)
     const bool planes = !tf32 && planes_on(p, st);
     const int bn = planes || tf32 ? pair_tile_width(p, count * (B / 256) * (H / 256), 128) : 256;
     TcParams P = base_params(p, st, first, count, B, H, H, bn, 0, 0, 256);
+    P.first_from_mu = first_from_mu ? 1 : 0;
     if (planes)
     {
       if ((rc = planes_need(p, st, PL_FE, r0, r0 + count)) != DPC_OK ||
@@ -2510,7 +2536,7 @@ int tc_update_state(dpc_plan* p, int first, int count, bool feed)
         return rc;
       // plain updates (no momentum, no residual term) take their error and belief through
       // shared memory and write belief and planes with bulk stores
-      bool plain = st->store_maps && !getenv("DPC_DISABLE_STAGED_OUTPUT") &&
+      bool plain = st->store_maps && (!first_from_mu || st->mu_map) && !getenv("DPC_DISABLE_STAGED_OUTPUT") &&
                    !getenv("DPC_DISABLE_STAGED_INPUT");
       for (int i = first; i < first + count && plain; ++i)
         plain = !p->h[i].v && !(p->h[i].flags & DPC_LAYER_RESIDUAL);
@@ -2526,14 +2552,15 @@ int tc_update_state(dpc_plan* p, int first, int count, bool feed)
       rc = scheme == 2 ? launch<TC_FB, 256, 2, 128, true>(p, st, st->fe_km, st->w_mn, P)
                        : launch<TC_FB, 256, 1, 128, true>(p, st, st->fe_km, st->w_mn, P);
   }
-  else if (tf32)
-    rc = launch<TC_FB, 256, 0>(p, st, st->fe_km, st->w_mn,
-                               base_params(p, st, first, count, B, H, H, 256, 0, 0));
   else
   {
-    TcParams P = base_params(p, st, first, count, B, H, H, 128, 0, 0);
-    rc = scheme == 2 ? launch<TC_FB, 128, 2>(p, st, st->fe_km, st->w_mn, P)
-                     : launch<TC_FB, 128, 1>(p, st, st->fe_km, st->w_mn, P);
+    TcParams P = base_params(p, st, first, count, B, H, H, tf32 ? 256 : 128, 0, 0);
+    P.first_from_mu = first_from_mu ? 1 : 0;
+    if (tf32)
+      rc = launch<TC_FB, 256, 0>(p, st, st->fe_km, st->w_mn, P);
+    else
+      rc = scheme == 2 ? launch<TC_FB, 128, 2>(p, st, st->fe_km, st->w_mn, P)
+                       : launch<TC_FB, 128, 1>(p, st, st->fe_km, st->w_mn, P);
   }
   if (rc == DPC_OK)
     planes_mark(st, PL_Z, r0, r0 + count, planes_kept(p, st) && (!st->simple || feed) ? 0 : 1);

@@ -122,8 +122,8 @@ public:
   void ProjectForward();
   float CalculateTerminalError();
   void DirectFeedbackUpdate();
-  float CalculateState(bool needEnergy);
-  void UpdateState(bool feedsForward = false); // a forward pass follows before UpdateWeights()
+  float CalculateState(bool needEnergy, bool skipInputError = false);
+  void UpdateState(bool feedsForward = false, bool firstFromPrediction = false); // a forward pass follows before UpdateWeights()
   float Step(bool computeEnergy = true);
   void UpdateWeights();
 
@@ -244,6 +244,8 @@ private:
   size_t gradCount = 0, gradWCount = 0;
   bool predictionsStale = false; // mu / preact in memory are older than the last energy pass
   bool sweepFeedsDfa = false; // inside a DirectKP train step, between sweep and direct feedback
+  void SettlePass(bool energy, bool feedsForward, bool last);
+  bool insidePhases = false, inputErrorZero = false; // see PhaseScope
   int transientFlag = 0; // DPC_FWD_TRANSIENT while a whole train step is being issued
   // key of the graph captured in slot s: mode*1e6+steps (train) or steps (predict); -1 none
   long graphKey[4] = {-1, -1, -1, -1};

@@ -318,8 +318,15 @@ DPC_API int dpc_epc_adjoint(dpc_plan* plan, int layer, int from_terminal, float 
  * may move on with the beliefs (a weight update uses f(z) as last fed to the forward product). */
 enum
 {
-  DPC_STATE_FEED = 1
+  DPC_STATE_FEED = 1,
+  /* The error of layer 1, the first of the range, has not been computed since its belief moved: the
+   * update takes z[1] - mu[0] (a clamped input layer's cached prediction) in its place and e[1] is
+   * neither read nor written.  Only where dpc_plan_state_from_prediction says so. */
+  DPC_STATE_FIRST_MU = 2
 };
+/* 1 when layer 1 is a tensor-core layer of the plan's run, whose state update can form its error from
+ * the prediction below (DPC_STATE_FIRST_MU). */
+DPC_API int dpc_plan_state_from_prediction(dpc_plan* plan);
 DPC_API int dpc_update_state_ex(dpc_plan* plan, int first, int count, int relax_from, int flags);
 /* z -= ir*e for one layer (the "output layer" branch of UpdateState). */
 DPC_API int dpc_relax(dpc_plan* plan, int layer);
