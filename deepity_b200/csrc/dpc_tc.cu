@@ -1670,17 +1670,28 @@ __global__ void __launch_bounds__(Cfg<OP, BN, THREE_X, BM, PAIR, KS>::THREADS, 1
         const float4* src = reinterpret_cast<const float4*>(stage_base + s * C::STAGE_BYTES);
         float4* dst = reinterpret_cast<float4*>(stage_base + s * C::STAGE_BYTES + C::A_BYTES +
                                                 C::B_BYTES);
-        constexpr int N4 = (C::A_BYTES + C::B_BYTES) / 16;
-#pragma unroll 4
-        for (int i = tid; i < N4; i += 128)
+        constexpr int N4 = (C::A_BYTES + C::B_BYTES) / 16; // a multiple of 256: tiles of 64 rows and more
+        // Half of the tile's loads before the first store: the products of a block wait for its
+        // remainders, and loads and stores taking turns four at a time made that 160 us instead of
+        // 153.5 for three 1024-wide layers at batch 4096 (all sixteen at once: the same).
+        constexpr int BATCH = N4 / 128 / 2;
+#pragma unroll
+        for (int i = tid; i < N4; i += 128 * BATCH)
         {
-          const float4 x = src[i];
-          float4 r;
-          r.x = x.x - __uint_as_float(__float_as_uint(x.x) & 0xffffe000u);
-          r.y = x.y - __uint_as_float(__float_as_uint(x.y) & 0xffffe000u);
-          r.z = x.z - __uint_as_float(__float_as_uint(x.z) & 0xffffe000u);
-          r.w = x.w - __uint_as_float(__float_as_uint(x.w) & 0xffffe000u);
-          dst[i] = r;
+          float4 x[BATCH];
+#pragma unroll
+          for (int q = 0; q < BATCH; ++q)
+            x[q] = src[i + 128 * q];
+#pragma unroll
+          for (int q = 0; q < BATCH; ++q)
+          {
+            float4 r;
+            r.x = x[q].x - __uint_as_float(__float_as_uint(x[q].x) & 0xffffe000u);
+            r.y = x[q].y - __uint_as_float(__float_as_uint(x[q].y) & 0xffffe000u);
+            r.z = x[q].z - __uint_as_float(__float_as_uint(x[q].z) & 0xffffe000u);
+            r.w = x[q].w - __uint_as_float(__float_as_uint(x[q].w) & 0xffffe000u);
+            dst[i + 128 * q] = r;
+          }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
