@@ -1,0 +1,115 @@
+"""The variants a launch is chosen from (GEMM tiles, widths of pair tiles, head kernels, the run of
+SimplePC layers, the state update that forms its own error) against the numpy oracle at the edges of
+their ranges.  Bounds: common.TOL per tensor (ADAM_TOL, TF32_TOL where those modes are on) and
+common.DELTA_TOL on the parameter updates."""
+import numpy as np
+import pytest
+
+from common import (ADAM_TOL, DELTA_TOL, DELTA_TOL_TF32, TF32_TOL, TOL, build_gpu_net, compare_outputs,
+                    initial_parameters, run_gpu, run_oracle)
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(kind, sizes, batch, act="tanh", T=3, steps=2, mode="train_step", lr=0.01, **options):
+    hyper = dict(lr=lr, ir=0.1, lmbda=0.0, act=act)
+    if kind != "simple":
+        hyper["fl"] = lr
+    return dict(kind=kind, sizes=sizes, batch=batch, T=T, steps=steps, hyper=hyper, options=options, mode=mode)
+
+
+def _check(case, name, precision="fp32"):
+    adam = "optimizer" in case["options"]
+    tol = TF32_TOL if precision == "tf32" else (ADAM_TOL if adam else TOL)
+    delta = DELTA_TOL_TF32 if precision == "tf32" else DELTA_TOL
+    compare_outputs(run_oracle(case), run_gpu(case, precision=precision), tol, name,
+                    init=None if adam else initial_parameters(case), delta_tol=None if adam else delta)
+
+
+GROUPED = {
+    # 32 x 32 tiles: one row over a tile, K not a multiple of the stage, rows not 16-byte aligned
+    "gemm_32_edges": _case("dkp", [33, 65, 31, 10], 65),
+    "gemm_32_aligned": _case("simple", [64, 96, 32, 4], 32, mode="projection"),
+    # as many 64 x 64 tiles as SMs and more
+    "gemm_64_edges": _case("dkp", [67, 641, 12], 961),
+    # the head kernels: partial groups of rows, one and two rows per warp, 16 units, softmax in the head
+    "head_ce": _case("full", [40, 128, 10], 301, "gelu", cross_entropy=1),
+    "head_ce_two_rows": _case("full", [40, 132, 16], 2051, cross_entropy=1),
+    "head_simple_ce": _case("simple", [40, 256, 10], 259, mode="projection", cross_entropy=1),
+    "head_simple": _case("simple", [40, 384, 13], 2051, mode="python"),
+    # column sums: more than one group of 32 columns, rows that end inside a buffer
+    "column_sums": _case("dkp", [24, 70, 33], 1031),
+}
+
+
+@pytest.mark.parametrize("name", sorted(GROUPED))
+def test_grouped_launches_match_oracle(name, built_library, monkeypatch):
+    monkeypatch.setenv("DPC_DISABLE_RESIDENT", "1")
+    _check(GROUPED[name], name)
+
+
+PAIR = {
+    "dkp": _case("dkp", [64] + [256] * 4 + [10], 256, T=4),
+    "full_residual_momentum": _case("full", [64] + [256] * 3 + [10], 512, "gelu", mupc=1, residual=1, momentum=0.9),
+}
+
+
+@pytest.mark.parametrize("width", ["64", "128", "256"])
+@pytest.mark.parametrize("precision", ["fp32", "tf32"])
+@pytest.mark.parametrize("name", sorted(PAIR))
+def test_pair_tile_widths_match_oracle(name, precision, width, built_library, monkeypatch):
+    monkeypatch.setenv("DPC_PAIR_TILE_WIDTH", width)
+    _check(PAIR[name], f"{name} {precision} {width}", precision)
+
+
+# The state update of the layer above the clamped input forms its error itself, except in the last pass:
+# one pass, several, single-CTA tiles (batch 128), 3xTF32 operands (Adam), a run that starts at the input
+FROM_PREDICTION = {
+    "one_pass": _case("dkp", [64] + [256] * 3 + [10], 256, T=1),
+    "single_cta": _case("full", [64] + [256] * 3 + [10], 128, "gelu", T=3),
+    "adam": _case("full", [64] + [256] * 3 + [10], 256, lr=1e-4, optimizer="ADAM", psi_optimizer="ADAM"),
+    "from_the_input": _case("dkp", [256] * 4 + [10], 256, T=3),
+    "ipc": _case("full", [64] + [256] * 3 + [10], 256, ipc=1),
+}
+
+
+@pytest.mark.parametrize("name", sorted(FROM_PREDICTION))
+def test_state_update_from_the_prediction_below(name, built_library):
+    _check(FROM_PREDICTION[name], name)
+
+
+SIMPLE_RUN = {
+    "train_step": _case("simple", [64] + [256] * 3 + [10], 256),
+    "projection": _case("simple", [64] + [256] * 3 + [10], 512, "gelu", mode="projection"),
+    "python": _case("simple", [256] * 4 + [10], 256, "sigmoid", mode="python"),
+    "softmax": _case("simple", [64] + [256] * 3 + [10], 256, mode="projection", cross_entropy=1),
+}
+
+
+@pytest.mark.parametrize("name", sorted(SIMPLE_RUN))
+def test_simple_layers_on_operand_planes(name, built_library, monkeypatch):
+    monkeypatch.setenv("DPC_RECTANGULAR_MIN_WORK", "0")
+    _check(SIMPLE_RUN[name], name)
+
+
+@pytest.mark.parametrize("sizes,batch", [((1000, 528, 10), 1152), ((1024, 512, 512, 10), 1024)])
+def test_single_layers_of_few_tiles(sizes, batch, built_library):
+    """Layers just over the tensor-core threshold: a quarter of the SMs' worth of full tiles or less."""
+    _check(_case("dkp", list(sizes), batch, T=2), str(sizes))
+
+
+@pytest.mark.parametrize("sizes,batch", [((20, 30, 5), 10), ((64, 256, 256, 256, 10), 256)])
+def test_rates_set_between_steps_take_effect(sizes, batch, built_library):
+    """A rate that is changed between two steps gives, bit for bit, what a network built with it gives."""
+    case = _case("dkp", list(sizes), batch)
+    a, x, y = build_gpu_net(case)
+    a.train_step(x, y, 2)
+    b, _, _ = build_gpu_net(dict(case, hyper=dict(case["hyper"], lr=0.03, ir=0.07)))
+    names = [(l, n) for l in range(len(sizes) - 1) for n in ("W", "b", "Psi")]
+    for l, n in names:
+        b.set_tensor(l, n, a.get_tensor(l, n))
+    a.set_learning_rate(0.03)
+    a.set_inference_rate(0.07)
+    assert a.train_step(x, y, 2) == b.train_step(x, y, 2)
+    for l, n in names:
+        assert np.array_equal(a.get_tensor(l, n), b.get_tensor(l, n)), (l, n)

@@ -1,0 +1,91 @@
+"""Row segments (dpc_resident.cu) and image segments (dpc_conv_resident.cu): whole settling loops in
+one kernel, against the numpy oracle, at the sizes where their splits change.  Bounds: common.TOL per
+tensor, common.ADAM_TOL with an Adam-type optimizer, common.DELTA_TOL on the parameter updates."""
+import ctypes
+
+import pytest
+
+from common import (ADAM_TOL, DELTA_TOL, TOL, build_gpu_net, compare_outputs, initial_parameters,
+                    run_gpu, run_oracle)
+from conv_common import build_conv_gpu_net, chain, run_conv_gpu, run_conv_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _available(case):
+    from deepity_b200 import _lib
+    lib = _lib.load()
+    lib.dpc_rows_available.argtypes, lib.dpc_rows_available.restype = [ctypes.c_void_p], ctypes.c_int
+    net, _, _ = build_gpu_net(case)
+    return lib.dpc_rows_available(lib.dpcn_plan(net._h))
+
+
+def _case(kind, sizes, batch, act, T=3, steps=2, **options):
+    hyper = dict(lr=0.01, ir=0.1, lmbda=0.0, act=act)
+    if options.get("optimizer"):
+        hyper["lr"] = 1e-3
+    if kind != "simple":
+        hyper["fl"] = hyper["lr"]
+    mode = options.pop("mode", "train_step")
+    return dict(kind=kind, sizes=sizes, batch=batch, T=T, steps=steps, hyper=hyper, options=options, mode=mode)
+
+
+ROWS = {
+    # 1, 2, 4 and 8 rows per block (148 SMs), the last block not full
+    "rows_1": _case("simple", [37, 70, 10], 147, "sigmoid", mode="projection"),
+    "rows_2": _case("dkp", [37, 70, 33, 10], 149, "tanh"),
+    "rows_4": _case("simple", [20, 33, 7], 299, "gelu", mode="python"),
+    "rows_8": _case("dkp", [16, 40, 40, 5], 601, "tanh"),
+    "rows_8_two_groups": _case("simple", [12, 24, 4], 1201, "tanh"),
+    # ordered sums (Adam-type optimizers, kinked activations) with streamed rows
+    "exact_adamw": _case("dkp", [100, 300, 200, 77, 10], 50, "relu", optimizer="ADAMW", psi_optimizer="ADAM"),
+    "exact_hard_tanh": _case("simple", [30, 129, 65, 3], 151, "hard_tanh"),
+    # every term of the state update, more layers than warps share evenly
+    "residual_momentum": _case("full", [33] + [64] * 9 + [10], 5, "gelu", mupc=1, residual=1, momentum=0.9),
+    "cross_entropy": _case("full", [45, 61, 32, 17], 149, "tanh", cross_entropy=1),
+    "simple_cross_entropy": _case("simple", [45, 61, 17], 9, "tanh", cross_entropy=1),
+    # weights beyond one SM's shared memory: some layers or rows are read from L2 on every pass
+    "streamed": _case("dkp", [64, 400, 350, 10], 20, "tanh"),
+}
+
+
+@pytest.mark.parametrize("name", sorted(ROWS))
+def test_row_segments_match_oracle(name, built_library):
+    case = ROWS[name]
+    assert _available(case) == 1
+    adam = "optimizer" in case["options"]
+    compare_outputs(run_oracle(case), run_gpu(case), ADAM_TOL if adam else TOL, name,
+                    init=None if adam else initial_parameters(case), delta_tol=None if adam else DELTA_TOL)
+
+
+def test_row_segments_stop_at_their_weight_limit(built_library):
+    case = _case("dkp", [64, 450, 400, 10], 20, "tanh")  # 736 KB above the first layer
+    assert _available(case) == 0
+    compare_outputs(run_oracle(case), run_gpu(case), TOL, "over the limit")
+
+
+def _images(shape, convs, act, batch, **kw):
+    return dict(layers=chain(shape, convs, act), batch=batch, T=3, steps=2, hyper=dict(lr=0.005, ir=0.1, lmbda=0.0),
+                **kw)
+
+
+IMAGES = {
+    # more images than SMs; rectangular kernels, strides and paddings that leave ragged tiles
+    "batch_over_sms": _images((1, 10, 10), [(8, 5, 5, 2, 2, 2, 2), (10, 5, 5, 1, 1, 0, 0)], "tanh", 151),
+    "rectangular": _images((2, 11, 9), [(9, 3, 2, 2, 1, 1, 0), (17, 2, 3, 1, 2, 0, 1), (5, 5, 4, 1, 1, 0, 0)],
+                           "sigmoid", 3),
+    # channel counts one off the 8- and 16-wide tiles, a projection sweep first
+    "channel_edges": _images((7, 8, 8), [(15, 3, 3, 1, 1, 1, 1), (33, 3, 3, 2, 2, 1, 1), (1, 4, 4, 1, 1, 0, 0)],
+                             "gelu", 2, projection=1),
+    "pointwise": _images((3, 4, 4), [(16, 1, 1, 1, 1, 0, 0), (10, 4, 4, 1, 1, 0, 0)], "relu", 1),
+}
+
+
+@pytest.mark.parametrize("name", sorted(IMAGES))
+def test_image_segments_match_oracle(name, built_library):
+    from deepity_b200 import _lib
+    lib = _lib.load()
+    lib.dpc_conv_images_available.argtypes, lib.dpc_conv_images_available.restype = [ctypes.c_void_p], ctypes.c_int
+    case = IMAGES[name]
+    assert lib.dpc_conv_images_available(lib.dpcn_conv_plan(build_conv_gpu_net(case)._h)) == 1
+    compare_outputs(run_conv_oracle(case), run_conv_gpu(case), TOL, name)
