@@ -57,6 +57,11 @@ SIGNATURES = {
     "dpc_error": (_i, [_vp, _i, _i]),
     "dpc_feedback_error": (_i, [_vp, _i, _i]),
     "dpc_update_state": (_i, [_vp, _i, _i]),
+    "dpc_update_state_ex": (_i, [_vp, _i, _i, _i, _i]),
+    "dpc_plan_fused_cross_entropy": (_i, [_vp]),
+    "dpc_plan_state_from_prediction": (_i, [_vp]),
+    "dpc_rows_available": (_i, [_vp]),
+    "dpc_rows_segment": (_i, [_vp, _i, _i, _i, _i]),
     "dpc_epc_reconstruct": (_i, [_vp, _i]),
     "dpc_epc_adjoint": (_i, [_vp, _i, _i, _f, _i]),
     "dpc_relax": (_i, [_vp, _i]),
@@ -67,6 +72,8 @@ SIGNATURES = {
     "dpc_error_energy_static": (_i, [_vp, _vp, _vp, _vp, _i64, _vp]),
     "dpc_energy_reset": (_i, [_vp]),
     "dpc_energy_read": (_i, [_vp, ctypes.POINTER(ctypes.c_double)]),
+    "dpc_energy_fetch": (_i, [_vp]),
+    "dpc_energy_wait": (_i, [_vp, ctypes.POINTER(ctypes.c_double)]),
     "dpcn_create": (_i, [_i, _i, _i, ctypes.POINTER(_vp)]),
     "dpcn_destroy": (_i, [_vp]),
     "dpcn_add_layer": (_i, [_vp, _i, _i, _i, _f, _f, _f, _f, _i]),
@@ -100,8 +107,13 @@ SIGNATURES = {
     "dpc_conv_update_state": (_i, [_vp, _i]),
     "dpc_conv_gate_with_prediction": (_i, [_vp, _i]),
     "dpc_conv_update_weights": (_i, [_vp, _i, _i]),
+    "dpc_conv_update_weights_range": (_i, [_vp, _i, _i, _i]),
+    "dpc_conv_images_available": (_i, [_vp]),
+    "dpc_conv_images_segment": (_i, [_vp, _i, _i, _i]),
     "dpc_conv_energy_reset": (_i, [_vp]),
     "dpc_conv_energy_read": (_i, [_vp, ctypes.POINTER(ctypes.c_double)]),
+    "dpc_conv_energy_fetch": (_i, [_vp]),
+    "dpc_conv_energy_wait": (_i, [_vp, ctypes.POINTER(ctypes.c_double)]),
     "dpcn_conv_create": (_i, [_i, _i, ctypes.POINTER(_vp)]),
     "dpcn_conv_destroy": (_i, [_vp]),
     "dpcn_conv_add_layer": (_i, [_vp] + [_i] * 10 + [_f] * 3 + [_i]),

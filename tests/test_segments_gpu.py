@@ -1,8 +1,6 @@
 """Row segments (dpc_resident.cu) and image segments (dpc_conv_resident.cu): whole settling loops in
 one kernel, against the numpy oracle, at the sizes where their splits change.  Bounds: common.TOL per
 tensor, common.ADAM_TOL with an Adam-type optimizer, common.DELTA_TOL on the parameter updates."""
-import ctypes
-
 import pytest
 
 from common import (ADAM_TOL, DELTA_TOL, TOL, build_gpu_net, compare_outputs, initial_parameters,
@@ -15,7 +13,6 @@ pytestmark = pytest.mark.gpu
 def _available(case):
     from deepity_b200 import _lib
     lib = _lib.load()
-    lib.dpc_rows_available.argtypes, lib.dpc_rows_available.restype = [ctypes.c_void_p], ctypes.c_int
     net, _, _ = build_gpu_net(case)
     return lib.dpc_rows_available(lib.dpcn_plan(net._h))
 
@@ -85,7 +82,6 @@ IMAGES = {
 def test_image_segments_match_oracle(name, built_library):
     from deepity_b200 import _lib
     lib = _lib.load()
-    lib.dpc_conv_images_available.argtypes, lib.dpc_conv_images_available.restype = [ctypes.c_void_p], ctypes.c_int
     case = IMAGES[name]
     assert lib.dpc_conv_images_available(lib.dpcn_conv_plan(build_conv_gpu_net(case)._h)) == 1
     compare_outputs(run_conv_oracle(case), run_conv_gpu(case), TOL, name)
