@@ -1180,6 +1180,15 @@ static int launch_dfa_group(dpc_plan* p, int i, int c, int from_output, bool v, 
     wide = p->h[k].next_size <= 0 || p->h[k].next_size % 128 == 0;
   const int ts4 = cdiv(std::max(p->h[i].terminal_size, 1), 4);
   const long long strips = (long long)cdiv(mxn, 128) * c;
+  // rows per block of the other two: 32, fewer while SMs are left without a block (the rows of a block
+  // follow one another: 8 blocks of 32 rows took 24 us for 100-300-200-77-10 at batch 50)
+  auto few_rows = [&](int blocks)
+  {
+    int rpb = 32;
+    while (rpb > 4 && (long long)blocks * cdiv(p->batch, rpb) < p->ctx->sm_count)
+      rpb /= 2;
+    return rpb;
+  };
   if (wide && ts4 <= 4)
   {
     // blocks of 128 columns x the whole batch, or a share of it while there are fewer than four blocks
@@ -1199,8 +1208,9 @@ static int launch_dfa_group(dpc_plan* p, int i, int c, int from_output, bool v, 
   }
   else if (v)
   {
-    const int rpb =
-        cdiv(mxn, 256) * cdiv(p->batch, DFA4_ROWS) * c >= 4 * p->ctx->sm_count ? DFA4_ROWS : 32;
+    int rpb = DFA4_ROWS;
+    if (cdiv(mxn, 256) * cdiv(p->batch, rpb) * c < 4 * p->ctx->sm_count)
+      rpb = few_rows(cdiv(mxn, 256) * c);
     dim3 grid(cdiv(mxn, 256), cdiv(p->batch, rpb), c);
     if (ts4 <= 1)
       dfa_proj4_kernel<1><<<grid, 64, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, rpb, planes);
@@ -1213,8 +1223,9 @@ static int launch_dfa_group(dpc_plan* p, int i, int c, int from_output, bool v, 
   }
   else
   {
-    dim3 grid(cdiv(mxn, 128), cdiv(p->batch, DFA_ROWS), c);
-    dfa_proj_kernel<<<grid, 128, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output);
+    const int rpb = few_rows(cdiv(mxn, 128) * c);
+    dim3 grid(cdiv(mxn, 128), cdiv(p->batch, rpb), c);
+    dfa_proj_kernel<<<grid, 128, 0, st>>>(p->d, i, p->n, p->batch, p->e_terminal, from_output, rpb);
   }
   int rc = check_launch(p->ctx, "dfa_proj kernel");
   if (rc != DPC_OK)

@@ -894,11 +894,13 @@ __global__ void relax_kernel(const dpc_layer* __restrict__ layers, int first, in
 }
 
 // DFA projection: fe[l] = (e_T · Psi[l+1]^T) * f'(preact[l])   (K = terminal_size).
-// One thread per output unit j with its Psi row in registers; a block covers DFA_ROWS batch
-// rows whose terminal errors sit in shared memory, so preact/fe stream through coalesced.
+// One thread per output unit j with its Psi row in registers; a block covers rows_per_block (at most
+// DFA_ROWS) batch rows whose terminal errors sit in shared memory, so preact/fe stream through
+// coalesced.
 constexpr int DFA_ROWS = 32;
 __global__ void dfa_proj_kernel(const dpc_layer* __restrict__ layers, int first, int n_layers,
-                                int batch, const float* __restrict__ eT, int from_output)
+                                int batch, const float* __restrict__ eT, int from_output,
+                                int rows_per_block)
 {
   const int li = first + blockIdx.z;
   if (li + 1 >= n_layers)
@@ -908,7 +910,7 @@ __global__ void dfa_proj_kernel(const dpc_layer* __restrict__ layers, int first,
   if (L.next_size <= 0 || Lup.Psi == nullptr)
     return;
   const int TS = L.terminal_size, n = L.next_size;
-  const int b0 = blockIdx.y * DFA_ROWS;
+  const int b0 = blockIdx.y * rows_per_block;
   if (b0 >= batch || (int)(blockIdx.x * blockDim.x) >= n)
     return;
   __shared__ __align__(16) float es[DFA_ROWS][16];
@@ -916,7 +918,7 @@ __global__ void dfa_proj_kernel(const dpc_layer* __restrict__ layers, int first,
   {
     const int kn = min(16, TS - kc);
     __syncthreads();
-    for (int idx = threadIdx.x; idx < DFA_ROWS * 16; idx += blockDim.x)
+    for (int idx = threadIdx.x; idx < rows_per_block * 16; idx += blockDim.x)
     {
       const int r = idx >> 4, k = idx & 15;
       es[r][k] = (b0 + r < batch && k < kn) ? eT[(size_t)(b0 + r) * TS + kc + k] : 0.0f;
@@ -932,7 +934,7 @@ __global__ void dfa_proj_kernel(const dpc_layer* __restrict__ layers, int first,
         psi[k] = k < kn ? pr[k] : 0.0f;
       const bool last = kc + 16 >= TS;
 #pragma unroll 4
-      for (int r = 0; r < DFA_ROWS; ++r)
+      for (int r = 0; r < rows_per_block; ++r)
       {
         if (b0 + r >= batch)
           break;
@@ -976,12 +978,11 @@ __device__ __forceinline__ __nv_bfloat16* fe_plane_of(const FePlanes& P, int li)
              : nullptr;
 }
 
-// The same projection, four output units per thread with 128-bit accesses, for the common
 // Rows per block of the aligned kernel: its per-thread rows of Psi are strided 4-byte loads that
 // cost as much L2 traffic as 32 rows of useful data, so a block amortises them over up to 128 rows
 // (the host picks fewer when that would leave SMs without a block).
 constexpr int DFA4_ROWS = 128;
-// aligned case: next_size a multiple of 4, terminal_size <= 4*TS4, 16-byte aligned rows.
+// The same projection, four output units per thread with 128-bit accesses, for the common aligned case: next_size a multiple of 4, terminal_size <= 4*TS4, 16-byte aligned rows.
 template <int TS4>
 __global__ void __launch_bounds__(64)
     dfa_proj4_kernel(const dpc_layer* __restrict__ layers, int first, int n_layers, int batch,
