@@ -18,7 +18,8 @@
 // are one 16-byte load, kDepth of them in flight.  mma.sync and not tcgen05: the products
 // of one image are 16..128 x 64..256 x 64..576, far below a 128-row tile.
 // Layers whose output is one pixel (dense heads) are dot products on the CUDA cores.
-// What bounds it: the tensor pipe and L2 bandwidth of the SM about equally.
+// What bounds it: the SM's load path -- every task reads its weight fragments again, 16 bytes a lane per
+// k step -- and behind it the tensor pipe.  32x32x3 network at batch 128, 10 steps: 4.57 -> 0.70 ms a step.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>

@@ -756,24 +756,24 @@ __global__ void cached_forward_kernel(const dpc_layer* __restrict__ layers, int 
       }
     }
     else
-    for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < total;
-         o += (size_t)gridDim.x * blockDim.x)
-    {
-      const float mu = L.mu[o];
-      if (do_copy)
-        Lup->z[o] = mu;
-      float e = 0.0f;
-      if (do_err)
+      for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < total;
+           o += (size_t)gridDim.x * blockDim.x)
       {
-        e = (do_copy ? mu : Lup->z[o]) - mu;
-        Lup->e[o] = e;
-        esum += e * e;
+        const float mu = L.mu[o];
+        if (do_copy)
+          Lup->z[o] = mu;
+        float e = 0.0f;
+        if (do_err)
+        {
+          e = (do_copy ? mu : Lup->z[o]) - mu;
+          Lup->e[o] = e;
+          esum += e * e;
+        }
+        else if (do_fe)
+          e = Lup->e[o];
+        if (do_fe)
+          L.fe[o] = e * act_deriv(L.act, L.preact[o]);
       }
-      else if (do_fe)
-        e = Lup->e[o];
-      if (do_fe)
-        L.fe[o] = e * act_deriv(L.act, L.preact[o]);
-    }
   }
   if (flags & DPC_FWD_ENERGY)
     block_energy_add(esum, energy);

@@ -506,7 +506,7 @@ __device__ __forceinline__ void fwd_epilogue_tile(const TcParams& P, const FwdMe
           *in->defer_o = o;
         }
         else
-        st8(up_z + o + k, mu);
+          st8(up_z + o + k, mu);
         if (L.upz_hi)
           st_planes8(L.upz_hi, P.act_elems, o + k, mu);
       }
@@ -2103,16 +2103,16 @@ static bool run_init(dpc_plan* plan, TcState* st, int best_first, int best_count
   bool ok = true;
   if (!st->simple)
   {
-  ok &= make_map(&st->z_km, L0.z, H, B, best_count, plan->run.z_stride, TBM, false);
-  ok &= make_map(&st->z_km64, L0.z, H, B, best_count, plan->run.z_stride, 64, false);
-  ok &= make_map(&st->fe_km, L0.fe, H, B, best_count, plan->run.out_stride, TBM, false);
-  ok &= make_map(&st->w_km32, L0.W, H, H, best_count, plan->run.w_stride, 32, false);
-  ok &= make_map(&st->w_km64, L0.W, H, H, best_count, plan->run.w_stride, 64, false);
-  ok &= make_map(&st->w_km128, L0.W, H, H, best_count, plan->run.w_stride, 128, false);
-  ok &= make_map(&st->w_km256, L0.W, H, H, best_count, plan->run.w_stride, 256, false);
-  ok &= make_map(&st->z_mn, L0.z, H, B, best_count, plan->run.z_stride, 32, true);
-  ok &= make_map(&st->fe_mn, L0.fe, H, B, best_count, plan->run.out_stride, 32, true);
-  ok &= make_map(&st->w_mn, L0.W, H, H, best_count, plan->run.w_stride, 32, true);
+    ok &= make_map(&st->z_km, L0.z, H, B, best_count, plan->run.z_stride, TBM, false);
+    ok &= make_map(&st->z_km64, L0.z, H, B, best_count, plan->run.z_stride, 64, false);
+    ok &= make_map(&st->fe_km, L0.fe, H, B, best_count, plan->run.out_stride, TBM, false);
+    ok &= make_map(&st->w_km32, L0.W, H, H, best_count, plan->run.w_stride, 32, false);
+    ok &= make_map(&st->w_km64, L0.W, H, H, best_count, plan->run.w_stride, 64, false);
+    ok &= make_map(&st->w_km128, L0.W, H, H, best_count, plan->run.w_stride, 128, false);
+    ok &= make_map(&st->w_km256, L0.W, H, H, best_count, plan->run.w_stride, 256, false);
+    ok &= make_map(&st->z_mn, L0.z, H, B, best_count, plan->run.z_stride, 32, true);
+    ok &= make_map(&st->fe_mn, L0.fe, H, B, best_count, plan->run.out_stride, 32, true);
+    ok &= make_map(&st->w_mn, L0.W, H, H, best_count, plan->run.w_stride, 32, true);
   }
   if (!ok)
   {
@@ -2319,8 +2319,7 @@ static bool fe_only_now(const dpc_plan* p, const TcState* st)
 // tiles re-read less of A and win where there are many waves.
 static int pair_tile_width(const dpc_plan* p, int tiles256, int narrowest)
 {
-  static const char* env = getenv("DPC_PAIR_TILE_WIDTH"); // (for comparing the variants)
-  if (env)
+  if (const char* env = getenv("DPC_PAIR_TILE_WIDTH")) // (for comparing the variants)
     return std::max(atoi(env), narrowest);
   const int pairs = p->ctx->sm_count / 2;
   int best = 256;
