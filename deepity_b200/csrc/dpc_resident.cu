@@ -1291,9 +1291,13 @@ int res_plan_init(dpc_plan* p)
     if ((L.flags & DPC_LAYER_SOFTMAX_CE) || (l > 0 && tc_extra_layer(p, l)))
       return 1;
   }
-  const size_t max_stream = 640 * 1024;
+  // Weights above the first layer that pay, against the phase kernels (10 settling steps of a DKP network,
+  // us a step at batch 50 / 300 / 1000).  Sliced sums: 245/437/737 against 416/566/930 at 647 KB.  Ordered
+  // sums read streamed weights in longer chains: 207/318/526 against 302/349/550 at 272 KB, 291/393/752
+  // against 340/386/649 at 404 KB, 399/576/2946 against 368/456/1246 at 605 KB.
+  const size_t kb = 1024, max_stream = !exact ? 640 * kb : p->batch <= p->ctx->sm_count ? 448 * kb : 320 * kb;
   const size_t w0 = sizeof(float) * (size_t)p->h[0].size * p->h[0].next_size;
-  if (wbytes > max_stream || w0 > 4 * max_stream)
+  if (wbytes > max_stream || w0 > 2560 * kb)
     return 1;
   int R = 1;
   while (R < 8 && (p->batch + R - 1) / R > p->ctx->sm_count)

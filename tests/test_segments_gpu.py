@@ -55,8 +55,11 @@ def test_row_segments_match_oracle(name, built_library):
                     init=None if adam else initial_parameters(case), delta_tol=None if adam else DELTA_TOL)
 
 
-def test_row_segments_stop_at_their_weight_limit(built_library):
-    case = _case("dkp", [64, 450, 400, 10], 20, "tanh")  # 736 KB above the first layer
+@pytest.mark.parametrize("sizes,batch,act", [((64, 450, 400, 10), 20, "tanh"),   # 736 KB above the first layer
+                                             ((64, 384, 384, 10), 20, "relu"),   # 605 KB, ordered sums
+                                             ((64, 384, 256, 10), 149, "relu")])  # 404 KB, two rows a block
+def test_row_segments_stop_at_their_weight_limit(sizes, batch, act, built_library):
+    case = _case("dkp", list(sizes), batch, act)
     assert _available(case) == 0
     compare_outputs(run_oracle(case), run_gpu(case), TOL, "over the limit")
 
