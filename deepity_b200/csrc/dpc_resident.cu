@@ -1275,6 +1275,7 @@ int res_plan_init(dpc_plan* p)
     return 1;
   size_t wbytes = 0;
   int S = 0;
+  int longest = 0;
   bool has_v = false, exact = false;
   for (int l = 0; l < nw; ++l)
   {
@@ -1285,23 +1286,32 @@ int res_plan_init(dpc_plan* p)
         ((L.flags ^ p->h[0].flags) & DPC_LAYER_INPUT_ACT) || (l == 0 && (L.flags & DPC_LAYER_RESIDUAL)))
       return 1;
     if (l > 0)
+    {
       wbytes += sizeof(float) * (size_t)L.size * L.next_size;
+      longest = std::max(longest, std::max(L.size, L.next_size));
+    }
     has_v |= L.v != nullptr && l > 0;
     S += up4(L.next_size);
     if ((L.flags & DPC_LAYER_SOFTMAX_CE) || (l > 0 && tc_extra_layer(p, l)))
       return 1;
   }
-  // Weights above the first layer that pay, against the phase kernels (10 settling steps of a DKP network,
-  // us a step at batch 50 / 300 / 1000).  Sliced sums: 245/437/737 against 416/566/930 at 647 KB.  Ordered
-  // sums read streamed weights in longer chains: 207/318/526 against 302/349/550 at 272 KB, 291/393/752
-  // against 340/386/649 at 404 KB, 399/576/2946 against 368/456/1246 at 605 KB.
-  const size_t kb = 1024, max_stream = !exact ? 640 * kb : p->batch <= p->ctx->sm_count ? 448 * kb : 320 * kb;
   const size_t w0 = sizeof(float) * (size_t)p->h[0].size * p->h[0].next_size;
-  if (wbytes > max_stream || w0 > 2560 * kb)
-    return 1;
   int R = 1;
   while (R < 8 && (p->batch + R - 1) / R > p->ctx->sm_count)
     R *= 2;
+  // Weights above the first layer that pay, against the phase kernels.  A segment's time grows with all
+  // weights of a pass, a phase kernel's with the longest sum of one of its layers (`longest`), since it
+  // takes the layers side by side.  Measured, segments / phase kernels in us a step of a DKP network with
+  // 10 settling steps at batch 50, 300, 1000:
+  //   sliced    64-512-310-10 (647 KB)  245/416  437/566  737/930    64-640-500-10  320/482  674/730  1090/1265
+  //             64-(128x10)-10 (596 KB) 263/283  418/383  747/698    64-(64x38)-10  413/372  720/561  1434/993
+  //             64-800-700-10  478/572, 1851/1242 at batch 600       64-(300x4)-10  368/335  628/558  1178/1040
+  //   ordered   64-256-256-10 (272 KB)  207/302  318/349  526/550    64-384-256-10  291/340  393/386  752/649
+  //             64-384-384-10 (605 KB)  399/368  576/456  2946/1246  64-512-310-10  429/415  621/566  1211/930
+  const double limit_kb = exact ? (R == 1 ? 100 + 1.0 * longest : 60 + 0.85 * longest)
+                                : (R == 1 ? 300 + 2.5 * longest : 100 + 2.5 * longest);
+  if (wbytes > limit_kb * 1024 || w0 > 2560 * 1024)
+    return 1;
   for (; R >= 1; R /= 2)
   {
     const int rc = build(p, R, S, has_v, exact);

@@ -55,7 +55,8 @@ def test_row_segments_match_oracle(name, built_library):
                     init=None if adam else initial_parameters(case), delta_tol=None if adam else DELTA_TOL)
 
 
-@pytest.mark.parametrize("sizes,batch,act", [((64, 450, 400, 10), 20, "tanh"),   # 736 KB above the first layer
+@pytest.mark.parametrize("sizes,batch,act", [((64, 1024, 1000, 10), 9, "tanh"),  # 4 MB above the first layer
+                                             ((64,) + (128,) * 10 + (10,), 149, "tanh"),  # short sums, many layers
                                              ((64, 384, 384, 10), 20, "relu"),   # 605 KB, ordered sums
                                              ((64, 384, 256, 10), 149, "relu")])  # 404 KB, two rows a block
 def test_row_segments_stop_at_their_weight_limit(sizes, batch, act, built_library):
