@@ -105,6 +105,8 @@ SIGNATURES = {
     "dpc_conv_plan_destroy": (_i, [_vp]),
     "dpc_conv_forward": (_i, [_vp, _i, _i]),
     "dpc_conv_update_state": (_i, [_vp, _i]),
+    "dpc_conv_forward_range": (_i, [_vp, _i, _i, _i]),
+    "dpc_conv_update_state_range": (_i, [_vp, _i, _i]),
     "dpc_conv_gate_with_prediction": (_i, [_vp, _i]),
     "dpc_conv_update_weights": (_i, [_vp, _i, _i]),
     "dpc_conv_update_weights_range": (_i, [_vp, _i, _i, _i]),

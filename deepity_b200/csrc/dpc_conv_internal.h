@@ -12,7 +12,7 @@ struct dpc_conv_plan
   dpc_conv_layer* d = nullptr; // device copy of the table
   double* energy = nullptr;
   double* energy_host = nullptr;
-  float* scratch = nullptr; // one state-sized buffer for split state updates (largest layer)
+  float* scratch = nullptr; // sums of split state updates, one buffer per layer
   size_t scratch_floats = 0;
   void* res = nullptr; // image-resident path state, owned by dpc_conv_resident.cu
 };

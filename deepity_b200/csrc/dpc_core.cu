@@ -715,8 +715,7 @@ static int forward_simt(dpc_plan* p, int first, int count, int flags)
 // The launches of one phase are independent of each other, and most of them leave SMs idle -- a head,
 // a cached input layer, a bias sum beside the tensor-core run -- so one after the other they would add
 // their latencies.
-using Job = std::function<int()>;
-static int run_side_by_side(dpc_ctx* ctx, const std::vector<Job>& jobs)
+int dpc::run_side_by_side(dpc_ctx* ctx, const std::vector<Job>& jobs)
 {
   int rc = DPC_OK;
   if (jobs.size() < 2 || !ctx->fork_ev)

@@ -304,11 +304,21 @@ float SimpleConvPCNetwork::CalculateState(bool needEnergy)
   const int n = (int)layers.size();
   // The bottom layer has no prediction from below: its error is zero.
   Check(dpc_zero(ctx, layers[0]->d.e, (size_t)batchSize * layers[0]->GetInputSize() * sizeof(float)));
+  const int flags = DPC_CONV_ERR_NEXT | (needEnergy ? DPC_CONV_ENERGY : 0);
+  int first = 0; // the clamped input fills its cache alone, or uses it beside the others
+  if (layers[0]->clamped && !layers[0]->cacheValid && n > 1)
+    ForwardLayer(first++, flags);
+  bool together = true;
+  for (int i = 1; i + 1 < n; ++i)
+    together = together && !layers[i]->clamped;
+  if (together && first + 1 < n)
+    Check(dpc_conv_forward_range(plan, first, n - 1 - first,
+                                 flags | (first == 0 && layers[0]->clamped ? DPC_CONV_CACHED : 0)));
+  else
+    for (int i = first; i + 1 < n; ++i)
+      ForwardLayer(i, flags);
   for (int i = 0; i + 1 < n; ++i)
-  {
-    ForwardLayer(i, DPC_CONV_ERR_NEXT | (needEnergy ? DPC_CONV_ENERGY : 0));
     layers[i]->gateIsPrediction = true;
-  }
   return 0.0f; // the energy stays in the plan's device accumulator
 }
 
@@ -319,12 +329,16 @@ void SimpleConvPCNetwork::UpdateState()
   const int n = (int)layers.size();
   for (int i = 0; i < n; ++i)
   {
-    SimpleConvPCLayer* l = layers[i].get();
-    if (l->d.out_c > 0)
-      l->gateIsPrediction = false; // the reference overwrites mu with f'(preact) here
-    if (l->clamped)
-      continue;
-    Check(dpc_conv_update_state(plan, i));
+    if (layers[i]->d.out_c > 0)
+      layers[i]->gateIsPrediction = false; // the reference overwrites mu with f'(preact) here
+  }
+  for (int i = 0, end; i < n; i = std::max(i + 1, end))
+  {
+    for (end = i; end < n && !layers[end]->clamped; ++end)
+    {
+    }
+    if (end > i)
+      Check(dpc_conv_update_state_range(plan, i, end - i));
   }
 }
 

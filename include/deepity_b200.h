@@ -547,6 +547,10 @@ DPC_API int dpc_conv_forward(dpc_conv_plan* plan, int layer, int flags);
 /* UpdateState (SimpleConvPCLayer.cpp:302-400): z += ir*(W^T (*) g - e), the transposed
  * convolution written as a gather; a layer without weights relaxes, z -= ir*e. */
 DPC_API int dpc_conv_update_state(dpc_conv_plan* plan, int layer);
+/* The same for layers [first, first+count) side by side, as within a settling pass.  DPC_CONV_CACHED
+ * applies to the first layer of the range; DPC_CONV_COPY_NEXT is refused. */
+DPC_API int dpc_conv_forward_range(dpc_conv_plan* plan, int first, int count, int flags);
+DPC_API int dpc_conv_update_state_range(dpc_conv_plan* plan, int first, int count);
 /* g = e_above * mu: the gate the reference's UpdateWeights sees when no UpdateState ran since
  * the last CalculateState (its mu buffer then still holds the prediction, :414). */
 DPC_API int dpc_conv_gate_with_prediction(dpc_conv_plan* plan, int layer);

@@ -7,6 +7,7 @@ import pytest
 
 from common import (ADAM_TOL, DELTA_TOL, DELTA_TOL_TF32, TF32_TOL, TOL, build_gpu_net, compare_outputs,
                     initial_parameters, run_gpu, run_oracle)
+from conv_common import chain, run_conv_gpu, run_conv_oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -113,3 +114,12 @@ def test_rates_set_between_steps_take_effect(sizes, batch, built_library):
     assert a.train_step(x, y, 2) == b.train_step(x, y, 2)
     for l, n in names:
         assert np.array_equal(a.get_tensor(l, n), b.get_tensor(l, n)), (l, n)
+
+
+@pytest.mark.parametrize("act,batch,projection", [("tanh", 3, 0), ("sigmoid", 1, 1)])
+def test_convolution_layers_side_by_side(act, batch, projection, built_library, monkeypatch):
+    monkeypatch.setenv("DPC_DISABLE_RESIDENT", "1")
+    case = dict(layers=chain((2, 9, 9), [(5, 3, 3, 1, 1, 1, 1), (70, 3, 3, 2, 2, 1, 1), (9, 3, 3, 1, 1, 0, 0),
+                                         (4, 3, 3, 1, 1, 0, 0)], act),
+                batch=batch, T=4, steps=2, projection=projection, hyper=dict(lr=0.005, ir=0.1, lmbda=0.0))
+    compare_outputs(run_conv_oracle(case), run_conv_gpu(case), TOL, "convolutions")
