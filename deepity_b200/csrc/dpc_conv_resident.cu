@@ -518,8 +518,11 @@ __global__ void __launch_bounds__(kThreads, 1) conv_resident_kernel(const RcPara
       __syncthreads();
     }
     else
+    {
       for (int i = tid; i < rl[0].O * rl[0].P; i += kThreads)
         mu0[i] = P.layers[0].mu[(size_t)img * rl[0].O * rl[0].P + i];
+      __syncthreads(); // the belief planes are clear before the loop below fills them
+    }
     // errors and gated errors (their borders stay zero); the image shared their memory
     for (int i = tid; i < P.gfloat; i += kThreads)
       sm[P.efloat + i] = 0.0f;

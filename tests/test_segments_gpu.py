@@ -1,6 +1,7 @@
 """Row segments (dpc_resident.cu) and image segments (dpc_conv_resident.cu): whole settling loops in
 one kernel, against the numpy oracle, at the sizes where their splits change.  Bounds: common.TOL per
 tensor, common.ADAM_TOL with an Adam-type optimizer, common.DELTA_TOL on the parameter updates."""
+import numpy as np
 import pytest
 
 from common import (ADAM_TOL, DELTA_TOL, TOL, build_gpu_net, compare_outputs, initial_parameters,
@@ -89,3 +90,24 @@ def test_image_segments_match_oracle(name, built_library):
     case = IMAGES[name]
     assert lib.dpc_conv_images_available(lib.dpcn_conv_plan(build_conv_gpu_net(case)._h)) == 1
     compare_outputs(run_conv_oracle(case), run_conv_gpu(case), TOL, name)
+
+
+def test_closing_segment_starts_from_the_stored_beliefs(built_library):
+    """A segment without the input layer's prediction clears its planes and fills them from memory: the
+    errors it leaves are z - mu of what memory holds, bit for bit, in every one of many runs.  Large
+    planes and a small prediction to copy in between."""
+    from conv_common import make_conv_case
+    from deepity_b200 import _lib
+    lib = _lib.load()
+    case = _images((1, 6, 6), [(1, 3, 3, 1, 1, 1, 1), (40, 3, 3, 1, 1, 2, 2), (40, 3, 3, 1, 1, 1, 1)], "tanh", 296)
+    net = build_conv_gpu_net(case)
+    _, x, y = make_conv_case(case)
+    net.train_step(x, y, 2)
+    plan, ctx = lib.dpcn_conv_plan(net._h), lib.dpcn_conv_context(net._h)
+    assert lib.dpc_conv_images_available(plan) == 1
+    z = [net.get_tensor(l, "z") for l in range(4)]
+    for _ in range(100):
+        _lib.check(lib.dpc_conv_images_segment(plan, 1 << 11 | 1 << 13, 0, 1))  # closing errors, predictions stored
+        _lib.check(lib.dpc_sync(ctx))
+        for l in (1, 2, 3):
+            assert np.array_equal(net.get_tensor(l, "e"), z[l] - net.get_tensor(l - 1, "mu")), l
