@@ -597,6 +597,9 @@ int dpc_plan_invalidate(dpc_plan* p, int first, int count, int what)
     tc_touch(p, 1, first, count);
   if (what & DPC_WROTE_W)
     tc_touch(p, 2, first, count);
+  for (int i = std::max(first, 1); (what & DPC_WROTE_E) && i < first + count; ++i)
+    if (p->h[i - 1].flags & DPC_LAYER_INPUT_ACT)
+      tc_touch(p, 1, i - 1, 1);
   return DPC_OK;
 }
 

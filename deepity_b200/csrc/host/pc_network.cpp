@@ -1707,9 +1707,9 @@ int dpcn_set_tensor(dpcn_net* net, int layer, const char* name, const float* hos
   }
   dpc_ctx* ctx = net->net->Context();
   const std::string nm(name);
-  if (nm == "z" || nm == "W" || nm == "fe")
+  if (nm == "z" || nm == "W" || nm == "fe" || nm == "e")
     dpc_plan_invalidate(net->net->Plan(), layer, 1,
-                        nm == "z" ? DPC_WROTE_Z : (nm == "W" ? DPC_WROTE_W : DPC_WROTE_FE));
+                        nm == "z" ? DPC_WROTE_Z : nm == "W" ? DPC_WROTE_W : nm == "fe" ? DPC_WROTE_FE : DPC_WROTE_E);
   if (st == c)
     return dpc_copy_h2d_sync(ctx, p, host_in, r * c * sizeof(float));
   std::vector<float> tmp(r * st, 0.0f);

@@ -228,7 +228,8 @@ DPC_API int dpc_plan_tensor_run(dpc_plan* plan, int* first, int* count);
  * (src/backend/cuda/CUDABackendGemm.cu:435-445).  Truncated to buf_bytes. */
 DPC_API int dpc_plan_describe(dpc_plan* plan, char* buf, int buf_bytes);
 /* The tensor-core kernels of an SGD network in FP32 mode read bf16 "hi"/"mid" operand copies of
- * z, fe and W of the run's layers, which every kernel of this library keeps up to date.  A
+ * z, fe and W of the run's layers (SimplePC layers: of f(z), of the error e of the layer above and of
+ * W), which every kernel of this library keeps up to date.  A
  * caller that writes one of these tensors ITSELF through a device pointer (dpcn_tensor_ptr, a
  * memcpy, an NCCL receive into z of a boundary layer) must say so before the next phase call;
  * the copies of those layers are then rebuilt on next use.  what: bit set of DPC_WROTE_*.
@@ -239,7 +240,8 @@ enum
 {
   DPC_WROTE_Z = 1,
   DPC_WROTE_FE = 2,
-  DPC_WROTE_W = 4
+  DPC_WROTE_W = 4,
+  DPC_WROTE_E = 8 /* errors: SimplePC layers in the run keep a copy of the error of the layer above */
 };
 DPC_API int dpc_plan_invalidate(dpc_plan* plan, int first, int count, int what);
 DPC_API int dpc_plan_sync_operands(dpc_plan* plan);

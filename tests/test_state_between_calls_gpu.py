@@ -1,0 +1,49 @@
+"""What a caller writes into or reads out of a network between two calls, on the kernels that keep copies of
+the state, against the CUDA-core kernels phase by phase, which keep none, or the numpy oracle.  Bounds:
+common.TOL per tensor."""
+import numpy as np
+import pytest
+
+from common import TOL, build_gpu_net, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def _simple(sizes, batch, act="tanh"):
+    return dict(kind="simple", sizes=sizes, batch=batch, T=3, steps=1, options={},
+                hyper=dict(lr=0.01, ir=0.1, lmbda=0.0, act=act))
+
+
+RUN = _simple([64, 256, 256, 256, 10], 256)  # SimplePC layers on operand planes
+ROWS = _simple([37, 70, 33, 10], 20)         # row segments
+
+
+@pytest.fixture
+def plan_of(built_library, monkeypatch):
+    """Builds a network with its kernels' copies, or ("plain") without any."""
+    from deepity_b200 import _lib
+    lib = _lib.load()
+    monkeypatch.setenv("DPC_RECTANGULAR_MIN_WORK", "0")
+
+    def build(case, plain=False, precision="fp32"):
+        for name in ("DPC_DISABLE_TENSOR_CORES", "DPC_DISABLE_RESIDENT"):
+            monkeypatch.setenv(name, "1") if plain else monkeypatch.delenv(name, raising=False)
+        net, x, y = build_gpu_net(case, precision)
+        return lib, net, lib.dpcn_plan(net._h), x, y
+    return build
+
+
+def test_written_errors_of_simple_layers_are_used(plan_of):
+    """The state update and the weight update read the errors a caller has set."""
+    rng = np.random.default_rng(5)
+    errors = {l: rng.normal(size=(256, 256)).astype(np.float32) for l in (1, 2, 3)}
+    got = []
+    for plain in (False, True):
+        lib, net, plan, x, y = plan_of(RUN, plain)
+        net.train_step_native(x, y, 3)
+        for l, e in errors.items():
+            net.set_tensor(l, "e", e)
+        assert lib.dpc_update_state(plan, 1, 2) == 0 and lib.dpc_update_weights(plan, 0, 4, 0) == 0
+        got.append({(l, n): net.get_tensor(l, n) for l in (1, 2) for n in ("z", "W")})
+    for key, ref in got[1].items():
+        assert rel_err(ref, got[0][key]) <= TOL, key
