@@ -50,6 +50,8 @@ SIGNATURES = {
     "dpc_plan_describe": (_i, [_vp, _cp, _i]),
     "dpc_plan_invalidate": (_i, [_vp, _i, _i, _i]),
     "dpc_plan_sync_operands": (_i, [_vp]),
+    "dpc_plan_sync_operands_of": (_i, [_vp, _i]),
+    "dpc_plan_sync_input_activations": (_i, [_vp, _i, _i]),
     "dpc_plan_set_wait_limit": (_i, [_vp, ctypes.c_double, _i]),
     "dpc_forward": (_i, [_vp, _i, _i, _i]),
     "dpc_project_forward": (_i, [_vp, _i, _i, _i]),

@@ -520,6 +520,11 @@ int dpc_plan_update(dpc_plan* p, const dpc_layer* layers, int n_layers)
                              p->ctx->stream));
     return DPC_OK;
   }
+  // f(z) of SimplePC layers, as last fed to the products, survives in zF
+  for (int i = 0; i < n_layers; ++i)
+    if (layers[i].zF && layers[i].zF == p->h[i].zF && layers[i].size == p->h[i].size &&
+        (rc = tc_zf_need(p, i, 1)) != DPC_OK)
+      return rc;
   DPC_CUDA(cudaStreamSynchronize(p->ctx->stream));
   if (p->e_terminal == p->h[p->n - 1].e)
     p->e_terminal = layers[n_layers - 1].e;
@@ -597,6 +602,10 @@ int dpc_plan_invalidate(dpc_plan* p, int first, int count, int what)
     tc_touch(p, 1, first, count);
   if (what & DPC_WROTE_W)
     tc_touch(p, 2, first, count);
+  if (what & DPC_WROTE_ZF)
+    tc_zf_written(p, first, count);
+  if (what & DPC_REPLAYED)
+    tc_replayed(p);
   for (int i = std::max(first, 1); (what & DPC_WROTE_E) && i < first + count; ++i)
     if (p->h[i - 1].flags & DPC_LAYER_INPUT_ACT)
       tc_touch(p, 1, i - 1, 1);
@@ -605,9 +614,20 @@ int dpc_plan_invalidate(dpc_plan* p, int first, int count, int what)
 
 int dpc_plan_sync_operands(dpc_plan* p)
 {
+  return dpc_plan_sync_operands_of(p, DPC_WROTE_Z | DPC_WROTE_FE | DPC_WROTE_W);
+}
+
+int dpc_plan_sync_operands_of(dpc_plan* p, int what)
+{
   if (!p)
     return fail(DPC_ERR_INVALID, "null plan");
-  return tc_sync_planes(p);
+  return tc_sync_planes(p, what);
+}
+
+int dpc_plan_sync_input_activations(dpc_plan* p, int first, int count)
+{
+  const int rc = check_range(p, first, count);
+  return rc == DPC_OK ? tc_zf_need(p, first, count) : rc;
 }
 
 int dpc_plan_set_wait_limit(dpc_plan* p, double milliseconds, int sweep_target_bias)
@@ -706,6 +726,8 @@ static int forward_simt(dpc_plan* p, int first, int count, int flags)
       return rc;
   }
   const bool simple = (p->h[first].flags & DPC_LAYER_INPUT_ACT) != 0;
+  if (simple && !(flags & DPC_FWD_CACHED))
+    tc_zf_written(p, first, count);
   if ((flags & DPC_FWD_FE) || (simple && (flags & DPC_FWD_ERR_NEXT)))
     wrote(p, K_FE, first, count);
   if (flags & DPC_FWD_COPY_NEXT)
@@ -1102,6 +1124,9 @@ static int weight_gemm_simt(dpc_plan* p, int first, int count, int mode, int fla
 {
   if (!(mode & WG_GRAD_ONLY))
     wrote(p, K_W, first, count);
+  const int ready = tc_zf_need(p, first, count); // (the operand of SimplePC layers)
+  if (ready != DPC_OK)
+    return ready;
   for (int f = first; f < first + count; f += kMaxZ)
   {
     const int c = std::min(kMaxZ, first + count - f);

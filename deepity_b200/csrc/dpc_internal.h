@@ -105,7 +105,13 @@ void tc_fe_planes(dpc_plan* plan, void** base, int* run_first, int* run_count, l
                   int* only);
 void tc_fe_written(dpc_plan* plan, int first, int count);
 int tc_fe_need(dpc_plan* plan, int first, int count);
-int tc_sync_planes(dpc_plan* plan);
+int tc_sync_planes(dpc_plan* plan, int what); // DPC_WROTE_* bits
+// SimplePC layers of the run: f(z) as last fed to the products lives in the belief planes or in zF.
+// tc_zf_need: bring zF of these layers up to date; tc_zf_written: it was written (the planes are
+// behind); tc_replayed: a recorded step left it in the planes.
+int tc_zf_need(dpc_plan* plan, int first, int count);
+void tc_zf_written(dpc_plan* plan, int first, int count);
+void tc_replayed(dpc_plan* plan);
 // Limit of every bounded device-side wait in clock cycles (<= 0: the default, ~2 s) and a bias
 // on the forward sweep's publication target (test hook: a target nothing reaches).
 void tc_set_wait_limit(dpc_plan* plan, long long cycles, int chain_target_bias);

@@ -73,6 +73,14 @@ enum
   FBP_FEED = 2    // SimplePC: f(z), the operand of the pass that follows
 };
 
+// f(z) of a SimplePC layer as last fed to the products
+enum
+{
+  FED_ZF = 0,     // in zF, the belief planes are behind
+  FED_PLANES = 1, // in the belief planes, zF is behind
+  FED_BOTH = 2
+};
+
 struct TcState
 {
   bool ok = false;
@@ -100,6 +108,7 @@ struct TcState
   std::vector<uint8_t> dirty[3];
   bool planes = false;
   bool simple = false; // the run's layers are SimplePC layers (planes only)
+  std::vector<uint8_t> fed; // ... FED_*: where each layer's f(z), as last fed to the products, is
   // The run's feedback errors exist only as planes: every reader of them is a kernel that takes
   // the planes (feedback and weight-shaped products of this file, the bias column sums).
   bool fe_only = false;
@@ -119,9 +128,12 @@ struct TcState
 };
 enum
 {
-  PL_Z = 0,
-  PL_FE = 1,
-  PL_W = 2
+  PL_Z = 0, // (SimplePC: f(z))
+  PL_FE = 1, // (SimplePC: the error of the layer above)
+  PL_W = 2,
+  // for split_layers, SimplePC: belief planes from zF and back
+  PL_ZF = 3,
+  PL_JOIN = 4
 };
 
 struct TcParams
@@ -1809,14 +1821,25 @@ bool make_store_map(CUtensorMap* map, const void* base, bool bf16, int cols, int
   return r == CUDA_SUCCESS;
 }
 
+// zF = hi + mid of the belief planes of layers [first, first + gridDim.y), for whoever reads zF.
+__global__ void join_planes_kernel(const dpc_layer* __restrict__ layers, int first, int run_first,
+                                   const __nv_bfloat16* base, long long elems)
+{
+  const dpc_layer& L = layers[first + blockIdx.y];
+  const __nv_bfloat16* hi = base + 2 * (long long)(first + (int)blockIdx.y - run_first) * elems;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < elems;
+       i += (long long)gridDim.x * blockDim.x)
+    L.zF[i] = __bfloat162float(hi[i]) + __bfloat162float(hi[elems + i]);
+}
+
 // Re-splits the operand planes of `kind` for layers [first, first + gridDim.y) from the fp32
-// tensors (after something other than a kernel of this file wrote them).
+// tensors (after something other than a kernel of this file wrote them); PL_ZF: the belief planes from zF.
 __global__ void split_planes_kernel(const dpc_layer* __restrict__ layers, int first, int run_first,
                                     int kind, __nv_bfloat16* base, long long elems)
 {
   const dpc_layer& L = layers[first + blockIdx.y];
   const bool simple = (L.flags & DPC_LAYER_INPUT_ACT) != 0;
-  const float* src = kind == PL_Z ? L.z : kind == PL_W ? L.W : simple ? (&L)[1].e : L.fe;
+  const float* src = kind == PL_Z ? L.z : kind == PL_W ? L.W : kind == PL_ZF ? L.zF : simple ? (&L)[1].e : L.fe;
   __nv_bfloat16* hi = base + 2 * (long long)(first + (int)blockIdx.y - run_first) * elems;
   for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8; i < elems;
        i += (long long)gridDim.x * blockDim.x * 8)
@@ -1938,8 +1961,7 @@ static bool planes_init(dpc_plan* plan, TcState* st, int first, int count, int H
   st->planes = true;
   if (st->simple)
   {
-    // (a weight update before any forward pass multiplies f(z) = 0, as the zeroed fp32 tensor would)
-    cudaMemset(st->zp, 0, 2 * (size_t)(count + 1) * act * sizeof(__nv_bfloat16));
+    st->fed.assign(count, FED_ZF);
     st->fe_only = true;
     return true;
   }
@@ -2002,7 +2024,7 @@ int tc_plan_init(dpc_plan* plan)
     const bool simple = (L0.flags & DPC_LAYER_INPUT_ACT) != 0;
     const float* out0 = simple ? plan->h[i + 1].e : L0.fe;
     const bool ok0 = L0.next_size == L0.size && L0.size % 256 == 0 && L0.size >= 256 && out0 &&
-                     (simple ? simple_ok : L0.preact != nullptr) &&
+                     (simple ? simple_ok && L0.zF && (uintptr_t)L0.zF % 16 == 0 : L0.preact != nullptr) &&
                      ((uintptr_t)L0.z % 128 == 0) && ((uintptr_t)L0.W % 128 == 0) &&
                      ((uintptr_t)out0 % 128 == 0);
     if (!ok0)
@@ -2017,6 +2039,8 @@ int tc_plan_init(dpc_plan* plan)
       const dpc_layer& Lj = plan->h[j];
       const dpc_layer& Lp = plan->h[j - 1];
       if (Lj.size != L0.size || Lj.next_size != L0.size || ((Lj.flags ^ L0.flags) & DPC_LAYER_INPUT_ACT))
+        break;
+      if (simple && (!Lj.zF || (uintptr_t)Lj.zF % 16 != 0))
         break;
       const int64_t dz = Lj.z - Lp.z, dw = Lj.W - Lp.W,
                     df = simple ? plan->h[j + 1].e - Lj.e : Lj.fe - Lp.fe;
@@ -2257,6 +2281,23 @@ static void planes_mark(TcState* st, int kind, int r0, int r1, uint8_t v)
     d[i] = v;
 }
 
+// One split (or PL_JOIN) launch over layers [i, j) of the run.
+static int split_layers(dpc_plan* p, TcState* st, int kind, int i, int j)
+{
+  const long long H = p->run.width;
+  const long long elems = kind == PL_W ? H * H : (long long)p->batch * H;
+  __nv_bfloat16* base = kind == PL_FE ? st->fep : kind == PL_W ? st->wp : st->zp;
+  dim3 grid((unsigned)std::min<long long>((elems / 8 + 255) / 256, 1024), (unsigned)(j - i));
+  if (kind == PL_JOIN)
+    join_planes_kernel<<<grid, 256, 0, p->ctx->stream>>>(p->d, p->run.first + i, p->run.first, base, elems);
+  else
+    split_planes_kernel<<<grid, 256, 0, p->ctx->stream>>>(p->d, p->run.first + i, p->run.first, kind, base, elems);
+  p->ctx->launches += 1;
+  if (cudaPeekAtLastError() != cudaSuccess)
+    return cuda_fail(cudaGetLastError(), "split_planes kernel launch");
+  return DPC_OK;
+}
+
 // Brings the planes of layers [r0, r1) up to date (one split launch per maximal stale sub-range).
 static int planes_need(dpc_plan* p, TcState* st, int kind, int r0, int r1)
 {
@@ -2265,9 +2306,6 @@ static int planes_need(dpc_plan* p, TcState* st, int kind, int r0, int r1)
   auto& d = st->dirty[kind];
   r0 = std::max(r0, 0);
   r1 = std::min(r1, (int)d.size());
-  const long long H = p->run.width;
-  const long long elems = kind == PL_W ? H * H : (long long)p->batch * H;
-  __nv_bfloat16* base = kind == PL_Z ? st->zp : (kind == PL_FE ? st->fep : st->wp);
   int i = r0;
   while (i < r1)
   {
@@ -2279,16 +2317,41 @@ static int planes_need(dpc_plan* p, TcState* st, int kind, int r0, int r1)
     int j = i;
     while (j < r1 && d[j] && j - i < 32768)
       ++j;
-    dim3 grid((unsigned)std::min<long long>((elems / 8 + 255) / 256, 1024), (unsigned)(j - i));
-    split_planes_kernel<<<grid, 256, 0, p->ctx->stream>>>(p->d, p->run.first + i, p->run.first,
-                                                          kind, base, elems);
-    p->ctx->launches += 1;
-    cudaError_t e = cudaPeekAtLastError();
-    if (e != cudaSuccess)
-      return cuda_fail(cudaGetLastError(), "split_planes kernel launch");
+    const int rc = split_layers(p, st, kind, i, j);
+    if (rc != DPC_OK)
+      return rc;
     for (int k = i; k < j; ++k)
       d[k] = 0;
     i = j;
+  }
+  return DPC_OK;
+}
+
+// f(z) as last fed of the run's SimplePC layers [r0, r1), into the planes or into zF.
+static int fed_need(dpc_plan* p, TcState* st, int r0, int r1, bool planes)
+{
+  r0 = std::max(r0, 0);
+  r1 = std::min(r1, (int)st->fed.size());
+  const uint8_t behind = planes ? FED_ZF : FED_PLANES;
+  for (int i = r0, j; i < r1; i = j)
+  {
+    for (j = i; j < r1 && st->fed[j] == behind && j - i < 32768; ++j)
+    {
+    }
+    if (j == i)
+    {
+      ++j;
+      continue;
+    }
+    const int rc = split_layers(p, st, planes ? PL_ZF : PL_JOIN, i, j);
+    if (rc != DPC_OK)
+      return rc;
+    for (int k = i; k < j; ++k)
+    {
+      st->fed[k] = FED_BOTH;
+      if (planes)
+        st->dirty[PL_Z][k] = 1; // (they may have held f of the present beliefs)
+    }
   }
   return DPC_OK;
 }
@@ -2435,6 +2498,8 @@ int tc_forward(dpc_plan* p, int first, int count, int flags)
   {
     // every variant's epilogue keeps the planes of what it writes (when the plan has planes)
     const uint8_t stale = planes_kept(p, st) ? 0 : 1;
+    for (int k = r0; st->simple && k < r0 + count; ++k)
+      st->fed[k] = FED_PLANES;
     if (flags & DPC_FWD_FE)
       planes_mark(st, PL_FE, r0, r0 + count, stale);
     if (flags & DPC_FWD_COPY_NEXT)
@@ -2574,6 +2639,8 @@ int tc_update_state(dpc_plan* p, int first, int count, bool feed, bool first_fro
   }
   if (rc == DPC_OK)
     planes_mark(st, PL_Z, r0, r0 + count, planes_kept(p, st) && (!st->simple || feed) ? 0 : 1);
+  for (int k = r0; rc == DPC_OK && st->simple && feed && k < r0 + count; ++k)
+    st->fed[k] = FED_PLANES;
   return rc;
 }
 
@@ -2596,7 +2663,7 @@ int tc_weight_gemm(dpc_plan* p, int first, int count, int mode, int decay_w)
       eligible = false;
     if (!eligible)
     {
-      if (fe_only_now(p, st))
+      if (fe_only_now(p, st) && !st->simple) // (SimplePC: the error stays in fp32 too)
         return fail(DPC_ERR_STATE, "weight-shaped product of a tensor-core layer is not eligible "
                                    "for the tensor-core kernel, and the fp32 feedback errors the "
                                    "CUDA-core kernel would read are not kept (DPC_KEEP_FE_FP32=1 "
@@ -2618,7 +2685,7 @@ int tc_weight_gemm(dpc_plan* p, int first, int count, int mode, int decay_w)
     {
       // (SimplePC: f(z) as last fed to the forward product, not of the beliefs as they are now)
       if ((rc = planes_need(p, st, PL_FE, r0, r0 + count)) != DPC_OK ||
-          (!st->simple && (rc = planes_need(p, st, PL_Z, r0, r0 + count)) != DPC_OK))
+          (rc = st->simple ? fed_need(p, st, r0, r0 + count, true) : planes_need(p, st, PL_Z, r0, r0 + count)) != DPC_OK)
         return rc;
       // in-place SGD updates take the weight tile through shared memory and write it and its
       // planes back with bulk stores
@@ -2689,18 +2756,56 @@ int tc_fe_need(dpc_plan* p, int first, int count)
   return planes_need(p, st, PL_FE, first - p->run.first, first + count - p->run.first);
 }
 
-int tc_sync_planes(dpc_plan* p)
+int tc_sync_planes(dpc_plan* p, int what)
 {
   auto* st = static_cast<TcState*>(p->tc);
   if (!st || !st->planes || !planes_on(p, st))
     return DPC_OK;
+  int rc;
+  const int n = (int)st->fed.size();
+  for (int k = 0; st->simple && (what & DPC_WROTE_Z) && k < n; ++k)
+    if (st->dirty[PL_Z][k])
+    {
+      // the planes become f of the present beliefs: what was last fed moves to zF
+      if ((rc = fed_need(p, st, k, k + 1, false)) != DPC_OK)
+        return rc;
+      st->fed[k] = FED_ZF;
+    }
+  if (st->simple && !(what & DPC_WROTE_Z) && (rc = fed_need(p, st, 0, n, true)) != DPC_OK)
+    return rc;
+  const int bits[3] = {DPC_WROTE_Z, DPC_WROTE_FE, DPC_WROTE_W}; // in the order of PL_*
   for (int kind = 0; kind < 3; ++kind)
-  {
-    int rc = planes_need(p, st, kind, 0, (int)st->dirty[kind].size());
-    if (rc != DPC_OK)
+    if ((what & bits[kind]) && (rc = planes_need(p, st, kind, 0, (int)st->dirty[kind].size())) != DPC_OK)
       return rc;
-  }
   return DPC_OK;
+}
+
+int tc_zf_need(dpc_plan* p, int first, int count)
+{
+  auto* st = static_cast<TcState*>(p->tc);
+  if (!st || !st->simple)
+    return DPC_OK;
+  return fed_need(p, st, first - p->run.first, first + count - p->run.first, false);
+}
+
+void tc_zf_written(dpc_plan* p, int first, int count)
+{
+  auto* st = static_cast<TcState*>(p->tc);
+  const int n = st && st->simple ? (int)st->fed.size() : 0;
+  for (int k = std::max(first - p->run.first, 0); k < std::min(first + count - p->run.first, n); ++k)
+    st->fed[k] = FED_ZF;
+}
+
+void tc_replayed(dpc_plan* p)
+{
+  auto* st = static_cast<TcState*>(p->tc);
+  if (!st || !st->simple)
+    return;
+  st->fed.assign(st->fed.size(), FED_PLANES);
+  // (the error under a softmax head is the work of a kernel that does not keep the planes)
+  const int top = p->run.first + p->run.count;
+  if (top < p->n && (p->h[top].flags & DPC_LAYER_SOFTMAX_CE))
+    planes_mark(st, PL_FE, p->run.count - 1, p->run.count, 1);
 }
 
 // ---- single layers outside the run (TcState::Extra) --------------------------------------------

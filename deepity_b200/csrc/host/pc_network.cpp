@@ -393,6 +393,25 @@ void PCNetwork::SyncPlan()
   dirty = ratesDirty = false;
 }
 
+// A recorded step holds no host logic: whatever operand copies are stale now are rebuilt before the graph
+// runs, so that recording and every replay start from the same state.  The operand f(z) of SimplePC
+// layers is what was last fed until the step's first forward pass, which is recorded with its split (the
+// beliefs of such a step always start from a reset).
+void PCNetwork::SyncOperands()
+{
+  if (kind == NetworkKind::SIMPLE)
+    Check(dpc_plan_sync_operands_of(plan, DPC_WROTE_FE | DPC_WROTE_W));
+  else
+    Check(dpc_plan_sync_operands(plan));
+}
+
+// (a replay runs no host code: the operand f(z) may be one state update behind the beliefs)
+void PCNetwork::StepDone(bool replayed)
+{
+  if (kind == NetworkKind::SIMPLE)
+    Check(dpc_plan_invalidate(plan, 0, (int)layers.size(), DPC_WROTE_Z | (replayed ? DPC_REPLAYED : 0)));
+}
+
 void PCNetwork::RandomizeWeights(std::mt19937& rng, const char* distribution)
 {
   RequireCompiled();
@@ -1006,9 +1025,7 @@ float PCNetwork::TrainStepRaw(int mode, const float* x, size_t nx, const float* 
   }
   for (int i = 1; i + 1 < n; ++i)
     layers[i]->clamped = false;
-  // A recorded step holds no host logic: whatever operand copies are stale now are rebuilt
-  // before the graph runs, so that recording and every replay start from the same state.
-  Check(dpc_plan_sync_operands(plan));
+  SyncOperands();
 
   if (useGraph && !gradSync)
   {
@@ -1042,9 +1059,7 @@ float PCNetwork::TrainStepRaw(int mode, const float* x, size_t nx, const float* 
   // (same condition as the TransientScope of RunTrainPhases; a graph replay runs no host code)
   predictionsStale = segments ? kind != NetworkKind::SIMPLE && !(layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE)
                               : kind != NetworkKind::SIMPLE && PredictionsTransient();
-  // (a replay runs no host code: the operand f(z) may be one state update behind the beliefs)
-  if (kind == NetworkKind::SIMPLE)
-    Check(dpc_plan_invalidate(plan, 0, n, DPC_WROTE_Z));
+  StepDone(useGraph && !gradSync);
 
   double energy = 0.0;
   if (readEnergy)
@@ -1112,7 +1127,7 @@ void PCNetwork::PredictRaw(const float* x, size_t nx, int steps, bool withProjec
   ClampHost(0, x, nx);
   for (int i = 1; i < n; ++i)
     layers[i]->clamped = false;
-  Check(dpc_plan_sync_operands(plan));
+  SyncOperands();
   if (useGraph)
   {
     const long key = (long)steps * 2 + (withProjection ? 1 : 0);
@@ -1140,8 +1155,7 @@ void PCNetwork::PredictRaw(const float* x, size_t nx, int steps, bool withProjec
   }
   else
     RunPredictPhases(steps, withProjection);
-  if (kind == NetworkKind::SIMPLE)
-    Check(dpc_plan_invalidate(plan, 0, n, DPC_WROTE_Z));
+  StepDone(useGraph);
   Check(dpc_copy_d2h_sync(ctx, pinnedOut, layers.back()->d.z, count * sizeof(float)));
   std::memcpy(out, pinnedOut, count * sizeof(float));
 }
@@ -1377,7 +1391,11 @@ bool PCNetwork::FindTensor(int layer, const std::string& name, float** ptr, size
   else if (name == "v")
     p = d.v, r = B, c = s;
   else if (name == "zF")
+  {
+    if (d.zF && (dpc_plan_sync_input_activations(plan, layer, 1) != DPC_OK || dpc_sync(ctx) != DPC_OK))
+      return false;
     p = d.zF, r = B, c = s;
+  }
   else if (name == "adj")
     p = d.adj, r = B, c = s;
   else if (name == "Psi" && n == 0 && d.Psi)
@@ -1707,9 +1725,10 @@ int dpcn_set_tensor(dpcn_net* net, int layer, const char* name, const float* hos
   }
   dpc_ctx* ctx = net->net->Context();
   const std::string nm(name);
-  if (nm == "z" || nm == "W" || nm == "fe" || nm == "e")
+  if (nm == "z" || nm == "W" || nm == "fe" || nm == "e" || nm == "zF")
     dpc_plan_invalidate(net->net->Plan(), layer, 1,
-                        nm == "z" ? DPC_WROTE_Z : nm == "W" ? DPC_WROTE_W : nm == "fe" ? DPC_WROTE_FE : DPC_WROTE_E);
+                        nm == "z" ? DPC_WROTE_Z : nm == "W" ? DPC_WROTE_W : nm == "fe" ? DPC_WROTE_FE
+                        : nm == "e" ? DPC_WROTE_E : DPC_WROTE_ZF);
   if (st == c)
     return dpc_copy_h2d_sync(ctx, p, host_in, r * c * sizeof(float));
   std::vector<float> tmp(r * st, 0.0f);

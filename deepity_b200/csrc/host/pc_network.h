@@ -209,6 +209,8 @@ private:
   void Dirty(); // hyper-parameters changed: re-upload the plan, drop captured graphs
   void RatesChanged(); // only learning / inference / feedback rates: re-upload the plan's table
   void SyncPlan();
+  void SyncOperands();
+  void StepDone(bool replayed);
   void EnsureOptimizerState();
   void EnsureGradientStaging();
   void RefreshPredictions();

@@ -191,7 +191,7 @@ typedef struct dpc_layer
   float *W, *b;
   float *preact, *mu, *fe;
   float* Psi;
-  float* zF; /* DPC_LAYER_INPUT_ACT only: f(z) as last fed to the GEMM */
+  float* zF; /* DPC_LAYER_INPUT_ACT only: f(z) as last fed to the GEMM (see dpc_plan_sync_input_activations) */
   float* v;  /* state momentum or NULL */
   float* adj; /* ePC adjoint [B,size] or NULL (FullPCLayer::ComputeAdjoint) */
   float *m_W, *v_W, *m_b, *v_b, *m_Psi, *v_Psi; /* Adam moments or NULL */
@@ -241,10 +241,19 @@ enum
   DPC_WROTE_Z = 1,
   DPC_WROTE_FE = 2,
   DPC_WROTE_W = 4,
-  DPC_WROTE_E = 8 /* errors: SimplePC layers in the run keep a copy of the error of the layer above */
+  DPC_WROTE_E = 8, /* errors: SimplePC layers in the run keep a copy of the error of the layer above */
+  DPC_WROTE_ZF = 16, /* zF */
+  DPC_REPLAYED = 32 /* a recorded step ran (no host code tells the plan what its kernels wrote) */
 };
 DPC_API int dpc_plan_invalidate(dpc_plan* plan, int first, int count, int what);
 DPC_API int dpc_plan_sync_operands(dpc_plan* plan);
+/* ... of the tensors in `what` only.  Without DPC_WROTE_Z the operand f(z) of SimplePC layers stays what
+ * was last fed to the products, for a weight update that comes before the next forward pass. */
+DPC_API int dpc_plan_sync_operands_of(dpc_plan* plan, int what);
+/* SimplePC layers in the run keep f(z) as last fed to the products in their operand copies: this writes
+ * it to zF (16 bits of each value, what the products read) where zF is behind.  Stream-ordered; the
+ * network classes call it when zF is asked for. */
+DPC_API int dpc_plan_sync_input_activations(dpc_plan* plan, int first, int count);
 /* Every device-side wait of the tensor-core kernels (pipeline barriers, the forward sweep's
  * row-block publications) gives up after this long; the kernel then drains, frees its tensor
  * memory and returns, and the next dpc_energy_read reports DPC_ERR_TIMEOUT.  milliseconds <= 0

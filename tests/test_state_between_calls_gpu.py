@@ -4,7 +4,7 @@ common.TOL per tensor."""
 import numpy as np
 import pytest
 
-from common import TOL, build_gpu_net, rel_err
+from common import DELTA_TOL, TOL, build_gpu_net, rel_err, rel_err_of_update
 
 pytestmark = pytest.mark.gpu
 
@@ -47,3 +47,48 @@ def test_written_errors_of_simple_layers_are_used(plan_of):
         got.append({(l, n): net.get_tensor(l, n) for l in (1, 2) for n in ("z", "W")})
     for key, ref in got[1].items():
         assert rel_err(ref, got[0][key]) <= TOL, key
+
+
+CALLS = {"python": lambda n, x, y: n.train_step(x, y, 3), "native": lambda n, x, y: n.train_step_native(x, y, 3),
+         "projection": lambda n, x, y: n.train_step_with_projection(x, y, 3),
+         "predict": lambda n, x, y: n.predict(x, 3)}
+
+
+@pytest.mark.parametrize("call", sorted(CALLS))
+def test_input_activations_read_back_as_last_fed(call, plan_of):
+    """zF, and the weight update of a caller that has written it."""
+    got = []
+    for plain in (False, True):
+        lib, net, plan, x, y = plan_of(RUN, plain)
+        for _ in range(2):
+            CALLS[call](net, x, y)
+        out = {f"zF.{l}": net.get_tensor(l, "zF") for l in range(4)}
+        mine = np.random.default_rng(6).normal(size=(256, 256)).astype(np.float32)
+        net.set_tensor(2, "zF", mine)
+        assert np.array_equal(net.get_tensor(2, "zF"), mine.ravel())
+        assert lib.dpc_update_weights(plan, 0, 4, 0) == 0
+        out.update({f"W.{l}": net.get_tensor(l, "W") for l in range(4)})
+        net.set_optimizer("ADAM")  # another plan, whose kernels read zF
+        lib.dpcn_plan(net._h)
+        out.update({f"kept.{l}": net.get_tensor(l, "zF") for l in range(4)})
+        got.append(out)
+    for key, ref in got[1].items():
+        assert rel_err(ref, got[0][key]) <= TOL, key
+
+
+@pytest.mark.parametrize("graph", [True, False])
+def test_a_step_without_settling_learns_from_what_was_last_fed(graph, plan_of):
+    """Mode 2 without a settling step is a weight update alone (train_step_python of the oracle)."""
+    from common import _oracle_kwargs, make_case, make_oracle
+    params, x, y = make_case("simple", RUN["sizes"], RUN["batch"])
+    orc = make_oracle("simple", RUN["sizes"], RUN["batch"], params, **_oracle_kwargs(RUN))
+    _, net, _, _, _ = plan_of(RUN)
+    net.set_use_graph(graph)
+    for T in (3, 0, 0, 2, 0):
+        orc.train_step_python(x, y, T)
+        net.train_step(x, y, T)
+    for l, p in enumerate(params):
+        for name in ("W", "b"):
+            update = np.asarray(orc.get(l, name)).reshape(p[name].shape) - p[name]
+            assert rel_err_of_update(orc.get(l, name), net.get_tensor(l, name), p[name]) <= DELTA_TOL, (l, name)
+            assert np.abs(update).max() > 0
