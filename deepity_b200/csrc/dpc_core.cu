@@ -872,7 +872,7 @@ int dpc_plan_fused_cross_entropy(dpc_plan* p)
 
 int dpc_plan_state_from_prediction(dpc_plan* p)
 {
-  return p && p->run.count > 0 && p->run.first <= 1 && p->run.first + p->run.count > 1 && p->h[0].mu &&
+  return p && tc_run_ready(p) && p->run.first <= 1 && p->run.first + p->run.count > 1 && p->h[0].mu &&
                  (uintptr_t)p->h[0].mu % 32 == 0 && !(p->h[1].flags & DPC_LAYER_SOFTMAX_CE)
              ? 1
              : 0;

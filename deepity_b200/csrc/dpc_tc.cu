@@ -125,6 +125,9 @@ struct TcState
     CUtensorMap z_km, w_km128, w_km64, fe_km, w_mn, fe_mn, z_mn;
   };
   std::vector<Extra> extras;
+  // A run of SimplePC layers has no fp32 operand maps: where the planes are off (precision or scheme
+  // changed on a live plan) its layers run one by one like the extras.
+  std::vector<Extra> run_extras;
 };
 enum
 {
@@ -2071,7 +2074,8 @@ int tc_plan_init(dpc_plan* plan)
   if (pair_ok(B, 256) && !getenv("DPC_DISABLE_RECTANGULAR"))
     for (int l = 0; l + 1 < n; ++l)
     {
-      if (best_count > 0 && l >= best_first && l < best_first + best_count)
+      const bool in_run = best_count > 0 && l >= best_first && l < best_first + best_count;
+      if (in_run && !st->simple)
         continue;
       const dpc_layer& L = plan->h[l];
       const bool simple = (L.flags & DPC_LAYER_INPUT_ACT) != 0;
@@ -2101,8 +2105,8 @@ int tc_plan_init(dpc_plan* plan)
       ok &= make_map(&x.w_km64, L.W, s_in, s_out, 1, (int64_t)s_in * s_out, 64, false);
       ok &= make_map(&x.w_mn, L.W, s_in, s_out, 1, (int64_t)s_in * s_out, 32, true);
       if (ok)
-        st->extras.push_back(x);
-      else
+        (in_run ? st->run_extras : st->extras).push_back(x);
+      else if (!in_run)
         fprintf(stderr, "deepity_b200: a tensor map for layer %d was refused: it runs on the "
                         "CUDA-core kernels\n", l);
     }
@@ -2432,6 +2436,28 @@ static TcParams base_params(dpc_plan* p, TcState* st, int first, int count, int 
   return P;
 }
 
+// The layers of a SimplePC run go one by one: `one` of each, or 1 (the CUDA-core kernels take them).
+static bool run_apart(const dpc_plan* p, const TcState* st)
+{
+  return st->simple && !planes_on(p, st);
+}
+template <typename Fn>
+static int one_by_one(const dpc_plan* p, const TcState* st, int first, int count, Fn one)
+{
+  if ((int)st->run_extras.size() != p->run.count)
+    return 1;
+  int rc = DPC_OK;
+  for (int l = first; l < first + count && rc == DPC_OK; ++l)
+    rc = one(l);
+  return rc;
+}
+
+bool tc_run_ready(dpc_plan* p)
+{
+  auto* st = static_cast<TcState*>(p->tc);
+  return st && st->ok && p->run.count > 0 && !(run_apart(p, st) && (int)st->run_extras.size() != p->run.count);
+}
+
 int tc_forward(dpc_plan* p, int first, int count, int flags)
 {
   auto* st = static_cast<TcState*>(p->tc);
@@ -2439,6 +2465,8 @@ int tc_forward(dpc_plan* p, int first, int count, int flags)
     return tc_extra_forward(p, first, flags);
   if (!st || !st->ok || !range_in_run(p, first, count))
     return 1;
+  if (run_apart(p, st))
+    return one_by_one(p, st, first, count, [&](int l) { return tc_extra_forward(p, l, flags); });
   const int H = p->run.width, B = p->batch;
   if (st->simple && (flags & DPC_FWD_ERR_NEXT))
     flags |= DPC_FWD_FE; // the error of the layer above as operand planes
@@ -2590,9 +2618,12 @@ int tc_update_state(dpc_plan* p, int first, int count, bool feed, bool first_fro
 {
   auto* st = static_cast<TcState*>(p->tc);
   if (st && st->ok && count == 1 && !range_in_run(p, first, 1))
-    return tc_extra_update_state(p, first);
+    return tc_extra_update_state(p, first, false);
   if (!st || !st->ok || !range_in_run(p, first, count))
     return 1;
+  if (run_apart(p, st))
+    return one_by_one(p, st, first, count,
+                      [&](int l) { return tc_extra_update_state(p, l, first_from_mu && l == first); });
   const int H = p->run.width, B = p->batch;
   const bool tf32 = p->ctx->precision == DPC_PRECISION_TF32;
   const int scheme = split_scheme(p);
@@ -2661,6 +2692,8 @@ int tc_weight_gemm(dpc_plan* p, int first, int count, int mode, int decay_w)
       eligible = false;
     if ((mode & 1) == WG_DFA_MODE && (i + 1 >= p->n || !p->h[i + 1].Psi))
       eligible = false;
+    if (eligible && i + 1 == first + count && run_apart(p, st))
+      return one_by_one(p, st, first, count, [&](int l) { return tc_extra_weight_gemm(p, l, mode, decay_w); });
     if (!eligible)
     {
       if (fe_only_now(p, st) && !st->simple) // (SimplePC: the error stays in fp32 too)
@@ -2814,16 +2847,17 @@ void tc_replayed(dpc_plan* p)
 // layer coordinate of every load is 0, the epilogue reads the layer above with per-lane loads.
 static const TcState::Extra* find_extra(const TcState* st, int layer)
 {
-  for (const auto& x : st->extras)
-    if (x.layer == layer)
-      return &x;
+  for (const auto* list : {&st->extras, &st->run_extras})
+    for (const auto& x : *list)
+      if (x.layer == layer)
+        return &x;
   return nullptr;
 }
 
 bool tc_extra_layer(dpc_plan* p, int layer)
 {
   auto* st = static_cast<TcState*>(p->tc);
-  return st && st->ok && find_extra(st, layer) != nullptr;
+  return st && st->ok && !range_in_run(p, layer, 1) && find_extra(st, layer) != nullptr;
 }
 
 // A product of few 256 x 256 tiles on single-CTA tiles instead (forward 128 x 64, weights 128 x 128):
@@ -2878,6 +2912,7 @@ int tc_extra_forward(dpc_plan* p, int layer, int flags)
     p->ctx->launches += 1;
     if (cudaPeekAtLastError() != cudaSuccess)
       return cuda_fail(cudaGetLastError(), "input_activation kernel launch");
+    tc_zf_written(p, layer, 1);
   }
   const bool narrow = !tf32 && scheme == 2 && extra_narrow(p, p->batch, L.next_size);
   TcParams P = narrow ? extra_params(p, st, layer, p->batch, L.next_size, L.size, flags, 0, 64, TBM)
@@ -2890,10 +2925,12 @@ int tc_extra_forward(dpc_plan* p, int layer, int flags)
   // the belief it may have written can be the first layer of the run: its planes are stale
   if (rc == DPC_OK && (flags & DPC_FWD_COPY_NEXT))
     tc_touch(p, PL_Z, layer + 1, 1);
+  if (rc == DPC_OK && (flags & DPC_FWD_ERR_NEXT) && range_in_run(p, layer, 1))
+    tc_touch(p, PL_FE, layer, 1);
   return rc;
 }
 
-int tc_extra_update_state(dpc_plan* p, int layer)
+int tc_extra_update_state(dpc_plan* p, int layer, bool from_mu)
 {
   auto* st = static_cast<TcState*>(p->tc);
   const TcState::Extra* x = (st && st->ok) ? find_extra(st, layer) : nullptr;
@@ -2903,6 +2940,9 @@ int tc_extra_update_state(dpc_plan* p, int layer)
   const bool tf32 = p->ctx->precision == DPC_PRECISION_TF32;
   const int scheme = split_scheme(p);
   TcParams P = extra_params(p, st, layer, p->batch, L.size, L.next_size, 0, 0);
+  P.first_from_mu = from_mu ? 1 : 0;
+  if (range_in_run(p, layer, 1))
+    tc_touch(p, PL_Z, layer, 1);
   return tf32 ? launch<TC_FB, 256, 0, 128, true>(p, st, x->fe_km, x->w_mn, P)
        : scheme == 2 ? launch<TC_FB, 256, 2, 128, true>(p, st, x->fe_km, x->w_mn, P)
                      : launch<TC_FB, 256, 1, 128, true>(p, st, x->fe_km, x->w_mn, P);
@@ -2923,6 +2963,11 @@ int tc_extra_weight_gemm(dpc_plan* p, int layer, int mode, int decay_w)
     return 1;
   const bool tf32 = p->ctx->precision == DPC_PRECISION_TF32 || fast_grad(p);
   const int scheme = split_scheme(p);
+  const int ready = tc_zf_need(p, layer, 1);
+  if (ready != DPC_OK)
+    return ready;
+  if (range_in_run(p, layer, 1) && !(mode & WG_GRAD_MODE))
+    tc_touch(p, PL_W, layer, 1);
   const bool narrow = !tf32 && scheme == 2 && extra_narrow(p, L.next_size, L.size);
   TcParams P = narrow ? extra_params(p, st, layer, L.next_size, L.size, p->batch, decay_w ? 1 : 0, mode, 128, TBM)
                       : extra_params(p, st, layer, L.next_size, L.size, p->batch, decay_w ? 1 : 0, mode);
@@ -2976,7 +3021,8 @@ std::string tc_describe(dpc_plan* p)
     out += "layer";
     for (int l = p->run.first; l < p->run.first + p->run.count; ++l)
       out += name(l);
-    out += " on tcgen05 (one launch per phase, CTA pairs 256x256, 3xBF16 from pre-split planes of f(z)); ";
+    out += run_apart(p, st) ? " on tcgen05 (CTA pairs 256x256, one launch per layer); "
+                            : " on tcgen05 (one launch per phase, CTA pairs, 3xBF16 from pre-split planes of f(z)); ";
     on_tc += p->run.count;
   }
   if (!st->extras.empty())

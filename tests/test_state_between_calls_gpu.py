@@ -4,7 +4,7 @@ common.TOL per tensor."""
 import numpy as np
 import pytest
 
-from common import DELTA_TOL, TOL, build_gpu_net, rel_err, rel_err_of_update
+from common import DELTA_TOL, TF32_TOL, TOL, build_gpu_net, rel_err, rel_err_of_update
 
 pytestmark = pytest.mark.gpu
 
@@ -92,3 +92,51 @@ def test_a_step_without_settling_learns_from_what_was_last_fed(graph, plan_of):
             update = np.asarray(orc.get(l, name)).reshape(p[name].shape) - p[name]
             assert rel_err_of_update(orc.get(l, name), net.get_tensor(l, name), p[name]) <= DELTA_TOL, (l, name)
             assert np.abs(update).max() > 0
+
+
+def test_precision_set_on_a_live_plan(plan_of):
+    """dpc_set_precision without a new plan: single-pass TF32 products from the next call on, and back."""
+    _, plain, _, _, _ = plan_of(RUN, plain=True)
+    _, ref, _, x, y = plan_of(RUN, precision="tf32")
+    lib, net, _, _, _ = plan_of(RUN)
+    ctx = lib.dpcn_context(net._h)
+    for n in (ref, net, plain):
+        n.set_use_graph(False)
+    lib.dpcn_plan(net._h)
+    assert lib.dpc_set_precision(ctx, 1) == 0
+    assert net.train_step_native(x, y, 3) == pytest.approx(ref.train_step_native(x, y, 3), rel=1e-6)
+    plain.train_step_native(x, y, 3)
+    for l in range(4):
+        for name in ("z", "e", "W", "b", "zF"):
+            assert rel_err(ref.get_tensor(l, name), net.get_tensor(l, name)) <= 1e-6, (l, name)
+    # the operands of the second step start from the same state on both sides
+    assert lib.dpc_set_precision(ctx, 0) == 0
+    for l in range(4):
+        plain.set_tensor(l, "W", net.get_tensor(l, "W"))
+        plain.set_tensor(l, "b", net.get_tensor(l, "b"))
+    for n in (net, plain):
+        n.train_step(x, y, 0)  # a weight update from the TF32 step's operands
+    for l in range(4):
+        assert rel_err(plain.get_tensor(l, "W"), net.get_tensor(l, "W")) <= TF32_TOL, l
+        plain.set_tensor(l, "W", net.get_tensor(l, "W"))
+        plain.set_tensor(l, "b", net.get_tensor(l, "b"))
+    for n in (net, plain):
+        n.train_step(x, y, 3)
+    for l in range(4):
+        for name in ("z", "e", "W", "b", "zF"):
+            assert rel_err(plain.get_tensor(l, name), net.get_tensor(l, name)) <= TOL, (l, name)
+
+
+def test_split_scheme_changed_on_a_live_plan(plan_of, monkeypatch):
+    """DPC_FP32_SCHEME is read when a phase is launched."""
+    _, plain, _, x, y = plan_of(RUN, plain=True)
+    _, net, _, _, _ = plan_of(RUN)
+    for n in (net, plain):
+        n.set_use_graph(False)
+    for scheme in ("tf32x3", None):
+        monkeypatch.setenv("DPC_FP32_SCHEME", scheme) if scheme else monkeypatch.delenv("DPC_FP32_SCHEME")
+        for n in (net, plain):
+            n.train_step(x, y, 3)
+        for l in range(4):
+            for name in ("z", "e", "W", "b", "zF"):
+                assert rel_err(plain.get_tensor(l, name), net.get_tensor(l, name)) <= TOL, (scheme, l, name)
