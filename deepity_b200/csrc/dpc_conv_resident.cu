@@ -46,6 +46,7 @@ struct RcLayer // per weight layer l; "up" is layer l + 1, the state it predicts
   int goff, gplane, gpix;        // gated errors of this layer's outputs (l = 0: none kept)
   int boff;                      // bias
   int dense;                     // one output pixel, no padding
+  int vec;                       // ... and rows of W that can be read 16 bytes at a time
   int ffirst, fcount;            // forward tasks
 };
 
@@ -406,7 +407,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_resident_kernel(const RcPara
         const float* W = P.layers[l].W + (size_t)t.m0 * K;
         const float* z = sm + L.zoff;
         float s = 0.0f;
-        if (K % 4 == 0)
+        if (L.vec)
         {
 #pragma unroll 4
           for (int k = lane * 4; k < K; k += 128)
@@ -846,6 +847,7 @@ int conv_res_init(dpc_conv_plan* p)
     q.C = L.in_c, q.HW = L.in_h * L.in_w, q.O = L.out_c, q.P = L.out_h * L.out_w;
     weights += sizeof(float) * (size_t)L.out_c * L.in_c * L.k_h * L.k_w;
     q.dense = dense(l);
+    q.vec = (q.C * q.HW) % 4 == 0 && (reinterpret_cast<uintptr_t>(L.W) & 15) == 0;
     if (q.dense && l > 0)
       gpitch[l] = grows[l] = 1;
     if (l > 0)

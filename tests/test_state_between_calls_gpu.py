@@ -1,6 +1,8 @@
 """What a caller writes into or reads out of a network between two calls, on the kernels that keep copies of
 the state, against the CUDA-core kernels phase by phase, which keep none, or the numpy oracle.  Bounds:
 common.TOL per tensor."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -140,3 +142,61 @@ def test_split_scheme_changed_on_a_live_plan(plan_of, monkeypatch):
         for l in range(4):
             for name in ("z", "e", "W", "b", "zF"):
                 assert rel_err(plain.get_tensor(l, name), net.get_tensor(l, name)) <= TOL, (scheme, l, name)
+
+
+class _ConvLayer(ctypes.Structure):  # dpc_conv_layer
+    _fields_ = ([(n, ctypes.c_int32) for n in
+                 "in_c out_c in_h in_w k_h k_w s_h s_w p_h p_w out_h out_w act opt".split()] +
+                [(n, ctypes.c_float) for n in "lr ir lmbda".split()] +
+                [(n, ctypes.c_void_p) for n in "z e W b preact mu g g_W g_b m_W v_W m_b v_b t".split()])
+
+
+@pytest.fixture
+def conv_plan(built_library):
+    """A convolution plan of one weight layer over tensors of the test's own: (lib, plan, tensors, sync)."""
+    import torch
+
+    from deepity_b200 import _lib
+    lib = _lib.load()
+    made = []
+
+    def build(B, C, O, H, k, pad, weight_offset=0):
+        torch.manual_seed(3)
+        P = H + 2 * pad - k + 1
+        flat = torch.randn(O * C * k * k + 4, device="cuda") / k
+        shapes = dict(z=(B, C, H, H), e=(B, C, H, H), b=(O,), preact=(B, O, P, P), mu=(B, O, P, P), g=(B, O, P, P),
+                      g_W=(O, C * k * k), g_b=(O,))
+        t = {n: torch.randn(*s, device="cuda") for n, s in shapes.items()}
+        t["W"] = flat[weight_offset:weight_offset + O * C * k * k].view(O, C * k * k)
+        top = {n: torch.randn(B, O, P, P, device="cuda") for n in ("z", "e")}
+        table = (_ConvLayer * 2)()
+        for n, v in dict(in_c=C, out_c=O, in_h=H, in_w=H, k_h=k, k_w=k, s_h=1, s_w=1, p_h=pad, p_w=pad, out_h=P,
+                         out_w=P, act=8, lr=0.1, ir=0.1).items():
+            setattr(table[0], n, v)
+        for n, v in dict(in_c=O, in_h=P, in_w=P, act=10, lr=0.1, ir=0.1).items():
+            setattr(table[1], n, v)
+        for layer, tensors in zip(table, (t, top)):
+            for n, v in tensors.items():
+                setattr(layer, n, v.data_ptr())
+        torch.cuda.synchronize()
+        ctx, plan = ctypes.c_void_p(), ctypes.c_void_p()
+        _lib.check(lib.dpc_create(0, ctypes.byref(ctx)))
+        _lib.check(lib.dpc_conv_plan_create(ctx, table, 2, B, ctypes.byref(plan)))
+        made.append((plan, ctx, t, top, flat))
+        return lib, plan, t, top, lambda: _lib.check(lib.dpc_sync(ctx))
+    yield build
+    for plan, ctx, *_ in made:
+        lib.dpc_conv_plan_destroy(plan)
+        lib.dpc_destroy(ctx)
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2])
+def test_dense_convolution_weights_of_any_alignment(offset, conv_plan):
+    """The whole image under one kernel, rows of 64 weights that start on any float."""
+    lib, plan, t, top, sync = conv_plan(3, 4, 5, 4, 4, 0, weight_offset=offset)
+    assert lib.dpc_conv_images_available(plan) == 1
+    assert lib.dpc_conv_images_segment(plan, 1 << 0 | 1 << 11 | 1 << 13, 0, 1) == 0  # first, closing errors, predictions
+    sync()
+    pre = t["z"].reshape(3, -1).double() @ t["W"].double().T + t["b"].double()
+    assert rel_err(pre.cpu(), t["preact"].cpu()) <= TOL
+    assert rel_err((top["z"].reshape(3, -1) - pre.tanh()).cpu(), top["e"].cpu()) <= TOL
