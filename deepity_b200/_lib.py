@@ -30,6 +30,7 @@ SIGNATURES = {
     "dpc_zero": (_i, [_vp, _vp, ctypes.c_size_t]),
     "dpc_copy_d2d": (_i, [_vp, _vp, _vp, ctypes.c_size_t]),
     "dpc_copy_h2d": (_i, [_vp, _vp, _vp, ctypes.c_size_t]),
+    "dpc_host_is_pageable": (_i, [_vp]),
     "dpc_copy_d2h": (_i, [_vp, _vp, _vp, ctypes.c_size_t]),
     "dpc_copy_h2d_sync": (_i, [_vp, _vp, _vp, ctypes.c_size_t]),
     "dpc_copy_d2h_sync": (_i, [_vp, _vp, _vp, ctypes.c_size_t]),

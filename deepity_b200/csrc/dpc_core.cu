@@ -275,6 +275,17 @@ int dpc_copy_h2d(dpc_ctx* ctx, void* dst, const void* host_src, size_t bytes)
   return DPC_OK;
 }
 
+int dpc_host_is_pageable(const void* host_ptr)
+{
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, host_ptr) != cudaSuccess)
+  {
+    cudaGetLastError();
+    return 1;
+  }
+  return a.type == cudaMemoryTypeUnregistered ? 1 : 0;
+}
+
 int dpc_copy_d2h(dpc_ctx* ctx, void* host_dst, const void* src, size_t bytes)
 {
   if (!ctx)

@@ -268,9 +268,7 @@ void SimpleConvPCNetwork::ClampRaw(int layer, const float* data, size_t n, bool 
   if (onDevice)
     Check(dpc_copy_d2d(ctx, l->d.z, data, count * sizeof(float)));
   else
-  {
     Check(dpc_copy_h2d(ctx, l->d.z, data, count * sizeof(float))); // (see PCNetwork::ClampHost)
-  }
   l->clamped = true;
   l->cacheValid = false;
 }
@@ -278,6 +276,8 @@ void SimpleConvPCNetwork::ClampRaw(int layer, const float* data, size_t n, bool 
 void SimpleConvPCNetwork::Clamp(const std::vector<float>& input)
 {
   ClampRaw(0, input.data(), input.size(), false);
+  if (!dpc_host_is_pageable(input.data()))
+    Check(dpc_sync(ctx));
 }
 
 // ComputeMuOnly of layer i with whatever the caller wants fused in; a clamped layer computes
@@ -435,6 +435,7 @@ float SimpleConvPCNetwork::TrainStepRaw(const float* x, size_t nx, const float* 
         dpc_graph_end(ctx, 0);
         dpc_graph_drop(ctx, 0);
         graphKey[0] = -1;
+        dpc_sync(ctx); // (the inputs' copies)
         throw;
       }
       Check(dpc_graph_end(ctx, 0));
@@ -516,6 +517,7 @@ void SimpleConvPCNetwork::PredictRaw(const float* x, size_t nx, int steps, bool 
         dpc_graph_end(ctx, 1);
         dpc_graph_drop(ctx, 1);
         graphKey[1] = -1;
+        dpc_sync(ctx); // (the inputs' copies)
         throw;
       }
       Check(dpc_graph_end(ctx, 1));

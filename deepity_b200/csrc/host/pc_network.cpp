@@ -501,11 +501,19 @@ void PCNetwork::ClampHost(int layer, const float* data, size_t n)
   const size_t count = std::min(n, cap);
   // Straight from the caller's memory: the driver's own staging overlaps its copies with the transfer,
   // 59 us for 0.8 MB and 0.63 ms for 12.6 MB where a copy into a pinned buffer and one transfer took 69
-  // and 914.  The call returns when `data` has been read.
+  // and 914.  Pageable `data` has been read when the copy returns, page-locked memory is read later: a
+  // call that ends without waiting for the stream calls WaitForHost.
   Check(dpc_copy_h2d(ctx, l->d.z, data, count * sizeof(float)));
   Check(dpc_plan_invalidate(plan, layer, 1, DPC_WROTE_Z));
   l->clamped = true;
   l->cacheValid = false;
+}
+
+// The caller may write its buffers again when this returns.
+void PCNetwork::WaitForHost(const float* a, const float* b)
+{
+  if (!dpc_host_is_pageable(a) || (b && !dpc_host_is_pageable(b)))
+    Check(dpc_sync(ctx));
 }
 
 void PCNetwork::ClampDevice(int layer, const float* data, size_t n)
@@ -522,6 +530,7 @@ void PCNetwork::ClampDevice(int layer, const float* data, size_t n)
 void PCNetwork::Clamp(const std::vector<float>& input)
 {
   ClampHost(0, input.data(), input.size());
+  WaitForHost(input.data());
 }
 
 // ------------------------------------------------------------------------------ phases
@@ -1022,6 +1031,8 @@ float PCNetwork::TrainStepRaw(int mode, const float* x, size_t nx, const float* 
   {
     ClampHost(0, x, nx);
     ClampHost(n - 1, y, ny);
+    if (!readEnergy)
+      WaitForHost(x, y);
   }
   for (int i = 1; i + 1 < n; ++i)
     layers[i]->clamped = false;
@@ -1042,6 +1053,7 @@ float PCNetwork::TrainStepRaw(int mode, const float* x, size_t nx, const float* 
         dpc_graph_end(ctx, 0);
         dpc_graph_drop(ctx, 0);
         graphKey[0] = -1;
+        dpc_sync(ctx); // (the inputs' copies)
         throw;
       }
       Check(dpc_graph_end(ctx, 0));
@@ -1143,6 +1155,7 @@ void PCNetwork::PredictRaw(const float* x, size_t nx, int steps, bool withProjec
         dpc_graph_end(ctx, 1);
         dpc_graph_drop(ctx, 1);
         graphKey[1] = -1;
+        dpc_sync(ctx); // (the inputs' copies)
         throw;
       }
       Check(dpc_graph_end(ctx, 1));

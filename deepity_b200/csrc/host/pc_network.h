@@ -115,7 +115,7 @@ public:
   // momentum) before it reads one, so clearing them is skipped.
   void ResetState(bool beliefsOverwritten = false, bool settleOverwritten = false);
   void Clamp(const std::vector<float>& input);
-  void ClampHost(int layer, const float* data, size_t n);
+  void ClampHost(int layer, const float* data, size_t n); // page-locked `data` is read in stream order
   void ClampDevice(int layer, const float* data, size_t n);
   void UnclampTerminal() { layers.back()->clamped = false; }
 
@@ -209,6 +209,7 @@ private:
   void Dirty(); // hyper-parameters changed: re-upload the plan, drop captured graphs
   void RatesChanged(); // only learning / inference / feedback rates: re-upload the plan's table
   void SyncPlan();
+  void WaitForHost(const float* a, const float* b = nullptr);
   void SyncOperands();
   void StepDone(bool replayed);
   void EnsureOptimizerState();

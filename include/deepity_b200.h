@@ -136,7 +136,10 @@ DPC_API int dpc_alloc(dpc_ctx* ctx, size_t bytes, void** out);
 DPC_API int dpc_free(dpc_ctx* ctx, void* ptr);
 DPC_API int dpc_zero(dpc_ctx* ctx, void* ptr, size_t bytes);
 DPC_API int dpc_copy_d2d(dpc_ctx* ctx, void* dst, const void* src, size_t bytes);
+/* (from pageable memory dpc_copy_h2d returns when the source has been read; page-locked or managed memory
+ * is read later, in stream order) */
 DPC_API int dpc_copy_h2d(dpc_ctx* ctx, void* dst, const void* host_src, size_t bytes);
+DPC_API int dpc_host_is_pageable(const void* host_ptr);
 DPC_API int dpc_copy_d2h(dpc_ctx* ctx, void* host_dst, const void* src, size_t bytes);
 DPC_API int dpc_copy_h2d_sync(dpc_ctx* ctx, void* dst, const void* host_src, size_t bytes);
 DPC_API int dpc_copy_d2h_sync(dpc_ctx* ctx, void* host_dst, const void* src, size_t bytes);

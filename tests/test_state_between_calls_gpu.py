@@ -200,3 +200,28 @@ def test_dense_convolution_weights_of_any_alignment(offset, conv_plan):
     pre = t["z"].reshape(3, -1).double() @ t["W"].double().T + t["b"].double()
     assert rel_err(pre.cpu(), t["preact"].cpu()) <= TOL
     assert rel_err((top["z"].reshape(3, -1) - pre.tanh()).cpu(), top["e"].cpu()) <= TOL
+
+
+def test_page_locked_inputs_may_be_written_again_after_the_call(built_library):
+    """dpcn_train_step without an energy returns when it has read its host inputs, page-locked or not: here
+    three steps are queued ahead of the copies of the fourth."""
+    import torch
+
+    from deepity_b200 import _lib
+    lib = _lib.load()
+    case = dict(kind="dkp", sizes=[512] * 25 + [10], batch=1024, T=2, steps=1, options={},
+                hyper=dict(lr=1e-3, ir=0.1, fl=1e-3, lmbda=0.0, act="tanh"))
+    got = []
+    for overwrite in (False, True):
+        net, x, y = build_gpu_net(case)
+        xs, ys = torch.from_numpy(x).pin_memory(), torch.from_numpy(y).pin_memory()
+        at = [ctypes.cast(t.data_ptr(), _lib.c_f32p) for t in (xs, ys)]
+        for _ in range(4):
+            _lib.check(lib.dpcn_train_step(net._h, at[0], xs.numel(), at[1], ys.numel(), 2, None))
+        if overwrite:
+            xs.fill_(7.0)
+            ys.zero_()
+        _lib.check(lib.dpc_sync(lib.dpcn_context(net._h)))
+        got.append([net.get_tensor(0, "z"), net.get_tensor(25, "z"), net.get_tensor(24, "W")])
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
