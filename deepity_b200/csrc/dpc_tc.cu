@@ -2386,8 +2386,10 @@ static bool fe_only_now(const dpc_plan* p, const TcState* st)
 // tiles re-read less of A and win where there are many waves.
 static int pair_tile_width(const dpc_plan* p, int tiles256, int narrowest)
 {
-  if (const char* env = getenv("DPC_PAIR_TILE_WIDTH")) // (for comparing the variants)
-    return std::max(atoi(env), narrowest);
+  const char* env = getenv("DPC_PAIR_TILE_WIDTH"); // (for comparing the variants)
+  const int fixed = env ? atoi(env) : 0;
+  if (fixed == 64 || fixed == 128 || fixed == 256)
+    return std::max(fixed, narrowest);
   const int pairs = p->ctx->sm_count / 2;
   int best = 256;
   double best_cost = 1e30;

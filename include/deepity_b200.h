@@ -40,6 +40,7 @@
  *                              on the context's stream instead of side by side on internal streams
  *                              that fork from it and join it again
  *   DPC_PAIR_TILE_WIDTH        64, 128 or 256: one width of the pair tiles of a run instead of the rule
+ *                              (at least 128 for state and weight updates; other values do nothing)
  *   DPC_DISABLE_RESIDENT       small networks run phase by phase instead of in row segments
  */
 #ifndef DEEPITY_B200_H

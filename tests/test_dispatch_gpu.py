@@ -63,6 +63,17 @@ def test_pair_tile_widths_match_oracle(name, precision, width, built_library, mo
     _check(PAIR[name], f"{name} {precision} {width}", precision)
 
 
+@pytest.mark.parametrize("width", ["0", "96", "100", "512"])
+def test_other_pair_tile_widths_do_nothing(width, built_library, monkeypatch):
+    """No other width is launched: the tiles are those of the rule, bit for bit."""
+    plain = run_gpu(PAIR["dkp"])
+    monkeypatch.setenv("DPC_PAIR_TILE_WIDTH", width)
+    got = run_gpu(PAIR["dkp"])
+    for key, ref in plain.items():
+        if key != "energies":
+            assert np.array_equal(ref, got[key]), key
+
+
 # The state update of the layer above the clamped input forms its error itself, except in the last pass:
 # one pass, several, single-CTA tiles (batch 128), 3xTF32 operands (Adam), a run that starts at the input
 FROM_PREDICTION = {
