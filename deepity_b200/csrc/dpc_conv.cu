@@ -534,10 +534,22 @@ __global__ void __launch_bounds__(THREADS)
   }
 }
 
+// Zeroes the sums that the gradient launch adds into.  blockIdx.y = layer.
+__global__ void conv_zero_sums_kernel(const dpc_conv_layer* __restrict__ layers, int first)
+{
+  const dpc_conv_layer& L = layers[first + blockIdx.y];
+  const size_t nW = L.out_c > 0 ? (size_t)L.out_c * L.in_c * L.k_h * L.k_w : 0;
+  const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (size_t o = tid; o < nW; o += (size_t)gridDim.x * blockDim.x)
+    L.g_W[o] = 0.0f;
+  for (int j = (int)tid; j < L.out_c; j += gridDim.x * blockDim.x)
+    L.g_b[j] = 0.0f;
+}
+
 // SGD / Adam / AdamW on W and b from the raw sums in g_W, g_b
 // (src/layers/SimpleConvPCLayer.cpp:424-556: SGD rate lr/B with decay (1-lambda) first;
 // Adam-type gradients are -(1/B) * sum).
-// The sums are zeroed behind the update: the next gradient launch adds into them.  blockIdx.y = layer.
+// blockIdx.y = layer.
 __global__ void conv_apply_kernel(const dpc_conv_layer* __restrict__ layers, int first, int batch)
 {
   const dpc_conv_layer L = layers[first + blockIdx.y];
@@ -557,13 +569,9 @@ __global__ void conv_apply_kernel(const dpc_conv_layer* __restrict__ layers, int
       if (decay != 1.0f)
         w *= decay;
       L.W[o] = fmaf(alpha, L.g_W[o], w);
-      L.g_W[o] = 0.0f;
     }
     for (size_t j = tid; j < (size_t)L.out_c; j += nthr)
-    {
       L.b[j] = fmaf(alpha, L.g_b[j], L.b[j]);
-      L.g_b[j] = 0.0f;
-    }
     return;
   }
   const float step = adam_step_size(L.lr, *L.t + 1); // (the counter itself moves on afterwards)
@@ -573,7 +581,6 @@ __global__ void conv_apply_kernel(const dpc_conv_layer* __restrict__ layers, int
   {
     float m = L.m_W[o], v = L.v_W[o];
     L.W[o] = adam_update(L.W[o], gs * L.g_W[o], m, v, step, lr_wd);
-    L.g_W[o] = 0.0f;
     L.m_W[o] = m;
     L.v_W[o] = v;
   }
@@ -581,7 +588,6 @@ __global__ void conv_apply_kernel(const dpc_conv_layer* __restrict__ layers, int
   {
     float m = L.m_b[j], v = L.v_b[j];
     L.b[j] = adam_update(L.b[j], gs * L.g_b[j], m, v, step, -1.0f);
-    L.g_b[j] = 0.0f;
     L.m_b[j] = m;
     L.v_b[j] = v;
   }
@@ -705,18 +711,12 @@ int validate(const dpc_conv_layer* l, int n)
   return DPC_OK;
 }
 
-// The layer table on the device; the gradient sums start at zero (the update kernel leaves them so).
+// The layer table on the device.
 int upload_layers(dpc_conv_plan* p)
 {
   if (!p->d)
     DPC_CUDA(cudaMalloc(&p->d, sizeof(dpc_conv_layer) * p->n));
   DPC_CUDA(cudaMemcpy(p->d, p->h.data(), sizeof(dpc_conv_layer) * p->n, cudaMemcpyHostToDevice));
-  for (const auto& L : p->h)
-    if (L.out_c > 0)
-    {
-      DPC_CUDA(cudaMemset(L.g_W, 0, sizeof(float) * (size_t)L.out_c * L.in_c * L.k_h * L.k_w));
-      DPC_CUDA(cudaMemset(L.g_b, 0, sizeof(float) * L.out_c));
-    }
   return DPC_OK;
 }
 
@@ -996,6 +996,9 @@ int dpc_conv_update_weights_range(dpc_conv_plan* p, int first, int count, int ce
     }
     if (G.count > 0)
     {
+      conv_zero_sums_kernel<<<dim3(elem_grid(p, max_w), c), THREADS, 0, st>>>(p->d, first);
+      if ((rc = conv_check_launch(p->ctx, "conv zero sums kernel")) != DPC_OK)
+        return rc;
       conv_gradient_kernel<<<blocks, THREADS, 0, st>>>(p->d, G, p->batch);
       if ((rc = conv_check_launch(p->ctx, "conv gradient kernel")) != DPC_OK)
         return rc;

@@ -225,3 +225,20 @@ def test_page_locked_inputs_may_be_written_again_after_the_call(built_library):
         got.append([net.get_tensor(0, "z"), net.get_tensor(25, "z"), net.get_tensor(24, "W")])
     for a, b in zip(*got):
         assert np.array_equal(a, b)
+
+
+def test_convolution_gradient_sums_stay_in_the_callers_buffers(conv_plan):
+    """g_W and g_b are the raw sums of one update whatever they held before it, and hold them after it."""
+    import torch
+    lib, plan, t, top, sync = conv_plan(3, 2, 4, 5, 3, 1)
+    for n in ("g_W", "g_b"):
+        t[n].fill_(7.0)
+    before = {n: t[n].double() for n in ("W", "b")}
+    cols = torch.nn.functional.unfold(t["z"], 3, padding=1).double()
+    dW = torch.einsum("bop,brp->or", t["g"].reshape(3, 4, -1).double(), cols)
+    db = t["g"].double().sum((0, 2, 3))
+    torch.cuda.synchronize()
+    assert lib.dpc_conv_update_weights(plan, 0, 0) == 0
+    sync()
+    for n, ref in (("g_W", dW), ("g_b", db), ("W", before["W"] + 0.1 / 3 * dW), ("b", before["b"] + 0.1 / 3 * db)):
+        assert rel_err(ref.cpu(), t[n].cpu()) <= 1e-5, n  # 75 products of unit size in fp32
