@@ -716,7 +716,8 @@ int upload_layers(dpc_conv_plan* p)
 {
   if (!p->d)
     DPC_CUDA(cudaMalloc(&p->d, sizeof(dpc_conv_layer) * p->n));
-  DPC_CUDA(cudaMemcpy(p->d, p->h.data(), sizeof(dpc_conv_layer) * p->n, cudaMemcpyHostToDevice));
+  DPC_CUDA(cudaMemcpyAsync(p->d, p->h.data(), sizeof(dpc_conv_layer) * p->n, cudaMemcpyHostToDevice,
+                           p->ctx->stream));
   return DPC_OK;
 }
 
@@ -748,7 +749,7 @@ int dpc_conv_plan_create(dpc_ctx* ctx, const dpc_conv_layer* layers, int n_layer
     delete p;
     return cuda_fail(cudaGetLastError(), "conv plan allocation");
   }
-  cudaMemset(p->energy, 0, sizeof(double));
+  cudaMemsetAsync(p->energy, 0, sizeof(double), ctx->stream);
   if ((rc = upload_layers(p)) != DPC_OK)
   {
     dpc_conv_plan_destroy(p);

@@ -1012,7 +1012,7 @@ int conv_res_init(dpc_conv_plan* p)
   p->res = st;
   if (cudaMalloc(&st->dev, host.size()) != cudaSuccess ||
       cudaMalloc(&st->packed, (B.packed + 32 * kDepth) * sizeof(float4)) != cudaSuccess ||
-      cudaMemcpy(st->dev, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+      cudaMemcpyAsync(st->dev, host.data(), host.size(), cudaMemcpyHostToDevice, p->ctx->stream) != cudaSuccess)
   {
     conv_res_free(p);
     return cuda_fail(cudaGetLastError(), "image-resident plan tables");

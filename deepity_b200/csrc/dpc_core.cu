@@ -487,9 +487,9 @@ int dpc_plan_create(dpc_ctx* ctx, const dpc_layer* layers, int n_layers, int bat
   if (err == cudaSuccess)
     err = cudaMallocHost(&p->energy_host, 2 * sizeof(double));
   if (err == cudaSuccess)
-    err = cudaMemcpy(p->d, layers, sizeof(dpc_layer) * n_layers, cudaMemcpyHostToDevice);
+    err = cudaMemcpyAsync(p->d, p->h.data(), sizeof(dpc_layer) * n_layers, cudaMemcpyHostToDevice, ctx->stream);
   if (err == cudaSuccess)
-    err = cudaMemset(p->energy, 0, 2 * sizeof(double));
+    err = cudaMemsetAsync(p->energy, 0, 2 * sizeof(double), ctx->stream);
   if (err != cudaSuccess)
   {
     dpc_plan_destroy(p);
@@ -540,7 +540,8 @@ int dpc_plan_update(dpc_plan* p, const dpc_layer* layers, int n_layers)
   if (p->e_terminal == p->h[p->n - 1].e)
     p->e_terminal = layers[n_layers - 1].e;
   p->h.assign(layers, layers + n_layers);
-  DPC_CUDA(cudaMemcpy(p->d, layers, sizeof(dpc_layer) * n_layers, cudaMemcpyHostToDevice));
+  DPC_CUDA(cudaMemcpyAsync(p->d, p->h.data(), sizeof(dpc_layer) * n_layers, cudaMemcpyHostToDevice,
+                           p->ctx->stream));
   tc_plan_free(p);
   res_plan_free(p);
   p->init_precision = p->ctx->precision;

@@ -1229,7 +1229,7 @@ int build(dpc_plan* p, int R, int S, bool has_v, bool exact)
   P.a_bt = put(bt.data(), sizeof(ResTask) * bt.size());
   P.table_vecs = (int)(at / 16);
   if (cudaMalloc(&st->dev, host.size()) != cudaSuccess ||
-      cudaMemcpy(st->dev, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+      cudaMemcpyAsync(st->dev, host.data(), host.size(), cudaMemcpyHostToDevice, p->ctx->stream) != cudaSuccess)
   {
     cudaFree(st->dev);
     delete st;

@@ -62,3 +62,21 @@ def test_bad_arguments_are_rejected(built_library):
         dp.DKPPCN(dp.Linear(4, 5), dp.Linear(6, 3), batch_size=2)
     with pytest.raises(TypeError):
         dp.DKPPCN(dp.TanH(), batch_size=2)
+
+
+def test_all_device_work_is_ordered_on_a_stream_of_the_library():
+    """Contexts use streams that do not wait for the default stream, and copies and clears on the default
+    stream return before they are done: every one of them, and every launch, names its stream."""
+    csrc = os.path.join(ROOT, "deepity_b200", "csrc")
+    for name in sorted(os.listdir(csrc)):
+        if not name.endswith((".cu", ".cuh", ".h")):
+            continue
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read())
+        assert not re.findall(r"\bcuda(?:Memset|Memcpy|Memcpy2D)\s*\(", text), name
+        for launch in re.findall(r"<<<(.*?)>>>", text, re.S):
+            depth, args = 0, 1
+            for c in launch:
+                depth += c in "([{"
+                depth -= c in ")]}"
+                args += c == "," and depth == 0
+            assert args == 4, (name, launch)
