@@ -693,6 +693,12 @@ static bool narrow_forward(const dpc_plan* p, int layer)
 static int forward_simt(dpc_plan* p, int first, int count, int flags)
 {
   cudaStream_t st = p->ctx->stream;
+  if ((flags & DPC_FWD_CE) && count > 1 && first + count == p->n - 1)
+  {
+    // the head's kernel forms the softmax error, so the head does not share a grouped launch
+    const int rc = forward_simt(p, first, count - 1, flags & ~DPC_FWD_CE);
+    return rc == DPC_OK ? forward_simt(p, p->n - 2, 1, flags) : rc;
+  }
   for (int f = first; f < first + count; f += kMaxZ)
   {
     const int c = std::min(kMaxZ, first + count - f);
@@ -845,6 +851,10 @@ int dpc_forward(dpc_plan* p, int first, int count, int flags)
   int rc = check_range(p, first, count);
   if (rc != DPC_OK)
     return rc;
+  const bool head_cached = ((flags & DPC_FWD_CACHED) && first + count >= p->n - 1) ||
+                           ((flags & DPC_FWD_CACHED_FIRST) && first == p->n - 2);
+  if ((flags & DPC_FWD_CE) && (head_cached || !dpc_plan_fused_cross_entropy(p)))
+    return fail(DPC_ERR_INVALID, "DPC_FWD_CE: the head's forward kernel does not run, use dpc_error");
   if (flags & DPC_FWD_CACHED)
     return forward_simt(p, first, count, flags);
   const bool cached_first = (flags & DPC_FWD_CACHED_FIRST) && count > 0;
@@ -877,8 +887,8 @@ int dpc_plan_fused_cross_entropy(dpc_plan* p)
   const int head = p->n - 2;
   auto tensor = [&](int l)
   { return (p->run.count > 0 && l >= p->run.first && l < p->run.first + p->run.count) || tc_extra_layer(p, l); };
-  // the head must be a launch of its own: above the (clamped, separate) input layer or a tensor-core
-  // layer, else it shares the grouped launch of the layers below it
+  // where the head shares the grouped launch of other layers, a launch of its own would cost more than the
+  // two small kernels it replaces: only above the (clamped, separate) input layer or a tensor-core layer
   return head >= 1 && narrow_forward(p, head) && !tensor(head) && (head == 1 || tensor(head - 1)) ? 1 : 0;
 }
 

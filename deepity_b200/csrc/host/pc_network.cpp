@@ -667,7 +667,7 @@ float PCNetwork::CalculateState(bool needEnergy, bool skipInputError)
   if (needEnergy && transientFlag)
     flags &= ~DPC_FWD_FE;
   const bool ce = (layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE) != 0;
-  const bool fused = ce && dpc_plan_fused_cross_entropy(plan);
+  const bool fused = ce && HeadFormsError();
   const int from = skipInputError ? 1 : 0;
   ForwardRange(from, n - 1 - from, flags | (fused ? DPC_FWD_CE : 0));
   if (ce && !fused)
@@ -797,7 +797,13 @@ struct PhaseScope
 
 bool PCNetwork::PredictionsTransient()
 {
-  return !(layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE) || dpc_plan_fused_cross_entropy(plan);
+  return !(layers.back()->d.flags & DPC_LAYER_SOFTMAX_CE) || HeadFormsError();
+}
+
+// The head's forward kernel forms the softmax error (a clamped layer's cached prediction runs none).
+bool PCNetwork::HeadFormsError()
+{
+  return !layers[layers.size() - 2]->clamped && dpc_plan_fused_cross_entropy(plan);
 }
 
 // The last pass of a train step computes every layer's prediction for the energy but does not

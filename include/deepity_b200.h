@@ -279,7 +279,8 @@ enum
                                  cached prediction, DirectKPPCLayer.cpp:275-280)          */
   DPC_FWD_CACHED_FIRST = 1 << 5, /* the first layer of the range is DPC_FWD_CACHED, the others not */
   DPC_FWD_CE = 1 << 6,        /* with ERR_NEXT: the head's kernel computes the softmax cross-entropy
-                                 error of the last layer itself (see dpc_plan_fused_cross_entropy)  */
+                                 error of the last layer itself; refused where it does not
+                                 (dpc_plan_fused_cross_entropy is 0, or the head itself is cached)  */
   DPC_FWD_NO_MU = 1 << 9,     /* with COPY_NEXT: mu[l] itself is not written (z[l+1] holds the
                                  same values and mu is recomputed before anyone reads it)  */
   DPC_FWD_NO_PREACT = 1 << 11, /* with COPY_NEXT and NO_MU: preact[l] is not written either (the

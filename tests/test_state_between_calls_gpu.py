@@ -242,3 +242,27 @@ def test_convolution_gradient_sums_stay_in_the_callers_buffers(conv_plan):
     sync()
     for n, ref in (("g_W", dW), ("g_b", db), ("W", before["W"] + 0.1 / 3 * dW), ("b", before["b"] + 0.1 / 3 * db)):
         assert rel_err(ref.cpu(), t[n].cpu()) <= 1e-5, n  # 75 products of unit size in fp32
+
+
+def test_softmax_error_formed_in_the_head_with_an_unclamped_input(built_library):
+    """The range of a forward pass starts at the input layer: the head is launched on its own all the same."""
+    from deepity_b200 import _lib
+    lib = _lib.load()
+    case = dict(kind="full", sizes=[40, 128, 10], batch=33, T=2, steps=1, options=dict(cross_entropy=1),
+                hyper=dict(lr=0.01, ir=0.1, fl=0.01, lmbda=0.0, act="tanh"))
+    net, x, y = build_gpu_net(case)
+    net.train_step(x, y, 2)
+    plan = lib.dpcn_plan(net._h)
+    assert lib.dpc_plan_fused_cross_entropy(plan) == 1
+    net.set_tensor(2, "e", np.zeros((33, 10), np.float32))
+    net.set_tensor(1, "fe", np.zeros((33, 10), np.float32))
+    ERR, FE, CACHED, CE = 2, 8, 16, 64
+    assert lib.dpc_forward(plan, 0, 2, ERR | FE | CE) == 0
+    z = [net.get_tensor(l, "z").reshape(33, -1) for l in range(3)]
+    W, b = net.get_tensor(1, "W").reshape(10, 128), net.get_tensor(1, "b")
+    pre = z[1].astype(np.float64) @ W.T + b
+    s = np.exp(np.tanh(pre) - np.tanh(pre).max(1, keepdims=True))
+    e = z[2] - s / s.sum(1, keepdims=True)
+    assert rel_err(e, net.get_tensor(2, "e")) <= TOL
+    assert rel_err(e * (1 - np.tanh(pre) ** 2), net.get_tensor(1, "fe")) <= TOL
+    assert lib.dpc_forward(plan, 1, 1, ERR | CACHED | CE) == -1  # no head kernel runs
