@@ -836,7 +836,9 @@ void PCNetwork::RowSegment(int ops, int steps)
     layers[0]->cacheValid = true;
   if (steps > 0 || (ops & DPC_ROWS_ENERGY_LAST))
     ops |= DPC_ROWS_STORE_E;
-  if (steps > 0 || (ops & (DPC_ROWS_SWEEP | DPC_ROWS_LOGITS | DPC_ROWS_ZERO_Z)))
+  // (SimplePC: f(z), which every forward pass leaves in zF, goes with the beliefs)
+  if (steps > 0 || (ops & (DPC_ROWS_SWEEP | DPC_ROWS_LOGITS | DPC_ROWS_ZERO_Z)) ||
+      (kind == NetworkKind::SIMPLE && (ops & DPC_ROWS_ENERGY_LAST)))
     ops |= DPC_ROWS_STORE_Z;
   if (steps > 0 && useMomentum)
     ops |= DPC_ROWS_STORE_V;

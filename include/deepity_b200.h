@@ -414,7 +414,7 @@ enum
   DPC_ROWS_GATE_LAST = 1 << 12,  /* ... and gated errors                                             */
   DPC_ROWS_PRED_CLOSE = 1 << 13, /* the closing pass stores mu and preact                            */
   DPC_ROWS_LOGITS = 1 << 14,     /* the last layer's belief becomes the prediction below it          */
-  DPC_ROWS_STORE_Z = 1 << 15,
+  DPC_ROWS_STORE_Z = 1 << 15,    /* beliefs, with SimplePC layers also zF                            */
   DPC_ROWS_STORE_E = 1 << 16,
   DPC_ROWS_STORE_G = 1 << 17,    /* fe */
   DPC_ROWS_STORE_V = 1 << 18

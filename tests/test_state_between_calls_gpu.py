@@ -78,6 +78,20 @@ def test_input_activations_read_back_as_last_fed(call, plan_of):
         assert rel_err(ref, got[0][key]) <= TOL, key
 
 
+@pytest.mark.parametrize("call", sorted(CALLS))
+def test_input_activations_after_row_segments(call, plan_of):
+    """zF is what the last forward pass of the call was fed, as phase by phase."""
+    got = []
+    for plain in (False, True):
+        lib, net, plan, x, y = plan_of(ROWS, plain)
+        assert lib.dpc_rows_available(plan) == (0 if plain else 1)
+        for _ in range(2):
+            CALLS[call](net, x, y)
+        got.append([net.get_tensor(l, "zF") for l in range(3)])
+    for l, (a, ref) in enumerate(zip(*got)):
+        assert rel_err(ref, a) <= TOL, l
+
+
 @pytest.mark.parametrize("graph", [True, False])
 def test_a_step_without_settling_learns_from_what_was_last_fed(graph, plan_of):
     """Mode 2 without a settling step is a weight update alone (train_step_python of the oracle)."""
