@@ -825,6 +825,12 @@ bool PCNetwork::UseRowSegments()
   return !useEPC && !ghostTop && !gradSync && dpc_rows_available(plan);
 }
 
+// (Without a settling step mode 2 is a weight update from whatever the last call left: no segment.)
+bool PCNetwork::TrainsInSegments(int mode, int steps)
+{
+  return UseRowSegments() && !(kind == NetworkKind::SIMPLE && mode == 2 && steps == 0);
+}
+
 // One row segment; what it stores follows from what it computes.
 void PCNetwork::RowSegment(int ops, int steps)
 {
@@ -917,7 +923,7 @@ void PCNetwork::RunTrainSegments(int mode, int steps)
 
 void PCNetwork::RunTrainPhases(int mode, int steps)
 {
-  if (UseRowSegments())
+  if (TrainsInSegments(mode, steps))
     RunTrainSegments(mode, steps);
   else
     RunGroupedPhases(mode, steps);
@@ -1025,7 +1031,7 @@ float PCNetwork::TrainStepRaw(int mode, const float* x, size_t nx, const float* 
   // DirectKP / Full steps open with the forward sweep over the whole stack; x and y must then
   // cover their layers completely (a short buffer leaves the rest at zero, as the memset would)
   // (a row segment starts from zero beliefs, errors and momentum by itself)
-  const bool segments = UseRowSegments();
+  const bool segments = TrainsInSegments(mode, steps);
   const bool sweepOverwrites = (kind != NetworkKind::SIMPLE || segments) &&
                                nx >= (size_t)batchSize * layers.front()->d.size &&
                                ny >= (size_t)batchSize * layers.back()->d.size;

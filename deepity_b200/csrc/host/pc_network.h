@@ -218,6 +218,7 @@ private:
   void SyncGradients(size_t count);
   void ForwardRange(int first, int count, int flags);
   bool UseRowSegments();
+  bool TrainsInSegments(int mode, int steps);
   bool HeadFormsError();
   bool PredictionsTransient(); // no pass but the last need store mu / preact
   void RowSegment(int ops, int steps);

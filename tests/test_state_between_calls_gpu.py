@@ -92,13 +92,14 @@ def test_input_activations_after_row_segments(call, plan_of):
         assert rel_err(ref, a) <= TOL, l
 
 
+@pytest.mark.parametrize("case", [RUN, ROWS], ids=["run", "rows"])
 @pytest.mark.parametrize("graph", [True, False])
-def test_a_step_without_settling_learns_from_what_was_last_fed(graph, plan_of):
+def test_a_step_without_settling_learns_from_what_was_last_fed(graph, case, plan_of):
     """Mode 2 without a settling step is a weight update alone (train_step_python of the oracle)."""
     from common import _oracle_kwargs, make_case, make_oracle
-    params, x, y = make_case("simple", RUN["sizes"], RUN["batch"])
-    orc = make_oracle("simple", RUN["sizes"], RUN["batch"], params, **_oracle_kwargs(RUN))
-    _, net, _, _, _ = plan_of(RUN)
+    params, x, y = make_case("simple", case["sizes"], case["batch"])
+    orc = make_oracle("simple", case["sizes"], case["batch"], params, **_oracle_kwargs(case))
+    _, net, _, _, _ = plan_of(case)
     net.set_use_graph(graph)
     for T in (3, 0, 0, 2, 0):
         orc.train_step_python(x, y, T)
