@@ -1312,6 +1312,21 @@ int res_plan_init(dpc_plan* p)
                                 : (R == 1 ? 300 + 2.5 * longest : 100 + 2.5 * longest);
   if (wbytes > limit_kb * 1024 || w0 > 2560 * 1024)
     return 1;
+  // Batches of more than one group of 8 rows per SM: a block walks its groups one after the other, reading
+  // the streamed weights and those of the input layer again for each, while the phase kernels fill the GPU
+  // better the larger the batch.  A network with feedback weights opens three segments a step, each with
+  // weights and state to load, a SimplePC network one or two, and the input layer's weights are read once a
+  // step: a quarter of the others' weight.  Limits on rounds x (input layer / 4 + others) in KB, from 3412
+  // random networks (batch 200 to 4096, 2 to 20 settling steps).  Geometric means of segments / phase kernels
+  // beyond one round were 1.10 (feedback, ordered sums; slowest 1.78) and 1.05 (sliced), 0.88 and 0.80
+  // (SimplePC); within the limits 1.03, 1.01, 0.85 and 0.79.  Segments / phase kernels in us a step:
+  //   ordered   DKP 784-(91x4)-100 at batch 3584, 2 steps 2043/1868    Full 400-256-256-2 at 3747, 6 steps 1551/870
+  //             SimplePC 717-287-100 at 2816, 4 steps 952/697, 1500-85-85-85-10 at 2217, 12 steps 534/804 (kept)
+  const long long rounds = ((long long)(p->batch + R - 1) / R + p->ctx->sm_count - 1) / p->ctx->sm_count;
+  const bool feedback = !(p->h[0].flags & DPC_LAYER_INPUT_ACT);
+  const double round_kb = exact ? (feedback ? 200 : 800) : (feedback ? 800 : 1600);
+  if (rounds > 1 && rounds * (w0 / 4 + wbytes) > round_kb * 1024)
+    return 1;
   for (; R >= 1; R /= 2)
   {
     const int rc = build(p, R, S, has_v, exact);

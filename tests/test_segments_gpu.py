@@ -59,11 +59,20 @@ def test_row_segments_match_oracle(name, built_library):
 @pytest.mark.parametrize("sizes,batch,act", [((64, 1024, 1000, 10), 9, "tanh"),  # 4 MB above the first layer
                                              ((64,) + (128,) * 10 + (10,), 149, "tanh"),  # short sums, many layers
                                              ((64, 384, 384, 10), 20, "relu"),   # 605 KB, ordered sums
-                                             ((64, 384, 256, 10), 149, "relu")])  # 404 KB, two rows a block
+                                             ((64, 384, 256, 10), 149, "relu"),  # 404 KB, two rows a block
+                                             # several groups of rows a block: input layer and others
+                                             ((784, 264, 64, 10), 2400, "tanh")])
 def test_row_segments_stop_at_their_weight_limit(sizes, batch, act, built_library):
     case = _case("dkp", list(sizes), batch, act)
     assert _available(case) == 0
     compare_outputs(run_oracle(case), run_gpu(case), TOL, "over the limit")
+
+
+@pytest.mark.parametrize("kind,batch,available", [("dkp", 1184, 1), ("dkp", 1185, 0), ("simple", 1185, 1),
+                                                  ("simple", 4096, 1)])
+def test_row_segments_of_several_groups_a_block(kind, batch, available, built_library):
+    """106 KB of ordered sums a round (the input layer's 279 KB count a quarter) on 148 SMs of 8-row blocks."""
+    assert _available(_case(kind, [784, 91, 91, 10], batch, "relu")) == available
 
 
 def _images(shape, convs, act, batch, **kw):
