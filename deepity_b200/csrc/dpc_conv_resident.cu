@@ -789,7 +789,7 @@ int conv_res_init(dpc_conv_plan* p)
     return 1;
   Builder B;
   B.rl.resize(nw);
-  size_t weights = 0;
+  size_t weights = 0, shared = 0;
   std::vector<int> low_y(nw + 1, 0), low_x(nw + 1, 0), zpitch(nw + 1), zrows(nw + 1);
   std::vector<int> glow_y(nw, 0), glow_x(nw, 0), gpitch(nw, 0), grows(nw, 0);
   auto dense = [&](int l)
@@ -845,8 +845,11 @@ int conv_res_init(dpc_conv_plan* p)
     const dpc_conv_layer& L = p->h[l];
     RcLayer& q = B.rl[l];
     q.C = L.in_c, q.HW = L.in_h * L.in_w, q.O = L.out_c, q.P = L.out_h * L.out_w;
-    weights += sizeof(float) * (size_t)L.out_c * L.in_c * L.k_h * L.k_w;
+    const size_t bytes = sizeof(float) * (size_t)L.out_c * L.in_c * L.k_h * L.k_w;
+    weights += bytes;
     q.dense = dense(l);
+    if (l > 0 && !q.dense)
+      shared += bytes;
     q.vec = (q.C * q.HW) % 4 == 0 && (reinterpret_cast<uintptr_t>(L.W) & 15) == 0;
     if (q.dense && l > 0)
       gpitch[l] = grows[l] = 1;
@@ -863,9 +866,20 @@ int conv_res_init(dpc_conv_plan* p)
   }
   P.gfloat = (int)(eg - at);
   at = std::max(eg, at + (size_t)P.xfloats);
-  // the weights of all layers but the first stream from L2 once or more per pass: beyond 4 MB the
-  // grouped kernels' reuse over the batch wins
-  if (at * sizeof(float) > kSmemLimit || weights > (4u << 20))
+  // A block reads the weights of every layer above the first from L2 in each pass, whatever the batch, where
+  // the phase kernels share them between images and split them over the SMs.  Segments / phase kernels,
+  // geometric means over random networks (8 to 28 pixels a side, 3 to 10 passes) by KB of weights in
+  // the layers between the first and the dense heads:
+  //            <= 100    100-200   200-300   300-450   450-1200  1200-4000
+  //   1-4      0.52      0.80      0.77      1.35      1.78      1.79      images
+  //   6-12     0.44      0.86      1.09      1.01      1.36      -
+  //   16-64    0.27      0.58      0.56      0.72      0.60      0.96
+  // (109-109-109 channels of 3x3 taps on 12x12 pixels, 8 images: 487/250 us, 411 before there were segments.)
+  // A single image pays for its heads too: 87 channels on 8x8 pixels and 37 outputs, 805 KB, 340/291 us.
+  // All weights together, at 128 images: 0-4 MB 0.35, 4-6 MB 0.34, 6-10 MB 0.54; at 32-64 images 0.61, 0.63, 1.05.
+  const size_t first = sizeof(float) * (size_t)p->h[0].out_c * p->h[0].in_c * p->h[0].k_h * p->h[0].k_w;
+  if (at * sizeof(float) > kSmemLimit || weights > (4u << 20) || (shared > 300 * 1024 && p->batch <= 12) ||
+      (weights - first > 768 * 1024 && p->batch == 1))
     return 1;
   // ---- pixel tables
   auto plane_table = [&](int h, int w, int pitch, int ly, int lx)

@@ -92,6 +92,17 @@ IMAGES = {
 }
 
 
+@pytest.mark.parametrize("channels,batch,available", [(92, 12, 1), (93, 12, 0), (93, 13, 1)])
+def test_image_segments_of_few_images_stop_at_large_kernels(channels, batch, available, built_library):
+    """92 x 92 kernels of 3 x 3 taps are 298 KB."""
+    from deepity_b200 import _lib
+    lib = _lib.load()
+    case = _images((1, 6, 6), [(channels, 3, 3, 1, 1, 1, 1), (channels, 3, 3, 2, 2, 1, 1), (4, 3, 3, 1, 1, 0, 0)],
+                   "tanh", batch)
+    assert lib.dpc_conv_images_available(lib.dpcn_conv_plan(build_conv_gpu_net(case)._h)) == available
+    compare_outputs(run_conv_oracle(case), run_conv_gpu(case), TOL, str(batch))
+
+
 @pytest.mark.parametrize("name", sorted(IMAGES))
 def test_image_segments_match_oracle(name, built_library):
     from deepity_b200 import _lib
