@@ -5,7 +5,8 @@
 // 32x32x3 network of 32-64-128 channels -- and walks projection, settling steps and energy in one
 // launch; the weights stream from L2.  The launches it replaces took 430 us per settling step of
 // that network at batch 128 (the transposed convolution alone 209 us: a gather over all taps of
-// which stride 2 wastes three in four, with integer divisions per element); this kernel takes 40 us.
+// which stride 2 wastes three in four, with integer divisions per element); this kernel takes 36 us
+// (433 us for a segment of ten, 73 of which are loads, the input layer and a closing pass).
 //
 // Both products are implicit GEMMs on the tensor cores with separable addresses: the operand of
 // (k, pixel) sits at koff[k] + base[pixel], with zero borders around the planes instead of tests.

@@ -1479,7 +1479,6 @@ int dpc_weight_gradients(dpc_plan* p, int first, int count, int which)
     return DPC_OK;
   if ((rc = staging_ready(p, first, count, which)) != DPC_OK)
     return rc;
-  cudaStream_t st = p->ctx->stream;
   if (which == 1)
   {
     if ((rc = launch_dfa_proj(p, first, count, 0)) != DPC_OK)

@@ -1310,6 +1310,13 @@ int res_plan_init(dpc_plan* p)
   //             64-384-384-10 (605 KB)  399/368  576/456  2946/1246  64-512-310-10  429/415  621/566  1211/930
   const double limit_kb = exact ? (R == 1 ? 100 + 1.0 * longest : 60 + 0.85 * longest)
                                 : (R == 1 ? 300 + 2.5 * longest : 100 + 2.5 * longest);
+  // The input layer's weights, read once a step by every block.  Segments / phase kernels, geometric means by
+  // their size, batch <= 148 and 149 to 592:       SimplePC ordered  sliced      feedback ordered  sliced
+  //   0.9-2.5 MB                                    0.39 / 0.46      0.27 / 0.33     0.79 / 0.94    0.50 / 0.56
+  //   2.5-4 MB                                      0.43 / 0.69      0.25 / 0.32     0.91 / 0.90    0.47 / 0.60
+  //   4-8 MB                                        0.45 / 0.53      0.24 / 0.40     0.88 / 1.14    0.48 / 0.67
+  // Feedback networks with ordered sums lose first: 1.12 at 593 to 1184 rows and 0.9-2 MB, 1.45 at 2.5-4.
+  // The line is where they reach the phase kernels' time; the others would go on.
   if (wbytes > limit_kb * 1024 || w0 > 2560 * 1024)
     return 1;
   // Batches of more than one group of 8 rows per SM: a block walks its groups one after the other, reading
