@@ -95,6 +95,10 @@ SIMPLE_RUN = {
     "projection": _case("simple", [64] + [256] * 3 + [10], 512, "gelu", mode="projection"),
     "python": _case("simple", [256] * 4 + [10], 256, "sigmoid", mode="python"),
     "softmax": _case("simple", [64] + [256] * 3 + [10], 256, mode="projection", cross_entropy=1),
+    # the softmax error is the work of a kernel of its own, right above the run
+    "softmax_above": _case("simple", [64] + [256] * 3, 256, mode="projection", cross_entropy=1),
+    "no_settling": _case("simple", [64] + [256] * 3 + [10], 256, T=0),
+    "centred": _case("simple", [64] + [256] * 3 + [10], 256, center_weights=1),
 }
 
 

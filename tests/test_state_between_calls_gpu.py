@@ -281,3 +281,17 @@ def test_softmax_error_formed_in_the_head_with_an_unclamped_input(built_library)
     assert rel_err(e, net.get_tensor(2, "e")) <= TOL
     assert rel_err(e * (1 - np.tanh(pre) ** 2), net.get_tensor(1, "fe")) <= TOL
     assert lib.dpc_forward(plan, 1, 1, ERR | CACHED | CE) == -1  # no head kernel runs
+
+
+def test_errors_under_a_softmax_top_after_a_recorded_step(plan_of):
+    """A replayed step leaves the top layer's softmax error in fp32 only; an update of the caller's own reads it."""
+    case = dict(RUN, sizes=[64, 256, 256, 256], options=dict(cross_entropy=1))
+    got = []
+    for plain in (False, True):
+        lib, net, plan, x, y = plan_of(case, plain)
+        for _ in range(3):
+            net.train_step_with_projection(x, y, 3)
+        assert lib.dpc_update_state(plan, 1, 2) == 0 and lib.dpc_update_weights(plan, 0, 3, 0) == 0
+        got.append({(l, n): net.get_tensor(l, n) for l in (1, 2) for n in ("z", "W")})
+    for key, ref in got[1].items():
+        assert rel_err(ref, got[0][key]) <= TOL, key
