@@ -73,6 +73,16 @@ class LayerView:
         self._net.set_tensor(self.index, "Psi", p)
 
 
+class DevicePointer(int):
+    """An address in a network's device memory that keeps the network alive: views made from it (through
+    __cuda_array_interface__, say) must not outlive the memory."""
+
+    def __new__(cls, value: int, owner):
+        self = super().__new__(cls, value)
+        self.owner = owner
+        return self
+
+
 class _Network:
     KIND = KIND_DKP
     NAME = "network"
@@ -175,11 +185,12 @@ class _Network:
         _lib.check(self._lib.dpcn_set_tensor(self._h, layer, name.encode(), _ptr(v), v.size))
 
     def tensor_ptr(self, layer: int, name: str) -> int:
+        """Device address of a state tensor; the network lives at least as long as the result."""
         p = ctypes.c_void_p()
         stride = ctypes.c_int64()
         _lib.check(self._lib.dpcn_tensor_ptr(self._h, layer, name.encode(), ctypes.byref(p),
                                              ctypes.byref(stride)))
-        return p.value
+        return p.value and DevicePointer(p.value, self)
 
     # ---- setters (deepity/DKPPCN.py:218-262) -------------------------------------------
     def set_optimizer(self, optimizer: str) -> None:

@@ -295,3 +295,17 @@ def test_errors_under_a_softmax_top_after_a_recorded_step(plan_of):
         got.append({(l, n): net.get_tensor(l, n) for l in (1, 2) for n in ("z", "W")})
     for key, ref in got[1].items():
         assert rel_err(ref, got[0][key]) <= TOL, key
+
+
+def test_device_pointers_keep_their_network_alive(built_library):
+    """Views made from a pointer read the network's memory: it must not go with the last name of the network."""
+    import gc
+    import weakref
+    net, _, _ = build_gpu_net(ROWS)
+    alive, ptr = weakref.ref(net), net.tensor_ptr(1, "W")
+    del net
+    gc.collect()
+    assert alive() is not None and ptr == alive().tensor_ptr(1, "W")
+    del ptr
+    gc.collect()
+    assert alive() is None
