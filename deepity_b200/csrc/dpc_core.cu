@@ -5,7 +5,7 @@
 #include <string>
 
 #include "dpc_internal.h"
-#include "dpc_simt.cuh"
+#include "dpc_batch.cuh"
 
 namespace dpc
 {
@@ -110,6 +110,18 @@ static int launch_gemm(dpc_plan* p, int first, int count, int flags, int mode, c
   auto kern = T == 32 ? pc_gemm_kernel<OP, 32> : pc_gemm_kernel<OP, 64>;
   kern<<<grid, NTHREADS, 0, p->ctx->stream>>>(p->d, first, p->n, p->batch, flags, mode, p->energy, epc_src);
   return check_launch(p->ctx, "grouped GEMM kernel");
+}
+
+// Networks with an Adam-type optimizer or an activation with a kink turn a rounding difference into a whole
+// step (an update m / (sqrt(v) + eps), a derivative that flips between 0 and 1): every sum of theirs keeps
+// one order of additions.
+bool ordered_sums(const dpc_plan* p)
+{
+  for (const dpc_layer& L : p->h)
+    if (L.next_size > 0 && (L.opt != DPC_OPT_SGD || (L.Psi && L.opt_psi != DPC_OPT_SGD) || L.act == DPC_ACT_RELU ||
+                            L.act == DPC_ACT_HARD_TANH))
+      return true;
+  return false;
 }
 
 static int elem_blocks(const dpc_plan* p, size_t max_elems)
@@ -1142,13 +1154,85 @@ int dpc_relax(dpc_plan* p, int layer)
   return check_launch(p->ctx, "relax kernel");
 }
 
-static int weight_gemm_simt(dpc_plan* p, int first, int count, int mode, int flags)
+// Whether a layer is on the tensor-core path.
+static bool tc_piece(dpc_plan* p, int i)
+{
+  return (p->run.count > 0 && i >= p->run.first && i < p->run.first + p->run.count) || tc_extra_layer(p, i);
+}
+
+// Batch products (dpc_batch.cuh) of layers [first, first+count), for networks whose sums may be split.
+// weights: the weight sums of the layers for which it holds; with_sums (learn): their bias sums and the Psi
+// sums of all layers too.
+template <typename F>
+static int launch_batch_products(dpc_plan* p, int first, int count, int mode, int flags, F weights, bool with_sums)
+{
+  bool tensor = p->run.count > 0;
+  for (int i = 0; i < p->n && !tensor; ++i)
+    tensor = tc_extra_layer(p, i);
+  for (int f = first; f < first + count; f += kListLayers)
+  {
+    BatchTiles T = {};
+    T.bias = with_sums;
+    T.list.first = f, T.list.count = std::min(kListLayers, first + count - f);
+    for (int q = 0; q < T.list.count; ++q)
+    {
+      const int i = f + q;
+      const dpc_layer& L = p->h[i];
+      T.list.start[q + 1] = T.list.start[q];
+      if (L.next_size <= 0)
+        continue;
+      // DirectFeedbackUpdate is a no-op unless the layer above owns feedback weights
+      const bool w = weights(i) && ((mode & ~WG_GRAD_ONLY) != WG_DFA || (i + 1 < p->n && p->h[i + 1].Psi));
+      const bool psi = with_sums && L.Psi && !(L.flags & DPC_LAYER_INPUT_ACT);
+      if (w)
+        T.weights[q / 32] |= 1u << (q % 32);
+      T.list.start[q + 1] +=
+          ((w ? cdiv(L.next_size, BP_T) : 0) + (psi ? cdiv(L.terminal_size, BP_T) : 0)) * cdiv(L.size, BP_T);
+    }
+    const int tiles = T.list.start[T.list.count];
+    if (tiles == 0)
+      continue;
+    // CTAs of a cluster that share a tile's batch rows: two groups of rows or more for each warp; beside
+    // tensor-core launches, which leave few SMs free, eight (clusters of eight held up the launches behind
+    // them: 784-(256x8)-10 at batch 256 250 us a step, single CTAs 238).
+    const int rows = BP_WARPS * BP_ROWS * (tensor ? 8 : 2);
+    int R = 1;
+    while (R < 8 && (long long)tiles * R < 2LL * p->ctx->sm_count && p->batch >= 2 * R * rows)
+      R *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles * R));
+    cfg.blockDim = dim3(32 * BP_WARPS);
+    cfg.stream = p->ctx->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim = {(unsigned)R, 1, 1};
+    cfg.attrs = attr;
+    cfg.numAttrs = R > 1 ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, batch_product_kernel, (const dpc_layer*)p->d, T, p->n, p->batch, flags, mode,
+                       p->e_terminal);
+    const int rc = check_launch(p->ctx, "batch product kernel");
+    if (rc != DPC_OK)
+      return rc;
+  }
+  return DPC_OK;
+}
+
+// Before the weight sums of layers outside the tensor-core kernels: the operand of SimplePC layers is brought
+// up to date, and the weights' operand planes are about to be behind.
+static int weight_sums_begin(dpc_plan* p, int first, int count, int mode)
 {
   if (!(mode & WG_GRAD_ONLY))
     wrote(p, K_W, first, count);
-  const int ready = tc_zf_need(p, first, count); // (the operand of SimplePC layers)
+  return tc_zf_need(p, first, count);
+}
+
+static int weight_gemm_simt(dpc_plan* p, int first, int count, int mode, int flags)
+{
+  const int ready = weight_sums_begin(p, first, count, mode);
   if (ready != DPC_OK)
     return ready;
+  if (!ordered_sums(p))
+    return launch_batch_products(p, first, count, mode, flags, [](int) { return true; }, false);
   for (int f = first; f < first + count; f += kMaxZ)
   {
     const int c = std::min(kMaxZ, first + count - f);
@@ -1355,8 +1439,11 @@ static void psi_jobs(dpc_plan* p, int f, int c, int grad_only, std::vector<Job>&
 }
 
 // Bias update (or its raw sums) of layers [f, f+c).
-static int launch_bias_update(dpc_plan* p, int f, int c, int max_next, int grad_only)
+static int launch_bias_update(dpc_plan* p, int f, int c, int grad_only)
 {
+  int max_next = 0;
+  for (int i = f; i < f + c; ++i)
+    max_next = std::max(max_next, p->h[i].next_size);
   const int rc = tc_fe_need(p, f, c);
   if (rc != DPC_OK)
     return rc;
@@ -1366,9 +1453,70 @@ static int launch_bias_update(dpc_plan* p, int f, int c, int max_next, int grad_
   const bool by_blocks = fp.only || p->batch >= kBiasBlockRows;
   dim3 gb(std::max(1, cdiv(max_next, by_blocks ? 64 : 32)), c);
   launch_row_split(bias_update_kernel, gb, 256,
-                   by_blocks ? row_split(p->ctx, (long long)gb.x * c, p->batch, 256) : 1, p->ctx->stream, p->d,
-                   f, p->n, p->batch, grad_only, fp);
+                   by_blocks ? row_split(p->ctx, (long long)gb.x * c, p->batch, ordered_sums(p) ? 256 : 1024) : 1,
+                   p->ctx->stream, p->d, f, p->n, p->batch, grad_only, fp);
   return check_launch(p->ctx, "bias_update kernel");
+}
+
+// Jobs of a learn phase (grad_only: the raw sums): the weight sums of tensor-core pieces by `tc`, the others',
+// bias and Psi sums by the kernels of this file.
+template <typename TcFn>
+static std::vector<Job> learn_jobs(dpc_plan* p, int first, int count, int grad_only, TcFn tc)
+{
+  const int mode = WG_LEARN | (grad_only ? WG_GRAD_ONLY : 0);
+  auto simt = [=](int f, int c) { return weight_gemm_simt(p, f, c, mode, 0); };
+  std::vector<Job> jobs;
+  if (ordered_sums(p))
+  {
+    jobs = pieces_of(p, first, count, tc, simt, true);
+    bool psi = false;
+    for (int i = first; i < first + count; ++i)
+      psi |= p->h[i].Psi != nullptr && !(p->h[i].flags & DPC_LAYER_INPUT_ACT);
+    for (int f = first; f < first + count; f += kMaxZ)
+    {
+      const int c = std::min(kMaxZ, first + count - f);
+      jobs.push_back([=] { return launch_bias_update(p, f, c, grad_only); });
+      if (psi)
+        psi_jobs(p, f, c, grad_only, jobs);
+    }
+    return jobs;
+  }
+  // Psi of tensor-core layers: strips of 128 columns x the whole batch where there are enough of them; tiles that
+  // share the batch else, in one launch with the sums of the other layers (a 32 x 32 tile of ten terminal units
+  // multiplies 1.6 times what it keeps).
+  long long strips = 0;
+  for (int i = first; i < first + count; ++i)
+    if (tc_piece(p, i) && p->h[i].Psi && p->h[i].size % 128 == 0 && p->h[i].terminal_size <= 16)
+      strips += p->h[i].size / 128;
+  const bool by_strips = strips >= 4LL * p->ctx->sm_count;
+  auto sums = [=](int f, int c)
+  {
+    for (int i = f; i < f + c; ++i)
+      if (const int rc = tc_piece(p, i) ? DPC_OK : weight_sums_begin(p, i, 1, mode))
+        return rc;
+    return launch_batch_products(p, f, c, mode, 0, [=](int i) { return !tc_piece(p, i); }, true);
+  };
+  for (int i = first, j; i < first + count; i = j)
+  {
+    const bool t = tc_piece(p, i);
+    for (j = i + 1; j < first + count && j - i < kMaxZ && tc_piece(p, j) == t;)
+      ++j;
+    const int f = i, c = j - i;
+    if (t)
+    {
+      // (a piece that `tc` declines gets its weight sums from `simt`)
+      const std::vector<Job> own = pieces_of(p, f, c, tc, simt, true);
+      jobs.insert(jobs.begin(), own.begin(), own.end());
+      jobs.push_back([=] { return launch_bias_update(p, f, c, grad_only); });
+      if (by_strips)
+        psi_jobs(p, f, c, grad_only, jobs);
+    }
+    else if (by_strips)
+      jobs.push_back([=] { return sums(f, c); });
+  }
+  if (!by_strips)
+    jobs.push_back([=] { return sums(first, count); });
+  return jobs;
 }
 
 int dpc_update_weights(dpc_plan* p, int first, int count, int center_rows)
@@ -1380,13 +1528,12 @@ int dpc_update_weights(dpc_plan* p, int first, int count, int center_rows)
     count -= 1;
   if (count <= 0)
     return DPC_OK;
-  bool any_adam = false, any_psi = false;
+  bool any_adam = false;
   int max_next = 0;
   for (int i = first; i < first + count; ++i)
   {
     const dpc_layer& L = p->h[i];
     any_adam |= L.opt != DPC_OPT_SGD || (L.Psi && L.opt_psi != DPC_OPT_SGD);
-    any_psi |= L.Psi != nullptr && !(L.flags & DPC_LAYER_INPUT_ACT);
     max_next = std::max(max_next, L.next_size);
   }
   if (any_adam)
@@ -1398,8 +1545,8 @@ int dpc_update_weights(dpc_plan* p, int first, int count, int center_rows)
   // the feedback-error planes are read by two of the jobs below: bring them up to date before the fork
   if ((rc = tc_fe_need(p, first, count)) != DPC_OK)
     return rc;
-  std::vector<Job> jobs = pieces_of(
-      p, first, count,
+  const std::vector<Job> jobs = learn_jobs(
+      p, first, count, 0,
       [=](int f, int c) -> int
       {
         bool all_sgd = true, all_staged = true;
@@ -1430,15 +1577,7 @@ int dpc_update_weights(dpc_plan* p, int first, int count, int center_rows)
             return r;
         }
         return DPC_OK;
-      },
-      [=](int f, int c) { return weight_gemm_simt(p, f, c, WG_LEARN, 0); }, true);
-  for (int f = first; f < first + count; f += kMaxZ)
-  {
-    const int c = std::min(kMaxZ, first + count - f);
-    jobs.push_back([=] { return launch_bias_update(p, f, c, max_next, 0); });
-    if (any_psi)
-      psi_jobs(p, f, c, 0, jobs);
-  }
+      });
   if ((rc = run_side_by_side(p->ctx, jobs)) != DPC_OK)
     return rc;
   for (int f = first; center_rows && f < first + count; f += kMaxZ)
@@ -1489,35 +1628,11 @@ int dpc_weight_gradients(dpc_plan* p, int first, int count, int which)
         [&](int f, int c) { return weight_gemm_simt(p, f, c, WG_DFA | WG_GRAD_ONLY, 0); },
         /*independent=*/true);
   }
-  rc = dispatch_range(
-      p, first, count,
-      [&](int f, int c) { return tc_weight_gemm(p, f, c, WG_LEARN | WG_GRAD_ONLY); },
-      [&](int f, int c) { return weight_gemm_simt(p, f, c, WG_LEARN | WG_GRAD_ONLY, 0); },
-      /*independent=*/true);
-  if (rc != DPC_OK)
+  if ((rc = tc_fe_need(p, first, count)) != DPC_OK)
     return rc;
-  bool any_psi = false;
-  int max_next = 0;
-  for (int i = first; i < first + count; ++i)
-  {
-    const dpc_layer& L = p->h[i];
-    any_psi |= L.Psi != nullptr && !(L.flags & DPC_LAYER_INPUT_ACT);
-    max_next = std::max(max_next, L.next_size);
-  }
-  for (int f = first; f < first + count; f += kMaxZ)
-  {
-    const int c = std::min(kMaxZ, first + count - f);
-    if ((rc = launch_bias_update(p, f, c, max_next, 1)) != DPC_OK)
-      return rc;
-    if (any_psi)
-    {
-      std::vector<Job> jobs;
-      psi_jobs(p, f, c, 1, jobs);
-      if ((rc = run_side_by_side(p->ctx, jobs)) != DPC_OK)
-        return rc;
-    }
-  }
-  return DPC_OK;
+  return run_side_by_side(
+      p->ctx, learn_jobs(p, first, count, 1,
+                         [=](int f, int c) { return tc_weight_gemm(p, f, c, WG_LEARN | WG_GRAD_ONLY); }));
 }
 
 int dpc_apply_gradients(dpc_plan* p, int first, int count, int which, int global_batch, int option)

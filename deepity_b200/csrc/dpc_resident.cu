@@ -1276,12 +1276,11 @@ int res_plan_init(dpc_plan* p)
   size_t wbytes = 0;
   int S = 0;
   int longest = 0;
-  bool has_v = false, exact = false;
+  bool has_v = false;
+  const bool exact = ordered_sums(p);
   for (int l = 0; l < nw; ++l)
   {
     const dpc_layer& L = p->h[l];
-    exact |= L.opt != DPC_OPT_SGD || (L.Psi && L.opt_psi != DPC_OPT_SGD) || L.act == DPC_ACT_RELU ||
-             L.act == DPC_ACT_HARD_TANH;
     if (L.next_size <= 0 || L.next_size > 8192 || (l > 0 && L.size > 16384) ||
         ((L.flags ^ p->h[0].flags) & DPC_LAYER_INPUT_ACT) || (l == 0 && (L.flags & DPC_LAYER_RESIDUAL)))
       return 1;

@@ -49,6 +49,24 @@ def test_grouped_launches_match_oracle(name, built_library, monkeypatch):
     _check(GROUPED[name], name)
 
 
+# Sums over the batch: fewer rows than a group, one over it, rows split over clusters; 16 and 17 rows in a tile;
+# more terminal units than a tile; more layers than a launch lists; Psi sums of tensor-core layers among others
+BATCH_SUMS = {
+    "one_row": _case("dkp", [20, 30, 5], 1),
+    "edges": _case("dkp", [33, 65, 31, 40], 9),
+    "clusters": _case("simple", [67, 31, 17], 1031, mode="projection"),
+    "many_layers": _case("dkp", [16] + [12] * 130 + [4], 5, T=2),
+    "beside_tensor_cores": _case("dkp", [64, 256, 256, 17], 256),
+    "beside_tensor_cores_rows_split": _case("full", [72, 256, 256, 16], 1024, "gelu"),
+}
+
+
+@pytest.mark.parametrize("name", sorted(BATCH_SUMS))
+def test_batch_sums_match_oracle(name, built_library, monkeypatch):
+    monkeypatch.setenv("DPC_DISABLE_RESIDENT", "1")
+    _check(BATCH_SUMS[name], name)
+
+
 PAIR = {
     "dkp": _case("dkp", [64] + [256] * 4 + [10], 256, T=4),
     "full_residual_momentum": _case("full", [64] + [256] * 3 + [10], 512, "gelu", mupc=1, residual=1, momentum=0.9),
