@@ -2,33 +2,10 @@
 // may be split: weight gradients g^T z, bias gradients (column sums of g) and feedback-weight gradients
 // z^T e_T, each with its update.
 #pragma once
-#include "dpc_simt.cuh"
+#include "dpc_gemm.cuh"
 
 namespace dpc
 {
-// The output tiles of a launch, layer by layer: start[i] is the first one of layer first + i.
-constexpr int kListLayers = 128;
-struct TileList
-{
-  int first, count;
-  int start[kListLayers + 1];
-};
-// Layer of tile t, which becomes the index within the layer.
-__device__ __forceinline__ int tile_layer(const TileList& T, int& t)
-{
-  int lo = 0;
-  for (int hi = T.count; hi - lo > 1;)
-  {
-    const int mid = (lo + hi) >> 1;
-    if (T.start[mid] <= t)
-      lo = mid;
-    else
-      hi = mid;
-  }
-  t -= T.start[lo];
-  return T.first + lo;
-}
-
 // One launch for all of them.  A CTA owns a 32 x 32 tile of one product; its eight warps take every eighth
 // group of eight batch rows, each warp all 1024 outputs (8 x 4 per lane, three 16-byte shared-memory reads
 // per 32 multiply-adds), with a cp.async ring of its own, so that the row loop holds no barrier.  The CTAs of

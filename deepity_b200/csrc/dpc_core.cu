@@ -87,29 +87,51 @@ static inline int cdiv(int a, int b)
   return (a + b - 1) / b;
 }
 
-// Launches the grouped GEMM over layers [first, first+count): 64 x 64 tiles, or 32 x 32 where the former
-// are fewer than the SMs (a CTA walks all of K by itself: smaller tiles are more and shorter walks).
+// A product of layers [first, first+count) in one launch (per 128 layers).
 template <int OP>
 static int launch_gemm(dpc_plan* p, int first, int count, int flags, int mode, const float* epc_src = nullptr)
 {
-  int mx = 0, my = 0;
-  long long tiles = 0;
-  for (int i = first; i < first + count; ++i)
+  for (int f = first; f < first + count; f += kListLayers)
   {
-    const dpc_layer& L = p->h[i];
-    if (L.next_size <= 0)
+    TileList list[2] = {}; // tiles of 32 and of 64
+    bool vec = true;       // rows can be copied 16 bytes at a time
+    for (int s = 0; s < 2; ++s)
+    {
+      TileList& T = list[s];
+      T.first = f, T.count = std::min(kListLayers, first + count - f);
+      for (int i = 0; i < T.count; ++i)
+      {
+        const dpc_layer& L = p->h[f + i];
+        const int M = OP == OP_WG ? L.next_size : p->batch, N = OP == OP_FWD ? L.next_size : L.size;
+        // (DirectFeedbackUpdate is a no-op unless the layer above owns feedback weights)
+        const bool any = L.next_size > 0 && (OP != OP_WG || (mode & ~WG_GRAD_ONLY) != WG_DFA ||
+                                             (f + i + 1 < p->n && p->h[f + i + 1].Psi));
+        T.start[i + 1] = T.start[i] + (any ? cdiv(M, 32 << s) * cdiv(N, 32 << s) : 0);
+        vec &= L.size % 4 == 0 && L.next_size % 4 == 0;
+      }
+    }
+    const int c = list[0].count, tiles = list[0].start[c], tiles64 = list[1].start[c], sm = p->ctx->sm_count;
+    if (tiles == 0)
       continue;
-    const int M = OP == OP_WG ? L.next_size : p->batch, N = OP == OP_FWD ? L.next_size : L.size;
-    mx = std::max(mx, N), my = std::max(my, M);
-    tiles += (long long)cdiv(M, 64) * cdiv(N, 64);
+    auto go = [&](auto kern, const TileList& T, int threads)
+    {
+      kern<<<T.start[c], threads, 0, p->ctx->stream>>>(p->d, T, p->n, p->batch, flags, mode, p->energy, epc_src);
+    };
+    // us, W = 4 / W = 2 / T = 64, by 32 x 32 tiles an SM:  0.9 (445 wide, batch 48) 16.5 / 24 / -,  1.4 (784 x 256
+    // weights) 31 / 26 / -,  3 (512 wide, batch 210) 25 / 22 / -,  3.7 (512 wide, batch 1089) 28 / 25 / -,  4.2 (403
+    // wide, batch 512: rows that are copied element by element, by twice the threads) 44 / 49 / 59, state 35 / 34 / 40,
+    // 7.3 (45 layers of 374 at batch 48, 1.8 tiles of 64 an SM) 51 / 43 / 36
+    if (4LL * tiles64 >= 7LL * sm)
+      go(pc_gemm_kernel<OP, 64, 4>, list[1], 128);
+    else if (tiles >= (OP == OP_WG ? sm : vec ? 3LL * sm : 6LL * sm))
+      go(pc_gemm_kernel<OP, 32, 2>, list[0], 64);
+    else
+      go(pc_gemm_kernel<OP, 32, 4>, list[0], 128);
+    const int rc = check_launch(p->ctx, "grouped GEMM kernel");
+    if (rc != DPC_OK)
+      return rc;
   }
-  if (tiles == 0)
-    return DPC_OK;
-  const int T = tiles < p->ctx->sm_count ? 32 : 64;
-  dim3 grid(cdiv(mx, T), cdiv(my, T), count);
-  auto kern = T == 32 ? pc_gemm_kernel<OP, 32> : pc_gemm_kernel<OP, 64>;
-  kern<<<grid, NTHREADS, 0, p->ctx->stream>>>(p->d, first, p->n, p->batch, flags, mode, p->energy, epc_src);
-  return check_launch(p->ctx, "grouped GEMM kernel");
+  return DPC_OK;
 }
 
 // Networks with an Adam-type optimizer or an activation with a kink turn a rounding difference into a whole

@@ -150,15 +150,15 @@ __device__ __forceinline__ void act_both(int act, float z, float& f, float& d)
   }
 }
 
-// Eight elements at once with ONE dispatch on the activation: with a run-time activation id the
+// N elements at once with ONE dispatch on the activation: with a run-time activation id the
 // per-element switch above costs a branch chain per element (a GEMM epilogue ran 3.5x slower with
-// it than with a compile-time activation); here the branch is taken once per eight elements.
-template <bool WITH_DERIV>
-__device__ __forceinline__ void act_both8(int act, const float (&z)[8], float (&f)[8], float (&d)[8])
+// it than with a compile-time activation); here the branch is taken once per N elements.
+template <bool WITH_DERIV, int N>
+__device__ __forceinline__ void act_many(int act, const float (&z)[N], float (&f)[N], float (&d)[N])
 {
-#define DPC_ACT8(A)                                        \
+#define DPC_ACT_N(A)                                        \
   case A:                                                  \
-    _Pragma("unroll") for (int q = 0; q < 8; ++q)          \
+    _Pragma("unroll") for (int q = 0; q < N; ++q)          \
     {                                                      \
       if (WITH_DERIV)                                      \
         act_both(A, z[q], f[q], d[q]);                     \
@@ -168,18 +168,18 @@ __device__ __forceinline__ void act_both8(int act, const float (&z)[8], float (&
     break;
   switch (act)
   {
-    DPC_ACT8(DPC_ACT_RELU)
-    DPC_ACT8(DPC_ACT_GELU)
-    DPC_ACT8(DPC_ACT_SIGMOID)
-    DPC_ACT8(DPC_ACT_ESIGMOID)
-    DPC_ACT8(DPC_ACT_TANH)
-    DPC_ACT8(DPC_ACT_HARD_TANH)
+    DPC_ACT_N(DPC_ACT_RELU)
+    DPC_ACT_N(DPC_ACT_GELU)
+    DPC_ACT_N(DPC_ACT_SIGMOID)
+    DPC_ACT_N(DPC_ACT_ESIGMOID)
+    DPC_ACT_N(DPC_ACT_TANH)
+    DPC_ACT_N(DPC_ACT_HARD_TANH)
   default:
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
+    for (int q = 0; q < N; ++q)
       f[q] = z[q], d[q] = 1.0f;
   }
-#undef DPC_ACT8
+#undef DPC_ACT_N
 }
 
 // f'(z) of four elements with one dispatch (a switch per element cost the head kernel of a simple

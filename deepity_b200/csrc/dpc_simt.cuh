@@ -9,16 +9,9 @@
 
 namespace dpc
 {
-constexpr int BK = 16, NTHREADS = 256;
+constexpr int NTHREADS = 256;
 
-enum GemmOp
-{
-  OP_FWD = 0, // mu = f(a z W^T + b)             M=B  N=next K=size
-  OP_FB = 1,  // z += ir (a fe W - e)            M=B  N=size K=next
-  OP_WG = 2   // W += alpha g^T zin              M=next N=size K=B
-};
-
-// mode of OP_WG
+// mode of a weight update
 enum
 {
   WG_LEARN = 0, // UpdateWeights: g = fe (or e_above for Simple), rate lr, optimizer
@@ -27,21 +20,6 @@ enum
   // update is applied later by apply_gradients_kernel (after a sum over batch shards)
   WG_GRAD_ONLY = 2
 };
-// mode of OP_FB
-enum
-{
-  FB_STATE = 0,  // UpdateState
-  FB_ADJOINT = 1 // ePC ComputeAdjoint + UpdateErrorEPC (fe holds src * f'(preact))
-};
-
-// Operand tiles of the grouped GEMM below in shared memory, filled by cp.async several K steps ahead.
-//   K-major  (rows are the M/N index, k contiguous in memory): [T][BK + 4], element (row, k); threads
-//            read 16 bytes along k of the rows t, t + 16, ..: a pitch of 20 floats puts the 16-byte
-//            reads of eight neighbouring rows into distinct banks
-//   MN-major ([K, cols], cols contiguous): [BK][T], threads read T / 16 neighbouring columns
-template <int T, bool KMAJOR>
-constexpr int kTileFloats = KMAJOR ? T * (BK + 4) : BK * T;
-
 __device__ __forceinline__ void cp_async4(float* dst, const float* src, bool valid)
 {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
@@ -54,53 +32,6 @@ __device__ __forceinline__ void cp_async16(float* dst, const float* src, bool va
                "l"(src), "r"(valid ? 16 : 0)
                : "memory");
 }
-
-// One 16-byte chunk of a tile (chunk index c < T * BK / 4); what lies outside the operand becomes zero.
-// vec: rows of the operand start on 16-byte boundaries and are multiples of four long.
-template <int J, typename F>
-__device__ __forceinline__ void tile_row(const float* p, F&& put)
-{
-  if (J == 4)
-  {
-    const float4 v = *reinterpret_cast<const float4*>(p);
-    put(0, v.x), put(1, v.y), put(J > 2 ? 2 : 0, v.z), put(J > 2 ? 3 : 0, v.w);
-  }
-  else
-  {
-    const float2 v = *reinterpret_cast<const float2*>(p);
-    put(0, v.x), put(1, v.y);
-  }
-}
-template <int T, bool KMAJOR>
-struct TileChunk
-{
-  int row, k;
-  __device__ __forceinline__ explicit TileChunk(int c)
-      : row(KMAJOR ? c / (BK / 4) : (c % (T / 4)) * 4), k(KMAJOR ? (c % (BK / 4)) * 4 : c / (T / 4))
-  {
-  }
-  __device__ __forceinline__ float* at(float* tile) const
-  {
-    return KMAJOR ? tile + row * (BK + 4) + k : tile + k * T + row;
-  }
-  __device__ __forceinline__ void load(float* tile, const float* __restrict__ G, int ld, int row0, int k0,
-                                       int nrows, int K, bool vec) const
-  {
-    float* dst = at(tile);
-    const int r = row0 + row, kk = k0 + k;
-    const bool in = r < nrows && kk < K;
-    const float* src = in ? (KMAJOR ? G + (size_t)r * ld + kk : G + (size_t)kk * ld + r) : G;
-    if (vec)
-    {
-      cp_async16(dst, src, in);
-      return;
-    }
-    const int left = KMAJOR ? K - kk : nrows - r;
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      cp_async4(dst + j, in && j < left ? src + j : G, in && j < left);
-  }
-};
 
 __device__ __forceinline__ bool aligned16(const void* p)
 {
@@ -242,7 +173,7 @@ __global__ void __launch_bounds__(NTHREADS)
             const float in[8] = {zv[r][i].x,     zv[r][i].y,     zv[r][i].z,     zv[r][i].w,
                                  zv[r][i + 1].x, zv[r][i + 1].y, zv[r][i + 1].z, zv[r][i + 1].w};
             float f[8], d[8];
-            act_both8<false>(L.act, in, f, d);
+            act_many<false>(L.act, in, f, d);
 #pragma unroll
             for (int q = 0; q < 2; ++q)
             {
@@ -361,355 +292,6 @@ __global__ void __launch_bounds__(NTHREADS)
   }
   if (flags & DPC_FWD_ENERGY)
     block_energy_add(do_err || do_ce ? esum : 0.0f, energy);
-}
-
-// ---------------------------------------------------------------------------------------
-// The grouped GEMM kernel.  OP selects operand layouts and the fused epilogue; T x T output tiles
-// (64: 4 x 4 outputs per thread, 32: 2 x 2 where 64 x 64 tiles would leave SMs idle), the operands
-// STAGES - 1 K steps ahead through cp.async.  Every output is one ascending sum over K whatever the
-// tile.  With one register-prefetched step the kernel waited for L2 in each of them: 784 -> 256 at
-// batch 256 took 67 us and takes 23 us now.
-// ---------------------------------------------------------------------------------------
-template <int OP, int T>
-__global__ void __launch_bounds__(NTHREADS)
-    pc_gemm_kernel(const dpc_layer* __restrict__ layers, int first, int n_layers, int batch,
-                   int flags, int mode, double* energy, const float* __restrict__ epc_src = nullptr)
-{
-  const int li = first + blockIdx.z;
-  const dpc_layer L = layers[li];
-  if (L.next_size <= 0)
-    return;
-  const bool simple = (L.flags & DPC_LAYER_INPUT_ACT) != 0;
-
-  int M, N, K;
-  if (OP == OP_FWD)
-    M = batch, N = L.next_size, K = L.size;
-  else if (OP == OP_FB)
-    M = batch, N = L.size, K = L.next_size;
-  else
-    M = L.next_size, N = L.size, K = batch;
-  const int m0 = blockIdx.y * T, n0 = blockIdx.x * T;
-  if (m0 >= M || n0 >= N)
-    return;
-  const bool wg_stage = OP == OP_WG && (mode & WG_GRAD_ONLY);
-  if (OP == OP_WG)
-    mode &= ~WG_GRAD_ONLY;
-  if (OP == OP_WG && mode == WG_DFA)
-  {
-    // DirectFeedbackUpdate is a no-op unless the layer above owns feedback weights.
-    if (li + 1 >= n_layers || layers[li + 1].Psi == nullptr)
-      return;
-  }
-
-  const dpc_layer* Lup = (li + 1 < n_layers) ? &layers[li + 1] : nullptr;
-  const float* A;
-  const float* Bm;
-  int lda, ldb;
-  if (OP == OP_FWD)
-    A = L.z, lda = L.size, Bm = L.W, ldb = L.size;
-  else if (OP == OP_FB)
-    A = (simple && mode == FB_STATE) ? Lup->e : L.fe, lda = L.next_size, Bm = L.W, ldb = L.size;
-  else
-    A = (simple && mode == WG_LEARN) ? Lup->e : L.fe, lda = L.next_size,
-    Bm = simple ? L.zF : L.z, ldb = L.size;
-
-  constexpr bool A_K = OP != OP_WG, B_K = OP == OP_FWD; // K-major operands
-  constexpr int J = T / 16, STAGES = T == 64 ? 4 : 8;
-  constexpr int CHUNKS = T * BK / 4, PER = CHUNKS / NTHREADS; // 16-byte chunks per operand, per thread
-  __shared__ __align__(16) float tile_a[STAGES][kTileFloats<T, A_K>];
-  __shared__ __align__(16) float tile_b[STAGES][kTileFloats<T, B_K>];
-  const bool vecA = aligned16(A) && (lda % 4 == 0);
-  const bool vecB = aligned16(Bm) && (ldb % 4 == 0);
-  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-  // T = 64: a chunk of both operands per thread; T = 32: half of the threads load each operand
-  const bool loads_a = PER > 0 || t < CHUNKS, loads_b = PER > 0 || t >= NTHREADS - CHUNKS;
-  const TileChunk<T, A_K> chunk_a(t % CHUNKS);
-  const TileChunk<T, B_K> chunk_b(t % CHUNKS);
-  auto load = [&](int k0, int slot)
-  {
-    if (k0 < K)
-    {
-      if (loads_a)
-        chunk_a.load(tile_a[slot], A, lda, m0, k0, M, K, vecA);
-      if (loads_b)
-        chunk_b.load(tile_b[slot], Bm, ldb, n0, k0, N, K, vecB);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-
-  float acc[J][J];
-#pragma unroll
-  for (int i = 0; i < J; ++i)
-#pragma unroll
-    for (int j = 0; j < J; ++j)
-      acc[i][j] = 0.0f;
-
-#pragma unroll
-  for (int q = 0; q < STAGES - 1; ++q)
-    load(q * BK, q);
-  int slot = 0;
-  for (int k0 = 0; k0 < K; k0 += BK)
-  {
-    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
-    if (OP == OP_FWD && simple && loads_a)
-    {
-      // SimplePC: the operand is f(z), kept as last fed to the GEMM for the weight update
-      // (src/layers/SimplePCLayer.cpp:146-150); each thread transforms what it copied
-      float* a = chunk_a.at(tile_a[slot]);
-      const int r = m0 + chunk_a.row, k = k0 + chunk_a.k;
-      if (r < M && k < K)
-      {
-        float4 v = *reinterpret_cast<const float4*>(a);
-        v.x = act_fwd(L.act, v.x);
-        v.y = k + 1 < K ? act_fwd(L.act, v.y) : 0.0f;
-        v.z = k + 2 < K ? act_fwd(L.act, v.z) : 0.0f;
-        v.w = k + 3 < K ? act_fwd(L.act, v.w) : 0.0f;
-        *reinterpret_cast<float4*>(a) = v;
-        if (blockIdx.x == 0 && L.zF != nullptr)
-        {
-          float* zf = L.zF + (size_t)r * L.size + k;
-          if (vecA && aligned16(L.zF))
-            *reinterpret_cast<float4*>(zf) = v;
-          else
-          {
-            zf[0] = v.x;
-            if (k + 1 < K)
-              zf[1] = v.y;
-            if (k + 2 < K)
-              zf[2] = v.z;
-            if (k + 3 < K)
-              zf[3] = v.w;
-          }
-        }
-      }
-    }
-    __syncthreads(); // the step has landed, and everybody is done with the slot that is refilled now
-    load(k0 + (STAGES - 1) * BK, slot == 0 ? STAGES - 1 : slot - 1);
-    const float* ta = tile_a[slot];
-    const float* tb = tile_b[slot];
-#pragma unroll
-    for (int k = 0; k < BK; k += 4)
-    {
-      float a[J][4], b[4][J];
-#pragma unroll
-      for (int i = 0; i < J; ++i)
-        if (A_K)
-        {
-          const float4 v = *reinterpret_cast<const float4*>(ta + (ty + 16 * i) * (BK + 4) + k);
-          a[i][0] = v.x, a[i][1] = v.y, a[i][2] = v.z, a[i][3] = v.w;
-        }
-#pragma unroll
-      for (int j = 0; j < J; ++j)
-        if (B_K)
-        {
-          const float4 v = *reinterpret_cast<const float4*>(tb + (tx + 16 * j) * (BK + 4) + k);
-          b[0][j] = v.x, b[1][j] = v.y, b[2][j] = v.z, b[3][j] = v.w;
-        }
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-      {
-        if (!A_K)
-          tile_row<J>(ta + (k + q) * T + ty * J, [&](int i, float v) { a[i][q] = v; });
-        if (!B_K)
-          tile_row<J>(tb + (k + q) * T + tx * J, [&](int j, float v) { b[q][j] = v; });
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int i = 0; i < J; ++i)
-#pragma unroll
-          for (int j = 0; j < J; ++j)
-            acc[i][j] = fmaf(a[i][q], b[q][j], acc[i][j]);
-    }
-    slot = slot + 1 == STAGES ? 0 : slot + 1;
-  }
-  // output (i, j) of this thread
-  auto out_m = [&](int i) { return m0 + (A_K ? ty + 16 * i : ty * J + i); };
-  auto out_n = [&](int j) { return n0 + (B_K ? tx + 16 * j : tx * J + j); };
-
-  // ------------------------------------------------------------------ epilogues
-  float esum = 0.0f;
-  if (OP == OP_FWD)
-  {
-    const bool next_ce = Lup && (Lup->flags & DPC_LAYER_SOFTMAX_CE);
-    const bool do_err = (flags & DPC_FWD_ERR_NEXT) && Lup && !next_ce;
-    const bool do_fe = (flags & DPC_FWD_FE) && Lup && !simple && !(next_ce && (flags & DPC_FWD_ERR_NEXT));
-    const bool do_copy = (flags & DPC_FWD_COPY_NEXT) && Lup;
-#pragma unroll
-    for (int i = 0; i < J; ++i)
-    {
-      const int m = out_m(i);
-      if (m >= M)
-        continue;
-#pragma unroll
-      for (int j = 0; j < J; ++j)
-      {
-        const int n = out_n(j);
-        if (n >= N)
-          continue;
-        const size_t o = (size_t)m * N + n;
-        const float pre = L.a * acc[i][j] + L.b[n];
-        float mu, d = 1.0f;
-        if (simple)
-          mu = pre;
-        else
-        {
-          if (do_fe)
-            act_both(L.act, pre, mu, d);
-          else
-            mu = act_fwd(L.act, pre);
-          if (L.flags & DPC_LAYER_RESIDUAL)
-            mu += L.z[o];
-        }
-        if (!(flags & DPC_FWD_TRANSIENT))
-        {
-          const bool no_mu = do_copy && (flags & DPC_FWD_NO_MU);
-          if (L.preact && !(no_mu && (flags & DPC_FWD_NO_PREACT)))
-            L.preact[o] = pre;
-          if (!no_mu)
-            L.mu[o] = mu;
-        }
-        if (do_copy)
-          Lup->z[o] = mu;
-        float e = 0.0f;
-        if (do_err)
-        {
-          e = (do_copy ? mu : Lup->z[o]) - mu;
-          Lup->e[o] = e;
-          esum += e * e;
-        }
-        else if (do_fe)
-          e = Lup->e[o];
-        if (do_fe)
-          L.fe[o] = e * d;
-      }
-    }
-    if (flags & DPC_FWD_ENERGY)
-      block_energy_add(do_err ? esum : 0.0f, energy);
-  }
-  else if (OP == OP_FB)
-  {
-#pragma unroll
-    for (int i = 0; i < J; ++i)
-    {
-      const int m = out_m(i);
-      if (m >= M)
-        continue;
-#pragma unroll
-      for (int j = 0; j < J; ++j)
-      {
-        const int n = out_n(j);
-        if (n >= N)
-          continue;
-        const size_t o = (size_t)m * N + n;
-        if (mode == FB_ADJOINT)
-        {
-          // ePC: adjoint of this layer and the error update driven by it.  `flags` carries the
-          // hop scale (+1 or -1) as float bits with bit 0 replaced by the clamp flag.
-          const float scale = __int_as_float(flags & ~1);
-          const bool clamped = flags & 1;
-          float adj = (L.a * scale) * acc[i][j];
-          if (L.flags & DPC_LAYER_RESIDUAL)
-            adj += scale * epc_src[o];
-          L.adj[o] = adj;
-          if (!clamped)
-            L.e[o] = (1.0f - L.ir) * L.e[o] - L.ir * adj;
-          continue;
-        }
-        float z = L.z[o];
-        if (simple)
-        {
-          z += L.ir * (acc[i][j] * act_deriv(L.act, z) - L.e[o]);
-        }
-        else
-        {
-          const float fb = L.a * acc[i][j] - L.e[o];
-          if (L.v)
-          {
-            const float v = L.momentum_beta * L.v[o] + (1.0f - L.momentum_beta) * fb;
-            L.v[o] = v;
-            z += L.ir * v;
-          }
-          else
-            z += L.ir * fb;
-          if (L.flags & DPC_LAYER_RESIDUAL)
-            z += L.ir * Lup->e[o];
-        }
-        L.z[o] = z;
-      }
-    }
-  }
-  else
-  {
-    if (wg_stage)
-    {
-#pragma unroll
-      for (int i = 0; i < J; ++i)
-      {
-        const int m = out_m(i);
-#pragma unroll
-        for (int j = 0; j < J; ++j)
-        {
-          const int n = out_n(j);
-          if (m < M && n < N)
-            L.g_W[(size_t)m * N + n] = acc[i][j];
-        }
-      }
-      return;
-    }
-    const float Bf = (float)batch;
-    const bool adam = (mode == WG_LEARN) && (L.opt != DPC_OPT_SGD);
-    float alpha, decay = 1.0f, step = 0.0f, lr_wd = -1.0f;
-    if (mode == WG_DFA)
-    {
-      alpha = L.fl * L.a / Bf;
-      if ((flags & 1) && L.lmbda > 0.0f && L.fl != 0.0f)
-        decay = 1.0f - L.lmbda;
-    }
-    else if (!adam)
-    {
-      alpha = simple ? (L.lr / Bf) : (L.a * L.lr / Bf);
-      if (L.lmbda > 0.0f)
-        decay = 1.0f - L.lmbda;
-    }
-    else
-    {
-      alpha = -1.0f * L.a;
-      step = adam_step_size(L.lr, *L.t);
-      if (L.opt == DPC_OPT_ADAMW)
-        lr_wd = L.lr * L.lmbda;
-    }
-#pragma unroll
-    for (int i = 0; i < J; ++i)
-    {
-      const int m = out_m(i);
-      if (m >= M)
-        continue;
-#pragma unroll
-      for (int j = 0; j < J; ++j)
-      {
-        const int n = out_n(j);
-        if (n >= N)
-          continue;
-        const size_t o = (size_t)m * N + n;
-        float w = L.W[o];
-        if (!adam)
-        {
-          if (decay != 1.0f)
-            w *= decay;
-          w = fmaf(alpha, acc[i][j], w);
-        }
-        else
-        {
-          float mm = L.m_W[o], vv = L.v_W[o];
-          w = adam_update(w, alpha * acc[i][j], mm, vv, step, lr_wd);
-          L.m_W[o] = mm;
-          L.v_W[o] = vv;
-        }
-        L.W[o] = w;
-      }
-    }
-  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1512,7 +1094,7 @@ __global__ void __launch_bounds__(256)
 // product has a K of 10: the tiled kernel spends its time on tile bookkeeping.  Here lane l of
 // every warp keeps the weights of columns 4l..4l+3 in registers, a block owns 128 columns and
 // `rows_per_block` batch rows, warp w the rows w, w+8, ...; the rows of the feedback error go
-// through shared memory 128 at a time.  Same arithmetic per element as pc_gemm_kernel<OP_FB>.
+// through shared memory 128 at a time.  Same arithmetic per element as GemmEpilogue::state.
 template <int KC>
 __global__ void __launch_bounds__(256)
     narrow_state_kernel(const dpc_layer* __restrict__ layers, int first, int n_layers, int batch,
@@ -1614,8 +1196,7 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// One entry of a weight update from the raw sum over the batch (the epilogue of
-// pc_gemm_kernel<OP_WG> for one element).
+// One entry of a weight update from the raw sum over the batch.
 __device__ __forceinline__ void weight_apply(const dpc_layer& L, size_t o, float sum, int batch,
                                              int mode, int flags, bool simple, float step)
 {

@@ -493,9 +493,9 @@ __device__ __forceinline__ void fwd_epilogue_tile(const TcParams& P, const FwdMe
       for (int q = 0; q < 8; ++q)
         pre[q] = L.a * v[k + q] + bb[q];
       if (do_fe)
-        act_both8<true>(act, pre, mu, d);
+        act_many<true>(act, pre, mu, d);
       else
-        act_both8<false>(act, pre, mu, d);
+        act_many<false>(act, pre, mu, d);
       if (residual && active)
       {
         float zz[8];
@@ -1225,7 +1225,7 @@ __global__ void __launch_bounds__(Cfg<OP, BN, THREE_X, BM, PAIR, KS>::THREADS, 1
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                   z8[i] = zz[k + i];
-                act_both8<true>(L.act, z8, f8, d8);
+                act_many<true>(L.act, z8, f8, d8);
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                   zz[k + i] += L.ir * (v[k + i] * d8[i] - ee[k + i]);
@@ -1250,7 +1250,7 @@ __global__ void __launch_bounds__(Cfg<OP, BN, THREE_X, BM, PAIR, KS>::THREADS, 1
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                   z8[i] = zz[k + i];
-                act_both8<false>(L.act, z8, f8, d8);
+                act_many<false>(L.act, z8, f8, d8);
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                   zz[k + i] = f8[i];
@@ -1853,7 +1853,7 @@ __global__ void split_planes_kernel(const dpc_layer* __restrict__ layers, int fi
     {
       const float in[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
       float f[8], d[8];
-      act_both8<false>(L.act, in, f, d);
+      act_many<false>(L.act, in, f, d);
       a = make_float4(f[0], f[1], f[2], f[3]), b = make_float4(f[4], f[5], f[6], f[7]);
     }
     uint4 h, m;
@@ -2890,7 +2890,7 @@ __global__ void input_activation_kernel(const dpc_layer* __restrict__ layers, in
     const float4 z = *reinterpret_cast<const float4*>(L.z + i);
     const float in[8] = {z.x, z.y, z.z, z.w, 0.0f, 0.0f, 0.0f, 0.0f};
     float f[8], d[8];
-    act_both8<false>(L.act, in, f, d);
+    act_many<false>(L.act, in, f, d);
     *reinterpret_cast<float4*>(L.zF + i) = make_float4(f[0], f[1], f[2], f[3]);
   }
 }

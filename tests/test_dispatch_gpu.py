@@ -31,8 +31,12 @@ GROUPED = {
     # 32 x 32 tiles: one row over a tile, K not a multiple of the stage, rows not 16-byte aligned
     "gemm_32_edges": _case("dkp", [33, 65, 31, 10], 65),
     "gemm_32_aligned": _case("simple", [64, 96, 32, 4], 32, mode="projection"),
-    # as many 64 x 64 tiles as SMs and more
     "gemm_64_edges": _case("dkp", [67, 641, 12], 961),
+    # ordered sums: blocks of four warps, of two (three tiles an SM and more), 64 x 64 tiles (1.75 an SM and more)
+    "gemm_four_warps": _case("full", [37, 45, 45, 6], 33, "relu", residual=1, momentum=0.9),
+    "gemm_two_warps": _case("simple", [64, 512, 512, 8], 961, "relu"),
+    "gemm_64_ordered": _case("dkp", [35, 1030, 1025, 6], 1100, "relu", T=2, steps=1),
+    "gemm_adamw": _case("dkp", [35, 66, 65, 6], 70, lr=1e-3, optimizer="ADAMW"),
     # the head kernels: partial groups of rows, one and two rows per warp, 16 units, softmax in the head
     "head_ce": _case("full", [40, 128, 10], 301, "gelu", cross_entropy=1),
     "head_ce_two_rows": _case("full", [40, 132, 16], 2051, cross_entropy=1),
