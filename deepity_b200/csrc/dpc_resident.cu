@@ -257,6 +257,80 @@ __device__ __forceinline__ void dot_rows(const float* __restrict__ w, const floa
       out[r * pitch] = acc[r];
 }
 
+// The same for the input layer's rows, which may be long.  A lane's sum is one chain over its row, and each batch of
+// loads costs the latency of L2 (1000 cycles): 16 loads in flight, 32 where they are single elements (32 rows of 1971
+// elements that are not 16-byte aligned 108 -> 33 us).  A function that is called: its registers are not the loop's.
+template <int RT>
+__device__ __noinline__ void dot_input(const float* __restrict__ w, const float* x, int S, int len,
+                                       float* out, int pitch, bool valid, bool vec)
+{
+  float acc[RT];
+#pragma unroll
+  for (int r = 0; r < RT; ++r)
+    acc[r] = 0.0f;
+  auto quads = [&](auto count, int k)
+  {
+    constexpr int C = decltype(count)::value;
+    float4 wv[C];
+#pragma unroll
+    for (int q = 0; q < C; ++q)
+      wv[q] = *reinterpret_cast<const float4*>(w + k + 4 * q);
+#pragma unroll
+    for (int q = 0; q < C; ++q)
+#pragma unroll
+      for (int r = 0; r < RT; ++r)
+      {
+        const float4 v = *reinterpret_cast<const float4*>(x + r * S + k + 4 * q);
+        acc[r] = fmaf(v.x, wv[q].x, acc[r]);
+        acc[r] = fmaf(v.y, wv[q].y, acc[r]);
+        acc[r] = fmaf(v.z, wv[q].z, acc[r]);
+        acc[r] = fmaf(v.w, wv[q].w, acc[r]);
+      }
+  };
+  auto singles = [&](auto count, int k)
+  {
+    constexpr int C = decltype(count)::value;
+    float wv[C];
+#pragma unroll
+    for (int q = 0; q < C; ++q)
+      wv[q] = w[k + q];
+#pragma unroll
+    for (int q = 0; q < C; ++q)
+#pragma unroll
+      for (int r = 0; r < RT; ++r)
+        acc[r] = fmaf(x[r * S + k + q], wv[q], acc[r]);
+  };
+  int k = 0;
+  if (vec)
+  {
+#pragma unroll 1
+    for (; k + 64 <= len; k += 64)
+      quads(std::integral_constant<int, 16>(), k);
+#pragma unroll 1
+    for (; k + 16 <= len; k += 16)
+      quads(std::integral_constant<int, 4>(), k);
+#pragma unroll 1
+    for (; k < len; k += 4)
+      quads(std::integral_constant<int, 1>(), k);
+  }
+  else
+  {
+#pragma unroll 1
+    for (; k + 32 <= len; k += 32)
+      singles(std::integral_constant<int, 32>(), k);
+#pragma unroll 1
+    for (; k + 8 <= len; k += 8)
+      singles(std::integral_constant<int, 8>(), k);
+#pragma unroll 1
+    for (; k < len; ++k)
+      singles(std::integral_constant<int, 1>(), k);
+  }
+  if (valid)
+#pragma unroll
+    for (int r = 0; r < RT; ++r)
+      out[r * pitch] = acc[r];
+}
+
 // One state task: sums over `len` rows of W for this lane's KW columns.
 template <int RT, int KW, int UNROLL>
 __device__ __forceinline__ void state_sum(float (&acc)[RT][KW], const float* w, int ldw, int len,
@@ -533,7 +607,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
           for (int t = warp; t < (L.N + 31) / 32 * RBS; t += kWarps)
           {
             const int c = t / RBS * 32 + lane, rb = t % RBS * RT;
-            dot_rows<RT>(sW[0] + (size_t)min(c, L.N - 1) * L.K, X + rb * P.K0p, P.K0p, L.K,
+            dot_input<RT>(sW[0] + (size_t)min(c, L.N - 1) * L.K, X + rb * P.K0p, P.K0p, L.K,
                          part + (c / G) * V + rb * G + c % G, G, c < L.N, L.vec != 0);
           }
         }

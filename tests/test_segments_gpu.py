@@ -38,6 +38,9 @@ ROWS = {
     # ordered sums (Adam-type optimizers, kinked activations) with streamed rows
     "exact_adamw": _case("dkp", [100, 300, 200, 77, 10], 50, "relu", optimizer="ADAMW", psi_optimizer="ADAM"),
     "exact_hard_tanh": _case("simple", [30, 129, 65, 3], 151, "hard_tanh"),
+    # ... over input rows that end inside each of the load groups
+    "exact_input_quads": _case("dkp", [84, 33, 9], 3, "relu"),
+    "exact_input_singles": _case("dkp", [107, 33, 9], 601, "relu"),
     # every term of the state update, more layers than warps share evenly
     "residual_momentum": _case("full", [33] + [64] * 9 + [10], 5, "gelu", mupc=1, residual=1, momentum=0.9),
     "cross_entropy": _case("full", [45, 61, 32, 17], 149, "tanh", cross_entropy=1),
