@@ -40,7 +40,7 @@ __device__ __forceinline__ float4 rows_cluster_load4(const float* own, uint32_t 
   return v;
 }
 
-__global__ void __launch_bounds__(32 * BP_WARPS, 3)
+__global__ void __launch_bounds__(32 * BP_WARPS, 2)
     batch_product_kernel(const dpc_layer* __restrict__ layers, const __grid_constant__ BatchTiles T,
                          int n_layers, int batch, int flags, int mode, const float* __restrict__ eT)
 {
@@ -108,6 +108,25 @@ __global__ void __launch_bounds__(32 * BP_WARPS, 3)
 #pragma unroll
   for (int q = 0; q < BP_STAGES - 1; ++q)
     load(g0 + q * stride, q);
+  // What this thread will update -- a quad of outputs, row q / 8, columns 4 (q % 8).., of its CTA's share of the
+  // tile, and a bias -- fetched while the sums are formed.
+  const int share = 32 * BP_WARPS / (int)R, q = (int)rank * share + (int)threadIdx.x;
+  const int m = m0 + (q >> 3), n = n0 + (q & 7) * 4;
+  const bool mine = (int)threadIdx.x < share && m < M && n < N, grad_only = (mode & WG_GRAD_ONLY) != 0;
+  const bool my_bias = bias && rank == 0 && threadIdx.x < BP_T && m0 + (int)threadIdx.x < M;
+  const bool vec = N % 4 == 0 && aligned16(L.W) && aligned16(L.g_W);
+  float old[4] = {}, old_bias = 0.0f;
+  if (mine && !grad_only)
+  {
+    if (!psi)
+      load4(old, L.W + (size_t)m * N + n, vec, N - n);
+    else
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        old[j] = n + j < N ? L.Psi[(size_t)(n + j) * L.psi_stride + m] : 0.0f;
+  }
+  if (my_bias && !grad_only)
+    old_bias = L.b[m0 + threadIdx.x];
   int slot = 0;
   for (int g = g0; g < groups; g += stride)
   {
@@ -164,33 +183,29 @@ __global__ void __launch_bounds__(32 * BP_WARPS, 3)
   if (bias)
     bpart[warp * BP_T + lane] = bsum;
   __syncthreads();
-  int q = threadIdx.x; // quad of outputs: row q / 8, columns 4 (q % 8)..
-  float4 s = *reinterpret_cast<const float4*>(sm + 4 * q);
+  const int busy = min(BP_WARPS, groups - (int)rank * BP_WARPS); // warps that had rows
+  float4 s = *reinterpret_cast<const float4*>(sm + 4 * threadIdx.x);
 #pragma unroll
   for (int w = 1; w < BP_WARPS; ++w)
-  {
-    const float4 v = *reinterpret_cast<const float4*>(sm + w * TILE + 4 * q);
-    s.x += v.x, s.y += v.y, s.z += v.z, s.w += v.w;
-  }
+    if (w < busy)
+    {
+      const float4 v = *reinterpret_cast<const float4*>(sm + w * TILE + 4 * threadIdx.x);
+      s.x += v.x, s.y += v.y, s.z += v.z, s.w += v.w;
+    }
   float bs = 0.0f;
   if (bias && threadIdx.x < BP_T)
-#pragma unroll
-    for (int w = 0; w < BP_WARPS; ++w)
+    for (int w = 0; w < busy; ++w)
       bs += bpart[w * BP_T + threadIdx.x];
-  bool mine = true;
   if (R > 1)
   {
-    *reinterpret_cast<float4*>(cta + 4 * q) = s;
+    *reinterpret_cast<float4*>(cta + 4 * threadIdx.x) = s;
     if (bias && threadIdx.x < BP_T)
       cta[TILE + threadIdx.x] = bs;
     rows_cluster_sync();
-    // every CTA finishes its share of the tile; the first one the bias too
-    const int share = 32 * BP_WARPS / (int)R;
-    mine = q < share;
-    if (mine)
+    // every CTA finishes its share of the tile; the first one the bias too (all loads before the first use)
+    if ((int)threadIdx.x < share)
     {
-      q += (int)rank * share;
-      float4 v[8]; // (all loads before the first use)
+      float4 v[8];
 #pragma unroll
       for (int r = 0; r < 8; ++r)
         if (r < (int)R)
@@ -215,28 +230,45 @@ __global__ void __launch_bounds__(32 * BP_WARPS, 3)
     }
     rows_cluster_sync(); // nobody leaves while its sums may still be read
   }
-  if (bias && rank == 0 && threadIdx.x < BP_T && m0 + (int)threadIdx.x < M)
-    bias_apply(L, m0 + threadIdx.x, bs, batch, mode & WG_GRAD_ONLY);
-  const int m = m0 + (q >> 3), n = n0 + (q & 7) * 4;
-  if (!mine || m >= M || n >= N)
+  // (every optimizer of these networks is SGD)
+  const float Bf = (float)batch;
+  if (my_bias)
+    (grad_only ? L.g_b : L.b)[m0 + threadIdx.x] = grad_only ? bs : old_bias + (L.lr / Bf) * bs;
+  if (!mine)
     return;
-  const float sv[4] = {s.x, s.y, s.z, s.w};
-  if (psi)
+  float out[4] = {s.x, s.y, s.z, s.w};
+  if (!grad_only)
   {
-    const bool full_kind = (L.flags & DPC_LAYER_FULLPC_PSI) != 0;
-    const int grad_only = mode & WG_GRAD_ONLY;
-    const float rate = full_kind ? L.fl * L.a : L.fl, step = psi_step(L, rate, grad_only);
+    float rate, decay;
+    if (psi)
+    {
+      const bool full_kind = (L.flags & DPC_LAYER_FULLPC_PSI) != 0;
+      rate = (full_kind ? L.fl * L.a : L.fl) / Bf;
+      decay = !full_kind && L.psi_decay > 0.0f ? 1.0f - L.psi_decay : 1.0f;
+    }
+    else if (mode == WG_DFA)
+    {
+      rate = L.fl * L.a / Bf;
+      decay = (flags & 1) && L.lmbda > 0.0f && L.fl != 0.0f ? 1.0f - L.lmbda : 1.0f;
+    }
+    else
+    {
+      rate = simple ? L.lr / Bf : L.a * L.lr / Bf;
+      decay = L.lmbda > 0.0f ? 1.0f - L.lmbda : 1.0f;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      out[j] = fmaf(rate, out[j], old[j] * decay);
+  }
+  if (!psi)
+    store4((grad_only ? L.g_W : L.W) + (size_t)m * N + n, out, vec, N - n);
+  else
+  {
+    float* dst = grad_only ? L.g_Psi : L.Psi;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (n + j < N)
-        psi_apply(L, n + j, m, sv[j], batch, grad_only, full_kind, rate, step);
-    return;
+        dst[(size_t)(n + j) * L.psi_stride + m] = out[j];
   }
-  const float step = mode == WG_LEARN && L.opt != DPC_OPT_SGD ? adam_step_size(L.lr, *L.t) : 0.0f;
-  const size_t o = (size_t)m * N + n;
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-    if (n + j < N)
-      weight_apply(L, o + j, sv[j], batch, mode, flags, simple, step);
 }
 } // namespace dpc
