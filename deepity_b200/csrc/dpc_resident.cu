@@ -395,18 +395,23 @@ __device__ __forceinline__ void put4(float* p, const float (&v)[4])
 {
   *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
 }
-// Sum of `slices` partial sums, four neighbours at once, in slice order.
+// Sum of `slices` partial sums, four neighbours at once, in slice order; four slices are read at a time.
 __device__ __forceinline__ void sum4(float (&v)[4], const float* p, int slices, int stride)
 {
   get4(v, p);
-#pragma unroll 3
-  for (int s = 1; s < slices; ++s)
+#pragma unroll 1
+  for (int s = 1; s < slices; s += 4)
   {
-    float t[4];
-    get4(t, p + s * stride);
+    float t[4][4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      v[j] += t[j];
+    for (int q = 0; q < 4; ++q)
+      get4(t[q], p + min(s + q, slices - 1) * stride);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (s + q < slices)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          v[j] += t[q][j];
   }
 }
 // Activation and derivative of four values with one dispatch.
@@ -431,21 +436,25 @@ __device__ __forceinline__ void act4(int act, const float (&z)[4], float (&f)[4]
   }
 #undef DPC_ACT4
 }
-// f'(z) of four values whose f(z) is known.
+// f'(z) of four values whose f(z) is known, with one dispatch (one per value was a quarter of the elementwise
+// phase of a state update).
 __device__ __forceinline__ void deriv4(int act, const float (&z)[4], const float (&f)[4], float (&d)[4])
 {
-  if (act_has_output_deriv(act))
+#define DPC_DERIV4(A)                                                                             \
+  case A:                                                                                         \
+    _Pragma("unroll") for (int j = 0; j < 4; ++j) d[j] = act_deriv_from_output(A, f[j]);          \
+    break;
+  switch (act)
   {
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      d[j] = act_deriv_from_output(act, f[j]);
+    DPC_DERIV4(DPC_ACT_TANH)
+    DPC_DERIV4(DPC_ACT_SIGMOID)
+    DPC_DERIV4(DPC_ACT_RELU)
+    DPC_DERIV4(DPC_ACT_LINEAR)
+    DPC_DERIV4(DPC_ACT_HARD_TANH)
+  default:
+    act_deriv4(act, z, d);
   }
-  else
-  {
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      d[j] = act_deriv(act, z[j]);
-  }
+#undef DPC_DERIV4
 }
 
 struct LayerConst // what a finished sum of layer l needs, one 16-byte read
