@@ -186,6 +186,90 @@ __device__ __forceinline__ void dot_streamed(float (&acc)[R * G], const float* _
     }
 }
 
+// Partial sums of the input layer, read once a segment from L2: tasks of G outputs x R rows x a slice of K, lanes
+// along K, the loads of two strips (four of single elements) in flight together.  A function that is called: its
+// registers are not the loop's.
+template <int R, int G>
+__device__ __noinline__ void input_sums(const float* __restrict__ W, int K, int N, const float* X, int xs, int slices,
+                                        int slice, float* part, int warp, int lane, bool vec)
+{
+  constexpr int V = R * G, LPV = 32 / V;
+  for (int t = warp; t < (N + G - 1) / G * slices; t += kWarps)
+  {
+    const int g0 = t / slices * G, k0 = (t - t / slices * slices) * slice, k1 = min(K, k0 + slice);
+    const float* row[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+      row[g] = W + (size_t)min(g0 + g, N - 1) * K;
+    float acc[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+      acc[i] = 0.0f;
+    auto strips = [&](auto width, auto count, int k) // `count` strips of 32 `width` elements from k
+    {
+      constexpr int E = decltype(width)::value, C = decltype(count)::value;
+      float w[C][G][E];
+#pragma unroll
+      for (int q = 0; q < C; ++q)
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+          if constexpr (E == 4)
+          {
+            const float4 v = *reinterpret_cast<const float4*>(row[g] + k + q * 128);
+            w[q][g][0] = v.x, w[q][g][1] = v.y, w[q][g][2] = v.z, w[q][g][3] = v.w;
+          }
+          else
+            w[q][g][0] = row[g][k + q * 32];
+#pragma unroll
+      for (int q = 0; q < C; ++q)
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+        {
+          float v[E];
+          const float* x = X + r * xs + k + q * 32 * E;
+          if constexpr (E == 4)
+          {
+            const float4 t4 = *reinterpret_cast<const float4*>(x);
+            v[0] = t4.x, v[1] = t4.y, v[2] = t4.z, v[3] = t4.w;
+          }
+          else
+            v[0] = *x;
+#pragma unroll
+          for (int g = 0; g < G; ++g)
+#pragma unroll
+            for (int j = 0; j < E; ++j)
+              acc[r * G + g] = fmaf(v[j], w[q][g][j], acc[r * G + g]);
+        }
+    };
+    using std::integral_constant;
+    if (vec)
+    {
+      int k = k0 + lane * 4;
+      if (V < 32) // (else the sums take the registers)
+#pragma unroll 1
+        for (; k + 128 < k1; k += 256)
+          strips(integral_constant<int, 4>(), integral_constant<int, 2>(), k);
+#pragma unroll 1
+      for (; k < k1; k += 128)
+        strips(integral_constant<int, 4>(), integral_constant<int, 1>(), k);
+    }
+    else
+    {
+      int k = k0 + lane;
+#pragma unroll 1
+      for (; k + 96 < k1; k += 128)
+        strips(integral_constant<int, 1>(), integral_constant<int, 4>(), k);
+#pragma unroll 1
+      for (; k < k1; k += 32)
+        strips(integral_constant<int, 1>(), integral_constant<int, 1>(), k);
+    }
+    __syncwarp();
+    const float v = reduce_values<V>(acc, lane);
+    if (lane % LPV == 0)
+      part[t * V + lane / LPV] = v;
+  }
+}
+
 // Resident weights: this lane's output over `len` inputs (walked four at a time, zero-padded).
 template <int RT>
 __device__ __forceinline__ void dot_resident(const float* w, const float* x, int S, int len, float* out,
@@ -459,8 +543,10 @@ __device__ __forceinline__ void deriv4(int act, const float (&z)[4], const float
 
 struct LayerConst // what a finished sum of layer l needs, one 16-byte read
 {
-  float a, ir;
-  int act, residual;
+  float a, ir, beta;
+  int kind; // activation, | 256: residual
+  __device__ __forceinline__ int act() const { return kind & 255; }
+  __device__ __forceinline__ bool residual() const { return (kind & 256) != 0; }
 };
 
 template <int R>
@@ -501,7 +587,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
   {
     const dpc_layer& L = P.layers[l];
     sW[l] = L.W;
-    lc[l] = LayerConst{L.a, L.ir, L.act, (L.flags & DPC_LAYER_RESIDUAL) ? 1 : 0};
+    lc[l] = LayerConst{L.a, L.ir, L.momentum_beta, L.act | ((L.flags & DPC_LAYER_RESIDUAL) ? 256 : 0)};
   }
   __syncthreads();
   for (int l = 1; l < nw; ++l)
@@ -576,7 +662,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
                   f[j] = 0.0f;
                 }
                 if (simple && l < nw)
-                  act4(lc[l].act, z, f, d);
+                  act4(lc[l].act(), z, f, d);
                 const int t = r * S + 4 * i;
                 put4(Z + t, z);
                 put4(E + t, e);
@@ -600,7 +686,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
               v = D.z[o];
               if (simple)
               {
-                v = act_fwd(lc[0].act, v);
+                v = act_fwd(lc[0].act(), v);
                 D.zF[o] = v;
               }
             }
@@ -608,7 +694,6 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
           }
         __syncthreads();
         float* part = X + R * P.K0p;
-        const int ng = (L.N + G - 1) / G, nt = ng * P.ks0;
         if (P.exact && !L.lanes_k)
         {
           // one ascending sum per output: lane = output
@@ -621,20 +706,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
           }
         }
         else
-          for (int t = warp; t < nt; t += kWarps)
-          {
-            const int g0 = (t / P.ks0) * G, s = t % P.ks0;
-            const int k0 = s * P.kslice0, k1 = min(L.K, k0 + P.kslice0);
-            float acc[V];
-#pragma unroll
-            for (int i = 0; i < V; ++i)
-              acc[i] = 0.0f;
-            dot_streamed<R, G>(acc, sW[0] + (size_t)g0 * L.K, L.K, L.N - g0, X, P.K0p, k0, k1, lane,
-                               L.vec != 0);
-            const float v = reduce_values<V>(acc, lane);
-            if (lane % LPV == 0)
-              part[t * V + lane / LPV] = v;
-          }
+          input_sums<R, G>(sW[0], L.K, L.N, X, P.K0p, P.ks0, P.kslice0, part, warp, lane, L.vec != 0);
         __syncthreads();
         for (int i = tid; i < R * L.N; i += kThreads)
         {
@@ -645,7 +717,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
           const float pre = lc[0].a * v + bias[L.noff + c];
           float mu = pre, d = 1.0f;
           if (!simple)
-            act_both(lc[0].act, pre, mu, d); // (a residual layer is never the first)
+            act_both(lc[0].act(), pre, mu, d); // (a residual layer is never the first)
           mu0[r * P.N1p + c] = mu;
           d0[r * P.N1p + c] = d;
           if (r < rows)
@@ -663,7 +735,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
           const int r = i / L.N, c = i - r * L.N;
           const size_t o = (size_t)(row0 + r) * L.N + c;
           mu0[r * P.N1p + c] = r < rows ? D.mu[o] : 0.0f;
-          d0[r * P.N1p + c] = (r < rows && !simple) ? act_deriv(lc[0].act, D.preact[o]) : 1.0f;
+          d0[r * P.N1p + c] = (r < rows && !simple) ? act_deriv(lc[0].act(), D.preact[o]) : 1.0f;
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -747,8 +819,8 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
             mu[j] = pre[j], d[j] = 1.0f;
         else
         {
-          act4(C.act, pre, mu, d);
-          if (C.residual)
+          act4(C.act(), pre, mu, d);
+          if (C.residual())
           {
             float z[4];
             get4(z, Z + r * S + q.down);
@@ -841,7 +913,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
             if (simple && l + 1 < nw)
             {
               float f4[4], d4[4];
-              act4(lc[l + 1].act, mu, f4, d4);
+              act4(lc[l + 1].act(), mu, f4, d4);
               put4(Gb + o, f4);
             }
           }
@@ -960,7 +1032,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
                   {
                     float f[4], d[4];
                     get4(f, Gb + o);
-                    deriv4(C.act, z, f, d);
+                    deriv4(C.act(), z, f, d);
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
                       z[j] += C.ir * (dz[j] * d[j] - e[j]);
@@ -973,7 +1045,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
                       fb[j] = C.a * dz[j] - e[j];
                     if (P.has_v)
                     {
-                      const float beta = P.layers[l].momentum_beta;
+                      const float beta = C.beta;
                       float v[4];
                       get4(v, Vb + o);
 #pragma unroll
@@ -981,13 +1053,13 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
                         fb[j] = beta * v[j] + (1.0f - beta) * fb[j];
                       put4(Vb + o, fb);
                     }
-                    if (C.residual)
+                    if (C.residual())
                       get4(u, E + r * S + q.up);
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
                     {
                       z[j] += C.ir * fb[j];
-                      if (C.residual)
+                      if (C.residual())
                         z[j] += C.ir * u[j];
                     }
                   }
@@ -999,7 +1071,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const ResParams P
                   if (refresh_f)
                   {
                     float f[4], d[4];
-                    act4(C.act, z, f, d);
+                    act4(C.act(), z, f, d);
                     put4(Gb + o, f);
                   }
                 });
