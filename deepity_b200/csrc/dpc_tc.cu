@@ -1893,7 +1893,17 @@ int launch(dpc_plan* p, TcState* st, const CUtensorMap& a, const CUtensorMap& b,
   {
     // one cluster of two CTAs per work item, as many clusters as SM pairs (the sweep: one
     // cluster per tile, all of them resident at once)
-    const int pairs = P.chain ? P.tiles_m * P.tiles_n : std::min(total, p->ctx->sm_count / 2);
+    int pairs = P.chain ? P.tiles_m * P.tiles_n : std::min(total, p->ctx->sm_count / 2);
+    if (!P.chain && !C::PRE)
+    {
+      // No more pairs than the number of waves needs: 192 tiles take three on 64 pairs as on 74, and the SMs that are
+      // left run the head and the cached input of the phase meanwhile (3072-(1024x4)-10 with Adam at batch 4096 8.10 ->
+      // 8.00 ms a step, 512-(512x12)-10 tf32 474 -> 459 us).  Not the kernels on operand planes, which wait for L2
+      // rather than for their own SM: with the head's traffic beside them all the time 784-(1024x4)-10 took 5.04 ms
+      // instead of 5.00.
+      const int waves = (total + pairs - 1) / pairs;
+      pairs = (total + waves - 1) / waves;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);
     cfg.blockDim = dim3(C::THREADS);
