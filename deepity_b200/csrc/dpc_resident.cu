@@ -9,8 +9,8 @@
 // from L2), beliefs, errors and gated errors of its rows in shared memory, no launch and no global
 // traffic inside the settling loop, only barriers of the CTA.
 //
-// Measured: 784-128-128-10 at batch 64, 20 steps, 879 -> 125 us a step (about 3 us a settling pass, bound
-// by issue slots and the two barriers of a pass); ordered sums with streamed weights, 100-300-200-77-10
+// Measured: 784-128-128-10 at batch 64, 20 steps, 879 -> 113 us a step (about 2.5 us a settling pass: 1600 and
+// 900 cycles of sums, two elementwise phases of 1000 that are chains of latencies); ordered sums with streamed weights, 100-300-200-77-10
 // at batch 50 with AdamW, 6 steps, 750 -> 183 us.
 //
 // A pass is a list of warp tasks that leave partial sums in shared memory, a barrier, and an
