@@ -75,12 +75,22 @@ class LayerView:
 
 class DevicePointer(int):
     """An address in a network's device memory that keeps the network alive: views made from it (through
-    __cuda_array_interface__, say) must not outlive the memory."""
+    __cuda_array_interface__, say) must not outlive the memory.  ``int(pointer)`` is the bare number, which keeps
+    nothing alive; so is what a pickle holds."""
 
     def __new__(cls, value: int, owner):
         self = super().__new__(cls, value)
         self.owner = owner
         return self
+
+    def __copy__(self):
+        return self
+
+    def __deepcopy__(self, memo):
+        return self
+
+    def __reduce__(self):
+        return int, (int(self),)
 
 
 class _Network:

@@ -80,3 +80,18 @@ def test_all_device_work_is_ordered_on_a_stream_of_the_library():
                 depth -= c in ")]}"
                 args += c == "," and depth == 0
             assert args == 4, (name, launch)
+
+
+def test_device_pointers_copy_and_pickle_like_integers():
+    """An address, or a table of addresses, can be copied (the copy keeps the network alive too) and pickled (what
+    comes back is the bare number)."""
+    import copy
+    import pickle
+    from deepity_b200.networks import DevicePointer
+    owner = object()
+    ptr = DevicePointer(4096, owner)
+    for got in (copy.copy(ptr), copy.deepcopy(ptr), copy.deepcopy({"W": ptr})["W"]):
+        assert got == 4096 and got.owner is owner
+    for protocol in range(pickle.HIGHEST_PROTOCOL + 1):
+        assert type(pickle.loads(pickle.dumps({"W": ptr}, protocol))["W"]) is int
+        assert pickle.loads(pickle.dumps(ptr, protocol)) == 4096
