@@ -22,9 +22,8 @@ constexpr int BP_SLOT = 2 * BP_ROWS * BP_T; // floats: rows of g, rows of z
 
 struct BatchTiles
 {
-  TileList list;
-  unsigned weights[kListLayers / 32]; // a bit per layer: its weight sums are among them ...
-  int bias;                           // ... and its bias sums
+  TileList list; // kind: the weight sums of these layers are among them ...
+  int sums;      // ... and their bias sums, and the Psi sums of all layers
 };
 
 __device__ __forceinline__ float4 rows_cluster_load4(const float* own, uint32_t rank)
@@ -46,12 +45,20 @@ __global__ void __launch_bounds__(32 * BP_WARPS, 2)
 {
   const uint32_t R = rows_cluster_size(), rank = rows_cluster_rank();
   int t = (int)(blockIdx.x / R);
-  const int li = tile_layer(T.list, t), rel = li - T.list.first;
+  bool weights;
+  const int li = tile_layer(T.list, t, weights);
   const dpc_layer L = layers[li];
   const bool simple = (L.flags & DPC_LAYER_INPUT_ACT) != 0;
   const int base_mode = mode & ~WG_GRAD_ONLY;
   const int N = L.size, nt = (N + BP_T - 1) / BP_T;
-  const int mt = (T.weights[rel >> 5] >> (rel & 31) & 1) ? (L.next_size + BP_T - 1) / BP_T : 0;
+  const int mt = weights ? (L.next_size + BP_T - 1) / BP_T : 0;
+  if (T.list.padded)
+  {
+    // (a layer with fewer tiles than its run, or none; all CTAs of the cluster)
+    const int pt = T.sums && L.Psi && !simple ? (L.terminal_size + BP_T - 1) / BP_T : 0;
+    if (L.next_size <= 0 || t >= (mt + pt) * nt || (base_mode == WG_DFA && !(li + 1 < n_layers && layers[li + 1].Psi)))
+      return;
+  }
   int m0 = t / nt;
   const int n0 = (t - m0 * nt) * BP_T;
   const bool psi = m0 >= mt;
@@ -60,7 +67,7 @@ __global__ void __launch_bounds__(32 * BP_WARPS, 2)
   const float* A = psi ? eT : simple && base_mode == WG_LEARN ? layers[li + 1].e : L.fe;
   const float* B = simple ? L.zF : L.z;
   const bool vecA = aligned16(A) && M % 4 == 0, vecB = aligned16(B) && N % 4 == 0;
-  const bool bias = T.bias && !psi && n0 == 0;
+  const bool bias = T.sums && !psi && n0 == 0;
 
   __shared__ __align__(16) float sm[BP_WARPS * BP_STAGES * BP_SLOT];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

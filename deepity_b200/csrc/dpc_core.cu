@@ -87,46 +87,94 @@ static inline int cdiv(int a, int b)
   return (a + b - 1) / b;
 }
 
-// A product of layers [first, first+count) in one launch (per 128 layers).
+// The tiles of layers [first, end), of which layer i has tiles(i) of kind(i); end becomes the first layer that is left
+// for another launch, which a network takes only where it has more runs than a list and layers of both kinds.
+template <typename Tiles, typename Kind>
+static int list_tiles(TileList& T, int first, int& end, Tiles tiles, Kind kind)
+{
+  T.first = first, T.layers = end - first, T.runs = T.padded = 0;
+  auto run = [&](int start, int per, int layer, bool k)
+  {
+    // (runs without tiles are never looked up)
+    T.run[T.runs++] = TileRun{start, per, per > 0 ? ~0u / per : 0u, (unsigned short)(layer - first), (unsigned short)k};
+  };
+  int total = 0;
+  for (int i = first; i < end; ++i)
+  {
+    const int n = tiles(i);
+    const bool k = kind(i);
+    if (T.runs == 0 || n != T.run[T.runs - 1].per || k != (T.run[T.runs - 1].kind != 0))
+    {
+      if (T.runs == kListRuns)
+        break;
+      run(total, n, i, k);
+    }
+    total += n;
+    if (i + 1 == end)
+      return total;
+  }
+  // one run of the largest number, as far as the kind stays the same
+  int most = 0, stop = first;
+  for (; stop < end && kind(stop) == kind(first); ++stop)
+  {
+    const int m = std::max(most, tiles(stop));
+    if (stop > first && (long long)m * (stop + 1 - first) > (1 << 27)) // (blocks of a launch, clusters of eight)
+      break;
+    most = m;
+  }
+  T.layers = stop - first, T.runs = 0, T.padded = 1;
+  run(0, most, first, kind(first));
+  end = stop;
+  return most * (stop - first);
+}
+
+// A product of layers [first, first+count) in one launch.
 template <int OP>
 static int launch_gemm(dpc_plan* p, int first, int count, int flags, int mode, const float* epc_src = nullptr)
 {
-  for (int f = first; f < first + count; f += kListLayers)
+  const int sm = p->ctx->sm_count;
+  auto tiles_of = [&](int i, int T)
   {
-    TileList list[2] = {}; // tiles of 32 and of 64
-    bool vec = true;       // rows can be copied 16 bytes at a time
-    for (int s = 0; s < 2; ++s)
-    {
-      TileList& T = list[s];
-      T.first = f, T.count = std::min(kListLayers, first + count - f);
-      for (int i = 0; i < T.count; ++i)
-      {
-        const dpc_layer& L = p->h[f + i];
-        const int M = OP == OP_WG ? L.next_size : p->batch, N = OP == OP_FWD ? L.next_size : L.size;
-        // (DirectFeedbackUpdate is a no-op unless the layer above owns feedback weights)
-        const bool any = L.next_size > 0 && (OP != OP_WG || (mode & ~WG_GRAD_ONLY) != WG_DFA ||
-                                             (f + i + 1 < p->n && p->h[f + i + 1].Psi));
-        T.start[i + 1] = T.start[i] + (any ? cdiv(M, 32 << s) * cdiv(N, 32 << s) : 0);
-        vec &= L.size % 4 == 0 && L.next_size % 4 == 0;
-      }
-    }
-    const int c = list[0].count, tiles = list[0].start[c], tiles64 = list[1].start[c], sm = p->ctx->sm_count;
-    if (tiles == 0)
+    const dpc_layer& L = p->h[i];
+    const int M = OP == OP_WG ? L.next_size : p->batch, N = OP == OP_FWD ? L.next_size : L.size;
+    // (DirectFeedbackUpdate is a no-op unless the layer above owns feedback weights)
+    const bool any = L.next_size > 0 && (OP != OP_WG || (mode & ~WG_GRAD_ONLY) != WG_DFA ||
+                                         (i + 1 < p->n && p->h[i + 1].Psi));
+    return any ? cdiv(M, T) * cdiv(N, T) : 0;
+  };
+  long long tiles = 0, tiles64 = 0;
+  bool vec = true; // rows can be copied 16 bytes at a time
+  for (int i = first; i < first + count; ++i)
+  {
+    tiles += tiles_of(i, 32), tiles64 += tiles_of(i, 64);
+    vec &= p->h[i].size % 4 == 0 && p->h[i].next_size % 4 == 0;
+  }
+  // us, W = 4 / W = 2 / T = 64, by 32 x 32 tiles an SM:  0.9 (445 wide, batch 48) 16.5 / 24 / -,  1.4 (784 x 256
+  // weights) 31 / 26 / -,  3 (512 wide, batch 210) 25 / 22 / -,  3.7 (512 wide, batch 1089) 28 / 25 / -,  4.2 (403
+  // wide, batch 512: rows that are copied element by element, by twice the threads) 44 / 49 / 59, state 35 / 34 / 40,
+  // 7.3 (45 layers of 374 at batch 48, 1.8 tiles of 64 an SM) 51 / 43 / 36
+  // Not 64 x 64 where layers are narrower than that and most of a tile is padding (20 passes over 400 layers of 32 at
+  // batch 300 1440 / 1000 us a step on 64 x 64 / 32 x 32 tiles, 140 of 96 at batch 20 518 / 367).
+  const bool large = 4 * tiles64 >= 7LL * sm && 8 * tiles64 <= 3 * tiles;
+  const bool two_warps = tiles >= (OP == OP_WG ? sm : vec ? 3LL * sm : 6LL * sm);
+  for (int f = first, end; f < first + count; f = end)
+  {
+    TileList T;
+    end = first + count;
+    const int blocks = list_tiles(
+        T, f, end, [&](int i) { return tiles_of(i, large ? 64 : 32); }, [](int) { return false; });
+    if (blocks == 0)
       continue;
-    auto go = [&](auto kern, const TileList& T, int threads)
+    auto go = [&](auto kern, int threads)
     {
-      kern<<<T.start[c], threads, 0, p->ctx->stream>>>(p->d, T, p->n, p->batch, flags, mode, p->energy, epc_src);
+      kern<<<blocks, threads, 0, p->ctx->stream>>>(p->d, T, p->n, p->batch, flags, mode, p->energy, epc_src);
     };
-    // us, W = 4 / W = 2 / T = 64, by 32 x 32 tiles an SM:  0.9 (445 wide, batch 48) 16.5 / 24 / -,  1.4 (784 x 256
-    // weights) 31 / 26 / -,  3 (512 wide, batch 210) 25 / 22 / -,  3.7 (512 wide, batch 1089) 28 / 25 / -,  4.2 (403
-    // wide, batch 512: rows that are copied element by element, by twice the threads) 44 / 49 / 59, state 35 / 34 / 40,
-    // 7.3 (45 layers of 374 at batch 48, 1.8 tiles of 64 an SM) 51 / 43 / 36
-    if (4LL * tiles64 >= 7LL * sm)
-      go(pc_gemm_kernel<OP, 64, 4>, list[1], 128);
-    else if (tiles >= (OP == OP_WG ? sm : vec ? 3LL * sm : 6LL * sm))
-      go(pc_gemm_kernel<OP, 32, 2>, list[0], 64);
+    if (large)
+      go(pc_gemm_kernel<OP, 64, 4>, 128);
+    else if (two_warps)
+      go(pc_gemm_kernel<OP, 32, 2>, 64);
     else
-      go(pc_gemm_kernel<OP, 32, 4>, list[0], 128);
+      go(pc_gemm_kernel<OP, 32, 4>, 128);
     const int rc = check_launch(p->ctx, "grouped GEMM kernel");
     if (rc != DPC_OK)
       return rc;
@@ -1191,27 +1239,23 @@ static int launch_batch_products(dpc_plan* p, int first, int count, int mode, in
   bool tensor = p->run.count > 0;
   for (int i = 0; i < p->n && !tensor; ++i)
     tensor = tc_extra_layer(p, i);
-  for (int f = first; f < first + count; f += kListLayers)
+  for (int f = first, end; f < first + count; f = end)
   {
-    BatchTiles T = {};
-    T.bias = with_sums;
-    T.list.first = f, T.list.count = std::min(kListLayers, first + count - f);
-    for (int q = 0; q < T.list.count; ++q)
+    // DirectFeedbackUpdate is a no-op unless the layer above owns feedback weights
+    auto sums = [&](int i)
+    { return weights(i) && ((mode & ~WG_GRAD_ONLY) != WG_DFA || (i + 1 < p->n && p->h[i + 1].Psi)); };
+    auto tiles_of = [&](int i)
     {
-      const int i = f + q;
       const dpc_layer& L = p->h[i];
-      T.list.start[q + 1] = T.list.start[q];
-      if (L.next_size <= 0)
-        continue;
-      // DirectFeedbackUpdate is a no-op unless the layer above owns feedback weights
-      const bool w = weights(i) && ((mode & ~WG_GRAD_ONLY) != WG_DFA || (i + 1 < p->n && p->h[i + 1].Psi));
       const bool psi = with_sums && L.Psi && !(L.flags & DPC_LAYER_INPUT_ACT);
-      if (w)
-        T.weights[q / 32] |= 1u << (q % 32);
-      T.list.start[q + 1] +=
-          ((w ? cdiv(L.next_size, BP_T) : 0) + (psi ? cdiv(L.terminal_size, BP_T) : 0)) * cdiv(L.size, BP_T);
-    }
-    const int tiles = T.list.start[T.list.count];
+      return L.next_size <= 0 ? 0
+                              : ((sums(i) ? cdiv(L.next_size, BP_T) : 0) + (psi ? cdiv(L.terminal_size, BP_T) : 0)) *
+                                    cdiv(L.size, BP_T);
+    };
+    BatchTiles T;
+    T.sums = with_sums;
+    end = first + count;
+    const int tiles = list_tiles(T.list, f, end, tiles_of, weights);
     if (tiles == 0)
       continue;
     // CTAs of a cluster that share a tile's batch rows: two groups of rows or more for each warp; beside

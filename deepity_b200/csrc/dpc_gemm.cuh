@@ -17,27 +17,48 @@ enum
   FB_ADJOINT = 1 // ePC ComputeAdjoint + UpdateErrorEPC (fe holds src * f'(preact))
 };
 
-// The output tiles of a launch, layer by layer: start[i] is the first one of layer first + i.
-constexpr int kListLayers = 128;
+// The output tiles of a launch, as runs of neighbouring layers with equally many (deep networks have few: one for each
+// shape).  A range of more runs than the list holds is one run of the largest number instead, whose blocks return where
+// a layer has fewer tiles or none.
+struct TileRun
+{
+  int start, per;       // its first tile, tiles of a layer
+  unsigned inverse;     // (2^32 - 1) / per
+  unsigned short layer; // its first layer, from the list's
+  unsigned short kind;
+};
+constexpr int kListRuns = 240;
 struct TileList
 {
-  int first, count;
-  int start[kListLayers + 1];
+  int first, layers, runs;
+  int padded; // layers may have fewer tiles than their run
+  TileRun run[kListRuns];
 };
 // Layer of tile t, which becomes the index within the layer.
-__device__ __forceinline__ int tile_layer(const TileList& T, int& t)
+__device__ __forceinline__ int tile_layer(const TileList& T, int& t, bool& kind)
 {
+  if (T.layers == 1) // (the steps of a sweep, one short launch after another)
+  {
+    kind = T.run[0].kind != 0;
+    return T.first;
+  }
   int lo = 0;
-  for (int hi = T.count; hi - lo > 1;)
+  for (int hi = T.runs; hi - lo > 1;)
   {
     const int mid = (lo + hi) >> 1;
-    if (T.start[mid] <= t)
+    if (T.run[mid].start <= t)
       lo = mid;
     else
       hi = mid;
   }
-  t -= T.start[lo];
-  return T.first + lo;
+  const TileRun& r = T.run[lo];
+  t -= r.start;
+  int layer = (int)__umulhi((unsigned)t, r.inverse); // t / per or one less
+  t -= layer * r.per;
+  if (t >= r.per)
+    ++layer, t -= r.per;
+  kind = r.kind != 0;
+  return T.first + r.layer + layer;
 }
 
 // Four neighbouring values of a row, of which `left` exist.
@@ -364,7 +385,8 @@ __global__ void __launch_bounds__(32 * W, T == 32 ? 20 / W : 4)
   float* pre = sm + STAGES * C::SLOT;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int t = blockIdx.x;
-  const int li = tile_layer(list, t);
+  bool kind;
+  const int li = tile_layer(list, t, kind);
   const dpc_layer* Lup = li + 1 < n_layers ? &layers[li + 1] : nullptr;
   Epilogue E(layers[li], Lup, batch, flags, mode, epc_src);
   const dpc_layer& L = E.L;
@@ -376,7 +398,13 @@ __global__ void __launch_bounds__(32 * W, T == 32 ? 20 / W : 4)
   const float* B = OP != OP_WG ? L.W : E.simple ? L.zF : L.z;
   const int lda = OP == OP_FWD ? L.size : L.next_size, ldb = L.size;
   const bool vec_a = aligned16(A) && lda % 4 == 0, vec_b = aligned16(B) && ldb % 4 == 0;
-  const int nt = (N + T - 1) / T, m0 = t / nt * T, n0 = (t - t / nt * nt) * T;
+  const int nt = (N + T - 1) / T;
+  // (a layer with fewer tiles than its run, or none: DirectFeedbackUpdate is a no-op unless the layer above owns
+  // feedback weights)
+  if (list.padded && (L.next_size <= 0 || t >= (M + T - 1) / T * nt ||
+                      (OP == OP_WG && base_mode == WG_DFA && !(Lup && Lup->Psi))))
+    return;
+  const int m0 = t / nt * T, n0 = (t - t / nt * nt) * T;
 
   auto load = [&](int k0, int slot)
   {
