@@ -1292,13 +1292,36 @@ static int weight_sums_begin(dpc_plan* p, int first, int count, int mode)
   return tc_zf_need(p, first, count);
 }
 
+// Whether the weight sums of layers [first, first+count) outside the tensor-core path are left to pc_gemm_kernel in a
+// network whose sums may be split: where there are tiles for every SM several times over, no batch has to be split,
+// and 64 x 64 outputs take half the operand traffic of batch_product_kernel's 32 x 32 (which costs 1.3 us a tile and SM
+// however few the rows).  us a step, batch products / pc_gemm_kernel, by 32 x 32 tiles an SM and the 64 x 64 ones' area
+// over theirs:  5.6, 1.0 (784-999-10, batch 16, 500, 2100) 221 / 220, 334 / 371, 629 / 781;  8.0, 1.3 (24 layers of 200,
+// batch 16, 500) 302 / 291, 658 / 699;  10.8, 1.0 (100 layers of 128, batch 16, 500, 2100) 627 / 616, 1132 / 1096,
+// 2779 / 2735;  11.2, 1.09 (four layers of 736, batch 48, 500) 248 / 236, 703 / 719;  13.8, 1.0 (eight of 512, batch
+// 100, 2100) 389 / 381, 2339 / 2299;  20, 1.3 (60 of 200, batch 48, 500) 685 / 667, 1403 / 1444;  97, 1.0 (fourteen of
+// 1024, batch 16, 1000) 889 / 738, 7720 / 7380.
+static bool weights_by_gemm(dpc_plan* p, int first, int count)
+{
+  long long tiles = 0, tiles64 = 0;
+  for (int i = first; i < first + count; ++i)
+    if (p->h[i].next_size > 0 && !tc_piece(p, i))
+    {
+      const int M = p->h[i].next_size, N = p->h[i].size;
+      tiles += (long long)cdiv(M, 32) * cdiv(N, 32), tiles64 += (long long)cdiv(M, 64) * cdiv(N, 64);
+    }
+  return tiles >= 10LL * p->ctx->sm_count && (p->batch <= 64 || 80 * tiles64 <= 21 * tiles);
+}
+
 static int weight_gemm_simt(dpc_plan* p, int first, int count, int mode, int flags)
 {
   const int ready = weight_sums_begin(p, first, count, mode);
   if (ready != DPC_OK)
     return ready;
   if (!ordered_sums(p))
-    return launch_batch_products(p, first, count, mode, flags, [](int) { return true; }, false);
+    return weights_by_gemm(p, first, count)
+               ? launch_gemm<OP_WG>(p, first, count, flags, mode)
+               : launch_batch_products(p, first, count, mode, flags, [](int) { return true; }, false);
   for (int f = first; f < first + count; f += kMaxZ)
   {
     const int c = std::min(kMaxZ, first + count - f);
@@ -1554,13 +1577,13 @@ static std::vector<Job> learn_jobs(dpc_plan* p, int first, int count, int grad_o
   for (int i = first; i < first + count; ++i)
     if (tc_piece(p, i) && p->h[i].Psi && p->h[i].size % 128 == 0 && p->h[i].terminal_size <= 16)
       strips += p->h[i].size / 128;
-  const bool by_strips = strips >= 4LL * p->ctx->sm_count;
+  const bool by_strips = strips >= 4LL * p->ctx->sm_count, by_gemm = weights_by_gemm(p, first, count);
   auto sums = [=](int f, int c)
   {
-    for (int i = f; i < f + c; ++i)
+    for (int i = f; i < f + c && !by_gemm; ++i)
       if (const int rc = tc_piece(p, i) ? DPC_OK : weight_sums_begin(p, i, 1, mode))
         return rc;
-    return launch_batch_products(p, f, c, mode, 0, [=](int i) { return !tc_piece(p, i); }, true);
+    return launch_batch_products(p, f, c, mode, 0, [=](int i) { return !by_gemm && !tc_piece(p, i); }, true);
   };
   for (int i = first, j; i < first + count; i = j)
   {
@@ -1577,8 +1600,16 @@ static std::vector<Job> learn_jobs(dpc_plan* p, int first, int count, int grad_o
       if (by_strips)
         psi_jobs(p, f, c, grad_only, jobs);
     }
-    else if (by_strips)
-      jobs.push_back([=] { return sums(f, c); });
+    else
+    {
+      if (by_gemm)
+      {
+        jobs.insert(jobs.begin(), [=] { return simt(f, c); });
+        jobs.push_back([=] { return launch_bias_update(p, f, c, grad_only); });
+      }
+      if (by_strips)
+        jobs.push_back([=] { return sums(f, c); });
+    }
   }
   if (!by_strips)
     jobs.push_back([=] { return sums(first, count); });

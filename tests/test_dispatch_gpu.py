@@ -75,6 +75,42 @@ def test_batch_sums_match_oracle(name, built_library, monkeypatch):
     _check(BATCH_SUMS[name], name)
 
 
+def _tiles(case, width):
+    """Output tiles of the weight sums."""
+    up = lambda v: -(-v // width)  # noqa: E731
+    return sum(up(a) * up(b) for a, b in zip(case["sizes"], case["sizes"][1:]))
+
+
+# Ten 32 x 32 tiles an SM and more: the weight sums leave the batch products, with few rows or with outputs that fill
+# 64 x 64 tiles; Psi stays
+WIDE = {
+    "few_rows": (_case("dkp", [40, 700, 1001, 900, 10], 33, T=2), True),
+    "rows": (_case("full", [40, 896, 1022, 700, 10], 70, "gelu", T=2), True),
+    "simple": (_case("simple", [40, 896, 1022, 700, 10], 70, mode="projection", T=4), True),
+    "padded": (_case("dkp", [40, 710, 707, 711, 710, 10], 70, T=2), False),
+}
+
+
+@pytest.mark.parametrize("staged", [False, True])
+@pytest.mark.parametrize("name", sorted(WIDE))
+def test_weight_sums_of_wide_layers_match_oracle(name, staged, built_library):
+    import torch
+    from deepity_b200 import _lib
+    case, by_gemm = WIDE[name]
+    sm = torch.cuda.get_device_properties(0).multi_processor_count
+    assert _tiles(case, 32) >= 10 * sm
+    assert (4 * _tiles(case, 64) <= 1.05 * _tiles(case, 32) or case["batch"] <= 64) == by_gemm
+    compare_outputs(run_oracle(case), run_gpu(case, staged_gradients=staged), TOL, name,
+                    init=initial_parameters(case), delta_tol=DELTA_TOL)
+    net, x, y = build_gpu_net(case)
+    counts = []
+    for _ in range(2):
+        _lib.check(net._lib.dpc_update_weights(net._lib.dpcn_plan(net._h), 0, len(case["sizes"]), 0))
+        counts.append(net.launch_count)
+    psi = case["kind"] != "simple"
+    assert counts[1] - counts[0] == (2 + psi if by_gemm else 1)  # weights, biases, Psi
+
+
 @pytest.mark.parametrize("kind", ["simple", "full"])
 @pytest.mark.parametrize("act", ["tanh", "relu"])
 @pytest.mark.parametrize("widths", [[32], [40, 12]])
