@@ -41,7 +41,7 @@ __device__ __forceinline__ float4 rows_cluster_load4(const float* own, uint32_t 
 
 __global__ void __launch_bounds__(32 * BP_WARPS, 2)
     batch_product_kernel(const dpc_layer* __restrict__ layers, const __grid_constant__ BatchTiles T,
-                         int n_layers, int batch, int flags, int mode, const float* __restrict__ eT)
+                         int batch, int flags, int mode, const float* __restrict__ eT)
 {
   const uint32_t R = rows_cluster_size(), rank = rows_cluster_rank();
   int t = (int)(blockIdx.x / R);
@@ -52,13 +52,6 @@ __global__ void __launch_bounds__(32 * BP_WARPS, 2)
   const int base_mode = mode & ~WG_GRAD_ONLY;
   const int N = L.size, nt = (N + BP_T - 1) / BP_T;
   const int mt = weights ? (L.next_size + BP_T - 1) / BP_T : 0;
-  if (T.list.padded)
-  {
-    // (a layer with fewer tiles than its run, or none; all CTAs of the cluster)
-    const int pt = T.sums && L.Psi && !simple ? (L.terminal_size + BP_T - 1) / BP_T : 0;
-    if (L.next_size <= 0 || t >= (mt + pt) * nt || (base_mode == WG_DFA && !(li + 1 < n_layers && layers[li + 1].Psi)))
-      return;
-  }
   int m0 = t / nt;
   const int n0 = (t - m0 * nt) * BP_T;
   const bool psi = m0 >= mt;

@@ -88,16 +88,11 @@ static inline int cdiv(int a, int b)
 }
 
 // The tiles of layers [first, end), of which layer i has tiles(i) of kind(i); end becomes the first layer that is left
-// for another launch, which a network takes only where it has more runs than a list and layers of both kinds.
+// for another launch, where the layers are more runs than a list holds.
 template <typename Tiles, typename Kind>
 static int list_tiles(TileList& T, int first, int& end, Tiles tiles, Kind kind)
 {
-  T.first = first, T.layers = end - first, T.runs = T.padded = 0;
-  auto run = [&](int start, int per, int layer, bool k)
-  {
-    // (runs without tiles are never looked up)
-    T.run[T.runs++] = TileRun{start, per, per > 0 ? ~0u / per : 0u, (unsigned short)(layer - first), (unsigned short)k};
-  };
+  T.first = first, T.runs = 0;
   int total = 0;
   for (int i = first; i < end; ++i)
   {
@@ -106,26 +101,17 @@ static int list_tiles(TileList& T, int first, int& end, Tiles tiles, Kind kind)
     if (T.runs == 0 || n != T.run[T.runs - 1].per || k != (T.run[T.runs - 1].kind != 0))
     {
       if (T.runs == kListRuns)
+      {
+        end = i;
         break;
-      run(total, n, i, k);
+      }
+      T.start[T.runs] = total; // (runs without tiles are never looked up)
+      T.run[T.runs++] = TileRun{n, n > 0 ? ~0u / n : 0u, (unsigned short)(i - first), (unsigned short)k};
     }
     total += n;
-    if (i + 1 == end)
-      return total;
   }
-  // one run of the largest number, as far as the kind stays the same
-  int most = 0, stop = first;
-  for (; stop < end && kind(stop) == kind(first); ++stop)
-  {
-    const int m = std::max(most, tiles(stop));
-    if (stop > first && (long long)m * (stop + 1 - first) > (1 << 27)) // (blocks of a launch, clusters of eight)
-      break;
-    most = m;
-  }
-  T.layers = stop - first, T.runs = 0, T.padded = 1;
-  run(0, most, first, kind(first));
-  end = stop;
-  return most * (stop - first);
+  T.layers = end - first;
+  return total;
 }
 
 // A product of layers [first, first+count) in one launch.
@@ -1274,7 +1260,7 @@ static int launch_batch_products(dpc_plan* p, int first, int count, int mode, in
     attr[0].val.clusterDim = {(unsigned)R, 1, 1};
     cfg.attrs = attr;
     cfg.numAttrs = R > 1 ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, batch_product_kernel, (const dpc_layer*)p->d, T, p->n, p->batch, flags, mode,
+    cudaLaunchKernelEx(&cfg, batch_product_kernel, (const dpc_layer*)p->d, T, p->batch, flags, mode,
                        p->e_terminal);
     const int rc = check_launch(p->ctx, "batch product kernel");
     if (rc != DPC_OK)

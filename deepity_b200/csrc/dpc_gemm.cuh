@@ -18,11 +18,10 @@ enum
 };
 
 // The output tiles of a launch, as runs of neighbouring layers with equally many (deep networks have few: one for each
-// shape).  A range of more runs than the list holds is one run of the largest number instead, whose blocks return where
-// a layer has fewer tiles or none.
+// shape; 240 are 3.9 KB of parameters, which a launch takes as fast as 0.5 KB).
 struct TileRun
 {
-  int start, per;       // its first tile, tiles of a layer
+  int per;              // tiles of a layer
   unsigned inverse;     // (2^32 - 1) / per
   unsigned short layer; // its first layer, from the list's
   unsigned short kind;
@@ -31,7 +30,7 @@ constexpr int kListRuns = 240;
 struct TileList
 {
   int first, layers, runs;
-  int padded; // layers may have fewer tiles than their run
+  int start[kListRuns]; // of a run: its first tile
   TileRun run[kListRuns];
 };
 // Layer of tile t, which becomes the index within the layer.
@@ -46,13 +45,13 @@ __device__ __forceinline__ int tile_layer(const TileList& T, int& t, bool& kind)
   for (int hi = T.runs; hi - lo > 1;)
   {
     const int mid = (lo + hi) >> 1;
-    if (T.run[mid].start <= t)
+    if (T.start[mid] <= t)
       lo = mid;
     else
       hi = mid;
   }
   const TileRun& r = T.run[lo];
-  t -= r.start;
+  t -= T.start[lo];
   int layer = (int)__umulhi((unsigned)t, r.inverse); // t / per or one less
   t -= layer * r.per;
   if (t >= r.per)
@@ -399,11 +398,6 @@ __global__ void __launch_bounds__(32 * W, T == 32 ? 20 / W : 4)
   const int lda = OP == OP_FWD ? L.size : L.next_size, ldb = L.size;
   const bool vec_a = aligned16(A) && lda % 4 == 0, vec_b = aligned16(B) && ldb % 4 == 0;
   const int nt = (N + T - 1) / T;
-  // (a layer with fewer tiles than its run, or none: DirectFeedbackUpdate is a no-op unless the layer above owns
-  // feedback weights)
-  if (list.padded && (L.next_size <= 0 || t >= (M + T - 1) / T * nt ||
-                      (OP == OP_WG && base_mode == WG_DFA && !(Lup && Lup->Psi))))
-    return;
   const int m0 = t / nt * T, n0 = (t - t / nt * nt) * T;
 
   auto load = [&](int k0, int slot)

@@ -37,7 +37,7 @@ GROUPED = {
     "gemm_two_warps": _case("simple", [64, 512, 512, 8], 961, "relu"),
     "gemm_64_ordered": _case("dkp", [35, 1030, 1025, 6], 1100, "relu", T=2, steps=1),
     # more runs of layers of one shape than a launch lists
-    "gemm_many_shapes": _case("dkp", [16] + [40, 12] * 70 + [4], 33, "relu", T=2),
+    "gemm_many_shapes": _case("dkp", [16] + [40, 12] * 125 + [4], 33, "relu", T=2),
     "gemm_adamw": _case("dkp", [35, 66, 65, 6], 70, lr=1e-3, optimizer="ADAMW"),
     # the head kernels: partial groups of rows, one and two rows per warp, 16 units, softmax in the head
     "head_ce": _case("full", [40, 128, 10], 301, "gelu", cross_entropy=1),
@@ -63,7 +63,7 @@ BATCH_SUMS = {
     "edges": _case("dkp", [33, 65, 31, 40], 9),
     "clusters": _case("simple", [67, 31, 17], 1031, mode="projection"),
     "many_layers": _case("dkp", [16] + [12] * 130 + [4], 5, T=2),
-    "many_shapes": _case("dkp", [16] + [40, 12] * 70 + [4], 9, T=2),
+    "many_shapes": _case("dkp", [16] + [40, 12] * 125 + [4], 9, T=2),
     "beside_tensor_cores": _case("dkp", [64, 256, 256, 17], 256),
     "beside_tensor_cores_rows_split": _case("full", [72, 256, 256, 16], 1024, "gelu"),
 }
@@ -113,12 +113,12 @@ def test_weight_sums_of_wide_layers_match_oracle(name, staged, built_library):
 
 @pytest.mark.parametrize("kind", ["simple", "full"])
 @pytest.mark.parametrize("act", ["tanh", "relu"])
-@pytest.mark.parametrize("widths", [[32], [40, 12]])
-def test_a_phase_of_a_deep_network_is_as_many_launches_as_of_a_shallow_one(widths, act, kind, built_library,
-                                                                         monkeypatch):
+@pytest.mark.parametrize("widths,deep", [([32], 400), ([40, 12], 200)])
+def test_a_phase_of_a_deep_network_is_as_many_launches_as_of_a_shallow_one(widths, deep, act, kind,
+                                                                         built_library, monkeypatch):
     monkeypatch.setenv("DPC_DISABLE_RESIDENT", "1")
     passes = {}
-    for layers in (20, 300):
+    for layers in (20, deep):
         net, x, y = build_gpu_net(_case(kind, [64] + widths * (layers // len(widths)) + [10], 4, act), use_graph=False)
         counts = []
         for T in (2, 8):
@@ -127,7 +127,7 @@ def test_a_phase_of_a_deep_network_is_as_many_launches_as_of_a_shallow_one(width
             net.train_step(x, y, T)
             counts.append(net.launch_count - before)
         passes[layers] = counts[1] - counts[0]  # (of six settling passes: a sweep is a launch a layer)
-    assert passes[300] == passes[20] > 0
+    assert passes[deep] == passes[20] > 0
 
 
 PAIR = {
