@@ -15,8 +15,9 @@ namespace dpc
 // What bounds it: such a launch has few outputs and a batch of rows to walk, so it is the chain of row loads
 // and the shared-memory reads of one SM.  (A tile that walked the whole batch step by step with 2 x 2 outputs
 // per thread took 0.5 us per 16 rows, beside kernels of their own for bias and Psi.)  A step of 22 layers of 45
-// units at batch 2167 769 -> 590 us, of 784-(256x8)-10 at batch 256 302 -> 276; the learn phase of
-// 32-32-2 at batch 715 38 -> 7 us.
+// units at batch 2167 769 -> 560 us, of 784-(256x8)-10 at batch 256 302 -> 268; the learn phase of
+// 32-32-2 at batch 715 38 -> 6 us.  Weights of ten tiles an SM and more are left to pc_gemm_kernel (weights_by_gemm
+// in dpc_core.cu).
 constexpr int BP_T = 32, BP_ROWS = 8, BP_WARPS = 8, BP_STAGES = 3;
 constexpr int BP_SLOT = 2 * BP_ROWS * BP_T; // floats: rows of g, rows of z
 
