@@ -16,7 +16,7 @@ namespace dpc
 // and the shared-memory reads of one SM.  (A tile that walked the whole batch step by step with 2 x 2 outputs
 // per thread took 0.5 us per 16 rows, beside kernels of their own for bias and Psi.)  A step of 22 layers of 45
 // units at batch 2167 769 -> 560 us, of 784-(256x8)-10 at batch 256 302 -> 268; the learn phase of
-// 32-32-2 at batch 715 38 -> 6 us.  Weights of ten tiles an SM and more are left to pc_gemm_kernel (weights_by_gemm
+// 32-32-2 at batch 715 38 -> 6 us.  Weights of twelve tiles an SM and more are left to pc_gemm_kernel (weights_by_gemm
 // in dpc_core.cu).
 constexpr int BP_T = 32, BP_ROWS = 8, BP_WARPS = 8, BP_STAGES = 3;
 constexpr int BP_SLOT = 2 * BP_ROWS * BP_T; // floats: rows of g, rows of z

@@ -1284,8 +1284,9 @@ static int weight_sums_begin(dpc_plan* p, int first, int count, int mode)
 // however few the rows).  us a step, batch products / pc_gemm_kernel, by 32 x 32 tiles an SM and the 64 x 64 ones' area
 // over theirs:  5.6, 1.0 (784-999-10, batch 16, 500, 2100) 221 / 220, 334 / 371, 629 / 781;  8.0, 1.3 (24 layers of 200,
 // batch 16, 500) 302 / 291, 658 / 699;  10.8, 1.0 (100 layers of 128, batch 16, 500, 2100) 627 / 616, 1132 / 1096,
-// 2779 / 2735;  11.2, 1.09 (four layers of 736, batch 48, 500) 248 / 236, 703 / 719;  13.8, 1.0 (eight of 512, batch
-// 100, 2100) 389 / 381, 2339 / 2299;  20, 1.3 (60 of 200, batch 48, 500) 685 / 667, 1403 / 1444;  97, 1.0 (fourteen of
+// 2779 / 2735;  10.8, 1.0 (three of 865, SimplePC, batch 192) 606 / 617;  11.2, 1.09 (four layers of 736, batch 48,
+// 500) 248 / 236, 703 / 719;  13.8, 1.0 (eight of 512, batch 100,
+// 2100) 389 / 381, 2339 / 2299;  20, 1.3 (60 of 200, batch 48, 500) 685 / 667, 1403 / 1444;  97, 1.0 (fourteen of
 // 1024, batch 16, 1000) 889 / 738, 7720 / 7380.
 static bool weights_by_gemm(dpc_plan* p, int first, int count)
 {
@@ -1296,7 +1297,7 @@ static bool weights_by_gemm(dpc_plan* p, int first, int count)
       const int M = p->h[i].next_size, N = p->h[i].size;
       tiles += (long long)cdiv(M, 32) * cdiv(N, 32), tiles64 += (long long)cdiv(M, 64) * cdiv(N, 64);
     }
-  return tiles >= 10LL * p->ctx->sm_count && (p->batch <= 64 || 80 * tiles64 <= 21 * tiles);
+  return tiles >= 12LL * p->ctx->sm_count && (p->batch <= 64 || 80 * tiles64 <= 21 * tiles);
 }
 
 static int weight_gemm_simt(dpc_plan* p, int first, int count, int mode, int flags)
