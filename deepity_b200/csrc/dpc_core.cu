@@ -139,9 +139,14 @@ static int launch_gemm(dpc_plan* p, int first, int count, int flags, int mode, c
   // weights) 31 / 26 / -,  3 (512 wide, batch 210) 25 / 22 / -,  3.7 (512 wide, batch 1089) 28 / 25 / -,  4.2 (403
   // wide, batch 512: rows that are copied element by element, by twice the threads) 44 / 49 / 59, state 35 / 34 / 40,
   // 7.3 (45 layers of 374 at batch 48, 1.8 tiles of 64 an SM) 51 / 43 / 36
+  // 64 x 64 from six 32 x 32 tiles an SM already in forward products of SimplePC layers, which apply the activation to
+  // their operand once for each column of tiles (two layers of 256 and one of 100, batch 1500: 1480 / 1340 us a step of
+  // 20 passes with esigmoid, 1310 / 1260 with tanh; at batch 1400, 5.9 tiles an SM, 1060 / 1233).
   // Not 64 x 64 where layers are narrower than that and most of a tile is padding (20 passes over 400 layers of 32 at
   // batch 300 1440 / 1000 us a step on 64 x 64 / 32 x 32 tiles, 140 of 96 at batch 20 518 / 367).
-  const bool large = 4 * tiles64 >= 7LL * sm && 8 * tiles64 <= 3 * tiles;
+  const bool feeds = OP == OP_FWD && (p->h[first].flags & DPC_LAYER_INPUT_ACT);
+  const bool large =
+      (4 * tiles64 >= 7LL * sm || (feeds && tiles64 > sm && tiles > 6LL * sm)) && 8 * tiles64 <= 3 * tiles;
   const bool two_warps = tiles >= (OP == OP_WG ? sm : vec ? 3LL * sm : 6LL * sm);
   for (int f = first, end; f < first + count; f = end)
   {
@@ -1285,9 +1290,8 @@ static int weight_sums_begin(dpc_plan* p, int first, int count, int mode)
 // over theirs:  5.6, 1.0 (784-999-10, batch 16, 500, 2100) 221 / 220, 334 / 371, 629 / 781;  8.0, 1.3 (24 layers of 200,
 // batch 16, 500) 302 / 291, 658 / 699;  10.8, 1.0 (100 layers of 128, batch 16, 500, 2100) 627 / 616, 1132 / 1096,
 // 2779 / 2735;  10.8, 1.0 (three of 865, SimplePC, batch 192) 606 / 617;  11.2, 1.09 (four layers of 736, batch 48,
-// 500) 248 / 236, 703 / 719;  13.8, 1.0 (eight of 512, batch 100,
-// 2100) 389 / 381, 2339 / 2299;  20, 1.3 (60 of 200, batch 48, 500) 685 / 667, 1403 / 1444;  97, 1.0 (fourteen of
-// 1024, batch 16, 1000) 889 / 738, 7720 / 7380.
+// 500) 248 / 236, 703 / 719;  13.8, 1.0 (eight of 512, batch 100, 2100) 389 / 381, 2339 / 2299;  20, 1.3 (60 of 200,
+// batch 48, 500) 685 / 667, 1403 / 1444;  97, 1.0 (fourteen of 1024, batch 16, 1000) 889 / 738, 7720 / 7380.
 static bool weights_by_gemm(dpc_plan* p, int first, int count)
 {
   long long tiles = 0, tiles64 = 0;

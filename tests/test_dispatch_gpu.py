@@ -19,6 +19,26 @@ def _case(kind, sizes, batch, act="tanh", T=3, steps=2, mode="train_step", lr=0.
     return dict(kind=kind, sizes=sizes, batch=batch, T=T, steps=steps, hyper=hyper, options=options, mode=mode)
 
 
+def _sms():
+    import torch
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+def _up(a, b):
+    return -(-a // b)
+
+
+def _tiles(case, width, phase="weights"):
+    """Output tiles of the CUDA-core products of a phase: all weight sums; a settling pass (the input layer's prediction
+    is cached) or the state update of the hidden layers, without heads of 16 units and less, which are not theirs."""
+    sizes, batch = case["sizes"], case["batch"]
+    pairs = list(zip(sizes, sizes[1:]))
+    if phase == "weights":
+        return sum(_up(a, width) * _up(b, width) for a, b in pairs)
+    pairs = [(a, b) for a, b in pairs[1:] if b > 16]
+    return sum(_up(batch, width) * _up(b if phase == "forward" else a, width) for a, b in pairs)
+
+
 def _check(case, name, precision="fp32"):
     adam = "optimizer" in case["options"]
     tol = TF32_TOL if precision == "tf32" else (ADAM_TOL if adam else TOL)
@@ -55,6 +75,23 @@ def test_grouped_launches_match_oracle(name, built_library, monkeypatch):
     _check(GROUPED[name], name)
 
 
+# Forward products of SimplePC layers on 64 x 64 tiles, which transform their operand: from six 32 x 32 tiles an SM on,
+# rows that are 16-byte aligned, that are not, and K that ends inside a step
+FED = {
+    "aligned": _case("simple", [64, 256, 256, 252, 100], 1508, "esigmoid", T=4),
+    "unaligned": _case("simple", [33, 250, 255, 251, 101], 1507, "tanh", T=4),
+    "ordered": _case("simple", [64, 256, 250, 256, 68], 1508, "relu", T=4, mode="projection"),
+}
+
+
+@pytest.mark.parametrize("name", sorted(FED))
+def test_operands_of_large_tiles_are_transformed(name, built_library, monkeypatch):
+    monkeypatch.setenv("DPC_DISABLE_RESIDENT", "1")
+    case = FED[name]
+    assert _tiles(case, 32, "forward") > 6 * _sms() and _sms() < _tiles(case, 64, "forward") < 1.75 * _sms()
+    _check(case, name)
+
+
 # Sums over the batch: fewer rows than a group, one over it, rows split over clusters; 16 and 17 rows in a tile;
 # more terminal units than a tile; deep networks, of more
 # shapes than a launch lists too; Psi sums of tensor-core layers among others
@@ -75,12 +112,6 @@ def test_batch_sums_match_oracle(name, built_library, monkeypatch):
     _check(BATCH_SUMS[name], name)
 
 
-def _tiles(case, width):
-    """Output tiles of the weight sums."""
-    up = lambda v: -(-v // width)  # noqa: E731
-    return sum(up(a) * up(b) for a, b in zip(case["sizes"], case["sizes"][1:]))
-
-
 # Twelve 32 x 32 tiles an SM and more: the weight sums leave the batch products, with few rows or with outputs that fill
 # 64 x 64 tiles; Psi stays
 WIDE = {
@@ -94,11 +125,9 @@ WIDE = {
 @pytest.mark.parametrize("staged", [False, True])
 @pytest.mark.parametrize("name", sorted(WIDE))
 def test_weight_sums_of_wide_layers_match_oracle(name, staged, built_library):
-    import torch
     from deepity_b200 import _lib
     case, by_gemm = WIDE[name]
-    sm = torch.cuda.get_device_properties(0).multi_processor_count
-    assert _tiles(case, 32) >= 12 * sm
+    assert _tiles(case, 32) >= 12 * _sms()
     assert (4 * _tiles(case, 64) <= 1.05 * _tiles(case, 32) or case["batch"] <= 64) == by_gemm
     compare_outputs(run_oracle(case), run_gpu(case, staged_gradients=staged), TOL, name,
                     init=initial_parameters(case), delta_tol=DELTA_TOL)
