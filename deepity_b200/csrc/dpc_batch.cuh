@@ -232,34 +232,17 @@ __global__ void __launch_bounds__(32 * BP_WARPS, 2)
     rows_cluster_sync(); // nobody leaves while its sums may still be read
   }
   // (every optimizer of these networks is SGD)
-  const float Bf = (float)batch;
   if (my_bias)
-    (grad_only ? L.g_b : L.b)[m0 + threadIdx.x] = grad_only ? bs : old_bias + (L.lr / Bf) * bs;
+    (grad_only ? L.g_b : L.b)[m0 + threadIdx.x] = grad_only ? bs : bias_sgd(L, batch)(old_bias, bs);
   if (!mine)
     return;
   float out[4] = {s.x, s.y, s.z, s.w};
   if (!grad_only)
   {
-    float rate, decay;
-    if (psi)
-    {
-      const bool full_kind = (L.flags & DPC_LAYER_FULLPC_PSI) != 0;
-      rate = (full_kind ? L.fl * L.a : L.fl) / Bf;
-      decay = !full_kind && L.psi_decay > 0.0f ? 1.0f - L.psi_decay : 1.0f;
-    }
-    else if (mode == WG_DFA)
-    {
-      rate = L.fl * L.a / Bf;
-      decay = (flags & 1) && L.lmbda > 0.0f && L.fl != 0.0f ? 1.0f - L.lmbda : 1.0f;
-    }
-    else
-    {
-      rate = simple ? L.lr / Bf : L.a * L.lr / Bf;
-      decay = L.lmbda > 0.0f ? 1.0f - L.lmbda : 1.0f;
-    }
+    const Sgd update = psi ? psi_sgd(L, batch) : weight_sgd(L, batch, mode == WG_DFA, (flags & 1) != 0);
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      out[j] = fmaf(rate, out[j], old[j] * decay);
+      out[j] = update(old[j], out[j]);
   }
   if (!psi)
     store4((grad_only ? L.g_W : L.W) + (size_t)m * N + n, out, vec, N - n);

@@ -185,8 +185,6 @@ struct GemmEpilogue
     return energy;
   }
 
-  // (roundings of the updates below are spelled out where the compiler has a choice of which product to fuse:
-  // an Adam-type update of a near-zero gradient is sensitive to them)
   __device__ __forceinline__ void state(int m, int n, const float (&sum)[4], const float (&x)[kPre][4]) const
   {
     const size_t o = (size_t)m * N + n;
@@ -271,8 +269,10 @@ struct GemmEpilogue
     float w[4];
     if (mode == WG_LEARN && L.opt != DPC_OPT_SGD)
     {
-      // (adam_update)
-      const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f, lr_wd = L.opt == DPC_OPT_ADAMW ? L.lr * L.lmbda : -1.0f;
+      // adam_update, its roundings spelled out as they always were here: of b2 v + (1 - b2) g^2 the compiler fuses one
+      // product in this kernel and the other in those of bias and Psi, and an update of a near-zero gradient is
+      // sensitive to which (an epoch of 16 AdamW steps ends 3 % apart)
+      const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f, lr_wd = weight_wd(L);
       float mm[4], vv[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j)
@@ -288,14 +288,10 @@ struct GemmEpilogue
     }
     else
     {
-      const float Bf = (float)batch;
-      const bool dfa = mode == WG_DFA;
-      const float alpha = dfa ? L.fl * L.a / Bf : simple ? L.lr / Bf : L.a * L.lr / Bf;
-      const bool decays = dfa ? (flags & 1) && L.lmbda > 0.0f && L.fl != 0.0f : L.lmbda > 0.0f;
-      const float decay = decays ? 1.0f - L.lmbda : 1.0f;
+      const Sgd update = weight_sgd(L, batch, mode == WG_DFA, (flags & 1) != 0);
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        w[j] = fmaf(alpha, sum[j], x[0][j] * decay);
+        w[j] = update(x[0][j], sum[j]);
     }
     store4(L.W + o, w, vec, left);
   }

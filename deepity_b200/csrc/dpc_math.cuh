@@ -229,4 +229,11 @@ __device__ __forceinline__ float adam_update(float p, float g, float& m, float& 
   p -= step * m / (sqrtf(v) + eps);
   return p;
 }
+
+// One element of an SGD update from the raw sum over the batch, decayed first.
+struct Sgd
+{
+  float rate, decay;
+  __device__ __forceinline__ float operator()(float p, float sum) const { return fmaf(rate, sum, p * decay); }
+};
 } // namespace dpc

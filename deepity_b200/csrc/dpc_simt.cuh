@@ -761,13 +761,46 @@ __global__ void bump_counters_kernel(const dpc_layer* __restrict__ layers, int f
     *L.t_Psi += 1;
 }
 
+// Rates and decays of a layer's updates, from the raw sums over `batch` rows.
+// dfa: the direct-feedback update, decay_w: which decays the weights
+__device__ __forceinline__ Sgd weight_sgd(const dpc_layer& L, int batch, bool dfa, bool decay_w)
+{
+  const float Bf = (float)batch;
+  const bool simple = (L.flags & DPC_LAYER_INPUT_ACT) != 0;
+  const bool decays = dfa ? decay_w && L.lmbda > 0.0f && L.fl != 0.0f : L.lmbda > 0.0f;
+  return Sgd{dfa ? L.fl * L.a / Bf : simple ? L.lr / Bf : L.a * L.lr / Bf, decays ? 1.0f - L.lmbda : 1.0f};
+}
+__device__ __forceinline__ Sgd bias_sgd(const dpc_layer& L, int batch)
+{
+  return Sgd{L.lr / (float)batch, 1.0f};
+}
+__device__ __forceinline__ float psi_rate(const dpc_layer& L)
+{
+  return (L.flags & DPC_LAYER_FULLPC_PSI) ? L.fl * L.a : L.fl;
+}
+__device__ __forceinline__ Sgd psi_sgd(const dpc_layer& L, int batch)
+{
+  const bool decays = !(L.flags & DPC_LAYER_FULLPC_PSI) && L.psi_decay > 0.0f;
+  return Sgd{psi_rate(L) / (float)batch, decays ? 1.0f - L.psi_decay : 1.0f};
+}
+// (of adam_update: AdamW's decay, or below zero)
+__device__ __forceinline__ float weight_wd(const dpc_layer& L)
+{
+  return L.opt == DPC_OPT_ADAMW ? L.lr * L.lmbda : -1.0f;
+}
+__device__ __forceinline__ float psi_wd(const dpc_layer& L)
+{
+  const bool own = !(L.flags & DPC_LAYER_FULLPC_PSI) && L.psi_decay >= 0.0f;
+  return L.opt_psi == DPC_OPT_ADAMW ? psi_rate(L) * (own ? L.psi_decay : L.lmbda) : -1.0f;
+}
+
 // b (+)= rate * s for one output unit (or s into the staging buffer): what follows the column sum.
 __device__ __forceinline__ void bias_apply(const dpc_layer& L, int j, float s, int batch, int grad_only)
 {
   if (grad_only)
     L.g_b[j] = s;
   else if (L.opt == DPC_OPT_SGD)
-    L.b[j] += (L.lr / (float)batch) * s;
+    L.b[j] = bias_sgd(L, batch)(L.b[j], s);
   else
   {
     float m = L.m_b[j], v = L.v_b[j];
@@ -924,31 +957,22 @@ __global__ void bias_update_kernel(const dpc_layer* __restrict__ layers, int fir
 }
 
 // `step`: adam_step_size of the layer (two powers and a root: once per thread, not per element)
-__device__ __forceinline__ float psi_step(const dpc_layer& L, float rate, int grad_only)
+__device__ __forceinline__ float psi_step(const dpc_layer& L, int grad_only)
 {
-  return grad_only || L.opt_psi == DPC_OPT_SGD ? 0.0f : adam_step_size(rate, *L.t_Psi);
+  return grad_only || L.opt_psi == DPC_OPT_SGD ? 0.0f : adam_step_size(psi_rate(L), *L.t_Psi);
 }
 __device__ __forceinline__ void psi_apply(const dpc_layer& L, int row, int k, float sum, int batch,
-                                          int grad_only, bool full_kind, float rate, float step)
+                                          int grad_only, float step)
 {
   const size_t o = (size_t)row * L.psi_stride + k;
   if (grad_only)
     L.g_Psi[o] = sum;
   else if (L.opt_psi == DPC_OPT_SGD)
-  {
-    const float decay = (!full_kind && L.psi_decay > 0.0f) ? 1.0f - L.psi_decay : 1.0f;
-    float p = L.Psi[o];
-    if (decay != 1.0f)
-      p *= decay;
-    L.Psi[o] = fmaf(rate / (float)batch, sum, p);
-  }
+    L.Psi[o] = psi_sgd(L, batch)(L.Psi[o], sum);
   else
   {
-    float lr_wd = -1.0f;
-    if (L.opt_psi == DPC_OPT_ADAMW)
-      lr_wd = rate * ((!full_kind && L.psi_decay >= 0.0f) ? L.psi_decay : L.lmbda);
     float m = L.m_Psi[o], v = L.v_Psi[o];
-    L.Psi[o] = adam_update(L.Psi[o], -sum, m, v, step, lr_wd);
+    L.Psi[o] = adam_update(L.Psi[o], -sum, m, v, step, psi_wd(L));
     L.m_Psi[o] = m;
     L.v_Psi[o] = v;
   }
@@ -1070,8 +1094,6 @@ __global__ void __launch_bounds__(256)
   if (L.next_size <= 0 || L.Psi == nullptr || (L.flags & DPC_LAYER_INPUT_ACT))
     return;
   const int TS = L.terminal_size, s = L.size;
-  const bool full_kind = (L.flags & DPC_LAYER_FULLPC_PSI) != 0;
-  const float rate = full_kind ? L.fl * L.a : L.fl;
   if ((int)blockIdx.x * 128 >= s)
     return;
   __shared__ __align__(16) float es[128][KC];
@@ -1080,13 +1102,13 @@ __global__ void __launch_bounds__(256)
   float acc[4][KC];
   if (!batch_outer4<KC>(L.z, s, col, eT, TS, TS, batch, acc, es, part))
     return;
-  const float step = psi_step(L, rate, grad_only);
+  const float step = psi_step(L, grad_only);
 #pragma unroll
   for (int c = 0; c < 4; ++c)
 #pragma unroll
     for (int k = 0; k < KC; ++k)
       if (k < TS)
-        psi_apply(L, col + c, k, acc[c][k], batch, grad_only, full_kind, rate, step);
+        psi_apply(L, col + c, k, acc[c][k], batch, grad_only, step);
 }
 
 // State update of a layer below a narrow one (at most KC <= 16 units above, own width a multiple of
@@ -1198,45 +1220,19 @@ __global__ void __launch_bounds__(256)
 
 // One entry of a weight update from the raw sum over the batch.
 __device__ __forceinline__ void weight_apply(const dpc_layer& L, size_t o, float sum, int batch,
-                                             int mode, int flags, bool simple, float step)
+                                             int mode, int flags, float step)
 {
   if (mode & WG_GRAD_ONLY)
-  {
     L.g_W[o] = sum;
-    return;
-  }
-  const float Bf = (float)batch;
-  float w = L.W[o];
-  if (mode == WG_LEARN && L.opt != DPC_OPT_SGD)
+  else if (mode == WG_LEARN && L.opt != DPC_OPT_SGD)
   {
-    float lr_wd = -1.0f;
-    if (L.opt == DPC_OPT_ADAMW)
-      lr_wd = L.lr * L.lmbda;
     float mm = L.m_W[o], vv = L.v_W[o];
-    w = adam_update(w, -1.0f * L.a * sum, mm, vv, step, lr_wd);
+    L.W[o] = adam_update(L.W[o], -1.0f * L.a * sum, mm, vv, step, weight_wd(L));
     L.m_W[o] = mm;
     L.v_W[o] = vv;
   }
   else
-  {
-    float alpha, decay = 1.0f;
-    if (mode == WG_DFA)
-    {
-      alpha = L.fl * L.a / Bf;
-      if ((flags & 1) && L.lmbda > 0.0f && L.fl != 0.0f)
-        decay = 1.0f - L.lmbda;
-    }
-    else
-    {
-      alpha = simple ? (L.lr / Bf) : (L.a * L.lr / Bf);
-      if (L.lmbda > 0.0f)
-        decay = 1.0f - L.lmbda;
-    }
-    if (decay != 1.0f)
-      w *= decay;
-    w = fmaf(alpha, sum, w);
-  }
-  L.W[o] = w;
+    L.W[o] = weight_sgd(L, batch, mode == WG_DFA, (flags & 1) != 0)(L.W[o], sum);
 }
 
 // Weight update of a narrow layer (at most KC <= 16 output units, input width a multiple of 128:
@@ -1273,7 +1269,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
     for (int k = 0; k < KC; ++k)
       if (k < M)
-        weight_apply(L, (size_t)k * s + col + c, acc[c][k], batch, mode, flags, simple, step);
+        weight_apply(L, (size_t)k * s + col + c, acc[c][k], batch, mode, flags, step);
 }
 
 // Feedback-weight update Psi[l] (+)= (fl*a/B) z[l]^T e_T.  A block of 256 threads owns 64 rows of
@@ -1292,9 +1288,7 @@ __global__ void __launch_bounds__(256)
   if (L.next_size <= 0 || L.Psi == nullptr || (L.flags & DPC_LAYER_INPUT_ACT))
     return;
   const int TS = L.terminal_size, s = L.size;
-  const bool full_kind = (L.flags & DPC_LAYER_FULLPC_PSI) != 0;
-  const float rate = full_kind ? L.fl * L.a : L.fl;
-  const float step = psi_step(L, rate, grad_only);
+  const float step = psi_step(L, grad_only);
   constexpr int PSI_ROWS = 64, GROUPS = 4, COLS = 64;
   __shared__ __align__(16) float es[PSI_ROWS][16];
   __shared__ float part[GROUPS][COLS][17];
@@ -1352,7 +1346,7 @@ __global__ void __launch_bounds__(256)
           if (k >= kn)
             continue;
           const float sum = ((part[0][rc][k] + part[1][rc][k]) + part[2][rc][k]) + part[3][rc][k];
-          psi_apply(L, row, kc + k, sum, batch, grad_only, full_kind, rate, step);
+          psi_apply(L, row, kc + k, sum, batch, grad_only, step);
         }
       }
       __syncthreads();
@@ -1375,7 +1369,6 @@ __global__ void apply_gradients_kernel(const dpc_layer* __restrict__ layers, int
   if (L.next_size <= 0)
     return;
   const bool simple = (L.flags & DPC_LAYER_INPUT_ACT) != 0;
-  const float Bf = (float)batch;
   const size_t nW = (size_t)L.next_size * L.size;
   const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t nthr = (size_t)gridDim.x * blockDim.x;
@@ -1383,37 +1376,23 @@ __global__ void apply_gradients_kernel(const dpc_layer* __restrict__ layers, int
   {
     if (layers[li + 1].Psi == nullptr)
       return;
-    const float alpha = L.fl * L.a / Bf;
-    const float decay = ((flags & 1) && L.lmbda > 0.0f && L.fl != 0.0f) ? 1.0f - L.lmbda : 1.0f;
+    const Sgd update = weight_sgd(L, batch, true, (flags & 1) != 0);
     for (size_t o = tid; o < nW; o += nthr)
-    {
-      float w = L.W[o];
-      if (decay != 1.0f)
-        w *= decay;
-      L.W[o] = fmaf(alpha, L.g_W[o], w);
-    }
+      L.W[o] = update(L.W[o], L.g_W[o]);
     return;
   }
   if (L.opt == DPC_OPT_SGD)
   {
-    const float alpha = simple ? (L.lr / Bf) : (L.a * L.lr / Bf);
-    const float decay = L.lmbda > 0.0f ? 1.0f - L.lmbda : 1.0f;
+    const Sgd update = weight_sgd(L, batch, false, false), bias = bias_sgd(L, batch);
     for (size_t o = tid; o < nW; o += nthr)
-    {
-      float w = L.W[o];
-      if (decay != 1.0f)
-        w *= decay;
-      L.W[o] = fmaf(alpha, L.g_W[o], w);
-    }
+      L.W[o] = update(L.W[o], L.g_W[o]);
     if (which != 2)
       for (size_t j = tid; j < (size_t)L.next_size; j += nthr)
-        L.b[j] += (L.lr / Bf) * L.g_b[j];
+        L.b[j] = bias(L.b[j], L.g_b[j]);
   }
   else
   {
-    const float step = adam_step_size(L.lr, *L.t);
-    const float lr_wd = L.opt == DPC_OPT_ADAMW ? L.lr * L.lmbda : -1.0f;
-    const float alpha = -1.0f * L.a;
+    const float step = adam_step_size(L.lr, *L.t), lr_wd = weight_wd(L), alpha = -1.0f * L.a;
     for (size_t o = tid; o < nW; o += nthr)
     {
       float mm = L.m_W[o], vv = L.v_W[o];
@@ -1432,29 +1411,20 @@ __global__ void apply_gradients_kernel(const dpc_layer* __restrict__ layers, int
   }
   if (L.Psi == nullptr || simple || which == 2)
     return;
-  const bool full_kind = (L.flags & DPC_LAYER_FULLPC_PSI) != 0;
-  const float rate = full_kind ? L.fl * L.a : L.fl;
   const int TS = L.terminal_size;
   const size_t nP = (size_t)L.size * TS;
   if (L.opt_psi == DPC_OPT_SGD)
   {
-    const float decay = (!full_kind && L.psi_decay > 0.0f) ? 1.0f - L.psi_decay : 1.0f;
-    const float alpha = rate / Bf;
+    const Sgd update = psi_sgd(L, batch);
     for (size_t q = tid; q < nP; q += nthr)
     {
       const size_t o = (q / TS) * L.psi_stride + q % TS;
-      float p = L.Psi[o];
-      if (decay != 1.0f)
-        p *= decay;
-      L.Psi[o] = fmaf(alpha, L.g_Psi[o], p);
+      L.Psi[o] = update(L.Psi[o], L.g_Psi[o]);
     }
   }
   else
   {
-    const float step = adam_step_size(rate, *L.t_Psi);
-    float lr_wd = -1.0f;
-    if (L.opt_psi == DPC_OPT_ADAMW)
-      lr_wd = rate * ((!full_kind && L.psi_decay >= 0.0f) ? L.psi_decay : L.lmbda);
+    const float step = adam_step_size(psi_rate(L), *L.t_Psi), lr_wd = psi_wd(L);
     for (size_t q = tid; q < nP; q += nthr)
     {
       const size_t o = (q / TS) * L.psi_stride + q % TS;
