@@ -174,8 +174,10 @@ static int launch_gemm(dpc_plan* p, int first, int count, int flags, int mode, c
 }
 
 // Networks with an Adam-type optimizer or an activation with a kink turn a rounding difference into a whole
-// step (an update m / (sqrt(v) + eps), a derivative that flips between 0 and 1): every sum of theirs keeps
-// one order of additions.
+// step (an update m / (sqrt(v) + eps), a derivative that flips between 0 and 1).  Sums over the width keep one
+// ascending order in all kernels of theirs.  Their sums over the batch stay on the kernels that have always formed
+// them -- some split the rows, over warps and clusters, in an order that a shape and a GPU fix -- and off
+// batch_product_kernel.
 bool ordered_sums(const dpc_plan* p)
 {
   for (const dpc_layer& L : p->h)
@@ -1250,8 +1252,9 @@ static int launch_batch_products(dpc_plan* p, int first, int count, int mode, in
     if (tiles == 0)
       continue;
     // CTAs of a cluster that share a tile's batch rows: two groups of rows or more for each warp; beside
-    // tensor-core launches, which leave few SMs free, eight (clusters of eight held up the launches behind
-    // them: 784-(256x8)-10 at batch 256 250 us a step, single CTAs 238).
+    // tensor-core launches, which wait where clusters take the SMs, eight (us a step with two / eight:
+    // 784-(256x8)-10 at batch 256 274 / 267, at batch 512 245 / 235; with 32 / eight, i.e. single CTAs / pairs at
+    // batch 1024: 512-(512x12)-10 515 / 511, in tf32 mode 466 / 458, 768-(768x6)-10 498 / 490).
     const int rows = BP_WARPS * BP_ROWS * (tensor ? 8 : 2);
     int R = 1;
     while (R < 8 && (long long)tiles * R < 2LL * p->ctx->sm_count && p->batch >= 2 * R * rows)
@@ -1529,7 +1532,9 @@ static int launch_bias_update(dpc_plan* p, int f, int c, int grad_only)
     return rc;
   const FePlanes fp = fe_planes(p);
   // 256 threads: blocks of 64 columns where the feedback error is read from its planes or the batch is
-  // large, of 32 columns elsewhere (a block takes several where the layer's own kind differs)
+  // large, of 32 columns elsewhere (a block takes several where the layer's own kind differs).  The CTAs of a cluster
+  // share the batch; 1024 rows each or more beside tensor-core products (us a step with 256 / 1024: 512-(512x12)-10 at
+  // batch 1024 523 / 515, in tf32 mode 470 / 462, 768-(768x6)-10 501 / 492), 256 where the order may not change.
   const bool by_blocks = fp.only || p->batch >= kBiasBlockRows;
   dim3 gb(std::max(1, cdiv(max_next, by_blocks ? 64 : 32)), c);
   launch_row_split(bias_update_kernel, gb, 256,
@@ -1563,7 +1568,9 @@ static std::vector<Job> learn_jobs(dpc_plan* p, int first, int count, int grad_o
   }
   // Psi of tensor-core layers: strips of 128 columns x the whole batch where there are enough of them; tiles that
   // share the batch else, in one launch with the sums of the other layers (a 32 x 32 tile of ten terminal units
-  // multiplies 1.6 times what it keeps).
+  // multiplies 1.6 times what it keeps).  us a step, strips / tiles: 40 layers of 512 at batch 1024 (160 strips)
+  // 1272 / 1254, 150 of 256 at batch 512 (300) 1813 / 1801, 155 of 512 (620) 4183 / 4149 with runs 50 apart, 300 of
+  // 512 (1200) 7860 / 7895.
   long long strips = 0;
   for (int i = first; i < first + count; ++i)
     if (tc_piece(p, i) && p->h[i].Psi && p->h[i].size % 128 == 0 && p->h[i].terminal_size <= 16)

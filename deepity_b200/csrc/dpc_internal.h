@@ -77,7 +77,8 @@ namespace dpc
 // dpc_core.cu -- independent launches of one phase on streams that fork from the context's and join it.
 using Job = std::function<int()>;
 int run_side_by_side(dpc_ctx* ctx, const std::vector<Job>& jobs);
-bool ordered_sums(const dpc_plan* p); // no sum of the plan's products may be split
+// Whether sums of the plan's products keep the order they have: ascending ones are not split, others not split otherwise.
+bool ordered_sums(const dpc_plan* p);
 // dpc_resident.cu — row segments of small networks.  DPC_OK: the plan has them, 1: it does not.
 int res_plan_init(dpc_plan* plan);
 void res_plan_free(dpc_plan* plan);

@@ -10,8 +10,8 @@
 // traffic inside the settling loop, only barriers of the CTA.
 //
 // Measured: 784-128-128-10 at batch 64, 20 steps, 879 -> 113 us a step (about 2.5 us a settling pass: 1600 and
-// 900 cycles of sums, two elementwise phases of 1000 that are chains of latencies); ordered sums with streamed weights, 100-300-200-77-10
-// at batch 50 with AdamW, 6 steps, 750 -> 183 us.
+// 900 cycles of sums, two elementwise phases of 1000 that are chains of latencies); ordered sums with streamed
+// weights, 100-300-200-77-10 at batch 50 with AdamW, 6 steps, 750 -> 183 us.
 //
 // A pass is a list of warp tasks that leave partial sums in shared memory, a barrier, and an
 // elementwise pass that adds them in a fixed order and finishes (activation, error, gated error, or
