@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from common import (ADAM_TOL, DELTA_TOL, DELTA_TOL_TF32, TF32_TOL, TOL, build_gpu_net, compare_outputs,
-                    initial_parameters, run_gpu, run_oracle)
+                    initial_parameters, make_case, make_oracle, run_gpu, run_oracle)
 from conv_common import chain, run_conv_gpu, run_conv_oracle
 
 pytestmark = pytest.mark.gpu
@@ -51,11 +51,10 @@ GROUPED = {
     # 32 x 32 tiles: one row over a tile, K not a multiple of the stage, rows not 16-byte aligned
     "gemm_32_edges": _case("dkp", [33, 65, 31, 10], 65),
     "gemm_32_aligned": _case("simple", [64, 96, 32, 4], 32, mode="projection"),
-    "gemm_64_edges": _case("dkp", [67, 641, 12], 961),
-    # ordered sums: blocks of four warps, of two (three tiles an SM and more), 64 x 64 tiles (1.75 an SM and more)
+    "gemm_32_many": _case("dkp", [67, 641, 12], 961),
+    # blocks of four warps, of two (three aligned tiles an SM and more)
     "gemm_four_warps": _case("full", [37, 45, 45, 6], 33, "relu", residual=1, momentum=0.9),
     "gemm_two_warps": _case("simple", [64, 512, 512, 8], 961, "relu"),
-    "gemm_64_ordered": _case("dkp", [35, 1030, 1025, 6], 1100, "relu", T=2, steps=1),
     # more runs of layers of one shape than a launch lists
     "gemm_many_shapes": _case("dkp", [16] + [40, 12] * 125 + [4], 33, "relu", T=2),
     "gemm_adamw": _case("dkp", [35, 66, 65, 6], 70, lr=1e-3, optimizer="ADAMW"),
@@ -64,8 +63,8 @@ GROUPED = {
     "head_ce_two_rows": _case("full", [40, 132, 16], 2051, cross_entropy=1),
     "head_simple_ce": _case("simple", [40, 256, 10], 259, mode="projection", cross_entropy=1),
     "head_simple": _case("simple", [40, 384, 13], 2051, mode="python"),
-    # column sums: more than one group of 32 columns, rows that end inside a buffer
-    "column_sums": _case("dkp", [24, 70, 33], 1031),
+    # column sums in row order: more than one group of 32 columns, rows that end inside a buffer
+    "column_sums": _case("dkp", [24, 70, 33], 1031, "relu"),
 }
 
 
@@ -73,6 +72,55 @@ GROUPED = {
 def test_grouped_launches_match_oracle(name, built_library, monkeypatch):
     monkeypatch.setenv("DPC_DISABLE_RESIDENT", "1")
     _check(GROUPED[name], name)
+
+
+# 64 x 64 tiles (1.75 an SM and more) and 32 x 32 ones of two warps with rows copied element by element (six an SM and
+# more): the tiles' edges, both ways of copying, every epilogue; the phases that are checked to take them
+LARGE = {
+    "unaligned": (_case("dkp", [35, 1030, 1025, 6], 1100, "relu", T=2, steps=1), 64, ("weights", "forward", "state")),
+    "residual_momentum": (_case("full", [64, 640, 640, 12], 1740, "gelu", mupc=1, residual=1, momentum=0.9), 64,
+                          ("forward", "state")),
+    "simple": (_case("simple", [64, 644, 640, 12], 1740, "sigmoid", mode="projection"), 64, ("forward", "state")),
+    # (smooth: of 1.6 million preactivations a pass one is likely to lie within 1e-7 of a kink, where f' depends on
+    # the order of additions)
+    "two_warps_forward": (_case("dkp", [33, 319, 319, 63], 2557, "tanh", T=2), 32, ("forward",)),
+    "two_warps_state": (_case("full", [33, 319, 319, 63], 1533, "tanh", residual=1, momentum=0.9), 32, ("state",)),
+}
+
+
+@pytest.mark.parametrize("name", sorted(LARGE))
+def test_large_launches_match_oracle(name, built_library, monkeypatch):
+    monkeypatch.setenv("DPC_DISABLE_RESIDENT", "1")
+    case, tile, phases = LARGE[name]
+    for phase in phases:
+        large = _tiles(case, 64, phase) >= 1.75 * _sms() and 8 * _tiles(case, 64, phase) <= 3 * _tiles(case, 32, phase)
+        assert large == (tile == 64) and (large or _tiles(case, 32, phase) >= 6 * _sms())
+    _check(case, name)
+
+
+@pytest.mark.parametrize("kind,sizes,batch,optimizer", [("dkp", [64, 1028, 1032, 12], 70, "ADAMW"),
+                                                        ("full", [67, 1030, 1025, 7], 61, "ADAM")])
+def test_adam_updates_on_large_tiles(kind, sizes, batch, optimizer, built_library):
+    """Of a million weights some have gradients of the size of the rounding, whose step may go the other way.  So the
+    moments, which are linear and quadratic in the gradient, are held to the bound of the SGD updates, and the weights
+    to the step that the network's own moments give (fp32 rounding of the step and of the sum)."""
+    case = _case(kind, sizes, batch, T=2, steps=1, lr=1e-3, optimizer=optimizer)
+    case["hyper"].update(lmbda=0.01, fl=0.0)  # (no direct feedback: the weights change in this update alone)
+    assert _tiles(case, 64) >= 1.75 * _sms()
+    params, x, y = make_case(kind, sizes, batch)
+    orc = make_oracle(kind, sizes, batch, params, **case["hyper"], optimizer=optimizer)
+    orc.train_step(x, y, 2)
+    net, _, _ = build_gpu_net(case)
+    net.train_step(x, y, 2)
+    for l in range(3):
+        m, v, w = (net.get_tensor(l, n).astype(np.float64) for n in ("weight.m", "weight.v", "W"))
+        for got, name, tol in ((m, "weight.m", DELTA_TOL), (v, "weight.v", 2 * DELTA_TOL)):
+            ref = np.asarray(orc.get(l, name), dtype=np.float64).ravel()
+            assert np.abs(ref - got).max() <= tol * np.abs(ref).max(), (l, name)
+        decay = 1e-3 * 0.01 if optimizer == "ADAMW" else 0.0
+        step = 1e-3 * np.sqrt(1 - 0.999) / (1 - 0.9)
+        ref = params[l]["W"].ravel().astype(np.float64) * (1 - decay) - step * m / (np.sqrt(v) + 1e-8)
+        assert np.abs(ref - w).max() <= 4 * np.finfo(np.float32).eps * np.abs(ref).max() + 1e-5 * 1e-3, l
 
 
 # Forward products of SimplePC layers on 64 x 64 tiles, which transform their operand: from six 32 x 32 tiles an SM on,
@@ -99,6 +147,7 @@ BATCH_SUMS = {
     "one_row": _case("dkp", [20, 30, 5], 1),
     "edges": _case("dkp", [33, 65, 31, 40], 9),
     "clusters": _case("simple", [67, 31, 17], 1031, mode="projection"),
+    "columns": _case("dkp", [24, 70, 33], 1031),
     "many_layers": _case("dkp", [16] + [12] * 130 + [4], 5, T=2),
     "many_shapes": _case("dkp", [16] + [40, 12] * 125 + [4], 9, T=2),
     "beside_tensor_cores": _case("dkp", [64, 256, 256, 17], 256),

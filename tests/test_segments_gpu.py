@@ -41,6 +41,9 @@ ROWS = {
     # ... over input rows that end inside each of the load groups
     "exact_input_quads": _case("dkp", [84, 33, 9], 3, "relu"),
     "exact_input_singles": _case("dkp", [107, 33, 9], 601, "relu"),
+    # sliced sums over input rows that are not 16-byte aligned: a strip of loads and a remainder, many
+    "input_singles": _case("dkp", [107, 33, 9], 3, "tanh"),
+    "input_singles_8_rows": _case("simple", [1971, 33, 9], 601, "sigmoid"),
     # every term of the state update, more layers than warps share evenly
     "residual_momentum": _case("full", [33] + [64] * 9 + [10], 5, "gelu", mupc=1, residual=1, momentum=0.9),
     "cross_entropy": _case("full", [45, 61, 32, 17], 149, "tanh", cross_entropy=1),
