@@ -23,8 +23,8 @@ constexpr int BP_SLOT = 2 * BP_ROWS * BP_T; // floats: rows of g, rows of z
 
 struct BatchTiles
 {
-  TileList list; // kind: the weight sums of these layers are among them ...
-  int sums;      // ... and their bias sums, and the Psi sums of all layers
+  int sums;      // their bias sums and the Psi sums of all layers are among them
+  TileList list; // kind: the weight sums of these layers are
 };
 
 __device__ __forceinline__ float4 rows_cluster_load4(const float* own, uint32_t rank)
@@ -41,8 +41,8 @@ __device__ __forceinline__ float4 rows_cluster_load4(const float* own, uint32_t 
 }
 
 __global__ void __launch_bounds__(32 * BP_WARPS, 2)
-    batch_product_kernel(const dpc_layer* __restrict__ layers, const __grid_constant__ BatchTiles T,
-                         int batch, int flags, int mode, const float* __restrict__ eT)
+    batch_product_kernel(const dpc_layer* __restrict__ layers, int batch, int flags, int mode,
+                         const float* __restrict__ eT, const __grid_constant__ BatchTiles T)
 {
   const uint32_t R = rows_cluster_size(), rank = rows_cluster_rank();
   int t = (int)(blockIdx.x / R);

@@ -105,8 +105,8 @@ static int list_tiles(TileList& T, int first, int& end, Tiles tiles, Kind kind)
         end = i;
         break;
       }
-      T.start[T.runs] = total; // (runs without tiles are never looked up)
-      T.run[T.runs++] = TileRun{n, n > 0 ? ~0u / n : 0u, (unsigned short)(i - first), (unsigned short)k};
+      // (runs without tiles are never looked up)
+      T.run[T.runs++] = TileRun{total, n, n > 0 ? ~0u / n : 0u, (unsigned short)(i - first), (unsigned short)k};
     }
     total += n;
   }
@@ -158,7 +158,7 @@ static int launch_gemm(dpc_plan* p, int first, int count, int flags, int mode, c
       continue;
     auto go = [&](auto kern, int threads)
     {
-      kern<<<blocks, threads, 0, p->ctx->stream>>>(p->d, T, p->n, p->batch, flags, mode, p->energy, epc_src);
+      kern<<<blocks, threads, 0, p->ctx->stream>>>(p->d, p->n, p->batch, flags, mode, p->energy, epc_src, T);
     };
     if (large)
       go(pc_gemm_kernel<OP, 64, 4>, 128);
@@ -1268,8 +1268,8 @@ static int launch_batch_products(dpc_plan* p, int first, int count, int mode, in
     attr[0].val.clusterDim = {(unsigned)R, 1, 1};
     cfg.attrs = attr;
     cfg.numAttrs = R > 1 ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, batch_product_kernel, (const dpc_layer*)p->d, T, p->batch, flags, mode,
-                       p->e_terminal);
+    cudaLaunchKernelEx(&cfg, batch_product_kernel, (const dpc_layer*)p->d, p->batch, flags, mode,
+                       (const float*)p->e_terminal, T);
     const int rc = check_launch(p->ctx, "batch product kernel");
     if (rc != DPC_OK)
       return rc;

@@ -18,10 +18,11 @@ enum
 };
 
 // The output tiles of a launch, as runs of neighbouring layers with equally many (deep networks have few: one for each
-// shape; 240 are 3.9 KB of parameters, which a launch takes as fast as 0.5 KB).
+// shape; 240 are 3.9 KB of parameters, which a launch takes as fast as 0.5 KB).  The last parameter of a kernel: the
+// others and the first runs then come in with the same line of the constant cache.
 struct TileRun
 {
-  int per;              // tiles of a layer
+  int start, per;       // its first tile, tiles of a layer
   unsigned inverse;     // (2^32 - 1) / per
   unsigned short layer; // its first layer, from the list's
   unsigned short kind;
@@ -30,7 +31,6 @@ constexpr int kListRuns = 240;
 struct TileList
 {
   int first, layers, runs;
-  int start[kListRuns]; // of a run: its first tile
   TileRun run[kListRuns];
 };
 // Layer of tile t, which becomes the index within the layer.
@@ -45,13 +45,13 @@ __device__ __forceinline__ int tile_layer(const TileList& T, int& t, bool& kind)
   for (int hi = T.runs; hi - lo > 1;)
   {
     const int mid = (lo + hi) >> 1;
-    if (T.start[mid] <= t)
+    if (T.run[mid].start <= t)
       lo = mid;
     else
       hi = mid;
   }
   const TileRun& r = T.run[lo];
-  t -= T.start[lo];
+  t -= r.start;
   int layer = (int)__umulhi((unsigned)t, r.inverse); // t / per or one less
   t -= layer * r.per;
   if (t >= r.per)
@@ -368,8 +368,8 @@ __device__ __forceinline__ void copy_tile(float* dst, const float* __restrict__ 
 
 template <int OP, int T, int W>
 __global__ void __launch_bounds__(32 * W, T == 32 ? 20 / W : 4)
-    pc_gemm_kernel(const dpc_layer* __restrict__ layers, const __grid_constant__ TileList list, int n_layers,
-                   int batch, int flags, int mode, double* energy, const float* __restrict__ epc_src)
+    pc_gemm_kernel(const dpc_layer* __restrict__ layers, int n_layers, int batch, int flags, int mode, double* energy,
+                   const float* __restrict__ epc_src, const __grid_constant__ TileList list)
 {
   using C = GemmTile<T, W>;
   constexpr int BK = C::BK, PITCH = C::PITCH, THREADS = C::THREADS, TM = C::TM, STAGES = C::STAGES;
