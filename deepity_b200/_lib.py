@@ -64,6 +64,7 @@ SIGNATURES = {
     "dpc_plan_fused_cross_entropy": (_i, [_vp]),
     "dpc_plan_state_from_prediction": (_i, [_vp]),
     "dpc_rows_available": (_i, [_vp]),
+    "dpc_rows_clusters": (_i, [_vp]),
     "dpc_rows_segment": (_i, [_vp, _i, _i, _i, _i]),
     "dpc_epc_reconstruct": (_i, [_vp, _i]),
     "dpc_epc_adjoint": (_i, [_vp, _i, _i, _f, _i]),

@@ -24,7 +24,8 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 OUT = os.path.join(PKG, "libdeepity_b200.so")
 
-SOURCES = ["dpc_core.cu", "dpc_tc.cu", "dpc_static.cu", "dpc_conv.cu", "dpc_resident.cu", "dpc_conv_resident.cu",
+SOURCES = ["dpc_core.cu", "dpc_tc.cu", "dpc_static.cu", "dpc_conv.cu", "dpc_resident.cu", "dpc_cluster.cu",
+           "dpc_conv_resident.cu",
            os.path.join("host", "pc_network.cpp"), os.path.join("host", "conv_network.cpp")]
 HEADERS = ["dpc_internal.h", "dpc_math.cuh", "dpc_simt.cuh", os.path.join("host", "pc_network.h"),
            os.path.join("host", "conv_network.h"),

@@ -573,6 +573,8 @@ int dpc_plan_create(dpc_ctx* ctx, const dpc_layer* layers, int n_layers, int bat
   rc = tc_plan_init(p);
   if (rc >= 0)
     rc = res_plan_init(p);
+  if (rc >= 0)
+    rc = cluster_plan_init(p);
   if (rc < 0)
   {
     dpc_plan_destroy(p);
@@ -619,10 +621,13 @@ int dpc_plan_update(dpc_plan* p, const dpc_layer* layers, int n_layers)
                            p->ctx->stream));
   tc_plan_free(p);
   res_plan_free(p);
+  cluster_plan_free(p);
   p->init_precision = p->ctx->precision;
   rc = tc_plan_init(p);
   if (rc >= 0)
     rc = res_plan_init(p);
+  if (rc >= 0)
+    rc = cluster_plan_init(p);
   return rc < 0 ? rc : DPC_OK;
 }
 
@@ -632,6 +637,7 @@ int dpc_plan_destroy(dpc_plan* p)
     return DPC_OK;
   tc_plan_free(p);
   res_plan_free(p);
+  cluster_plan_free(p);
   if (p->d)
     cudaFree(p->d);
   if (p->energy)

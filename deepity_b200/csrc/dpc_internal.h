@@ -70,6 +70,7 @@ struct dpc_plan
   dpc::TensorRun run;
   void* tc = nullptr; // tensor-core path state (tensor maps), owned by dpc_tc.cu
   void* res = nullptr; // row-segment path state, owned by dpc_resident.cu
+  void* seg = nullptr; // the same on clusters, owned by dpc_cluster.cu
 };
 
 namespace dpc
@@ -82,6 +83,11 @@ bool ordered_sums(const dpc_plan* p);
 // dpc_resident.cu — row segments of small networks.  DPC_OK: the plan has them, 1: it does not.
 int res_plan_init(dpc_plan* plan);
 void res_plan_free(dpc_plan* plan);
+bool res_plan_streams(const dpc_plan* plan); // some weights are read from L2 on every pass
+// dpc_cluster.cu — row segments whose weights are shared out over the blocks of a cluster; same convention.
+int cluster_plan_init(dpc_plan* plan);
+void cluster_plan_free(dpc_plan* plan);
+int cluster_segment(dpc_plan* plan, int ops, int steps, int top_clamped, int top_down_off);
 // dpc_tc.cu — tensor-core (tcgen05/TMEM/TMA) path.  Each returns DPC_OK when it handled
 // layers [first, first+count) completely, 1 when the range is not eligible (the caller
 // then uses the CUDA-core kernels), or a negative status.

@@ -1158,6 +1158,7 @@ struct ResState
   ResParams P = {};
   int R = 1;
   size_t smem = 0;
+  bool streams = false;
   void* dev = nullptr; // tables
 };
 
@@ -1401,6 +1402,8 @@ int build(dpc_plan* p, int R, int S, bool has_v, bool exact)
   P.has_v = has_v ? 1 : 0;
   P.exact = exact ? 1 : 0;
   P.energy = p->energy;
+  for (int l = 1; l < nw; ++l)
+    st->streams |= rl[l].rrows < rl[l].N;
   st->R = R;
   st->smem = o;
   p->res = st;
@@ -1416,6 +1419,11 @@ void res_plan_free(dpc_plan* p)
   cudaFree(s->dev);
   delete s;
   p->res = nullptr;
+}
+
+bool res_plan_streams(const dpc_plan* p)
+{
+  return p->res && static_cast<const ResState*>(p->res)->streams;
 }
 
 // Which plans run here: by shape only.  Plans with tensor-core layers do not; the others do while
@@ -1524,8 +1532,10 @@ int dpc_rows_available(dpc_plan* p)
 
 int dpc_rows_segment(dpc_plan* p, int ops, int steps, int top_clamped, int top_down_off)
 {
-  if (!p || !p->res || steps < 0)
+  if (!p || !(p->res || p->seg) || steps < 0)
     return fail(DPC_ERR_INVALID, "dpc_rows_segment: not a row-resident plan, or a bad step count");
+  if (p->seg)
+    return cluster_segment(p, ops, steps, top_clamped, top_down_off);
   const auto* st = static_cast<const ResState*>(p->res);
   ResParams P = st->P;
   P.ops = ops, P.steps = steps;

@@ -822,7 +822,7 @@ void PCNetwork::RefreshPredictions()
 // without the features whose phases interleave rows (gradient staging, ePC sweeps, a ghost layer).
 bool PCNetwork::UseRowSegments()
 {
-  return !useEPC && !ghostTop && !gradSync && dpc_rows_available(plan);
+  return !useEPC && !ghostTop && !gradSync && (dpc_rows_available(plan) || dpc_rows_clusters(plan) > 0);
 }
 
 // (Without a settling step mode 2 is a weight update from whatever the last call left: no segment.)

@@ -42,6 +42,9 @@
  *   DPC_PAIR_TILE_WIDTH        64, 128 or 256: one width of the pair tiles of a run instead of the rule
  *                              (at least 128 for state and weight updates; other values do nothing)
  *   DPC_DISABLE_RESIDENT       small networks run phase by phase instead of in row segments
+ *   DPC_DISABLE_CLUSTERS       row segments on single blocks only
+ *   DPC_CLUSTER_SIZE           1, 2, 4, 8 or 16: row segments on clusters of so many blocks wherever they fit, instead of
+ *                              the rule
  */
 #ifndef DEEPITY_B200_H
 #define DEEPITY_B200_H
@@ -390,7 +393,7 @@ DPC_API int dpc_apply_gradients(dpc_plan* plan, int first, int count, int which,
 DPC_API int dpc_error_energy_static(void* stream, const float* z_dev, const float* mu_dev,
                                     float* e_dev, int64_t count, float* energy_dev);
 /* Row segments.  Between two weight updates a step is row-local: a plan whose weights are small
- * enough (dpc_rows_available) runs everything from one update to the next -- sweep, settling steps,
+ * enough (dpc_rows_available: for one block, dpc_rows_clusters: for a cluster) runs everything from one update to the next -- sweep, settling steps,
  * refresh, energy -- in ONE launch in which a thread block keeps a few batch rows' state on the chip.
  * ops: bit set of DPC_ROWS_*, executed in this order; steps: settling steps (CalculateState +
  * UpdateState, FullPCNetwork.cpp / DirectKPPCNetwork.cpp / SimplePCNetwork.cpp) between the sweep
@@ -420,6 +423,9 @@ enum
   DPC_ROWS_STORE_V = 1 << 18
 };
 DPC_API int dpc_rows_available(dpc_plan* plan);
+/* Blocks of a thread-block cluster that share a row group and hold all weights of a segment between them, 0: the plan
+ * has no such segments.  dpc_rows_segment runs where this or dpc_rows_available is not 0. */
+DPC_API int dpc_rows_clusters(dpc_plan* plan);
 DPC_API int dpc_rows_segment(dpc_plan* plan, int ops, int steps, int top_clamped,
                              int top_down_off);
 /* Energy accumulator of the plan (device-resident double). */

@@ -81,6 +81,63 @@ def test_row_segments_of_several_groups_a_block(kind, batch, available, built_li
     assert _available(_case(kind, [784, 91, 91, 10], batch, "relu")) == available
 
 
+# Segments on clusters: layers narrower than a block's share of four columns, rows that are not 16-byte aligned, the last
+# group not full; one, two and four rows a task, several tasks a warp; an input that streams in one step and in many.
+CLUSTERS = {
+    # (SGD: with AdamW at three rows a belief of all kernels, whose bits are equal, is 1.7e-3 from the oracle's)
+    "ordered_rows_1": _case("dkp", [100, 300, 200, 77, 10], 3, "relu"),
+    "ordered_adamw": _case("dkp", [100, 300, 200, 77, 10], 50, "relu", optimizer="ADAMW", psi_optimizer="ADAM"),
+    "ordered_rows_2": _case("dkp", [129, 131, 33, 7], 50, "hard_tanh"),
+    "ordered_rows_4": _case("simple", [1971, 65, 65, 65, 3], 300, "relu", mode="projection"),
+    "ordered_heads": _case("full", [256, 256, 128, 16], 33, "relu", momentum=0.9),  # lanes along K
+    "ordered_ipc": _case("full", [64] * 5 + [16], 70, "gelu", optimizer="ADAMW", mupc=1, residual=1, momentum=0.9, ipc=1),
+    "one_layer": _case("dkp", [784, 10], 50, "relu"),
+    "sliced": _case("dkp", [70, 285, 131, 10], 16, "tanh"),
+    "sliced_simple": _case("simple", [37, 202, 61, 10], 60, "sigmoid", mode="python"),
+    "deep_residual": _case("full", [21] * 40 + [5], 6, "tanh", mupc=1, residual=1, momentum=0.9),
+    "cross_entropy": _case("full", [45, 130, 66, 17], 20, "gelu", cross_entropy=1),
+    "simple_cross_entropy": _case("simple", [45, 61, 17], 9, "tanh", cross_entropy=1),
+}
+
+
+@pytest.mark.parametrize("blocks", [1, 2, 4, 8, 16])
+@pytest.mark.parametrize("name", sorted(CLUSTERS))
+def test_cluster_segments_match_oracle(name, blocks, monkeypatch, built_library):
+    from deepity_b200 import _lib
+    lib = _lib.load()
+    monkeypatch.setenv("DPC_CLUSTER_SIZE", str(blocks))
+    case = CLUSTERS[name]
+    net, _, _ = build_gpu_net(case)
+    clusters = lib.dpc_rows_clusters(lib.dpcn_plan(net._h))
+    del net
+    if clusters == 0:
+        pytest.skip("the weights do not fit the shared memory of so many blocks")
+    assert clusters == blocks
+    adam = "optimizer" in case["options"]
+    got = run_gpu(case)
+    compare_outputs(run_oracle(case), got, ADAM_TOL if adam else TOL, name,
+                    init=None if adam else initial_parameters(case), delta_tol=None if adam else DELTA_TOL)
+    if name.startswith("ordered"):
+        # one order of additions: the bits of the other kernels (energies are sums over blocks in any order)
+        monkeypatch.setenv("DPC_DISABLE_CLUSTERS", "1")
+        ref = run_gpu(case)
+        for k, v in ref.items():
+            assert k == "energies" or np.array_equal(v, got[k]), k
+
+
+@pytest.mark.parametrize("kind,sizes,batch,act,blocks",
+                         [("dkp", [100, 300, 200, 77, 10], 50, "relu", 4), ("simple", [784, 441, 441, 10], 25, "relu", 16),
+                          ("dkp", [100, 47, 47, 10], 54, "relu", 0),   # a short chain: blocks by themselves
+                          ("dkp", [64, 128, 128, 10], 64, "tanh", 0),  # sliced sums that fit one block
+                          ("dkp", [100, 273, 273, 273, 10], 1, "tanh", 8),
+                          ("dkp", [64, 1024, 1024, 10], 1, "tanh", 0)])  # weights that fit no cluster
+def test_which_networks_run_on_clusters(kind, sizes, batch, act, blocks, built_library):
+    from deepity_b200 import _lib
+    lib = _lib.load()
+    net, _, _ = build_gpu_net(_case(kind, sizes, batch, act))
+    assert lib.dpc_rows_clusters(lib.dpcn_plan(net._h)) == blocks
+
+
 def _images(shape, convs, act, batch, **kw):
     return dict(layers=chain(shape, convs, act), batch=batch, T=3, steps=2, hyper=dict(lr=0.005, ir=0.1, lmbda=0.0),
                 **kw)
