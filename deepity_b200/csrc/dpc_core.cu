@@ -3,6 +3,7 @@
 #include <functional>
 #include <cstring>
 #include <string>
+#include <type_traits>
 
 #include "dpc_internal.h"
 #include "dpc_batch.cuh"
@@ -128,12 +129,15 @@ static int launch_gemm(dpc_plan* p, int first, int count, int flags, int mode, c
                                          (i + 1 < p->n && p->h[i + 1].Psi));
     return any ? cdiv(M, T) * cdiv(N, T) : 0;
   };
-  long long tiles = 0, tiles64 = 0;
+  long long tiles = 0, tiles64 = 0, aligned = 0;
   bool vec = true; // rows can be copied 16 bytes at a time
   for (int i = first; i < first + count; ++i)
   {
     tiles += tiles_of(i, 32), tiles64 += tiles_of(i, 64);
     vec &= p->h[i].size % 4 == 0 && p->h[i].next_size % 4 == 0;
+    const int K = OP == OP_FWD ? p->h[i].size : OP == OP_FB ? p->h[i].next_size : p->batch;
+    if (p->h[i].size % 4 == 0 && (OP == OP_FWD || p->h[i].next_size % 4 == 0) && K >= 128)
+      aligned += tiles_of(i, 32);
   }
   // us, W = 4 / W = 2 / T = 64, by 32 x 32 tiles an SM:  0.9 (445 wide, batch 48) 16.5 / 24 / -,  1.4 (784 x 256
   // weights) 31 / 26 / -,  3 (512 wide, batch 210) 25 / 22 / -,  3.7 (512 wide, batch 1089) 28 / 25 / -,  4.2 (403
@@ -147,6 +151,14 @@ static int launch_gemm(dpc_plan* p, int first, int count, int flags, int mode, c
   const bool feeds = OP == OP_FWD && (p->h[first].flags & DPC_LAYER_INPUT_ACT);
   const bool large =
       (4 * tiles64 >= 7LL * sm || (feeds && tiles64 > sm && tiles > 6LL * sm)) && 8 * tiles64 <= 3 * tiles;
+  // Long steps, where most tiles have rows that are copied 16 bytes at a time and sums of 128 or more, and the tiles of
+  // a kernel are at most one wave with the shared memory they take (76 KB, 43 KB; 64 x 64 tiles in any number).  us a
+  // step, short / long: thirteen layers of 812 at batch 4 637 / 593, three of 768 at batch 128 649 / 615, twelve of 300
+  // at batch 60 294 / 277; two warps: three of 320 at batch 900 1018 / 963; 64 x 64: fourteen of 1024 at batch 100
+  // 1211 / 1165.  Four layers of 208 at batch 1000, 4.5 tiles an SM on four warps, 471 / 512; ten of 512 at batch 170,
+  // 6.5 tiles on two, 634 / 657; six of 445 at batch 48, copied element by element, 196 / 208; 400 of 32 at batch 300
+  // 932 / 1092.
+  const bool long_steps = 2 * aligned > tiles;
   const bool two_warps = tiles >= (OP == OP_WG ? sm : vec ? 3LL * sm : 6LL * sm);
   for (int f = first, end; f < first + count; f = end)
   {
@@ -156,16 +168,31 @@ static int launch_gemm(dpc_plan* p, int first, int count, int flags, int mode, c
         T, f, end, [&](int i) { return tiles_of(i, large ? 64 : 32); }, [](int) { return false; });
     if (blocks == 0)
       continue;
-    auto go = [&](auto kern, int threads)
+    auto go = [&](auto tile)
     {
-      kern<<<blocks, threads, 0, p->ctx->stream>>>(p->d, p->n, p->batch, flags, mode, p->energy, epc_src, T);
+      using C = decltype(tile);
+      constexpr int bytes = C::bytes(GemmEpilogue<OP>::kPre);
+      auto kern = pc_gemm_kernel<OP, C>;
+      // (more than 48 KB have to be asked for, once a device)
+      static thread_local int configured = -1;
+      if (configured != p->ctx->device)
+      {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
+          return;
+        configured = p->ctx->device;
+      }
+      kern<<<blocks, C::THREADS, bytes, p->ctx->stream>>>(p->d, p->n, p->batch, flags, mode, p->energy, epc_src, T);
     };
-    if (large)
-      go(pc_gemm_kernel<OP, 64, 4>, 128);
+    if (large && long_steps)
+      go(GemmTile<64, 4, true>());
+    else if (large)
+      go(GemmTile<64, 4, false>());
     else if (two_warps)
-      go(pc_gemm_kernel<OP, 32, 2>, 64);
+      long_steps && tiles <= 5LL * sm ? go(GemmTile<32, 2, true>()) : go(GemmTile<32, 2, false>());
+    else if (long_steps && tiles <= 2LL * sm)
+      go(GemmTile<32, 4, true>());
     else
-      go(pc_gemm_kernel<OP, 32, 4>, 128);
+      go(GemmTile<32, 4, false>());
     const int rc = check_launch(p->ctx, "grouped GEMM kernel");
     if (rc != DPC_OK)
       return rc;

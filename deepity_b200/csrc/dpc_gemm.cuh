@@ -319,7 +319,9 @@ __device__ __forceinline__ void feed4(const dpc_layer& L, float* p, int r, int k
 // whatever the tile (a belief that the sweep produced has an error of exactly zero in the passes that follow).
 //   T = 32, W = 4: 8 x 32 outputs a warp, 2 x 4 per lane        few tiles: all schedulers of an SM on one
 //   T = 32, W = 2: 16 x 32, 4 x 4 per lane                      several tiles an SM: fewer shared-memory reads
-//   T = 64, W = 4: 32 x 32, 8 x 4 per lane, steps of 16 K        many: half the operand traffic too
+//   T = 64, W = 4: 32 x 32, 8 x 4 per lane                       many: half the operand traffic too
+// Steps of 64, 32 and 16 K, twice as many with LONG: a step's copies, wait and barrier cost about 600 cycles beside the
+// 25 a K of a lone 32 x 32 tile (1 600 cycles per 32 K as steps of 32, 1 150 as steps of 128).
 // Operands come through a cp.async ring, 16 bytes at a time where rows start on 16-byte boundaries, else element
 // by element; a warp reads contiguous bytes of few rows either way.  What bounds it: with several tiles an SM reads
 // of shared memory (24, 16 and 12 cycles per k and 32 x 32 outputs, against 8 of the multiply-adds), else
@@ -328,12 +330,14 @@ __device__ __forceinline__ void feed4(const dpc_layer& L, float* p, int r, int k
 // start with cold instruction caches).  us, 32 x 32 tiles of 2 x 2 outputs per thread before / now: 784 -> 256 at
 // batch 256 22 / 19, 116 -> 116 at batch 64 7.1 / 5.5, six 445-wide layers at batch 48 24.7 / 16.5, three 403-wide
 // ones at batch 512 67 / 44, thirteen 153-wide ones at batch 1421 68 / 56 and their weights 240 / 125.
-template <int T, int W>
+template <int T_, int W_, bool LONG>
 struct GemmTile
 {
-  static constexpr int BK = T == 32 ? 32 : 16, PITCH = BK + 4; // (the lanes' 16-byte reads share no bank)
+  static constexpr int T = T_, W = W_;
+  static constexpr int BK = (T == 64 ? 16 : W == 4 ? 64 : 32) * (LONG ? 2 : 1), PITCH = BK + 4; // (the lanes' 16-byte reads share no bank)
   static constexpr int THREADS = 32 * W, TM = T == 32 ? 8 / W : 8;
-  static constexpr int STAGES = T == 32 ? 3 : 4, OPERAND = T * PITCH, SLOT = 2 * OPERAND;
+  static constexpr int STAGES = T == 64 ? (LONG ? 3 : 4) : W == 4 || LONG ? 2 : 3, OPERAND = T * PITCH, SLOT = 2 * OPERAND;
+  static constexpr int bytes(int pre) { return (STAGES * SLOT + (T == 32 ? pre : 0) * T * T) * (int)sizeof(float); }
 };
 
 // H lines of W contiguous elements from (h0, c0) of a matrix with `lines` lines of `width`, zeros beyond it.
@@ -366,17 +370,16 @@ __device__ __forceinline__ void copy_tile(float* dst, const float* __restrict__ 
   }
 }
 
-template <int OP, int T, int W>
-__global__ void __launch_bounds__(32 * W, T == 32 ? 20 / W : 4)
+template <int OP, typename C>
+__global__ void __launch_bounds__(C::THREADS, C::T == 32 ? 20 / C::W : 4)
     pc_gemm_kernel(const dpc_layer* __restrict__ layers, int n_layers, int batch, int flags, int mode, double* energy,
                    const float* __restrict__ epc_src, const __grid_constant__ TileList list)
 {
-  using C = GemmTile<T, W>;
-  constexpr int BK = C::BK, PITCH = C::PITCH, THREADS = C::THREADS, TM = C::TM, STAGES = C::STAGES;
+  constexpr int T = C::T, W = C::W, BK = C::BK, PITCH = C::PITCH, THREADS = C::THREADS, TM = C::TM, STAGES = C::STAGES;
   constexpr bool A_K = OP != OP_WG, B_K = OP == OP_FWD; // K contiguous in memory, else the tile's rows
   using Epilogue = GemmEpilogue<OP>;
   constexpr int PRE = T == 32 ? Epilogue::kPre : 0; // (64 x 64 tiles: others on the SM hide it)
-  __shared__ __align__(16) float sm[STAGES * C::SLOT + PRE * T * T];
+  extern __shared__ __align__(16) float sm[]; // C::bytes(Epilogue::kPre)
   float* pre = sm + STAGES * C::SLOT;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int t = blockIdx.x;
@@ -518,8 +521,9 @@ __global__ void __launch_bounds__(32 * W, T == 32 ? 20 / W : 4)
     {
       Fragment f0, f1;
       read(f0, a, b, 0);
+      const int left = K - k0;
 #pragma unroll 1
-      for (int k = 0; k < BK; k += 8)
+      for (int k = 0; k < BK && k < left; k += 8)
       {
         read(f1, a, b, k + 4);
         multiply(f0);

@@ -98,6 +98,29 @@ def test_large_launches_match_oracle(name, built_library, monkeypatch):
     _check(case, name)
 
 
+# Steps of twice the length (aligned rows, sums of 128 and more): sums that end with a step, one quad behind it, in a
+# step's last and first eight; rows of a tile that do not exist; on 32 x 32 tiles of four warps (two tiles an SM and
+# less), of two (up to five) and on 64 x 64 ones
+LONG = {
+    "four_warps_128": _case("dkp", [128, 128, 132, 128, 10], 33),
+    "four_warps_260": _case("simple", [260, 252, 248, 140, 12], 5, "sigmoid", mode="projection"),
+    "four_warps_batch": _case("full", [132, 256, 256, 132, 12], 129, "gelu", momentum=0.9),
+    "four_warps_adamw": _case("dkp", [128, 256, 260, 12], 128, "relu", lr=1e-3, optimizer="ADAMW"),
+    "two_warps": _case("dkp", [64, 320, 320, 320, 320, 100], 452, T=2),
+    "large": _case("dkp", [132, 1028, 1032, 100], 1000, T=2, steps=1),
+}
+
+
+@pytest.mark.parametrize("name", sorted(LONG))
+def test_long_steps_match_oracle(name, built_library, monkeypatch):
+    monkeypatch.setenv("DPC_DISABLE_RESIDENT", "1")
+    case, sms = LONG[name], _sms()
+    tiles = _tiles(case, 32, "forward")
+    assert tiles <= 2 * sms if name.startswith("four") else 3 * sms <= tiles <= 5 * sms if name == "two_warps" else \
+        _tiles(case, 64, "forward") >= 1.75 * sms
+    _check(case, name)
+
+
 @pytest.mark.parametrize("kind,sizes,batch,optimizer", [("dkp", [64, 1028, 1032, 12], 70, "ADAMW"),
                                                         ("full", [67, 1030, 1025, 7], 61, "ADAM")])
 def test_adam_updates_on_large_tiles(kind, sizes, batch, optimizer, built_library):
