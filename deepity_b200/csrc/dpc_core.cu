@@ -1526,7 +1526,7 @@ static int launch_psi_range(dpc_plan* p, int f, int c, int max_size, int grad_on
   }
   else
   {
-    dim3 g(std::max(1, cdiv(max_size, 64)), c);
+    dim3 g(std::max(1, cdiv(max_size, 32)), c, std::max(1, cdiv(ts, 16)));
     psi_update_kernel<<<g, 256, 0, st>>>(p->d, f, p->n, p->batch, p->e_terminal, grad_only);
   }
   return check_launch(p->ctx, grad_only ? "psi gradient kernel" : "psi_update kernel");

@@ -5,6 +5,9 @@
 // layer's own tile grid return at once.
 #pragma once
 #include <cuda_bf16.h>
+
+#include <type_traits>
+
 #include "dpc_math.cuh"
 
 namespace dpc
@@ -810,7 +813,7 @@ __device__ __forceinline__ void bias_apply(const dpc_layer& L, int j, float s, i
   }
 }
 
-// Bias update from the column sums of the local gradient: one thread per output unit,
+// Bias update from the column sums of the local gradient: a lane per output unit,
 // summing the batch in row order like CPUBackend::SumRows (CPUBackend.cpp:243-248).
 // Layers whose feedback error exists only as bf16 planes (see FePlanes) are summed by whole
 // blocks instead: 32 row groups x 8 threads of 8 columns each (16-byte loads of both planes,
@@ -899,59 +902,73 @@ __global__ void bias_update_kernel(const dpc_layer* __restrict__ layers, int fir
   }
   if (rank != 0)
     return; // (a row-split launch over a layer that takes the column sums: one CTA does them)
-  // Column sums in row order (the reference's): up to 32 columns at a time, the block copies groups of
-  // rows into shared memory, one buffer ahead, and one warp adds them up, a chain of dependent
-  // additions and nothing else.  (A thread that loads what it adds pays a memory latency every few
-  // rows: five 2048-wide layers and a ten-column head at batch 4096 took 145 us so, 113 with sixteen
-  // loads in flight and a barrier per group, 71 this way.)
-  constexpr int STAGE = 4096; // floats per buffer
-  __shared__ float stage[2][STAGE];
-  const int cols = n < 32 ? n : 32;
-  const int CR = STAGE / cols; // rows per buffer
+  // Column sums in row order (the reference's), 32 columns at a time: seven warps copy groups of rows into shared memory,
+  // three buffers ahead, the other one adds them up, a chain of dependent additions and nothing else.  It bounds the
+  // kernel, with the barrier of a group: 784-(91x4)-100 at batch 3584 281 -> 45 us a launch, 3072-(37x3)-16 at batch 768
+  // 204 -> 178 a step (76 us where all warps copied and seven then waited for the sums).
+  constexpr int STAGES = 4, ROWS = 64, AT_ONCE = 16;
+  __shared__ __align__(16) float stage[STAGES][ROWS][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int j0 = blockIdx.x * 32; j0 < n; j0 += gridDim.x * 32)
   {
-    const int width = min(cols, n - j0);
-    auto copy = [&](int b0, int buf)
+    const int j = j0 + lane;
+    auto copy = [&](int b0)
     {
-      const int total = max(0, min(CR, batch - b0)) * cols;
+      float* to = &stage[b0 / ROWS % STAGES][0][lane];
 #pragma unroll
-      for (int q = 0; q < STAGE / 256; ++q)
-      {
-        const int i = q * 256 + threadIdx.x, r = i / cols, c = i - r * cols;
-        if (i < total && c < width)
-        {
-          const size_t o = (size_t)(b0 + r) * n + j0 + c;
-          stage[buf][i] = hi ? __bfloat162float(hi[o]) + __bfloat162float(hi[planes.elems + o]) : g[o];
-        }
-      }
+      for (int r = warp - 1; r < ROWS; r += 7)
+        if (b0 + r < batch && j < n)
+          cp_async4(to + r * 32, g + (size_t)(b0 + r) * n + j, true);
+      asm volatile("cp.async.commit_group;" ::: "memory");
     };
     float s = 0.0f;
-    copy(0, 0);
-    for (int b0 = 0, buf = 0; b0 < batch; b0 += CR, buf ^= 1)
+    if (warp > 0)
+#pragma unroll 1
+      for (int q = 0; q < STAGES - 1; ++q)
+        copy(q * ROWS);
+#pragma unroll 1
+    for (int b0 = -ROWS; b0 < batch; b0 += ROWS)
     {
-      __syncthreads();
-      copy(b0 + CR, buf ^ 1);
-      if (threadIdx.x < (unsigned)width)
+      if (warp > 0)
       {
-        const int rows = min(CR, batch - b0);
-        const float* p = stage[buf] + threadIdx.x;
-        int r = 0;
-        for (; r + 16 <= rows; r += 16)
-        {
-          float v[16];
-#pragma unroll
-          for (int q = 0; q < 16; ++q)
-            v[q] = p[(r + q) * cols];
-#pragma unroll
-          for (int q = 0; q < 16; ++q)
-            s += v[q];
-        }
-        for (; r < rows; ++r)
-          s += p[r * cols];
+        if (b0 >= 0)
+          copy(b0 + (STAGES - 1) * ROWS);
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory"); // the next group of rows
       }
+      else if (b0 >= 0)
+      {
+        const int rows = min(ROWS, batch - b0);
+        const float* p = &stage[b0 / ROWS % STAGES][0][lane];
+        float v[2][AT_ONCE]; // (what is added next is read before these are)
+        auto read = [&](float (&x)[AT_ONCE], int r)
+        {
+#pragma unroll
+          for (int q = 0; q < AT_ONCE; ++q)
+            x[q] = p[(r + q) * 32];
+        };
+        auto add = [&](const float (&x)[AT_ONCE], int count)
+        {
+#pragma unroll
+          for (int q = 0; q < AT_ONCE; ++q)
+            if (q < count)
+              s += x[q];
+        };
+        read(v[0], 0);
+#pragma unroll
+        for (int r = 0; r < ROWS; r += 2 * AT_ONCE)
+        {
+          read(v[1], r + AT_ONCE);
+          add(v[0], rows - r);
+          if (r + 2 * AT_ONCE < ROWS)
+            read(v[0], r + 2 * AT_ONCE);
+          add(v[1], rows - r - AT_ONCE);
+        }
+      }
+      __syncthreads();
     }
-    if (threadIdx.x < (unsigned)width)
-      bias_apply(L, j0 + threadIdx.x, s, batch, grad_only);
+    if (warp == 0 && j < n)
+      bias_apply(L, j, s, batch, grad_only);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
   }
 }
@@ -1272,11 +1289,13 @@ __global__ void __launch_bounds__(256)
         weight_apply(L, (size_t)k * s + col + c, acc[c][k], batch, mode, flags, step);
 }
 
-// Feedback-weight update Psi[l] (+)= (fl*a/B) z[l]^T e_T.  A block of 256 threads owns 64 rows of
-// Psi (= 64 columns of z): thread (g, i) adds up the batch rows b = g, g+4, ... for column i with
-// the terminal columns in registers (chunks of 16), the four row groups are then summed in a
-// fixed order through shared memory.  The terminal errors of PSI_ROWS batch rows at a time go
-// through shared memory (zero padded to 16 columns).
+// Feedback-weight update Psi[l] (+)= (fl*a/B) z[l]^T e_T.  A block of 256 threads owns 32 rows of Psi (= 32 columns of z)
+// and 16 terminal columns: thread (g, q, i) adds up the batch rows b = g, g+4, ... for columns i, i+16 and terminal
+// columns 4q .. 4q+3, the four row groups are then summed in a fixed order through shared memory.  64 batch rows at a
+// time come into shared memory two buffers ahead.  What bounds it: the copies, element by element where rows are not
+// aligned, and the reads of shared memory.  (Blocks of 64 columns that walked the batch once for every 16 terminal
+// columns kept few SMs busy: 784-(91x4)-100 at batch 3584 1049 -> 113 us, 784-(500x3)-100
+// at batch 2000 603 -> 55; with 16 columns a block 109 and 89.)
 __global__ void __launch_bounds__(256)
     psi_update_kernel(const dpc_layer* __restrict__ layers, int first, int n_layers, int batch,
                       const float* __restrict__ eT, int grad_only)
@@ -1288,70 +1307,88 @@ __global__ void __launch_bounds__(256)
   if (L.next_size <= 0 || L.Psi == nullptr || (L.flags & DPC_LAYER_INPUT_ACT))
     return;
   const int TS = L.terminal_size, s = L.size;
-  const float step = psi_step(L, grad_only);
-  constexpr int PSI_ROWS = 64, GROUPS = 4, COLS = 64;
-  __shared__ __align__(16) float es[PSI_ROWS][16];
+  constexpr int ROWS = 64, GROUPS = 4, COLS = 32, STAGES = 3;
+  const int i0 = blockIdx.x * COLS, kc = blockIdx.z * 16;
+  if (i0 >= s || kc >= TS)
+    return;
+  __shared__ __align__(16) float es[STAGES][ROWS][16], zs[STAGES][ROWS][COLS];
   __shared__ float part[GROUPS][COLS][17];
-  const int g = threadIdx.x >> 6, ci = threadIdx.x & 63;
-  for (int i0 = blockIdx.x * COLS; i0 < s; i0 += gridDim.x * COLS)
+  const int tid = threadIdx.x, i = tid & 15, q = (tid >> 4) & 3, g = tid >> 6;
+  const int kn = min(16, TS - kc), width = min(COLS, s - i0);
+  const bool vec_z = s % 4 == 0 && aligned16(L.z), vec_e = TS % 4 == 0 && aligned16(eT);
+  // 64 rows from b0 of `count` columns (a multiple of 4 where they are copied by fours), zeros beyond
+  auto rows_of = [&](auto per_row, auto fours, float* to, const float* from, int ld, int b0, int count)
   {
-    const int i = i0 + ci;
-    for (int kc = 0; kc < TS; kc += 16)
+    constexpr int PER_ROW = decltype(per_row)::value, W = decltype(fours)::value ? 4 : 1, PER = PER_ROW / W;
+    const int c = tid % PER * W;
+#pragma unroll
+    for (int u = 0; u < ROWS * PER / 256; ++u)
     {
-      float acc[16];
-#pragma unroll
-      for (int k = 0; k < 16; ++k)
-        acc[k] = 0.0f;
-      const int kn = min(16, TS - kc);
-      for (int b0 = 0; b0 < batch; b0 += PSI_ROWS)
-      {
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < PSI_ROWS * 16; idx += blockDim.x)
-        {
-          const int r = idx >> 4, k = idx & 15;
-          es[r][k] = (b0 + r < batch && k < kn) ? eT[(size_t)(b0 + r) * TS + kc + k] : 0.0f;
-        }
-        __syncthreads();
-        if (i < s)
-        {
-          const int rows = min(PSI_ROWS, batch - b0);
+      const int r = tid / PER + u * (256 / PER);
+      const bool in = b0 + r < batch && c < count;
+      const float* src = in ? from + (size_t)(b0 + r) * ld + c : from;
+      if (W == 4)
+        cp_async16(to + r * PER_ROW + c, src, in);
+      else
+        cp_async4(to + r * PER_ROW + c, src, in);
+    }
+  };
+  auto copy = [&](int b0, int buf)
+  {
+    if (b0 < batch)
+    {
+      const std::integral_constant<int, COLS> columns;
+      const std::integral_constant<int, 16> terminals;
+      if (vec_z)
+        rows_of(columns, std::true_type(), &zs[buf][0][0], L.z + i0, s, b0, width);
+      else
+        rows_of(columns, std::false_type(), &zs[buf][0][0], L.z + i0, s, b0, width);
+      if (vec_e)
+        rows_of(terminals, std::true_type(), &es[buf][0][0], eT + kc, TS, b0, kn);
+      else
+        rows_of(terminals, std::false_type(), &es[buf][0][0], eT + kc, TS, b0, kn);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float acc[2][4] = {};
+#pragma unroll 1
+  for (int u = 0; u < STAGES - 1; ++u)
+    copy(u * ROWS, u);
+  const float step = psi_step(L, grad_only);
+  int buf = 0;
+#pragma unroll 1
+  for (int b0 = 0; b0 < batch; b0 += ROWS, buf = buf + 1 == STAGES ? 0 : buf + 1)
+  {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    __syncthreads(); // this buffer has landed, and everybody is done with the one that is filled now
+    copy(b0 + (STAGES - 1) * ROWS, buf == 0 ? STAGES - 1 : buf - 1);
+    const int rows = min(ROWS, batch - b0);
 #pragma unroll 4
-          for (int r = g; r < rows; r += GROUPS)
-          {
-            const float zv = L.z[(size_t)(b0 + r) * s + i];
+    for (int r = g; r < rows; r += GROUPS)
+    {
+      const float4 e4 = *reinterpret_cast<const float4*>(&es[buf][r][4 * q]);
 #pragma unroll
-            for (int k4 = 0; k4 < 16; k4 += 4)
-            {
-              const float4 e4 = *reinterpret_cast<const float4*>(&es[r][k4]);
-              acc[k4] = fmaf(zv, e4.x, acc[k4]);
-              acc[k4 + 1] = fmaf(zv, e4.y, acc[k4 + 1]);
-              acc[k4 + 2] = fmaf(zv, e4.z, acc[k4 + 2]);
-              acc[k4 + 3] = fmaf(zv, e4.w, acc[k4 + 3]);
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < 16; ++k)
-        part[g][ci][k] = acc[k];
-      __syncthreads();
-      // thread t < 64 * 4: column t / 4, terminal columns 4 (t % 4) .. +3
-      const int rc = threadIdx.x >> 2, k0 = (threadIdx.x & 3) * 4, row = i0 + rc;
-      if (row < s)
+      for (int c = 0; c < 2; ++c)
       {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-        {
-          const int k = k0 + q;
-          if (k >= kn)
-            continue;
-          const float sum = ((part[0][rc][k] + part[1][rc][k]) + part[2][rc][k]) + part[3][rc][k];
-          psi_apply(L, row, kc + k, sum, batch, grad_only, step);
-        }
+        const float zv = zs[buf][r][i + 16 * c];
+        acc[c][0] = fmaf(zv, e4.x, acc[c][0]);
+        acc[c][1] = fmaf(zv, e4.y, acc[c][1]);
+        acc[c][2] = fmaf(zv, e4.z, acc[c][2]);
+        acc[c][3] = fmaf(zv, e4.w, acc[c][3]);
       }
-      __syncthreads();
     }
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      part[g][i + 16 * c][4 * q + k] = acc[c][k];
+  __syncthreads();
+  const int k = tid & 15;
+  for (int row = tid >> 4; row < width && k < kn; row += 16)
+    psi_apply(L, i0 + row, kc + k, ((part[0][row][k] + part[1][row][k]) + part[2][row][k]) + part[3][row][k], batch,
+              grad_only, step);
 }
 
 // Applies staged gradients (the raw sums that the WG_GRAD_ONLY weight kernel and the grad_only

@@ -65,6 +65,11 @@ GROUPED = {
     "head_simple": _case("simple", [40, 384, 13], 2051, mode="python"),
     # column sums in row order: more than one group of 32 columns, rows that end inside a buffer
     "column_sums": _case("dkp", [24, 70, 33], 1031, "relu"),
+    # batches that end with a group of 64 rows, one row behind it, inside the first; feedback weights of one more
+    # terminal unit than 16, of three times 16, rows that are aligned and that are not
+    "batch_sums_64": _case("dkp", [36, 33, 17], 64, "relu"),
+    "batch_sums_257": _case("full", [32, 68, 64, 48], 257, "hard_tanh"),
+    "batch_sums_3": _case("dkp", [70, 31, 32, 20], 3, "relu"),
 }
 
 
