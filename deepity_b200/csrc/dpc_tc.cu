@@ -1931,6 +1931,8 @@ int launch(dpc_plan* p, TcState* st, const CUtensorMap& a, const CUtensorMap& b,
   return DPC_OK;
 }
 
+#include "dpc_sweep.cuh"
+
 bool range_in_run(const dpc_plan* p, int first, int count)
 {
   return p->run.count > 0 && count > 0 && first >= p->run.first &&
@@ -2559,6 +2561,26 @@ int tc_project_forward(dpc_plan* p, int first, int count, int flags)
   if (!st || !st->ok || !range_in_run(p, first, count) || count < 2 || st->simple)
     return 1;
   const int H = p->run.width, B = p->batch;
+  if (all_sgd(p) && (flags & DPC_FWD_COPY_NEXT))
+  {
+    // (the order of additions: see the K-split variant below)
+    const bool tf32 = p->ctx->precision == DPC_PRECISION_TF32;
+    const int r0 = first - p->run.first;
+    const TcParams P = base_params(p, st, first, count, B, H, H, 128, flags, 0);
+    int rc = 1;
+    if (tf32)
+      rc = launch_cluster_sweep<true>(p, st, st->w_km128, P);
+    else if (planes_on(p, st))
+    {
+      if ((rc = planes_need(p, st, PL_W, r0, r0 + count)) != DPC_OK)
+        return rc;
+      rc = launch_cluster_sweep<false>(p, st, st->wp_km128, P);
+    }
+    if (rc == DPC_OK)
+      planes_mark(st, PL_Z, r0 + 1, r0 + count + 1, planes_kept(p, st) ? 0 : 1);
+    if (rc <= 0)
+      return rc;
+  }
   // Narrow 128 x 32 tiles: B/128 * H/32 CTAs (128 for the 1024 x 512 layers of the deep-stack
   // benchmark) keep the epilogue and the publish step on the dependent path short.  (Tiles of
   // 64 rows were measured too: a tcgen05.mma costs about the same whatever M and N are, so

@@ -31,6 +31,8 @@
  *                              epilogues of the pair-tile kernels read / write global memory lane
  *                              by lane instead of through shared memory and bulk tensor copies
  *   DPC_DISABLE_KSPLIT         forward sweep without the two-CTA split of K
+ *   DPC_DISABLE_CLUSTER_SWEEP  forward sweep of runs of 256 or 512 units with tiles that hand their
+ *                              rows on through global memory instead of on thread-block clusters
  *   DPC_DISABLE_RECTANGULAR    single layers outside the run of identical square layers stay on
  *                              the CUDA-core kernels even where their shapes fit the pair tiles
  *   DPC_RECTANGULAR_MIN_WORK   such a layer goes to the pair tiles only when batch x inputs x

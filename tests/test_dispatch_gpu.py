@@ -47,6 +47,33 @@ def _check(case, name, precision="fp32"):
                     init=None if adam else initial_parameters(case), delta_tol=None if adam else delta)
 
 
+# The sweep on clusters: 8, 16 and 32 rows a cluster of two and four blocks, one and two waves of them, the shortest run,
+# beliefs with and without stored predictions, pre-activations and the residual term.  Smooth activations: a pre-activation
+# of 1 280 x 256 x 6 that rounds to the other side of a ReLU's kink moves a whole row (1e-3 of the largest error here with
+# the residual term, on these kernels and on the tiles alike; 5e-4 without it, on CUDA cores too).
+SWEEPS = {
+    "sweep_2x8_shortest": _case("dkp", [20] + [256] * 3 + [10], 256),
+    "sweep_2x16": _case("full", [20] + [256] * 5 + [10], 1024, "gelu"),
+    "sweep_2x32_residual": _case("full", [20] + [256] * 6 + [10], 1280, "tanh", residual=1),
+    "sweep_4x8": _case("dkp", [20] + [512] * 4 + [10], 256, "sigmoid"),
+    "sweep_4x16_residual": _case("full", [20] + [512] * 5 + [10], 512, "gelu", residual=1, momentum=0.9),
+    "sweep_4x32": _case("dkp", [20] + [512] * 4 + [10], 1024),
+    "sweep_4x32_two_waves": _case("dkp", [20] + [512] * 4 + [10], 1280, T=2, steps=1),
+}
+
+
+@pytest.mark.parametrize("precision", ["fp32", "tf32"])
+@pytest.mark.parametrize("name", list(SWEEPS))
+def test_cluster_sweep(name, precision, monkeypatch):
+    case = SWEEPS[name]
+    _check(case, name, precision)
+    # its products are summed in another order than the tiles' that it replaces: the same to rounding, not to the bit
+    own = run_gpu(case, precision=precision)
+    monkeypatch.setenv("DPC_DISABLE_CLUSTER_SWEEP", "1")
+    other = run_gpu(case, precision=precision)
+    assert any(not np.array_equal(own[key], other[key]) for key in own), "the case must sweep on clusters"
+
+
 GROUPED = {
     # 32 x 32 tiles: one row over a tile, K not a multiple of the stage, rows not 16-byte aligned
     "gemm_32_edges": _case("dkp", [33, 65, 31, 10], 65),
