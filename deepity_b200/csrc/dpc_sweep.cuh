@@ -194,20 +194,20 @@ __global__ void __launch_bounds__(kSweepThreads<ROWS>, 1)
         {
           const uint32_t more = ks > 0 || i > 0;
           if (TF32)
-            tc_mma_tf32_elect(tmem, da + (uint64_t)((ks >> 2) * (16384 >> 4) + (ks & 3) * (32 >> 4)),
+            tc_mma_tf32(tmem, da + (uint64_t)((ks >> 2) * (16384 >> 4) + (ks & 3) * (32 >> 4)),
                               db + (uint64_t)(ks * (1024 >> 4)), ONE, more);
           else
           {
-            tc_mma_bf16_elect(tmem, da + (uint64_t)(ks * (32 >> 4)), db + (uint64_t)(ks * (2048 >> 4)), BOTH, more);
-            tc_mma_bf16_elect(tmem + HALF, da + (uint64_t)((16384 + ks * 32) >> 4), db + (uint64_t)(ks * (2048 >> 4)), ONE, 1);
+            tc_mma_bf16(tmem, da + (uint64_t)(ks * (32 >> 4)), db + (uint64_t)(ks * (2048 >> 4)), BOTH, more);
+            tc_mma_bf16(tmem + HALF, da + (uint64_t)((16384 + ks * 32) >> 4), db + (uint64_t)(ks * (2048 >> 4)), ONE, 1);
           }
         }
-        tc_commit_elect(&empty[s]);
+        tc_commit(&empty[s]);
         if (++s == stages)
           s = 0, phase ^= 1;
       }
       if (alive)
-        tc_commit_elect(tfull);
+        tc_commit(tfull);
     }
   }
   else if (BULK && warp == 2 + 4 * GROUPS)

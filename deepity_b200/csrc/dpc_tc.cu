@@ -926,8 +926,8 @@ __global__ void __launch_bounds__(Cfg<OP, BN, THREE_X, BM, PAIR, KS>::THREADS, 1
   }
   else if (warp == 1)
   {
-    // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0 && leader)
+    // ---------------------------------------------------------------- MMA issuer (the warp together, one lane issues)
+    if (leader)
     {
       int s = 0, tile_iter = 0;
       uint32_t phase = 0; // parity to wait for on full[s] / xf[s]
@@ -955,22 +955,23 @@ __global__ void __launch_bounds__(Cfg<OP, BN, THREE_X, BM, PAIR, KS>::THREADS, 1
       for (int t = t_begin; t < t_end && alive; t += t_step, ++tile_iter)
       {
         const int acc = tile_iter & 1;
-        if (!(PAIR ? mbar_wait_cluster(&tempty[acc], ((tile_iter >> 1) & 1) ^ 1, abort_flag)
-                   : mbar_wait(&tempty[acc], ((tile_iter >> 1) & 1) ^ 1, abort_flag)))
+        if (!__all_sync(0xffffffffu,
+                        PAIR ? mbar_wait_cluster(&tempty[acc], ((tile_iter >> 1) & 1) ^ 1, abort_flag)
+                             : mbar_wait(&tempty[acc], ((tile_iter >> 1) & 1) ^ 1, abort_flag)))
           break;
         tc_fence_after();
         const uint32_t d_tmem0 = tmem_base + acc * (BN * C::NACC);
         for (int kb = 0; kb < kblocks; ++kb)
         {
           uint64_t* ready = C::SPLITW ? &xf[s] : &full[s];
-          if (!(PAIR ? mbar_wait_cluster(ready, phase, abort_flag)
-                     : mbar_wait(ready, phase, abort_flag)))
+          if (!__all_sync(0xffffffffu, PAIR ? mbar_wait_cluster(ready, phase, abort_flag)
+                                            : mbar_wait(ready, phase, abort_flag)))
           {
             alive = false;
             break;
           }
           tc_fence_after();
-          if (P.chain && kb == 0)
+          if (P.chain && kb == 0 && lane == 0)
             trace_stamp(P, t, 1);
           // Descriptors differ between stages and k-steps only in the 14-bit start-address
           // field (units of 16 bytes): one add per operand per instruction.

@@ -183,18 +183,24 @@ __device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* m
                "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_addr), "r"(c0), "r"(c1), "r"(c2)
                : "memory");
 }
+// Multiplications and commits are issued by one lane of a warp that is converged (the warp as a whole runs the loop around
+// them): the elected lane is known to the compiler, which keeps the descriptors in uniform registers.  40 cycles an
+// instruction, 125 where a branch of one lane formed them as it went.
 __device__ __forceinline__ void tc_commit_pair(uint32_t bar_addr)
 {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+  asm volatile("{\n\t.reg .pred q;\n\t"
+               "elect.sync _|q, 0xffffffff;\n\t"
+               "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
                    bar_addr)
                : "memory");
 }
 __device__ __forceinline__ void tc_mma_tf32_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                                  uint32_t idesc, uint32_t accumulate)
 {
-  asm volatile("{\n\t.reg .pred p;\n\t"
+  asm volatile("{\n\t.reg .pred p, q;\n\t"
+               "elect.sync _|q, 0xffffffff;\n\t"
                "setp.ne.b32 p, %4, 0;\n\t"
-               "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+               "@q tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
                "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
                : "memory");
 }
@@ -209,33 +215,14 @@ __device__ __forceinline__ void tc_fence_after()
 }
 __device__ __forceinline__ void tc_commit(uint64_t* bar)
 {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+  asm volatile("{\n\t.reg .pred q;\n\t"
+               "elect.sync _|q, 0xffffffff;\n\t"
+               "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
                    smem_u32(bar))
                : "memory");
 }
 __device__ __forceinline__ void tc_mma_tf32(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                             uint32_t idesc, uint32_t accumulate)
-{
-  asm volatile("{\n\t.reg .pred p;\n\t"
-               "setp.ne.b32 p, %4, 0;\n\t"
-               "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-               "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-               : "memory");
-}
-__device__ __forceinline__ void tc_mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                            uint32_t idesc, uint32_t accumulate)
-{
-  asm volatile("{\n\t.reg .pred p;\n\t"
-               "setp.ne.b32 p, %4, 0;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-               "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-               : "memory");
-}
-// The same issued by one lane of a warp that is converged: the elected lane is known to the compiler, which keeps the
-// descriptors in uniform registers (40 cycles an instruction where a branch of one lane that forms them as it goes took
-// 125 in the cluster sweep).
-__device__ __forceinline__ void tc_mma_tf32_elect(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                                  uint32_t accumulate)
 {
   asm volatile("{\n\t.reg .pred p, q;\n\t"
                "elect.sync _|q, 0xffffffff;\n\t"
@@ -244,8 +231,8 @@ __device__ __forceinline__ void tc_mma_tf32_elect(uint32_t d_tmem, uint64_t a_de
                "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
                : "memory");
 }
-__device__ __forceinline__ void tc_mma_bf16_elect(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                                  uint32_t accumulate)
+__device__ __forceinline__ void tc_mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                            uint32_t idesc, uint32_t accumulate)
 {
   asm volatile("{\n\t.reg .pred p, q;\n\t"
                "elect.sync _|q, 0xffffffff;\n\t"
@@ -254,19 +241,13 @@ __device__ __forceinline__ void tc_mma_bf16_elect(uint32_t d_tmem, uint64_t a_de
                "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
                : "memory");
 }
-__device__ __forceinline__ void tc_commit_elect(uint64_t* bar)
-{
-  asm volatile("{\n\t.reg .pred q;\n\t"
-               "elect.sync _|q, 0xffffffff;\n\t"
-               "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
-               : "memory");
-}
 __device__ __forceinline__ void tc_mma_bf16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                                  uint32_t idesc, uint32_t accumulate)
 {
-  asm volatile("{\n\t.reg .pred p;\n\t"
+  asm volatile("{\n\t.reg .pred p, q;\n\t"
+               "elect.sync _|q, 0xffffffff;\n\t"
                "setp.ne.b32 p, %4, 0;\n\t"
-               "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
                "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
                : "memory");
 }
