@@ -798,6 +798,50 @@ static bool narrow_forward(const dpc_plan* p, int layer)
          (!(L.flags & DPC_LAYER_INPUT_ACT) || (L.opt == DPC_OPT_SGD && ((uintptr_t)L.zF % 16) == 0));
 }
 
+template <int RPW, bool SIMPLE, bool SMEM>
+static int launch_narrow_forward(dpc_plan* p, int f, int c, int flags, int blocks, size_t weights)
+{
+  auto kern = narrow_forward_kernel<RPW, SIMPLE, SMEM>;
+  const size_t smem = sizeof(float) * kHeadRingFloats<RPW> + (SMEM ? weights : 0);
+  static thread_local int configured = -1; // (the limit is an attribute of a device)
+  if (configured != p->ctx->device)
+  {
+    DPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448 - 1024));
+    configured = p->ctx->device;
+  }
+  kern<<<dim3(blocks, 1, c), NTHREADS, smem, p->ctx->stream>>>(p->d, f, p->n, p->batch, flags, p->energy);
+  return check_launch(p->ctx, "narrow forward kernel");
+}
+
+static int narrow_forward_simt(dpc_plan* p, int f, int c, int flags, bool simple)
+{
+  size_t weights = 0;
+  for (int i = f; i < f + c; ++i)
+    if (p->h[i].next_size > 0)
+      weights = std::max(weights, sizeof(float) * (cdiv(p->h[i].next_size, 2) * 2) * ((size_t)cdiv(p->h[i].size, 512) * 512));
+  const bool staged = weights <= 160 * 1024; // (beside the ring)
+  // Single rows where pairs would leave SMs without a block (batch 256 x 256 -> 10: 4.1 us in 32 blocks); from 256 blocks of
+  // pairs two to four a warp, which share a copy of the weights (four from 64 blocks on: 16.7 us instead of 9.8 for 4096 x
+  // 1024 -> 10 alone, the same beside a tensor launch).
+  const int pair_blocks = cdiv(p->batch, 16);
+  if ((long long)pair_blocks * c < 64)
+  {
+    const int blocks = cdiv(p->batch, 8);
+    if (!staged)
+      return simple ? launch_narrow_forward<2, true, false>(p, f, c, flags, pair_blocks, 0)
+                    : launch_narrow_forward<2, false, false>(p, f, c, flags, pair_blocks, 0);
+    return simple   ? launch_narrow_forward<1, true, true>(p, f, c, flags, blocks, weights)
+                    : launch_narrow_forward<1, false, true>(p, f, c, flags, blocks, weights);
+  }
+  const int turns = (int)std::min<long long>(4, std::max<long long>(1, (long long)pair_blocks * c / 128));
+  const int blocks = cdiv(pair_blocks, turns);
+  if (!staged)
+    return simple ? launch_narrow_forward<2, true, false>(p, f, c, flags, blocks, 0)
+                  : launch_narrow_forward<2, false, false>(p, f, c, flags, blocks, 0);
+  return simple ? launch_narrow_forward<2, true, true>(p, f, c, flags, blocks, weights)
+                : launch_narrow_forward<2, false, true>(p, f, c, flags, blocks, weights);
+}
+
 static int forward_simt(dpc_plan* p, int first, int count, int flags)
 {
   cudaStream_t st = p->ctx->stream;
@@ -827,17 +871,10 @@ static int forward_simt(dpc_plan* p, int first, int count, int flags)
       const bool simple = (p->h[f].flags & DPC_LAYER_INPUT_ACT) != 0;
       if (narrow)
       {
-        if (p->batch >= 2048 && !simple) // (two rows of f(z) take too many registers)
-        {
-          dim3 grid(cdiv(p->batch, 2 * (NTHREADS / 32)), 1, c);
-          narrow_forward_kernel<2, false><<<grid, NTHREADS, 0, st>>>(p->d, f, p->n, p->batch, flags, p->energy);
-        }
-        else
-        {
-          dim3 grid(cdiv(p->batch, NTHREADS / 32), 1, c);
-          auto kern = simple ? narrow_forward_kernel<1, true> : narrow_forward_kernel<1, false>;
-          kern<<<grid, NTHREADS, 0, st>>>(p->d, f, p->n, p->batch, flags, p->energy);
-        }
+        const int rc = narrow_forward_simt(p, f, c, flags, simple);
+        if (rc != DPC_OK)
+          return rc;
+        continue;
       }
       else
       {
@@ -1131,17 +1168,27 @@ static int update_state_simt(dpc_plan* p, int first, int count)
     {
       // layers under a narrow one (the heads): 128 columns x a share of the batch rows per block
       int mxs = 0;
+      bool plain = true; // no momentum, no residual term
       for (int i = f; i < f + cg; ++i)
+      {
         mxs = std::max(mxs, p->h[i].size);
+        plain = plain && ((p->h[i].flags & DPC_LAYER_INPUT_ACT) || (!p->h[i].v && !(p->h[i].flags & DPC_LAYER_RESIDUAL)));
+      }
       const int gx = cdiv(mxs, 128);
       int rpb = cdiv(p->batch, 32) * 32;
       while (rpb > 32 && (long long)gx * cg * cdiv(p->batch, rpb) < p->ctx->sm_count)
         rpb = cdiv(rpb / 2, 32) * 32;
       dim3 grid(gx, cdiv(p->batch, rpb), cg);
-      if (narrow_kc <= 12)
-        narrow_state_kernel<12><<<grid, 256, 0, st>>>(p->d, f, p->n, p->batch, rpb);
-      else
-        narrow_state_kernel<16><<<grid, 256, 0, st>>>(p->d, f, p->n, p->batch, rpb);
+      auto kern = narrow_kc <= 12 ? (plain ? narrow_state_kernel<12, true> : narrow_state_kernel<12, false>)
+                                  : (plain ? narrow_state_kernel<16, true> : narrow_state_kernel<16, false>);
+      static thread_local int configured[4] = {-1, -1, -1, -1};
+      int& device = configured[2 * (narrow_kc <= 12) + plain];
+      if (device != p->ctx->device)
+      {
+        DPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeadStateSmem));
+        device = p->ctx->device;
+      }
+      kern<<<grid, 256, kHeadStateSmem, st>>>(p->d, f, p->n, p->batch, rpb);
       int rc = check_launch(p->ctx, "narrow update_state kernel");
       if (rc != DPC_OK)
         return rc;

@@ -124,10 +124,19 @@ __device__ __forceinline__ float warp_reduce16(float (&a)[16], int lane)
   return a[0] + __shfl_xor_sync(0xffffffffu, a[0], 1);
 }
 
-// RPW batch rows per warp (2 on large batches: every weight vector fetched from L1 then serves two
-// rows).  SIMPLE: SimplePC layers, whose operand is f(z).
-template <int RPW, bool SIMPLE>
-__global__ void __launch_bounds__(NTHREADS)
+// A block stages the weights once (SMEM; zeros fill chunks of 512 columns and an even number of rows) or reads them through
+// L1, and its warps take pairs of rows (RPW; single rows where the batch has few) in turn, a lane 16 of each 512 elements:
+// the copies of the next two chunks are under way meanwhile.  Two units at a time: a unit alone is one chain of additions.
+// SIMPLE: SimplePC layers, whose operand is f(z).
+// What bounds it: instructions (950 a warp and row of 1024 with tanh, half of them the activation) on few SMs -- 20 beside
+// a tensor launch take 80 us for 4096 rows, where the head must fit in --, one memory latency after another on many.  Alone,
+// us, rows that each began with their loads and then read the weights through L2 / this: 4096 x 1024 -> 10 12.3 / 9.8, as
+// SimplePC 15.4 / 13.9, 4096 x 2048 -> 16 32 / 19, 1024 x 512 -> 10 6.6 / 5.1, 256 x 256 -> 10 6.7 / 4.1.
+constexpr int kHeadRing = 2;
+template <int RPW>
+constexpr int kHeadRingFloats = (NTHREADS / 32) * kHeadRing * RPW * 512;
+template <int RPW, bool SIMPLE, bool SMEM>
+__global__ void __launch_bounds__(NTHREADS, 2)
     narrow_forward_kernel(const dpc_layer* __restrict__ layers, int first, int n_layers, int batch,
                           int flags, double* energy)
 {
@@ -135,43 +144,86 @@ __global__ void __launch_bounds__(NTHREADS)
   const dpc_layer L = layers[li];
   if (L.next_size <= 0)
     return;
-  const int N = L.next_size, K = L.size;
+  extern __shared__ __align__(16) float head_smem[];
+  const int N = L.next_size, K = L.size, KP = (K + 511) & ~511;
   constexpr bool simple = SIMPLE;
   const dpc_layer* Lup = (li + 1 < n_layers) ? &layers[li + 1] : nullptr;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = (blockIdx.x * (NTHREADS / 32) + warp) * RPW;
-  float acc[RPW][16];
-#pragma unroll
-  for (int r = 0; r < RPW; ++r)
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      acc[r][j] = 0.0f;
-  if (m0 < batch)
-  {
-    // 1024 elements of the rows at a time: the lane's eight 16-byte loads per row are all issued
-    // before the first use (4 KB in flight per row), then every weight row is walked over the
-    // same chunk
-    for (int kc = 0; kc < K; kc += 1024)
+  constexpr int WARPS = NTHREADS / 32, CH = 4; // a chunk: four 16-byte pieces a lane
+  const int chunks = KP / 512, stride = gridDim.x * WARPS * RPW;
+  float* head_w = head_smem + kHeadRingFloats<RPW>;
+  if (SMEM)
+    for (int i = threadIdx.x; i < ((N + 1) & ~1) * (KP / 4); i += NTHREADS)
     {
-      const int k0 = kc + lane * 4;
-      float4 zv[RPW][8];
+      const int j = i / (KP / 4), k = 4 * (i - j * (KP / 4));
+      const bool in = j < N && k < K;
+      cp_async16(&head_w[4 * i], in ? L.W + (size_t)j * K + k : L.W, in);
+    }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  // a lane copies and reads its own pieces: no barrier
+  float* ring = head_smem + (warp * kHeadRing * RPW) * 512 + lane * 4;
+  int slot = 0, fm = (blockIdx.x * WARPS + warp) * RPW, fc = 0; // the chunk to copy next
+  auto fetch = [&](int to)
+  {
+    if (fm < batch)
+    {
 #pragma unroll
       for (int r = 0; r < RPW; ++r)
-      {
-        const float* zrow = L.z + (size_t)(m0 + r) * K;
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-          zv[r][i] = (m0 + r < batch && k0 + i * 128 < K)
-                         ? *reinterpret_cast<const float4*>(zrow + k0 + i * 128)
-                         : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      }
+        for (int i = 0; i < CH; ++i)
+        {
+          const int k = fc * 512 + lane * 4 + i * 128;
+          const bool in = fm + r < batch && k < K;
+          cp_async16(ring + (to * RPW + r) * 512 + i * 128, in ? L.z + (size_t)(fm + r) * K + k : L.z, in);
+        }
+      if (++fc == chunks)
+        fc = 0, fm += stride;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  int m0 = fm;
+#pragma unroll
+  for (int q = 0; q < kHeadRing; ++q)
+    fetch(q);
+  if (SMEM)
+  {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kHeadRing) : "memory");
+    __syncthreads();
+  }
+  float esum = 0.0f;
+  const bool next_ce = Lup && (Lup->flags & DPC_LAYER_SOFTMAX_CE);
+  const bool do_err = (flags & DPC_FWD_ERR_NEXT) && Lup && !next_ce;
+  const bool do_fe =
+      (flags & DPC_FWD_FE) && Lup && !simple && !(next_ce && (flags & DPC_FWD_ERR_NEXT));
+  const bool do_copy = (flags & DPC_FWD_COPY_NEXT) && Lup;
+  const bool do_ce = next_ce && (flags & DPC_FWD_ERR_NEXT) && (flags & DPC_FWD_CE);
+  for (; m0 < batch; m0 += stride)
+  {
+    float acc[RPW][16];
+#pragma unroll
+    for (int r = 0; r < RPW; ++r)
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        acc[r][j] = 0.0f;
+    for (int kc = 0; kc < K; kc += 512)
+    {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kHeadRing - 1) : "memory");
+      float4 zv[RPW][CH];
+#pragma unroll
+      for (int r = 0; r < RPW; ++r)
+#pragma unroll
+        for (int i = 0; i < CH; ++i)
+          zv[r][i] = *reinterpret_cast<const float4*>(ring + (slot * RPW + r) * 512 + i * 128);
+      __syncwarp();
+      fetch(slot);
+      slot = slot + 1 == kHeadRing ? 0 : slot + 1;
       if (simple)
       {
         // the operand is f(z), kept for the weight update (src/layers/SimplePCLayer.cpp:146-150)
 #pragma unroll
         for (int r = 0; r < RPW; ++r)
 #pragma unroll
-          for (int i = 0; i < 8; i += 2)
+          for (int i = 0; i < CH; i += 2)
           {
             const float in[8] = {zv[r][i].x,     zv[r][i].y,     zv[r][i].z,     zv[r][i].w,
                                  zv[r][i + 1].x, zv[r][i + 1].y, zv[r][i + 1].z, zv[r][i + 1].w};
@@ -180,7 +232,7 @@ __global__ void __launch_bounds__(NTHREADS)
 #pragma unroll
             for (int q = 0; q < 2; ++q)
             {
-              const int k = k0 + (i + q) * 128;
+              const int k = kc + lane * 4 + (i + q) * 128;
               const bool in_range = m0 + r < batch && k < K;
               zv[r][i + q] = in_range ? make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3])
                                       : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -190,106 +242,105 @@ __global__ void __launch_bounds__(NTHREADS)
           }
       }
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
+      for (int j = 0; j < 16; j += 2)
       {
         if (j < N)
         {
-          const float* wrow = L.W + (size_t)j * K + k0;
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
+          for (int i = 0; i < CH; ++i)
           {
-            if (k0 + i * 128 < K)
-            {
-              const float4 wv = __ldg(reinterpret_cast<const float4*>(wrow + i * 128));
+            const int k = kc + lane * 4 + i * 128;
+            float4 wv[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+              if (SMEM)
+                wv[h] = *reinterpret_cast<const float4*>(&head_w[(j + h) * KP + k]);
+              else
+                wv[h] = j + h < N && k < K ? __ldg(reinterpret_cast<const float4*>(L.W + (size_t)(j + h) * K + k))
+                                           : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
 #pragma unroll
               for (int r = 0; r < RPW; ++r)
               {
-                acc[r][j] = fmaf(zv[r][i].x, wv.x, acc[r][j]);
-                acc[r][j] = fmaf(zv[r][i].y, wv.y, acc[r][j]);
-                acc[r][j] = fmaf(zv[r][i].z, wv.z, acc[r][j]);
-                acc[r][j] = fmaf(zv[r][i].w, wv.w, acc[r][j]);
+                acc[r][j + h] = fmaf(zv[r][i].x, wv[h].x, acc[r][j + h]);
+                acc[r][j + h] = fmaf(zv[r][i].y, wv[h].y, acc[r][j + h]);
+                acc[r][j + h] = fmaf(zv[r][i].z, wv[h].z, acc[r][j + h]);
+                acc[r][j + h] = fmaf(zv[r][i].w, wv[h].w, acc[r][j + h]);
               }
-            }
           }
         }
       }
     }
-  }
-  float esum = 0.0f;
-  const bool next_ce = Lup && (Lup->flags & DPC_LAYER_SOFTMAX_CE);
-  const bool do_err = (flags & DPC_FWD_ERR_NEXT) && Lup && !next_ce;
-  const bool do_fe =
-      (flags & DPC_FWD_FE) && Lup && !simple && !(next_ce && (flags & DPC_FWD_ERR_NEXT));
-  const bool do_copy = (flags & DPC_FWD_COPY_NEXT) && Lup;
-  const bool do_ce = next_ce && (flags & DPC_FWD_ERR_NEXT) && (flags & DPC_FWD_CE);
 #pragma unroll
-  for (int r = 0; r < RPW; ++r)
-  {
-    // lanes 2n and 2n+1 end with the sum of output unit n; the even one finishes it
-    const float mine = warp_reduce16(acc[r], lane);
-    const int m = m0 + r, n = lane >> 1;
-    float out_pre = 0.0f, out_mu = 0.0f;
-    if (m < batch && !(lane & 1) && n < N)
+    for (int r = 0; r < RPW; ++r)
     {
-      const size_t o = (size_t)m * N + n;
-      const float pre = L.a * mine + L.b[n];
-      float mu, d = 1.0f;
-      if (simple)
-        mu = pre;
-      else if (do_fe)
-        act_both(L.act, pre, mu, d);
-      else
-        mu = act_fwd(L.act, pre);
-      if (!simple && (L.flags & DPC_LAYER_RESIDUAL))
-        mu += L.z[o];
-      out_pre = pre, out_mu = mu;
-      if (!(flags & DPC_FWD_TRANSIENT))
+      // lanes 2n and 2n+1 end with the sum of output unit n; the even one finishes it
+      const float mine = warp_reduce16(acc[r], lane);
+      const int m = m0 + r, n = lane >> 1;
+      float out_pre = 0.0f, out_mu = 0.0f;
+      if (m < batch && !(lane & 1) && n < N)
       {
-        const bool no_mu = do_copy && (flags & DPC_FWD_NO_MU);
-        if (L.preact && !(no_mu && (flags & DPC_FWD_NO_PREACT)))
-          L.preact[o] = pre;
-        if (!no_mu)
-          L.mu[o] = mu;
+        const size_t o = (size_t)m * N + n;
+        const float pre = L.a * mine + L.b[n];
+        float mu, d = 1.0f;
+        if (simple)
+          mu = pre;
+        else if (do_fe)
+          act_both(L.act, pre, mu, d);
+        else
+          mu = act_fwd(L.act, pre);
+        if (!simple && (L.flags & DPC_LAYER_RESIDUAL))
+          mu += L.z[o];
+        out_pre = pre, out_mu = mu;
+        if (!(flags & DPC_FWD_TRANSIENT))
+        {
+          const bool no_mu = do_copy && (flags & DPC_FWD_NO_MU);
+          if (L.preact && !(no_mu && (flags & DPC_FWD_NO_PREACT)))
+            L.preact[o] = pre;
+          if (!no_mu)
+            L.mu[o] = mu;
+        }
+        if (do_copy)
+          Lup->z[o] = mu;
+        float e = 0.0f;
+        if (do_err)
+        {
+          e = (do_copy ? mu : Lup->z[o]) - mu;
+          Lup->e[o] = e;
+          esum += e * e;
+        }
+        else if (do_fe)
+          e = Lup->e[o];
+        if (do_fe)
+          L.fe[o] = e * d;
       }
-      if (do_copy)
-        Lup->z[o] = mu;
-      float e = 0.0f;
-      if (do_err)
+      if (do_ce)
       {
-        e = (do_copy ? mu : Lup->z[o]) - mu;
-        Lup->e[o] = e;
-        esum += e * e;
-      }
-      else if (do_fe)
-        e = Lup->e[o];
-      if (do_fe)
-        L.fe[o] = e * d;
-    }
-    if (do_ce)
-    {
-      // Softmax cross-entropy error of the layer above (softmax_ce_kernel and feedback_error_kernel in
-      // their order of operations): unit j moves to lane j.
-      const float logit = __shfl_sync(0xffffffffu, out_mu, 2 * lane & 31);
-      const float pre = __shfl_sync(0xffffffffu, out_pre, 2 * lane & 31);
-      const bool in = lane < N;
-      float mx = in ? logit : -INFINITY;
+        // Softmax cross-entropy error of the layer above (softmax_ce_kernel and feedback_error_kernel in
+        // their order of operations): unit j moves to lane j.
+        const float logit = __shfl_sync(0xffffffffu, out_mu, 2 * lane & 31);
+        const float pre = __shfl_sync(0xffffffffu, out_pre, 2 * lane & 31);
+        const bool in = lane < N;
+        float mx = in ? logit : -INFINITY;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      float s = in ? expf(logit - mx) : 0.0f;
+        for (int o = 16; o > 0; o >>= 1)
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        float s = in ? expf(logit - mx) : 0.0f;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
-        s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (in && m < batch)
-      {
-        const size_t o = (size_t)m * N + lane;
-        const float p = expf(logit - mx) / s;
-        const float z = do_copy ? logit : Lup->z[o];
-        esum -= 2.0f * z * logf(p + 1e-8f); // (halved with the Gaussian energies)
-        const float e = z - p;
-        Lup->e[o] = e;
-        if ((flags & DPC_FWD_FE) && !simple)
-          L.fe[o] = e * act_deriv(L.act, pre);
+        for (int o = 16; o > 0; o >>= 1)
+          s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (in && m < batch)
+        {
+          const size_t o = (size_t)m * N + lane;
+          const float p = expf(logit - mx) / s;
+          const float z = do_copy ? logit : Lup->z[o];
+          esum -= 2.0f * z * logf(p + 1e-8f); // (halved with the Gaussian energies)
+          const float e = z - p;
+          Lup->e[o] = e;
+          if ((flags & DPC_FWD_FE) && !simple)
+            L.fe[o] = e * act_deriv(L.act, pre);
+        }
       }
     }
   }
@@ -1134,8 +1185,15 @@ __global__ void __launch_bounds__(256)
 // every warp keeps the weights of columns 4l..4l+3 in registers, a block owns 128 columns and
 // `rows_per_block` batch rows, warp w the rows w, w+8, ...; the rows of the feedback error go
 // through shared memory 128 at a time.  Same arithmetic per element as GemmEpilogue::state.
-template <int KC>
-__global__ void __launch_bounds__(256)
+// PLAIN: no momentum, no residual term.  What bounds it: latency times bytes in flight, so eight rows a warp (PLAIN, else
+// four) are under way as copies into shared memory (one row, because the next one's loads could not pass this one's
+// stores, took 117 us of 4096 x 1024 on the 20 SMs beside a tensor launch, four in registers 71, this 65; SimplePC, which
+// forms tanh' too, 105 with four in registers, 88).
+template <bool PLAIN>
+constexpr int kHeadStateRing = PLAIN ? 8 : 4; // rows a warp has under way
+constexpr int kHeadStateSmem = 8 * 4 * 4 * 128 * 4;
+template <int KC, bool PLAIN>
+__global__ void __launch_bounds__(256, 2)
     narrow_state_kernel(const dpc_layer* __restrict__ layers, int first, int n_layers, int batch,
                         int rows_per_block)
 {
@@ -1152,10 +1210,35 @@ __global__ void __launch_bounds__(256)
   if ((int)blockIdx.x * 128 >= s)
     return;
   const float* g = simple ? Lup->e : L.fe;
-  constexpr int ROWS = 128;
+  constexpr int ROWS = 128, D = kHeadStateRing<PLAIN>, PIECES = PLAIN ? 2 : 4;
   __shared__ __align__(16) float gs[ROWS][KC];
+  extern __shared__ __align__(16) float state_ring[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = blockIdx.x * 128 + lane * 4;
+  const int b_begin = blockIdx.y * rows_per_block;
+  const int b_end = min(batch, b_begin + rows_per_block);
+  // a lane copies and reads its own pieces of the warp's rows: no barrier
+  float* ring = state_ring + warp * D * PIECES * 128 + lane * 4;
+  int fr = b_begin + warp; // the row to copy next
+  auto fetch = [&](int to)
+  {
+    if (fr < b_end)
+    {
+      const size_t o = (size_t)fr * s + col;
+      float* d = ring + to * PIECES * 128;
+      cp_async16(d, L.e + o, true);
+      cp_async16(d + 128, L.z + o, true);
+      if (!PLAIN && !simple && L.v)
+        cp_async16(d + 256, L.v + o, true);
+      if (!PLAIN && !simple && residual)
+        cp_async16(d + 384, Lup->e + o, true);
+    }
+    fr += 8;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int q = 0; q < D; ++q)
+    fetch(q);
   float w[4][KC];
 #pragma unroll
   for (int k = 0; k < KC; ++k)
@@ -1165,8 +1248,7 @@ __global__ void __launch_bounds__(256)
       w4 = *reinterpret_cast<const float4*>(L.W + (size_t)k * s + col);
     w[0][k] = w4.x, w[1][k] = w4.y, w[2][k] = w4.z, w[3][k] = w4.w;
   }
-  const int b_begin = blockIdx.y * rows_per_block;
-  const int b_end = min(batch, b_begin + rows_per_block);
+  int slot = 0;
   for (int b0 = b_begin; b0 < b_end; b0 += ROWS)
   {
     __syncthreads();
@@ -1177,17 +1259,21 @@ __global__ void __launch_bounds__(256)
     }
     __syncthreads();
     const int rows = min(ROWS, b_end - b0);
-#pragma unroll 4
     for (int r = warp; r < rows; r += 8)
     {
-      const size_t o = (size_t)(b0 + r) * s + col;
-      const float4 e4 = *reinterpret_cast<const float4*>(L.e + o);
-      const float4 z4 = *reinterpret_cast<const float4*>(L.z + o);
+      asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
+      const float* piece = ring + slot * PIECES * 128;
+      const float4 e4 = *reinterpret_cast<const float4*>(piece);
+      const float4 z4 = *reinterpret_cast<const float4*>(piece + 128);
       float4 v4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), u4 = v4;
-      if (!simple && L.v)
-        v4 = *reinterpret_cast<const float4*>(L.v + o);
-      if (!simple && residual)
-        u4 = *reinterpret_cast<const float4*>(Lup->e + o);
+      if (!PLAIN && !simple && L.v)
+        v4 = *reinterpret_cast<const float4*>(piece + 256);
+      if (!PLAIN && !simple && residual)
+        u4 = *reinterpret_cast<const float4*>(piece + 384);
+      __syncwarp();
+      fetch(slot);
+      slot = (slot + 1) & (D - 1);
+      const size_t o = (size_t)(b0 + r) * s + col;
       float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
       for (int k4 = 0; k4 < KC; k4 += 4)
@@ -1217,18 +1303,18 @@ __global__ void __launch_bounds__(256)
         else
         {
           const float fb = L.a * acc[c] - ee[c];
-          if (L.v)
+          if (!PLAIN && L.v)
           {
             vv[c] = L.momentum_beta * vv[c] + (1.0f - L.momentum_beta) * fb;
             zz[c] += L.ir * vv[c];
           }
           else
             zz[c] += L.ir * fb;
-          if (residual)
+          if (!PLAIN && residual)
             zz[c] += L.ir * uu[c];
         }
       }
-      if (!simple && L.v)
+      if (!PLAIN && !simple && L.v)
         *reinterpret_cast<float4*>(L.v + o) = make_float4(vv[0], vv[1], vv[2], vv[3]);
       *reinterpret_cast<float4*>(L.z + o) = make_float4(zz[0], zz[1], zz[2], zz[3]);
     }

@@ -1895,13 +1895,12 @@ int launch(dpc_plan* p, TcState* st, const CUtensorMap& a, const CUtensorMap& b,
     // one cluster of two CTAs per work item, as many clusters as SM pairs (the sweep: one
     // cluster per tile, all of them resident at once)
     int pairs = P.chain ? P.tiles_m * P.tiles_n : std::min(total, p->ctx->sm_count / 2);
-    if (!P.chain && !C::PRE)
+    if (!P.chain)
     {
       // No more pairs than the number of waves needs: 192 tiles take three on 64 pairs as on 74, and the SMs that are
-      // left run the head and the cached input of the phase meanwhile (3072-(1024x4)-10 with Adam at batch 4096 8.10 ->
-      // 8.00 ms a step, 512-(512x12)-10 tf32 474 -> 459 us).  Not the kernels on operand planes, which wait for L2
-      // rather than for their own SM: with the head's traffic beside them all the time 784-(1024x4)-10 took 5.04 ms
-      // instead of 5.00.
+      // left run the head and the cached input of the phase meanwhile (784-(1024x4)-10 SimplePC at batch 4096 4.60 ->
+      // 3.96 ms a step, 3072-(1024x4)-10 with Adam 8.10 -> 8.00, 512-(512x12)-10 tf32 474 -> 459 us).  The head must fit
+      // into the launch's time there: with one that took 110 us of 20 SMs beside 85 the first of these was 1 % slower.
       const int waves = (total + pairs - 1) / pairs;
       pairs = (total + waves - 1) / waves;
     }

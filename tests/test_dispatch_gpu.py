@@ -90,6 +90,13 @@ GROUPED = {
     "head_ce_two_rows": _case("full", [40, 132, 16], 2051, cross_entropy=1),
     "head_simple_ce": _case("simple", [40, 256, 10], 259, mode="projection", cross_entropy=1),
     "head_simple": _case("simple", [40, 384, 13], 2051, mode="python"),
+    # ... several pairs of rows a warp, an odd number of units, a second chunk of 512 that is not full; weights beyond shared
+    # memory; momentum and 14 units in the state update, rows that end inside its ring
+    "head_turns": _case("dkp", [40, 640, 9], 4099),
+    "head_unstaged": _case("full", [20, 2564, 15], 67),
+    "head_unstaged_simple": _case("simple", [20, 2568, 16], 1030, mode="projection"),
+    "head_state_momentum": _case("full", [40, 256, 14], 301, "gelu", momentum=0.9),
+    "head_state_simple_16": _case("simple", [40, 128, 14], 1027, mode="projection"),
     # column sums in row order: more than one group of 32 columns, rows that end inside a buffer
     "column_sums": _case("dkp", [24, 70, 33], 1031, "relu"),
     # batches that end with a group of 64 rows, one row behind it, inside the first; feedback weights of one more
