@@ -5,24 +5,24 @@
 // layer for the cluster's 8, 16 or 32 rows -- D[output][row], so that the weights are the 128-row operand A of
 // tcgen05.mma and the beliefs the operand B -- and hands them, as operands of the next layer, to the other blocks: with
 // st.async, or where a block's 128 k are whole 128-byte rows (32 rows) as bulk copies, either way counted in bytes on a
-// barrier of their source.  A block multiplies its own outputs first and the others' as they come.  Weights stream
+// barrier of their source.  A block multiplies its own half of K first.  Weights stream
 // through a TMA ring that does not wait for anything of the chain.
 //
 //   beliefs      [k][rows], 128 bytes a k: the rows' bf16 "hi" values, then their "mid" values, one MN-major block
 //                (128-byte swizzle), or up to 32 fp32 values (TF32: swizzle of 32-byte units); two buffers
-//   products     bf16 planes: A_hi x [B_hi B_mid], A_mid x B_hi onto the latter, the epilogue adds the two sums; TF32: one
-//                pass.  (A_mid x B_hi onto the large sum cost 2 to 8 % in accuracy against 64 bits; so the beliefs are
-//                as exact as the tiles'.)  The three terms of the settling passes: with the fourth, an error z - mu
-//                that is rounding grew to 1e-6
+//   products     two sums, one per half of K, that the epilogue adds: the K-split tiles' order of additions, so that their
+//                bits stay (the errors right after a sweep are its rounding against the settling passes': another order
+//                of the same accuracy moved those of 512 layers by 1e-3).  bf16 planes: x_hi w_hi and x_mid w_hi onto one
+//                accumulator, x_hi w_mid onto another; TF32: one pass
 //   fp32 beliefs and operand planes in global memory are written beside the next layer's multiplications
 //
-// What bounds a layer, in cycles of 512 units and 32 rows (bf16; 8 500 in all, 7 300 with TF32): 64 multiplications, 4 500
-// (40 each where nothing else reads shared memory), tensor memory -> activation -> own shared memory 1 500, waits for the
-// second block's outputs 700 (between blocks 15 to 20 bytes a cycle leave an SM whichever instruction moves them; sent
-// without an order of the targets they took 1 550) and for weights 1 200 (a layer's 256 KB an SM at 30 bytes a cycle).
-// us of 24 layers, tiles that publish their rows in global memory -> this: 512 units at batch 256 168 -> 86, 512 177 -> 106,
-// 1024 176 -> 114 (TF32 168 -> 100), 2048 387 -> 226; 256 units at batch 256 148 -> 48, 1024 155 -> 55, 4096 284 -> 147,
-// 8192 367 -> 291.
+// What bounds a layer, in cycles of 512 units and 32 rows (bf16; 9 500 in all, 7 300 with TF32): 96 multiplications (40 each
+// where nothing else reads shared memory), tensor memory -> activation -> own shared memory 1 500, waits for the other
+// blocks' outputs 700 (between blocks 15 to 20 bytes a cycle leave an SM whichever instruction moves them; sent without an
+// order of the targets they took 1 550) and for weights 1 200 (a layer's 256 KB an SM at 30 bytes a cycle).
+// us, tiles that publish their rows in global memory -> this: 512 layers of 512 units at batch 1024 4202 -> 2845; 12 of
+// them with TF32 88 -> 60; 24 of 512 at batch 256 168 -> 100; 8 of 256 units at batch 256 44 -> 19, 29 residual ones
+// 203 -> 66; 24 of 256 at batch 2048 150 -> 90.
 #pragma once
 
 template <int ROWS>
@@ -36,6 +36,7 @@ __global__ void __launch_bounds__(kSweepThreads<ROWS>, 1)
   constexpr int GROUPS = ROWS / 8;            // of four epilogue warps
   constexpr bool BULK = ROWS == 32;
   constexpr int HALF = ROWS < 16 ? 16 : ROWS; // columns of the "hi" values (N of an instruction is a multiple of 16)
+  constexpr uint32_t COLUMNS = 4 * HALF;      // tensor memory: "hi" and "mid" sums of each half of K
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* zbuf = smem; // two buffers of H x 128 bytes
@@ -73,10 +74,12 @@ __global__ void __launch_bounds__(kSweepThreads<ROWS>, 1)
   if (warp == 1)
   {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_holder)),
-                 "r"(64u)
+                 "r"(COLUMNS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  // The block whose outputs are multiplied i-th: the own half of K first, each half in ascending order.
+  auto source = [&](int i) { return blocks == 2 ? (int)rank ^ i : (((int)rank & 2) ^ (i & 2)) | (i & 1); };
   // Eight rows of one k as operand values: two 16-byte chunks at these offsets of a buffer.
   auto chunk = [](int k, int rows8, int half)
   {
@@ -129,7 +132,7 @@ __global__ void __launch_bounds__(kSweepThreads<ROWS>, 1)
         const int layer = P.first + l - P.run_first;
         for (int i = 0; i < blocks * SOURCE_KB; ++i)
         {
-          const int kb = (SOURCE_KB * (int)rank + i) & (blocks * SOURCE_KB - 1);
+          const int kb = SOURCE_KB * source(i / SOURCE_KB) + i % SOURCE_KB;
           if (!mbar_wait(&empty[s], phase, abort_flag))
           {
             alive = false;
@@ -165,6 +168,7 @@ __global__ void __launch_bounds__(kSweepThreads<ROWS>, 1)
     constexpr uint32_t BYTES = BULK ? 128 * 128 : 128 * 4 * ROWS;
     const uint64_t da0 = make_desc(smem_u32(ring), 16, 1024, 2);
     const uint64_t db0 = make_desc(smem_u32(zbuf), 8192, TF32 ? 512 : 1024, TF32 ? 1 : 2);
+    const int half_kb = blocks * SOURCE_KB / 2;
     int s = 0;
     uint32_t phase = 0;
     bool alive = true;
@@ -177,7 +181,7 @@ __global__ void __launch_bounds__(kSweepThreads<ROWS>, 1)
       __syncwarp();
       for (int i = 0; i < blocks * SOURCE_KB; ++i)
       {
-        const int kb = (SOURCE_KB * (int)rank + i) & (blocks * SOURCE_KB - 1);
+        const int kb = SOURCE_KB * source(i / SOURCE_KB) + i % SOURCE_KB;
         if (l > 0 && i % SOURCE_KB == 0)
         {
           alive = __all_sync(0xffffffffu, mbar_wait_cluster(&ready[kb / SOURCE_KB], ((l - 1) >> 1) & 1, abort_flag));
@@ -187,19 +191,22 @@ __global__ void __launch_bounds__(kSweepThreads<ROWS>, 1)
         if (!alive)
           break;
         tc_fence_after();
+        const uint32_t sum = tmem + (uint32_t)(i < half_kb ? 0 : 2 * HALF);
         const uint64_t da = da0 + (uint64_t)(s * (STAGE_BYTES >> 4));
         const uint64_t db = db0 + (uint64_t)(((l & 1) * H + kb * KB) * (128 >> 4));
 #pragma unroll
         for (int ks = 0; ks < (TF32 ? 8 : 4); ++ks)
         {
-          const uint32_t more = ks > 0 || i > 0;
+          const uint32_t more = ks > 0 || i % half_kb != 0;
           if (TF32)
-            tc_mma_tf32(tmem, da + (uint64_t)((ks >> 2) * (16384 >> 4) + (ks & 3) * (32 >> 4)),
+            tc_mma_tf32(sum, da + (uint64_t)((ks >> 2) * (16384 >> 4) + (ks & 3) * (32 >> 4)),
                               db + (uint64_t)(ks * (1024 >> 4)), ONE, more);
           else
           {
-            tc_mma_bf16(tmem, da + (uint64_t)(ks * (32 >> 4)), db + (uint64_t)(ks * (2048 >> 4)), BOTH, more);
-            tc_mma_bf16(tmem + HALF, da + (uint64_t)((16384 + ks * 32) >> 4), db + (uint64_t)(ks * (2048 >> 4)), ONE, 1);
+            const uint64_t wh = da + (uint64_t)(ks * (32 >> 4)), bh = db + (uint64_t)(ks * (2048 >> 4));
+            tc_mma_bf16(sum, wh, bh, ONE, more);
+            tc_mma_bf16(sum, wh, bh + (uint64_t)((2 * HALF) >> 4), ONE, 1);
+            tc_mma_bf16(sum + HALF, wh + (uint64_t)(16384 >> 4), bh, ONE, more);
           }
         }
         tc_commit(&empty[s]);
@@ -222,7 +229,7 @@ __global__ void __launch_bounds__(kSweepThreads<ROWS>, 1)
         const int buffer = (l + 1) & 1;
         for (int b = 1; b < blocks && alive; ++b)
         {
-          const uint32_t to = (rank - (uint32_t)b) & (uint32_t)(blocks - 1);
+          const uint32_t to = rank ^ (uint32_t)b;
           const uint32_t ready = mapa_u32(smem_u32(&zfull[4 * buffer + rank]), to);
           for (int q = 0; q < 4; ++q)
           {
@@ -261,8 +268,9 @@ __global__ void __launch_bounds__(kSweepThreads<ROWS>, 1)
       if (!__all_sync(0xffffffffu, mbar_wait(tfull, l & 1, abort_flag))) // (the warp gives up as a whole)
         break;
       tc_fence_after();
-      float pre[8];
+      float pre[8], half1[8]; // the two halves of K, each "hi" + "mid"
       tc_ld8(taddr, pre);
+      tc_ld8(taddr + (uint32_t)(2 * HALF), half1);
       if (!TF32)
       {
         float m[8];
@@ -270,7 +278,14 @@ __global__ void __launch_bounds__(kSweepThreads<ROWS>, 1)
 #pragma unroll
         for (int r = 0; r < 8; ++r)
           pre[r] += m[r];
+        tc_ld8(taddr + (uint32_t)(3 * HALF), m);
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+          half1[r] += m[r];
       }
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        pre[r] += half1[r];
       tc_fence_before(); // the accumulator is free when the next layer's operands are complete
       float f[8], d[8];
 #pragma unroll
@@ -306,7 +321,7 @@ __global__ void __launch_bounds__(kSweepThreads<ROWS>, 1)
             const uint32_t at = smem_u32(next + chunk(j, grp, half));
             for (int b = 1; b < blocks; ++b)
             {
-              const uint32_t to = (rank - (uint32_t)b) & (uint32_t)(blocks - 1);
+              const uint32_t to = rank ^ (uint32_t)b;
               asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 "
                            "[%0], {%1, %2, %3, %4}, [%5];" ::"r"(mapa_u32(at, to)),
                            "r"(out[half].x), "r"(out[half].y), "r"(out[half].z), "r"(out[half].w),
@@ -357,7 +372,7 @@ __global__ void __launch_bounds__(kSweepThreads<ROWS>, 1)
   if (warp == 1)
   {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(64u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLUMNS) : "memory");
   }
 }
 
@@ -368,16 +383,14 @@ int launch_cluster_sweep(dpc_plan* p, TcState* st, const CUtensorMap& w, const T
   const int H = p->run.width, B = p->batch, blocks = H / 128;
   if (getenv("DPC_DISABLE_CLUSTER_SWEEP") || (H != 256 && H != 512) || st->trace)
     return 1;
+  // Where the tiles would split K (their bits stay), and one wave of clusters is enough.  Larger batches fill the SMs with
+  // tiles; several waves of clusters took as long (24 layers of 512 units at batch 4096 453 us, a launch a layer 425).
+  if (2 * (B / TBM) * (H / 64) > p->ctx->sm_count || getenv("DPC_DISABLE_KSPLIT"))
+    return 1;
   // As few rows a cluster as there are SMs for, so that every layer's epilogue and exchange are short.
   int rows = 8;
   while (rows < 32 && (B / rows) * blocks > p->ctx->sm_count * 7 / 8)
     rows *= 2;
-  if (B % rows != 0)
-    return 1;
-  // A third wave of clusters costs more than a launch a layer (512 units: batch 4096 453 us of 24 layers against 425, 8192
-  // 907 against 680); clusters of two blocks have four for less (above).
-  if (H == 512 && (B / rows) * blocks > 2 * p->ctx->sm_count)
-    return 1;
   const int stages = (232448 - 1024 - 512 - 2 * H * 128) / 32768;
   const int smem = 2 * H * 128 + stages * 32768 + 1024 + 512;
   if (smem > st->max_smem)

@@ -2563,7 +2563,7 @@ int tc_project_forward(dpc_plan* p, int first, int count, int flags)
   const int H = p->run.width, B = p->batch;
   if (all_sgd(p) && (flags & DPC_FWD_COPY_NEXT))
   {
-    // (the order of additions: see the K-split variant below)
+    // (the K-split variant's order of additions, see below)
     const bool tf32 = p->ctx->precision == DPC_PRECISION_TF32;
     const int r0 = first - p->run.first;
     const TcParams P = base_params(p, st, first, count, B, H, H, 128, flags, 0);
