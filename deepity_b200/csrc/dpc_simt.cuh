@@ -1053,41 +1053,77 @@ __device__ __forceinline__ void psi_apply(const dpc_layer& L, int row, int k, fl
 // batch rows at a time sit in shared memory.  The eight warps' partial sums are added in a fixed
 // tree order through shared memory, then the CTAs of a row-split cluster in rank order.  Returns
 // true in the threads that end up with the sums (warp 0 of CTA 0 of the cluster).
-// (Measured alternatives, both slower: two columns per lane at twice the blocks per SM, and the
-// rows of g of the whole batch in shared memory so that the row loop has no barrier.)
+// What bounds it: bytes in flight.  A lane copies its pieces of the warp's next eight rows ahead (it alone reads them: no
+// barrier), also across groups of 128 rows, and the next group's rows of g are read before this one's products (four rows in
+// registers, drained at every group, took 500 us for 512 layers of 1024 x 512 instead of 302, the reads take 161).
+template <int KC>
+constexpr int kOuterFloats = 2 * 128 * KC + 8 * 8 * 128; // rows of g, twice; eight rows a warp, then the partial sums
 template <int KC>
 __device__ __forceinline__ bool batch_outer4(const float* __restrict__ zin, int s, int col,
                                              const float* __restrict__ g, int ldg, int TS,
-                                             int batch, float (&acc)[4][KC], float (*es)[KC],
-                                             float (*part)[4 * KC][32])
+                                             int batch, float (&acc)[4][KC], float* smem)
 {
-  constexpr int ROWS = 128;
+  constexpr int ROWS = 128, D = 8, PER = ROWS * KC / 256;
+  static_assert(4 * 4 * KC * 32 <= 8 * D * 128, "the partial sums fit where the rows were");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float(*part)[4 * KC][32] = reinterpret_cast<float(*)[4 * KC][32]>(smem + 2 * ROWS * KC);
 #pragma unroll
   for (int c = 0; c < 4; ++c)
 #pragma unroll
     for (int k = 0; k < KC; ++k)
       acc[c][k] = 0.0f;
   const uint32_t R = rows_cluster_size(), rank = rows_cluster_rank();
-  for (int b0 = (int)rank * ROWS; b0 < batch; b0 += (int)R * ROWS)
+  const int stride = (int)R * ROWS;
+  float* ring = smem + 2 * ROWS * KC + warp * D * 128 + lane * 4;
+  int fb = (int)rank * ROWS, fr = warp; // the row to copy next: group and row in it
+  auto fetch = [&](int to)
   {
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < ROWS * KC; idx += 256)
+    if (fb + fr < batch)
     {
-      const int r = idx / KC, k = idx - r * KC;
-      es[r][k] = (b0 + r < batch && k < TS) ? g[(size_t)(b0 + r) * ldg + k] : 0.0f;
+      cp_async16(ring + to * 128, zin + (size_t)(fb + fr) * s + col, true);
+      fr += 8;
+      if (fr >= ROWS)
+        fb += stride, fr = warp;
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int q = 0; q < D; ++q)
+    fetch(q);
+  float next[PER];
+  auto read_g = [&](int b0)
+  {
+#pragma unroll
+    for (int q = 0; q < PER; ++q)
+    {
+      const int idx = threadIdx.x + 256 * q, r = idx / KC, k = idx - r * KC;
+      next[q] = (b0 + r < batch && k < TS) ? g[(size_t)(b0 + r) * ldg + k] : 0.0f;
+    }
+  };
+  read_g((int)rank * ROWS);
+  int slot = 0;
+  float* es = smem;
+  for (int b0 = (int)rank * ROWS; b0 < batch; b0 += stride)
+  {
+#pragma unroll
+    for (int q = 0; q < PER; ++q)
+      es[threadIdx.x + 256 * q] = next[q];
     __syncthreads();
+    read_g(b0 + stride);
     const int rows = min(ROWS, batch - b0);
-#pragma unroll 4
+#pragma unroll 2
     for (int r = warp; r < rows; r += 8)
     {
-      const float4 z4 = *reinterpret_cast<const float4*>(zin + (size_t)(b0 + r) * s + col);
+      asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
+      const float4 z4 = *reinterpret_cast<const float4*>(ring + slot * 128);
+      __syncwarp();
+      fetch(slot);
+      slot = (slot + 1) & (D - 1);
       const float zv[4] = {z4.x, z4.y, z4.z, z4.w};
 #pragma unroll
       for (int k4 = 0; k4 < KC; k4 += 4)
       {
-        const float4 e4 = *reinterpret_cast<const float4*>(&es[r][k4]);
+        const float4 e4 = *reinterpret_cast<const float4*>(es + r * KC + k4);
 #pragma unroll
         for (int c = 0; c < 4; ++c)
         {
@@ -1098,7 +1134,9 @@ __device__ __forceinline__ bool batch_outer4(const float* __restrict__ zin, int 
         }
       }
     }
+    es = es == smem ? smem + ROWS * KC : smem; // (the barrier of the group in between guards it)
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
   // tree over the warps: (w, w+4), then (w, w+2), then (0, 1)
 #pragma unroll
   for (int half = 4; half >= 1; half >>= 1)
@@ -1151,7 +1189,7 @@ __device__ __forceinline__ bool batch_outer4(const float* __restrict__ zin, int 
 // The Psi update for the common aligned case (layer width a multiple of 128, at most KC terminal
 // units, KC = 12 or 16): a block owns 128 rows of Psi (= 128 columns of z).
 template <int KC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
     psi_update4_kernel(const dpc_layer* __restrict__ layers, int first, int n_layers, int batch,
                        const float* __restrict__ eT, int grad_only)
 {
@@ -1164,11 +1202,10 @@ __global__ void __launch_bounds__(256)
   const int TS = L.terminal_size, s = L.size;
   if ((int)blockIdx.x * 128 >= s)
     return;
-  __shared__ __align__(16) float es[128][KC];
-  __shared__ float part[4][4 * KC][32];
+  __shared__ __align__(16) float smem[kOuterFloats<KC>];
   const int col = blockIdx.x * 128 + (threadIdx.x & 31) * 4;
   float acc[4][KC];
-  if (!batch_outer4<KC>(L.z, s, col, eT, TS, TS, batch, acc, es, part))
+  if (!batch_outer4<KC>(L.z, s, col, eT, TS, TS, batch, acc, smem))
     return;
   const float step = psi_step(L, grad_only);
 #pragma unroll
@@ -1343,7 +1380,7 @@ __device__ __forceinline__ void weight_apply(const dpc_layer& L, size_t o, float
 // a layer size/64 blocks that each walk the whole batch; here the batch is split over warps and
 // over the CTAs of a cluster as in the Psi update, whose shape this product shares.
 template <int KC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
     narrow_weight_kernel(const dpc_layer* __restrict__ layers, int first, int n_layers, int batch,
                          int flags, int mode)
 {
@@ -1360,11 +1397,10 @@ __global__ void __launch_bounds__(256)
     return;
   const float* g = (simple && base_mode == WG_LEARN) ? layers[li + 1].e : L.fe;
   const float* zin = simple ? L.zF : L.z;
-  __shared__ __align__(16) float es[128][KC];
-  __shared__ float part[4][4 * KC][32];
+  __shared__ __align__(16) float smem[kOuterFloats<KC>];
   const int col = blockIdx.x * 128 + (threadIdx.x & 31) * 4;
   float acc[4][KC];
-  if (!batch_outer4<KC>(zin, s, col, g, M, M, batch, acc, es, part))
+  if (!batch_outer4<KC>(zin, s, col, g, M, M, batch, acc, smem))
     return;
   const float step = mode == WG_LEARN && L.opt != DPC_OPT_SGD ? adam_step_size(L.lr, *L.t) : 0.0f;
 #pragma unroll
