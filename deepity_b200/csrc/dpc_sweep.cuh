@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kSweepThreads<ROWS>, 1)
     // ---------------------------------------------------------------- multiplications (the warp together, one lane issues)
     constexpr uint32_t FMT = TF32 ? 2u : 1u;
     constexpr uint32_t BASE = (1u << 4) | (FMT << 7) | (FMT << 10) | (1u << 16) | ((uint32_t)(128 >> 4) << 24);
-    constexpr uint32_t ONE = BASE | ((uint32_t)(HALF >> 3) << 17), BOTH = BASE | ((uint32_t)(2 * HALF >> 3) << 17);
+    constexpr uint32_t ONE = BASE | ((uint32_t)(HALF >> 3) << 17);
     constexpr uint32_t BYTES = BULK ? 128 * 128 : 128 * 4 * ROWS;
     const uint64_t da0 = make_desc(smem_u32(ring), 16, 1024, 2);
     const uint64_t db0 = make_desc(smem_u32(zbuf), 8192, TF32 ? 512 : 1024, TF32 ? 1 : 2);
@@ -182,9 +182,15 @@ __global__ void __launch_bounds__(kSweepThreads<ROWS>, 1)
       for (int i = 0; i < blocks * SOURCE_KB; ++i)
       {
         const int kb = SOURCE_KB * source(i / SOURCE_KB) + i % SOURCE_KB;
+        // A layer's first multiplications overwrite the sums.  What orders them behind this block's epilogue of the layer
+        // below, which loads them, is its own part of the operand: with two blocks, and for the even ones of four, that is
+        // also the part that is multiplied first; the odd ones of four begin with another block's, which may be here while
+        // their own epilogue still loads (a block whose weights came late), so all wait for both.
+        if (l > 0 && i == 0)
+          alive = __all_sync(0xffffffffu, mbar_wait_cluster(&ready[rank], ((l - 1) >> 1) & 1, abort_flag));
         if (l > 0 && i % SOURCE_KB == 0)
         {
-          alive = __all_sync(0xffffffffu, mbar_wait_cluster(&ready[kb / SOURCE_KB], ((l - 1) >> 1) & 1, abort_flag));
+          alive = alive && __all_sync(0xffffffffu, mbar_wait_cluster(&ready[kb / SOURCE_KB], ((l - 1) >> 1) & 1, abort_flag));
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
         alive = alive && __all_sync(0xffffffffu, mbar_wait(&full[s], phase, abort_flag));
@@ -286,7 +292,7 @@ __global__ void __launch_bounds__(kSweepThreads<ROWS>, 1)
 #pragma unroll
       for (int r = 0; r < 8; ++r)
         pre[r] += half1[r];
-      tc_fence_before(); // the accumulator is free when the next layer's operands are complete
+      tc_fence_before(); // (arriving at ready[rank] below says that the sums have been loaded)
       float f[8], d[8];
 #pragma unroll
       for (int r = 0; r < 8; ++r)

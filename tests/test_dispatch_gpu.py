@@ -78,6 +78,33 @@ def test_cluster_sweep(name, precision, monkeypatch):
     assert not different, different
 
 
+@pytest.mark.parametrize("precision", ["fp32", "tf32"])
+@pytest.mark.parametrize("batch", [256, 1024])
+def test_deep_cluster_sweep_repeats(batch, precision, monkeypatch, built_library):
+    """130 layers of 512 units, 8 and 32 rows a cluster of four blocks: weights beyond L2, blocks of a cluster that drift
+    apart.  The beliefs after a sweep are those of the tiles, bit for bit, every time (predictions change no weights)."""
+    import torch
+    case = _case("dkp", [512] * 131 + [10], batch, T=0)
+
+    def beliefs(net, x):
+        net.predict(x, 0)
+        return torch.cat([torch.as_tensor(_View(net.tensor_ptr(l, "z"), (batch, 512)), device="cuda")
+                          for l in range(1, 131)]).clone()
+
+    net, x, _ = build_gpu_net(case, precision)
+    first = beliefs(net, x)
+    for _ in range(5):
+        assert torch.equal(beliefs(net, x), first)
+    monkeypatch.setenv("DPC_DISABLE_CLUSTER_SWEEP", "1")
+    net, x, _ = build_gpu_net(case, precision)
+    assert torch.equal(beliefs(net, x), first)
+
+
+class _View:
+    def __init__(self, ptr, shape):
+        self.__cuda_array_interface__ = {"shape": shape, "typestr": "<f4", "version": 3, "data": (ptr, False)}
+
+
 GROUPED = {
     # 32 x 32 tiles: one row over a tile, K not a multiple of the stage, rows not 16-byte aligned
     "gemm_32_edges": _case("dkp", [33, 65, 31, 10], 65),
