@@ -106,6 +106,27 @@ def build_plugin(force: bool = False) -> str | None:
     return PLUGIN_OUT
 
 
+PLUGIN_KERNELS_OUT = os.path.join(PKG, "build", "libb200_plugin_kernels.so")
+
+
+def build_plugin_kernels(force: bool = False) -> str:
+    """The plugin's CUDA translation unit, which needs nothing of the reference, behind the flat C functions of
+    tests/plugin_kernels.cpp: its kernels compile and are tested where the reference's header is absent too."""
+    driver = os.path.join(ROOT, "tests", "plugin_kernels.cpp")
+    srcs = [os.path.join(PLUGIN_DIR, f) for f in os.listdir(PLUGIN_DIR)] + \
+           [os.path.join(CSRC, "dpc_tcgen05.cuh"), driver, os.path.abspath(__file__)]
+    if not force and os.path.exists(PLUGIN_KERNELS_OUT) and \
+            all(os.path.getmtime(f) <= os.path.getmtime(PLUGIN_KERNELS_OUT) for f in srcs):
+        return PLUGIN_KERNELS_OUT
+    os.makedirs(os.path.dirname(PLUGIN_KERNELS_OUT), exist_ok=True)
+    print("[deepity_b200] building", PLUGIN_KERNELS_OUT, file=sys.stderr)
+    subprocess.run([nvcc_path(), "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3",
+                    "-std=c++17", "-shared", "-Xcompiler", "-fPIC,-fvisibility=hidden,-O2", "-I", CSRC,
+                    "-I", PLUGIN_DIR, os.path.join(PLUGIN_DIR, "b200_backend.cu"), driver,
+                    "-o", PLUGIN_KERNELS_OUT], check=True)
+    return PLUGIN_KERNELS_OUT
+
+
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="-v" in sys.argv))
     if "--plugin" in sys.argv:

@@ -183,9 +183,10 @@ __device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* m
                "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_addr), "r"(c0), "r"(c1), "r"(c2)
                : "memory");
 }
-// Multiplications and commits are issued by one lane of a warp that is converged (the warp as a whole runs the loop around
-// them): the elected lane is known to the compiler, which keeps the descriptors in uniform registers.  40 cycles an
-// instruction, 125 where a branch of one lane formed them as it went.
+// Multiplications and commits (tc_mma_*, tc_commit*) are issued by one lane of a warp that is converged: ALL 32 lanes call
+// them, with the same arguments -- the election names the full warp, and inside a branch of one lane it is undefined.
+// Waits before them end for the warp as a whole (__all_sync).  The elected lane is known to the compiler, which keeps the
+// descriptors in uniform registers: 40 cycles an instruction, 125 where a branch of one lane formed them as it went.
 __device__ __forceinline__ void tc_commit_pair(uint32_t bar_addr)
 {
   asm volatile("{\n\t.reg .pred q;\n\t"

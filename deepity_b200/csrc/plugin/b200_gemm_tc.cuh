@@ -4,8 +4,9 @@
 // own GPU backend uses by default (src/backend/cuda/CUDABackendGemm.cu:435-445,
 // CUDABackendCore.cu:54-67).  One CTA per 128 x BN output tile: warp 0 streams 32-wide k-blocks
 // of both operands through a shared-memory ring by TMA (2-D tensor maps built per call from the
-// caller's pointers and leading dimensions; every CTA loads its own tiles), warp 1 issues the MMAs, warps 2-5
-// read the accumulator (one tensor-memory quarter each) and apply alpha / beta.
+// caller's pointers and leading dimensions; every CTA loads its own tiles), warp 1 issues the MMAs
+// (as a whole: they elect a lane), warps 2-5 read the accumulator (one tensor-memory quarter each) and apply
+// alpha / beta.
 //
 // Either operand may be "K-major" (k contiguous in memory: A not transposed, B transposed) or
 // "MN-major" (A transposed, B not transposed).  32-bit MN-major operands need the 128-byte
@@ -127,45 +128,42 @@ __global__ void __launch_bounds__(192, 1)
   }
   else if (warp == 1)
   {
-    if (lane == 0)
+    // K-major fp32 tiles: 128-byte rows, 8 per swizzle atom (1024 B between row groups), 32 B per
+    // K = 8 step.  MN-major: slabs of 32 columns BK*128 bytes apart, 4 k-rows per 32-byte-atom
+    // swizzle group (512 B between groups), 1024 B per K = 8 step.
+    const uint64_t da0 = make_desc(smem_u32(smem), A_MN ? BK * 128 : 16, A_MN ? 512 : 1024, A_MN ? 1 : 2);
+    const uint64_t db0 = make_desc(smem_u32(smem) + C::A_BYTES, B_MN ? BK * 128 : 16,
+                                   B_MN ? 512 : 1024, B_MN ? 1 : 2);
+    const uint32_t a_adv = A_MN ? 1024 : 32, b_adv = B_MN ? 1024 : 32;
+    uint32_t phase = 0;
+    bool alive = true;
+    for (int kb = 0, s = 0; kb < kblocks; ++kb)
     {
-      // K-major fp32 tiles: 128-byte rows, 8 per swizzle atom (1024 B between row groups), 32 B per
-      // K = 8 step.  MN-major: slabs of 32 columns BK*128 bytes apart, 4 k-rows per 32-byte-atom
-      // swizzle group (512 B between groups), 1024 B per K = 8 step.
-      const uint64_t da0 = make_desc(smem_u32(smem), A_MN ? BK * 128 : 16, A_MN ? 512 : 1024, A_MN ? 1 : 2);
-      const uint64_t db0 = make_desc(smem_u32(smem) + C::A_BYTES, B_MN ? BK * 128 : 16,
-                                     B_MN ? 512 : 1024, B_MN ? 1 : 2);
-      const uint32_t a_adv = A_MN ? 1024 : 32, b_adv = B_MN ? 1024 : 32;
-      uint32_t phase = 0;
-      bool alive = true;
-      for (int kb = 0, s = 0; kb < kblocks; ++kb)
+      if (!__all_sync(0xffffffffu, mbar_wait(&full[s], phase, abort_flag)))
       {
-        if (!mbar_wait(&full[s], phase, abort_flag))
-        {
-          alive = false;
-          break;
-        }
-        tc_fence_after();
-        const uint64_t sa = da0 + (uint64_t)(s * (C::STAGE_BYTES >> 4));
-        const uint64_t sb = db0 + (uint64_t)(s * (C::STAGE_BYTES >> 4));
-#pragma unroll
-        for (int ks = 0; ks < BK / 8; ++ks)
-          tc_mma_tf32(tmem_base, sa + (uint64_t)(ks * (a_adv >> 4)), sb + (uint64_t)(ks * (b_adv >> 4)),
-                      C::IDESC, (kb | ks) != 0);
-        tc_commit(&empty[s]);
-        if (++s == C::STAGES)
-          s = 0, phase ^= 1;
+        alive = false;
+        break;
       }
-      if (alive)
-        tc_commit(tfull);
+      tc_fence_after();
+      const uint64_t sa = da0 + (uint64_t)(s * (C::STAGE_BYTES >> 4));
+      const uint64_t sb = db0 + (uint64_t)(s * (C::STAGE_BYTES >> 4));
+#pragma unroll
+      for (int ks = 0; ks < BK / 8; ++ks)
+        tc_mma_tf32(tmem_base, sa + (uint64_t)(ks * (a_adv >> 4)), sb + (uint64_t)(ks * (b_adv >> 4)),
+                    C::IDESC, (kb | ks) != 0);
+      tc_commit(&empty[s]);
+      if (++s == C::STAGES)
+        s = 0, phase ^= 1;
     }
+    if (alive)
+      tc_commit(tfull);
   }
   else
   {
     // epilogue: warp w reads tensor-memory lanes 32 (w & 3) .. +31 = rows of the tile
     const int quarter = warp & 3;
     const int m = m0 + quarter * 32 + lane;
-    if (kblocks == 0 || mbar_wait(tfull, 0, abort_flag))
+    if (kblocks == 0 || __all_sync(0xffffffffu, mbar_wait(tfull, 0, abort_flag)))
     {
       tc_fence_after();
       float* crow = P.C + (size_t)m * P.ldc + n0;

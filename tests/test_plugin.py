@@ -5,6 +5,7 @@ DEVICE_GPU -- the compiled reference host of oracle/_ref, whose loader dlopens t
 its own directory -- trains on this repository's kernels and agrees with the reference's CPU
 backend at the reference's own CPU-vs-GPU bound of 1e-2
 (tests/tDirectKPBatchedGPUVerify.cpp:47-58 in the reference)."""
+import ctypes
 import os
 import shutil
 import subprocess
@@ -152,6 +153,47 @@ def test_plugin_matmul_matches_blas(shape, plugin_beside_host):
                     assert err <= tol * np.sqrt(K), (shape, ta, tb, alpha, beta, allow, err)
                     # the padding columns of C are not part of the product: untouched
                     assert np.array_equal(got[:, N:], C0[:, N:])
+
+
+@pytest.fixture(scope="module")
+def plugin_kernels():
+    """The plugin's kernels by themselves (no reference host): one flat C function."""
+    from deepity_b200 import build
+    lib = ctypes.CDLL(build.build_plugin_kernels())
+    f32, i = np.ctypeslib.ndpointer(np.float32, flags="C_CONTIGUOUS"), ctypes.c_int
+    lib.plugin_matmul.argtypes = [i] * 5 + [ctypes.c_float, f32, ctypes.c_size_t, i, f32, ctypes.c_size_t, i,
+                                            ctypes.c_float, f32, ctypes.c_size_t, i, i, i]
+    return lib
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", GEMM_SHAPES + [(128, 64, 1024), (640, 320, 224)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_plugin_kernels_matmul(shape, plugin_kernels):
+    """The GEMM behind MatMul against numpy in 64 bits, one TF32 pass and (not allowed) fp32: K of one block and of
+    more than the ring's six stages, several tiles, padded rows, three calls in a row."""
+    M, N, K = shape
+    rng = np.random.default_rng(M * 1000 + N * 10 + K)
+    pad = 4 if (M % 4 == 0 and N % 4 == 0 and K % 4 == 0) else 3
+    for ta, tb in ((0, 0), (0, 1), (1, 0), (1, 1)):
+        a_cols, b_cols = (M if ta else K), (K if tb else N)
+        A = rng.normal(size=((K if ta else M), a_cols + pad)).astype(np.float32)
+        B = rng.normal(size=((N if tb else K), b_cols + pad)).astype(np.float32)
+        C0 = rng.normal(size=(M, N + pad)).astype(np.float32)
+        opA, opB = A[:, :a_cols].astype(np.float64), B[:, :b_cols].astype(np.float64)
+        opA, opB = opA.T if ta else opA, opB.T if tb else opB
+        product, size = opA @ opB, np.abs(opA) @ np.abs(opB)
+        for alpha, beta, calls in ((1.0, 0.0, 3), (-2.0, 0.25, 1)):
+            want = alpha * product + beta * C0[:, :N]
+            # an element's error: TF32 drops less than 2^-10 of each operand, fp32 sums round K times, the result twice
+            rounds = 2.0 ** -24 * (K * abs(alpha) * size + 2 * np.abs(want) + 2)
+            for allow, bound in ((-1, 2.0 ** -9 * 1.001 * abs(alpha) * size + rounds), (0, rounds)):
+                C = C0.copy()
+                assert plugin_kernels.plugin_matmul(ta, tb, M, N, K, alpha, A, A.size, A.shape[1], B, B.size,
+                                                    B.shape[1], beta, C, C.size, C.shape[1], allow, calls) == 0
+                worst = (np.abs(C[:, :N] - want) / bound).max()
+                assert worst <= 1.0, (ta, tb, alpha, beta, allow, worst)
+                assert np.array_equal(C[:, N:], C0[:, N:])
 
 
 @pytest.mark.gpu
