@@ -24,6 +24,7 @@
 // at batch 6 101 / 59.  With two outputs a lane (half the operand reads) the same step took 155, with three or four quads
 // ahead 131.
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
@@ -1045,8 +1046,9 @@ struct Layout
 };
 
 // one_block: the plan has the segments of dpc_resident.cu, whose order of additions an ordered network keeps; else that
-// of the phase kernels.
-bool lay_out(const dpc_plan* p, int C, int R, int RT, bool exact, bool one_block, bool has_v, int S, Layout& out)
+// of the phase kernels.  Without `tables` the tasks are counted, which is all that the estimate needs.
+bool lay_out(const dpc_plan* p, int C, int R, int RT, bool exact, bool one_block, bool has_v, int S, bool tables,
+             Layout& out)
 {
   const int nw = p->n - 1, rbs = R / RT;
   const bool ce = (p->h[p->n - 1].flags & DPC_LAYER_SOFTMAX_CE) != 0;
@@ -1081,17 +1083,17 @@ bool lay_out(const dpc_plan* p, int C, int R, int RT, bool exact, bool one_block
   while (!exact && lg0 < 2 && (rows0 + (16 >> lg0) - 1) / (16 >> lg0) * R <= kWarps)
     ++lg0;
 
-  std::vector<std::vector<unsigned char>> tables(C);
   std::vector<int> counts;
-  size_t region = 0, bytes = 0, most_ft = 0, most_bt = 0;
+  size_t region = 0, most_ft = 0, most_bt = 0;
   double forward = 0.0, state = 0.0, sweep = 0.0;
-  std::vector<std::vector<SegLayer>> layers(C, std::vector<SegLayer>(nw));
+  std::vector<std::vector<SegLayer>> layers(tables ? C : 1, std::vector<SegLayer>(nw));
   std::vector<std::vector<SegTask>> ft(C), bt(C);
   for (int r = 0; r < C; ++r)
   {
+    std::vector<SegLayer>& mine = layers[tables ? r : 0];
     size_t at = 0;
-    int off = 0;
-    std::vector<double> warp_f(kWarps, 0.0), warp_b(kWarps, 0.0);
+    int off = 0, nf = 0, nb = 0; // tasks
+    std::array<double, kWarps> warp_f{}, warp_b{};
     double reads_f = 0.0, reads_b = 0.0;
     auto cost = [&](int len, int lg) // cycles of a task alone, and of its shared-memory reads
     {
@@ -1101,15 +1103,15 @@ bool lay_out(const dpc_plan* p, int C, int R, int RT, bool exact, bool one_block
     for (int l = 0; l < nw; ++l)
     {
       const dpc_layer& L = p->h[l];
-      SegLayer& q = layers[r][l];
+      SegLayer& q = mine[l];
       q.K = L.size, q.N = L.next_size;
-      q.noff = off, q.zoff = l ? layers[r][l - 1].noff : 0;
+      q.noff = off, q.zoff = l ? mine[l - 1].noff : 0;
       off += up4(q.N);
       const int each = share(q.N);
       const bool whole = l + 1 == nw && ce;
       q.o0 = whole ? (r ? q.N : 0) : std::min(q.N, r * each);
       q.o1 = whole ? q.N : std::min(q.N, (r + 1) * each);
-      q.c0 = l ? layers[r][l - 1].o0 : 0, q.c1 = l ? layers[r][l - 1].o1 : 0;
+      q.c0 = l ? mine[l - 1].o0 : 0, q.c1 = l ? mine[l - 1].o1 : 0;
       q.vec = L.size % 4 == 0 && ((uintptr_t)L.W % 16) == 0;
       // (the shapes of the narrow forward kernel)
       q.lanes_k = exact && q.N <= 16 && q.K % 4 == 0 && q.K >= 128 && ((uintptr_t)L.z % 16) == 0 && q.vec &&
@@ -1123,9 +1125,11 @@ bool lay_out(const dpc_plan* p, int C, int R, int RT, bool exact, bool one_block
     }
     auto forward_tasks = [&](int l, int kind)
     {
-      const SegLayer& q = layers[r][l];
+      SegLayer& q = mine[l];
       const int lg = kind == T_DOT ? lanes[0][l] : 0, per = kind == T_LANES ? 2 : 32 >> lg;
-      for (int b = q.o0; b < q.o1; b += per)
+      q.f0 = nf;
+      q.f1 = nf += (q.o1 - q.o0 + per - 1) / per * rbs;
+      for (int b = q.o0; tables && b < q.o1; b += per)
         for (int rb = 0; rb < rbs; ++rb)
         {
           SegTask t = {};
@@ -1145,31 +1149,32 @@ bool lay_out(const dpc_plan* p, int C, int R, int RT, bool exact, bool one_block
     for (int k = 1; k <= nw; ++k)
     {
       const int l = k % nw;
-      SegLayer& q = layers[r][l];
+      const SegLayer& q = mine[l];
       const bool alone = one_block || nw == 2;
-      const int kind = l == 0 ? T_PLAIN : q.lanes_k && alone ? T_LANES : T_DOT;
-      q.f0 = (int)ft[r].size();
-      forward_tasks(l, kind);
-      q.f1 = (int)ft[r].size();
+      forward_tasks(l, l == 0 ? T_PLAIN : q.lanes_k && alone ? T_LANES : T_DOT);
       const auto c = l == 0 ? std::make_pair(400 + 60.0 * RT, 10.0) : cost(q.K, lanes[0][l]);
       for (int t = q.f0; t < q.f1; ++t)
         warp_f[t % kWarps] += c.first, reads_f += c.second;
       sweep = std::max(sweep, c.first * ((q.f1 - q.f0 + kWarps - 1) / kWarps));
     }
-    counts.push_back((int)ft[r].size());
+    counts.push_back(nf);
     for (int l = 1; l < nw; ++l)
-      if (SegLayer& q = layers[r][l]; q.lanes_k && !one_block && nw > 2)
-      {
-        q.f0 = (int)ft[r].size();
+      if (mine[l].lanes_k && !one_block && nw > 2)
         forward_tasks(l, T_LANES);
-        q.f1 = (int)ft[r].size();
-      }
     for (int l = 1; l <= nw; ++l)
     {
       const bool relax = l == nw;
-      const int c0 = layers[r][l - 1].o0, c1 = layers[r][l - 1].o1, off_l = layers[r][l - 1].noff;
+      const int c0 = mine[l - 1].o0, c1 = mine[l - 1].o1, off_l = mine[l - 1].noff;
       const int lg = relax ? 0 : lanes[1][l], per = 32 >> lg;
-      for (int b = c0; b < c1; b += per)
+      const int end = nb + (c1 - c0 + per - 1) / per * rbs;
+      if (!relax)
+      {
+        const auto c = cost(mine[l].N, lg);
+        for (int t = nb; t < end; ++t)
+          warp_b[t % kWarps] += c.first, reads_b += c.second;
+      }
+      nb = end;
+      for (int b = c0; tables && b < c1; b += per)
         for (int rb = 0; rb < rbs; ++rb)
         {
           SegTask t = {};
@@ -1177,21 +1182,19 @@ bool lay_out(const dpc_plan* p, int C, int R, int RT, bool exact, bool one_block
           t.units = (unsigned char)std::min(per, c1 - b), t.lg = (unsigned char)lg;
           if (!relax)
           {
-            const SegLayer& q = layers[r][l];
+            const SegLayer& q = mine[l];
             t.w = q.boff + b - c0, t.pitch = (unsigned short)q.bpitch;
             t.x = q.noff + rb * RT * S, t.len = (unsigned short)q.N;
             t.slice = (unsigned short)(lg ? odd4((q.N + (1 << lg) - 1) >> lg) : q.N);
             t.other = q.noff - q.zoff;
-            const auto c = cost(q.N, lg);
-            warp_b[bt[r].size() % kWarps] += c.first, reads_b += c.second;
           }
           t.first = off_l + b, t.row0 = (short)(rb * RT), t.layer = (short)l, t.j0 = (short)b;
           bt[r].push_back(t);
         }
     }
-    counts.push_back((int)bt[r].size());
+    counts.push_back(nb);
     region = std::max(region, at);
-    most_ft = std::max(most_ft, ft[r].size()), most_bt = std::max(most_bt, bt[r].size());
+    most_ft = std::max(most_ft, (size_t)nf), most_bt = std::max(most_bt, (size_t)nb);
     forward = std::max({forward, reads_f, *std::max_element(warp_f.begin(), warp_f.end())});
     state = std::max({state, reads_b, *std::max_element(warp_b.begin(), warp_b.end())});
   }
@@ -1219,11 +1222,12 @@ bool lay_out(const dpc_plan* p, int C, int R, int RT, bool exact, bool one_block
   out.C = C, out.R = R, out.RT = RT;
   out.smem = fixed + region * sizeof(float);
   const double sync = C > 1 ? 350 + 60 * C : 80;
-  for (int r = 0; r < C; ++r)
-    bytes = std::max(bytes, region * sizeof(float));
-  out.cycles = 6000 + bytes / 50.0 + (double)rows0 * K0p * 4 / 50.0 + R * (K0p + S) / 100.0 +
+  // (the whole region, the input layer's steps included: the rule below was measured with it)
+  out.cycles = 6000 + region * sizeof(float) / 50.0 + (double)rows0 * K0p * 4 / 50.0 + R * (K0p + S) / 100.0 +
                nw * (sweep + sync) + 8 * (forward + state + 2 * sync);
 
+  if (!tables)
+    return true;
   SegParams& P = out.P;
   P = SegParams{};
   P.table_vecs = (int)(table / 16), P.a_ft = (int)a_ft, P.a_bt = (int)a_bt, P.a_lq = (int)a_lq;
@@ -1286,26 +1290,43 @@ int cluster_plan_init(dpc_plan* p)
     has_v |= L.v != nullptr && l > 0;
     S += up4(L.next_size);
   }
-  Layout best;
   const char* force = getenv("DPC_CLUSTER_SIZE");
-  for (int C = 1; C <= 16; C *= 2)
+  const bool streams = res_plan_streams(p), either = p->res && !force; // single blocks can, too
+  // (cheap answers first: weights that fit no cluster, held twice; what the rule below turns down by the network's shape)
+  if (8 * weights > 16 * kSmemLimit || (either && !exact && !streams && (weights < 16000 || longest < 48)))
+    return 1;
+  auto estimate = [&](int C, int R, int RT, Layout& x)
+  { return lay_out(p, C, R, RT, exact, p->res != nullptr, has_v, S, false, x); };
+  // The best layout of clusters of C blocks, so many of them at once.  (One group of rows a cluster: weights that are loaded
+  // again for the next group are what phase kernels do better.)
+  auto choose = [&](int C, int clusters, Layout& best)
   {
-    if (force && atoi(force) != C)
-      continue;
-    const int clusters = resident_clusters(p->ctx, C);
-    if (clusters == 0)
-      continue;
-    // (one group of rows a cluster: weights that are loaded again for the next group are what phase kernels do better)
     const int rows = (p->batch + clusters - 1) / clusters;
     for (int RT = 1; RT <= 4 && RT < 2 * rows; RT *= 2)
     {
       Layout x;
       const int R = (rows + RT - 1) / RT * RT;
-      if (R <= 64 && lay_out(p, C, R, RT, exact, p->res != nullptr, has_v, S, x) &&
-          (best.C == 0 || x.cycles < best.cycles))
+      if (R <= 64 && estimate(C, R, RT, x) && (best.C == 0 || x.cycles < best.cycles))
         best = x;
     }
+  };
+  Layout best;
+  if (!force || atoi(force) == 1)
+    choose(1, p->ctx->sm_count, best);
+  // Sliced segments that fit one block leave it only for clusters with one row each.  Where these are no faster than one
+  // block, the device need not be asked how many clusters it holds (1 ms in a process's first plan).
+  bool ask = !(either && !exact && !streams);
+  for (int C = 2; C <= 16 && !ask; C *= 2)
+  {
+    Layout x;
+    ask = p->batch <= p->ctx->sm_count / C && estimate(C, 1, 1, x) && (best.C == 0 || x.cycles < best.cycles);
   }
+  if (!ask)
+    return 1;
+  for (int C = 2; C <= 16; C *= 2)
+    if (!force || atoi(force) == C)
+      if (const int clusters = resident_clusters(p->ctx, C))
+        choose(C, clusters, best);
   if (best.C == 0)
     return 1;
   // Against the segments of single blocks, us a step: ordered sums are one chain either way, and gain where it was read
@@ -1315,9 +1336,10 @@ int cluster_plan_init(dpc_plan* p)
   // pass (202-202-202-10 at batch 167 171 / 121, 100-(273x4)-10 268 / 117) or blocks were left over (784-(58x6)-10 at
   // batch 3 110 / 89; 784-(76x4)-10 at batch 153 125 / 146, 784-(40x23)-10 at batch 19 136 / 146).
   // Against phase kernels everything that fits gains (1.1 to 3).
-  const bool streams = res_plan_streams(p);
-  if (p->res && !force && (exact ? (best.C == 1 && longest < 64 && p->h[0].size < 2048) || (best.R > 8 && !streams)
-                       : !streams && !(best.R == 1 && best.C > 1 && weights >= 16000 && longest >= 48)))
+  if (either && (exact ? (best.C == 1 && longest < 64 && p->h[0].size < 2048) || (best.R > 8 && !streams)
+                       : !streams && !(best.R == 1 && best.C > 1)))
+    return 1;
+  if (!lay_out(p, best.C, best.R, best.RT, exact, p->res != nullptr, has_v, S, true, best))
     return 1;
   auto* st = new SegState();
   if (cudaMalloc(&st->dev, best.host.size()) != cudaSuccess ||
