@@ -1331,13 +1331,30 @@ int cluster_plan_init(dpc_plan* p)
     return 1;
   // Against the segments of single blocks, us a step: ordered sums are one chain either way, and gain where it was read
   // from L2 (784-441-441-10, SimplePC, ReLU, batch 25, T 11 401 / 141, 784-(77x7)-10 165 / 116) or the input layer's was
-  // (3072-(53x3)-10 182 / 159), little where it is short (100-(47x3)-10 60 / 69, 100-(28x30)-10 147 / 163) or many rows
+  // (3072-(53x3)-10 182 / 159), little where it is short (100-(47x3)-10 60 / 69, 100-(28x30)-10 141 / 161) or many rows
   // share a cluster (3072-74-10 at batch 460 398 / 412).  Sliced ones gain where a block reads weights from L2 on every
   // pass (202-202-202-10 at batch 167 171 / 121, 100-(273x4)-10 268 / 117) or blocks were left over (784-(58x6)-10 at
   // batch 3 110 / 89; 784-(76x4)-10 at batch 153 125 / 146, 784-(40x23)-10 at batch 19 136 / 146).
-  // Against phase kernels everything that fits gains (1.1 to 3).
-  if (either && (exact ? (best.C == 1 && longest < 64 && p->h[0].size < 2048) || (best.R > 8 && !streams)
-                       : !streams && !(best.R == 1 && best.C > 1)))
+  if (either && (exact ? best.C == 1 && longest < 64 && p->h[0].size < 2048 : !streams && !(best.R == 1 && best.C > 1)))
+    return 1;
+  // With one row a cluster almost all that fits gains, against phase kernels 1.1 to 3.  With several the rows share a
+  // cluster's few warps, and every layer of a sweep and every pass pays a barrier of the cluster's size, so the more a
+  // step takes by the estimate and the shorter its sums, the less is gained; single blocks and phase kernels spread rows
+  // over the SMs.  Lines from 7000 random networks (0.98 to 1.0 of the others' speed in the mean where they lie); beyond
+  // them, others / clusters: phase kernels 784-(64x20)-10, Adam, batch 80, T 10 241 / 367, 784-(128x9)-37, ReLU, batch 51
+  // 132 / 194, 48-(48x18)-10, Adam, batch 320 194 / 274; single blocks 784-(32x44)-10 at batch 79 231 / 395,
+  // 188-(188x3)-37, SimplePC, batch 192 112 / 161, 100-(320x2)-2, SimplePC, batch 128 202 / 315, with ordered sums
+  // 100-(80x5)-10, SimplePC, Adam, batch 512 157 / 245.
+  struct Limit
+  {
+    double few, many; // cycles that two or three rows a cluster may take, and more rows
+    int longest;      // by sums shorter than this
+  };
+  const Limit limit = !p->res ? Limit{120e3, 90e3, 150} : exact ? Limit{70e3, 50e3, 100} : Limit{100e3, 65e3, 200};
+  if (!force && !(p->res && exact && streams) &&
+      (best.R > 8 || (!p->res && !exact && best.R > 2) ||
+       (best.R > 1 && longest < limit.longest && best.cycles > (best.R < 4 ? limit.few : limit.many)) ||
+       (p->res && exact && longest < 40 && best.cycles > limit.few)))
     return 1;
   if (!lay_out(p, best.C, best.R, best.RT, exact, p->res != nullptr, has_v, S, true, best))
     return 1;

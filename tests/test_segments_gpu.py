@@ -130,7 +130,10 @@ def test_cluster_segments_match_oracle(name, blocks, monkeypatch, built_library)
                           ("dkp", [100, 47, 47, 10], 54, "relu", 0),   # a short chain: blocks by themselves
                           ("dkp", [64, 128, 128, 10], 64, "tanh", 0),  # sliced sums that fit one block
                           ("dkp", [100, 273, 273, 273, 10], 1, "tanh", 8),
-                          ("dkp", [64, 1024, 1024, 10], 1, "tanh", 0)])  # weights that fit no cluster
+                          ("dkp", [64, 1024, 1024, 10], 1, "tanh", 0),  # weights that fit no cluster
+                          # several rows a cluster, where other kernels take 0.6 to 0.7 of the time
+                          ("dkp", [784] + [128] * 9 + [37], 51, "relu", 0), ("dkp", [784] + [32] * 44 + [10], 79, "tanh", 0),
+                          ("simple", [188] * 4 + [37], 192, "sigmoid", 0), ("simple", [100, 320, 320, 2], 128, "gelu", 0)])
 def test_which_networks_run_on_clusters(kind, sizes, batch, act, blocks, built_library):
     from deepity_b200 import _lib
     lib = _lib.load()
