@@ -1335,11 +1335,12 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
       for (int c = 0; c < 4; ++c)
       {
+        // (said which product is fused: the compiler shares the subtraction of both branches in one instance, not in others)
         if (simple)
-          zz[c] += L.ir * (acc[c] * dd[c] - ee[c]);
+          zz[c] += L.ir * fmaf(acc[c], dd[c], -ee[c]);
         else
         {
-          const float fb = L.a * acc[c] - ee[c];
+          const float fb = fmaf(L.a, acc[c], -ee[c]);
           if (!PLAIN && L.v)
           {
             vv[c] = L.momentum_beta * vv[c] + (1.0f - L.momentum_beta) * fb;

@@ -138,6 +138,26 @@ GROUPED = {
 }
 
 
+@pytest.mark.parametrize("act", ["sigmoid", "tanh", "gelu", "esigmoid"])
+@pytest.mark.parametrize("kind,units", [("simple", 10), ("simple", 14), ("full", 10)])
+def test_head_state_update_rounds_like_the_general_kernel(kind, units, act, built_library, monkeypatch):
+    """Rows of a batch are independent and both kernels add up in ascending order: the beliefs under a head (a kernel of its
+    own from 256 rows on) are those of the general kernel at one row less, bit for bit."""
+    monkeypatch.setenv("DPC_DISABLE_RESIDENT", "1")
+    params, x, y = make_case(kind, [64, 256, units], 256)
+    out = []
+    for batch in (255, 256):
+        options = dict(mupc=1) if kind == "full" else {}
+        net, _, _ = build_gpu_net(_case(kind, [64, 256, units], batch, act, **options))
+        for l, p in enumerate(params):
+            for name, v in p.items():
+                net.set_tensor(l, name, v)
+        step = net.train_step_with_projection if kind == "simple" else net.train_step
+        step(x[:batch], y[:batch], 4)
+        out.append(np.asarray(net.get_tensor(1, "z")).reshape(batch, 256))
+    assert np.array_equal(out[0], out[1][:255])
+
+
 @pytest.mark.parametrize("name", sorted(GROUPED))
 def test_grouped_launches_match_oracle(name, built_library, monkeypatch):
     monkeypatch.setenv("DPC_DISABLE_RESIDENT", "1")
