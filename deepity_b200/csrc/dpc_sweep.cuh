@@ -389,8 +389,8 @@ int launch_cluster_sweep(dpc_plan* p, TcState* st, const CUtensorMap& w, const T
   const int H = p->run.width, B = p->batch, blocks = H / 128;
   if (getenv("DPC_DISABLE_CLUSTER_SWEEP") || (H != 256 && H != 512) || st->trace)
     return 1;
-  // Where the tiles would split K (their bits stay), and one wave of clusters is enough.  Larger batches fill the SMs with
-  // tiles; several waves of clusters took as long (24 layers of 512 units at batch 4096 453 us, a launch a layer 425).
+  // Where the tiles would split K (their bits stay).  Larger batches fill the SMs with tiles; several waves of clusters
+  // took as long (24 layers of 512 units at batch 4096 453 us, a launch a layer 425).
   if (2 * (B / TBM) * (H / 64) > p->ctx->sm_count || getenv("DPC_DISABLE_KSPLIT"))
     return 1;
   // As few rows a cluster as there are SMs for, so that every layer's epilogue and exchange are short.
@@ -404,13 +404,6 @@ int launch_cluster_sweep(dpc_plan* p, TcState* st, const CUtensorMap& w, const T
   auto kern = rows == 32   ? cluster_sweep_kernel<TF32, 32>
               : rows == 16 ? cluster_sweep_kernel<TF32, 16>
                            : cluster_sweep_kernel<TF32, 8>;
-  static thread_local int configured[3] = {-1, -1, -1};
-  int& device = configured[rows / 16];
-  if (device != p->ctx->device)
-  {
-    DPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
-    device = p->ctx->device;
-  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(B / rows * blocks));
   cfg.blockDim = dim3((unsigned)(rows == 32 ? kSweepThreads<32> : rows == 16 ? kSweepThreads<16> : kSweepThreads<8>));
@@ -421,6 +414,23 @@ int launch_cluster_sweep(dpc_plan* p, TcState* st, const CUtensorMap& w, const T
   attr[0].val.clusterDim = {(unsigned)blocks, 1, 1};
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  // One wave of clusters or none: how many run at once depends on how the SMs are grouped (33 of four blocks where 148 SMs
+  // would hold 37).  24 layers of 512 units with TF32, tiles / clusters: batch 1024 174 / 117 us, 1152, 36 clusters,
+  // 174 / 230.
+  struct Known
+  {
+    int device = -1, clusters = 0;
+  };
+  static thread_local Known known[2][3];
+  Known& at_once = known[H / 512][rows / 16];
+  if (at_once.device != p->ctx->device)
+  {
+    DPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
+    DPC_CUDA(cudaOccupancyMaxActiveClusters(&at_once.clusters, kern, &cfg));
+    at_once.device = p->ctx->device;
+  }
+  if (B / rows > at_once.clusters)
+    return 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, w, P, H, stages, st->chain_target_bias);
   p->ctx->launches += 1;
   return e == cudaSuccess ? DPC_OK : cuda_fail(e, "cluster sweep launch");

@@ -78,6 +78,16 @@ def test_cluster_sweep(name, precision, monkeypatch):
     assert not different, different
 
 
+def test_sweep_of_more_clusters_than_run_at_once():
+    """36 clusters of four blocks: 148 SMs hold fewer, so the tiles take the sweep (1152 rows, TF32)."""
+    from torch.profiler import ProfilerActivity, profile
+    case = _case("dkp", [20] + [512] * 3 + [10], 1152, T=1, steps=1)
+    with profile(activities=[ProfilerActivity.CUDA]) as launches:
+        _check(case, "sweep_4x32_two_waves", "tf32")
+    names = [event.key for event in launches.key_averages()]
+    assert any("pc_tc_kernel" in name for name in names) and not any("cluster_sweep" in name for name in names)
+
+
 @pytest.mark.parametrize("precision", ["fp32", "tf32"])
 @pytest.mark.parametrize("batch", [256, 1024])
 def test_deep_cluster_sweep_repeats(batch, precision, monkeypatch, built_library):
