@@ -149,14 +149,6 @@ __global__ void __launch_bounds__(kSweepThreads<ROWS>, 1)
             s = 0, phase ^= 1;
         }
       }
-      if (!alive)
-        for (int q = 0; q < stages; ++q) // copies in flight land before the shared memory goes away
-        {
-          const long long t0 = clock64();
-          while (clock64() - t0 < 2000000LL)
-          {
-          }
-        }
     }
   }
   else if (warp == 1)
@@ -372,9 +364,18 @@ __global__ void __launch_bounds__(kSweepThreads<ROWS>, 1)
 
   // ------------------------------------------------------------------ teardown
   tc_fence_before();
-  cluster_sync_all(); // no block leaves while another may still store to its shared memory
+  __syncthreads(); // whichever role gave up, all have ended and start no more copies
   if (threadIdx.x == 0 && *abort_flag)
+  {
     atomicExch(P.error_flag, 1);
+    // weights and other blocks' outputs that nobody waited for land before the shared memory goes away
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000LL)
+    {
+    }
+  }
+  __syncwarp();
+  cluster_sync_all(); // no block leaves while another may still store to its shared memory
   if (warp == 1)
   {
     tc_fence_after();
