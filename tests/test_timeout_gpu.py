@@ -24,8 +24,8 @@ def _case(width, batch):
                 hyper=dict(lr=1e-3, ir=0.1, fl=1e-3, lmbda=0.0, act="tanh"))
 
 
-# the sweep on clusters of four blocks with 32 rows and of two with 8
-@pytest.mark.parametrize("width,batch", [(512, 1024), (256, 256)])
+# the sweep on clusters (32 and 8 rows each) and on tiles that publish their rows, with K split and whole
+@pytest.mark.parametrize("width,batch", [(512, 1024), (256, 256), (768, 512), (768, 1024)])
 def test_a_wait_that_runs_out_is_reported_and_the_context_survives(width, batch, built_library):
     case = _case(width, batch)
     import deepity_b200 as dp
