@@ -1356,6 +1356,16 @@ int cluster_plan_init(dpc_plan* p)
        (best.R > 1 && longest < limit.longest && best.cycles > (best.R < 4 ? limit.few : limit.many)) ||
        (p->res && exact && longest < 40 && best.cycles > limit.few)))
     return 1;
+  // Networks of a head on a wide layer: their passes are the head's alone, and the wide layer's one product is what phase
+  // kernels spread over all SMs.  Multiply-adds of a block for it, in millions, and others / clusters in us:
+  // 0.6 784-1190-10, ReLU, batch 48 212 / 177;  1.9 1960-1960-2, ReLU, batch 48 159 / 327;  4.2 1026-512-2, batch 1024
+  // 436 / 568;  4.8 784-768-16, batch 878 314 / 451;  SimplePC, which has one segment a step:  1.9 784-1190-10, Adam, batch
+  // 256 476 / 324;  6.3 3072-512-10, batch 320 376 / 496.  (0.86 of the others' speed in the mean of 115 random networks
+  // beyond the line, 1.4 in 1685 before it.)
+  const dpc_layer& L0 = p->h[0];
+  const double product = 1.0 * best.R * std::min(L0.next_size, up4((L0.next_size + best.C - 1) / best.C)) * L0.size;
+  if (!force && nw == 2 && product > ((L0.flags & DPC_LAYER_INPUT_ACT) ? 3.5e6 : 1.2e6))
+    return 1;
   if (!lay_out(p, best.C, best.R, best.RT, exact, p->res != nullptr, has_v, S, true, best))
     return 1;
   auto* st = new SegState();

@@ -133,7 +133,9 @@ def test_cluster_segments_match_oracle(name, blocks, monkeypatch, built_library)
                           ("dkp", [64, 1024, 1024, 10], 1, "tanh", 0),  # weights that fit no cluster
                           # several rows a cluster, where other kernels take 0.6 to 0.7 of the time
                           ("dkp", [784] + [128] * 9 + [37], 51, "relu", 0), ("dkp", [784] + [32] * 44 + [10], 79, "tanh", 0),
-                          ("simple", [188] * 4 + [37], 192, "sigmoid", 0), ("simple", [100, 320, 320, 2], 128, "gelu", 0)])
+                          ("simple", [188] * 4 + [37], 192, "sigmoid", 0), ("simple", [100, 320, 320, 2], 128, "gelu", 0),
+                          # a head on a wide layer, whose product is most of a step
+                          ("dkp", [1960, 1960, 2], 48, "relu", 0), ("dkp", [784, 768, 16], 878, "sigmoid", 0)])
 def test_which_networks_run_on_clusters(kind, sizes, batch, act, blocks, built_library):
     from deepity_b200 import _lib
     lib = _lib.load()
