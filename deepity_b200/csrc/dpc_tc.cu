@@ -1898,8 +1898,8 @@ int launch(dpc_plan* p, TcState* st, const CUtensorMap& a, const CUtensorMap& b,
     if (!P.chain)
     {
       // No more pairs than the number of waves needs: 192 tiles take three on 64 pairs as on 74, and the SMs that are
-      // left run the head and the cached input of the phase meanwhile (784-(1024x4)-10 SimplePC at batch 4096 4.60 ->
-      // 3.96 ms a step, 3072-(1024x4)-10 with Adam 8.10 -> 8.00, 512-(512x12)-10 tf32 474 -> 459 us).  The head must fit
+      // left run the head and the cached input of the phase meanwhile (784-(1024x4)-10 SimplePC at batch 4096 4.93 ->
+      // 4.57 ms a step, 3072-(1024x4)-10 with Adam 8.10 -> 8.00, 512-(512x12)-10 tf32 474 -> 459 us).  The head must fit
       // into the launch's time there: with one that took 110 us of 20 SMs beside 85 the first of these was 1 % slower.
       const int waves = (total + pairs - 1) / pairs;
       pairs = (total + waves - 1) / waves;
