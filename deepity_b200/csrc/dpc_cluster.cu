@@ -1340,31 +1340,34 @@ int cluster_plan_init(dpc_plan* p)
   // With one row a cluster almost all that fits gains, against phase kernels 1.1 to 3.  With several the rows share a
   // cluster's few warps, and every layer of a sweep and every pass pays a barrier of the cluster's size, so the more a
   // step takes by the estimate and the shorter its sums, the less is gained; single blocks and phase kernels spread rows
-  // over the SMs.  Lines from 7000 random networks (0.98 to 1.0 of the others' speed in the mean where they lie); beyond
-  // them, others / clusters: phase kernels 784-(64x20)-10, Adam, batch 80, T 10 241 / 367, 784-(128x9)-37, ReLU, batch 51
-  // 132 / 194, 48-(48x18)-10, Adam, batch 320 194 / 274; single blocks 784-(32x44)-10 at batch 79 231 / 395,
-  // 188-(188x3)-37, SimplePC, batch 192 112 / 161, 100-(320x2)-2, SimplePC, batch 128 202 / 315, with ordered sums
-  // 100-(80x5)-10, SimplePC, Adam, batch 512 157 / 245.
+  // over the SMs.  SimplePC networks, with one segment a step instead of three, gain longer against phase kernels.  Lines
+  // from 8000 random networks (0.98 to 1.0 of the others' speed in the mean where they lie).  Beyond them, others /
+  // clusters: phase kernels 784-(64x20)-10, Adam, batch 80, T 10 241 / 367, 784-(128x9)-37, ReLU, batch 51 132 / 194,
+  // 48-(48x18)-10, Adam, batch 320 194 / 274; single blocks 784-(32x44)-10 at batch 79 231 / 395, 188-(188x3)-37,
+  // SimplePC, batch 192 112 / 161, 100-(320x2)-2, SimplePC, batch 128 202 / 315, with ordered sums 100-(80x5)-10,
+  // SimplePC, Adam, batch 512 157 / 245.
   struct Limit
   {
     double few, many; // cycles that two or three rows a cluster may take, and more rows
     int longest;      // by sums shorter than this
   };
-  const Limit limit = !p->res ? Limit{120e3, 90e3, 150} : exact ? Limit{70e3, 50e3, 100} : Limit{100e3, 65e3, 200};
+  const bool simple = p->h[0].flags & DPC_LAYER_INPUT_ACT;
+  const Limit limit = p->res ? (exact ? Limit{70e3, 50e3, 100} : Limit{longest < 46 ? 100e3 : 180e3, 65e3, 200})
+                             : (simple ? Limit{155e3, 155e3, 150} : Limit{120e3, 90e3, 150});
   if (!force && !(p->res && exact && streams) &&
-      (best.R > 8 || (!p->res && !exact && best.R > 2) ||
+      ((best.R > 8 && (p->res || !simple)) || (!p->res && !exact && !simple && best.R > 2) ||
        (best.R > 1 && longest < limit.longest && best.cycles > (best.R < 4 ? limit.few : limit.many)) ||
        (p->res && exact && longest < 40 && best.cycles > limit.few)))
     return 1;
   // Networks of a head on a wide layer: their passes are the head's alone, and the wide layer's one product is what phase
   // kernels spread over all SMs.  Multiply-adds of a block for it, in millions, and others / clusters in us:
-  // 0.6 784-1190-10, ReLU, batch 48 212 / 177;  1.9 1960-1960-2, ReLU, batch 48 159 / 327;  4.2 1026-512-2, batch 1024
+  // 0.5 784-1280-10, ReLU, batch 48 212 / 177;  1.9 1960-1960-2, ReLU, batch 48 159 / 327;  4.2 1026-512-2, batch 1024
   // 436 / 568;  4.8 784-768-16, batch 878 314 / 451;  SimplePC, which has one segment a step:  1.9 784-1190-10, Adam, batch
   // 256 476 / 324;  6.3 3072-512-10, batch 320 376 / 496.  (0.86 of the others' speed in the mean of 115 random networks
   // beyond the line, 1.4 in 1685 before it.)
   const dpc_layer& L0 = p->h[0];
   const double product = 1.0 * best.R * std::min(L0.next_size, up4((L0.next_size + best.C - 1) / best.C)) * L0.size;
-  if (!force && nw == 2 && product > ((L0.flags & DPC_LAYER_INPUT_ACT) ? 3.5e6 : 1.2e6))
+  if (!force && nw == 2 && product > (simple ? 3.5e6 : 1.2e6))
     return 1;
   if (!lay_out(p, best.C, best.R, best.RT, exact, p->res != nullptr, has_v, S, true, best))
     return 1;
